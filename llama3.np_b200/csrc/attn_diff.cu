@@ -58,25 +58,69 @@ __global__ void __launch_bounds__(256) diff_prep_kernel(DiffPrepArgs a) {
     for (int d = lane; d < DK; d += 32) { const float v = src[d] + bs[d]; ss = fmaf(v, v, ss); }
     const float rinv = 1.0f / sqrtf(warp_sum(ss) / (float)DK + a.eps);
     KVT* kdst = isq ? nullptr : (KVT*)a.cache_k + (((size_t)b * nk + (vec - nq)) * a.M + pos) * DK;
-    float* qdst = isq ? a.q_out + r * ((size_t)nq * DK) + (size_t)vec * DK : nullptr;
+    float* qdst = isq && a.q_out ? a.q_out + r * ((size_t)nq * DK) + (size_t)vec * DK : nullptr;
+    bf16* qhi = isq && a.q16 ? a.q16 + (r * nq + vec) * 2 * (size_t)a.q16_ld : nullptr;
+    auto put_q = [&](int d, float v) {
+      if (qdst) qdst[d] = v;
+      if (qhi) { qhi[d] = __float2bfloat16_rn(v); qhi[a.q16_ld + d] = __float2bfloat16_rn(bf16_rest(v)); }
+    };
     // a lane holds both entries of a rotated pair (i, i + half): no exchange between lanes
     for (int i = lane; i < half; i += 32) {
       const float lo = (src[i] + bs[i]) * rinv * w[i], hi = (src[i + half] + bs[i + half]) * rinv * w[i + half];
       const float sn = sn_tab[i], cs = cs_tab[i];
       const float o_lo = lo * cs - hi * sn, o_hi = hi * cs + lo * sn;
-      if (isq) { qdst[i] = o_lo; qdst[i + half] = o_hi; }
+      if (isq) { put_q(i, o_lo); put_q(i + half, o_hi); }
       else { kdst[i] = from_f32<KVT>(o_lo); kdst[i + half] = from_f32<KVT>(o_hi); }
     }
     for (int d = a.rot_dims + lane; d < DK; d += 32) {
       const float o = (src[d] + bs[d]) * rinv * w[d];
-      if (isq) qdst[d] = o;
+      if (isq) put_q(d, o);
       else kdst[d] = from_f32<KVT>(o);
     }
+    if (qhi)
+      for (int d = DK + lane; d < a.q16_ld; d += 32) qhi[d] = qhi[a.q16_ld + d] = __float2bfloat16_rn(0.f);
   }
   const int nv = a.G * a.DV;
   for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < nv; i += gridDim.y * blockDim.x) {
     const int g = i / a.DV, d = i - g * a.DV;
     ((KVT*)a.cache_v)[(((size_t)b * a.G + g) * a.M + pos) * a.DV + d] = from_f32<KVT>(pr[a.v_off + i] + a.bias[a.v_off + i]);
+  }
+}
+
+// Behind the tensor-core kernel (attn_latent_tc.cu): a warp per (row, head) combines the two maps' outputs and norms the head.
+// Bound by its traffic: 2 DV floats in, DV bf16 out.
+__global__ void __launch_bounds__(256) diff_combine_kernel(const float* __restrict__ maps, DiffAttnArgs a, int n) {
+  pdl_launch();
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);  // row * H + head
+  if (i >= n) return;
+  const float lam = *a.lambda;
+  const float* m1 = maps + (size_t)i * 2 * a.DV;
+  float ss = 0.f;
+  float4 o[2];  // DV <= 192: up to two groups of four entries per lane
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int d = (k * 32 + lane) * 4;
+    o[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (d >= a.DV) continue;
+    const float4 x = *reinterpret_cast<const float4*>(m1 + d), y = *reinterpret_cast<const float4*>(m1 + a.DV + d);
+    o[k] = make_float4(x.x - lam * y.x, x.y - lam * y.y, x.z - lam * y.z, x.w - lam * y.w);
+    ss = fmaf(o[k].x, o[k].x, ss); ss = fmaf(o[k].y, o[k].y, ss); ss = fmaf(o[k].z, o[k].z, ss); ss = fmaf(o[k].w, o[k].w, ss);
+  }
+  const float f = (1.0f - a.diff) / sqrtf(warp_sum(ss) / (float)a.DV + a.eps);
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int d = (k * 32 + lane) * 4;
+    if (d >= a.DV) continue;
+    const float4 v = make_float4(o[k].x * f, o[k].y * f, o[k].z * f, o[k].w * f);
+    const size_t at = (size_t)i * a.DV + d;
+    if (a.out) *reinterpret_cast<float4*>(a.out + at) = v;
+    if (a.out16) {
+      union { __nv_bfloat162 b[2]; uint2 u; } t;
+      t.b[0] = __floats2bfloat162_rn(v.x, v.y); t.b[1] = __floats2bfloat162_rn(v.z, v.w);
+      *reinterpret_cast<uint2*>(a.out16 + at) = t.u;
+    }
   }
 }
 
@@ -698,4 +742,10 @@ cudaError_t launch_diff_attn(const DiffAttnArgs& a, bool kv_bf16, float* part_o,
   auto kern = attn_diff_cta_kernel<float>;
   if (smem > 48 * 1024) { cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); if (e != cudaSuccess) return e; }
   return launch_k(kern, grid, dim3(DIFF_CTA_WARPS * 32), smem, s, a);
+}
+
+cudaError_t launch_diff_combine(const DiffAttnArgs& a, const float* maps, cudaStream_t s) {
+  if (a.DV % 4 || a.DV > 256) return cudaErrorInvalidValue;
+  const int n = a.B * a.L * a.H;
+  return launch_k(diff_combine_kernel, dim3((n + 7) / 8), dim3(256), 0, s, maps, a, n);
 }

@@ -18,8 +18,11 @@
 //                 rescaled lazily, only when a maximum has grown by more than 2^8.  At the end the two groups merge, add the
 //                 sink's term to the denominator, and apply the output gate.
 //      warp 10    TMA: the value blocks
-// Window and chunk attention (attn_window.cu) of prompts runs the same kernel with its caches as the key and value operands: the
-// key blocks then start at the first key the tile's first query sees, and scores outside a row's window are masked.
+// Softmax, window, chunk and differential attention of prompts run the same kernel with their caches as the key and value
+// operands: the key blocks then start at the first key the tile's first query sees (kept first keys come in blocks of their own
+// ahead of them), and scores outside a row's window are masked.  Mixers whose queries were fp32 hand them over as (high, low) bf16
+// pairs - the score products run twice, 16 significant bits -, sigmoid weights need neither maximum nor sum, and the two maps of
+// differential attention are two query heads over one set of values.
 // Every wait is bounded: one that runs out sets a flag, the CTA drains and the host reports an error.
 #include <cuda.h>
 
@@ -182,15 +185,17 @@ __global__ void __launch_bounds__(256) latent_q_pack_kernel(LatentQPackArgs a) {
 // ---------------------------------------------------------------- attention
 struct Shape {
   int nks, nrs, nqs, nvs;  // 64-entry slices of the un-rotated keys, the rotated part, both, the values
+  int qp;                  // bf16 parts of a query
   int kst, vst;            // depths of the key and value rings
-  __host__ __device__ int q_bytes() const { return nqs * SLICE_Q; }
+  __host__ __device__ int q_bytes() const { return qp * nqs * SLICE_Q; }
   __host__ __device__ int k_bytes() const { return nqs * SLICE_K; }
   __host__ __device__ int v_bytes() const { return nvs * SLICE_K; }
   __host__ __device__ int smem() const { return 1024 + q_bytes() + kst * k_bytes() + vst * v_bytes() + 4 * P_TILE + TAIL; }
 };
 
-__host__ __device__ inline Shape make_shape(int dim, int rot_dim, int vdim) {
+__host__ __device__ inline Shape make_shape(int dim, int rot_dim, int vdim, int q_parts) {
   Shape s;
+  s.qp = q_parts;
   s.nks = (dim + 63) / 64; s.nrs = (rot_dim + 63) / 64; s.nqs = s.nks + s.nrs; s.nvs = (vdim + 63) / 64;
   // a key block is refilled from L2 while the other ones of the ring are used: the keys, needed first, get the spare stage
   s.kst = s.vst = STAGES_MAX;
@@ -198,11 +203,12 @@ __host__ __device__ inline Shape make_shape(int dim, int rot_dim, int vdim) {
   return s;
 }
 
+template <bool SIGMOID>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmE,
                       const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmV, LatentTcArgs a) {
   extern __shared__ uint8_t smem_raw[];
-  const Shape sh = make_shape(a.dim, a.rot_dim, a.vdim);
+  const Shape sh = make_shape(a.dim, a.rot_dim, a.vdim, a.q_parts);
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sQ = (raw + 1023u) & ~1023u;
   const uint32_t sK = sQ + sh.q_bytes(), sV = sK + sh.kst * sh.k_bytes(), sP = sV + sh.vst * sh.v_bytes();
@@ -250,26 +256,29 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const int start = *a.pos_ptr;
   const int last_q = min(q0 + BQ, a.L) - 1;                // last real query row of this tile
   auto first_key = [&](int p) { return a.window <= 0 ? 0 : a.chunked ? p - p % a.window : max(0, p - a.window + 1); };
-  const int key_lo = first_key(start + q0);                // first key of the tile's blocks
-  const int nb = (start + last_q - key_lo) / BKV + 1;      // key blocks holding a visible key
-  const int kv_head = head / a.rep;
-  const int kv_row = bl * a.seq_rows + kv_head * a.head_rows + key_lo;
+  const int key_lo = first_key(start + q0);                // first key of the tile's blocks of window keys
+  const int n_keep = min(a.keep_first, key_lo);            // kept first keys ahead of them, in blocks of their own
+  const int nkb = (n_keep + BKV - 1) / BKV;
+  const int nb = nkb + (start + last_q - key_lo) / BKV + 1;  // key blocks holding a visible key
+  auto block_key = [&](int j) { return j < nkb ? j * BKV : key_lo + (j - nkb) * BKV; };
+  const int v_head = head / a.maps / a.rep, k_head = v_head * a.maps + head % a.maps;
+  const int k_row = bl * a.k_seq_rows + k_head * a.head_rows, v_row = bl * a.v_seq_rows + v_head * a.head_rows;
   const uint32_t tS = tmem_base, tO = tmem_base + 2 * BKV; // two score buffers, then the two groups' outputs
   const int o_cols = (a.vdim + 31) & ~31;
-  const int kcol0 = a.k_col + kv_head * a.k_cols, vcol0 = a.v_col + kv_head * a.v_cols;
+  const int kcol0 = a.k_col + k_head * a.k_cols, vcol0 = a.v_col + v_head * a.v_cols;
 
   if (warp == 0) {
     if (lane == 0) {  // ---------------- queries and keys
-      const int DQ = sh.nqs * 64;
+      const int nq = sh.qp * sh.nqs, DQ = nq * 64;
       mbar_expect_tx(q_full, sh.q_bytes());
-      for (int s = 0; s < sh.nqs; ++s) tma_load_2d(sQ + s * SLICE_Q, &tmQ, head * DQ + s * 64, b * a.L + q0, q_full);
+      for (int s = 0; s < nq; ++s) tma_load_2d(sQ + s * SLICE_Q, &tmQ, head * DQ + s * 64, b * a.L + q0, q_full);
       for (int j = 0; j < nb; ++j) {
         const int st = j % sh.kst, use = j / sh.kst;
         if (use > 0 && !mbar_wait(k_empty + 8 * st, (use - 1) & 1, fail)) break;
         const uint32_t kb = sK + st * sh.k_bytes(), bar = k_full + 8 * st;
         mbar_expect_tx(bar, sh.k_bytes());
-        for (int s = 0; s < sh.nks; ++s) tma_load_2d(kb + s * SLICE_K, &tmE, kcol0 + s * 64, kv_row + j * BKV, bar);
-        for (int s = 0; s < sh.nrs; ++s) tma_load_2d(kb + (sh.nks + s) * SLICE_K, &tmC, a.kv_rank + s * 64, b * a.M + j * BKV, bar);
+        for (int s = 0; s < sh.nks; ++s) tma_load_2d(kb + s * SLICE_K, &tmE, kcol0 + s * 64, k_row + block_key(j), bar);
+        for (int s = 0; s < sh.nrs; ++s) tma_load_2d(kb + (sh.nks + s) * SLICE_K, &tmC, a.kv_rank + s * 64, b * a.M + block_key(j), bar);
       }
     }
   } else if (warp == 10) {
@@ -279,7 +288,7 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (use > 0 && !mbar_wait(v_empty + 8 * st, (use - 1) & 1, fail)) break;
         mbar_expect_tx(v_full + 8 * st, sh.v_bytes());
         for (int s = 0; s < sh.nvs; ++s)
-          tma_load_2d(sV + st * sh.v_bytes() + s * SLICE_K, &tmV, vcol0 + s * 64, kv_row + j * BKV, v_full + 8 * st);
+          tma_load_2d(sV + st * sh.v_bytes() + s * SLICE_K, &tmV, vcol0 + s * 64, v_row + block_key(j), v_full + 8 * st);
       }
     }
   } else if (warp == 1) {
@@ -299,13 +308,15 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         tc_fence_after();
         const uint64_t dk = dk0 + (uint64_t)((st * sh.k_bytes()) >> 4);
         const uint32_t td = tS + w * BKV;
-        for (int s = 0; s < sh.nqs; ++s) {
-          const uint64_t ad = dq + (uint64_t)(s * (SLICE_Q >> 4)), bd = dk + (uint64_t)(s * (SLICE_K >> 4));
-          const int n = (steps >> (4 * s)) & 15;
+        uint64_t ad = dq;
+        for (int part = 0; part < sh.qp; ++part)  // high part of the queries, then what it leaves
+          for (int s = 0; s < sh.nqs; ++s, ad += SLICE_Q >> 4) {
+            const uint64_t bd = dk + (uint64_t)(s * (SLICE_K >> 4));
+            const int n = (steps >> (4 * s)) & 15;
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            if (kk < n) mma_bf16(td, ad + kk * 2, bd + kk * 2, IDESC_S, (s | kk) ? 1u : 0u);
-        }
+            for (int kk = 0; kk < 4; ++kk)
+              if (kk < n) mma_bf16(td, ad + kk * 2, bd + kk * 2, IDESC_S, (part | s | kk) ? 1u : 0u);
+          }
         tc_commit(k_empty + 8 * st);
         tc_commit(s_full + 8 * w);
         if (++st == sh.kst) { st = 0; ph ^= 1; }
@@ -339,6 +350,7 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const int qlo = first_key(qpos);
     const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
     const float sc = a.scale * LOG2E;                        // p = 2^((s - m) * sc)
+    const float sig_b = SIGMOID ? a.sink[head] * LOG2E : 0.f;
     const uint32_t tOw = tO + w * o_cols + lane_off;
     uint8_t* pw = sP_ptr + (2 * w) * P_TILE + r * 128;
     float m_used = -INFINITY, l_run = 0.f;
@@ -355,45 +367,48 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       tmem_ld_wait();
       tc_fence_before();
       mbar_arrive(s_empty + 8 * w);                          // S_j is in registers
-      const int key0 = key_lo + j * BKV;
-      if (key0 + BKV - 1 > qpos) {
+      const int key0 = block_key(j);
+      const int top = j < nkb ? n_keep - 1 : qpos;           // a block of kept keys ends with them: the rest lies in window blocks
+      if (key0 + BKV - 1 > top) {
 #pragma unroll
         for (int i = 0; i < BKV; ++i)
-          if (key0 + i > qpos) v[i] = -INFINITY;
+          if (key0 + i > top) v[i] = -INFINITY;
       }
-      if (key0 < qlo) {
+      if (j >= nkb && key0 < qlo) {
 #pragma unroll
         for (int i = 0; i < BKV; ++i)
-          if (key0 + i < qlo) v[i] = -INFINITY;
+          if (key0 + i < qlo && key0 + i >= a.keep_first) v[i] = -INFINITY;
       }
-      float mx4[4] = {v[0], v[1], v[2], v[3]};
-#pragma unroll
-      for (int i = 4; i < BKV; i += 4) {
-        mx4[0] = fmaxf(mx4[0], v[i]); mx4[1] = fmaxf(mx4[1], v[i + 1]);
-        mx4[2] = fmaxf(mx4[2], v[i + 2]); mx4[3] = fmaxf(mx4[3], v[i + 3]);
-      }
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       bool waited = false;
-      if (it == 0) {
-        m_used = mx;                                         // may stay -inf: this row sees no key of the block
-      } else {
-        const bool grow = (mx - m_used) * sc > 8.0f;         // false for two -inf (NaN)
-        if (__any_sync(L3_FULL, grow)) {
-          ok = __all_sync(L3_FULL, mbar_wait(p_empty + 8 * w, (it - 1) & 1, fail));  // the group's last PV is done: O is stable
-          if (!ok) break;
-          waited = true;
-          tc_fence_after();
-          const float alpha = grow ? fast_exp2((m_used - mx) * sc) : 1.0f;
-          if (grow) { m_used = mx; l_run *= alpha; }
-          for (int c = 0; c < o_cols; c += 32) {
-            float ov[32];
-            tmem_ld32_issue(tOw + c, ov);
-            tmem_ld_wait();
+      if constexpr (!SIGMOID) {
+        float mx4[4] = {v[0], v[1], v[2], v[3]};
 #pragma unroll
-            for (int i = 0; i < 32; ++i) ov[i] *= alpha;
-            tmem_st32(tOw + c, ov);
+        for (int i = 4; i < BKV; i += 4) {
+          mx4[0] = fmaxf(mx4[0], v[i]); mx4[1] = fmaxf(mx4[1], v[i + 1]);
+          mx4[2] = fmaxf(mx4[2], v[i + 2]); mx4[3] = fmaxf(mx4[3], v[i + 3]);
+        }
+        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+        if (it == 0) {
+          m_used = mx;                                         // may stay -inf: this row sees no key of the block
+        } else {
+          const bool grow = (mx - m_used) * sc > 8.0f;         // false for two -inf (NaN)
+          if (__any_sync(L3_FULL, grow)) {
+            ok = __all_sync(L3_FULL, mbar_wait(p_empty + 8 * w, (it - 1) & 1, fail));  // the group's last PV is done: O is stable
+            if (!ok) break;
+            waited = true;
+            tc_fence_after();
+            const float alpha = grow ? fast_exp2((m_used - mx) * sc) : 1.0f;
+            if (grow) { m_used = mx; l_run *= alpha; }
+            for (int c = 0; c < o_cols; c += 32) {
+              float ov[32];
+              tmem_ld32_issue(tOw + c, ov);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 32; ++i) ov[i] *= alpha;
+              tmem_st32(tOw + c, ov);
+            }
+            tc_fence_before();
           }
-          tc_fence_before();
         }
       }
       const float moff = m_used == -INFINITY ? 0.f : m_used * sc;
@@ -401,8 +416,14 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       uint32_t hi[BKV / 2], lo[BKV / 2];
 #pragma unroll
       for (int i = 0; i < BKV; i += 2) {
-        const float p0 = fast_exp2(fmaf(v[i], sc, -moff)), p1 = fast_exp2(fmaf(v[i + 1], sc, -moff));  // 2^-inf = 0
-        rs4[(i >> 1) & 3] += p0 + p1;
+        float p0, p1;
+        if constexpr (SIGMOID) {  // 1 / (1 + 2^-z): 0 for a masked score
+          p0 = __fdividef(1.0f, 1.0f + fast_exp2(fmaf(v[i], -sc, -sig_b)));
+          p1 = __fdividef(1.0f, 1.0f + fast_exp2(fmaf(v[i + 1], -sc, -sig_b)));
+        } else {
+          p0 = fast_exp2(fmaf(v[i], sc, -moff)); p1 = fast_exp2(fmaf(v[i + 1], sc, -moff));  // 2^-inf = 0
+          rs4[(i >> 1) & 3] += p0 + p1;
+        }
         const uint32_t t = pack_bf16(p0, p1);
         hi[i >> 1] = t;
         lo[i >> 1] = pack_bf16(p0 - __uint_as_float(t << 16), p1 - __uint_as_float(t & 0xffff0000u));
@@ -429,10 +450,13 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     tc_fence_after();
     if (*fail == 0) {
       const float2 g0 = ml[r], g1 = ml[BQ + r];
-      const float sk = a.sink ? a.sink[head] * LOG2E : -INFINITY;
-      const float mm = fmaxf(fmaxf(g0.x, g1.x), sk);
-      float f0 = fast_exp2(g0.x - mm), f1 = fast_exp2(g1.x - mm);  // a real row sees at least its own key: mm is finite
-      const float den = g0.y * f0 + g1.y * f1 + fast_exp2(sk - mm);
+      float f0 = 1.0f, f1 = 1.0f, den = 1.0f;
+      if constexpr (!SIGMOID) {
+        const float sk = a.sink ? a.sink[head] * LOG2E : -INFINITY;
+        const float mm = fmaxf(fmaxf(g0.x, g1.x), sk);
+        f0 = fast_exp2(g0.x - mm); f1 = fast_exp2(g1.x - mm);  // a real row sees at least its own key: mm is finite
+        den = g0.y * f0 + g1.y * f1 + fast_exp2(sk - mm);
+      }
       const bool real = q0 + r < a.L;
       const size_t row = (size_t)b * a.L + q0 + r;
       float inv = a.out_scale / den;
@@ -487,53 +511,62 @@ int latent_tc_q_ld(int dim, int rot_dim) { return ((dim + 63) & ~63) + ((rot_dim
 
 bool latent_tc_supported(int dim, int rot_dim, int vdim, int kv_rank) {
   if (dim % 8 || rot_dim % 8 || vdim % 8 || kv_rank % 8 || dim < 8 || vdim < 8 || vdim > 192 || !tc_gemm_supported(kv_rank + rot_dim)) return false;
-  return make_shape(dim, rot_dim, vdim).smem() <= 227 * 1024;
+  return make_shape(dim, rot_dim, vdim, 1).smem() <= 227 * 1024;
 }
 
 cudaError_t launch_latent_q_pack(const LatentQPackArgs& a, int rows, cudaStream_t s) {
   return launch_k(latent_q_pack_kernel, dim3(rows), dim3(256), (size_t)std::max(1, a.rot_dims) * sizeof(float), s, a);
 }
 
-static cudaError_t launch_tc(const CUtensorMap* mq, const CUtensorMap* mk, const CUtensorMap* mc, const CUtensorMap* mv, const LatentTcArgs& a,
-                             int n_seq, cudaStream_t s) {
+template <bool SIGMOID>
+static cudaError_t launch_tc_t(const CUtensorMap* mq, const CUtensorMap* mk, const CUtensorMap* mc, const CUtensorMap* mv, const LatentTcArgs& a,
+                               int n_seq, cudaStream_t s) {
   static bool done[16] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!done[dev & 15]) {
-    const cudaError_t e = cudaFuncSetAttribute(attn_latent_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    const cudaError_t e = cudaFuncSetAttribute(attn_latent_tc_kernel<SIGMOID>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return e;
     done[dev & 15] = true;
   }
   if (!mq || !mk || !mc || !mv) return cudaErrorInvalidValue;
   const dim3 grid(a.H, (a.L + BQ - 1) / BQ, n_seq);
-  return launch_k(attn_latent_tc_kernel, grid, dim3(THREADS), (size_t)make_shape(a.dim, a.rot_dim, a.vdim).smem(), s, *mq, *mk, *mc, *mv, a);
+  return launch_k(attn_latent_tc_kernel<SIGMOID>, grid, dim3(THREADS), (size_t)make_shape(a.dim, a.rot_dim, a.vdim, a.q_parts).smem(), s, *mq, *mk,
+                  *mc, *mv, a);
+}
+
+static cudaError_t launch_tc(const CUtensorMap* mq, const CUtensorMap* mk, const CUtensorMap* mc, const CUtensorMap* mv, const LatentTcArgs& a,
+                             int n_seq, cudaStream_t s) {
+  return a.sigmoid ? launch_tc_t<true>(mq, mk, mc, mv, a, n_seq, s) : launch_tc_t<false>(mq, mk, mc, mv, a, n_seq, s);
 }
 
 cudaError_t launch_attn_latent_tc(const LatentTcArgs& args, int n_seq, cudaStream_t s) {
   LatentTcArgs a = args;
-  a.rep = 1; a.seq_rows = a.e_rows; a.head_rows = 0;
+  a.rep = a.maps = a.q_parts = 1; a.k_seq_rows = a.v_seq_rows = a.e_rows; a.head_rows = 0;
   a.k_col = 0; a.k_cols = a.dim; a.v_col = a.H * a.dim; a.v_cols = a.vdim;
-  a.window = 0; a.chunked = 0; a.ld_out = a.H * a.vdim; a.out_scale = 1.f;
+  a.window = 0; a.chunked = 0; a.keep_first = 0; a.sigmoid = 0; a.ld_out = a.H * a.vdim; a.out_scale = 1.f;
   const CUtensorMap* me = tc_get_map(a.expand, true, a.e_seqs * a.e_rows, a.H * (a.dim + a.vdim), BKV);
   return launch_tc(tc_get_map(a.q16, true, a.n_rows, a.H * latent_tc_q_ld(a.dim, a.rot_dim), BQ), me,
                    tc_get_map(a.cache, true, a.c_seqs * a.M, a.kv_rank + a.rot_dim, BKV), me, a, n_seq, s);
 }
 
-bool win_attn_tc_supported(int DK, int DV, int kind, int keep_first, float scale, int ld_out) {
+bool win_attn_tc_supported(int DK, int DV, float scale, int ld_out, int q_parts) {
   // 16-byte rows in the caches and in the output; the map's box is one 64-entry slice wide
-  if (kind == L3_ATTN_SIGMOID || keep_first > 0 || !(scale > 0.f) || DK % 8 || DV % 8 || ld_out % 8 || DK < 64 || DV < 64 || DV > 192) return false;
-  return tc_gemm_supported(DK) && make_shape(DK, 0, DV).smem() <= 227 * 1024;
+  if (!(scale > 0.f) || DK % 8 || DV % 8 || ld_out % 8 || DK < 64 || DV < 64 || DV > 192) return false;
+  return tc_gemm_supported(DK) && make_shape(DK, 0, DV, q_parts).smem() <= 227 * 1024;
 }
 
-cudaError_t launch_win_attn_tc(const WinAttnArgs& w, const bf16* q16, int cache_seqs, int* err, cudaStream_t s) {
-  if (!win_attn_tc_supported(w.DK, w.DV, w.kind, w.keep_first, w.scale, w.ld_out) || w.H % w.G) return cudaErrorInvalidValue;
+cudaError_t launch_win_attn_tc(const WinAttnArgs& w, const bf16* q16, int q_parts, int cache_seqs, int* err, cudaStream_t s, int maps) {
+  if (!win_attn_tc_supported(w.DK, w.DV, w.scale, w.ld_out, q_parts) || w.H % (w.G * maps)) return cudaErrorInvalidValue;
   if (((uintptr_t)w.out | (uintptr_t)w.out16) & 15) return cudaErrorInvalidValue;
   LatentTcArgs a{};
   a.q16 = q16; a.out = w.out; a.out16 = w.out16; a.gate = w.gate; a.ld_gate = w.ld_gate; a.sink = w.head_vec; a.pos_ptr = w.pos_ptr;
   a.scale = w.scale; a.err = err; a.n_rows = w.B * w.L; a.L = w.L; a.H = w.H; a.dim = w.DK; a.vdim = w.DV; a.M = w.M;
-  a.rep = w.H / w.G; a.seq_rows = w.G * w.M; a.head_rows = w.M;
-  a.window = w.window; a.chunked = w.chunked; a.ld_out = w.ld_out; a.out_scale = w.out_scale;
-  const int rows = cache_seqs * w.G * w.M;
-  const CUtensorMap* mk = tc_get_map(w.cache_k, true, rows, w.DK, BKV);
-  return launch_tc(tc_get_map(q16, true, a.n_rows, a.H * latent_tc_q_ld(w.DK, 0), BQ), mk, mk, tc_get_map(w.cache_v, true, rows, w.DV, BKV), a, w.B, s);
+  a.maps = maps; a.rep = w.H / maps / w.G; a.k_seq_rows = w.G * maps * w.M; a.v_seq_rows = w.G * w.M; a.head_rows = w.M; a.q_parts = q_parts;
+  a.window = w.window; a.chunked = w.chunked; a.keep_first = w.keep_first; a.sigmoid = w.kind == L3_ATTN_SIGMOID;
+  a.ld_out = w.ld_out; a.out_scale = w.out_scale;
+  const int k_rows = cache_seqs * a.k_seq_rows, v_rows = cache_seqs * a.v_seq_rows;
+  const CUtensorMap* mk = tc_get_map(w.cache_k, true, k_rows, w.DK, BKV);
+  return launch_tc(tc_get_map(q16, true, a.n_rows, a.H * q_parts * latent_tc_q_ld(w.DK, 0), BQ), mk, mk,
+                   tc_get_map(w.cache_v, true, v_rows, w.DV, BKV), a, w.B, s);
 }

@@ -104,7 +104,12 @@ __global__ void __launch_bounds__(256) win_prep_kernel(WinPrepArgs a) {
     };
     KVT* ck = (KVT*)a.cache_k + (((size_t)b * a.G + g) * a.M + pos) * a.DK;
     float* qf = a.q_out ? a.q_out + ((size_t)r * a.H + v) * a.DK : nullptr;
-    bf16* qp = a.q16 ? a.q16 + ((size_t)r * a.H + v) * a.q16_ld : nullptr;
+    bf16* qp = a.q16 ? a.q16 + ((size_t)r * a.H + v) * a.q16_parts * a.q16_ld : nullptr;
+    bf16* ql = a.q16_parts == 2 ? qp + a.q16_ld : nullptr;  // what the first part leaves
+    auto put_q4 = [&](int i, float x0, float x1, float x2, float x3) {
+      put4(qp + i, x0, x1, x2, x3);
+      if (ql) put4(ql + i, bf16_rest(x0), bf16_rest(x1), bf16_rest(x2), bf16_rest(x3));
+    };
     if (n % 4 == 0 && a.rot_layout == 1 && half % 4 == 0) {  // a group of four turns with the group half a rotation away
       for (int i = lane * 4; i < n; i += 128) {
         auto in4 = [&](int c) {
@@ -126,7 +131,7 @@ __global__ void __launch_bounds__(256) win_prep_kernel(WinPrepArgs a) {
         if (!is_q) put4(ck + i, x.x, x.y, x.z, x.w);
         else {
           if (qf) put4(qf + i, x.x, x.y, x.z, x.w);
-          if (qp) put4(qp + i, x.x, x.y, x.z, x.w);
+          if (qp) put_q4(i, x.x, x.y, x.z, x.w);
         }
       }
     } else if (n % 4 == 0) {
@@ -135,7 +140,7 @@ __global__ void __launch_bounds__(256) win_prep_kernel(WinPrepArgs a) {
         if (!is_q) put4(ck + i, x0, x1, x2, x3);
         else {
           if (qf) put4(qf + i, x0, x1, x2, x3);
-          if (qp) put4(qp + i, x0, x1, x2, x3);
+          if (qp) put_q4(i, x0, x1, x2, x3);
         }
       }
     } else {
@@ -145,11 +150,15 @@ __global__ void __launch_bounds__(256) win_prep_kernel(WinPrepArgs a) {
         else {
           if (qf) qf[i] = x;
           if (qp) qp[i] = __float2bfloat16_rn(x);
+          if (ql) ql[i] = __float2bfloat16_rn(bf16_rest(x));
         }
       }
     }
     if (is_q && qp)
-      for (int i = n + lane; i < a.q16_ld; i += 32) qp[i] = __float2bfloat16_rn(0.f);
+      for (int i = n + lane; i < a.q16_ld; i += 32) {
+        qp[i] = __float2bfloat16_rn(0.f);
+        if (ql) ql[i] = __float2bfloat16_rn(0.f);
+      }
     __syncwarp();
   }
 }

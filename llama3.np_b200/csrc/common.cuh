@@ -51,6 +51,11 @@ __device__ __forceinline__ float to_f32(bf16 v) { return __bfloat162float(v); }
 template <typename T> __device__ __forceinline__ T from_f32(float v);
 template <> __device__ __forceinline__ float from_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ bf16 from_f32<bf16>(float v) { return __float2bfloat16_rn(v); }
+// what the nearest bf16 leaves of v (16 significant bits with it); 0 for an infinity or NaN, which the first part holds
+__device__ __forceinline__ float bf16_rest(float v) {
+  const float r = v - __bfloat162float(__float2bfloat16_rn(v));
+  return r == r ? r : 0.f;
+}
 
 // Exact split of an fp32 value for the 3xTF32 tensor-core scheme (gemm_tc.cu): hi keeps the
 // sign, exponent and top 10 mantissa bits (a valid TF32 number), lo = v - hi is exact in fp32.

@@ -957,12 +957,32 @@ static bool ll_latent_on_tc(const L3Model* m, const L3LayerSpec& s) {
          latent_tc_supported(s.dim, s.rot_dim, s.vdim, s.kv_rank);
 }
 
-// do prompts of this window-attention mixer run on the tensor cores?  (base: its first column of the output projection's input)
-static bool ll_window_on_tc(const L3Model* m, const LLLayer& U) {
+// Prompts of the softmax mixers with heads of 64 and more in multiples of 8 run on the tensor cores in bf16 mode, where the caches
+// hold bf16 rows (attn_latent_tc.cu); other sizes and fp32 mode keep the FFMA kernels.  The queries of plain-softmax, differential,
+// sigmoid and keep-first attention go there as (high, low) pairs, those of the window kinds without kept tokens as one rounded part.
+// Against the FFMA kernels at width 2048: a three-layer prompt of 2048 tokens with one softmax layer 2720 -> 1991 us, two differential
+// layers over 2000 tokens 2791 -> 1300 us, one sigmoid window layer of three over 3 x 701 tokens 3137 -> 2874 us; the logits' distance
+// from 64-bit ones does not change (2.7e-3, 2.2e-3, 4.9e-3: bf16 operands).  L3_WINDOW_TC=0 turns all of them off.
+static int ll_attn_parts(const L3LayerSpec& s) {
+  return s.mixer != L3_MIX_WINDOW || s.attn_kind == L3_ATTN_SIGMOID || s.keep_first > 0 ? 2 : 1;
+}
+
+static bool ll_attn_on_tc(const L3Model* m, const L3LayerSpec& s, int ld_out) {
   static const bool off = getenv("L3_WINDOW_TC") && atoi(getenv("L3_WINDOW_TC")) == 0;
-  const L3LayerSpec& s = U.spec;
-  return !off && m->tc_ok && s.mixer == L3_MIX_WINDOW && U.ctx_base % 8 == 0 &&
-         win_attn_tc_supported(s.dim, s.vdim, s.attn_kind, s.keep_first, s.scale, U.ctx_ld);
+  return !off && m->tc_ok && win_attn_tc_supported(s.dim, s.mixer == L3_MIX_SOFTMAX ? s.dim : s.vdim, s.scale, ld_out, ll_attn_parts(s));
+}
+
+// (a window mixer writes into its columns of the output projection's input, which start at ctx_base)
+static bool ll_window_on_tc(const L3Model* m, const LLLayer& U) {
+  return U.spec.mixer == L3_MIX_WINDOW && U.ctx_base % 8 == 0 && ll_attn_on_tc(m, U.spec, U.ctx_ld);
+}
+
+static bool ll_softmax_on_tc(const L3Model* m, const L3LayerSpec& s) {
+  return s.mixer == L3_MIX_SOFTMAX && ll_attn_on_tc(m, s, s.heads * s.dim);
+}
+
+static bool ll_diff_on_tc(const L3Model* m, const L3LayerSpec& s) {
+  return s.mixer == L3_MIX_DIFF && ll_attn_on_tc(m, s, 2 * s.heads * s.vdim);
 }
 
 int ll_finalize(L3Model* m) {
@@ -1164,11 +1184,16 @@ int ll_finalize(L3Model* m) {
     CK(m, cudaMalloc(&ll->lat_exp, ll->exp_seqs * per));
     CK(m, cudaMemsetAsync(ll->lat_exp, 0, ll->exp_seqs * per, m->stream));  // never anything but finite numbers
   }
-  size_t wq_ld = 0;
+  size_t wq_ld = 0, maps_ld = 0;
   for (auto& L0 : ll->layers)
-    for (const LLLayer* U = &L0; units && U; U = U->pair)
-      if (ll_window_on_tc(m, *U)) wq_ld = std::max(wq_ld, (size_t)U->spec.heads * latent_tc_q_ld(U->spec.dim, 0));
+    for (const LLLayer* U = &L0; U; U = U->pair) {
+      const L3LayerSpec& s = U->spec;
+      const size_t q_ld = (size_t)s.heads * ll_attn_parts(s) * latent_tc_q_ld(s.dim, 0);
+      if ((units && ll_window_on_tc(m, *U)) || ll_softmax_on_tc(m, s)) wq_ld = std::max(wq_ld, q_ld);
+      if (ll_diff_on_tc(m, s)) { wq_ld = std::max(wq_ld, 2 * q_ld); maps_ld = std::max(maps_ld, (size_t)2 * s.heads * s.vdim); }
+    }
   if (wq_ld && ct > 8) CK(m, cudaMalloc(&ll->win_q16, ct * wq_ld * 2));
+  if (maps_ld && ct > 8) CK(m, cudaMalloc((void**)&ll->diff_maps, ct * maps_ld * 4));
   m->max_split = 32;
   int max_hn = 1, max_hd = 1;
   for (auto& L : ll->layers)
@@ -1228,7 +1253,7 @@ void ll_destroy(L3Model* m) {
   fr(ll->loop_in); fr(ll->embed_norm); fr(ll->final_b); fr(ll->final_alpha); fr(ll->x0); fr(ll->cat); fr(ll->cat16); fr(ll->win_part_o); fr(ll->win_part_ml); fr(ll->xs);
   fr(ll->diff_part_o); fr(ll->diff_part_ml);
   fr(ll->Xs); fr(ll->hn); fr(ll->hf); fr(ll->hf16); fr(ll->y1); fr(ll->y2); fr(ll->moe_gu);
-  fr(ll->lat_q16); fr(ll->win_q16); fr(ll->lat_exp); fr(ll->lat_part_o); fr(ll->lat_part_ml);
+  fr(ll->lat_q16); fr(ll->win_q16); fr(ll->diff_maps); fr(ll->lat_exp); fr(ll->lat_part_o); fr(ll->lat_part_ml);
   if (ll->h_err) cudaFreeHost(ll->h_err);
   fr(ll->loop_step); fr(ll->qlat); fr(ll->aux16); fr(ll->moe_sel); fr(ll->moe_w); fr(ll->moe_dense); fr(ll->moe_idw);
   fr(ll->pin); fr(ll->aux); fr(ll->rk); fr(ll->rv); fr(ll->rg); fr(ll->rbeta); fr(ll->o); fr(ll->sg); fr(ll->sg16); fr(ll->x2); fr(ll->chunk_ws);
@@ -1466,7 +1491,8 @@ static int ll_mix_unit(L3Model* m, LLLayer& Ly, LLState& St, const float* pin, i
     pa.rot_dims = s.rot_dims; pa.rot_layout = s.rot_layout; pa.unit_norm = s.qk_unit; pa.eps = eps;
     pa.bias = Ly.in_bias; pa.wq = Ly.q_norm; pa.wk = Ly.k_norm;
     const bool tc = L > 8 && ll->win_q16 && ll_window_on_tc(m, Ly);
-    pa.q_out = tc ? nullptr : m->q; pa.q16 = tc ? (bf16*)ll->win_q16 : nullptr; pa.q16_ld = latent_tc_q_ld(DK, 0);
+    pa.q_out = tc ? nullptr : m->q; pa.q16 = tc ? (bf16*)ll->win_q16 : nullptr;
+    pa.q16_ld = latent_tc_q_ld(DK, 0); pa.q16_parts = ll_attn_parts(s);
     pa.cache_k = St.ck; pa.cache_v = St.cv; pa.pos_ptr = d_pos;
     pa.L = L; pa.H = H; pa.G = G; pa.DK = DK; pa.DV = DV; pa.M = m->M;
     LAUNCH(m, launch_win_prep(pa, ntok, m->bf16, m->stream));
@@ -1476,7 +1502,7 @@ static int ll_mix_unit(L3Model* m, LLLayer& Ly, LLState& St, const float* pin, i
     at.chunked = s.chunked; at.gate = s.head_gate ? pin + Ly.off_g : nullptr; at.ld_gate = ld;
     at.B = B; at.L = L; at.H = H; at.G = G; at.DK = DK; at.DV = DV; at.M = m->M;
     if (tc) {
-      LAUNCH(m, launch_win_attn_tc(at, pa.q16, m->maxB, ll->h_err, m->stream));
+      LAUNCH(m, launch_win_attn_tc(at, pa.q16, pa.q16_parts, m->maxB, ll->h_err, m->stream));
       return L3_OK;
     }
     at.nsplit = win_attn_splits(B, L, H, G, s.window, s.keep_first, m->M, 32);
@@ -1853,14 +1879,23 @@ static int ll_enqueue_parallel(L3Model* m, int B, int L, float* d_resid) {
     if ((rc = ll_linear(m, Ly.w_in, hm, hm16, 0, ntok, Ly.n_in, W, EPI_STORE, store_to(ll->pin, nullptr, Ly.n_in))) != L3_OK) return rc;
     DiffPrepArgs pa{};
     pa.proj = ll->pin; pa.ld = Ly.n_in; pa.q_off = Ly.off_q; pa.k_off = Ly.off_k; pa.v_off = Ly.off_v; pa.bias = Ly.in_bias;
-    pa.wq = Ly.q_norm; pa.wk = Ly.k_norm; pa.eps = eps; pa.inv_freq = Ly.inv_freq; pa.q_out = m->q; pa.cache_k = St.ck; pa.cache_v = St.cv;
+    pa.wq = Ly.q_norm; pa.wk = Ly.k_norm; pa.eps = eps; pa.inv_freq = Ly.inv_freq; pa.cache_k = St.ck; pa.cache_v = St.cv;
     pa.pos_ptr = d_pos; pa.L = L; pa.H = H; pa.G = G; pa.DK = DK; pa.DV = DV; pa.M = m->M; pa.rot_dims = s.rot_dims;
+    const bool tc = L > 8 && ll->diff_maps && ll_diff_on_tc(m, s);
+    pa.q_out = tc ? nullptr : m->q; pa.q16 = tc ? (bf16*)ll->win_q16 : nullptr; pa.q16_ld = latent_tc_q_ld(DK, 0);
     LAUNCH(m, launch_diff_prep(pa, ntok, m->bf16, m->stream));
     DiffAttnArgs at{};
     at.q = m->q; at.cache_k = St.ck; at.cache_v = St.cv; at.out = m->ctx; at.out16 = (bf16*)m->ctx16; at.lambda = Ly.lambda;
     at.pos_ptr = d_pos; at.scale = s.scale; at.diff = s.diff; at.eps = eps; at.window = s.window;
     at.B = B; at.L = L; at.H = H; at.G = G; at.DK = DK; at.DV = DV; at.M = m->M;
-    LAUNCH(m, launch_diff_attn(at, m->bf16, ll->diff_part_o, ll->diff_part_ml, m->stream));
+    if (tc) {  // the maps as 2 H heads over the key heads' values, then their combination
+      WinAttnArgs wa{};
+      wa.cache_k = St.ck; wa.cache_v = St.cv; wa.out = ll->diff_maps; wa.ld_out = 2 * H * DV; wa.out_scale = 1.f; wa.pos_ptr = d_pos;
+      wa.scale = s.scale; wa.kind = L3_ATTN_SOFTMAX; wa.window = s.window; wa.B = B; wa.L = L; wa.H = 2 * H; wa.G = G; wa.DK = DK; wa.DV = DV; wa.M = m->M;
+      LAUNCH(m, launch_win_attn_tc(wa, pa.q16, 2, m->maxB, ll->h_err, m->stream, 2));
+      if (ll_takes_mirror(m, ntok, W, H * DV)) at.out = nullptr;
+      LAUNCH(m, launch_diff_combine(at, ll->diff_maps, m->stream));
+    } else LAUNCH(m, launch_diff_attn(at, m->bf16, ll->diff_part_o, ll->diff_part_ml, m->stream));
     if ((rc = ll_linear(m, Ly.w_o, m->ctx, m->ctx16, 0, ntok, W, H * DV, EPI_STORE, store_to(ll->y1, nullptr, W))) != L3_OK) return rc;
     if (Ly.ff_total) {
       const int E = s.experts, ff = s.ff, F = Ly.ff_total;
@@ -1960,7 +1995,9 @@ int ll_enqueue_layers(L3Model* m, const int32_t* d_ids, int ids_ld, int ids_off,
     if (s.mixer == L3_MIX_SOFTMAX) {
       QkNormArgs qa{};
       qa.proj = ll->pin; qa.ld = Ly.n_in; qa.k_off = Ly.off_k; qa.wq = Ly.q_norm; qa.wk = Ly.k_norm; qa.eps = eps;
-      qa.q_out = m->q; qa.cache_k = St.ck; qa.cache_v = St.cv; qa.pos_ptr = d_pos;
+      const bool tc = L > 8 && ll->win_q16 && ll_softmax_on_tc(m, s);
+      qa.q_out = tc ? nullptr : m->q; qa.q16 = tc ? (bf16*)ll->win_q16 : nullptr; qa.q16_ld = latent_tc_q_ld(DK, 0);
+      qa.cache_k = St.ck; qa.cache_v = St.cv; qa.pos_ptr = d_pos;
       qa.L = L; qa.HN = H; qa.KVHN = G; qa.HD = DK; qa.M = m->M;
       LAUNCH(m, launch_qk_norm_cache(qa, ntok, m->bf16, m->stream));
       AttnArgs at{};
@@ -1971,7 +2008,13 @@ int ll_enqueue_layers(L3Model* m, const int32_t* d_ids, int ids_ld, int ids_off,
       at.scale = s.scale; at.head_gate = ll->pin + Ly.off_g; at.ld_gate = Ly.n_in;
       at.force_exact = 1;  // scores and softmax weights stay fp32
       at.nsplit = 1;
-      if (!attn_head_dim_supported(DK)) LAUNCH(m, launch_attn_any(at, m->bf16, m->stream));
+      if (tc) {
+        WinAttnArgs wa{};
+        wa.cache_k = St.ck; wa.cache_v = St.cv; wa.out = ll_takes_mirror(m, ntok, W, O) ? nullptr : m->ctx; wa.out16 = (bf16*)m->ctx16; wa.ld_out = O;
+        wa.out_scale = 1.f; wa.gate = at.head_gate; wa.ld_gate = at.ld_gate; wa.pos_ptr = d_pos; wa.scale = s.scale; wa.kind = L3_ATTN_SOFTMAX;
+        wa.B = B; wa.L = L; wa.H = H; wa.G = G; wa.DK = DK; wa.DV = DK; wa.M = m->M;
+        LAUNCH(m, launch_win_attn_tc(wa, qa.q16, 2, m->maxB, ll->h_err, m->stream));
+      } else if (!attn_head_dim_supported(DK)) LAUNCH(m, launch_attn_any(at, m->bf16, m->stream));
       else if (L == 1) {
         at.nsplit = std::max(1, std::min(std::min(m->max_split, m->M / 16), (4 * 148) / std::max(1, B * G)));
         LAUNCH(m, launch_attn_decode(at, m->bf16, m->stream));

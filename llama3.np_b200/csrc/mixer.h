@@ -16,7 +16,9 @@ struct QkNormArgs {
   const float* wq;     // [HN * HD], [KVHN * HD] plain norm weights over the whole projection
   const float* wk;
   float eps;
-  float* q_out;        // [rows, HN * HD] normalised q
+  float* q_out;        // [rows, HN * HD] normalised q, and / or
+  bf16* q16;           // [rows, HN, 2, q16_ld] its (high, low) bf16 parts, zeros behind HD
+  int q16_ld;
   void* cache_k;       // [maxB, KVHN, M, HD]: normalised k
   void* cache_v;       // same shape: k as projected
   const int* pos_ptr;  // device scalar: position of token 0 of every sequence in this call
@@ -184,15 +186,18 @@ struct LatentTcArgs {
   float* out;
   const float* gate;     // sigmoid(gate[r * ld_gate + h]), or with gate_wide + h * vdim + d, multiplies the output (null: none)
   int ld_gate, gate_wide;
-  const float* sink;     // [H] or null
+  const float* sink;     // [H] or null; with `sigmoid` the bias inside it
   const int* pos_ptr;
   float scale;           // > 0
   int* err;              // set to 1 when a wait inside the kernel ran out
   int n_rows, L, H, dim, rot_dim, vdim, kv_rank, M, c_seqs, b0, e_rows, e_seqs;
-  // Set by the launchers.  Where head h of a launch's sequence i finds its keys and values: rows i * seq_rows + (h / rep) *
-  // head_rows + key, columns k_col + (h / rep) * k_cols and v_col + (h / rep) * v_cols of the two tensor maps
-  int rep, seq_rows, head_rows, k_col, k_cols, v_col, v_cols;
-  int window, chunked;   // as WinAttnArgs (window 0: every key up to the query)
+  // Set by the launchers.  Query head h belongs to the value head g = h / maps / rep and the key head g * maps + h % maps (maps 2:
+  // differential attention, two maps over one set of values).  Sequence i's keys are rows i * k_seq_rows + key head * head_rows +
+  // key of their tensor map from column k_col + key head * k_cols on, its values likewise
+  int rep, maps, k_seq_rows, v_seq_rows, head_rows, k_col, k_cols, v_col, v_cols;
+  int window, chunked, keep_first;   // as WinAttnArgs (window 0: every key up to the query)
+  int sigmoid;           // weights sigmoid(score + bias), not normalised
+  int q_parts;           // 2: a packed query is a pair of bf16 parts [high | low] that add up to it, 1: one rounded part
   int ld_out;            // row stride of out / out16
   float out_scale;
 };
@@ -249,7 +254,9 @@ struct DiffPrepArgs {
   const float *wq, *wk;  // [DK] norm weights shared by all heads and maps
   float eps;
   const float* inv_freq; // [rot_dims / 2]
-  float* q_out;          // [rows, H, 2, DK]
+  float* q_out;          // [rows, H, 2, DK], and / or
+  bf16* q16;             // [rows, H, 2, 2, q16_ld] the (high, low) bf16 parts of every map, zeros behind DK
+  int q16_ld;
   void* cache_k;         // [maxB, 2 G, M, DK] of KVT: head g, map m at index 2 g + m
   void* cache_v;         // [maxB, G, M, DV]
   const int* pos_ptr;
@@ -274,6 +281,9 @@ bool diff_attn_supported(int DK, int DV);
 bool diff_attn_tiled(int DK, int DV);
 // floats of split scratch (part_o; part_ml needs a DV-th of it, times 2) for calls of up to max_rows rows of <= 8 tokens per sequence
 size_t diff_attn_part_floats(int max_rows, int H, int DV);
+// The combination alone, behind launch_win_attn_tc with maps 2: maps [rows, H, 2, DV] -> a1 - lambda a2, head norm, multiplier (out,
+// out16, lambda, diff, eps, B, L, H and DV of `a`)
+cudaError_t launch_diff_combine(const DiffAttnArgs& a, const float* maps, cudaStream_t s);
 // part_o / part_ml: scratch of the split decode kernel (null: the decode kernel is not used)
 cudaError_t launch_diff_attn(const DiffAttnArgs& a, bool kv_bf16, float* part_o, float* part_ml, cudaStream_t s);
 
@@ -327,8 +337,8 @@ struct WinPrepArgs {
   const float* bias;     // [columns of proj up to the end of v] added to q, k and v (null: none)
   const float *wq, *wk;  // [DK]: q and k over their root mean square per head, times these, ahead of the rotation (null: none)
   float* q_out;          // [rows, H, DK], and / or
-  bf16* q16;             // [rows, H, q16_ld] with zeros behind DK: the operand of launch_win_attn_tc
-  int q16_ld;
+  bf16* q16;             // [rows, H, q16_parts, q16_ld] with zeros behind DK: the operand of launch_win_attn_tc
+  int q16_ld, q16_parts; // 2 parts: the bf16 value and what it leaves
   void* cache_k;         // [maxB, G, M, DK] of KVT
   void* cache_v;         // [maxB, G, M, DV]
   const int* pos_ptr;
@@ -359,10 +369,11 @@ bool win_attn_supported(int DK, int DV);
 int win_attn_splits(int B, int L, int H, int G, int window, int keep_first, int max_keys, int max_split);
 size_t win_attn_part_floats(int max_rows, int H, int DV, int max_split);
 cudaError_t launch_win_attn(const WinAttnArgs& a, bool kv_bf16, cudaStream_t s);
-// the same softmax attention for prompts in bf16 mode on the tensor cores (attn_latent_tc.cu); no kept first tokens.  q16 [n_seq
-// * L, H, latent_tc_q_ld(DK, 0)] takes the place of WinAttnArgs::q; cache_seqs = sequences the caches hold; err as LatentTcArgs::err
-bool win_attn_tc_supported(int DK, int DV, int kind, int keep_first, float scale, int ld_out);
-cudaError_t launch_win_attn_tc(const WinAttnArgs& a, const bf16* q16, int cache_seqs, int* err, cudaStream_t s);
+// the same attention for prompts in bf16 mode on the tensor cores (attn_latent_tc.cu).  q16 [n_seq * L, H, q_parts,
+// latent_tc_q_ld(DK, 0)] takes the place of WinAttnArgs::q; cache_seqs = sequences the caches hold; err as LatentTcArgs::err.
+// maps 2: differential attention - H, out and q16 count maps (head h, map m at 2 h + m), cache_k has 2 G heads, cache_v G
+bool win_attn_tc_supported(int DK, int DV, float scale, int ld_out, int q_parts);
+cudaError_t launch_win_attn_tc(const WinAttnArgs& a, const bf16* q16, int q_parts, int cache_seqs, int* err, cudaStream_t s, int maps = 1);
 
 // ---- state-space and gated-linear mixers, output stage, small row kernels (hybrid_ops.cu)
 struct SsdPrepArgs {

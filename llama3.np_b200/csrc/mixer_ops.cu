@@ -101,7 +101,26 @@ __global__ void __launch_bounds__(256) qk_norm_cache_kernel(QkNormArgs a) {
   float ss = 0.f;
   for (int i = threadIdx.x; i < nq; i += blockDim.x) { const float v = row[i]; ss = fmaf(v, v, ss); }
   const float rq = 1.0f / sqrtf(block_sum(ss, red) / (float)nq + a.eps);
-  for (int i = threadIdx.x; i < nq; i += blockDim.x) a.q_out[(size_t)r * nq + i] = row[i] * rq * a.wq[i];
+  if (a.q_out)
+    for (int i = threadIdx.x; i < nq; i += blockDim.x) a.q_out[(size_t)r * nq + i] = row[i] * rq * a.wq[i];
+  if (a.q16) {  // operand of the tensor-core kernel: the bf16 value of four entries at a time, then what it leaves
+    const int n4 = a.HN * a.q16_ld / 4;
+    for (int g = threadIdx.x; g < n4; g += blockDim.x) {
+      const int h = g * 4 / a.q16_ld, d = g * 4 - h * a.q16_ld;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (d < a.HD) {  // HD is a multiple of 8
+        const float* src = row + h * a.HD + d;
+        const float* w = a.wq + h * a.HD + d;
+        v = make_float4(src[0] * rq * w[0], src[1] * rq * w[1], src[2] * rq * w[2], src[3] * rq * w[3]);
+      }
+      bf16* dst = a.q16 + ((size_t)r * a.HN + h) * 2 * a.q16_ld + d;
+      union { __nv_bfloat162 b[2]; uint2 u; } hi, lo;
+      hi.b[0] = __floats2bfloat162_rn(v.x, v.y); hi.b[1] = __floats2bfloat162_rn(v.z, v.w);
+      lo.b[0] = __floats2bfloat162_rn(bf16_rest(v.x), bf16_rest(v.y)); lo.b[1] = __floats2bfloat162_rn(bf16_rest(v.z), bf16_rest(v.w));
+      *reinterpret_cast<uint2*>(dst) = hi.u;
+      *reinterpret_cast<uint2*>(dst + a.q16_ld) = lo.u;
+    }
+  }
   const float* krow = row + a.k_off;
   ss = 0.f;
   for (int i = threadIdx.x; i < nk; i += blockDim.x) { const float v = krow[i]; ss = fmaf(v, v, ss); }
