@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(256) ssd_prep_kernel(SsdPrepArgs a) {
 
 __global__ void gla_prep_kernel(const float* __restrict__ q, int ld, float q_mul, const float* __restrict__ z, int ld_z,
                                 const float* __restrict__ bias, float inv_tau, int64_t rows, int n, float* __restrict__ q_out,
-                                float* __restrict__ g_out) {
+                                float* __restrict__ g_out, bool log_decay) {
   pdl_launch();
   pdl_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -70,7 +70,8 @@ __global__ void gla_prep_kernel(const float* __restrict__ q, int ld, float q_mul
   const int c = (int)(i - r * n);
   q_out[i] = q[r * ld + c] * q_mul;
   const float zz = z[r * ld_z + c] + (bias ? bias[c] : 0.f);
-  g_out[i] = expf(-softplus_f(-zz) * inv_tau);  // log sigmoid(z) = -softplus(-z)
+  const float lg = -softplus_f(-zz) * inv_tau;  // log sigmoid(z) = -softplus(-z)
+  g_out[i] = log_decay ? lg : expf(lg);
 }
 
 // wpg warps share a group (wpg in 1, 2, 4, 8); a CTA of 8 warps holds 8 / wpg groups, blockIdx.y walks the groups
@@ -205,10 +206,10 @@ cudaError_t launch_ssd_prep(const SsdPrepArgs& a, int rows, cudaStream_t s) {
 }
 
 cudaError_t launch_gla_prep(const float* q, int ld, float q_mul, const float* z, int ld_z, const float* bias, float tau, int rows,
-                            int n, float* q_out, float* g_out, cudaStream_t s) {
+                            int n, float* q_out, float* g_out, bool log_decay, cudaStream_t s) {
   const int64_t tot = (int64_t)rows * n;
   return launch_k(gla_prep_kernel, dim3((unsigned)((tot + 255) / 256)), dim3(256), 0, s, q, ld, q_mul, z, ld_z, bias, 1.0f / tau,
-                  (int64_t)rows, n, q_out, g_out);
+                  (int64_t)rows, n, q_out, g_out, log_decay);
 }
 
 cudaError_t launch_mix_out(const MixOutArgs& a, int rows, cudaStream_t s) {

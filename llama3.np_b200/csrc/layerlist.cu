@@ -1149,6 +1149,13 @@ int ll_finalize(L3Model* m) {
       if (chunked && recur_chunk_shape(s.dim, s.vdim) && ct >= 128)
         ll->chunk_ws_floats = std::max(ll->chunk_ws_floats, (ct / 64 + m->maxB) * ((size_t)s.heads * s.dim * s.vdim + s.heads + (s.mixer == L3_MIX_MLSTM ? s.heads * s.dim : 0)) + 8);
     }
+  for (const LLLayer& L0 : ll->layers)
+    for (const LLLayer* U = &L0; U; U = U->pair) {  // bf16 mode: recurrences with a decay per key channel (at most 256 MB; long prompts go in segments)
+      const L3LayerSpec& s = U->spec;
+      if (!m->bf16 || (s.mixer != L3_MIX_GATED_DELTA && s.mixer != L3_MIX_GLA) || !recur_channel_shape(s.dim, s.vdim) || ct < RECUR_CHANNEL_MIN) continue;
+      const size_t need = recur_channel_ws_floats(1, (int)ct, s.heads, s.dim, s.vdim) + recur_channel_ws_floats(m->maxB, 1, s.heads, s.dim, s.vdim);
+      ll->chunk_ws_floats = std::max(ll->chunk_ws_floats, std::min(need, (size_t)64 << 20));
+    }
   if (ll->chunk_ws_floats) CK(m, cudaMalloc((void**)&ll->chunk_ws, ll->chunk_ws_floats * 4));
   // tensor cores: bf16 mode only.  fp32 mode is the exact mode of this family: every product is an fp32 FFMA chain
   // (the 3xTF32 scheme of the Llama path would need a (hi, lo) copy of the residual stream beside the stream itself).
@@ -1472,6 +1479,14 @@ static EpiArgs resid_into(float* x, int ld) {
   return e;
 }
 
+// A recurrence with a decay per key channel (ra filled, decays in ll->rg): where its prompt runs on the tensor products, its
+// preparation leaves the decays' logarithms in ll->rg instead.
+static void ll_recur_channels(const L3Model* m, RecurArgs& ra) {
+  ra.bf16_ops = m->tc_ok; ra.ws = m->ll->chunk_ws; ra.ws_floats = m->ll->chunk_ws_floats; ra.log_c = m->ll->rg;
+  if (recur_channel_supported(ra)) ra.g = nullptr;
+  else ra.log_c = nullptr;
+}
+
 // One unit mixer (window attention, state-space, gated linear attention, gated delta rule) of a pre-norm layer: from its
 // columns of the fused input projection (pin, row stride ld) to its columns of the output projection's input (m->ctx, row
 // stride Ly.ctx_ld, already times the mixer's scale).
@@ -1555,8 +1570,9 @@ static int ll_mix_unit(L3Model* m, LLLayer& Ly, LLState& St, const float* pin, i
     const int nd = H * DK;
     float* z = ll->aux;  // [ntok, H * DK] decay logits
     if ((rc = ll_linear(m, Ly.w_a2, pin + Ly.off_a1, nullptr, ld, ntok, nd, s.rank_decay, EPI_STORE, store_to(z, nullptr, nd))) != L3_OK) return rc;
-    LAUNCH(m, launch_gla_prep(pin + Ly.off_q, ld, 1.0f / sqrtf((float)DK), z, nd, Ly.a2_bias, s.tau, ntok, nd, m->q, ll->rg, m->stream));
     ra.mode = 2; ra.q = m->q; ra.ld_q = nd; ra.k = pin + Ly.off_k; ra.ld_k = ld; ra.v = pin + Ly.off_v; ra.ld_v = ld; ra.g = ll->rg; ra.rep = 1;
+    ll_recur_channels(m, ra);
+    LAUNCH(m, launch_gla_prep(pin + Ly.off_q, ld, 1.0f / sqrtf((float)DK), z, nd, Ly.a2_bias, s.tau, ntok, nd, m->q, ll->rg, ra.log_c != nullptr, m->stream));
     LAUNCH(m, launch_recur(ra, m->stream));
     mo.gate = pin + Ly.off_g; mo.ld_gate = ld; mo.gate_act = 1; mo.pre_gate = 0; mo.w = Ly.mix_norm; mo.wlen = DV; mo.group = DV;
   } else {
@@ -1570,10 +1586,12 @@ static int ll_mix_unit(L3Model* m, LLLayer& Ly, LLState& St, const float* pin, i
     pa.conv_w = Ly.conv_w; pa.conv_tail = St.conv_tail; pa.A_log = Ly.A_log; pa.dt_bias = Ly.dt_bias;
     pa.q_out = m->q; pa.k_out = ll->rk; pa.v_out = ll->rv; pa.decay_out = ll->rg; pa.beta_out = ll->rbeta;
     pa.L = L; pa.H = H; pa.G = G; pa.DK = DK; pa.DV = DV; pa.taps = s.conv_taps; pa.update_tail = L == 1;
-    LAUNCH(m, launch_delta_prep(pa, ntok, m->stream));
-    if (s.conv_taps > 1 && L > 1) LAUNCH(m, launch_conv_tail(St.conv_tail, pin, ld, B, L, 2 * nq + O, s.conv_taps - 1, m->stream));
     ra.mode = 1; ra.q = m->q; ra.k = ll->rk; ra.v = ll->rv; ra.ld_q = ra.ld_k = nq; ra.ld_v = O;
     ra.g = ll->rg; ra.beta = ll->rbeta; ra.rep = H / G;
+    ll_recur_channels(m, ra);
+    pa.log_decay = ra.log_c != nullptr;
+    LAUNCH(m, launch_delta_prep(pa, ntok, m->stream));
+    if (s.conv_taps > 1 && L > 1) LAUNCH(m, launch_conv_tail(St.conv_tail, pin, ld, B, L, 2 * nq + O, s.conv_taps - 1, m->stream));
     LAUNCH(m, launch_recur(ra, m->stream));
     mo.gate = og; mo.ld_gate = O; mo.gate_act = 0; mo.pre_gate = 0; mo.w = Ly.mix_norm; mo.wlen = DV; mo.group = DV;
   }
@@ -2038,12 +2056,14 @@ int ll_enqueue_layers(L3Model* m, const int32_t* d_ids, int ids_ld, int ids_off,
       pa.conv_w = Ly.conv_w; pa.conv_tail = St.conv_tail; pa.A_log = Ly.A_log; pa.dt_bias = Ly.dt_bias;
       pa.q_out = m->q; pa.k_out = ll->rk; pa.v_out = ll->rv; pa.decay_out = ll->rg; pa.beta_out = ll->rbeta;
       pa.L = L; pa.H = H; pa.G = G; pa.DK = DK; pa.DV = DV; pa.taps = s.conv_taps;
-      LAUNCH(m, launch_delta_prep(pa, ntok, m->stream));
-      if (s.conv_taps > 1) LAUNCH(m, launch_conv_tail(St.conv_tail, ll->pin, Ly.n_in, B, L, 2 * nq + O, s.conv_taps - 1, m->stream));
       RecurArgs ra{};
       ra.mode = 1; ra.q = m->q; ra.k = ll->rk; ra.v = ll->rv; ra.ld_q = ra.ld_k = nq; ra.ld_v = O;
       ra.g = ll->rg; ra.beta = ll->rbeta; ra.state = St.S; ra.out = ll->o;
       ra.B = B; ra.L = L; ra.H = H; ra.rep = H / G; ra.DK = DK; ra.DV = DV;
+      ll_recur_channels(m, ra);
+      pa.log_decay = ra.log_c != nullptr;
+      LAUNCH(m, launch_delta_prep(pa, ntok, m->stream));
+      if (s.conv_taps > 1) LAUNCH(m, launch_conv_tail(St.conv_tail, ll->pin, Ly.n_in, B, L, 2 * nq + O, s.conv_taps - 1, m->stream));
       LAUNCH(m, launch_recur(ra, m->stream));
       LAUNCH(m, launch_gated_rmsnorm(ll->o, og, O, Ly.mix_norm, DV, DV, eps, ntok, O, m->ctx, (bf16*)m->ctx16, m->stream));
     }

@@ -42,7 +42,8 @@ struct DeltaPrepArgs {
   const float* dt_bias;   // [H * DK]
   float *q_out, *k_out;   // [rows, G * DK]
   float* v_out;           // [rows, H * DV]
-  float* decay_out;       // [rows, H * DK]
+  float* decay_out;       // [rows, H * DK] the decays, or with log_decay their natural logarithms
+  int log_decay;
   float* beta_out;        // [rows, H]
   int L, H, G, DK, DV, taps;
   int update_tail;        // L == 1 only: the kernel also moves conv_tail on by this token (no launch_conv_tail afterwards)
@@ -68,6 +69,8 @@ struct RecurArgs {
   int g_head;
   const float* log_g;     // mode 2 with g_head, may be null: [B * L, H] the decays' natural logarithms (finite); with it and
                           // `ws`, prompts of the common shapes run in the chunk-parallel form
+  const float* log_c;     // mode 1, 2 without g_head, may be null: [B * L, H * DK] the decays' natural logarithms; only where
+                          // recur_channel_supported says that a call runs there (g is then not read)
   const float* beta;      // mode 1: [B * L, H]
   float* state;           // [maxB, H, DK, DV]
   float* out;             // [B * L, H * DV]
@@ -77,7 +80,8 @@ struct RecurArgs {
   float q_mul;            // multiplies the queries (0: 1)
   float* n_state;         // [maxB, H, DK] a running sum of the keys with the state's own decay (the normaliser of an mLSTM) ...
   float* nq;              // ... and its product with the query, [B * L, H]
-  int bf16_ops;           // with n_state, chunk-parallel form: q, k and v may be rounded to bf16 (they are bf16 projections' outputs)
+  int bf16_ops;           // bf16 mode.  With n_state, chunk-parallel form: q, k and v may be rounded to bf16 (they are bf16 projections'
+                          // outputs).  Without: prompts may run on tensor products of (hi, lo) pairs (recur_channel.cu)
   float* ws;              // mode 0, may be null: room for one state matrix per (sequence, head, chunk of 64 tokens);
   size_t ws_floats;       // with it, prompts of the common shapes run in the chunk-parallel form (recur_chunk.cu)
 };
@@ -88,6 +92,13 @@ size_t recur_chunk_ws_floats(int B, int L, int H, int DK, int DV);
 bool recur_chunk_shape(int DK, int DV);
 bool recur_chunk_supported(const RecurArgs& a);
 cudaError_t launch_recur_chunk(const RecurArgs& a, cudaStream_t s);
+
+// chunk-parallel form on tensor products (recur_channel.cu), decays per key channel or per head; workspace `ws`, in segments where it is small
+constexpr int RECUR_CHANNEL_MIN = 48;  // tokens
+bool recur_channel_shape(int DK, int DV);
+size_t recur_channel_ws_floats(int B, int L, int H, int DK, int DV);
+bool recur_channel_supported(const RecurArgs& a);
+cudaError_t launch_recur_channel(const RecurArgs& a, cudaStream_t s);
 
 // ---- attention for head sizes the tiled kernels do not take (attn_any.cu): same arguments, any HD
 cudaError_t launch_attn_any(const AttnArgs& a, bool kv_bf16, cudaStream_t s);
@@ -393,9 +404,9 @@ struct SsdPrepArgs {
   int update_tail;        // L == 1 only: the kernel also moves conv_tail on by this token (no launch_conv_tail afterwards)
 };
 cudaError_t launch_ssd_prep(const SsdPrepArgs& a, int rows, cudaStream_t s);
-// q_out[r, i] = q[r * ld + i] * q_mul;  g_out[r, i] = sigmoid(z[r * ld_z + i] + bias[i])^(1 / tau)   (i < n)
+// q_out[r, i] = q[r * ld + i] * q_mul;  g_out[r, i] = sigmoid(z[r * ld_z + i] + bias[i])^(1 / tau), or its logarithm   (i < n)
 cudaError_t launch_gla_prep(const float* q, int ld, float q_mul, const float* z, int ld_z, const float* bias, float tau, int rows,
-                            int n, float* q_out, float* g_out, cudaStream_t s);
+                            int n, float* q_out, float* g_out, bool log_decay, cudaStream_t s);
 // Output stage of a recurrent mixer, a CTA per row of n = H * DV values:
 //   y = o + skip_d[i / DV] * skip_x[r, i]                       (skip_d null: y = o)
 //   pre_gate 1:  y <- y * act(gate), then out = y / rms_group(y) * w[i % wlen]

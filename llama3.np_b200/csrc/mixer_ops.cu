@@ -195,7 +195,8 @@ __global__ void __launch_bounds__(256) delta_prep_kernel(DeltaPrepArgs a) {
       const float rate = expf(a.A_log[h]);
       for (int i = lane; i < a.DK; i += 32) {
         const int c = h * a.DK + i;
-        a.decay_out[(size_t)r * a.H * a.DK + c] = expf(-rate * softplus_f(a.dt_in[(size_t)r * a.ld_dt + c] + a.dt_bias[c]));
+        const float lg = -rate * softplus_f(a.dt_in[(size_t)r * a.ld_dt + c] + a.dt_bias[c]);
+        a.decay_out[(size_t)r * a.H * a.DK + c] = a.log_decay ? lg : expf(lg);
       }
     } else {
       for (int h = lane; h < a.H; h += 32) a.beta_out[(size_t)r * a.H + h] = sigmoid_f(a.proj[(size_t)r * a.ld + a.beta_off + h]);

@@ -1,0 +1,508 @@
+// Chunk-parallel form of the linear recurrences on warp-level tensor products, for prompts in bf16 mode: the gated delta rule and
+// gated linear attention, whose decay is a number per key channel and token, and the fixed-decay and state-space recurrences,
+// whose decay is one number per head (RecurArgs modes 0, 1 and 2).
+//
+//   S_t = diag(g_t) S_(t-1) + k_t u_t^T,   o_t = S_t^T q_t,   u_t = v_t, or with the delta rule beta_t (v_t - (diag(g_t) S_(t-1))^T k_t)
+//
+// With c_t the running sum of log g inside a chunk of 64 tokens that starts from the state P:
+//   o_t = P^T (q_t e^(c_t)) + sum_{j <= t} B_tj u_j,   B_tj = sum_d q_t k_j e^(c_t - c_j)       (d: key channels)
+//   the chunk leaves  diag(e^(c_C)) P + sum_j (k_j e^(c_C - c_j)) u_j^T
+//   delta rule:  (I + diag(beta) A) U = diag(beta) (V - (K e^c) P),   A_tj = sum_d k_t k_j e^(c_t - c_j) for j < t,
+//   so  U = U' - W P  with  T = (I + diag(beta) A)^-1,  U' = T diag(beta) V,  W = T diag(beta) (K e^c)
+//  1. channel_chunk_kernel  a CTA per (chunk, head, sequence), none waits for another: B, A, T, W, U', the decayed queries and keys,
+//                           written to the workspace in the order in which the lanes of kernel 2 read them as MMA operands
+//  2. channel_chain_kernel  a CTA per (16 value columns, head, sequence) walks the chunks: S^T (16 x DK) stays in fp32 accumulator
+//                           registers - a warp owns 16 key channels -, which are the left operand of the next product without a
+//                           move.  Per chunk two products against S (W and the decayed queries), a sum over the warps through shared
+//                           memory, then the state's and the outputs' products with U; operand blocks are fetched a phase ahead.
+// Every exponential has an argument <= 0: c is kept relative to blocks of 16 tokens, products between blocks take a reference
+// between them (e^(c_t - ref) e^(ref - c_j)), 8 x 8 blocks on the diagonal are formed pair by pair.  All operands of the tensor
+// products - keys, queries, scores, T, U and the state - are pairs hi + lo of bf16 values (16 significant bits), a product is
+// hi hi + hi lo + lo hi with fp32 accumulation; the inverse is fp32.
+#include <stdint.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "mixer.h"
+
+namespace {
+
+constexpr int CT = 64;   // tokens per chunk
+
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&t);
+}
+// (a, b) as bf16 pairs: hi + lo = value up to 2^-17 of it
+__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
+  hi = pack2(a, b);
+  lo = pack2(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
+}
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// c += (ah + al) (b.hi + b.lo); b = (hi b0, hi b1, lo b0, lo b1)
+__device__ __forceinline__ void mma3(float (&c)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4], const uint4& b) {
+  mma16816(c, ah, b.x, b.y);
+  mma16816(c, al, b.x, b.y);
+  mma16816(c, ah, b.z, b.w);
+}
+__device__ __forceinline__ float act_silu(int act_in, float x) {
+  return act_in == 0 ? x : act_in == 2 ? __fdividef(x, 1.0f + __expf(-x)) : silu_ref(x);
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// One (chunk, head, sequence) of the workspace, in 16-byte units: operand blocks W and decayed queries [token tile 8][k step DK / 16]
+// [lane], decayed keys [channel tile DK / 8][k step 4][lane], B [token tile 8][k step 4][lane], then e^(c_C) and U' as floats
+template <int DK> struct Ws {
+  static constexpr int W = 8 * (DK / 16) * 32, Q = W, K = (DK / 8) * 4 * 32, B = 8 * 4 * 32, E = DK / 4;
+  static constexpr int oQ = W, oK = oQ + Q, oB = oK + K, oE = oB + B, oU = oE + E;
+  __host__ __device__ static size_t total(int DV, bool delta) { return (size_t)oU + (delta ? (size_t)CT * DV / 4 : 0); }
+};
+
+// ---------------------------------------------------------------------------------------------- 1. what a chunk needs by itself
+template <int DK, bool DELTA>
+__global__ void __launch_bounds__(512) channel_chunk_kernel(RecurArgs a, int c0) {
+  extern __shared__ __align__(16) float sm[];
+  constexpr int LD = DK + 8, LDA = CT + 4;
+  float* qf = sm;                       // [CT][LD]
+  float* kf = qf + CT * LD;
+  float* lf = kf + CT * LD;             // running log decay inside a block of 16 tokens, token included
+  float* Bm = lf + CT * LD;             // [CT][LDA]
+  float* tot = Bm + CT * LDA;           // [4][DK] the blocks' totals
+  float* Am = tot + 4 * DK;             // [CT][LDA] diag(beta) A, strictly lower (delta rule, as what follows)
+  float* Tm = Am + CT * LDA;            // [CT][LDA]
+  float* tmp = Tm + CT * LDA;           // [3][16][17]
+  float* beta = tmp + 3 * 16 * 17;      // [CT]
+  pdl_launch();
+  pdl_wait();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q2 = (lane & 3) * 2;
+  const int c = c0 + blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int n = min(CT, a.L - c * CT);
+  const size_t row0 = (size_t)b * a.L + (size_t)c * CT;
+  {
+    const float q_mul = a.q_mul != 0.f ? a.q_mul : 1.f;
+    const float* qs = a.q + row0 * a.ld_q + (size_t)(h / a.rep) * DK;
+    const float* ks = a.k + row0 * a.ld_k + (size_t)(h / a.rep) * DK;
+    const float fixed = a.log_c || a.log_g ? 0.f : logf(a.head_decay[h]);
+    for (int i = tid; i < CT * DK / 4; i += 512) {
+      const int t = i / (DK / 4), d = (i % (DK / 4)) * 4;
+      float4 qv = make_float4(0.f, 0.f, 0.f, 0.f), kv = qv, lv = qv;
+      if (t < n) {
+        qv = *reinterpret_cast<const float4*>(qs + (size_t)t * a.ld_q + d);
+        kv = *reinterpret_cast<const float4*>(ks + (size_t)t * a.ld_k + d);
+        if (a.log_c) lv = *reinterpret_cast<const float4*>(a.log_c + (row0 + t) * a.H * DK + (size_t)h * DK + d);
+        else { const float l = a.log_g ? a.log_g[(row0 + t) * a.H + h] : fixed; lv = make_float4(l, l, l, l); }
+        // a decay of zero: far below every exponential, but finite
+        lv.x = lv.x < -1e30f ? -1e30f : lv.x; lv.y = lv.y < -1e30f ? -1e30f : lv.y; lv.z = lv.z < -1e30f ? -1e30f : lv.z; lv.w = lv.w < -1e30f ? -1e30f : lv.w;
+        if (a.act_in) {
+          qv.x = act_silu(a.act_in, qv.x); qv.y = act_silu(a.act_in, qv.y); qv.z = act_silu(a.act_in, qv.z); qv.w = act_silu(a.act_in, qv.w);
+          kv.x = act_silu(a.act_in, kv.x); kv.y = act_silu(a.act_in, kv.y); kv.z = act_silu(a.act_in, kv.z); kv.w = act_silu(a.act_in, kv.w);
+        }
+        qv.x *= q_mul; qv.y *= q_mul; qv.z *= q_mul; qv.w *= q_mul;
+      }
+      *reinterpret_cast<float4*>(qf + t * LD + d) = qv;
+      *reinterpret_cast<float4*>(kf + t * LD + d) = kv;
+      *reinterpret_cast<float4*>(lf + t * LD + d) = lv;
+    }
+    if (DELTA && tid < CT) beta[tid] = tid < n ? a.beta[(row0 + tid) * a.H + h] : 0.f;
+    for (int i = tid; i < CT * LDA; i += 512) { Bm[i] = 0.f; if (DELTA) Am[i] = 0.f; }
+  }
+  __syncthreads();
+  for (int i = tid; i < 4 * DK; i += 512) {
+    const int blk = i / DK, d = i % DK;
+    float s = 0.f;
+#pragma unroll
+    for (int r = 0; r < 16; ++r) { s += lf[(blk * 16 + r) * LD + d]; lf[(blk * 16 + r) * LD + d] = s; }
+    tot[i] = s;
+  }
+  __syncthreads();
+  // ---- A and B between blocks of 16, and between the halves of a block: one 16 x 16 (16 x 8) tile per warp
+  {
+    // warps 0 - 5: queries of block I against keys of block J < I; 6 - 11: keys likewise (delta); 12 - 15: second half of a block
+    const bool mid = warp >= 12;
+    const int pr = warp % 6;
+    const int I = mid ? warp - 12 : pr < 1 ? 1 : pr < 3 ? 2 : 3, J = mid ? I : pr < 1 ? 0 : pr < 3 ? pr - 1 : pr - 3;
+    if (mid || warp < 6 || DELTA) {
+      const float* xa = mid ? kf : warp < 6 ? qf : kf;   // rows 0 - 7 of the tile
+      const float* xb = mid ? qf : xa;                   // rows 8 - 15
+      const int ta = mid ? 16 * I + 8 + g : 16 * I + g, tb = mid ? ta : ta + 8;
+      const int j0 = 16 * J;
+      float acc[2][4] = {};
+#pragma unroll 2
+      for (int k0 = 0; k0 < DK; k0 += 16) {
+        uint32_t ah[4], al[4];
+        uint4 bb[2];
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          const int d = k0 + q2 + 8 * s;
+          // the reference between rows and columns: the start of block I, or the token ahead of its second half
+          float2 ref = mid ? *reinterpret_cast<const float2*>(lf + (16 * I + 7) * LD + d) : make_float2(0.f, 0.f);
+          const float2 va = *reinterpret_cast<const float2*>(xa + ta * LD + d), la = *reinterpret_cast<const float2*>(lf + ta * LD + d);
+          const float2 vb = *reinterpret_cast<const float2*>(xb + tb * LD + d), lb = *reinterpret_cast<const float2*>(lf + tb * LD + d);
+          split2(va.x * __expf(la.x - ref.x), va.y * __expf(la.y - ref.y), ah[2 * s], al[2 * s]);
+          split2(vb.x * __expf(lb.x - ref.x), vb.y * __expf(lb.y - ref.y), ah[2 * s + 1], al[2 * s + 1]);
+          if (!mid) {  // decay from the end of token j to the start of block I
+            ref = make_float2(0.f, 0.f);
+            for (int m = J; m < I; ++m) { const float2 t = *reinterpret_cast<const float2*>(tot + m * DK + d); ref.x += t.x; ref.y += t.y; }
+          }
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) {
+            if (mid && nt) continue;
+            const int j = j0 + nt * 8 + g;
+            const float2 kv = *reinterpret_cast<const float2*>(kf + j * LD + d), lj = *reinterpret_cast<const float2*>(lf + j * LD + d);
+            uint32_t hi, lo;
+            split2(kv.x * __expf(ref.x - lj.x), kv.y * __expf(ref.y - lj.y), hi, lo);
+            if (s) { bb[nt].y = hi; bb[nt].w = lo; } else { bb[nt].x = hi; bb[nt].z = lo; }
+          }
+        }
+        mma3(acc[0], ah, al, bb[0]);
+        if (!mid) mma3(acc[1], ah, al, bb[1]);
+      }
+      float* outa = mid || warp >= 6 ? Am : Bm;
+      float* outb = !mid && warp >= 6 ? Am : Bm;
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        if (mid && nt) continue;
+        const int j = j0 + nt * 8 + q2;
+        if (outa == Bm || DELTA) {
+          const float f = outa == Bm ? 1.f : beta[ta];
+          *reinterpret_cast<float2*>(outa + ta * LDA + j) = make_float2(acc[nt][0] * f, acc[nt][1] * f);
+        }
+        const float f = outb == Bm ? 1.f : beta[tb];
+        *reinterpret_cast<float2*>(outb + tb * LDA + j) = make_float2(acc[nt][2] * f, acc[nt][3] * f);
+      }
+    }
+  }
+  // ---- the 8 x 8 blocks on the diagonal, pair by pair: lane = (token, one of four keys)
+  {
+    const int t = (warp >> 1) * 8 + g, j = (warp >> 1) * 8 + (warp & 1) * 4 + (lane & 3);
+    float sa = 0.f, sb = 0.f;
+#pragma unroll 4
+    for (int d = 0; d < DK; d += 4) {
+      const float4 lt = *reinterpret_cast<const float4*>(lf + t * LD + d), lj = *reinterpret_cast<const float4*>(lf + j * LD + d);
+      const float4 kj = *reinterpret_cast<const float4*>(kf + j * LD + d), qt = *reinterpret_cast<const float4*>(qf + t * LD + d);
+      const float ex = kj.x * __expf(lt.x - lj.x), ey = kj.y * __expf(lt.y - lj.y), ez = kj.z * __expf(lt.z - lj.z), ew = kj.w * __expf(lt.w - lj.w);
+      sb = fmaf(qt.x, ex, sb); sb = fmaf(qt.y, ey, sb); sb = fmaf(qt.z, ez, sb); sb = fmaf(qt.w, ew, sb);
+      if (DELTA) {
+        const float4 kt = *reinterpret_cast<const float4*>(kf + t * LD + d);
+        sa = fmaf(kt.x, ex, sa); sa = fmaf(kt.y, ey, sa); sa = fmaf(kt.z, ez, sa); sa = fmaf(kt.w, ew, sa);
+      }
+    }
+    if (j <= t) Bm[t * LDA + j] = sb;                    // a key behind the query has a positive exponent: never stored
+    if (DELTA && j < t) Am[t * LDA + j] = sa * beta[t];
+  }
+  __syncthreads();
+  // ---- operands of the chain kernel
+  using Wk = Ws<DK>;
+  uint4* ws = reinterpret_cast<uint4*>(a.ws) + ((size_t)(b * a.H + h) * gridDim.x + blockIdx.x) * Wk::total(a.DV, DELTA);
+  auto before = [&](int blk, int d) { float s = 0.f; for (int m = 0; m < blk; ++m) s += tot[m * DK + d]; return s; };
+  for (int i = tid; i < Wk::Q; i += 512) {               // decayed queries: (token, channel pair)
+    const int l = i & 31, ks = (i >> 5) % (DK / 16), nt = (i >> 5) / (DK / 16), t = nt * 8 + (l >> 2), d = ks * 16 + (l & 3) * 2, blk = t >> 4;
+    uint4 o;
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const int e = d + 8 * s;
+      const float x = qf[t * LD + e] * __expf(lf[t * LD + e] + before(blk, e));
+      const float y = qf[t * LD + e + 1] * __expf(lf[t * LD + e + 1] + before(blk, e + 1));
+      if (s) split2(x, y, o.y, o.w); else split2(x, y, o.x, o.z);
+    }
+    ws[Wk::oQ + i] = o;
+  }
+  for (int i = tid; i < Wk::K; i += 512) {               // decayed keys: (channel, token pair)
+    const int l = i & 31, ks = (i >> 5) & 3, nt = i >> 7, d = nt * 8 + (l >> 2), t = ks * 16 + (l & 3) * 2;
+    float rest = tot[ks * DK + d];                       // from the start of the block to the end of the chunk
+    for (int m = ks + 1; m < 4; ++m) rest += tot[m * DK + d];
+    uint4 o;
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const int u = t + 8 * s;
+      const float x = kf[u * LD + d] * __expf(rest - lf[u * LD + d]), y = kf[(u + 1) * LD + d] * __expf(rest - lf[(u + 1) * LD + d]);
+      if (s) split2(x, y, o.y, o.w); else split2(x, y, o.x, o.z);
+    }
+    ws[Wk::oK + i] = o;
+  }
+  for (int i = tid; i < Wk::B; i += 512) {
+    const int l = i & 31, ks = (i >> 5) & 3, nt = i >> 7;
+    const float* p = Bm + (nt * 8 + (l >> 2)) * LDA + ks * 16 + (l & 3) * 2;
+    uint4 o;
+    split2(p[0], p[1], o.x, o.z);
+    split2(p[8], p[9], o.y, o.w);
+    ws[Wk::oB + i] = o;
+  }
+  for (int d = tid; d < DK; d += 512) reinterpret_cast<float*>(ws + Wk::oE)[d] = __expf(before(4, d));
+  if constexpr (DELTA) {
+    // ---- T = (I + Am)^-1, blocks of 16: the diagonal ones column by column, then by distance from the diagonal
+    if (tid < CT) {
+      const int blk = tid >> 4, cc = tid & 15;
+      const float* Ld = Am + (blk * 16) * LDA + blk * 16;
+      float x[16];
+#pragma unroll
+      for (int r = 0; r < 16; ++r) {
+        float s = 0.f;
+#pragma unroll
+        for (int m = 0; m < r; ++m) s = fmaf(Ld[r * LDA + m], x[m], s);
+        x[r] = r == cc ? 1.f : r < cc ? 0.f : -s;
+        Tm[(blk * 16 + r) * LDA + blk * 16 + cc] = x[r];
+      }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int dist = 1; dist < 4; ++dist) {
+      const int items = (4 - dist) * 256;
+      for (int i = tid; i < items; i += 512) {           // sum_m L_Im T_mJ
+        const int J = i >> 8, I = J + dist, r = (i >> 4) & 15, cc = i & 15;
+        float s = 0.f;
+        for (int m = J * 16; m < I * 16; ++m) s = fmaf(Am[(I * 16 + r) * LDA + m], Tm[m * LDA + J * 16 + cc], s);
+        tmp[J * 272 + r * 17 + cc] = s;
+      }
+      __syncthreads();
+      for (int i = tid; i < items; i += 512) {
+        const int J = i >> 8, I = J + dist, r = (i >> 4) & 15, cc = i & 15;
+        float s = 0.f;
+#pragma unroll
+        for (int m = 0; m < 16; ++m) s = fmaf(Tm[(I * 16 + r) * LDA + I * 16 + m], tmp[J * 272 + m * 17 + cc], s);
+        Tm[(I * 16 + r) * LDA + J * 16 + cc] = -s;
+      }
+      __syncthreads();
+    }
+    // ---- W and U': 16 columns of [K e^c | V] per warp and turn
+    const int n_w = DK / 16, n_all = n_w + a.DV / 16;
+    float* up = reinterpret_cast<float*>(ws + Wk::oU);
+    for (int ct = warp; ct < n_all; ct += 16) {
+      const bool is_w = ct < n_w;
+      const int col0 = is_w ? ct * 16 : (ct - n_w) * 16;
+      float acc[4][2][4] = {};
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) {
+        uint4 bb[2];
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          const int col = col0 + nt * 8 + g;
+          float v[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int t = ks * 16 + q2 + (u & 1) + (u >> 1) * 8;
+            if (is_w) v[u] = beta[t] * kf[t * LD + col] * __expf(lf[t * LD + col] + before(ks, col));
+            else v[u] = t < n ? beta[t] * a.v[(row0 + t) * a.ld_v + (size_t)h * a.DV + col] : 0.f;
+          }
+          split2(v[0], v[1], bb[nt].x, bb[nt].z);
+          split2(v[2], v[3], bb[nt].y, bb[nt].w);
+        }
+#pragma unroll
+        for (int mt = ks; mt < 4; ++mt) {
+          uint32_t ah[4], al[4];
+          const float* p = Tm + (mt * 16 + g) * LDA + ks * 16 + q2;
+          const float2 t0 = *reinterpret_cast<const float2*>(p), t1 = *reinterpret_cast<const float2*>(p + 8 * LDA);
+          const float2 t2 = *reinterpret_cast<const float2*>(p + 8), t3 = *reinterpret_cast<const float2*>(p + 8 * LDA + 8);
+          split2(t0.x, t0.y, ah[0], al[0]); split2(t1.x, t1.y, ah[1], al[1]);
+          split2(t2.x, t2.y, ah[2], al[2]); split2(t3.x, t3.y, ah[3], al[3]);
+          mma3(acc[mt][0], ah, al, bb[0]);
+          mma3(acc[mt][1], ah, al, bb[1]);
+        }
+      }
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {                    // tokens mt * 16 + g (+ 8): token tile 2 mt + u
+          if (is_w) {                                    // accumulator and operand layouts agree lane by lane
+            uint4 o;
+            split2(acc[mt][0][2 * u], acc[mt][0][2 * u + 1], o.x, o.z);
+            split2(acc[mt][1][2 * u], acc[mt][1][2 * u + 1], o.y, o.w);
+            ws[((2 * mt + u) * n_w + ct) * 32 + lane] = o;
+          } else {
+            float* p = up + (size_t)(mt * 16 + u * 8 + g) * a.DV + col0 + q2;
+            *reinterpret_cast<float2*>(p) = make_float2(acc[mt][0][2 * u], acc[mt][0][2 * u + 1]);
+            *reinterpret_cast<float2*>(p + 8) = make_float2(acc[mt][1][2 * u], acc[mt][1][2 * u + 1]);
+          }
+        }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------- 2. the chain over the chunks
+// grid (DV / 16, H, B); DK / 16 warps, warp w owns key channels 16 w .. 16 w + 15 of S^T and the token tiles w, w + DK / 16, ..
+template <int DK, bool DELTA>
+__global__ void __launch_bounds__(DK * 2, 1) channel_chain_kernel(RecurArgs a, int c0, int NC) {
+  extern __shared__ __align__(16) uint4 sm4[];
+  using Wk = Ws<DK>;
+  constexpr int NW = DK / 16, TH = DK * 2, TPW = 8 / NW;
+  uint4* sW = sm4;                                       // W (delta) and decayed queries
+  uint4* sQ = sW + (DELTA ? Wk::W : 0);
+  uint4* sK = sQ + Wk::Q;                                // decayed keys
+  uint4* sB = sK + Wk::K;
+  float4* exU = reinterpret_cast<float4*>(sB + Wk::B);   // [warp][token tile][lane] partial products with S
+  float4* exO = exU + (DELTA ? NW * 256 : 0);
+  uint4* sU = reinterpret_cast<uint4*>(exO + NW * 256);  // U^T as left operand: [k step 4][hi, lo][lane]
+  pdl_launch();
+  pdl_wait();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q2 = (lane & 3) * 2;
+  const int e0 = blockIdx.x * 16, h = blockIdx.y, b = blockIdx.z;
+  const size_t per = Wk::total(a.DV, DELTA);
+  const uint4* ws = reinterpret_cast<const uint4*>(a.ws) + (size_t)(b * a.H + h) * NC * per;
+  const int O = a.H * a.DV;
+  float* st = a.state + ((size_t)b * a.H + h) * DK * a.DV + e0;
+  float sacc[2][4];                                      // S^T: value column g (+ 8), channel 16 warp + 8 t + q2 (+ 1)
+#pragma unroll
+  for (int t = 0; t < 2; ++t)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) sacc[t][u] = st[(size_t)(warp * 16 + t * 8 + q2 + (u & 1)) * a.DV + g + (u >> 1) * 8];
+  auto fetch_wq = [&](int c) {
+    if (c < NC) {
+      const uint4* src = ws + (size_t)c * per + (DELTA ? 0 : Wk::oQ);
+      for (int i = tid; i < (DELTA ? Wk::W : 0) + Wk::Q; i += TH) cp_async16(sW + i, src + i);
+    }
+    cp_commit();
+  };
+  auto fetch_kb = [&](int c) {
+    if (c < NC) {
+      const uint4* src = ws + (size_t)c * per + Wk::oK;
+      for (int i = tid; i < Wk::K + Wk::B; i += TH) cp_async16(sK + i, src + i);
+    }
+    cp_commit();
+  };
+  fetch_wq(0);
+  fetch_kb(0);
+#pragma unroll 1
+  for (int c = 0; c < NC; ++c) {
+    const int n = min(CT, a.L - (c0 + c) * CT);
+    const size_t row0 = (size_t)b * a.L + (size_t)(c0 + c) * CT;
+    // what this lane needs of U' or V (value columns g, g + 8; tokens q2, q2 + 1 of its tiles) and the chunk's decays
+    float uv[TPW][4], ec[2][2];
+#pragma unroll
+    for (int p = 0; p < TPW; ++p)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int t = (warp + p * NW) * 8 + q2 + (u & 1), e = e0 + g + (u >> 1) * 8;
+        if (DELTA) uv[p][u] = reinterpret_cast<const float*>(ws + (size_t)c * per + Wk::oU)[(size_t)t * a.DV + e];
+        else uv[p][u] = t < n ? a.v[(row0 + t) * a.ld_v + (size_t)h * a.DV + e] : 0.f;
+      }
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const float2 v = *reinterpret_cast<const float2*>(reinterpret_cast<const float*>(ws + (size_t)c * per + Wk::oE) + warp * 16 + t * 8 + q2);
+      ec[t][0] = v.x; ec[t][1] = v.y;
+    }
+    cp_wait<1>();
+    __syncthreads();
+    {
+      uint32_t ah[4], al[4];
+      split2(sacc[0][0], sacc[0][1], ah[0], al[0]); split2(sacc[0][2], sacc[0][3], ah[1], al[1]);
+      split2(sacc[1][0], sacc[1][1], ah[2], al[2]); split2(sacc[1][2], sacc[1][3], ah[3], al[3]);
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt) {
+        if (DELTA) {
+          float p[4] = {};
+          mma3(p, ah, al, sW[(nt * NW + warp) * 32 + lane]);
+          exU[(warp * 8 + nt) * 32 + lane] = make_float4(p[0], p[1], p[2], p[3]);
+        }
+        float p[4] = {};
+        mma3(p, ah, al, sQ[(nt * NW + warp) * 32 + lane]);
+        exO[(warp * 8 + nt) * 32 + lane] = make_float4(p[0], p[1], p[2], p[3]);
+      }
+    }
+    __syncthreads();
+    fetch_wq(c + 1);
+    float o[TPW][4];
+#pragma unroll
+    for (int p = 0; p < TPW; ++p) {
+      const int nt = warp + p * NW;
+      float4 so = make_float4(0.f, 0.f, 0.f, 0.f), su = so;
+#pragma unroll
+      for (int w = 0; w < NW; ++w) {
+        const float4 x = exO[(w * 8 + nt) * 32 + lane];
+        so.x += x.x; so.y += x.y; so.z += x.z; so.w += x.w;
+        if (DELTA) {
+          const float4 y = exU[(w * 8 + nt) * 32 + lane];
+          su.x += y.x; su.y += y.y; su.z += y.z; su.w += y.w;
+        }
+      }
+      o[p][0] = so.x; o[p][1] = so.y; o[p][2] = so.z; o[p][3] = so.w;
+      float u0 = uv[p][0], u1 = uv[p][1], u2 = uv[p][2], u3 = uv[p][3];
+      if (DELTA) { u0 -= su.x; u1 -= su.y; u2 -= su.z; u3 -= su.w; }
+      else if (a.act_in) { u0 = act_silu(a.act_in, u0); u1 = act_silu(a.act_in, u1); u2 = act_silu(a.act_in, u2); u3 = act_silu(a.act_in, u3); }
+      uint2 hi, lo;                                      // half of an operand's four registers: tokens (nt & 1) * 8 + q2 of step nt / 2
+      split2(u0, u1, hi.x, lo.x);
+      split2(u2, u3, hi.y, lo.y);
+      uint2* dst = reinterpret_cast<uint2*>(sU + ((nt >> 1) * 2) * 32 + lane) + (nt & 1);
+      dst[0] = hi;
+      dst[64] = lo;                                      // 32 lanes of 16 bytes further
+    }
+    cp_wait<1>();
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < 2; ++t) { sacc[t][0] *= ec[t][0]; sacc[t][1] *= ec[t][1]; sacc[t][2] *= ec[t][0]; sacc[t][3] *= ec[t][1]; }
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+      const uint4 uh = sU[(ks * 2) * 32 + lane], ul = sU[(ks * 2 + 1) * 32 + lane];
+      const uint32_t ah[4] = {uh.x, uh.y, uh.z, uh.w}, al[4] = {ul.x, ul.y, ul.z, ul.w};
+#pragma unroll
+      for (int t = 0; t < 2; ++t) mma3(sacc[t], ah, al, sK[((warp * 2 + t) * 4 + ks) * 32 + lane]);
+#pragma unroll
+      for (int p = 0; p < TPW; ++p)
+        if (ks <= (warp + p * NW) >> 1) mma3(o[p], ah, al, sB[((warp + p * NW) * 4 + ks) * 32 + lane]);  // keys up to the query
+    }
+#pragma unroll
+    for (int p = 0; p < TPW; ++p)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int t = (warp + p * NW) * 8 + q2 + (u & 1);
+        if (t < n) a.out[(row0 + t) * O + (size_t)h * a.DV + e0 + g + (u >> 1) * 8] = o[p][u];
+      }
+    __syncthreads();
+    fetch_kb(c + 1);
+  }
+  cp_wait<0>();
+#pragma unroll
+  for (int t = 0; t < 2; ++t)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) st[(size_t)(warp * 16 + t * 8 + q2 + (u & 1)) * a.DV + g + (u >> 1) * 8] = sacc[t][u];
+}
+
+template <int DK> size_t per_chunk(int DV, bool delta) { return Ws<DK>::total(DV, delta) * 4; }  // floats
+
+template <int DK, bool DELTA>
+cudaError_t launch_channel_t(const RecurArgs& a, cudaStream_t s) {
+  using Wk = Ws<DK>;
+  const size_t sm1 = (size_t)(3 * CT * (DK + 8) + CT * (CT + 4) + 4 * DK + (DELTA ? 2 * CT * (CT + 4) + 3 * 16 * 17 + CT : 0)) * sizeof(float);
+  const size_t sm2 = (size_t)((DELTA ? Wk::W : 0) + Wk::Q + Wk::K + Wk::B + (DELTA ? 2 : 1) * (DK / 16) * 256 + 256) * 16;
+  cudaError_t e;
+  if ((e = cudaFuncSetAttribute(channel_chunk_kernel<DK, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(channel_chain_kernel<DK, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2)) != cudaSuccess) return e;
+  const int NC = (a.L + CT - 1) / CT;
+  const int seg = (int)std::min<size_t>(NC, a.ws_floats / ((size_t)a.B * a.H * per_chunk<DK>(a.DV, DELTA)));  // chunks the workspace holds
+  for (int c0 = 0; c0 < NC; c0 += seg) {
+    const int nc = std::min(seg, NC - c0);
+    if ((e = launch_k(channel_chunk_kernel<DK, DELTA>, dim3(nc, a.H, a.B), dim3(512), sm1, s, a, c0)) != cudaSuccess) return e;
+    if ((e = launch_k(channel_chain_kernel<DK, DELTA>, dim3(a.DV / 16, a.H, a.B), dim3(DK * 2), sm2, s, a, c0, nc)) != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+}  // namespace
+
+bool recur_channel_shape(int DK, int DV) { return (DK == 64 || DK == 128) && DV % 16 == 0 && DV >= 16; }
+
+size_t recur_channel_ws_floats(int B, int L, int H, int DK, int DV) {
+  const size_t per = DK == 64 ? per_chunk<64>(DV, true) : per_chunk<128>(DV, true);
+  return (size_t)B * H * ((L + CT - 1) / CT) * per;
+}
+
+bool recur_channel_supported(const RecurArgs& a) {
+  if (!a.bf16_ops || a.n_state || a.k_scale || !a.ws || a.L < RECUR_CHANNEL_MIN || !recur_channel_shape(a.DK, a.DV)) return false;
+  if (a.mode == 0 ? a.head_decay == nullptr : a.log_c == nullptr && !(a.mode == 2 && a.log_g)) return false;
+  const uintptr_t al = (uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.log_c | (uintptr_t)a.ws;
+  if (a.ld_q % 4 || a.ld_k % 4 || (al & 15)) return false;
+  return recur_channel_ws_floats(a.B, 1, a.H, a.DK, a.DV) <= a.ws_floats;
+}
+
+cudaError_t launch_recur_channel(const RecurArgs& a, cudaStream_t s) {
+  if (!recur_channel_supported(a)) return cudaErrorInvalidValue;
+  if (a.DK == 64) return a.mode == 1 ? launch_channel_t<64, true>(a, s) : launch_channel_t<64, false>(a, s);
+  return a.mode == 1 ? launch_channel_t<128, true>(a, s) : launch_channel_t<128, false>(a, s);
+}

@@ -1,0 +1,63 @@
+"""The gated delta rule and gated linear attention of prompts in bf16 mode in the chunk-parallel form on tensor products: lengths at
+the edges of the 64-token chunks and of the rule (48 tokens), key sizes 64 and 128, value sizes down to 16, grouped keys, batches,
+decays that empty a channel within a few tokens and decays near one.  Against the float64 oracle at the families' bf16 bar (6e-2 of
+the logit scale), and against the same prompt in portions of 40 tokens, which the token-by-token chain takes: there only roundings of
+bf16 activations differ, 2^-9 each and averaged by every sum, so 1e-2."""
+import numpy as np
+import pytest
+
+import test_debuzen_gpu as deb
+import test_risalix_gpu as ris
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(m, o, vocab, n, batch, run, oracle=True):
+    ids = np.random.default_rng(n).integers(0, vocab, (batch, n))
+    whole = m.forward_rows(ids, 0, list(range(batch * n))).reshape(batch, n, -1)
+    parts = np.concatenate([m.forward_rows(ids[:, p:p + 40], p, list(range(batch * len(ids[0, p:p + 40])))).reshape(batch, -1, whole.shape[-1])
+                            for p in range(0, n, 40)], axis=1)
+    for b in range(batch):
+        if oracle:
+            assert deb.err(whole[b], run(o, ids[b])) < 6e-2
+        assert deb.err(whole[b], parts[b]) < 1e-2
+    # a second portion of chunks continues the state of the first
+    cut = min(n - 9, 70) if n >= 57 else 0
+    if cut >= 48:
+        a = m.forward_rows(ids[:, :cut], 0, list(range(batch * cut))).reshape(batch, cut, -1)
+        c = m.forward_rows(ids[:, cut:], cut, list(range(batch * (n - cut)))).reshape(batch, n - cut, -1)
+        for b in range(batch):
+            assert deb.err(np.concatenate([a[b], c[b]]), whole[b]) < 1e-2
+    m.close()
+
+
+def _rates(t, kind):
+    """A_log / a2.b of a layer: slow (decays near one), mixed, fast (a channel is empty after a few tokens)"""
+    for k in t:
+        if k.endswith("A_log"):
+            t[k] = np.full_like(t[k], {"slow": -4.0, "mixed": 0.0, "fast": 3.0}[kind])
+        if k.endswith("a2.b"):
+            t[k] = np.full_like(t[k], {"slow": 5.0, "mixed": 1.0, "fast": -40.0}[kind])
+    return t
+
+
+@pytest.mark.parametrize("n,batch", [(48, 2), (63, 1), (64, 3), (65, 1), (127, 1), (200, 2)])
+@pytest.mark.parametrize("heads,kv,dim,vdim,rate", [(2, 2, 128, 128, "mixed"), (4, 2, 64, 16, "fast"), (2, 1, 64, 80, "slow"), (2, 2, 128, 48, "fast")])
+def test_delta_rule(n, batch, heads, kv, dim, vdim, rate):
+    cfg = ris.config([ris.delta(heads, kv, dim, vdim, 4), ris.delta(heads, kv, dim, vdim, 2, ff=96)], width=96)
+    t = _rates(ris.random_model(cfg, 8), rate)
+    m, o = ris.build(cfg, dtype="bfloat16", max_seq_len=n + 2, max_batch_size=batch, tensors=t)
+    _check(m, o, cfg["vocab"], n, batch, lambda o, ids: o.run(ids))
+
+
+@pytest.mark.parametrize("n,batch", [(48, 2), (64, 1), (65, 3), (200, 1)])
+@pytest.mark.parametrize("heads,dim,vdim,rate", [(2, 128, 256, "mixed"), (3, 64, 16, "fast"), (1, 128, 80, "slow")])
+def test_gated_linear_attention(n, batch, heads, dim, vdim, rate):
+    layer = deb.gla(heads, dim, vdim, tau=1.0 if rate == "fast" else 8.0, mlp={"kind": "dense", "ff": 128})
+    cfg = deb.config([layer, layer], width=96)
+    t = _rates(deb.random_tensors(cfg, 9), rate)
+    m, o = deb.build(cfg, dtype="bfloat16", max_seq_len=n + 2, max_batch_size=batch, tensors=t)
+    # With decays of zero a head's output is v (q . k), and its norm makes that v times the sign of q . k: a row whose q . k is within
+    # the rounding of its bf16 projections is off by order one whatever the kernel does (the chain is 0.230 off on 200 tokens, the
+    # chunks 0.230 off, the two 0.002 apart).  Those cases are held to the chain alone.
+    _check(m, o, cfg["vocab"], n, batch, lambda o, ids: (deb.fresh(o), o.run(ids))[1], oracle=rate != "fast")
