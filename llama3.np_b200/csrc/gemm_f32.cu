@@ -1,0 +1,390 @@
+// fp32 projections of many rows on the 5th-generation tensor cores without giving up fp32's precision: C = A W^T with fp32 A and
+// W [N, K] fp32 or bf16.  Every fp32 value is cut into three bf16 parts of 8 significant bits each, x = x1 + x2 + x3 exactly, by
+// truncation, inside the kernel: TMA brings raw fp32 tiles, converter warps write the parts as operand tiles, and one thread
+// issues the products of the parts whose order is above 2^-24,
+//   a1 b1 | a1 b2 + a2 b1 + a2 b2 + a1 b3 + a3 b1          (W in bf16: a1 w | a2 w + a3 w),
+// the leading one and the corrections into two TMEM accumulators.  The tensor core drops the bits below an accumulator's last one
+// at every instruction (a drift of ~0.5 ulp each, 3.5e-6 relative over K = 4096 with the 3xTF32 scheme of gemm_tc.cu), so an
+// accumulator takes only 128 summed terms (8 instructions); the converter warps then add it to running fp32 sums in registers.
+// 600 x 4096 x 1024: 87 us (58 TFLOP/s of fp32 products), the FFMA tiles it replaces 350 us; measured per rule in layerlist.cu (ll_linear).
+//
+// One 128 x 128 tile per CTA and turn, persistent; 320 threads:
+//   warp 0: TMA   warp 1: TMEM + MMA issue   warps 2 - 9: conversion, running sums, epilogue
+// A step is 32 values of K.  The parts' tiles hold 64 (128-byte swizzled rows); their halves are two buffers of a ring, so that a
+// step is converted while the previous one is multiplied.  Bound by the MMAs: an M = 128 instruction takes ~132 cycles for N = 128 as
+// for N = 256 (mma_probe.cu), 12 of them per step against ~600 issue slots of conversion per scheduler; a 256-wide tile would halve
+// that but its parts and raw tiles do not fit the shared memory together.
+// Every wait is bounded: one that runs out sets a flag, all warps run on without waiting, and the host reports an error.
+#include <cuda.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "gemm_tc.h"
+
+namespace {
+
+constexpr int TILE = 128, STEP = 32, CHUNK = 4;          // tile edge; values of K per step; steps per accumulator turn
+constexpr int HALF = TILE * 128;                         // bytes of a 128-row tile of 128-byte rows
+constexpr int THREADS = 320, RAW = 4, WST = 3;        // raw tiles, and weight tiles of the bf16 form, in flight
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count)); }
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, volatile int* fail) {
+  for (uint32_t spins = 0; spins < (1u << 20); ++spins) {
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    if (ok) return;
+    if ((spins & 63) == 63 && *fail) return;
+  }
+  *fail = 1;
+}
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* tm, int c0, int c1, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+      ::"r"(dst), "l"(tm), "r"(c0), "r"(c1), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TILE >> 3) << 17) | ((128u >> 4) << 24);  // bf16 x bf16 -> fp32, 128 x 128
+__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t accum) {
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
+      ::"r"(d), "l"(a), "l"(b), "r"(IDESC), "r"(accum) : "memory");
+}
+__device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, float* v) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(v);
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr));
+}
+// K-major, 128-byte-swizzled operand tile: rows of 128 bytes, 8-row groups 1024 bytes apart
+__device__ __forceinline__ uint64_t desc_sw128(uint32_t smem_addr) {
+  return (uint64_t)((smem_addr & 0x3FFFF) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+
+// eight fp32 values -> three 16-byte pieces of bf16 parts; every subtraction is exact
+__device__ __forceinline__ void cut8(const float4& x, const float4& y, uint4& p1, uint4& p2, uint4& p3) {
+  const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+  uint32_t* o1 = reinterpret_cast<uint32_t*>(&p1);
+  uint32_t* o2 = reinterpret_cast<uint32_t*>(&p2);
+  uint32_t* o3 = reinterpret_cast<uint32_t*>(&p3);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float a = v[2 * i], b = v[2 * i + 1];
+    const float ra = a - __uint_as_float(__float_as_uint(a) & 0xffff0000u), rb = b - __uint_as_float(__float_as_uint(b) & 0xffff0000u);
+    const float sa = ra - __uint_as_float(__float_as_uint(ra) & 0xffff0000u), sb = rb - __uint_as_float(__float_as_uint(rb) & 0xffff0000u);
+    o1[i] = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+    o2[i] = __byte_perm(__float_as_uint(ra), __float_as_uint(rb), 0x7632);
+    o3[i] = __byte_perm(__float_as_uint(sa), __float_as_uint(sb), 0x7632);
+  }
+}
+
+template <bool WB16> constexpr int raw_bytes() { return WB16 ? HALF : 2 * HALF; }
+template <bool WB16> constexpr int smem_bytes() { return 1024 + 3 * HALF + (WB16 ? WST : 3) * HALF + RAW * raw_bytes<WB16>() + 512; }
+
+template <bool WB16, int EPI>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, int rows, int N, int K, int ksplit, float* part,
+                int* tile_cnt, int* err, EpiArgs e) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t sA = (raw + 1023u) & ~1023u, sW = sA + 3 * HALF, sR = sW + (WB16 ? WST : 3) * HALF, bars = sR + RAW * raw_bytes<WB16>();
+  uint8_t* base = smem_raw + (sA - raw);
+  const uint32_t r_full = bars, r_empty = r_full + 8 * RAW, h_full = r_empty + 8 * RAW, h_empty = h_full + 16, w_full = h_empty + 16,
+                 w_empty = w_full + 8 * WST, a_full = w_empty + 8 * WST, a_empty = a_full + 16, slot = a_empty + 16;
+  uint32_t* slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (slot - raw));
+  volatile int* fail = reinterpret_cast<volatile int*>(slot_ptr + 1);
+  int* last_flag = reinterpret_cast<int*>(slot_ptr + 2);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_launch();
+  if (warp == 0 && lane == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmA));
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmW));
+    *fail = 0;
+    for (int s = 0; s < RAW; ++s) { mbar_init(r_full + 8 * s, 1); mbar_init(r_empty + 8 * s, 8); }
+    for (int s = 0; s < WST; ++s) { mbar_init(w_full + 8 * s, 1); mbar_init(w_empty + 8 * s, 1); }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(h_full + 8 * s, 8); mbar_init(h_empty + 8 * s, 1);
+      mbar_init(a_full + 8 * s, 1); mbar_init(a_empty + 8 * s, 8);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(slot));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *slot_ptr;
+  pdl_wait();
+  const int tiles_m = (rows + TILE - 1) / TILE, tiles_n = (N + TILE - 1) / TILE, ntiles_mn = tiles_m * tiles_n, ntiles = ntiles_mn * ksplit;
+  const int blocks = (K + 63) / 64, per = (blocks + ksplit - 1) / ksplit;  // K in blocks of 64 = two steps (the surplus reads zeros)
+  // steps [0, n) of tile t: K values k0 + 32 s
+  auto slice = [&](int t, int& k0, int& n) {
+    const int ks = t / ntiles_mn, b0 = ks * per, b1 = min(blocks, b0 + per);
+    k0 = b0 * 64;
+    n = 2 * (b1 - b0);
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {  // ---------------- TMA
+      uint32_t it = 0, wt = 0;
+      for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const int tmn = t % ntiles_mn, m0 = (tmn % tiles_m) * TILE, n0 = (tmn / tiles_m) * TILE;
+        int k0, n;
+        slice(t, k0, n);
+        for (int s = 0; s < n; ++s, ++it) {
+          if (WB16 && !(s & 1)) {
+            const uint32_t st = wt % WST;
+            if (wt >= WST) mbar_wait(w_empty + 8 * st, (wt / WST - 1) & 1, fail);
+            mbar_expect_tx(w_full + 8 * st, HALF);
+            tma_load_2d(sW + st * HALF, &tmW, k0 + s * STEP, n0, w_full + 8 * st);
+            ++wt;
+          }
+          const uint32_t st = it % RAW;
+          if (it >= RAW) mbar_wait(r_empty + 8 * st, (it / RAW - 1) & 1, fail);
+          mbar_expect_tx(r_full + 8 * st, raw_bytes<WB16>());
+          tma_load_2d(sR + st * raw_bytes<WB16>(), &tmA, k0 + s * STEP, m0, r_full + 8 * st);
+          if (!WB16) tma_load_2d(sR + st * raw_bytes<WB16>() + HALF, &tmW, k0 + s * STEP, n0, r_full + 8 * st);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {  // ---------------- products
+      const uint64_t da = desc_sw128(sA), dw = desc_sw128(sW);
+      constexpr uint64_t PART = HALF >> 4;
+      uint32_t it = 0, wt = 0, ci = 0;
+      for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        int k0, n;
+        slice(t, k0, n);
+        for (int s = 0; s < n; ++s, ++it) {
+          const uint32_t h = it & 1, buf = ci & 1;
+          if (s % CHUNK == 0 && ci >= 2) mbar_wait(a_empty + 8 * buf, (ci / 2 - 1) & 1, fail);
+          if (WB16 && h == 0) mbar_wait(w_full + 8 * (wt % WST), (wt / WST) & 1, fail);
+          mbar_wait(h_full + 8 * h, (it >> 1) & 1, fail);
+          tc_fence_after();
+          const uint32_t lead = tmem + buf * 256, corr = lead + TILE;
+          const uint64_t wd = WB16 ? dw + (wt % WST) * PART : dw;
+#pragma unroll
+          for (int kk = 0; kk < 2; ++kk) {
+            const uint64_t a = da + (h * 2 + kk) * 2, w = wd + (h * 2 + kk) * 2;
+            const uint32_t go = (s % CHUNK) | kk ? 1u : 0u;
+            mma(lead, a, w, go);
+            if (WB16) {
+              mma(corr, a + PART, w, go);
+              mma(corr, a + 2 * PART, w, 1u);
+            } else {
+              mma(corr, a, w + PART, go);
+              mma(corr, a + PART, w, 1u);
+              mma(corr, a + PART, w + PART, 1u);
+              mma(corr, a, w + 2 * PART, 1u);
+              mma(corr, a + 2 * PART, w, 1u);
+            }
+          }
+          tc_commit(h_empty + 8 * h);
+          if (WB16 && h == 1) { tc_commit(w_empty + 8 * (wt % WST)); ++wt; }
+          if (s % CHUNK == CHUNK - 1 || s == n - 1) { tc_commit(a_full + 8 * buf); ++ci; }
+        }
+      }
+    }
+  } else {  // ---------------- conversion, running sums, epilogue
+    const int ct = threadIdx.x - 64, quarter = warp & 3, c0 = ((warp - 2) >> 2) * 64;  // TMEM lanes and columns of this warp
+    const uint32_t tl = tmem + ((uint32_t)(quarter * 32) << 16) + c0;
+    uint32_t it = 0, pi = 0;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+      const int tmn = t % ntiles_mn, m0 = (tmn % tiles_m) * TILE, n0 = (tmn / tiles_m) * TILE;
+      int k0, n;
+      slice(t, k0, n);
+      float run[64];
+#pragma unroll
+      for (int j = 0; j < 64; ++j) run[j] = 0.f;
+      auto promote = [&]() {
+        const uint32_t buf = pi & 1;
+        mbar_wait(a_full + 8 * buf, (pi >> 1) & 1, fail);
+        __syncwarp();
+        tc_fence_after();
+#pragma unroll
+        for (int c = 0; c < 64; c += 32) {
+          float x[32], y[32];
+          tmem_ld32_issue(tl + buf * 256 + c, x);
+          tmem_ld32_issue(tl + buf * 256 + TILE + c, y);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < 32; ++j) run[c + j] += x[j] + y[j];
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(a_empty + 8 * buf);
+        ++pi;
+      };
+#pragma unroll 1
+      for (int s = 0; s < n; ++s, ++it) {
+        const uint32_t st = it % RAW, h = it & 1;
+        mbar_wait(r_full + 8 * st, (it / RAW) & 1, fail);
+        if (it >= 2) mbar_wait(h_empty + 8 * h, ((it >> 1) - 1) & 1, fail);
+        // a thread: a row of 32 values (W bf16: half a row of A); 16-byte pieces swizzled inside the 128-byte rows on both sides
+        const int r = WB16 ? ct >> 1 : ct & 127, op = WB16 ? 0 : ct >> 7, q0 = WB16 ? (ct & 1) * 4 : 0;
+        const uint8_t* src = base + (sR - sA) + st * raw_bytes<WB16>() + op * HALF + r * 128;
+        uint8_t* dst = base + op * 3 * HALF + r * 128;
+#pragma unroll
+        for (int q = 0; q < (WB16 ? 4 : 8); q += 2) {
+          const int qq = q0 + q;
+          const float4 x = *reinterpret_cast<const float4*>(src + ((qq ^ (r & 7)) << 4)), y = *reinterpret_cast<const float4*>(src + (((qq + 1) ^ (r & 7)) << 4));
+          uint4 p1, p2, p3;
+          cut8(x, y, p1, p2, p3);
+          const int o = ((h * 4 + (qq >> 1)) ^ (r & 7)) << 4;
+          *reinterpret_cast<uint4*>(dst + o) = p1;
+          *reinterpret_cast<uint4*>(dst + HALF + o) = p2;
+          *reinterpret_cast<uint4*>(dst + 2 * HALF + o) = p3;
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) { mbar_arrive(r_empty + 8 * st); mbar_arrive(h_full + 8 * h); }
+        if (s % CHUNK == CHUNK - 1 && s >= CHUNK) promote();  // the turn before this one: its products are long issued
+      }
+      for (int left = (n + CHUNK - 1) / CHUNK - max(0, n / CHUNK - 1); left > 0; --left) promote();
+      const int m = m0 + quarter * 32 + lane, nc = n0 + c0;
+      if (ksplit > 1) {
+        // publish this slice's sums; the slice that arrives last adds all of them in slice order (the result does not depend on timing)
+        const int Mp = tiles_m * TILE, Np = tiles_n * TILE, ks = t / ntiles_mn;
+        float* p = part + ((size_t)ks * Mp + m) * Np + nc;
+        if (m < rows)
+#pragma unroll
+          for (int j = 0; j < 64; j += 4) __stcg(reinterpret_cast<float4*>(p + j), make_float4(run[j], run[j + 1], run[j + 2], run[j + 3]));
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (ct == 0) {
+          int old;
+          asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(old) : "l"(tile_cnt + tmn) : "memory");
+          *last_flag = old == ksplit - 1;
+          if (old == ksplit - 1) tile_cnt[tmn] = 0;  // ready for the next launch
+        }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        const bool is_last = *last_flag != 0;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (!is_last) continue;
+        if (m < rows) {
+          const float* q = part + (size_t)m * Np + nc;
+#pragma unroll
+          for (int j = 0; j < 64; j += 4) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int k2 = 0; k2 < ksplit; ++k2) {
+              const float4 x = __ldcg(reinterpret_cast<const float4*>(q + (size_t)k2 * Mp * Np + j));
+              v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+            }
+            run[j] = v.x; run[j + 1] = v.y; run[j + 2] = v.z; run[j + 3] = v.w;
+          }
+        }
+      }
+      if (m >= rows) continue;
+      const bool plain = !e.out_lo && !e.out_bf16 && !e.glu_w && !(e.ld_out & 3) && !(N & 3);
+#pragma unroll
+      for (int j = 0; j < 64; j += 4) {
+        const int col = nc + j;
+        if (col >= N) break;
+        if (plain && EPI != EPI_SWIGLU) {
+          float4 v = make_float4(run[j], run[j + 1], run[j + 2], run[j + 3]);
+          const size_t o = (size_t)m * e.ld_out + col;
+          if (EPI == EPI_RESID) {
+            const float4 x = *reinterpret_cast<const float4*>(e.resid + o);
+            v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+          } else if (e.unary) {
+            v.x = unary_act(e.unary, v.x); v.y = unary_act(e.unary, v.y); v.z = unary_act(e.unary, v.z); v.w = unary_act(e.unary, v.w);
+          }
+          *reinterpret_cast<float4*>(e.out + o) = v;
+        } else if (plain) {
+          const float2 v = make_float2(glu_pair<false>(e, run[j], run[j + 1]), glu_pair<false>(e, run[j + 2], run[j + 3]));
+          *reinterpret_cast<float2*>(e.out + (size_t)m * e.ld_out + (col >> 1)) = v;
+        } else {
+          epilogue_pair<float>(EPI, e, m, col, run[j], run[j + 1], col + 1 < N);
+          if (col + 2 < N) epilogue_pair<float>(EPI, e, m, col + 2, run[j + 2], run[j + 3], col + 3 < N);
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x == 0 && *fail) {
+    if (err) *err = 1;
+    __nanosleep(1000000);  // copies still in flight land before the shared memory is given up
+  }
+  __syncthreads();
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+}
+
+template <bool WB16, int EPI>
+cudaError_t launch_t(const GemmF32Args& a, cudaStream_t s) {
+  auto kern = gemm_f32_kernel<WB16, EPI>;
+  static bool done[16] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!done[dev & 15]) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<WB16>());
+    if (e != cudaSuccess) return e;
+    done[dev & 15] = true;
+  }
+  const CUtensorMap* ma = tc_get_map(a.A, false, a.rows, a.K, TILE, a.lda);
+  const CUtensorMap* mw = tc_get_map(a.W, WB16, a.N, a.K, TILE);
+  if (!ma || !mw) return cudaErrorInvalidValue;
+  static int n_sm[16] = {0};
+  if (!n_sm[dev & 15]) cudaDeviceGetAttribute(&n_sm[dev & 15], cudaDevAttrMultiProcessorCount, dev);
+  const int sms = n_sm[dev & 15] > 0 ? n_sm[dev & 15] : 148;
+  const int tm = (a.rows + TILE - 1) / TILE, tn = (a.N + TILE - 1) / TILE, tiles = tm * tn, blocks = (a.K + 63) / 64;
+  // K split over CTAs: the rounds of the machine times a slice's length, with ~2 blocks of 64 for a slice's start, publication and end
+  int ksplit = 1;
+  if (a.part && a.tile_cnt && tiles <= a.tile_cnt_len) {
+    long best = 0;
+    for (int ks = 1; ks <= 8; ++ks) {
+      const int per = (blocks + ks - 1) / ks;
+      if (ks > 1 && (per < 2 || (ks - 1) * per >= blocks || (size_t)tm * tn * TILE * TILE * 4 * ks > a.part_bytes)) continue;
+      const long cost = (long)((tiles * ks + sms - 1) / sms) * (per + 2);
+      if (!best || cost < best) { best = cost; ksplit = ks; }
+    }
+  }
+  return launch_k(kern, dim3(std::min(tiles * ksplit, sms)), dim3(THREADS), (size_t)smem_bytes<WB16>(), s, *ma, *mw, a.rows, a.N, a.K, ksplit, a.part,
+                  a.tile_cnt, a.err, a.e);
+}
+
+template <bool WB16>
+cudaError_t launch_e(const GemmF32Args& a, cudaStream_t s) {
+  switch (a.epi) {
+    case EPI_STORE: return launch_t<WB16, EPI_STORE>(a, s);
+    case EPI_RESID: return launch_t<WB16, EPI_RESID>(a, s);
+    case EPI_SWIGLU: return launch_t<WB16, EPI_SWIGLU>(a, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+}  // namespace
+
+bool gemm_f32_supported(const GemmF32Args& a) {
+  if (a.epi != EPI_STORE && a.epi != EPI_RESID && a.epi != EPI_SWIGLU) return false;
+  const int lda = a.lda ? a.lda : a.K;
+  if ((((uintptr_t)a.A | (uintptr_t)a.W) & 15) || lda % 4 || a.K % (a.w_bf16 ? 8 : 4)) return false;  // 16-byte rows of the tensor maps
+  // 16-byte rows of what the epilogue reads and writes
+  return !(((uintptr_t)a.e.out | (uintptr_t)a.e.resid) & 15) && tc_gemm_supported(8);
+}
+
+cudaError_t launch_gemm_f32(const GemmF32Args& a, cudaStream_t s) {
+  if (!gemm_f32_supported(a)) return cudaErrorInvalidValue;
+  return a.w_bf16 ? launch_e<true>(a, s) : launch_e<false>(a, s);
+}

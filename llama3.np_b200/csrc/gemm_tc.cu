@@ -88,12 +88,12 @@ static EncodeTiledFn encode_fn() {
 }
 
 // [rows, K] row-major matrix, box = 128 bytes of K x box_rows rows, 128-byte swizzle, zero OOB fill
-static bool make_map(CUtensorMap* tm, const void* ptr, bool is_bf16, int rows, int K, int box_rows) {
+static bool make_map(CUtensorMap* tm, const void* ptr, bool is_bf16, int rows, int K, int box_rows, int ld) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
   const size_t es = is_bf16 ? 2 : 4;
   cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)K * es};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * es};
   cuuint32_t box[2] = {(cuuint32_t)(128 / es), (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(tm, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
@@ -103,22 +103,23 @@ static bool make_map(CUtensorMap* tm, const void* ptr, bool is_bf16, int rows, i
 }
 
 struct MapCache {
-  std::map<std::tuple<const void*, int, int, int, int>, CUtensorMap> m;
+  std::map<std::tuple<const void*, int, int, int, int, int>, CUtensorMap> m;
   std::mutex mu;
-  const CUtensorMap* get(const void* ptr, bool is_bf16, int rows, int K, int box_rows) {
+  const CUtensorMap* get(const void* ptr, bool is_bf16, int rows, int K, int box_rows, int ld = 0) {
     std::lock_guard<std::mutex> g(mu);
-    auto key = std::make_tuple(ptr, (int)is_bf16, rows, K, box_rows);
+    if (!ld) ld = K;
+    auto key = std::make_tuple(ptr, (int)is_bf16, rows, K, box_rows, ld);
     auto it = m.find(key);
     if (it != m.end()) return &it->second;
     CUtensorMap tm;
-    if (!make_map(&tm, ptr, is_bf16, rows, K, box_rows)) return nullptr;
+    if (!make_map(&tm, ptr, is_bf16, rows, K, box_rows, ld)) return nullptr;
     return &m.emplace(key, tm).first->second;
   }
 };
 static MapCache g_maps;
 
-const CUtensorMap* tc_get_map(const void* ptr, bool is_bf16, int rows, int cols, int box_rows) {
-  return g_maps.get(ptr, is_bf16, rows, cols, box_rows);
+const CUtensorMap* tc_get_map(const void* ptr, bool is_bf16, int rows, int cols, int box_rows, int ld) {
+  return g_maps.get(ptr, is_bf16, rows, cols, box_rows, ld);
 }
 
 int tc_debug_timeline(int enable, unsigned long long* out64) {

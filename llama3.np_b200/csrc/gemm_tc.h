@@ -34,4 +34,22 @@ void tc_forget_maps();
 int tc_debug_timeline(int enable, unsigned long long* out64);
 // cached 2-D tensor map of a row-major [rows, cols] matrix: box = 128 bytes of columns x box_rows rows,
 // 128-byte swizzle (null if the driver entry point is unavailable)
-const CUtensorMap* tc_get_map(const void* ptr, bool is_bf16, int rows, int cols, int box_rows);
+// (ld: row stride in elements, 0 = cols; multiples of 16 bytes)
+const CUtensorMap* tc_get_map(const void* ptr, bool is_bf16, int rows, int cols, int box_rows, int ld = 0);
+
+// fp32 projections at fp32 precision on the tensor cores (gemm_f32.cu): fp32 A, W fp32 or bf16; EPI_STORE, EPI_RESID, EPI_SWIGLU
+struct GemmF32Args {
+  const float* A;       // [rows, K], row stride lda (0: K)
+  int lda;
+  const void* W;        // [N, K]
+  bool w_bf16;
+  int rows, N, K, epi;
+  EpiArgs e;
+  float* part;          // scratch of the K split, as TcGemmArgs (null: never split)
+  size_t part_bytes;
+  int* tile_cnt;
+  int tile_cnt_len;
+  int* err;             // set to 1 when a wait inside the kernel ran out
+};
+bool gemm_f32_supported(const GemmF32Args& a);
+cudaError_t launch_gemm_f32(const GemmF32Args& a, cudaStream_t s);

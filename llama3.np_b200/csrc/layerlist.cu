@@ -1157,15 +1157,17 @@ int ll_finalize(L3Model* m) {
       ll->chunk_ws_floats = std::max(ll->chunk_ws_floats, std::min(need, (size_t)64 << 20));
     }
   if (ll->chunk_ws_floats) CK(m, cudaMalloc((void**)&ll->chunk_ws, ll->chunk_ws_floats * 4));
-  // tensor cores: bf16 mode only.  fp32 mode is the exact mode of this family: every product is an fp32 FFMA chain
-  // (the 3xTF32 scheme of the Llama path would need a (hi, lo) copy of the residual stream beside the stream itself).
-  m->tc_ok = m->bf16 && !(m->cfg.flags & L3_FLAG_NO_TENSORCORE) && tc_gemm_supported(W);
+  // tensor cores: in bf16 mode every projection of many rows with a bf16 mirror; in both modes the ones that read fp32 rows, at fp32
+  // precision (gemm_f32.cu).  (The 3xTF32 scheme of the Llama path is further from 64-bit sums than an fp32 FFMA chain: 3.5e-6 against
+  // 1.2e-6 of the result at K = 4096.)
+  ll->f32_tc = !(m->cfg.flags & L3_FLAG_NO_TENSORCORE) && tc_gemm_supported(W);
+  m->tc_ok = m->bf16 && ll->f32_tc;
+  if (ll->f32_tc && !(getenv("L3_GEMM_KSPLIT") && atoi(getenv("L3_GEMM_KSPLIT")) == 0)) {
+    CK(m, cudaMalloc((void**)&m->gemm_part, (size_t)32 << 20));
+    CK(m, cudaMalloc((void**)&m->gemm_cnt, 1024 * sizeof(int)));
+    CK(m, cudaMemsetAsync(m->gemm_cnt, 0, 1024 * sizeof(int), m->stream));
+  }
   if (m->tc_ok) {
-    if (!(getenv("L3_GEMM_KSPLIT") && atoi(getenv("L3_GEMM_KSPLIT")) == 0)) {
-      CK(m, cudaMalloc((void**)&m->gemm_part, (size_t)32 << 20));
-      CK(m, cudaMalloc((void**)&m->gemm_cnt, 1024 * sizeof(int)));
-      CK(m, cudaMemsetAsync(m->gemm_cnt, 0, 1024 * sizeof(int), m->stream));
-    }
     CK(m, cudaMalloc(&m->xn16, ct * W * 2));  // mirror of the residual stream
     CK(m, cudaMalloc(&m->ctx16, ct * ll->max_ctx * 2));
     CK(m, cudaMemsetAsync(m->ctx16, 0, ct * ll->max_ctx * 2, m->stream));
@@ -1456,6 +1458,20 @@ static int ll_linear(L3Model* m, const void* W, const float* x32, const void* x1
     if (swap_on && gemm_swap_supported(rows, N)) LAUNCH(m, launch_gemm_swap(t, m->stream));
     else LAUNCH(m, launch_gemm_tc(t, m->stream));
     return L3_OK;
+  }
+  // More than 8 fp32 rows (or more than the row-streaming kernel's shared memory holds): cut into bf16 parts on the tensor cores.
+  // Against the FFMA tiles (linear_simt_kernel), which a call takes only where a row is no multiple of 16 bytes or a side is below
+  // half a tile: 600 rows at width 1024, per product 141 -> 52 us; the two-layer fp32 prompt 2852 -> 1630 us, at 12 tokens 1112 -> 554
+  // us, at 20 tokens 1624 -> 668 us, an 8-sequence fp32 decode step of a pre-norm stack of width 1024 1.20 -> 0.35 ms.  The logits'
+  // distance from 64-bit ones: 1.5e-6 -> 3.7e-7 of their size (sums of 128 terms in the tensor core, then fp32 sums).
+  if (ll->f32_tc && K >= 64 && N >= 64) {
+    GemmF32Args t{};
+    t.A = a.x; t.lda = ld; t.W = W; t.w_bf16 = m->bf16; t.rows = rows; t.N = N; t.K = K; t.epi = epi; t.e = e;
+    t.part = m->gemm_part; t.part_bytes = (size_t)32 << 20; t.tile_cnt = m->gemm_cnt; t.tile_cnt_len = 1024; t.err = ll->h_err;
+    if (gemm_f32_supported(t)) {
+      LAUNCH(m, launch_gemm_f32(t, m->stream));
+      return L3_OK;
+    }
   }
   if (K % 4 == 0 && ld % 4 == 0) LAUNCH(m, launch_linear_simt(a, m->bf16, m->bf16, m->stream));
   else LAUNCH(m, launch_linear_any(a, m->bf16, m->stream));

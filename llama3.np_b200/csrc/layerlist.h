@@ -138,6 +138,7 @@ struct LayerList {
   float *y1 = nullptr, *y2 = nullptr;      // the two sublayers' results [cap_tok, width] (with streams: y1 alone)
   float* moe_gu = nullptr;                 // [cap_tok, 2 ff_total] gate | up of every expert
   float *diff_part_o = nullptr, *diff_part_ml = nullptr;  // split scratch of the differential decode attention
+  bool f32_tc = false;  // fp32 rows of many tokens run the fp32-precision tensor-core GEMM (gemm_f32.cu)
   int max_in = 0, max_o = 0, max_ctx = 0, max_ff = 0;  // max_ctx: columns of an output projection's input
   int head_rows = 0;  // rows the LM head's buffers hold
 };
