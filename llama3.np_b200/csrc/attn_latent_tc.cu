@@ -182,6 +182,28 @@ __global__ void __launch_bounds__(256) latent_q_pack_kernel(LatentQPackArgs a) {
   }
 }
 
+// fp32 mode: the rotated part turned in place
+__global__ void __launch_bounds__(256) latent_q_rot_kernel(LatentQPackArgs a) {
+  extern __shared__ float trig[];
+  pdl_launch();
+  pdl_wait();
+  const size_t r = blockIdx.x;
+  const int half = a.rot_dims >> 1;
+  const int pos = *a.pos_ptr + (int)(r % a.L);
+  for (int i = threadIdx.x; i < half; i += blockDim.x) sincosf((float)pos * a.inv_freq[i], &trig[half + i], &trig[i]);
+  __syncthreads();
+  const int hd = a.dim + a.rot_dim;
+  for (int i = threadIdx.x; i < a.H * half; i += blockDim.x) {
+    const int h = i / half, p = i - h * half;
+    float* v = const_cast<float*>(a.q) + (r * a.H + h) * (size_t)hd + a.dim;
+    float* x = v + (a.rot_layout ? p : 2 * p);
+    float* y = v + (a.rot_layout ? p + half : 2 * p + 1);
+    const float u = *x, w = *y, c = trig[p], s = trig[half + p];
+    *x = u * c - w * s;
+    *y = w * c + u * s;
+  }
+}
+
 // ---------------------------------------------------------------- attention
 struct Shape {
   int nks, nrs, nqs, nvs;  // 64-entry slices of the un-rotated keys, the rotated part, both, the values
@@ -516,6 +538,10 @@ bool latent_tc_supported(int dim, int rot_dim, int vdim, int kv_rank) {
 
 cudaError_t launch_latent_q_pack(const LatentQPackArgs& a, int rows, cudaStream_t s) {
   return launch_k(latent_q_pack_kernel, dim3(rows), dim3(256), (size_t)std::max(1, a.rot_dims) * sizeof(float), s, a);
+}
+
+cudaError_t launch_latent_q_rot(const LatentQPackArgs& a, int rows, cudaStream_t s) {
+  return launch_k(latent_q_rot_kernel, dim3(rows), dim3(256), (size_t)std::max(1, a.rot_dims) * sizeof(float), s, a);
 }
 
 template <bool SIGMOID>

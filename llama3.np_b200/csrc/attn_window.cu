@@ -245,8 +245,10 @@ __global__ void __launch_bounds__(256) win_attn_kernel(WinAttnArgs a) {
 #pragma unroll
     for (int j = 0; j < NJ; ++j) o[qi][j] = 0.f;
   }
-  const KVT* ck = (const KVT*)a.cache_k + ((size_t)b * a.G + g) * a.M * a.DK;
-  const KVT* cv = (const KVT*)a.cache_v + ((size_t)b * a.G + g) * a.M * a.DV;
+  const int dk1 = a.DK - a.dk2, k_ld = a.k_ld ? a.k_ld : a.DK, v_ld = a.k_ld ? a.k_ld : a.DV;
+  const KVT* ck = (const KVT*)a.cache_k + (a.k_ld ? (size_t)b * a.kv_seq + (size_t)g * dk1 : ((size_t)b * a.G + g) * a.M * a.DK);
+  const KVT* cv = (const KVT*)a.cache_v + (a.k_ld ? (size_t)b * a.kv_seq + (size_t)g * a.DV : ((size_t)b * a.G + g) * a.M * a.DV);
+  const KVT* ck2 = (const KVT*)a.k2 + (size_t)b * a.k2_seq;
   float* myP = sP + (size_t)warp * WA_QW * WA_KEYS;
 
   for (int tile = tile_lo; tile < tile_hi; ++tile) {
@@ -255,8 +257,9 @@ __global__ void __launch_bounds__(256) win_attn_kernel(WinAttnArgs a) {
     for (int kk = tid >> 3; kk < WA_KEYS; kk += 32) {  // 8 threads per key / value row
       const int vi = v0 + kk;
       const int j = vi < nkeys ? (vi < ka ? vi : w_lo + (vi - ka)) : -1;
-      stage_row<KVT>(j >= 0 ? ck + (size_t)j * a.DK : nullptr, a.DK, DKP, sK + (size_t)kk * KS, tid & 7, 8);
-      stage_row<KVT>(j >= 0 ? cv + (size_t)j * a.DV : nullptr, a.DV, DVP, sV + (size_t)kk * DVP, tid & 7, 8);
+      stage_row<KVT>(j >= 0 ? ck + (size_t)j * k_ld : nullptr, dk1, a.dk2 ? dk1 : DKP, sK + (size_t)kk * KS, tid & 7, 8);
+      if (a.dk2) stage_row<KVT>(j >= 0 ? ck2 + (size_t)j * a.k2_ld : nullptr, a.dk2, DKP - dk1, sK + (size_t)kk * KS + dk1, tid & 7, 8);
+      stage_row<KVT>(j >= 0 ? cv + (size_t)j * v_ld : nullptr, a.DV, DVP, sV + (size_t)kk * DVP, tid & 7, 8);
     }
     __syncthreads();
     // scores: a lane holds keys lane and lane + 32 of the tile
@@ -355,12 +358,13 @@ __global__ void __launch_bounds__(256) win_attn_kernel(WinAttnArgs a) {
       continue;
     }
     float mul = a.out_scale * (a.kind == L3_ATTN_SIGMOID ? 1.f : (sum[qi] > 0.f ? 1.0f / sum[qi] : 0.f));
-    if (a.gate) mul *= sigmoid_f(a.gate[r * a.ld_gate + h]);
+    if (a.gate && !a.gate_wide) mul *= sigmoid_f(a.gate[r * a.ld_gate + h]);
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
       const int d = win_col<NJ>(lane, j);
       if (d < a.DV) {
-        const float v = o[qi][j] * mul;
+        float v = o[qi][j] * mul;
+        if (a.gate && a.gate_wide) v *= sigmoid_f(a.gate[r * a.ld_gate + (size_t)h * a.DV + d]);
         const size_t oi = r * a.ld_out + (size_t)h * a.DV + d;
         if (a.out) a.out[oi] = v;
         if (a.out16) a.out16[oi] = __float2bfloat16_rn(v);
@@ -640,6 +644,10 @@ cudaError_t launch_win_prep(const WinPrepArgs& a, int rows, bool kv_bf16, cudaSt
 cudaError_t launch_win_attn(const WinAttnArgs& a, bool kv_bf16, cudaStream_t s) {
   if (!win_attn_supported(a.DK, a.DV) || a.H % a.G != 0 || a.nsplit < 1 || a.nsplit > WA_SPLIT_MAX) return cudaErrorInvalidValue;
   if (a.nsplit > 1 && (!a.part_o || !a.part_ml)) return cudaErrorInvalidValue;
+  if ((a.k_ld || a.gate_wide) && (a.nsplit > 1 || a.L < 2 || a.H != a.G)) return cudaErrorInvalidValue;
+  // 16-byte pieces of every row
+  if (a.k_ld && ((((uintptr_t)a.cache_k | (uintptr_t)a.cache_v | (uintptr_t)a.k2) & 15) || a.k_ld % 8 || a.k2_ld % 8 || a.DK % 8 || a.dk2 % 8 || a.DV % 8))
+    return cudaErrorInvalidValue;
   const int rep = a.H / a.G;
   const dim3 grid((a.L * rep + WA_ROWS - 1) / WA_ROWS, a.G, a.B * a.nsplit);
   cudaError_t e = kv_bf16 ? launch_win_t<bf16>(a, grid, s) : launch_win_t<float>(a, grid, s);

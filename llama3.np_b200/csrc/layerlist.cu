@@ -957,6 +957,17 @@ static bool ll_latent_on_tc(const L3Model* m, const L3LayerSpec& s) {
          latent_tc_supported(s.dim, s.rot_dim, s.vdim, s.kv_rank);
 }
 
+// In fp32 mode, portions of LATENT_F32_MIN tokens and more expand the cached rows as well: 2 (dim + rot_dim + vdim) FLOPs per (query,
+// key, head) instead of the folded form's 2 (2 kv_rank + rot_dim), for an expansion of 2 (dim + vdim) kv_rank per (key, head), which
+// runs on the tensor cores while the attention is FFMA in both forms.  8 heads of 128 + 64, values 128, rank 512, per layer: 600 tokens
+// 338 + 90 us (attention, products of the folded form) -> 123 + 45 us; the two-layer prompt 1624 -> 1097 us, at 64 tokens 670 -> 587 us;
+// a short portion behind a long prefix would expand the whole prefix for little, so it starts there.
+constexpr int LATENT_F32_MIN = 64;
+static bool ll_latent_expands_f32(const L3Model* m, const L3LayerSpec& s) {
+  return !m->bf16 && m->ll->f32_tc && s.mixer == L3_MIX_LATENT && s.dim % 8 == 0 && s.rot_dim % 8 == 0 && s.vdim % 8 == 0 && s.kv_rank % 8 == 0 &&
+         s.heads * (s.dim + s.vdim) >= 64 && s.kv_rank + s.rot_dim >= 64 && win_attn_supported(s.dim + s.rot_dim, s.vdim);
+}
+
 // Prompts of the softmax mixers with heads of 64 and more in multiples of 8 run on the tensor cores in bf16 mode, where the caches
 // hold bf16 rows (attn_latent_tc.cu); other sizes and fp32 mode keep the FFMA kernels.  The queries of plain-softmax, differential,
 // sigmoid and keep-first attention go there as (high, low) pairs, those of the window kinds without kept tokens as one rounded part.
@@ -1186,6 +1197,16 @@ int ll_finalize(L3Model* m) {
       q_ld = std::max(q_ld, (size_t)L.spec.heads * latent_tc_q_ld(L.spec.dim, L.spec.rot_dim));
       e_ld = std::max(e_ld, (size_t)L.spec.heads * (L.spec.dim + L.spec.vdim));
     }
+  if (!m->bf16) {
+    size_t f_ld = 0;
+    for (auto& L : ll->layers)
+      if (ll_latent_expands_f32(m, L.spec)) f_ld = std::max(f_ld, (size_t)L.spec.heads * (L.spec.dim + L.spec.vdim));
+    const size_t per = (size_t)m->M * f_ld * 4;
+    if (f_ld && ct >= LATENT_F32_MIN && per <= ((size_t)1 << 30)) {  // longer contexts keep the folded form
+      ll->exp_seqs = (int)std::max<size_t>(1, std::min<size_t>(m->maxB, ((size_t)1 << 28) / per));
+      CK(m, cudaMalloc(&ll->lat_exp, ll->exp_seqs * per));
+    }
+  }
   if (e_ld && ct > 8) {
     const size_t per = (size_t)m->M * e_ld * 2;  // one sequence's keys and values; sequences share the workspace in turns
     ll->exp_seqs = (int)std::max<size_t>(1, std::min<size_t>(m->maxB, ((size_t)1 << 30) / per));
@@ -1652,6 +1673,41 @@ static int ll_latent_prompt(L3Model* m, LLLayer& Ly, LLState& St, int B, int L) 
   return L3_OK;
 }
 
+// fp32 mode: the same expansion by the fp32-precision GEMM, FFMA attention per head on the expanded rows and the rotated cache part.
+static int ll_latent_prompt_f32(L3Model* m, LLLayer& Ly, LLState& St, int B, int L) {
+  LayerList* ll = m->ll;
+  const L3LayerSpec& s = Ly.spec;
+  const int ntok = B * L, H = s.heads, DK = s.dim, DV = s.vdim, Dk = s.kv_rank + s.rot_dim, n_exp = H * (DK + DV);
+  int* d_pos = m->d_scal + 0;
+  if (s.rot_dims > 0) {
+    LatentQPackArgs qa{};
+    qa.q = m->q; qa.inv_freq = Ly.inv_freq; qa.pos_ptr = d_pos; qa.L = L; qa.H = H; qa.dim = DK; qa.rot_dim = s.rot_dim; qa.rot_dims = s.rot_dims; qa.rot_layout = s.rot_layout;
+    LAUNCH(m, launch_latent_q_rot(qa, ntok, m->stream));
+  }
+  const int T = std::min(m->M, (ll->keys_end + 127) / 128 * 128);
+  for (int b0 = 0; b0 < B; b0 += ll->exp_seqs) {
+    const int n = std::min(ll->exp_seqs, B - b0);
+    float* exp = (float*)ll->lat_exp;
+    for (int i = 0; i < n; ++i) {
+      GemmF32Args t{};
+      t.A = (const float*)St.lat + (size_t)(b0 + i) * m->M * Dk; t.W = Ly.w_ukv; t.rows = T; t.N = n_exp; t.K = Dk; t.epi = EPI_STORE;
+      t.e = store_to(exp + (size_t)i * m->M * n_exp, nullptr, n_exp);
+      t.part = m->gemm_part; t.part_bytes = (size_t)32 << 20; t.tile_cnt = m->gemm_cnt; t.tile_cnt_len = 1024; t.err = ll->h_err;
+      LAUNCH(m, launch_gemm_f32(t, m->stream));
+    }
+    WinAttnArgs at{};
+    at.q = m->q + (size_t)b0 * L * H * (DK + s.rot_dim);
+    at.cache_k = exp; at.cache_v = exp + H * DK; at.kv_seq = (int64_t)m->M * n_exp; at.k_ld = n_exp;
+    at.k2 = (const float*)St.lat + (size_t)b0 * m->M * Dk + s.kv_rank; at.k2_seq = (int64_t)m->M * Dk; at.k2_ld = Dk; at.dk2 = s.rot_dim;
+    at.out = m->ctx + (size_t)b0 * L * H * DV; at.ld_out = H * DV; at.out_scale = 1.f; at.head_vec = s.sink ? Ly.head_vec : nullptr;
+    at.gate = ll->pin + (size_t)b0 * L * Ly.n_in + Ly.off_g; at.ld_gate = Ly.n_in; at.gate_wide = s.gate_wide;
+    at.pos_ptr = d_pos; at.scale = s.scale; at.kind = s.sink ? L3_ATTN_SINK : L3_ATTN_SOFTMAX;
+    at.B = n; at.L = L; at.H = at.G = H; at.DK = DK + s.rot_dim; at.DV = DV; at.M = m->M; at.nsplit = 1;
+    LAUNCH(m, launch_win_attn(at, false, m->stream));
+  }
+  return L3_OK;
+}
+
 static int ll_enqueue_prenorm(L3Model* m, int B, int L, float* d_resid) {
   LayerList* ll = m->ll;
   const int ntok = B * L, W = m->D;
@@ -1770,6 +1826,8 @@ static int ll_enqueue_prenorm(L3Model* m, int B, int L, float* d_resid) {
       if ((rc = ll_linear(m, Ly.w_uq, ll->aux, ll->aux16, 0, ntok, nq, s.q_rank, EPI_STORE, store_to(m->q, nullptr, nq))) != L3_OK) return rc;
       if (L > 8 && ll->lat_exp && ll_latent_on_tc(m, s)) {
         if ((rc = ll_latent_prompt(m, Ly, St, B, L)) != L3_OK) return rc;
+      } else if (L >= LATENT_F32_MIN && ll->lat_exp && ll_latent_expands_f32(m, s)) {
+        if ((rc = ll_latent_prompt_f32(m, Ly, St, B, L)) != L3_OK) return rc;
       } else {
         // queries onto the latent: qlat[r, h] = [Wuk_h^T q_c | rot(q_r)]
         HeadGemmArgs ga{};

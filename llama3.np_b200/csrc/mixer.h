@@ -212,6 +212,7 @@ struct LatentTcArgs {
   int ld_out;            // row stride of out / out16
   float out_scale;
 };
+cudaError_t launch_latent_q_rot(const LatentQPackArgs& a, int rows, cudaStream_t s);  // turns the rotated part of the fp32 queries in place
 int latent_tc_q_ld(int dim, int rot_dim);  // entries of a packed query head
 bool latent_tc_supported(int dim, int rot_dim, int vdim, int kv_rank);
 cudaError_t launch_latent_q_pack(const LatentQPackArgs& a, int rows, cudaStream_t s);
@@ -373,6 +374,13 @@ struct WinAttnArgs {
   int window, keep_first;  // query i sees key j <= i with i - j < window (0: all) or j < keep_first
   int chunked;           // 1: instead of i - j < window, i / window == j / window (chunks counted from position 0)
   int B, L, H, G, DK, DV, M;
+  // Prompts over expanded latent rows (k_ld > 0; one key head per query head, more than one token): key j of sequence b, head h is
+  // cache_k[b * kv_seq + j * k_ld + h * (DK - dk2)] (DK - dk2 entries), then k2[b * k2_seq + j * k2_ld] (dk2 entries, all heads); its
+  // value cache_v[b * kv_seq + j * k_ld + h * DV]
+  int64_t kv_seq, k2_seq;
+  int k_ld, k2_ld, dk2;
+  const void* k2;
+  int gate_wide;         // 1: the gate has an entry per value, gate[r * ld_gate + h * DV + d] (win_attn_kernel without splits)
   int nsplit;            // > 1: the key tiles of a query spread over that many CTAs; partials in part_o / part_ml
   float *part_o, *part_ml;
 };
