@@ -266,11 +266,13 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       const int m = m0 + quarter * 32 + lane, nc = n0 + c0;
       if (ksplit > 1) {
         // publish this slice's sums; the slice that arrives last adds all of them in slice order (the result does not depend on timing)
-        const int Mp = tiles_m * TILE, Np = tiles_n * TILE, ks = t / ntiles_mn;
-        float* p = part + ((size_t)ks * Mp + m) * Np + nc;
+        // scratch [k slice][output tile][column / 4][row of the tile] float4: a warp's rows are contiguous
+        const size_t slice_len = (size_t)ntiles_mn * (TILE / 4) * TILE;
+        float4* p = reinterpret_cast<float4*>(part) + ((size_t)tmn * (TILE / 4) + c0 / 4) * TILE + quarter * 32 + lane;
+        const int ks = t / ntiles_mn;
         if (m < rows)
 #pragma unroll
-          for (int j = 0; j < 64; j += 4) __stcg(reinterpret_cast<float4*>(p + j), make_float4(run[j], run[j + 1], run[j + 2], run[j + 3]));
+          for (int j = 0; j < 64; j += 4) __stcg(p + ks * slice_len + (size_t)(j / 4) * TILE, make_float4(run[j], run[j + 1], run[j + 2], run[j + 3]));
         asm volatile("bar.sync 1, 256;" ::: "memory");
         if (ct == 0) {
           int old;
@@ -283,15 +285,14 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         asm volatile("bar.sync 1, 256;" ::: "memory");
         if (!is_last) continue;
         if (m < rows) {
-          const float* q = part + (size_t)m * Np + nc;
 #pragma unroll
-          for (int j = 0; j < 64; j += 4) {
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int k2 = 0; k2 < ksplit; ++k2) {
-              const float4 x = __ldcg(reinterpret_cast<const float4*>(q + (size_t)k2 * Mp * Np + j));
-              v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
-            }
-            run[j] = v.x; run[j + 1] = v.y; run[j + 2] = v.z; run[j + 3] = v.w;
+          for (int j = 0; j < 64; ++j) run[j] = 0.f;
+          for (int k2 = 0; k2 < ksplit; ++k2) {
+            float4 q[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) q[j] = __ldcg(p + k2 * slice_len + (size_t)j * TILE);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) { run[4 * j] += q[j].x; run[4 * j + 1] += q[j].y; run[4 * j + 2] += q[j].z; run[4 * j + 3] += q[j].w; }
           }
         }
       }

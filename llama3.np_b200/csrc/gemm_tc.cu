@@ -156,6 +156,40 @@ int tc_pick_bn(int kind, int rows, int N) {
   return 32;
 }
 
+static int sm_count() {
+  static int n[16] = {0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!n[dev & 15]) cudaDeviceGetAttribute(&n[dev & 15], cudaDevAttrMultiProcessorCount, dev);
+  return n[dev & 15] > 0 ? n[dev & 15] : 148;
+}
+
+// bf16: tile width and K split together, by the cycles of the busiest CTA.  A k-block (64 of K) costs four MMAs of ~132 cycles
+// whatever the width (mma_probe.cu), or the 85 bytes per cycle that a CTA's tiles arrive at (128 x 256: 578 cycles) - so wide tiles
+// are as cheap as narrow ones, and few tiles are better cut along K than along N.  The last tile's epilogue is not overlapped
+// (~14 cycles per column for a plain store, 20 - 24 where it reads as well), a split adds the partial tiles' way through L2.
+// Against the rule this replaces (the widest tile that gives 120 tiles, K cut only below 74): 1462 x 2048 x 8192, 116 -> 70 us (96
+// tiles of 256 in one round instead of 192 of 128 in two); 768 x 2048 x 10240, 150 -> 55 us (48 tiles x 3 slices instead of 192 of 64);
+// two-layer prompts: 2 x 731 tokens at width 2048 775 -> 676 us, 200 tokens at width 4096 647 -> 524 us, 700 tokens 1035 -> 841 us.
+static void pick_bf16(const TcGemmArgs& a, int sms, int* bn_out, int* ks_out) {
+  const int tm = (a.rows + 127) / 128, nkb = (a.K + 63) / 64;
+  const int per_col = a.epi == EPI_ROPE_KV ? 24 : a.epi == EPI_RESID ? 20 : 14;
+  double best = 0;
+  for (int bn = 256; bn >= 32; bn >>= 1) {
+    const int tiles = tm * ((a.N + bn - 1) / bn);
+    const double block = std::max(528.0, (16384.0 + 128.0 * bn) / 85.0), epi = per_col * bn;
+    for (int ks = 1; ks <= 8; ++ks) {
+      const int per = (nkb + ks - 1) / ks;
+      if (ks > 1 && (!a.part || !a.tile_cnt || tiles > a.tile_cnt_len || per < 3 || (ks - 1) * per >= nkb ||
+                     (size_t)tm * 128 * ((a.N + bn - 1) / bn) * bn * sizeof(float) * ks > a.part_bytes)) continue;
+      const int rounds = (tiles * ks + sms - 1) / sms;
+      const double main = per * block;
+      const double cost = (rounds - 1) * std::max(main, epi) + main + epi + (ks > 1 ? bn * (28.0 + 11.0 * ks) : 0.0);
+      if (best == 0 || cost < best * 0.99) { best = cost; *bn_out = bn; *ks_out = ks; }
+    }
+  }
+}
+
 template <int KIND, int BN, int EPI>
 static cudaError_t launch_tc_t(const TcGemmArgs& a, cudaStream_t s) {
   using Cf = TcCfg<KIND, BN>;
@@ -176,15 +210,13 @@ static cudaError_t launch_tc_t(const TcGemmArgs& a, cudaStream_t s) {
   const CUtensorMap* B1 = Cf::PARTS == 2 ? g_maps.get(a.W[1], b16, a.N, a.K, BN) : B0;
   if (!A0 || !B0 || !A1 || !B1) return cudaErrorInvalidValue;
   const int ntiles = ((a.N + BN - 1) / BN) * ((a.rows + 127) / 128);
-  static int n_sm[16] = {0};
-  if (!n_sm[dev & 15]) cudaDeviceGetAttribute(&n_sm[dev & 15], cudaDevAttrMultiProcessorCount, dev);
-  const int sms = n_sm[dev & 15] > 0 ? n_sm[dev & 15] : 148;
+  const int sms = sm_count();
   const int nkb_all = (a.K + Cf::BK - 1) / Cf::BK;
   // K-split (deterministic, see the epilogue) when the output tiles cover less than half the machine:
   // short-and-wide decode projections (N = D = 288: 18 tiles) otherwise leave most SMs idle while
   // each CTA walks the whole K loop.  Needs caller-owned scratch (TcGemmArgs::part / tile_cnt).
-  int ksplit = 1;
-  if (a.part && a.tile_cnt && ntiles * 2 <= sms && ntiles <= a.tile_cnt_len) {
+  int ksplit = std::max(1, a.ksplit);
+  if (!a.ksplit && a.part && a.tile_cnt && ntiles * 2 <= sms && ntiles <= a.tile_cnt_len) {
     ksplit = std::min(std::min(8, sms / ntiles), nkb_all / 3);
     const size_t need = (size_t)((a.rows + 127) / 128 * 128) * ((a.N + BN - 1) / BN * BN) * sizeof(float);
     while (ksplit > 1 && need * ksplit > a.part_bytes) --ksplit;
@@ -214,8 +246,10 @@ static cudaError_t launch_tc_e(const TcGemmArgs& a, cudaStream_t s) {
   }
 }
 
-cudaError_t launch_gemm_tc(const TcGemmArgs& a, cudaStream_t s) {
-  const int bn = a.bn > 0 ? a.bn : tc_pick_bn(a.kind, a.rows, a.N);
+cudaError_t launch_gemm_tc(const TcGemmArgs& args, cudaStream_t s) {
+  TcGemmArgs a = args;
+  int bn = a.bn > 0 ? a.bn : tc_pick_bn(a.kind, a.rows, a.N);
+  if (a.kind == TC_BF16 && a.bn <= 0 && a.epi != EPI_ARGMAX) pick_bf16(a, sm_count(), &bn, &a.ksplit);
   if (a.kind == TC_BF16) {
     switch (bn) {
       case 256: return launch_tc_e<TC_BF16, 256>(a, s);

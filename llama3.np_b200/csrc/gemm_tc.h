@@ -13,11 +13,12 @@ struct TcGemmArgs {
   const void* A[2];     // activations [rows, K]: bf16, or fp32 (hi, lo) pair
   const void* W[2];     // weights [N, K], same element kind
   int rows, N, K;
-  int bn;               // 0 = choose
+  int bn;               // 0 = choose (bf16: together with the K split)
+  int ksplit;           // set by the launcher
   int epi;
   EpiArgs e;
   // optional caller-owned scratch for the deterministic K-split of gemm_tc.cu (null: never split)
-  float* part;       // [ksplit][rows padded to 128][N padded to the tile] fp32 partial tiles
+  float* part;       // room for ksplit x (rows padded to 128) x (N padded to the tile) fp32 partial sums
   size_t part_bytes;
   int* tile_cnt;     // zero-initialised arrival counters, one per output tile
   int tile_cnt_len;

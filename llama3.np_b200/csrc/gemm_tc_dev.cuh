@@ -284,19 +284,20 @@ __device__ __forceinline__ void tc_gemm_run(TcPipe& p, const CUtensorMap* tmA0p,
           }
         }
       };
-      const int Mp = tiles_m * Cf::BM, Np = tiles_n * BN;  // padded extents of the K-split scratch
+      // K-split scratch: [k slice][output tile][column / 4][row of the tile] float4, so that a warp's 32 rows are contiguous both ways
+      const size_t slice = (size_t)ntiles_mn * (BN / 4) * Cf::BM;
+      float4* pt = reinterpret_cast<float4*>(part) + (size_t)tmn * (BN / 4) * Cf::BM + quarter * 32 + lane;
       if (ksplit > 1) {
         // K-split: publish this slice's partial tile, then the LAST slice to arrive (per output tile)
         // sums all slices in slice order - a fixed order, so the result does not depend on timing -
         // and runs the fused epilogue on the sum.
-        float* prow = part + ((size_t)ks * Mp + m0 + quarter * 32 + lane) * Np + n0;
 #pragma unroll 1
         for (int c = 0; c < BN; c += 32) {
           if (n0 + c >= N || !rows_live) break;
           float v[32];
           load_acc(c, v);
 #pragma unroll
-          for (int j = 0; j < 32; j += 4) __stcg(reinterpret_cast<float4*>(prow + c + j), make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]));
+          for (int j = 0; j < 32; j += 4) __stcg(pt + ks * slice + (size_t)((c + j) / 4) * Cf::BM, make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]));
         }
         tc_fence_before();
         __syncwarp();
@@ -361,26 +362,23 @@ __device__ __forceinline__ void tc_gemm_run(TcPipe& p, const CUtensorMap* tmA0p,
           if (ksplit == 1) {
             load_acc(c0 + cc, v);
           } else {  // sum of the slices' partials, slice 0 first
-            const float* src = part + ((size_t)(m0 + quarter * 32 + lane)) * Np + n0 + c0 + cc;
+            const float4* src = pt + (size_t)((c0 + cc) / 4) * Cf::BM;
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = 0.f;
-            // Same additions in the same order as a plain loop, so bit-identical:
-            // slice k2 + 1 is in flight while slice k2 is added - the loop below pays one L2 round trip per slice
-            // (3-8 per tile at the stories15M shapes), this one about one per tile.
-            float4 nxt[8];
+            // three slices' values are requested before the first is added (slice order: the sum does not depend on timing): one L2
+            // round trip per three slices.  With one slice ahead of the additions, and rows a tile's width apart, the reading took
+            // longer than the main loop it saved
+            for (int k2 = 0; k2 < ksplit; k2 += 3) {
+              float4 q[3][8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) nxt[j] = __ldcg(reinterpret_cast<const float4*>(src + 4 * j));
-            for (int k2 = 0; k2 < ksplit; ++k2) {
-              float4 cur[8];
+              for (int u = 0; u < 3; ++u)
 #pragma unroll
-              for (int j = 0; j < 8; ++j) cur[j] = nxt[j];
-              const size_t nk = (size_t)min(k2 + 1, ksplit - 1) * Mp * Np;  // clamped: the last prefetch is not used
+                for (int j = 0; j < 8; ++j)
+                  q[u][j] = k2 + u < ksplit ? __ldcg(src + (size_t)(k2 + u) * slice + (size_t)j * Cf::BM) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-              for (int j = 0; j < 8; ++j) nxt[j] = __ldcg(reinterpret_cast<const float4*>(src + nk + 4 * j));
+              for (int u = 0; u < 3; ++u)
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                v[4 * j] += cur[j].x; v[4 * j + 1] += cur[j].y; v[4 * j + 2] += cur[j].z; v[4 * j + 3] += cur[j].w;
-              }
+                for (int j = 0; j < 8; ++j) { v[4 * j] += q[u][j].x; v[4 * j + 1] += q[u][j].y; v[4 * j + 2] += q[u][j].z; v[4 * j + 3] += q[u][j].w; }
             }
           }
 #pragma unroll
