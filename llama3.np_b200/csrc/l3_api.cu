@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/llama3_b200.h"
+#include "cluster.h"
 #include "common.cuh"
 #include "gemm_tc.h"
 #include "internal.h"
@@ -152,7 +153,7 @@ extern "C" int l3_destroy(L3Model* m) {
   fr(m->xn_lo); fr(m->ctx_lo); fr(m->h_lo); fr(m->xlast_lo); fr(m->lm_hi); fr(m->lm_lo);
   fr(m->gemm_part); fr(m->gemm_cnt); fr(m->xn16); fr(m->ctx16); fr(m->h16); fr(m->xlast16); fr(m->q16);
   fr(m->stage); fr(m->x); fr(m->xn); fr(m->q); fr(m->ctx); fr(m->h); fr(m->xlast); fr(m->logits);
-  fr(m->d_mega_layers); fr(m->d_mega_bar); fr(m->d_mega_ll); fr(m->d_mega_dbg);
+  fr(m->d_cl_done); fr(m->d_mega_layers); fr(m->d_mega_bar); fr(m->d_mega_ll); fr(m->d_mega_dbg);
   fr(m->d_stack_layers); fr(m->d_stack_dbg); fr(m->d_stack_dbgx);
   for (auto p : m->stack_wpack) fr(p);
   fr(m->d_rowlen); fr(m->d_rowpos); fr(m->d_done); fr(m->d_lastrow);
@@ -391,11 +392,20 @@ extern "C" int l3_finalize(L3Model* m) {
     const char* env = getenv("L3_MEGA");
     m->mega_ok = !(env && atoi(env) == 0) && !(m->cfg.flags & L3_FLAG_NO_MEGA) &&
                  decode_mega_supported(m->D, m->HN, m->KVHN, m->HD, m->FD, m->VS);
-    if (m->mega_ok) {
+    // small fp32 models: a step of up to 8 sequences in one cluster (see enqueue_decode_nodes); a timeline asked for is decode_mega's
+    if (!m->bf16 && m->G == 1 && !(env && atoi(env) == 0) && !(m->cfg.flags & L3_FLAG_NO_MEGA) && !getenv("L3_MEGA_DBG"))
+      m->cl_maxB = std::min(m->maxB, decode_cluster_max_batch(m->cfg.n_layers, m->D, m->HN, m->KVHN, m->HD, m->FD, m->M));
+    if (m->mega_ok || m->cl_maxB) {
       std::vector<MegaLayer> hl;
       for (auto& L : m->layers) hl.push_back(MegaLayer{L.wqkv, L.wo, L.w13, L.w2, L.norm_in, L.norm_post, L.ck, L.cv});
       CK(m, cudaMalloc(&m->d_mega_layers, hl.size() * sizeof(MegaLayer)));
       CK(m, cudaMemcpy(m->d_mega_layers, hl.data(), hl.size() * sizeof(MegaLayer), cudaMemcpyHostToDevice));
+    }
+    if (m->cl_maxB) {
+      CK(m, cudaMalloc((void**)&m->d_cl_done, sizeof(int)));
+      CK(m, cudaMemset(m->d_cl_done, 0, sizeof(int)));
+    }
+    if (m->mega_ok) {
       CK(m, cudaMalloc((void**)&m->d_mega_bar, 64));
       CK(m, cudaMemset(m->d_mega_bar, 0, 64));
       const size_t llw = (size_t)2 * L3_LL_WORDS + (size_t)m->HN * m->HD + (size_t)2 * L3_LL_VEC;
@@ -621,6 +631,18 @@ static int tp_row_parallel(L3Model* m, LinearArgs& a, Feed feed, const float* w_
   return tp_allreduce_sum(m, m->xn, m->x, count);
 }
 
+// All layers of one token per sequence of a small fp32 model in one cluster (decode_cluster.cu); the stream lands in m->x.
+static int enqueue_cluster_layers(L3Model* m, const int32_t* d_ids, int ids_ld, int ids_off, int B) {
+  ClusterArgs a{};
+  a.layers = (const MegaLayer*)m->d_mega_layers;
+  a.NL = m->cfg.n_layers; a.D = m->D; a.HN = m->HN; a.KVHN = m->KVHN; a.HD = m->HD; a.FD = m->FD; a.M = m->M; a.B = B; a.vocab = m->cfg.vocab_size;
+  a.embed = (const float*)m->embed; a.eps = m->cfg.norm_eps; a.cos_tab = m->cos_tab; a.sin_tab = m->sin_tab;
+  a.ids = d_ids; a.ids_ld = ids_ld; a.ids_off = ids_off; a.d_next = m->d_next; a.scal = m->d_scal; a.x = m->x;
+  a.pdl = !(m->cfg.flags & L3_FLAG_NO_PDL);
+  LAUNCH(m, launch_decode_cluster(a, m->stream));
+  return L3_OK;
+}
+
 // Enqueue one chunk: tokens ids[b * ids_ld + ids_off + t], t < L, at start_pos = *d_pos.
 // Layer-list handles: d_rows / n_rows choose the rows whose logits are wanted (null: the last token of every sequence),
 // d_resid (may be null) receives the residual stream after every layer.
@@ -643,13 +665,17 @@ static int enqueue_chunk(L3Model* m, const int32_t* d_ids, int ids_ld, int ids_o
   const bool tc_rows = m->tc_ok && !linear_rows_supported(ntok, D);
   const bool tc_h = m->tc_ok && !linear_rows_supported(ntok, m->FD);
   const bool tc_ctx = m->tc_ok && !linear_rows_supported(ntok, m->HN * HD);
-  LAUNCH(m, launch_embed(m->embed, m->bf16, d_ids, ids_ld, ids_off, L, ntok, D, m->cfg.vocab_size, m->x, m->stream));
+  const bool in_cluster = L == 1 && !rg && B <= m->cl_maxB;
+  int rc;
+  if (in_cluster) {
+    if ((rc = enqueue_cluster_layers(m, d_ids, ids_ld, ids_off, B)) != L3_OK) return rc;
+  } else LAUNCH(m, launch_embed(m->embed, m->bf16, d_ids, ids_ld, ids_off, L, ntok, D, m->cfg.vocab_size, m->x, m->stream));
   EpiArgs base{};
   base.cos_tab = m->cos_tab; base.sin_tab = m->sin_tab; base.pos_ptr = d_pos;
   base.L = L; base.HD = HD; base.HN = m->HN; base.KVHN = m->KVHN; base.M = m->M;
   if (rg) { base.row_pos = rg->row_pos; base.row_len = rg->row_len; }
-  int rc;
   for (auto& Ly : m->layers) {
+    if (in_cluster) break;
     LinearArgs a{};
     // q, k, v = rope(norm(x) @ Wqkv^T); k, v -> cache            llama3.py:248, 166-187
     a.W = Ly.wqkv; a.x = m->x; a.rows = ntok; a.N = m->qkv_rows; a.K = D;
@@ -916,6 +942,20 @@ static int enqueue_decode_nodes(L3Model* m, int B, int ragged, int eos) {
     return L3_OK;
   }
   if (m->stack_ok && B >= m->stack_min_B) return enqueue_decode_stack(m, B);
+  // Small fp32 models: layers in one cluster, then the LM head with its argmax.  stories15M, 50 new tokens, us per call before (batch 1:
+  // decode_mega, 2 - 8: a kernel per product) -> here: batch 1 5874 -> 3628, 2 10105 -> 4502, 4 12632 -> 6162, 8 19323 -> 10046; 150 + 90
+  // tokens: batch 1 12316 -> 7936, 8 38394 -> 22714.  One forward step 265 -> 132, of batch 8 567 -> 313.  Larger models do not fit the
+  // cluster's shared memory (decode_cluster_max_batch); from stack_min_B sequences the clusters of decode_stack share the weights' loads.
+  if (B <= m->cl_maxB) {
+    const int rc = enqueue_cluster_layers(m, nullptr, 0, 0, B);
+    if (rc != L3_OK) return rc;
+    ClusterHeadArgs h{};
+    h.x = m->x; h.w = (const float*)m->lm_head; h.norm = m->norm_final; h.eps = m->cfg.norm_eps; h.B = B; h.D = m->D; h.VS = m->VS; h.M = m->M;
+    h.best = m->d_best; h.done = m->d_cl_done; h.d_next = m->d_next; h.d_tokens = m->d_tokens; h.scal = m->d_scal;
+    g_l3_pdl_next = !(m->cfg.flags & L3_FLAG_NO_PDL);
+    LAUNCH(m, launch_cluster_head(h, m->n_sm, m->stream));
+    return L3_OK;
+  }
   // under tensor parallelism the kernel runs the peer-memory exchange itself (needs the mapped slots)
   if (B == 1 && m->mega_ok && m->D <= L3_LL_VEC && (m->G == 1 || (m->comm && m->comm->oneshot)))
     return enqueue_decode_mega(m);

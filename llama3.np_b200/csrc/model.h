@@ -88,6 +88,8 @@ struct L3Model {
   int l2_phase = 0;
   // persistent batch-1 decode kernel (decode_mega.cu)
   bool mega_ok = false;
+  int cl_maxB = 0;                 // most sequences of the one-cluster decode step (decode_cluster.cu), 0: not this model
+  int* d_cl_done = nullptr;        // its LM head's finished CTAs, zero between steps
   int n_sm = 0;
   void* d_mega_layers = nullptr;
   unsigned* d_mega_bar = nullptr;  // [0] arrival count [1] generation [2] exchange counter (single GPU)

@@ -1,0 +1,76 @@
+"""The decode step in one cluster (decode_cluster.cu) against the oracle and against the path of a kernel per product: every batch slot
+count, rows that do not divide evenly over the CTAs, heads of 16 to 128, shared KV heads, the first and the last position of a cache and
+contexts of more keys than one turn of the attention takes."""
+import numpy as np
+import pytest
+
+from llama3_np_b200 import Llama, ModelArgs, _cabi
+from llama3_np_b200.synth import make_weights
+from oracle import ref_llama3 as orc
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = {
+    # name: (dim, layers, heads, kv_heads, hidden, vocab, max_seq)
+    "hd48": (288, 3, 6, 6, 768, 1001, 72),     # 4 or 5 fours of rows per CTA, three pieces of K
+    "hd16": (64, 2, 4, 2, 160, 96, 40),        # one four per CTA, K below a warp's turn, idle attention CTAs
+    "hd96": (192, 1, 2, 1, 200, 130, 24),      # K = 192 and 200: last turns of 16 and 18 lanes; 32 lanes per key
+    "hd128": (256, 2, 2, 1, 392, 200, 300),    # 16 keys per row of threads: several turns over 300 positions
+    "hd32": (128, 1, 4, 1, 264, 64, 512),      # eight lanes of 16 per key, the longest cache it takes
+}
+
+
+def _args(name, B):
+    d, nl, hn, kv, hid, vs, msl = SHAPES[name]
+    args = ModelArgs(dim=d, n_layers=nl, n_heads=hn, n_kv_heads=kv, vocab_size=vs, max_seq_len=msl, max_batch_size=B)
+    return args, make_weights(args, hid, seed=5)
+
+
+@pytest.mark.parametrize("B", [1, 2, 3, 4, 8])
+@pytest.mark.parametrize("name", list(SHAPES))
+def test_steps_match_the_oracle(name, B):
+    """Forward steps at position 0, at the edges of the attention's turns and at the last position; fp32 against the fp32 oracle: sums
+    of K <= 768 terms differ by their order only, K eps / 2 = 5e-5 of the largest value at the worst."""
+    args, w = _args(name, B)
+    M = args.max_seq_len
+    rng = np.random.default_rng(B)
+    ids = rng.integers(0, args.vocab_size, (B, M))
+    m, o, m2 = Llama(w, args), orc.OracleLlama(w, args), Llama(w, args, flags=_cabi.FLAG_NO_MEGA)
+    tol = lambda want: 5e-5 * np.abs(want).max()
+
+    def check(lo, hi):
+        want = np.asarray(o(ids[:, lo:hi], lo))
+        got, ref = np.asarray(m(ids[:, lo:hi], lo)), np.asarray(m2(ids[:, lo:hi], lo))
+        np.testing.assert_allclose(got, want, rtol=0, atol=tol(want))
+        np.testing.assert_allclose(got, ref, rtol=0, atol=tol(want))
+
+    edges = sorted({p for p in (1, 31, 32, 33, 63, 64, 127, 128, 129, 255, 256, 257, M - 2, M - 1) if p < M})
+    check(0, 1)
+    at = 1
+    for p in edges:
+        if p < at:
+            continue
+        if p > at:
+            check(at, p)
+        check(p, p + 1)
+        at = p + 1
+    for li in range(args.n_layers):
+        for a, b in zip(m.read_cache(li), m2.read_cache(li)):
+            np.testing.assert_allclose(a, b, rtol=0, atol=tol(b))
+    m.close()
+    m2.close()
+
+
+@pytest.mark.parametrize("B", [1, 2, 3, 5, 8])
+@pytest.mark.parametrize("name", ["hd48", "hd16", "hd96"])
+def test_greedy_tokens_match_the_oracle(name, B):
+    args, w = _args(name, B)
+    ids = np.random.default_rng(3).integers(0, args.vocab_size, (B, 5))
+    cap = args.max_seq_len
+    want = np.concatenate(list(orc.OracleLlama(w, args).generate(ids, cap)), axis=1)
+    m = Llama(w, args)
+    for _ in range(2):  # the head's counters are back at zero behind a run
+        assert np.array_equal(m.generate_all(ids, cap), want)
+        m.reset_cache()
+    assert np.array_equal(np.concatenate(list(m.generate(ids, cap)), axis=1), want)
+    m.close()
