@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(256) win_prep_kernel(WinPrepArgs a) {
     KVT* ck = (KVT*)a.cache_k + (((size_t)b * a.G + g) * a.M + pos) * a.DK;
     float* qf = a.q_out ? a.q_out + ((size_t)r * a.H + v) * a.DK : nullptr;
     bf16* qp = a.q16 ? a.q16 + ((size_t)r * a.H + v) * a.q16_parts * a.q16_ld : nullptr;
-    bf16* ql = a.q16_parts == 2 ? qp + a.q16_ld : nullptr;  // what the first part leaves
+    bf16* ql = qp && a.q16_parts == 2 ? qp + a.q16_ld : nullptr;  // what the first part leaves
     auto put_q4 = [&](int i, float x0, float x1, float x2, float x3) {
       put4(qp + i, x0, x1, x2, x3);
       if (ql) put4(ql + i, bf16_rest(x0), bf16_rest(x1), bf16_rest(x2), bf16_rest(x3));
