@@ -951,9 +951,12 @@ static int ll_reset_unit_state(L3Model* m, const L3LayerSpec& s, LLState& St, in
 }
 
 // do prompts of this latent-attention layer run on the tensor cores?
+static bool ll_latent_expands_on() {
+  static const bool on = !(getenv("L3_LATENT_TC") && atoi(getenv("L3_LATENT_TC")) == 0);
+  return on;
+}
 static bool ll_latent_on_tc(const L3Model* m, const L3LayerSpec& s) {
-  static const bool off = getenv("L3_LATENT_TC") && atoi(getenv("L3_LATENT_TC")) == 0;
-  return !off && m->tc_ok && s.mixer == L3_MIX_LATENT && s.scale > 0.f && s.kv_rank + s.rot_dim >= 64 && s.heads * (s.dim + s.vdim) >= 64 &&
+  return ll_latent_expands_on() && m->tc_ok && s.mixer == L3_MIX_LATENT && s.scale > 0.f && s.kv_rank + s.rot_dim >= 64 && s.heads * (s.dim + s.vdim) >= 64 &&
          latent_tc_supported(s.dim, s.rot_dim, s.vdim, s.kv_rank);
 }
 
@@ -964,7 +967,7 @@ static bool ll_latent_on_tc(const L3Model* m, const L3LayerSpec& s) {
 // a short portion behind a long prefix would expand the whole prefix for little, so it starts there.
 constexpr int LATENT_F32_MIN = 64;
 static bool ll_latent_expands_f32(const L3Model* m, const L3LayerSpec& s) {
-  return !m->bf16 && m->ll->f32_tc && s.mixer == L3_MIX_LATENT && s.dim % 8 == 0 && s.rot_dim % 8 == 0 && s.vdim % 8 == 0 && s.kv_rank % 8 == 0 &&
+  return ll_latent_expands_on() && !m->bf16 && m->ll->f32_tc && s.mixer == L3_MIX_LATENT && s.dim % 8 == 0 && s.rot_dim % 8 == 0 && s.vdim % 8 == 0 && s.kv_rank % 8 == 0 &&
          s.heads * (s.dim + s.vdim) >= 64 && s.kv_rank + s.rot_dim >= 64 && win_attn_supported(s.dim + s.rot_dim, s.vdim);
 }
 

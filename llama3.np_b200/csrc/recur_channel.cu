@@ -20,6 +20,7 @@
 // products - keys, queries, scores, T, U and the state - are pairs hi + lo of bf16 values (16 significant bits), a product is
 // hi hi + hi lo + lo hi with fp32 accumulation; the inverse is fp32.
 #include <stdint.h>
+#include <stdlib.h>
 
 #include <algorithm>
 
@@ -494,7 +495,8 @@ size_t recur_channel_ws_floats(int B, int L, int H, int DK, int DV) {
 }
 
 bool recur_channel_supported(const RecurArgs& a) {
-  if (!a.bf16_ops || a.n_state || a.k_scale || !a.ws || a.L < RECUR_CHANNEL_MIN || !recur_channel_shape(a.DK, a.DV)) return false;
+  static const bool on = !(getenv("L3_RECUR_CHUNK") && atoi(getenv("L3_RECUR_CHUNK")) == 0);
+  if (!on || !a.bf16_ops || a.n_state || a.k_scale || !a.ws || a.L < RECUR_CHANNEL_MIN || !recur_channel_shape(a.DK, a.DV)) return false;
   if (a.mode == 0 ? a.head_decay == nullptr : a.log_c == nullptr && !(a.mode == 2 && a.log_g)) return false;
   const uintptr_t al = (uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.log_c | (uintptr_t)a.ws;
   if (a.ld_q % 4 || a.ld_k % 4 || (al & 15)) return false;
