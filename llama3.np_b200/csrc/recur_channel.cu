@@ -100,8 +100,9 @@ __global__ void __launch_bounds__(512) channel_chunk_kernel(RecurArgs a, int c0)
         kv = *reinterpret_cast<const float4*>(ks + (size_t)t * a.ld_k + d);
         if (a.log_c) lv = *reinterpret_cast<const float4*>(a.log_c + (row0 + t) * a.H * DK + (size_t)h * DK + d);
         else { const float l = a.log_g ? a.log_g[(row0 + t) * a.H + h] : fixed; lv = make_float4(l, l, l, l); }
-        // a decay of zero: far below every exponential, but finite
-        lv.x = lv.x < -1e30f ? -1e30f : lv.x; lv.y = lv.y < -1e30f ? -1e30f : lv.y; lv.z = lv.z < -1e30f ? -1e30f : lv.z; lv.w = lv.w < -1e30f ? -1e30f : lv.w;
+        // From -104 on a decay is zero in fp32.  Stronger ones are held at -110: the decays of the tokens behind them are differences
+        // of running sums, which are right to 2^-14 of a unit that way (a block's stay above -16 x 110), with one such token to 2^-18
+        lv.x = lv.x < -110.f ? -110.f : lv.x; lv.y = lv.y < -110.f ? -110.f : lv.y; lv.z = lv.z < -110.f ? -110.f : lv.z; lv.w = lv.w < -110.f ? -110.f : lv.w;
         if (a.act_in) {
           qv.x = act_silu(a.act_in, qv.x); qv.y = act_silu(a.act_in, qv.y); qv.z = act_silu(a.act_in, qv.z); qv.w = act_silu(a.act_in, qv.w);
           kv.x = act_silu(a.act_in, kv.x); kv.y = act_silu(a.act_in, kv.y); kv.z = act_silu(a.act_in, kv.z); kv.w = act_silu(a.act_in, kv.w);

@@ -61,3 +61,43 @@ def test_gated_linear_attention(n, batch, heads, dim, vdim, rate):
     # the rounding of its bf16 projections is off by order one whatever the kernel does (the chain is 0.230 off on 200 tokens, the
     # chunks 0.230 off, the two 0.002 apart).  Those cases are held to the chain alone.
     _check(m, o, cfg["vocab"], n, batch, lambda o, ids: (deb.fresh(o), o.run(ids))[1], oracle=rate != "fast")
+
+
+def _forget(t, a1, a2, embed, token, z):
+    """One token (and no other) adds z to the decay logits of all channels of a layer: rank 0 of the decay's two matrices reads an
+    embedding entry that only this token has."""
+    t[embed][:, 0] = 0.0
+    t[embed][token, 0] = 1.0
+    t[a1][0] = 0.0
+    t[a1][0, 0] = 1.0
+    t[a2][:, 0] = z
+    return t
+
+
+def _check_forget(m, o, vocab, token, run):
+    ids = np.random.default_rng(4).integers(0, vocab - 1, 150)
+    ids[[3, 20, 85, 86]] = token    # the tokens behind it in the same block of 16 keep their own decays
+    whole = m.forward_rows(ids[None], 0, list(range(150)))
+    parts = np.concatenate([m.forward_rows(ids[None, p:p + 40], p, list(range(len(ids[p:p + 40])))) for p in range(0, 150, 40)])
+    m.close()
+    assert deb.err(whole, run(o, ids)) < 6e-2
+    assert deb.err(whole, parts) < 1e-2
+
+
+@pytest.mark.parametrize("strength", [-30.0, -200.0, -1e5, -1e7, -3e38])
+def test_delta_rule_behind_a_token_that_empties_its_channels(strength):
+    cfg = ris.config([ris.delta(2, 2, 64, 64, 2, ff=96), ris.delta(2, 1, 128, 32, 2)], width=96, side=0)
+    t = _rates(ris.random_model(cfg, 8), "mixed")
+    t = _forget(t, "l0.mix.a1", "l0.mix.a2", "embed", cfg["vocab"] - 1, -strength)  # log decay = -softplus(dt)
+    m, o = ris.build(cfg, dtype="bfloat16", max_seq_len=152, tensors=t)
+    _check_forget(m, o, cfg["vocab"], cfg["vocab"] - 1, lambda o, ids: o.run(ids))
+
+
+@pytest.mark.parametrize("strength", [-30.0, -200.0, -1e5, -1e7, -3e38])
+def test_gated_linear_attention_behind_a_token_that_empties_its_channels(strength):
+    cfg = deb.config([deb.gla(2, 64, 64, tau=2.0, mlp={"kind": "dense", "ff": 96})], width=96)
+    t = _rates(deb.random_tensors(cfg, 9), "mixed")
+    t = _forget(t, "l0.mix.a1", "l0.mix.a2", "embed", cfg["vocab"] - 1, strength)   # log decay = -softplus(-z) / tau
+    t["l0.shift"][:] = 0.0                                 # the layer reads this token's row alone
+    m, o = deb.build(cfg, dtype="bfloat16", max_seq_len=152, tensors=t)
+    _check_forget(m, o, cfg["vocab"], cfg["vocab"] - 1, lambda o, ids: (deb.fresh(o), o.run(ids))[1])
