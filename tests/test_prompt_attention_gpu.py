@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 import test_debuzen_gpu as deb
+import test_gifudra_gpu as gif
 import test_mabedra_gpu as mab
 import test_risalix_gpu as ris
 
@@ -53,3 +54,47 @@ def test_windows_with_kept_tokens(n, more, kind, heads, kv, dim, vdim, size, kee
     m, o = deb.build(cfg, 5, "bfloat16", max_seq_len=n + more + 3)
     got, want = _run(m, o, n, more, cfg["vocab"], lambda o, ids: (deb.fresh(o), o.run(ids))[1])
     assert deb.err(got, want) < 6e-2
+
+
+def _family(kind):
+    """test module of the family, configuration, its random weights, an oracle run from a fresh state"""
+    if kind == "softmax":
+        return ris, ris.config([ris.attn(4, 2, 64, 0.125), ris.attn(2, 1, 72, 0.2)], width=128, side=0), ris.random_model, lambda o, ids: o.run(ids)
+    if kind == "differential":
+        cfg = mab.config([mab.attn(2, 1, 64, 128, window=70, scale=0.125, mlp=mab.dense(128))] * 2, width=128)
+        return mab, cfg, mab.random_model, lambda o, ids: (mab.fresh(o), o.run(ids))[1]
+    if kind == "latent":
+        cfg = gif.config([gif.latent(heads=2, dim=64, rot_dim=16, vdim=72, kv_rank=64, scale=0.125, ff=64)], width=128)
+        return gif, cfg, gif.random_model, lambda o, ids: (o.reset(), o.run(ids))[1]
+    left = deb.attn(4, 2, 64, 64, size=23, keep_first=None if kind == "window" else 3, dims=32, scale=0.125)
+    mlp = {"kind": "dense", "ff": 128}
+    layer = deb.par(left=left, mlp=mlp) if kind == "sigmoid" else deb.par2(left=left, mlp=mlp)
+    return deb, deb.config([layer, layer], width=96), deb.random_tensors, lambda o, ids: (deb.fresh(o), o.run(ids))[1]
+
+
+@pytest.mark.parametrize("kind", ["softmax", "differential", "sigmoid", "sink", "window", "latent"])
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+def test_rows_that_no_query_sees_do_not_count(kind, value):
+    """Infinities and NaN in cache rows behind a sequence's own: left by an earlier, longer request of the slot, and in the rows of the
+    next head and the next sequence, which the last key block of a full cache reaches into (100 rows are no multiple of 64)."""
+    M = 100
+    fam, cfg, tensors, run = _family(kind)
+    t = tensors(cfg, 12)
+    big = cfg["vocab"] - 1
+    t["embed"][big] = value
+    m, o = fam.build(cfg, dtype="bfloat16", max_seq_len=M, max_batch_size=2, tensors=t)
+    rng = np.random.default_rng(11)
+    ids = rng.integers(0, big, (2, M))
+    spoiled = ids.copy()
+    spoiled[:, [25, 40, 70]] = big
+    assert not np.isfinite(m.forward_rows(spoiled[:, :90], 0, [70, 160])).any()
+    # the slots again, shorter, the second portion with kept tokens in a block of their own
+    got = np.concatenate([m.forward_rows(ids[:, :20], 0, list(range(40))).reshape(2, 20, -1),
+                          m.forward_rows(ids[:, 20:34], 20, list(range(28))).reshape(2, 14, -1)], 1)
+    for b in range(2):
+        assert ris.err(got[b][:, :big], run(o, ids[b, :34])[:, :big]) < 6e-2   # (a tied output projection has the token's row, too)
+    # a sequence that fills its cache, ahead of one that is spoiled
+    ids[1, [5, 20]] = big
+    got = m.forward_rows(ids, 0, list(range(M)))
+    assert ris.err(got[:, :big], run(o, ids[0])[:, :big]) < 6e-2
+    m.close()
