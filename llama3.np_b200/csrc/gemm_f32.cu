@@ -14,10 +14,13 @@
 // step is converted while the previous one is multiplied.  Bound by the MMAs: an M = 128 instruction takes ~132 cycles for N = 128 as
 // for N = 256 (mma_probe.cu), 12 of them per step against ~600 issue slots of conversion per scheduler; a 256-wide tile would halve
 // that but its parts and raw tiles do not fit the shared memory together.
+// An infinite operand leaves NaN behind (its parts are inf, NaN, NaN; inf times a zero part is NaN too): sums that end as NaN are
+// taken again as a plain chain of fp32 products, so that an infinity gives what it gives there.
 // Every wait is bounded: one that runs out sets a flag, all warps run on without waiting, and the host reports an error.
 #include <cuda.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "gemm_tc.h"
@@ -98,13 +101,21 @@ __device__ __forceinline__ void cut8(const float4& x, const float4& y, uint4& p1
   }
 }
 
+// a . w in fp32, until it is NaN
+template <typename WT>
+__device__ float plain_dot(const float* a, const WT* w, int K) {
+  float s = 0.f;
+  for (int k = 0; k < K && s == s; ++k) s = fmaf(a[k], to_f32(w[k]), s);
+  return s;
+}
+
 template <bool WB16> constexpr int raw_bytes() { return WB16 ? HALF : 2 * HALF; }
 template <bool WB16> constexpr int smem_bytes() { return 1024 + 3 * HALF + (WB16 ? WST : 3) * HALF + RAW * raw_bytes<WB16>() + 512; }
 
 template <bool WB16, int EPI>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, int rows, int N, int K, int ksplit, float* part,
-                int* tile_cnt, int* err, EpiArgs e) {
+                int* tile_cnt, int* err, const float* A, int lda, const void* W, EpiArgs e) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sA = (raw + 1023u) & ~1023u, sW = sA + 3 * HALF, sR = sW + (WB16 ? WST : 3) * HALF, bars = sR + RAW * raw_bytes<WB16>();
@@ -297,6 +308,16 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
       }
       if (m >= rows) continue;
+      uint64_t odd = 0;
+#pragma unroll
+      for (int j = 0; j < 64; ++j) odd |= (uint64_t)(run[j] != run[j]) << j;
+      for (; odd; odd &= odd - 1) {
+        const int c = __ffsll(odd) - 1;
+        if (nc + c >= N) break;
+        const float v = plain_dot(A + (size_t)m * lda, reinterpret_cast<const std::conditional_t<WB16, bf16, float>*>(W) + (size_t)(nc + c) * K, K);
+#pragma unroll
+        for (int j = 0; j < 64; ++j) run[j] = j == c ? v : run[j];
+      }
       const bool plain = !e.out_lo && !e.out_bf16 && !e.glu_w && !(e.ld_out & 3) && !(N & 3);
 #pragma unroll
       for (int j = 0; j < 64; j += 4) {
@@ -362,7 +383,7 @@ cudaError_t launch_t(const GemmF32Args& a, cudaStream_t s) {
     }
   }
   return launch_k(kern, dim3(std::min(tiles * ksplit, sms)), dim3(THREADS), (size_t)smem_bytes<WB16>(), s, *ma, *mw, a.rows, a.N, a.K, ksplit, a.part,
-                  a.tile_cnt, a.err, a.e);
+                  a.tile_cnt, a.err, a.A, a.lda ? a.lda : a.K, a.W, a.e);
 }
 
 template <bool WB16>

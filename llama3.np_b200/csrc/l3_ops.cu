@@ -112,6 +112,21 @@ extern "C" int l3_op_linear(int device, const float* x, const float* w, int rows
     tc_forget_maps();  // the scratch buffers are about to be freed
     if (rc == L3_OK) cudaMemcpy(out, dout, (size_t)rows * n * 4, cudaMemcpyDeviceToHost);
     return rc;
+  } else if (path == 5) {  // fp32 operands (or fp32 rows and a bf16 matrix) cut into bf16 parts, fp32 precision
+    GemmF32Args t{};
+    t.A = dx; t.W = dw; t.w_bf16 = w_bf16 != 0; t.rows = rows; t.N = n; t.K = k; t.epi = EPI_STORE; t.e = a.e;
+    t.part_bytes = (size_t)32 << 20;
+    t.part = sc.dev<float>(t.part_bytes / 4);
+    t.tile_cnt = sc.dev<int>(1024); t.tile_cnt_len = 1024;
+    t.err = sc.dev<int>(1);
+    if (!t.part || !t.tile_cnt || !t.err) return L3_ENOMEM;
+    if (cudaMemsetAsync(t.tile_cnt, 0, 1024 * sizeof(int), sc.s) != cudaSuccess || cudaMemsetAsync(t.err, 0, sizeof(int), sc.s) != cudaSuccess) return L3_ECUDA;
+    if (!gemm_f32_supported(t)) return L3_EINVAL;
+    int rc = finish(sc, launch_gemm_f32(t, sc.s)), err = 0;
+    tc_forget_maps();
+    if (rc == L3_OK) cudaMemcpy(&err, t.err, sizeof err, cudaMemcpyDeviceToHost);
+    if (rc == L3_OK) cudaMemcpy(out, dout, (size_t)rows * n * 4, cudaMemcpyDeviceToHost);
+    return err ? L3_ESTATE : rc;
   } else {
     return L3_EINVAL;
   }

@@ -48,3 +48,29 @@ def test_gated_units_and_strided_second_projections(dtype):
     m.close()
     assert ris.err(whole, want) < (2e-5 if dtype == "float32" else 6e-2)
     assert ris.err(whole, parts) < (2e-5 if dtype == "float32" else 1e-2)
+
+
+def _product(x, w, bf16):
+    from llama3_np_b200 import _cabi
+    out = np.empty((len(x), len(w)), np.float32)
+    _cabi.check(_cabi.lib().l3_op_linear(0, _cabi.f32p(x), _cabi.f32p(w), len(x), len(w), x.shape[1], 5, int(bf16), _cabi.f32p(out)))
+    return out
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("rows,n,k", [(9, 64, 64), (130, 260, 320), (128, 128, 4096)])
+def test_infinities_and_nan(rows, n, k, bf16):
+    """Infinities and NaN in the rows and in the matrix give what they give in a plain sum (an infinity of the sign of the products, NaN
+    for a sum of both signs or for a zero); results without them are as exact as ever.  With and without a K split."""
+    rng = np.random.default_rng(k)
+    x, w = rng.standard_normal((rows, k)).astype(np.float32), (rng.integers(-64, 65, (n, k)) / 64).astype(np.float32)  # bf16 numbers, some 0
+    x[1, 5], x[2, k - 1], x[3, [0, 7]], x[4, 9], x[rows - 1, 31] = np.inf, -np.inf, [np.inf, -np.inf], np.nan, 3e38
+    w[3, 2], w[n - 1, 33], w[7, 1] = np.inf, -np.inf, np.nan
+    got = _product(x, w, bf16)
+    with np.errstate(all="ignore"):
+        want = np.stack([(x[i].astype(np.float64) * w).sum(-1) for i in range(rows)])
+    want32 = want.astype(np.float32)
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(got[np.isinf(want32)], want32[np.isinf(want32)])
+    fine = np.isfinite(want32)
+    fine[-1] = False
+    assert np.abs(got[fine] - want[fine]).max() < 6e-7 * np.sqrt(k) * 4
