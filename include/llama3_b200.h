@@ -395,6 +395,10 @@ int l3_debug_mega_timeline(L3Model* m, uint64_t* out, int64_t capacity);
  * which 1: float [n_layers][max_batch_size][dim], the residual stream after every layer. */
 int l3_debug_stack(L3Model* m, int which, void* out, int64_t capacity_bytes);
 
+/* Debug: sets the word that a kernel sets when one of its bounded waits runs out, so that the next call that waits for the
+ * GPU reports it (for tests of the host side).  L3_EINVAL for a handle none of whose kernels reports its waits. */
+int l3_debug_fail_wait(L3Model* m);
+
 /* Micro-benchmark of the row-streaming GEMV (y = W x, W [n, k]) at one shape, weights rotated
  * over more copies than fit the L2: average ms per launch over `iters` launches. */
 int l3_bench_gemv(int device, int n, int k, int w_bf16, int rows, int iters, float* avg_ms);

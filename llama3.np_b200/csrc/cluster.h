@@ -18,6 +18,7 @@ struct ClusterArgs {
   const int32_t* d_next;
   const int* scal;
   float* x;                          // [B, D] the residual stream behind the last layer
+  int* err;                          // mapped host memory: set to 1 when a wait inside the kernel ran out
   bool pdl;                          // starts in its predecessor's tail: weights are drawn ahead
 };
 struct ClusterHeadArgs {             // next = argmax(norm(x) W^T), then the step's bookkeeping

@@ -58,7 +58,8 @@ __device__ __forceinline__ uint32_t s32(const void* p) { return (uint32_t)__cvta
 __device__ __forceinline__ void bar_arm(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// False: gave up.  The kernel then runs on without waiting and writes NaN, so that nobody hangs and the result shows it.
+// False: gave up.  The thread then waits no more, its CTA leaves the layers at the next barrier of all its threads, the others run out of
+// data and do the same, and the host finds the error word.
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, bool ok) {
   uint32_t done = 0;
   for (uint32_t n = ok ? 1u << 22 : 1u; !done && n; --n)
@@ -272,7 +273,7 @@ __global__ void __launch_bounds__(TH, 1) decode_cluster_kernel(const __grid_cons
     const uint32_t par = li & 1;
     auto wait = [&](int p) {  // all outputs of phase p are here
       ok = bar_wait(bar0 + 8 * (p - 1), par, ok);
-      if (tid == 0 && more) bar_arm(bar0 + 8 * (p - 1), bytes[p - 1]);
+      if (tid == 0 && more && ok) bar_arm(bar0 + 8 * (p - 1), bytes[p - 1]);
     };
     auto refill = [&] { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); };  // all reads lie behind a barrier: before the next copy
     // ---- 1
@@ -281,7 +282,8 @@ __global__ void __launch_bounds__(TH, 1) decode_cluster_kernel(const __grid_cons
     if (n1 <= 4 * NW) gemv<NB, 4, true>(sA + D, n1, D, pd, x, sA, a.eps, out());
     else gemv<NB, 6, true>(sA + D, n1, D, pd, x, sA, a.eps, out());
     if (NB > 2) fetch(ly, it_b, it_h, 0);
-    __syncthreads();
+    ok = __syncthreads_and(ok);
+    if (!ok) break;
     {
       float* o = out();
       if (act1) {
@@ -296,7 +298,7 @@ __global__ void __launch_bounds__(TH, 1) decode_cluster_kernel(const __grid_cons
       send_rows(o, n1, s32(qkv + f1), QKV, 1);
       flip ^= 1;
     }
-    if (tid == 0) { refill(); load4(ly); }
+    if (tid == 0 && ok) { refill(); load4(ly); }
     wait(1);
     // ---- 2: keys of the cache from registers, this step's from the exchange.  Every warp keeps the running maximum of its own keys.
     {
@@ -401,7 +403,7 @@ __global__ void __launch_bounds__(TH, 1) decode_cluster_kernel(const __grid_cons
     gemv<NB, 4, false>(sB, n3, qc, p3, att, nullptr, 0.f, out());
     __syncthreads();
     add_rows(3, ks3);
-    if (tid == 0) { refill(); load5(ly); }
+    if (tid == 0 && ok) { refill(); load5(ly); }
     wait(3);
     // ---- 4
     ok = bar_wait(barA, 1, ok);
@@ -419,21 +421,23 @@ __global__ void __launch_bounds__(TH, 1) decode_cluster_kernel(const __grid_cons
       send_rows(o, nh, s32(qkv + fh), FD, 4);
       flip ^= 1;
     }
-    if (tid == 0 && more) { refill(); load1(tab[li + 1]); }
+    if (tid == 0 && more && ok) { refill(); load1(tab[li + 1]); }
     wait(4);
     // ---- 5
     ok = bar_wait(barB, 1, ok);
     gemv<NB, 4, false>(sB, n3, FD, p5, qkv, nullptr, 0.f, out());
     __syncthreads();
     add_rows(5, ks5);
-    if (tid == 0 && more) { refill(); load3(tab[li + 1]); }
+    if (tid == 0 && more && ok) { refill(); load3(tab[li + 1]); }
     wait(5);
   }
   for (int i = tid; i < n3 * B; i += TH) {
     const int b = i / n3, row = i % n3;
-    a.x[(size_t)b * D + f3 + row] = ok ? x[b * D + f3 + row] : NAN;
+    a.x[(size_t)b * D + f3 + row] = x[b * D + f3 + row];
   }
+  if (!ok) *a.err = 1;
   cl.sync();  // nobody leaves while something is on its way to it
+  if (!ok) __nanosleep(1000000);  // what this CTA did not wait for lands before its shared memory is given up
 }
 
 // LM head and argmax: four rows of W per warp and turn, eight lanes per row; the CTA that finishes last settles the step.  Bound by the

@@ -5,6 +5,8 @@
 #include "model.h"
 
 void set_err(L3Model* m, const char* fmt, ...);  // l3_api.cu
+int make_err_word(L3Model* m);                   // L3Model::h_err
+int check_waits(L3Model* m);                     // behind a synchronisation: did a kernel of the calls before it give up waiting?
 extern const bool g_l3_debug_sync;               // L3_DEBUG_SYNC=1: synchronise after every launch
 
 #define CK(m, call)                                                                         \

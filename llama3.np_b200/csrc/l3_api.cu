@@ -130,6 +130,26 @@ extern "C" int l3_create(const L3Config* c, L3Model** out) {
   return L3_OK;
 }
 
+int make_err_word(L3Model* m) {
+  CK(m, cudaHostAlloc((void**)&m->h_err, sizeof(int), cudaHostAllocMapped));
+  *m->h_err = 0;
+  return L3_OK;
+}
+
+int check_waits(L3Model* m) {
+  if (!m->h_err || !*(volatile int*)m->h_err) return L3_OK;
+  *m->h_err = 0;
+  set_err(m, "a kernel gave up waiting for its own pipeline; the results of this call are not valid");
+  return L3_ESTATE;
+}
+
+extern "C" int l3_debug_fail_wait(L3Model* m) {
+  if (!m || !m->finalized) return L3_ESTATE;
+  REQUIRE(m, m->h_err != nullptr, "no kernel of this handle reports its waits");
+  *m->h_err = 1;
+  return L3_OK;
+}
+
 extern "C" int l3_destroy(L3Model* m) {
   if (!m) return L3_OK;
   cudaSetDevice(m->cfg.device);
@@ -159,6 +179,7 @@ extern "C" int l3_destroy(L3Model* m) {
   fr(m->d_rowlen); fr(m->d_rowpos); fr(m->d_done); fr(m->d_lastrow);
   fr(m->part_o); fr(m->part_ml); fr(m->attn_cnt); fr(m->d_ids); fr(m->d_fwd_ids); fr(m->d_next); fr(m->d_fwd_next); fr(m->d_scal); fr(m->d_tokens); fr(m->d_fwd_arg); fr(m->d_best); fr(m->l2buf);
   if (m->h_next) cudaFreeHost(m->h_next);
+  if (m->h_err) cudaFreeHost(m->h_err);
   if (m->ev0) cudaEventDestroy(m->ev0);
   if (m->ev1) cudaEventDestroy(m->ev1);
   if (m->stream) cudaStreamDestroy(m->stream);
@@ -404,6 +425,7 @@ extern "C" int l3_finalize(L3Model* m) {
     if (m->cl_maxB) {
       CK(m, cudaMalloc((void**)&m->d_cl_done, sizeof(int)));
       CK(m, cudaMemset(m->d_cl_done, 0, sizeof(int)));
+      if (const int rc = make_err_word(m)) return rc;
     }
     if (m->mega_ok) {
       CK(m, cudaMalloc((void**)&m->d_mega_bar, 64));
@@ -638,7 +660,7 @@ static int enqueue_cluster_layers(L3Model* m, const int32_t* d_ids, int ids_ld, 
   a.NL = m->cfg.n_layers; a.D = m->D; a.HN = m->HN; a.KVHN = m->KVHN; a.HD = m->HD; a.FD = m->FD; a.M = m->M; a.B = B; a.vocab = m->cfg.vocab_size;
   a.embed = (const float*)m->embed; a.eps = m->cfg.norm_eps; a.cos_tab = m->cos_tab; a.sin_tab = m->sin_tab;
   a.ids = d_ids; a.ids_ld = ids_ld; a.ids_off = ids_off; a.d_next = m->d_next; a.scal = m->d_scal; a.x = m->x;
-  a.pdl = !(m->cfg.flags & L3_FLAG_NO_PDL);
+  a.err = m->h_err; a.pdl = !(m->cfg.flags & L3_FLAG_NO_PDL);
   LAUNCH(m, launch_decode_cluster(a, m->stream));
   return L3_OK;
 }
@@ -821,7 +843,7 @@ extern "C" int l3_forward(L3Model* m, const int32_t* ids, int B, int L, int star
   if (argmax_out)
     CK(m, cudaMemcpyAsync(argmax_out, m->d_fwd_arg, (size_t)B * 8, cudaMemcpyDeviceToHost, m->stream));
   CK(m, cudaStreamSynchronize(m->stream));
-  return ll_check(m);
+  return check_waits(m);
 }
 
 extern "C" int l3_forward_rows(L3Model* m, const int32_t* ids, int B, int L, int start_pos, const int32_t* rows, int n_rows,
@@ -857,7 +879,7 @@ extern "C" int l3_forward_rows(L3Model* m, const int32_t* ids, int B, int L, int
   if (rc != L3_OK) return rc;
   CK(m, e);
   CK(m, e2);
-  return ll_check(m);
+  return check_waits(m);
 }
 
 // ------------------------------------------------------------------------------ greedy loop
@@ -1041,7 +1063,7 @@ extern "C" int l3_generate_greedy(L3Model* m, const int32_t* ids, int B, int L, 
   CK(m, cudaMemcpy2DAsync(out, (size_t)n_out * 8, m->d_tokens, (size_t)m->M * 8, (size_t)n_out * 8, B,
                           cudaMemcpyDeviceToHost, m->stream));
   CK(m, cudaStreamSynchronize(m->stream));
-  return ll_check(m);
+  return check_waits(m);
 }
 
 // Greedy generation for prompts of DIFFERENT lengths (the reference handles equal
@@ -1128,7 +1150,7 @@ extern "C" int l3_generate_next(L3Model* m, int64_t* out_B) {
   CK(m, cudaMemcpyAsync(m->h_next, m->d_next, (size_t)m->gen_B * 4, cudaMemcpyDeviceToHost, m->stream));
   CK(m, cudaStreamSynchronize(m->stream));
   for (int b = 0; b < m->gen_B; ++b) out_B[b] = m->h_next[b];
-  return ll_check(m);
+  return check_waits(m);
 }
 
 // ------------------------------------------------------------------------------ measurement helpers
@@ -1136,7 +1158,7 @@ extern "C" int l3_sync(L3Model* m) {
   if (!m) return L3_EINVAL;
   CK(m, cudaSetDevice(m->cfg.device));
   CK(m, cudaStreamSynchronize(m->stream));
-  return ll_check(m);
+  return check_waits(m);
 }
 extern "C" int l3_timer_start(L3Model* m) {
   if (!m) return L3_EINVAL;

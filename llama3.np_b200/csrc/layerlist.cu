@@ -1192,8 +1192,7 @@ int ll_finalize(L3Model* m) {
     if (ll->hf) CK(m, cudaMalloc(&ll->hf16, ct * W * 2));
     if (ll->cat) CK(m, cudaMalloc(&ll->cat16, ct * 2 * W * 2));
   }
-  CK(m, cudaHostAlloc((void**)&ll->h_err, sizeof(int), cudaHostAllocMapped));
-  *ll->h_err = 0;
+  if (const int rc = make_err_word(m)) return rc;
   size_t q_ld = 0, e_ld = 0;
   for (auto& L : ll->layers)
     if (ll_latent_on_tc(m, L.spec)) {
@@ -1287,7 +1286,6 @@ void ll_destroy(L3Model* m) {
   fr(ll->diff_part_o); fr(ll->diff_part_ml);
   fr(ll->Xs); fr(ll->hn); fr(ll->hf); fr(ll->hf16); fr(ll->y1); fr(ll->y2); fr(ll->moe_gu);
   fr(ll->lat_q16); fr(ll->win_q16); fr(ll->diff_maps); fr(ll->lat_exp); fr(ll->lat_part_o); fr(ll->lat_part_ml);
-  if (ll->h_err) cudaFreeHost(ll->h_err);
   fr(ll->loop_step); fr(ll->qlat); fr(ll->aux16); fr(ll->moe_sel); fr(ll->moe_w); fr(ll->moe_dense); fr(ll->moe_idw);
   fr(ll->pin); fr(ll->aux); fr(ll->rk); fr(ll->rv); fr(ll->rg); fr(ll->rbeta); fr(ll->o); fr(ll->sg); fr(ll->sg16); fr(ll->x2); fr(ll->chunk_ws);
   delete ll;
@@ -1338,13 +1336,6 @@ int ll_reset_slots(L3Model* m, int slot0, int n, bool kv_too) {
   }
   for (int b = slot0; b < slot0 + n; ++b) ll->slot_pos[b] = 0;
   return L3_OK;
-}
-
-int ll_check(L3Model* m) {
-  if (!m->ll || !m->ll->h_err || !*(volatile int*)m->ll->h_err) return L3_OK;
-  *m->ll->h_err = 0;
-  set_err(m, "a kernel gave up waiting for its own pipeline; the results of this call are not valid");
-  return L3_ESTATE;
 }
 
 int ll_begin_call(L3Model* m, int B, int L, int start_pos) {
@@ -1491,7 +1482,7 @@ static int ll_linear(L3Model* m, const void* W, const float* x32, const void* x1
   if (ll->f32_tc && K >= 64 && N >= 64) {
     GemmF32Args t{};
     t.A = a.x; t.lda = ld; t.W = W; t.w_bf16 = m->bf16; t.rows = rows; t.N = N; t.K = K; t.epi = epi; t.e = e;
-    t.part = m->gemm_part; t.part_bytes = (size_t)32 << 20; t.tile_cnt = m->gemm_cnt; t.tile_cnt_len = 1024; t.err = ll->h_err;
+    t.part = m->gemm_part; t.part_bytes = (size_t)32 << 20; t.tile_cnt = m->gemm_cnt; t.tile_cnt_len = 1024; t.err = m->h_err;
     if (gemm_f32_supported(t)) {
       LAUNCH(m, launch_gemm_f32(t, m->stream));
       return L3_OK;
@@ -1557,7 +1548,7 @@ static int ll_mix_unit(L3Model* m, LLLayer& Ly, LLState& St, const float* pin, i
     at.chunked = s.chunked; at.gate = s.head_gate ? pin + Ly.off_g : nullptr; at.ld_gate = ld;
     at.B = B; at.L = L; at.H = H; at.G = G; at.DK = DK; at.DV = DV; at.M = m->M;
     if (tc) {
-      LAUNCH(m, launch_win_attn_tc(at, pa.q16, pa.q16_parts, m->maxB, ll->h_err, m->stream));
+      LAUNCH(m, launch_win_attn_tc(at, pa.q16, pa.q16_parts, m->maxB, m->h_err, m->stream));
       return L3_OK;
     }
     at.nsplit = win_attn_splits(B, L, H, G, s.window, s.keep_first, m->M, 32);
@@ -1655,7 +1646,7 @@ static int ll_latent_prompt(L3Model* m, LLLayer& Ly, LLState& St, int B, int L) 
   at.q16 = qa.q16; at.expand = (const bf16*)ll->lat_exp; at.cache = (const bf16*)St.lat; at.out16 = (bf16*)m->ctx16;
   at.out = ll_takes_mirror(m, ntok, m->D, H * DV) ? nullptr : m->ctx;
   at.gate = ll->pin + Ly.off_g; at.ld_gate = Ly.n_in; at.gate_wide = s.gate_wide; at.sink = s.sink ? Ly.head_vec : nullptr;
-  at.pos_ptr = d_pos; at.scale = s.scale; at.err = ll->h_err;
+  at.pos_ptr = d_pos; at.scale = s.scale; at.err = m->h_err;
   at.n_rows = ntok; at.L = L; at.H = H; at.dim = DK; at.rot_dim = s.rot_dim; at.vdim = DV; at.kv_rank = s.kv_rank; at.M = m->M;
   at.c_seqs = m->maxB; at.e_rows = m->M; at.e_seqs = ll->exp_seqs;
   // rows to expand: up to the chunk's last token, in steps of 128 (few distinct tensor maps; the surplus rows are stale but finite)
@@ -1695,7 +1686,7 @@ static int ll_latent_prompt_f32(L3Model* m, LLLayer& Ly, LLState& St, int B, int
       GemmF32Args t{};
       t.A = (const float*)St.lat + (size_t)(b0 + i) * m->M * Dk; t.W = Ly.w_ukv; t.rows = T; t.N = n_exp; t.K = Dk; t.epi = EPI_STORE;
       t.e = store_to(exp + (size_t)i * m->M * n_exp, nullptr, n_exp);
-      t.part = m->gemm_part; t.part_bytes = (size_t)32 << 20; t.tile_cnt = m->gemm_cnt; t.tile_cnt_len = 1024; t.err = ll->h_err;
+      t.part = m->gemm_part; t.part_bytes = (size_t)32 << 20; t.tile_cnt = m->gemm_cnt; t.tile_cnt_len = 1024; t.err = m->h_err;
       LAUNCH(m, launch_gemm_f32(t, m->stream));
     }
     WinAttnArgs at{};
@@ -1987,7 +1978,7 @@ static int ll_enqueue_parallel(L3Model* m, int B, int L, float* d_resid) {
       WinAttnArgs wa{};
       wa.cache_k = St.ck; wa.cache_v = St.cv; wa.out = ll->diff_maps; wa.ld_out = 2 * H * DV; wa.out_scale = 1.f; wa.pos_ptr = d_pos;
       wa.scale = s.scale; wa.kind = L3_ATTN_SOFTMAX; wa.window = s.window; wa.B = B; wa.L = L; wa.H = 2 * H; wa.G = G; wa.DK = DK; wa.DV = DV; wa.M = m->M;
-      LAUNCH(m, launch_win_attn_tc(wa, pa.q16, 2, m->maxB, ll->h_err, m->stream, 2));
+      LAUNCH(m, launch_win_attn_tc(wa, pa.q16, 2, m->maxB, m->h_err, m->stream, 2));
       if (ll_takes_mirror(m, ntok, W, H * DV)) at.out = nullptr;
       LAUNCH(m, launch_diff_combine(at, ll->diff_maps, m->stream));
     } else LAUNCH(m, launch_diff_attn(at, m->bf16, ll->diff_part_o, ll->diff_part_ml, m->stream));
@@ -2108,7 +2099,7 @@ int ll_enqueue_layers(L3Model* m, const int32_t* d_ids, int ids_ld, int ids_off,
         wa.cache_k = St.ck; wa.cache_v = St.cv; wa.out = ll_takes_mirror(m, ntok, W, O) ? nullptr : m->ctx; wa.out16 = (bf16*)m->ctx16; wa.ld_out = O;
         wa.out_scale = 1.f; wa.gate = at.head_gate; wa.ld_gate = at.ld_gate; wa.pos_ptr = d_pos; wa.scale = s.scale; wa.kind = L3_ATTN_SOFTMAX;
         wa.B = B; wa.L = L; wa.H = H; wa.G = G; wa.DK = DK; wa.DV = DK; wa.M = m->M;
-        LAUNCH(m, launch_win_attn_tc(wa, qa.q16, 2, m->maxB, ll->h_err, m->stream));
+        LAUNCH(m, launch_win_attn_tc(wa, qa.q16, 2, m->maxB, m->h_err, m->stream));
       } else if (!attn_head_dim_supported(DK)) LAUNCH(m, launch_attn_any(at, m->bf16, m->stream));
       else if (L == 1) {
         at.nsplit = std::max(1, std::min(std::min(m->max_split, m->M / 16), (4 * 148) / std::max(1, B * G)));

@@ -126,7 +126,6 @@ struct LayerList {
   void* win_q16 = nullptr;                 // softmax, window and differential attention of prompts on the tensor cores: packed queries
   float* diff_maps = nullptr;              // differential attention of prompts there: the two maps' outputs [cap_tok, heads, 2, vdim]
   int exp_seqs = 0;
-  int* h_err = nullptr;                    // pinned: a kernel sets it when one of its bounded waits ran out
   int keys_end = 0;                        // position behind the last token of the chunk being enqueued
   float *lat_part_o = nullptr, *lat_part_ml = nullptr;  // split scratch of the latent attention
   float *moe_w = nullptr, *moe_dense = nullptr, *moe_idw = nullptr;  // [rows, top] | [rows, experts] | [rows]
@@ -155,7 +154,6 @@ int ll_reset_slots(L3Model* m, int slot0, int n, bool kv_too);
 // position bookkeeping of a call that feeds L tokens to slots [0, B) at start_pos; start_pos 0 zeroes their state
 int ll_begin_call(L3Model* m, int B, int L, int start_pos);
 // after a synchronise: did a kernel of this handle give up waiting?
-int ll_check(L3Model* m);
 // all layers of one chunk; x in m->x (and its bf16 mirror) on entry and exit.  d_resid: null, or
 // [n_layers, B * L, width] receiving the residual stream after every layer
 int ll_enqueue_layers(L3Model* m, const int32_t* d_ids, int ids_ld, int ids_off, int B, int L, float* d_resid);

@@ -75,6 +75,7 @@ struct L3Model {
   int64_t* d_fwd_arg = nullptr; // [maxB] argmax of l3_forward
   unsigned long long* d_best = nullptr;  // [maxB] fused-argmax keys (gemm_tc.cu EPI_ARGMAX)
   int32_t* h_next = nullptr;  // pinned
+  int* h_err = nullptr;       // mapped host memory: a kernel sets it when one of its bounded waits ran out (null: no such kernel)
   // greedy-loop state
   int gen_B = 0, gen_L = 0, gen_step = 0, pend_B = 0, pend_L = 0;
   int gen_off = 0, pend_off = 0;

@@ -74,3 +74,33 @@ def test_greedy_tokens_match_the_oracle(name, B):
         m.reset_cache()
     assert np.array_equal(np.concatenate(list(m.generate(ids, cap)), axis=1), want)
     m.close()
+
+
+def test_a_wait_that_ran_out_is_reported():
+    """The host side of the cluster step's error word, which the test sets in the kernel's place: the call that finds it fails, the next one
+    is whole again.  The same word serves the layer-list kernels."""
+    import test_risalix_gpu as ris
+    args, w = _args("hd48", 2)
+    ids = np.random.default_rng(3).integers(0, args.vocab_size, (2, 5))
+    m = Llama(w, args)
+    want = m.generate_all(ids, 20)
+    step = m(ids[:, :1], 0).copy()
+    calls = [lambda: m.generate_all(ids, 20), lambda: m(ids[:, :1], 0), lambda: list(m.generate(ids, 20))]
+    for call in calls:
+        _cabi.check(_cabi.lib().l3_debug_fail_wait(m._h), m._h)
+        with pytest.raises(RuntimeError, match="gave up waiting"):
+            call()
+        assert np.array_equal(m.generate_all(ids, 20), want) and np.array_equal(m(ids[:, :1], 0), step)
+    m.close()
+    cfg = ris.config([ris.lightning()])
+    m, _ = ris.build(cfg)
+    ids = ids[:1] % cfg["vocab"]
+    want = m.forward_rows(ids, 0, [4])
+    _cabi.check(_cabi.lib().l3_debug_fail_wait(m._h), m._h)
+    with pytest.raises(RuntimeError, match="gave up waiting"):
+        m.forward_rows(ids, 0, [4])
+    assert np.array_equal(m.forward_rows(ids, 0, [4]), want)
+    m.close()
+    m = Llama(w, args, flags=_cabi.FLAG_NO_MEGA)   # no kernel of this handle has such a wait
+    assert _cabi.lib().l3_debug_fail_wait(m._h) == -1
+    m.close()
