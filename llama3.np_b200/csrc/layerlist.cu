@@ -963,9 +963,17 @@ static bool ll_latent_on_tc(const L3Model* m, const L3LayerSpec& s) {
 // In fp32 mode, portions of LATENT_F32_MIN tokens and more expand the cached rows as well: 2 (dim + rot_dim + vdim) FLOPs per (query,
 // key, head) instead of the folded form's 2 (2 kv_rank + rot_dim), for an expansion of 2 (dim + vdim) kv_rank per (key, head), which
 // runs on the tensor cores while the attention is FFMA in both forms.  8 heads of 128 + 64, values 128, rank 512, per layer: 600 tokens
-// 338 + 90 us (attention, products of the folded form) -> 123 + 45 us; the two-layer prompt 1624 -> 1097 us, at 64 tokens 670 -> 587 us;
-// a short portion behind a long prefix would expand the whole prefix for little, so it starts there.
+// 338 + 90 us (attention, products of the folded form) -> 123 + 45 us; the two-layer prompt 1624 -> 1097 us, at 64 tokens 436 -> 329 us.
+// A portion expands its whole prefix again, and the window kernel walks a tile's keys in one CTA where the folded kernel splits them, so
+// behind a prefix it takes enough query rows to fill the chip: from 128 tokens and 2048 rows (sequences x heads x tokens) on it gains for
+// every prefix (two layers of width 1024, 256 tokens behind 6144: 1.07, 400 behind 6000: 1.98; 16 heads, 128 behind 2048: 1.08), below
+// that up to a prefix of twice the portion where sequences x heads are at most 32 (64 behind 128: 1.15, 64 behind 2048: 0.52, 64 behind
+// 8000: 0.32; 64 sequence-heads, 64 behind 128: 0.87).
 constexpr int LATENT_F32_MIN = 64;
+static bool ll_latent_expansion_pays(const L3Model* m, const L3LayerSpec& s, int B, int L) {
+  const int prefix = m->ll->keys_end - L, seq_heads = B * s.heads;
+  return prefix == 0 || (L >= 128 && (int64_t)seq_heads * L >= 2048) || (prefix <= 2 * L && seq_heads <= 32);
+}
 static bool ll_latent_expands_f32(const L3Model* m, const L3LayerSpec& s) {
   return ll_latent_expands_on() && !m->bf16 && m->ll->f32_tc && s.mixer == L3_MIX_LATENT && s.dim % 8 == 0 && s.rot_dim % 8 == 0 && s.vdim % 8 == 0 && s.kv_rank % 8 == 0 &&
          s.heads * (s.dim + s.vdim) >= 64 && s.kv_rank + s.rot_dim >= 64 && win_attn_supported(s.dim + s.rot_dim, s.vdim);
@@ -1820,7 +1828,7 @@ static int ll_enqueue_prenorm(L3Model* m, int B, int L, float* d_resid) {
       if ((rc = ll_linear(m, Ly.w_uq, ll->aux, ll->aux16, 0, ntok, nq, s.q_rank, EPI_STORE, store_to(m->q, nullptr, nq))) != L3_OK) return rc;
       if (L > 8 && ll->lat_exp && ll_latent_on_tc(m, s)) {
         if ((rc = ll_latent_prompt(m, Ly, St, B, L)) != L3_OK) return rc;
-      } else if (L >= LATENT_F32_MIN && ll->lat_exp && ll_latent_expands_f32(m, s)) {
+      } else if (L >= LATENT_F32_MIN && ll->lat_exp && ll_latent_expands_f32(m, s) && ll_latent_expansion_pays(m, s, B, L)) {
         if ((rc = ll_latent_prompt_f32(m, Ly, St, B, L)) != L3_OK) return rc;
       } else {
         // queries onto the latent: qlat[r, h] = [Wuk_h^T q_c | rot(q_r)]

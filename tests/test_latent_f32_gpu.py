@@ -40,3 +40,24 @@ def test_head_gates_and_rotary_pairs(n, batch):
     cfg = rak.config([rak.latent(4, 32, 16, 40, kv_rank=64, dims=8), rak.latent(2, 64, 16, 64, kv_rank=48)], width=72)
     m, o = rak.build(cfg, 7, max_seq_len=n + 3, max_batch_size=batch)
     _check(m, o, cfg["vocab"], n, batch)
+
+
+def test_short_portions_behind_long_prefixes_keep_the_folded_form():
+    """A portion expands its whole prefix again: 64 tokens do it at the start of a sequence and behind up to twice their number, not behind
+    a longer prefix, 256 tokens of eight heads behind any (the launches of a call tell the two forms apart)."""
+    cfg = gif.config([gif.latent(heads=8, dim=16, rot_dim=8, vdim=24, kv_rank=64, scale=0.2, ff=40)], width=72)
+    m, o = gif.build(cfg, 8, max_seq_len=900, max_batch_size=3)
+    ids = np.random.default_rng(5).integers(0, cfg["vocab"], (3, 900))
+    at, count, got = 0, {}, []
+    for n in (64, 64, 64, 300, 64, 40, 256, 48):
+        m.launch_count(reset=True)
+        got.append(m.forward_rows(ids[:, at:at + n], at, list(range(3 * n))).reshape(3, n, -1))
+        count[at, n] = m.launch_count()
+        at += n
+    for b in range(3):
+        o.reset()
+        assert gif.err(np.concatenate([g[b] for g in got]), o.run(ids[b, :at])) < 1e-4
+    m.close()
+    expanded = count[0, 64]   # a GEMM per sequence
+    assert [count[64, 64], count[128, 64], count[192, 300], count[596, 256]] == [expanded] * 4
+    assert all(count[k] < expanded for k in ((492, 64), (556, 40), (852, 48)))
