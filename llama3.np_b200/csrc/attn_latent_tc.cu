@@ -349,41 +349,48 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     // ---------------- outputs
     const uint32_t idesc_pv = IDESC_PV | ((uint32_t)(((a.vdim + 15) & ~15) >> 3) << 17);
     const uint64_t dp0 = desc_k_sw128(sP), dv0 = desc_mn_sw128(sV, SLICE_K);
-    int st = 0, ph = 0;
-    for (int j = 0; j < nb; ++j) {
-      const int w = j & 1;
-      // Rows of the block behind the last key this tile sees are what an earlier sequence left, or another head's: their weight is 0, but
-      // 0 times an infinity or a NaN is not.  They become zeros first, in the last block and in a kept block of a short sequence (a
-      // slice's row is 128 bytes, however its pieces are swizzled): at most 24 KB by one warp.
-      const int live = start + last_q + 1 - block_key(j);
-      if (live < BKV) {
-        if (!__all_sync(L3_FULL, mbar_wait(v_full + 8 * st, ph, fail))) break;
-        uint8_t* vb = smem_raw + (sV - raw) + st * sh.v_bytes();
-        for (int i = lane; i < sh.nvs * (BKV - live) * 8; i += 32) {
-          const int row = i >> 3, s = row / (BKV - live);
-          *reinterpret_cast<uint4*>(vb + s * SLICE_K + (live + row - s * (BKV - live)) * 128 + (i & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-      }
-      bool ok = true;
-      if (lane == 0) {
-        ok = mbar_wait(v_full + 8 * st, ph, fail) && mbar_wait(p_full + 8 * w, (j >> 1) & 1, fail);
-        if (ok) {
-          tc_fence_after();
-          const uint64_t dv = dv0 + (uint64_t)((st * sh.v_bytes()) >> 4), dp = dp0 + (uint64_t)(w * (2 * P_TILE >> 4));
-          const uint32_t td = tO + w * o_cols;
+    auto product = [&](int j) {  // false: a wait ran out
+      const int w = j & 1, st = j % sh.vst;
+      if (!mbar_wait(v_full + 8 * st, (j / sh.vst) & 1, fail) || !mbar_wait(p_full + 8 * w, (j >> 1) & 1, fail)) return false;
+      tc_fence_after();
+      const uint64_t dv = dv0 + (uint64_t)((st * sh.v_bytes()) >> 4), dp = dp0 + (uint64_t)(w * (2 * P_TILE >> 4));
+      const uint32_t td = tO + w * o_cols;
 #pragma unroll
-          for (int part = 0; part < 2; ++part)  // high part, then low part
+      for (int part = 0; part < 2; ++part)  // high part, then low part
 #pragma unroll
-            for (int kk = 0; kk < BKV / 16; ++kk)  // 16 keys per MMA
-              mma_bf16(td, dp + part * (P_TILE >> 4) + kk * 2, dv + kk * (2048 >> 4), idesc_pv, (part | kk) ? 1u : (j < 2 ? 0u : 1u));
-          tc_commit(v_empty + 8 * st);
-          tc_commit(p_empty + 8 * w);
-        }
+        for (int kk = 0; kk < BKV / 16; ++kk)  // 16 keys per MMA
+          mma_bf16(td, dp + part * (P_TILE >> 4) + kk * 2, dv + kk * (2048 >> 4), idesc_pv, (part | kk) ? 1u : (j < 2 ? 0u : 1u));
+      tc_commit(v_empty + 8 * st);
+      tc_commit(p_empty + 8 * w);
+      return true;
+    };
+    // Rows of a block behind the last key this tile sees are what an earlier sequence left, or another head's: their weight is 0, but
+    // 0 times an infinity or a NaN is not.  They become zeros first, in the last block and in a kept block of a short sequence (a
+    // slice's row is 128 bytes, however its pieces are swizzled): at most 24 KB by one warp, while the block's weights are formed.
+    int j = 0;
+    bool ok = true;
+    while (j < nb && ok) {
+      int live = start + last_q + 1 - block_key(j);          // the blocks up to the next one with such rows: one thread alone
+      int stop = j;
+      while (stop < nb && (live = start + last_q + 1 - block_key(stop)) >= BKV) ++stop;
+      if (lane == 0)
+        for (; j < stop && ok; ++j) ok = product(j);
+      ok = __shfl_sync(L3_FULL, ok, 0);
+      j = stop;
+      if (!ok || j == nb) break;
+      const int st = j % sh.vst;
+      ok = __all_sync(L3_FULL, mbar_wait(v_full + 8 * st, (j / sh.vst) & 1, fail));
+      if (!ok) break;
+      uint8_t* vb = smem_raw + (sV - raw) + st * sh.v_bytes();
+      for (int i = lane; i < sh.nvs * (BKV - live) * 8; i += 32) {
+        const int row = i >> 3, s = row / (BKV - live);
+        *reinterpret_cast<uint4*>(vb + s * SLICE_K + (live + row - s * (BKV - live)) * 128 + (i & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
       }
-      if (!__shfl_sync(L3_FULL, ok, 0)) break;
-      if (++st == sh.vst) { st = 0; ph ^= 1; }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) ok = product(j);
+      ok = __shfl_sync(L3_FULL, ok, 0);
+      ++j;
     }
   } else {  // ---------------- softmax and output: thread = query row
     const int w = (warp - 2) >> 2, quarter = warp & 3;       // group; TMEM lanes this warp may read
