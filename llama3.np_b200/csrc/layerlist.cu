@@ -1007,6 +1007,59 @@ static bool ll_diff_on_tc(const L3Model* m, const L3LayerSpec& s) {
   return s.mixer == L3_MIX_DIFF && ll_attn_on_tc(m, s, 2 * s.heads * s.vdim);
 }
 
+// A workspace without which a call takes a slower path: at most a quarter of what is free, or L3_SCRATCH_MB megabytes, null beyond that
+// or where it cannot be had, so that a model whose weights and caches just fit is made all the same.
+static void* optional_ws(size_t bytes) {
+  const char* mb = getenv("L3_SCRATCH_MB");
+  size_t limit = 0, total = 0;
+  if (mb) limit = (size_t)std::max(0ll, atoll(mb)) << 20;
+  else if (cudaMemGetInfo(&limit, &total) == cudaSuccess) limit /= 4;
+  void* p = nullptr;
+  if (!bytes || bytes > limit) return nullptr;
+  if (cudaMalloc(&p, bytes) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  return p;
+}
+
+// The workspaces of prompt paths that have another path beside them, behind everything a model cannot do without.
+static int ll_workspaces(L3Model* m, bool units, bool ksplit) {
+  LayerList* ll = m->ll;
+  const size_t ct = (size_t)m->cap_tok;
+  if (ll->f32_tc && ksplit) {  // the K split of the tensor-core GEMMs
+    CK(m, cudaMalloc((void**)&m->gemm_cnt, 1024 * sizeof(int)));
+    CK(m, cudaMemsetAsync(m->gemm_cnt, 0, 1024 * sizeof(int), m->stream));
+    if (!m->gemm_part) m->gemm_part = (float*)optional_ws((size_t)32 << 20);
+  }
+  size_t wq_ld = 0, maps_ld = 0, chan = 0, f_ld = 0;
+  for (auto& L0 : ll->layers)
+    for (const LLLayer* U = &L0; U; U = U->pair) {
+      const L3LayerSpec& s = U->spec;
+      const size_t q_ld = (size_t)s.heads * ll_attn_parts(s) * latent_tc_q_ld(s.dim, 0);
+      if ((units && ll_window_on_tc(m, *U)) || ll_softmax_on_tc(m, s)) wq_ld = std::max(wq_ld, q_ld);
+      if (ll_diff_on_tc(m, s)) { wq_ld = std::max(wq_ld, 2 * q_ld); maps_ld = std::max(maps_ld, (size_t)2 * s.heads * s.vdim); }
+      if (m->tc_ok && (s.mixer == L3_MIX_GATED_DELTA || s.mixer == L3_MIX_GLA) && recur_channel_shape(s.dim, s.vdim) && ct >= RECUR_CHANNEL_MIN)
+        chan = std::max(chan, recur_channel_ws_floats(1, (int)ct, s.heads, s.dim, s.vdim) + recur_channel_ws_floats(m->maxB, 1, s.heads, s.dim, s.vdim));
+      if (ll_latent_expands_f32(m, s)) f_ld = std::max(f_ld, (size_t)s.heads * (s.dim + s.vdim));
+    }
+  if (ct > 8) {  // packed queries, maps of differential attention
+    ll->win_q16 = optional_ws(ct * wq_ld * 2);
+    ll->diff_maps = (float*)optional_ws(ct * maps_ld * 4);
+  }
+  chan = std::min(chan, (size_t)64 << 20);  // recurrences with a decay per key channel: at most 256 MB, long prompts go in segments
+  if (chan > ll->chunk_ws_floats)
+    if (float* p = (float*)optional_ws(chan * 4)) {
+      if (ll->chunk_ws) CK(m, cudaFree(ll->chunk_ws));
+      ll->chunk_ws = p;
+      ll->chunk_ws_floats = chan;
+    }
+  const size_t per = (size_t)m->M * f_ld * 4;
+  if (f_ld && ct >= LATENT_F32_MIN && per <= ((size_t)1 << 30)) {  // expanded latent rows in fp32 mode; longer contexts keep the folded form
+    const int seqs = (int)std::max<size_t>(1, std::min<size_t>(m->maxB, ((size_t)1 << 28) / per));
+    ll->lat_exp = optional_ws(seqs * per);
+    ll->exp_seqs = ll->lat_exp ? seqs : 0;
+  }
+  return L3_OK;
+}
+
 int ll_finalize(L3Model* m) {
   LayerList* ll = m->ll;
   for (const auto& name : ll_expected(m))
@@ -1171,25 +1224,15 @@ int ll_finalize(L3Model* m) {
       if (chunked && recur_chunk_shape(s.dim, s.vdim) && ct >= 128)
         ll->chunk_ws_floats = std::max(ll->chunk_ws_floats, (ct / 64 + m->maxB) * ((size_t)s.heads * s.dim * s.vdim + s.heads + (s.mixer == L3_MIX_MLSTM ? s.heads * s.dim : 0)) + 8);
     }
-  for (const LLLayer& L0 : ll->layers)
-    for (const LLLayer* U = &L0; U; U = U->pair) {  // bf16 mode: recurrences with a decay per key channel (at most 256 MB; long prompts go in segments)
-      const L3LayerSpec& s = U->spec;
-      if (!m->bf16 || (s.mixer != L3_MIX_GATED_DELTA && s.mixer != L3_MIX_GLA) || !recur_channel_shape(s.dim, s.vdim) || ct < RECUR_CHANNEL_MIN) continue;
-      const size_t need = recur_channel_ws_floats(1, (int)ct, s.heads, s.dim, s.vdim) + recur_channel_ws_floats(m->maxB, 1, s.heads, s.dim, s.vdim);
-      ll->chunk_ws_floats = std::max(ll->chunk_ws_floats, std::min(need, (size_t)64 << 20));
-    }
   if (ll->chunk_ws_floats) CK(m, cudaMalloc((void**)&ll->chunk_ws, ll->chunk_ws_floats * 4));
   // tensor cores: in bf16 mode every projection of many rows with a bf16 mirror; in both modes the ones that read fp32 rows, at fp32
   // precision (gemm_f32.cu).  (The 3xTF32 scheme of the Llama path is further from 64-bit sums than an fp32 FFMA chain: 3.5e-6 against
   // 1.2e-6 of the result at K = 4096.)
   ll->f32_tc = !(m->cfg.flags & L3_FLAG_NO_TENSORCORE) && tc_gemm_supported(W);
   m->tc_ok = m->bf16 && ll->f32_tc;
-  if (ll->f32_tc && !(getenv("L3_GEMM_KSPLIT") && atoi(getenv("L3_GEMM_KSPLIT")) == 0)) {
-    CK(m, cudaMalloc((void**)&m->gemm_part, (size_t)32 << 20));
-    CK(m, cudaMalloc((void**)&m->gemm_cnt, 1024 * sizeof(int)));
-    CK(m, cudaMemsetAsync(m->gemm_cnt, 0, 1024 * sizeof(int), m->stream));
-  }
+  const bool ksplit = !(getenv("L3_GEMM_KSPLIT") && atoi(getenv("L3_GEMM_KSPLIT")) == 0);
   if (m->tc_ok) {
+    if (ksplit) CK(m, cudaMalloc((void**)&m->gemm_part, (size_t)32 << 20));
     CK(m, cudaMalloc(&m->xn16, ct * W * 2));  // mirror of the residual stream
     CK(m, cudaMalloc(&m->ctx16, ct * ll->max_ctx * 2));
     CK(m, cudaMemsetAsync(m->ctx16, 0, ct * ll->max_ctx * 2, m->stream));
@@ -1207,16 +1250,6 @@ int ll_finalize(L3Model* m) {
       q_ld = std::max(q_ld, (size_t)L.spec.heads * latent_tc_q_ld(L.spec.dim, L.spec.rot_dim));
       e_ld = std::max(e_ld, (size_t)L.spec.heads * (L.spec.dim + L.spec.vdim));
     }
-  if (!m->bf16) {
-    size_t f_ld = 0;
-    for (auto& L : ll->layers)
-      if (ll_latent_expands_f32(m, L.spec)) f_ld = std::max(f_ld, (size_t)L.spec.heads * (L.spec.dim + L.spec.vdim));
-    const size_t per = (size_t)m->M * f_ld * 4;
-    if (f_ld && ct >= LATENT_F32_MIN && per <= ((size_t)1 << 30)) {  // longer contexts keep the folded form
-      ll->exp_seqs = (int)std::max<size_t>(1, std::min<size_t>(m->maxB, ((size_t)1 << 28) / per));
-      CK(m, cudaMalloc(&ll->lat_exp, ll->exp_seqs * per));
-    }
-  }
   if (e_ld && ct > 8) {
     const size_t per = (size_t)m->M * e_ld * 2;  // one sequence's keys and values; sequences share the workspace in turns
     ll->exp_seqs = (int)std::max<size_t>(1, std::min<size_t>(m->maxB, ((size_t)1 << 30) / per));
@@ -1224,16 +1257,6 @@ int ll_finalize(L3Model* m) {
     CK(m, cudaMalloc(&ll->lat_exp, ll->exp_seqs * per));
     CK(m, cudaMemsetAsync(ll->lat_exp, 0, ll->exp_seqs * per, m->stream));  // never anything but finite numbers
   }
-  size_t wq_ld = 0, maps_ld = 0;
-  for (auto& L0 : ll->layers)
-    for (const LLLayer* U = &L0; U; U = U->pair) {
-      const L3LayerSpec& s = U->spec;
-      const size_t q_ld = (size_t)s.heads * ll_attn_parts(s) * latent_tc_q_ld(s.dim, 0);
-      if ((units && ll_window_on_tc(m, *U)) || ll_softmax_on_tc(m, s)) wq_ld = std::max(wq_ld, q_ld);
-      if (ll_diff_on_tc(m, s)) { wq_ld = std::max(wq_ld, 2 * q_ld); maps_ld = std::max(maps_ld, (size_t)2 * s.heads * s.vdim); }
-    }
-  if (wq_ld && ct > 8) CK(m, cudaMalloc(&ll->win_q16, ct * wq_ld * 2));
-  if (maps_ld && ct > 8) CK(m, cudaMalloc((void**)&ll->diff_maps, ct * maps_ld * 4));
   m->max_split = 32;
   int max_hn = 1, max_hd = 1;
   for (auto& L : ll->layers)
@@ -1257,6 +1280,7 @@ int ll_finalize(L3Model* m) {
   CK(m, cudaGetDeviceProperties(&prop, m->cfg.device));
   m->n_sm = prop.multiProcessorCount;
   ll->head_rows = m->maxB;
+  if (const int rc = ll_workspaces(m, units, ksplit)) return rc;
   m->finalized = true;
   const int rc = ll_reset_slots(m, 0, m->maxB, true);
   if (rc != L3_OK) { m->finalized = false; return rc; }
@@ -1975,7 +1999,7 @@ static int ll_enqueue_parallel(L3Model* m, int B, int L, float* d_resid) {
     pa.proj = ll->pin; pa.ld = Ly.n_in; pa.q_off = Ly.off_q; pa.k_off = Ly.off_k; pa.v_off = Ly.off_v; pa.bias = Ly.in_bias;
     pa.wq = Ly.q_norm; pa.wk = Ly.k_norm; pa.eps = eps; pa.inv_freq = Ly.inv_freq; pa.cache_k = St.ck; pa.cache_v = St.cv;
     pa.pos_ptr = d_pos; pa.L = L; pa.H = H; pa.G = G; pa.DK = DK; pa.DV = DV; pa.M = m->M; pa.rot_dims = s.rot_dims;
-    const bool tc = L > 8 && ll->diff_maps && ll_diff_on_tc(m, s);
+    const bool tc = L > 8 && ll->win_q16 && ll->diff_maps && ll_diff_on_tc(m, s);
     pa.q_out = tc ? nullptr : m->q; pa.q16 = tc ? (bf16*)ll->win_q16 : nullptr; pa.q16_ld = latent_tc_q_ld(DK, 0);
     LAUNCH(m, launch_diff_prep(pa, ntok, m->bf16, m->stream));
     DiffAttnArgs at{};
