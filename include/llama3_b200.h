@@ -360,6 +360,16 @@ int l3_op_attention(int device, const float* q, const float* k, const float* v,
                     int kv_bf16 /* 0 fp32 cache, 1 bf16 cache, 2 bf16 tensor-core prefill (L > 1, head_dim 64/128),
                                    3 bf16 cache, decode through the exact (non tensor-core) kernels */,
                     int nsplit /* decode split-KV factor, 0 = auto */, float* out);
+/* Prompt attention of the layer-list decoders in bf16 mode on the tensor cores (attn_latent_tc.cu), two-part queries.  qkv [B, start + L,
+ * H DK | G DK | G DV]: the first `start` rows of a sequence are its prefix; caches of M rows; kind L3_ATTN_*, head_vec [H] the sinks or
+ * the sigmoid's biases (may be NULL for L3_ATTN_SOFTMAX); window, chunked, keep_first as in L3LayerSpec.  out [B, L, H, DV]. */
+int l3_op_prompt_attention(int device, const float* qkv, const float* head_vec, int B, int L, int H, int G, int DK, int DV,
+                           int start, int M, int kind, int window, int chunked, int keep_first, float scale, float* out);
+/* Recurrences with a decay per key channel: gated linear attention, or the gated delta rule where beta is not NULL.  q, k, log_decay
+ * [B, L, H, DK], v, out [B, L, H, DV], beta [B, L, H], state [B, H, DK, DV] in and out.  ws_chunks 0: the token-by-token chain; else the
+ * chunk-parallel form (recur_channel.cu) with a workspace of that many chunks of 64 tokens per (sequence, head). */
+int l3_op_recurrence(int device, const float* q, const float* k, const float* v, const float* log_decay, const float* beta,
+                     float* state, int B, int L, int H, int DK, int DV, int ws_chunks, float* out);
 /* logits[:, -1, :].argmax(-1) (llama3.py:320): first maximum wins. */
 int l3_op_argmax(int device, const float* logits, int rows, int n, int64_t* out);
 

@@ -110,6 +110,8 @@ SIGNATURES = {
     "l3_op_rope": (_I, [_I, _F32P, _F64P, _F64P, _I, _I, _I, _I, _I, _F32P]),
     "l3_op_swiglu": (_I, [_I, _F32P, _F32P, C.c_int64, _F32P]),
     "l3_op_attention": (_I, [_I, _F32P, _F32P, _F32P, _I, _I, _I, _I, _I, _I, _I, _I, _F32P]),
+    "l3_op_prompt_attention": (_I, [_I, _F32P, _F32P] + [_I] * 12 + [C.c_float, _F32P]),
+    "l3_op_recurrence": (_I, [_I] + [_F32P] * 6 + [_I] * 6 + [_F32P]),
     "l3_op_argmax": (_I, [_I, _F32P, _I, _I, _I64P]),
     "l3_debug_tc_timeline": (_I, [_I, _I, C.POINTER(C.c_uint64)]),
     "l3_sync": (_I, [_P]),

@@ -9,6 +9,7 @@
 #include "../../include/llama3_b200.h"
 #include "common.cuh"
 #include "gemm_tc.h"
+#include "mixer.h"
 
 namespace {
 struct Scratch {  // frees everything it handed out
@@ -211,6 +212,78 @@ extern "C" int l3_op_attention(int device, const float* q, const float* k, const
   int rc = finish(sc, e);
   tc_forget_maps();  // the tensor-core decode kernel maps the scratch caches, which are about to be freed
   if (rc == L3_OK) cudaMemcpy(out, dout, nq * 4, cudaMemcpyDeviceToHost);
+  return rc;
+}
+
+extern "C" int l3_op_prompt_attention(int device, const float* qkv, const float* head_vec, int B, int L, int H, int G, int DK, int DV, int start, int M,
+                                      int kind, int window, int chunked, int keep_first, float scale, float* out) {
+  if (B < 1 || L < 1 || start < 0 || start + L > M || G < 1 || H < G || H % G || (kind == L3_ATTN_SIGMOID && !head_vec)) return L3_EINVAL;
+  if (!win_attn_tc_supported(DK, DV, scale, H * DV, 2)) return L3_EINVAL;
+  Scratch sc;
+  if (begin(sc, device)) return L3_ECUDA;
+  const int T = start + L, ld = H * DK + G * (DK + DV), q_ld = latent_tc_q_ld(DK, 0);
+  const size_t nk = (size_t)B * G * M * DK, nv = (size_t)B * G * M * DV, no = (size_t)B * L * H * DV;
+  float* proj = sc.dev<float>((size_t)B * T * ld);
+  float* hv = head_vec ? sc.up(head_vec, H) : nullptr;
+  bf16 *ck = sc.dev<bf16>(nk), *cv = sc.dev<bf16>(nv), *q16 = sc.dev<bf16>((size_t)B * T * H * 2 * q_ld);
+  float* dout = sc.dev<float>(no);
+  int *err = sc.dev<int>(1), *pos = sc.dev<int>(1);
+  if (!proj || (head_vec && !hv) || !ck || !cv || !q16 || !dout || !err || !pos) return L3_ENOMEM;
+  if (cudaMemset(ck, 0xff, nk * 2) || cudaMemset(cv, 0xff, nv * 2) || cudaMemset(err, 0, sizeof(int))) return L3_ECUDA;  // rows nobody writes: NaN
+  WinPrepArgs pa{};
+  pa.proj = proj; pa.ld = ld; pa.k_off = H * DK; pa.v_off = H * DK + G * DK; pa.q16 = q16; pa.q16_ld = q_ld; pa.q16_parts = 2;
+  pa.cache_k = ck; pa.cache_v = cv; pa.pos_ptr = pos; pa.H = H; pa.G = G; pa.DK = DK; pa.DV = DV; pa.M = M;
+  cudaError_t e = cudaSuccess;
+  for (int p0 = 0; p0 < T && e == cudaSuccess; p0 = p0 < start ? start : T) {  // the prefix, then the portion
+    pa.L = p0 < start ? start : L;
+    e = cudaMemcpy(pos, &p0, sizeof(int), cudaMemcpyHostToDevice);
+    for (int b = 0; b < B && e == cudaSuccess; ++b)
+      e = cudaMemcpy(proj + (size_t)b * pa.L * ld, qkv + ((size_t)b * T + p0) * ld, (size_t)pa.L * ld * sizeof(float), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = launch_win_prep(pa, B * pa.L, true, sc.s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(sc.s);
+  }
+  WinAttnArgs a{};
+  a.cache_k = ck; a.cache_v = cv; a.out = dout; a.ld_out = H * DV; a.out_scale = 1.f; a.head_vec = kind == L3_ATTN_SOFTMAX ? nullptr : hv;
+  a.pos_ptr = pos; a.scale = scale; a.kind = kind; a.window = window; a.chunked = chunked; a.keep_first = keep_first;
+  a.B = B; a.L = L; a.H = H; a.G = G; a.DK = DK; a.DV = DV; a.M = M;
+  if (e == cudaSuccess) e = launch_win_attn_tc(a, q16, 2, B, err, sc.s);
+  int rc = finish(sc, e), bad = 0;
+  tc_forget_maps();
+  if (rc == L3_OK) cudaMemcpy(&bad, err, sizeof bad, cudaMemcpyDeviceToHost);
+  if (rc == L3_OK) cudaMemcpy(out, dout, no * 4, cudaMemcpyDeviceToHost);
+  return bad ? L3_ESTATE : rc;
+}
+
+extern "C" int l3_op_recurrence(int device, const float* q, const float* k, const float* v, const float* log_decay, const float* beta, float* state, int B,
+                                int L, int H, int DK, int DV, int ws_chunks, float* out) {
+  if (B < 1 || L < 1 || H < 1 || !recur_supported(DK, DV)) return L3_EINVAL;
+  Scratch sc;
+  if (begin(sc, device)) return L3_ECUDA;
+  const size_t rows = (size_t)B * L, nk = rows * H * DK, nv = rows * H * DV, ns = (size_t)B * H * DK * DV;
+  RecurArgs a{};
+  a.mode = beta ? 1 : 2; a.rep = 1; a.ld_q = a.ld_k = H * DK; a.ld_v = H * DV; a.B = B; a.L = L; a.H = H; a.DK = DK; a.DV = DV;
+  a.q = sc.up(q, nk); a.k = sc.up(k, nk); a.v = sc.up(v, nv);
+  a.beta = beta ? sc.up(beta, rows * H) : nullptr;
+  a.state = sc.up(state, ns);
+  a.out = sc.dev<float>(nv);
+  if (ws_chunks > 0) {
+    if (!recur_channel_shape(DK, DV)) return L3_EINVAL;
+    a.log_c = sc.up(log_decay, nk);
+    a.ws_floats = recur_channel_ws_floats(B, 1, H, DK, DV) * (size_t)ws_chunks;
+    a.ws = sc.dev<float>(a.ws_floats);
+    a.bf16_ops = 1;
+    if (!a.log_c || !a.ws) return L3_ENOMEM;
+    if (!recur_channel_supported(a)) return L3_EINVAL;
+  } else {
+    std::vector<float> g(nk);
+    for (size_t i = 0; i < nk; ++i) g[i] = expf(log_decay[i]);
+    a.g = sc.up(g.data(), nk);
+    if (!a.g) return L3_ENOMEM;
+  }
+  if (!a.q || !a.k || !a.v || (beta && !a.beta) || !a.state || !a.out) return L3_ENOMEM;
+  const int rc = finish(sc, launch_recur(a, sc.s));
+  if (rc == L3_OK) cudaMemcpy(out, a.out, nv * 4, cudaMemcpyDeviceToHost);
+  if (rc == L3_OK) cudaMemcpy(state, a.state, ns * 4, cudaMemcpyDeviceToHost);
   return rc;
 }
 
