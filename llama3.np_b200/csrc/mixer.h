@@ -94,7 +94,7 @@ bool recur_chunk_supported(const RecurArgs& a);
 cudaError_t launch_recur_chunk(const RecurArgs& a, cudaStream_t s);
 
 // chunk-parallel form on tensor products (recur_channel.cu), decays per key channel or per head; workspace `ws`, in segments where it is small
-constexpr int RECUR_CHANNEL_MIN = 48;  // tokens
+constexpr int RECUR_CHANNEL_MIN = 48;  // tokens of the shortest portion that can run there (recur_channel_supported: the rule)
 bool recur_channel_shape(int DK, int DV);
 size_t recur_channel_ws_floats(int B, int L, int H, int DK, int DV);
 bool recur_channel_supported(const RecurArgs& a);

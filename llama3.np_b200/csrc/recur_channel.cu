@@ -495,9 +495,19 @@ size_t recur_channel_ws_floats(int B, int L, int H, int DK, int DV) {
   return (size_t)B * H * ((L + CT - 1) / CT) * per;
 }
 
+// Portions from this length on.  A chunk costs ~20 us (gated linear attention) to ~35 us (delta rule: the triangular system) from one end to
+// the other whatever it holds; the chain costs 0.2 - 0.3 us per token, and more where its CTAs (a multiple of sequences x heads) fill
+// the chip.  One layer, prompt through the public call, chain against chunks in us: delta rule, 1 x 16 heads, 48 tokens 240 : 256, 96
+// 272 : 284, 128 306 : 308, 192 267 : 253, 400 347 : 284; 4 x 16 heads, 48 255 : 265, 64 278 : 269, 128 341 : 294.  Gated linear
+// attention, 1 x 2 heads, 48 tokens 152 : 158, 72 177 : 176, 96 188 : 180; 1 x 8 heads, 48 218 : 217, 64 228 : 220, 128 285 : 253.
+static int least_tokens(const RecurArgs& a) {
+  if (a.mode == 1) return a.B * a.H >= 64 ? 64 : 128;
+  return a.B * a.H >= 8 ? RECUR_CHANNEL_MIN : 72;
+}
+
 bool recur_channel_supported(const RecurArgs& a) {
   static const bool on = !(getenv("L3_RECUR_CHUNK") && atoi(getenv("L3_RECUR_CHUNK")) == 0);
-  if (!on || !a.bf16_ops || a.n_state || a.k_scale || !a.ws || a.L < RECUR_CHANNEL_MIN || !recur_channel_shape(a.DK, a.DV)) return false;
+  if (!on || !a.bf16_ops || a.n_state || a.k_scale || !a.ws || a.L < least_tokens(a) || !recur_channel_shape(a.DK, a.DV)) return false;
   if (a.mode == 0 ? a.head_decay == nullptr : a.log_c == nullptr && !(a.mode == 2 && a.log_g)) return false;
   const uintptr_t al = (uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.log_c | (uintptr_t)a.ws;
   if (a.ld_q % 4 || a.ld_k % 4 || (al & 15)) return false;

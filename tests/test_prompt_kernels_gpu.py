@@ -88,3 +88,16 @@ def test_recurrences(B, L, chunks, H, DK, DV, delta, rate):
         _call("l3_op_recurrence", q, k, v, lg, beta, S, B, L, H, DK, DV, ws, out)
         errs = [np.linalg.norm(a - b) / np.linalg.norm(b) for a, b in ((out, want), (S, end))]
         assert max(errs) < bar, (ws, errs)
+
+
+@pytest.mark.parametrize("delta,B,H,least", [(True, 1, 2, 128), (True, 3, 21, 128), (True, 4, 16, 64), (False, 1, 7, 72), (False, 4, 2, 48)])
+def test_which_portions_run_in_chunks(delta, B, H, least):
+    """The chunk-parallel form takes the lengths from which it is the faster one, and no shorter ones."""
+    def run(L):
+        q, k, lg, v = (np.full((B, L, H, d), -0.1, np.float32) for d in (64, 64, 64, 16))
+        beta = np.full((B, L, H), 0.5, np.float32) if delta else None
+        _call("l3_op_recurrence", q, k, v, lg, beta, np.zeros((B, H, 64, 16), np.float32), B, L, H, 64, 16, 9, np.empty_like(v))
+
+    run(least)
+    with pytest.raises(ValueError):
+        run(least - 1)

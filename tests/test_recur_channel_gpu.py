@@ -1,5 +1,6 @@
 """The gated delta rule and gated linear attention of prompts in bf16 mode in the chunk-parallel form on tensor products: lengths at
-the edges of the 64-token chunks and of the rule (48 tokens), key sizes 64 and 128, value sizes down to 16, grouped keys, batches,
+the edges of the 64-token chunks and of the rule (delta rule: 128 tokens, 64 from 64 sequence-heads on; gated linear attention: 72, 48
+from 8 sequence-heads on), key sizes 64 and 128, value sizes down to 16, grouped keys, batches,
 decays that empty a channel within a few tokens and decays near one.  Against the float64 oracle at the families' bf16 bar (6e-2 of
 the logit scale), and against the same prompt in portions of 40 tokens, which the token-by-token chain takes: there only roundings of
 bf16 activations differ, 2^-9 each and averaged by every sum, so 1e-2."""
@@ -41,7 +42,7 @@ def _rates(t, kind):
     return t
 
 
-@pytest.mark.parametrize("n,batch", [(48, 2), (63, 1), (64, 3), (65, 1), (127, 1), (200, 2)])
+@pytest.mark.parametrize("n,batch", [(48, 2), (63, 1), (64, 3), (65, 1), (127, 1), (200, 2), (128, 1), (129, 2), (191, 1), (193, 1)])
 @pytest.mark.parametrize("heads,kv,dim,vdim,rate", [(2, 2, 128, 128, "mixed"), (4, 2, 64, 16, "fast"), (2, 1, 64, 80, "slow"), (2, 2, 128, 48, "fast")])
 def test_delta_rule(n, batch, heads, kv, dim, vdim, rate):
     cfg = ris.config([ris.delta(heads, kv, dim, vdim, 4), ris.delta(heads, kv, dim, vdim, 2, ff=96)], width=96)
@@ -61,6 +62,22 @@ def test_gated_linear_attention(n, batch, heads, dim, vdim, rate):
     # the rounding of its bf16 projections is off by order one whatever the kernel does (the chain is 0.230 off on 200 tokens, the
     # chunks 0.230 off, the two 0.002 apart).  Those cases are held to the chain alone.
     _check(m, o, cfg["vocab"], n, batch, lambda o, ids: (deb.fresh(o), o.run(ids))[1], oracle=rate != "fast")
+
+
+@pytest.mark.parametrize("n", [64, 65, 127])
+def test_delta_rule_of_many_heads(n):
+    cfg = ris.config([ris.delta(32, 8, 64, 16, 3)], width=96)
+    t = _rates(ris.random_model(cfg, 8), "mixed")
+    m, o = ris.build(cfg, dtype="bfloat16", max_seq_len=n + 2, max_batch_size=2, tensors=t)
+    _check(m, o, cfg["vocab"], n, 2, lambda o, ids: o.run(ids))
+
+
+@pytest.mark.parametrize("heads,n,batch", [(8, 48, 1), (8, 63, 2), (8, 64, 1), (8, 65, 2), (2, 72, 1), (2, 127, 2), (2, 128, 1), (2, 129, 1)])
+def test_gated_linear_attention_at_the_edges(heads, n, batch):
+    cfg = deb.config([deb.gla(heads, 64, 16, tau=8.0, mlp={"kind": "dense", "ff": 64})], width=96)
+    t = _rates(deb.random_tensors(cfg, 9), "mixed")
+    m, o = deb.build(cfg, dtype="bfloat16", max_seq_len=n + 2, max_batch_size=batch, tensors=t)
+    _check(m, o, cfg["vocab"], n, batch, lambda o, ids: (deb.fresh(o), o.run(ids))[1])
 
 
 def _forget(t, a1, a2, embed, token, z):
