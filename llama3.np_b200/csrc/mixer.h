@@ -81,7 +81,7 @@ struct RecurArgs {
   float* n_state;         // [maxB, H, DK] a running sum of the keys with the state's own decay (the normaliser of an mLSTM) ...
   float* nq;              // ... and its product with the query, [B * L, H]
   int bf16_ops;           // bf16 mode.  With n_state, chunk-parallel form: q, k and v may be rounded to bf16 (they are bf16 projections'
-                          // outputs).  Without: prompts may run on tensor products of (hi, lo) pairs (recur_channel.cu)
+                          // outputs).  With log_c: prompts run on tensor products of (hi, lo) pairs (recur_channel.cu)
   float* ws;              // mode 0, may be null: room for one state matrix per (sequence, head, chunk of 64 tokens);
   size_t ws_floats;       // with it, prompts of the common shapes run in the chunk-parallel form (recur_chunk.cu)
 };
@@ -93,7 +93,7 @@ bool recur_chunk_shape(int DK, int DV);
 bool recur_chunk_supported(const RecurArgs& a);
 cudaError_t launch_recur_chunk(const RecurArgs& a, cudaStream_t s);
 
-// chunk-parallel form on tensor products (recur_channel.cu), decays per key channel or per head; workspace `ws`, in segments where it is small
+// chunk-parallel form on tensor products (recur_channel.cu), decays per key channel; workspace `ws`, in segments where it is small
 constexpr int RECUR_CHANNEL_MIN = 48;  // tokens of the shortest portion that can run there (recur_channel_supported: the rule)
 bool recur_channel_shape(int DK, int DV);
 size_t recur_channel_ws_floats(int B, int L, int H, int DK, int DV);

@@ -1,6 +1,7 @@
-// Chunk-parallel form of the linear recurrences on warp-level tensor products, for prompts in bf16 mode: the gated delta rule and
-// gated linear attention, whose decay is a number per key channel and token, and the fixed-decay and state-space recurrences,
-// whose decay is one number per head (RecurArgs modes 0, 1 and 2).
+// Chunk-parallel form of the linear recurrences with a decay per key channel and token on warp-level tensor products, for prompts in
+// bf16 mode: the gated delta rule (RecurArgs mode 1) and gated linear attention (mode 2 with log_c).  The chunked mathematics is that
+// of "Gated Linear Attention Transformers with Hardware-Efficient Training" (Yang et al., 2023) and, for the delta rule's triangular
+// system, "Parallelizing Linear Transformers with the Delta Rule over Sequence Length" (Yang et al., 2024).
 //
 //   S_t = diag(g_t) S_(t-1) + k_t u_t^T,   o_t = S_t^T q_t,   u_t = v_t, or with the delta rule beta_t (v_t - (diag(g_t) S_(t-1))^T k_t)
 //
@@ -50,9 +51,6 @@ __device__ __forceinline__ void mma3(float (&c)[4], const uint32_t (&ah)[4], con
   mma16816(c, al, b.x, b.y);
   mma16816(c, ah, b.z, b.w);
 }
-__device__ __forceinline__ float act_silu(int act_in, float x) {
-  return act_in == 0 ? x : act_in == 2 ? __fdividef(x, 1.0f + __expf(-x)) : silu_ref(x);
-}
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
@@ -88,26 +86,18 @@ __global__ void __launch_bounds__(512) channel_chunk_kernel(RecurArgs a, int c0)
   const int n = min(CT, a.L - c * CT);
   const size_t row0 = (size_t)b * a.L + (size_t)c * CT;
   {
-    const float q_mul = a.q_mul != 0.f ? a.q_mul : 1.f;
     const float* qs = a.q + row0 * a.ld_q + (size_t)(h / a.rep) * DK;
     const float* ks = a.k + row0 * a.ld_k + (size_t)(h / a.rep) * DK;
-    const float fixed = a.log_c || a.log_g ? 0.f : logf(a.head_decay[h]);
     for (int i = tid; i < CT * DK / 4; i += 512) {
       const int t = i / (DK / 4), d = (i % (DK / 4)) * 4;
       float4 qv = make_float4(0.f, 0.f, 0.f, 0.f), kv = qv, lv = qv;
       if (t < n) {
         qv = *reinterpret_cast<const float4*>(qs + (size_t)t * a.ld_q + d);
         kv = *reinterpret_cast<const float4*>(ks + (size_t)t * a.ld_k + d);
-        if (a.log_c) lv = *reinterpret_cast<const float4*>(a.log_c + (row0 + t) * a.H * DK + (size_t)h * DK + d);
-        else { const float l = a.log_g ? a.log_g[(row0 + t) * a.H + h] : fixed; lv = make_float4(l, l, l, l); }
+        lv = *reinterpret_cast<const float4*>(a.log_c + (row0 + t) * a.H * DK + (size_t)h * DK + d);
         // From -104 on a decay is zero in fp32.  Stronger ones are held at -110: the decays of the tokens behind them are differences
         // of running sums, which are right to 2^-14 of a unit that way (a block's stay above -16 x 110), with one such token to 2^-18
         lv.x = lv.x < -110.f ? -110.f : lv.x; lv.y = lv.y < -110.f ? -110.f : lv.y; lv.z = lv.z < -110.f ? -110.f : lv.z; lv.w = lv.w < -110.f ? -110.f : lv.w;
-        if (a.act_in) {
-          qv.x = act_silu(a.act_in, qv.x); qv.y = act_silu(a.act_in, qv.y); qv.z = act_silu(a.act_in, qv.z); qv.w = act_silu(a.act_in, qv.w);
-          kv.x = act_silu(a.act_in, kv.x); kv.y = act_silu(a.act_in, kv.y); kv.z = act_silu(a.act_in, kv.z); kv.w = act_silu(a.act_in, kv.w);
-        }
-        qv.x *= q_mul; qv.y *= q_mul; qv.z *= q_mul; qv.w *= q_mul;
       }
       *reinterpret_cast<float4*>(qf + t * LD + d) = qv;
       *reinterpret_cast<float4*>(kf + t * LD + d) = kv;
@@ -427,7 +417,6 @@ __global__ void __launch_bounds__(DK * 2, 1) channel_chain_kernel(RecurArgs a, i
       o[p][0] = so.x; o[p][1] = so.y; o[p][2] = so.z; o[p][3] = so.w;
       float u0 = uv[p][0], u1 = uv[p][1], u2 = uv[p][2], u3 = uv[p][3];
       if (DELTA) { u0 -= su.x; u1 -= su.y; u2 -= su.z; u3 -= su.w; }
-      else if (a.act_in) { u0 = act_silu(a.act_in, u0); u1 = act_silu(a.act_in, u1); u2 = act_silu(a.act_in, u2); u3 = act_silu(a.act_in, u3); }
       uint2 hi, lo;                                      // half of an operand's four registers: tokens (nt & 1) * 8 + q2 of step nt / 2
       split2(u0, u1, hi.x, lo.x);
       split2(u2, u3, hi.y, lo.y);
@@ -507,8 +496,8 @@ static int least_tokens(const RecurArgs& a) {
 
 bool recur_channel_supported(const RecurArgs& a) {
   static const bool on = !(getenv("L3_RECUR_CHUNK") && atoi(getenv("L3_RECUR_CHUNK")) == 0);
-  if (!on || !a.bf16_ops || a.n_state || a.k_scale || !a.ws || a.L < least_tokens(a) || !recur_channel_shape(a.DK, a.DV)) return false;
-  if (a.mode == 0 ? a.head_decay == nullptr : a.log_c == nullptr && !(a.mode == 2 && a.log_g)) return false;
+  if (!on || !a.bf16_ops || !a.ws || a.L < least_tokens(a) || !recur_channel_shape(a.DK, a.DV)) return false;
+  if ((a.mode != 1 && a.mode != 2) || !a.log_c || a.act_in || a.q_mul != 0.f || a.n_state || a.k_scale) return false;
   const uintptr_t al = (uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.log_c | (uintptr_t)a.ws;
   if (a.ld_q % 4 || a.ld_k % 4 || (al & 15)) return false;
   return recur_channel_ws_floats(a.B, 1, a.H, a.DK, a.DV) <= a.ws_floats;
