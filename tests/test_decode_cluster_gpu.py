@@ -36,6 +36,10 @@ def test_steps_match_the_oracle(name, B):
     rng = np.random.default_rng(B)
     ids = rng.integers(0, args.vocab_size, (B, M))
     m, o, m2 = Llama(w, args), orc.OracleLlama(w, args), Llama(w, args, flags=_cabi.FLAG_NO_MEGA)
+    for model in (m, m2):      # the layers are one launch here and five or more each there
+        model.launch_count(reset=True)
+        model(ids[:, :1], 0)
+    assert m.launch_count() < 6 and m2.launch_count() >= 5 * args.n_layers
     tol = lambda want: 5e-5 * np.abs(want).max()
 
     def check(lo, hi):
@@ -69,9 +73,13 @@ def test_greedy_tokens_match_the_oracle(name, B):
     cap = args.max_seq_len
     want = np.concatenate(list(orc.OracleLlama(w, args).generate(ids, cap)), axis=1)
     m = Llama(w, args)
-    for _ in range(2):  # the head's counters are back at zero behind a run
-        assert np.array_equal(m.generate_all(ids, cap), want)
+    counts = []
+    for n in (cap, cap, cap - 10):  # the head's counters are back at zero behind a run
+        m.launch_count(reset=True)
+        assert np.array_equal(m.generate_all(ids, n), want[:, :n - 5])
+        counts.append(m.launch_count())
         m.reset_cache()
+    assert counts[1] - counts[2] == 2 * 10  # layers, LM head: the step is the cluster's
     assert np.array_equal(np.concatenate(list(m.generate(ids, cap)), axis=1), want)
     m.close()
 

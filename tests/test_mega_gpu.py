@@ -1,6 +1,6 @@
 """The persistent batch-1 decode kernel (decode_mega.cu) against the oracle and against the
-kernel-per-projection path: same greedy tokens in fp32 mode at the head shapes of every
-BASELINE config (stories15M 48/MHA, 1B 64/GQA-4, 8B 128/GQA-4), including rows that are cut
+kernel-per-projection path: same greedy tokens in fp32 mode at the head shapes of the
+shipped configurations (stories15M 48/MHA, 1B 64/GQA-4, 8B 128/GQA-4), including rows that are cut
 into chunks (K > 2048 fp32 / 4096 bf16) and several row pairs per ring stage (small K)."""
 import numpy as np
 import pytest
@@ -105,4 +105,30 @@ def test_mega_cache_rows_match_the_oracle_over_repeated_generates():
             k, v = m.read_cache(l)
             np.testing.assert_allclose(k, o.layers[l]["cache_k"][:1], rtol=0, atol=2e-5, err_msg=f"iteration {it} layer {l} K")
             np.testing.assert_allclose(v, o.layers[l]["cache_v"][:1], rtol=0, atol=2e-5, err_msg=f"iteration {it} layer {l} V")
+    m.close()
+
+
+@pytest.mark.parametrize("name", ["s15m-like", "hd48-gqa2", "tiny-mha"])
+def test_small_models_of_long_contexts_run_the_persistent_kernel(name):
+    """Up to 512 positions these fp32 models decode in one cluster (decode_cluster.cu, so do their cases above); longer ones keep
+    decode_mega.  One launch per step says that it ran."""
+    import dataclasses
+    args, w = _make(name)
+    args = dataclasses.replace(args, max_seq_len=600)
+    ids = np.random.default_rng(3).integers(3, args.vocab_size, (1, 6))
+    o = orc.OracleLlama(w, args)
+    want = np.concatenate(list(o.generate(ids, 60)), axis=1)
+    m = Llama(w, args)
+    assert np.array_equal(m.generate_all(ids, 60), want)
+    counts = []
+    for cap in (20, 60):
+        m.reset_cache()
+        m.launch_count(reset=True)
+        assert np.array_equal(m.generate_all(ids, cap), want[:, :cap - 6])
+        counts.append(m.launch_count())
+    assert counts[1] - counts[0] == 40
+    for l in range(args.n_layers):
+        k, v = m.read_cache(l)
+        np.testing.assert_allclose(k[:, :60], o.layers[l]["cache_k"][:1, :60], rtol=0, atol=2e-5)
+        np.testing.assert_allclose(v[:, :60], o.layers[l]["cache_v"][:1, :60], rtol=0, atol=2e-5)
     m.close()
