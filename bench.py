@@ -73,7 +73,7 @@ def make_prompts(n, seed=1):
 
 
 class ClockSampler:
-    """nvidia-smi clocks / throttle reasons sampled DURING the timed region (B200_PROFILING.md)."""
+    """nvidia-smi clocks / throttle reasons sampled DURING the timed region."""
     Q = ("clocks.sm,clocks.max.sm,clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
          "clocks_event_reasons.sw_thermal_slowdown,clocks_event_reasons.sw_power_cap")
 
@@ -548,7 +548,7 @@ def run_b200(a):
         pos_mid = (PROMPT_LEN + TOTAL_LEN) // 2
         step_ms = dev_ms / a.steps / N_OUT  # one decode step of the whole batch (the prefill is 1 of 248 steps)
         # Dominant kernel of a decode step: decode_stack_kernel (every layer of the step, one launch), ~88 % of the
-        # step's device time (profiles/r02_launches_decode_step.csv); the LM head + finalize are the rest.
+        # step's device time (profiles/launches_decode_step.csv); the LM head + finalize are the rest.
         # Its algorithmic bytes per launch: the layers' weights once (each of the ceil(B / 12) clusters
         # streams them, but from L2) + K and V of every cached position of every sequence and layer.
         stack_ms, lm_ms = C.c_float(), C.c_float()
@@ -559,7 +559,7 @@ def run_b200(a):
         stack_bytes = layer_params * wb + kv_bytes + B * D * wb * 3      # + embedding rows in, normalised rows (hi, lo) out
         traffic, traffic_note = None, None
         try:  # DRAM bytes per launch from the committed ncu --set full capture of the same kernel and shape
-            with open(os.path.join(ROOT, "profiles", "r02_traffic.json")) as f:
+            with open(os.path.join(ROOT, "profiles", "traffic.json")) as f:
                 t = json.load(f)["decode_stack_kernel"]
             if B == 256 and a.dtype == "f32" and TOTAL_LEN == 256:
                 traffic, traffic_note = t["traffic_bytes_per_launch"], t["config"] + "; " + t["source"]

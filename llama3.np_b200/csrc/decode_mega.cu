@@ -307,7 +307,7 @@ __device__ __forceinline__ void consume_matrix(const MegaArgs& a, const MegaLaye
         if (lane == pr) { my0 = acc0; my1 = acc1; }
       }
       // generic-proxy reads (LDS) before the async-proxy refill (cp.async.bulk): each reader fences its own reads
-      // (the same hazard was measured in decode_stack.cu: profiles/r02_stack_race.txt)
+      // (the same hazard was measured in decode_stack.cu: profiles/stack_race.txt)
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(rg.empty0 + 8 * slot);  // stage drained: the producer may refill it
@@ -457,7 +457,7 @@ __device__ __forceinline__ void stage_sum(const MegaArgs& a, unsigned epoch, flo
   float ss = 0.f;
   // No grid barrier precedes this staging any more, so nothing else separates the previous phase's reads of xs from
   // the writes below: a warp that has finished its row pairs must not overwrite the vector other warps of this CTA
-  // are still multiplying with (measured without this barrier: rare wrong K / V rows, scripts/mega_cache_check.py).
+  // are still multiplying with (measured without this barrier: rare wrong K / V rows).
   cons_sync();
   if (a.tp_world >= 4) {
     // Two levels: if every CTA summed all `world` regions itself, the chip would read world x K x 8 bytes x CTAs from

@@ -15,14 +15,14 @@
 // Data movement: every CTA streams ITS slice of the layer's weights (pre-packed k-major slabs, 648 KB per layer
 // at the stories15M shape) and the K / V rows of its head from L2 / HBM with cp.async.bulk into a ring of 8 x 18 KB
 // stages.  Four producer warps issue the copies (one thread sustains only ~49 GB/s of bulk copies, four reach
-// ~220 GB/s per SM: scripts/ubench, profiles/r02_ubench.jsonl); nine compute warps consume.  Weights and cached
+// ~220 GB/s per SM: scripts/ubench, profiles/ubench.jsonl); nine compute warps consume.  Weights and cached
 // K / V do not depend on this step's activations, so the producers run ahead across phase changes.
 //
 // Math: plain fp32 FFMA.  Thread tile = 4 output features x ALL S sequences (48 accumulators) over a k-group (1/4 or
 // 1/8 of each slab's k rows): per k row one float4 of weights from the k-major slab (quarter warps read 128
 // contiguous bytes) and S / 4 broadcast float4s of activations from a k-major [K][S + 8] buffer (80-byte rows keep
 // the k-groups' reads in different banks) feed 48 FFMAs; k-groups are the high lane bits and are summed with shuffles.  (tcgen05 is the wrong tool
-// for S = 12 rows: an M = 128 MMA costs 128 cycles whatever N is - profiles/r02_mma_cost.jsonl - and the legacy
+// for S = 12 rows: an M = 128 MMA costs 128 cycles whatever N is - profiles/mma_cost.jsonl - and the legacy
 // mma.sync path at 3xTF32 is only 1.4x the FFMA peak.)
 #include <stdio.h>
 
@@ -147,14 +147,14 @@ struct SCfg {
   static constexpr int NPW = 4;          // producer warps
   static constexpr int LPP = SK_LPP;     // issuing lanes per producer warp.  The ~3 bulk copies per us a thread can issue are a
                                          // per-THREAD limit and lanes of one warp scale like separate warps in isolation
-                                         // (r02_ubench.jsonl), but here 2 lanes bought nothing (836 vs 844 k tok/s) and 4 lanes
+                                         // (ubench.jsonl), but here 2 lanes bought nothing (836 vs 844 k tok/s) and 4 lanes
                                          // with 16 stages lost 10 %: the divergent lanes' back-off sleeps stall each other
   static constexpr int NISS = NPW * LPP; // issuers; unit n belongs to issuer n % NISS
   static constexpr int NTHREADS = NCOMP + NPW * 32 + 32;  // + one warp whose lane 0 prefetches the next layer's K / V into L2
-  // Ring: ST stages of 144 KB / ST.  Measured on the headline (profiles/r02_stack_sweep.jsonl): 8 x 18 KB is faster than
+  // Ring: ST stages of 144 KB / ST.  Measured on the headline (profiles/stack_sweep.jsonl): 8 x 18 KB is faster than
   // 16 x 9 KB although the latter lets an attention warp own two stages (its next unit loads under the current one's
   // math: units phase 10.5 -> 8.4 us per layer) - one thread issues only ~3 bulk copies per us whatever their size
-  // (profiles/r02_ubench.jsonl), so halving the copies halves what the four producers can feed the GEMM phases.
+  // (profiles/ubench.jsonl), so halving the copies halves what the four producers can feed the GEMM phases.
   static constexpr int ST = SK_ST;       // ring stages
   static constexpr int STAGE = 147456 / ST;  // bytes per stage
   static constexpr int TCH = STAGE / (2 * HD * 4);  // cache rows per attention unit: [TCH K rows | TCH V rows] in one stage
@@ -343,7 +343,7 @@ __device__ __forceinline__ void gemm_phase(const Ring<Cf>& rg, const uint8_t* ri
     // The stages were read through the generic proxy (LDS) and will be overwritten through the async proxy
     // (cp.async.bulk): every reader orders its own reads before the release with a proxy fence.  Without it the
     // refill occasionally overtook a slow warp's loads (measured: 30 % of 24-token runs at B = 256 deviated
-    // bitwise; none with the fence - profiles/r02_stack_race.txt).
+    // bitwise; none with the fence - profiles/stack_race.txt).
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
     if (lane < cnt) mbar_arrive_n(rg.empty((n + lane) % Cf::ST), 1);  // this warp is done with the stages

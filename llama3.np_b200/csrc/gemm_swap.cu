@@ -460,7 +460,7 @@ cudaError_t launch_sw_t(const TcGemmArgs& a, cudaStream_t s) {
     while (ksplit > 1 && (ksplit - 1) * ((nkb + ksplit - 1) / ksplit) >= nkb) --ksplit;
     if (ksplit < 1) ksplit = 1;
   }
-  // Measured and rejected at the 8B shape, batch 32 (round 2, profiles/r02_swap_gemm_experiments.txt): balanced K-ranges
+  // Measured and rejected at the 8B shape, batch 32 (profiles/swap_gemm_experiments.txt): balanced K-ranges
   // (every CTA an equal contiguous range of (row block, k-block) units: gate|up 55.9 vs 54.2 us - the kernel is not
   // bound by the ragged second wave), a tile-contiguous copy of the weights read with one 16 KB bulk copy per stage
   // (5.06 vs 5.08 ms per step: not DRAM page locality either), a whole ring of weight stages requested ahead of the first

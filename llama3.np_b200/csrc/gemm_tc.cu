@@ -143,7 +143,7 @@ int tc_pick_bn(int kind, int rows, int N) {
   // epilogue and mainloop), BN = 64 leaves room for two - preferred unless L3_TF32_BN128 is set
   static const bool tf32_128 = getenv("L3_TF32_BN128") && atoi(getenv("L3_TF32_BN128")) != 0;
   if (kind == TC_TF32X3_2) {
-    // An M = 128 tcgen05.mma occupies the tensor pipe for 128 cycles whatever N is (profiles/r02_mma_cost.jsonl:
+    // An M = 128 tcgen05.mma occupies the tensor pipe for 128 cycles whatever N is (profiles/mma_cost.jsonl:
     // 132.7 cycles per MMA for N = 16 .. 256, bf16 and tf32 alike), so a tile's main loop costs the same for every
     // width and only the number of tile rounds matters: always the widest tile.
     static const int lm_bn = getenv("L3_LM_BN") ? atoi(getenv("L3_LM_BN")) : 256;

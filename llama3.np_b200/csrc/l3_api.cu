@@ -937,7 +937,7 @@ static int enqueue_decode_stack(L3Model* m, int B, int part = 0) {
   a.xlast_hi = m->xlast; a.xlast_lo = m->xlast_lo;
   a.dbg = m->d_stack_dbg;
   a.dbg_x = m->d_stack_dbgx;
-  // measured on the headline (profiles/r02_stack_sweep.jsonl): 64 rows + evict-first 841 k tok/s, both off 822 k, 256 rows 810 k
+  // measured on the headline (profiles/stack_sweep.jsonl): 64 rows + evict-first 841 k tok/s, both off 822 k, 256 rows 810 k
   static const int pf_rows = [] { const char* v = getenv("L3_STACK_PF"); return v ? atoi(v) : 64; }();
   static const int kv_ef = [] { const char* v = getenv("L3_STACK_KV_EVICT_FIRST"); return v ? atoi(v) : 1; }();
   a.pf_rows = pf_rows; a.kv_evict_first = kv_ef;

@@ -7,7 +7,7 @@
   8b-prefill   Llama-3-8B-shaped, bf16: prefill 2048                    (north_star 60 % target)
 
 Random-init weights generated on the device (l3_fill_random); timing = CUDA events on the
-library stream; decode tok/s counts generated tokens only; roofline per SURVEY.md 8(d).
+library stream; decode tok/s counts generated tokens only.
 """
 import argparse
 import ctypes as C

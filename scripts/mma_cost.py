@@ -6,7 +6,7 @@ alone, operands resident in shared memory (csrc/mma_probe.cu).  One JSON line pe
   python scripts/mma_cost.py --ctas 148 # every SM at once (power / clock effects)
 
 Reading: `total` / `peak` is the fraction of the dense tensor rate the MMA stream reaches; a flat `total` over N
-means narrow tiles waste the pipe (DESIGN.md 6)."""
+means narrow tiles waste the pipe."""
 import argparse
 import ctypes as C
 import json

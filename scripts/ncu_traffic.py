@@ -1,9 +1,9 @@
 #!/usr/bin/env python
-"""profiles/r02_traffic.json from an `ncu --set full` capture of decode_stack_kernel: DRAM bytes per launch
-(dram__bytes_read.sum + dram__bytes_write.sum), duration and the pipe / issue figures quoted in DESIGN.md 4.0.
+"""profiles/traffic.json from an `ncu --set full` capture of decode_stack_kernel: DRAM bytes per launch
+(dram__bytes_read.sum + dram__bytes_write.sum), duration and the pipe / issue figures.
 
-  ncu -i gpurun_out/r02_stack.ncu-rep --page raw --csv > profiles/r02_stack_kernel_ncu_full_raw.csv
-  python scripts/ncu_traffic.py profiles/r02_stack_kernel_ncu_full_raw.csv "<config text>" """
+  ncu -i gpurun_out/stack.ncu-rep --page raw --csv > profiles/stack_kernel_ncu_full_raw.csv
+  python scripts/ncu_traffic.py profiles/stack_kernel_ncu_full_raw.csv "<config text>" """
 import csv, json, os, sys
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 path, config = sys.argv[1], sys.argv[2]
@@ -32,5 +32,5 @@ for k in ("sm__inst_executed_pipe_fma.avg.pct_of_peak_sustained_active", "sm__th
             out["decode_stack_kernel"][k] = float(r[hdr.index(k)].replace(",", ""))
         except ValueError:
             pass
-json.dump(out, open(os.path.join(ROOT, "profiles", "r02_traffic.json"), "w"), indent=2)
+json.dump(out, open(os.path.join(ROOT, "profiles", "traffic.json"), "w"), indent=2)
 print(json.dumps(out, indent=2))

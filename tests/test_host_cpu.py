@@ -33,7 +33,7 @@ def test_tokenizer_matches_reference_on_its_own_vocabulary():
         ids = ref.encode(text)
         assert mine.encode(text) == ids
         assert mine.decode(ids) == ref.decode(ids)
-    assert mine.encode("I have a dream") == [1, 76, 505, 263, 12561]  # SURVEY.md 3.1
+    assert mine.encode("I have a dream") == [1, 76, 505, 263, 12561]
 
 
 def test_hf_permutation_roundtrip_and_meaning():

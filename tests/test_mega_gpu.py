@@ -90,7 +90,7 @@ def test_mega_cache_rows_match_the_oracle_over_repeated_generates():
     """Race detector for the persistent kernel's hand-offs: K / V rows of EVERY layer after repeated generates (bulk and
     lazy) against the oracle's caches.  A missing barrier between a phase's reads of the staged vector and the next
     staging's writes showed up only as a rare wrong row at the positions where the split count of the decode attention
-    changes - tokens mostly unchanged (scripts/mega_cache_check.py found it: 27 of 30 generates deviated)."""
+    changes - tokens mostly unchanged (27 of 30 generates deviated)."""
     args, w = _make("8b-like")
     ids = np.random.default_rng(3).integers(3, args.vocab_size, (1, 6))
     cap = args.max_seq_len

@@ -430,7 +430,7 @@ def test_batched_decode_ksplit_swapped_gemm_token_identical_fp32():
 
 def test_forward_between_generate_steps_leaves_the_loop_alone():
     """A forward call (with argmax) between l3_generate_begin and the first step, and between two steps, must not change
-    the generated stream: the forward entry points own their id / argmax buffers (advisor finding, round 1)."""
+    the generated stream: the forward entry points own their id / argmax buffers."""
     args = ModelArgs(dim=64, n_layers=2, n_heads=4, n_kv_heads=2, vocab_size=300, max_seq_len=48, max_batch_size=2)
     w = make_weights(args, 128, seed=31)
     ids = np.array([[5, 6, 7, 8], [9, 10, 11, 12]])

@@ -92,7 +92,7 @@ def test_stack_functional_surface_position_schedule():
 
 def test_stack_is_bitwise_deterministic():
     """Every reduction in the kernel has a fixed order, so repeated runs must agree bit for bit.  (This is the
-    detector of the cross-proxy race described in profiles/r02_stack_race.txt: without the proxy fence ~30 % of
+    detector of the cross-proxy race described in profiles/stack_race.txt: without the proxy fence ~30 % of
     such runs deviated.)"""
     import hashlib
     args, w = _model(6, 2000, 40, 256)
