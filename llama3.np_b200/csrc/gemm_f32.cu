@@ -1,6 +1,7 @@
 // fp32 projections of many rows on the 5th-generation tensor cores without giving up fp32's precision: C = A W^T with fp32 A and
-// W [N, K] fp32 or bf16.  Every fp32 value is cut into three bf16 parts of 8 significant bits each, x = x1 + x2 + x3 exactly, by
-// truncation, inside the kernel: TMA brings raw fp32 tiles, converter warps write the parts as operand tiles, and one thread
+// W [N, K] fp32 or bf16.  Every fp32 value is cut into three bf16 parts of 8 significant bits each, x = x1 + x2 + x3, by truncation,
+// inside the kernel (exact from 2^-110 up: the third part of a smaller number ends at bf16's smallest, 2^-133): TMA brings raw fp32
+// tiles, converter warps write the parts as operand tiles, and one thread
 // issues the products of the parts whose order is above 2^-24,
 //   a1 b1 | a1 b2 + a2 b1 + a2 b2 + a1 b3 + a3 b1          (W in bf16: a1 w | a2 w + a3 w),
 // the leading one and the corrections into two TMEM accumulators.  The tensor core drops the bits below an accumulator's last one

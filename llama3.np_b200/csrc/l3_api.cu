@@ -964,10 +964,12 @@ static int enqueue_decode_nodes(L3Model* m, int B, int ragged, int eos) {
     return L3_OK;
   }
   if (m->stack_ok && B >= m->stack_min_B) return enqueue_decode_stack(m, B);
-  // Small fp32 models: layers in one cluster, then the LM head with its argmax.  stories15M, 50 new tokens, us per call before (batch 1:
-  // decode_mega, 2 - 8: a kernel per product) -> here: batch 1 5874 -> 3628, 2 10105 -> 4502, 4 12632 -> 6162, 8 19323 -> 10046; 150 + 90
-  // tokens: batch 1 12316 -> 7936, 8 38394 -> 22714.  One forward step 265 -> 132, of batch 8 567 -> 313.  Larger models do not fit the
-  // cluster's shared memory (decode_cluster_max_batch); from stack_min_B sequences the clusters of decode_stack share the weights' loads.
+  // Small fp32 models: layers in one cluster, then the LM head with its argmax.  stories15M, us per call before (batch 1: decode_mega,
+  // 2 - 8: a kernel per product) -> here.  5 + 45 tokens: batch 1 5466 -> 3463, 2 9461 -> 4355, 4 12295 -> 5951, 8 19050 -> 9791; 400 + 111
+  // tokens: batch 1 14821 -> 10985, 2 23670 -> 12857, 4 30876 -> 20772, 5 38503 -> 29316, 8 47911 -> 36211.  One forward step at position
+  // 100 and 511: batch 1 267 -> 130 and 264 -> 143, 8 564 -> 316 and 565 -> 402.  Longer caches are not taken (one CTA walks a head's keys).
+  // Larger models do not fit the cluster's shared memory (decode_cluster_max_batch); from stack_min_B sequences the clusters of
+  // decode_stack share the weights' loads, between the two a kernel per product remains.
   if (B <= m->cl_maxB) {
     const int rc = enqueue_cluster_layers(m, nullptr, 0, 0, B);
     if (rc != L3_OK) return rc;

@@ -18,8 +18,11 @@
 //                           memory, then the state's and the outputs' products with U; operand blocks are fetched a phase ahead.
 // Every exponential has an argument <= 0: c is kept relative to blocks of 16 tokens, products between blocks take a reference
 // between them (e^(c_t - ref) e^(ref - c_j)), 8 x 8 blocks on the diagonal are formed pair by pair.  All operands of the tensor
-// products - keys, queries, scores, T, U and the state - are pairs hi + lo of bf16 values (16 significant bits), a product is
-// hi hi + hi lo + lo hi with fp32 accumulation; the inverse is fp32.
+// products - keys, queries, scores, T, U and the state - are pairs hi + lo of bf16 values (right to 2^-18), a product is
+// hi hi + hi lo + lo hi with fp32 accumulation; the inverse is fp32.  The chain these prompts took before keeps them in fp32: alone, a
+// layer's outputs are within 2^-15 of 64-bit ones here and within 2^-19 there; the logits, whose projections read bf16, are as far from
+// 64-bit ones either way (new over old, 8 seeds each: delta rule 1.0012 +- 0.0022 and 0.9992 +- 0.0018, gated linear attention
+// 1.0028 +- 0.0016, all three layers of that family 0.9945 +- 0.0022).  L3_RECUR_CHUNK=0 keeps the chain.
 #include <stdint.h>
 #include <stdlib.h>
 

@@ -98,3 +98,42 @@ def test_rows_that_no_query_sees_do_not_count(kind, value):
     got = m.forward_rows(ids, 0, list(range(M)))
     assert ris.err(got[:, :big], run(o, ids[0])[:, :big]) < 6e-2
     m.close()
+
+
+def _against_portions_of_8(m, vocab, batch, n):
+    """Several sequences at once against portions of 8 tokens, which run the FFMA kernels on fp32 queries and the same bf16 caches."""
+    ids = np.random.default_rng(n).integers(0, vocab, (batch, n))
+    whole = m.forward_rows(ids, 0, list(range(batch * n))).reshape(batch, n, -1)
+    parts = np.concatenate([m.forward_rows(ids[:, p:p + 8], p, list(range(batch * len(ids[0, p:p + 8])))).reshape(batch, -1, whole.shape[-1])
+                            for p in range(0, n, 8)], 1)
+    m.close()
+    return max(ris.err(whole[b], parts[b]) for b in range(batch))
+
+
+@pytest.mark.parametrize("n,batch", [(65, 3), (129, 2)])
+def test_packed_queries_of_softmax_layers(n, batch):
+    """Scores of a few hundred: queries rounded to 16 bits would move the logits by 5e-2 (restated in 64 bits), their pairs move them
+    by 1e-4."""
+    cfg = ris.config([ris.attn(4, 2, 64, 16.0, ff=128)], width=128, side=0)
+    m, _ = ris.build(cfg, 3, "bfloat16", max_seq_len=n + 3, max_batch_size=batch)
+    assert _against_portions_of_8(m, cfg["vocab"], batch, n) < 1e-2
+
+
+@pytest.mark.parametrize("n,batch", [(65, 3), (129, 2)])
+def test_two_maps_that_nearly_cancel(n, batch):
+    """lambda = 1 and queries of the second map 1 % from the first's: the head norm lifts what is left of a1 - a2, so that queries of 16
+    bits would move the logits by 0.18 and weights of 16 bits by 5e-2 (restated in 64 bits), pairs by 6e-4."""
+    a = mab.attn(2, 1, 64, 128, window=0, diff=0.3, scale=0.5, scaling=None, mlp=mab.dense(128))
+    cfg = mab.config([a], width=128)
+    t = mab.random_model(cfg, 4)
+    rng = np.random.default_rng(0)
+    for name, heads, off in (("q", 2, 0.01), ("k", 1, 0.0)):
+        for key in (f"l0.mix.{name}", f"l0.mix.{name}.b"):
+            w = t[key].reshape((heads, 2, 64) + t[key].shape[1:])
+            w[:, 1] = w[:, 0] * (1.0 + off * rng.standard_normal(w[:, 0].shape))
+            t[key] = w.reshape(t[key].shape)
+    for key in ("lq1", "lk1", "lq2"):
+        t[f"l0.mix.{key}"][:] = 0.0
+    t["l0.mix.lq1"][0], t["l0.mix.lk1"][0] = 1.0, np.log(1.7)    # lambda = 1.7 - 1 + 0.3
+    m, _ = mab.build(cfg, dtype="bfloat16", max_seq_len=n + 3, max_batch_size=batch, tensors=t)
+    assert _against_portions_of_8(m, cfg["vocab"], batch, n) < 2e-2
