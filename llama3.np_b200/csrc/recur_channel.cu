@@ -487,9 +487,9 @@ size_t recur_channel_ws_floats(int B, int L, int H, int DK, int DV) {
   return (size_t)B * H * ((L + CT - 1) / CT) * per;
 }
 
-// Portions from this length on.  A chunk costs ~20 us (gated linear attention) to ~35 us (delta rule: the triangular system) from one end to
-// the other whatever it holds; the chain costs 0.2 - 0.3 us per token, and more where its CTAs (a multiple of sequences x heads) fill
-// the chip.  One layer, prompt through the public call, chain against chunks in us: delta rule, 1 x 16 heads, 48 tokens 240 : 256, 96
+// Portions from this length on.  A chunk's CTA takes ~20 us (gated linear attention: 264 of them in 37 us) to ~39 us (delta rule, with the
+// triangular system: 512 in 155 us, one per SM at a time) whatever it holds; the chain takes 0.2 - 0.3 us per token, and more where its
+// CTAs (a multiple of sequences x heads) fill the chip.  One layer, prompt through the public call, chain against chunks in us: delta rule, 1 x 16 heads, 48 tokens 240 : 256, 96
 // 272 : 284, 128 306 : 308, 192 267 : 253, 400 347 : 284; 4 x 16 heads, 48 255 : 265, 64 278 : 269, 128 341 : 294.  Gated linear
 // attention, 1 x 2 heads, 48 tokens 152 : 158, 72 177 : 176, 96 188 : 180; 1 x 8 heads, 48 218 : 217, 64 228 : 220, 128 285 : 253.
 static int least_tokens(const RecurArgs& a) {
