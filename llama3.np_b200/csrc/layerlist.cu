@@ -1515,7 +1515,11 @@ static int ll_linear(L3Model* m, const void* W, const float* x32, const void* x1
   // half a tile: 600 rows at width 1024, per product 141 -> 52 us; the two-layer fp32 prompt 2852 -> 1630 us, at 12 tokens 1112 -> 554
   // us, at 20 tokens 1624 -> 668 us, an 8-sequence fp32 decode step of a pre-norm stack of width 1024 1.20 -> 0.35 ms.  The logits'
   // distance from 64-bit ones: 1.5e-6 -> 3.7e-7 of their size (sums of 128 terms in the tensor core, then fp32 sums).
-  if (ll->f32_tc && K >= 64 && N >= 64) {
+  // Below K = 128 a product is over before its pipeline is full, and the FFMA tiles win until there are ~1.5 million outputs: two layers
+  // at widths 64 and 96, FFMA below 128 : here for all, prompt of 9 tokens 168 : 197 and 180 : 208 us, 8 + 30 greedy tokens of 9
+  // sequences 2778 : 3696 and 3341 : 4252; 4096 columns at K = 64, 256 rows 130 : 132, 400 rows 125 : 124, 2000 rows 214 : 203.  At width
+  // 128 it wins from 9 rows on (265 -> 255, 6029 -> 5631).
+  if (ll->f32_tc && N >= 64 && (K >= 128 || (K >= 64 && (int64_t)rows * N >= 3 << 19))) {
     GemmF32Args t{};
     t.A = a.x; t.lda = ld; t.W = W; t.w_bf16 = m->bf16; t.rows = rows; t.N = N; t.K = K; t.epi = epi; t.e = e;
     t.part = m->gemm_part; t.part_bytes = (size_t)32 << 20; t.tile_cnt = m->gemm_cnt; t.tile_cnt_len = 1024; t.err = m->h_err;

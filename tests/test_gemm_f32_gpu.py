@@ -74,3 +74,15 @@ def test_infinities_and_nan(rows, n, k, bf16):
     fine = np.isfinite(want32)
     fine[-1] = False
     assert np.abs(got[fine] - want[fine]).max() < 6e-7 * np.sqrt(k) * 4
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("rows,n,k", [(9, 64, 64), (128, 97, 72), (129, 130, 64), (300, 64, 136), (127, 384, 96), (640, 256, 4096)])
+def test_products_alone(rows, n, k, bf16):
+    """The kernel by itself at sizes whose products the decoders leave to the FFMA tiles as well (K below 128): same bound."""
+    rng = np.random.default_rng(rows + n)
+    x, w = rng.standard_normal((rows, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
+    if bf16:
+        w = (np.ascontiguousarray(w).view(np.uint32) & 0xFFFF0000).view(np.float32)
+    want = x.astype(np.float64) @ w.astype(np.float64).T
+    assert np.linalg.norm(_product(x, w, bf16) - want) < 6e-7 * np.linalg.norm(want)
