@@ -26,9 +26,9 @@ extern bool g_l3_pdl_next;  // l3_api.cu; set right before ONE launch that shoul
 // GEMM needs ~200 KB of shared memory; if its neighbours in the stream ran with the default
 // carveout every GEMM launch would pay an SM drain + L1/shared reconfiguration.
 bool l3_carveout_seen(const void* fn);
+// cluster: blocks per thread-block cluster
 template <typename... KArgs, typename... Args>
-static inline cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                                   Args... args) {
+static inline cudaError_t launch_kc(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, int cluster, Args... args) {
   if (!l3_carveout_seen((const void*)kern))
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
   cudaLaunchConfig_t cfg{};
@@ -36,13 +36,27 @@ static inline cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute at[2];
+  int n = 0;
+  if (g_l3_pdl || g_l3_pdl_next) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = cluster;
+    at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+    ++n;
+  }
   cfg.attrs = at;
-  cfg.numAttrs = (g_l3_pdl || g_l3_pdl_next) ? 1 : 0;
+  cfg.numAttrs = n;
   g_l3_pdl_next = false;
   return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+static inline cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+  return launch_kc(kern, grid, block, smem, s, 1, args...);
 }
 
 // ------------------------------------------------------------------ numeric helpers

@@ -22,7 +22,7 @@
 // 1/8 of each slab's k rows): per k row one float4 of weights from the k-major slab (quarter warps read 128
 // contiguous bytes) and S / 4 broadcast float4s of activations from a k-major [K][S + 8] buffer (80-byte rows keep
 // the k-groups' reads in different banks) feed 48 FFMAs; k-groups are the high lane bits and are summed with shuffles.  (tcgen05 is the wrong tool
-// for S = 12 rows: an M = 128 MMA costs 128 cycles whatever N is - profiles/mma_cost.jsonl - and the legacy
+// for S = 12 rows: an M = 128 MMA costs 40 cycles below N = 64 - profiles/mma_cost.jsonl -, three of them less than FFMAs do, and the legacy
 // mma.sync path at 3xTF32 is only 1.4x the FFMA peak.)
 #include <stdio.h>
 

@@ -16,13 +16,14 @@
 //               accumulators and the two correction products go to a fourth; the epilogue adds
 //               the four in fp32.  End-to-end logits stay within ~1e-6 of the float64 reference.
 //
-// Warp roles in a 192-thread CTA (one 128 x BN output tile per CTA):
-//   warp 0: TMA producer   warp 1: TMEM allocator + MMA issuer   warps 2-5: epilogue
+// Warp roles in a 320-thread CTA:
+//   warp 0: TMA producer   warp 1: TMEM allocator + MMA issuer   warps 2-9: epilogue
 // synchronised by a STAGES-deep ring of full/empty mbarriers and one accumulator barrier.
 #include <cuda.h>
 #include <stdlib.h>
 
 #include <algorithm>
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -30,13 +31,8 @@
 #include "common.cuh"
 #include "gemm_tc.h"
 
-// Debug timeline (l3_debug_tc_timeline): CTA (0,0) stamps clock64 at pipeline milestones when enabled.
 __device__ unsigned long long g_tc_dbg[64];
-__device__ int g_tc_dbg_on = 0;
-#define TC_STAMP(i)                                                             \
-  do {                                                                          \
-    if (g_tc_dbg_on && blockIdx.x == 0 && blockIdx.y == 0) g_tc_dbg[i] = clock64(); \
-  } while (0)
+static std::atomic<unsigned long long*> g_tc_dbg_to{nullptr};  // where launches leave their timeline (null: nowhere)
 
 #include "gemm_tc_dev.cuh"
 
@@ -44,29 +40,34 @@ __device__ int g_tc_dbg_on = 0;
 // tile fastest, so the CTAs running at one time share a few weight tiles through L2).  The TMA
 // producer and the MMA issuer run ahead across tile boundaries; with two TMEM accumulator buffers
 // the epilogue warps drain tile i while the tensor core already works on tile i + 1.
-template <int KIND, int BN, int EPI>
-__global__ void __launch_bounds__(192, 1)
+template <int KIND, int BN, int CG, int EPI>
+__global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmB1,
-               int rows, int N, int K, int a_box_rows, int nst, int ksplit, float* part, int* tile_cnt, EpiArgs e) {
+               int rows, int N, int K, int bn, int a_box_rows, int nst, int ksplit, float* part, int* tile_cnt, int* err,
+               unsigned long long* dbg, EpiArgs e) {
   extern __shared__ uint8_t smem_raw[];
   pdl_launch();  // the next kernel may start its own prologue now
   if (threadIdx.x == 0) {
-    TC_STAMP(0);
-    // descriptor fetches overlap the barrier / TMEM set-up (the first TMA otherwise waits ~0.7 us for them)
+    TC_STAMP(dbg, 0);
+    // descriptor fetches overlap the barrier set-up (the first TMA otherwise waits ~0.7 us for them)
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmA0));
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmB0));
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmA1));
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmB1));
+    if (KIND != TC_BF16) {
+      asm volatile("prefetch.tensormap [%0];" ::"l"(&tmA1));
+      asm volatile("prefetch.tensormap [%0];" ::"l"(&tmB1));
+    }
   }
   TcPipe p;
-  tc_pipe_setup<KIND, BN>(p, smem_raw, nst);
+  p.dbg = dbg;
+  tc_pipe_setup<KIND, BN, CG>(p, smem_raw, nst, BN ? BN : bn);
+  tc_pipe_ready(p);
   pdl_wait();  // everything above overlapped the previous kernel; its outputs are visible from here
-  if (threadIdx.x == 0) TC_STAMP(1);
-  tc_gemm_run<KIND, BN, EPI>(p, &tmA0, &tmA1, &tmB0, &tmB1, rows, N, K, a_box_rows, ksplit, part, tile_cnt, e, blockIdx.x, gridDim.x);
-  if (threadIdx.x == 64) TC_STAMP(34);
-  tc_pipe_teardown<KIND, BN>(p);
-  if (threadIdx.x == 0) TC_STAMP(35);
+  if (threadIdx.x == 0) TC_STAMP(dbg, 1);
+  tc_gemm_run<KIND, BN, CG, EPI>(p, &tmA0, &tmA1, &tmB0, &tmB1, rows, N, K, a_box_rows, ksplit, part, tile_cnt, e, blockIdx.x / CG, gridDim.x / CG);
+  if (threadIdx.x == 64) TC_STAMP(dbg, 34);
+  tc_pipe_teardown<KIND, BN, CG>(p, err);
+  if (threadIdx.x == 0) TC_STAMP(dbg, 35);
 }
 
 // ------------------------------------------------------------------------------ host side
@@ -125,8 +126,10 @@ const CUtensorMap* tc_get_map(const void* ptr, bool is_bf16, int rows, int cols,
 int tc_debug_timeline(int enable, unsigned long long* out64) {
   if (out64 && cudaMemcpyFromSymbol(out64, g_tc_dbg, sizeof(unsigned long long) * 64) != cudaSuccess) return -1;
   unsigned long long z[64] = {0};
-  cudaMemcpyToSymbol(g_tc_dbg, z, sizeof z);
-  return cudaMemcpyToSymbol(g_tc_dbg_on, &enable, sizeof(int)) == cudaSuccess ? 0 : -1;
+  void* p = nullptr;
+  if (cudaMemcpyToSymbol(g_tc_dbg, z, sizeof z) != cudaSuccess || cudaGetSymbolAddress(&p, g_tc_dbg) != cudaSuccess) return -1;
+  g_tc_dbg_to = enable ? (unsigned long long*)p : nullptr;
+  return 0;
 }
 
 void tc_forget_maps() {
@@ -136,23 +139,17 @@ void tc_forget_maps() {
 
 bool tc_gemm_supported(int K) { return K % 8 == 0 && encode_fn() != nullptr; }
 
-int tc_pick_bn(int kind, int rows, int N) {
+static int pick_tf32(int kind, int rows, int N) {
   const int tm = (rows + 127) / 128;
-  const int cand[4] = {256, 128, 64, 32};
   // 3xTF32 keeps four accumulators per tile: BN = 128 fills the TMEM with ONE buffer (no overlap of
   // epilogue and mainloop), BN = 64 leaves room for two - preferred unless L3_TF32_BN128 is set
   static const bool tf32_128 = getenv("L3_TF32_BN128") && atoi(getenv("L3_TF32_BN128")) != 0;
   if (kind == TC_TF32X3_2) {
-    // An M = 128 tcgen05.mma occupies the tensor pipe for 128 cycles whatever N is (profiles/mma_cost.jsonl:
-    // 132.7 cycles per MMA for N = 16 .. 256, bf16 and tf32 alike), so a tile's main loop costs the same for every
-    // width and only the number of tile rounds matters: always the widest tile.
     static const int lm_bn = getenv("L3_LM_BN") ? atoi(getenv("L3_LM_BN")) : 256;
     return lm_bn;
   }
-  for (int i = (kind == TC_TF32X3 ? (tf32_128 ? 1 : 2) : 0); i < 4; ++i) {
-    const int bn = cand[i];
-    if ((long)tm * ((N + bn - 1) / bn) >= 120 || bn == 32) return bn;
-  }
+  for (int bn = tf32_128 ? 128 : 64; bn > 32; bn >>= 1)
+    if ((long)tm * ((N + bn - 1) / bn) >= 120) return bn;
   return 32;
 }
 
@@ -164,52 +161,58 @@ static int sm_count() {
   return n[dev & 15] > 0 ? n[dev & 15] : 148;
 }
 
-// bf16: tile width and K split together, by the cycles of the busiest CTA.  A k-block (64 of K) costs four MMAs of ~132 cycles
-// whatever the width (mma_probe.cu), or the 85 bytes per cycle that a CTA's tiles arrive at (128 x 256: 578 cycles) - so wide tiles
-// are as cheap as narrow ones, and few tiles are better cut along K than along N.  The last tile's epilogue is not overlapped
-// (~14 cycles per column for a plain store, 20 - 24 where it reads as well), a split adds the partial tiles' way through L2.
-// Against the rule this replaces (the widest tile that gives 120 tiles, K cut only below 74): 1462 x 2048 x 8192, 116 -> 70 us (96
-// tiles of 256 in one round instead of 192 of 128 in two); 768 x 2048 x 10240, 150 -> 55 us (48 tiles x 3 slices instead of 192 of 64);
-// two-layer prompts: 2 x 731 tokens at width 2048 775 -> 676 us, 200 tokens at width 4096 647 -> 524 us, 700 tokens 1035 -> 841 us.
-static void pick_bf16(const TcGemmArgs& a, int sms, int* bn_out, int* ks_out) {
-  const int tm = (a.rows + 127) / 128, nkb = (a.K + 63) / 64;
-  const int per_col = a.epi == EPI_ROPE_KV ? 24 : a.epi == EPI_RESID ? 20 : 14;
+// bf16: CTAs per tile (1, or a pair on 256 rows), tile width and K split together, by the cycles of the busiest CTA.  A k-block (64 of
+// K) costs a CTA four MMAs of bn / 2 cycles (mma_probe.cu: 128 at 256 columns, 64 at 128, not below 40 - 48) or its shared memory's
+// bandwidth, which the arriving tiles and the products' reads share: measured 583 cycles at 256 columns and 354 at 128 for a CTA alone,
+// 500, 390 and 275 at 256, 192 and 128 in a pair, whose CTAs hold half of the weight tile each.  The last tile's epilogue is not
+// overlapped, a split adds the partial tiles' way through L2, a pair its barrier at the start.  Any width in steps of 32 is taken, so
+// that the tiles of a shape fill the machine's last round.  Over 36 shapes of 130 - 4096 rows the choice is 0.8 % behind the best of
+// all (at most 7 %); what it gave against single CTAs and widths of 2^n, us (fp32 results; swiglu: bf16): 1462 x 2048 x 8192 66 -> 45,
+// 1462 x 16384 x 2048 swiglu 122 -> 73, 4096 x 28672 x 4096 swiglu 700 -> 593 (1.62 PFLOP/s), 4096 x 6144 x 4096 165 -> 138,
+// 2048 x 2048 x 8192 59 -> 51, 200 x 6144 x 4096 27 -> 20, 300 x 1024 x 1024 12.5 -> 8.5.
+static void pick_bf16(const TcGemmArgs& a, int sms, int* cg_out, int* bn_out, int* ks_out) {
+  const int nkb = (a.K + 63) / 64;
+  const double per_col = a.epi == EPI_ROPE_KV ? 26 : a.epi == EPI_RESID ? 24 : a.epi == EPI_SWIGLU ? 14 : 20;
   double best = 0;
-  for (int bn = 256; bn >= 32; bn >>= 1) {
-    const int tiles = tm * ((a.N + bn - 1) / bn);
-    const double block = std::max(528.0, (16384.0 + 128.0 * bn) / 85.0), epi = per_col * bn;
-    for (int ks = 1; ks <= 8; ++ks) {
-      const int per = (nkb + ks - 1) / ks;
-      if (ks > 1 && (!a.part || !a.tile_cnt || tiles > a.tile_cnt_len || per < 3 || (ks - 1) * per >= nkb ||
-                     (size_t)tm * 128 * ((a.N + bn - 1) / bn) * bn * sizeof(float) * ks > a.part_bytes)) continue;
-      const int rounds = (tiles * ks + sms - 1) / sms;
-      const double main = per * block;
-      const double cost = (rounds - 1) * std::max(main, epi) + main + epi + (ks > 1 ? bn * (28.0 + 11.0 * ks) : 0.0);
-      if (best == 0 || cost < best * 0.99) { best = cost; *bn_out = bn; *ks_out = ks; }
+  for (int cg = 1; cg <= (a.rows > 128 ? 2 : 1); ++cg) {
+    const int tm = (a.rows + 128 * cg - 1) / (128 * cg);
+    for (int bn = 256; bn >= 32; bn -= 32) {
+      const int tn = (a.N + bn - 1) / bn, tiles = tm * tn;
+      const double block = std::max(2.0 * bn, cg == 1 ? 128 + 1.79 * bn : 160 + 0.93 * bn), epi = 1500 + per_col * bn;
+      for (int ks = 1; ks <= (a.epi == EPI_ARGMAX ? 1 : 8); ++ks) {
+        const int per = (nkb + ks - 1) / ks;
+        if (ks > 1 && (!a.part || !a.tile_cnt || tiles * cg > a.tile_cnt_len || per < 3 || (ks - 1) * per >= nkb ||
+                       (size_t)tiles * cg * 128 * bn * sizeof(float) * ks > a.part_bytes)) continue;
+        const int rounds = (tiles * ks + sms / cg - 1) / (sms / cg);
+        const double main = per * block;
+        const double cost = (cg - 1) * 1230 + (rounds - 1) * std::max(main, epi) + main + epi + (ks > 1 ? 1500 + bn * (28.0 + 11.0 * ks) : 0.0);
+        if (best == 0 || cost < best * 0.99) { best = cost; *cg_out = cg; *bn_out = bn; *ks_out = ks; }
+      }
     }
   }
 }
 
-template <int KIND, int BN, int EPI>
+template <int KIND, int BN, int CG, int EPI>
 static cudaError_t launch_tc_t(const TcGemmArgs& a, cudaStream_t s) {
-  using Cf = TcCfg<KIND, BN>;
-  auto kern = gemm_tc_kernel<KIND, BN, EPI>;
+  using Cf = TcCfg<KIND, BN, CG>;
+  auto kern = gemm_tc_kernel<KIND, BN, CG, EPI>;
   static bool attr_done[16] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_done[dev & 15]) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cf::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cf::SMEM_MAX);
     if (e != cudaSuccess) return e;
     attr_done[dev & 15] = true;
   }
   constexpr bool b16 = KIND == TC_BF16;
+  const int bn = BN ? BN : a.bn, TM = 128 * CG;
   const int a_box = a.rows >= 128 ? 128 : ((a.rows + 7) & ~7);
   const CUtensorMap* A0 = g_maps.get(a.A[0], b16, a.rows, a.K, a_box);
-  const CUtensorMap* B0 = g_maps.get(a.W[0], b16, a.N, a.K, BN);
+  const CUtensorMap* B0 = g_maps.get(a.W[0], b16, a.N, a.K, bn / CG);
   const CUtensorMap* A1 = Cf::PARTS == 2 ? g_maps.get(a.A[1], b16, a.rows, a.K, a_box) : A0;
-  const CUtensorMap* B1 = Cf::PARTS == 2 ? g_maps.get(a.W[1], b16, a.N, a.K, BN) : B0;
+  const CUtensorMap* B1 = Cf::PARTS == 2 ? g_maps.get(a.W[1], b16, a.N, a.K, bn / CG) : B0;
   if (!A0 || !B0 || !A1 || !B1) return cudaErrorInvalidValue;
-  const int ntiles = ((a.N + BN - 1) / BN) * ((a.rows + 127) / 128);
+  const int ntiles = ((a.N + bn - 1) / bn) * ((a.rows + TM - 1) / TM);
   const int sms = sm_count();
   const int nkb_all = (a.K + Cf::BK - 1) / Cf::BK;
   // K-split (deterministic, see the epilogue) when the output tiles cover less than half the machine:
@@ -218,58 +221,53 @@ static cudaError_t launch_tc_t(const TcGemmArgs& a, cudaStream_t s) {
   int ksplit = std::max(1, a.ksplit);
   if (!a.ksplit && a.part && a.tile_cnt && ntiles * 2 <= sms && ntiles <= a.tile_cnt_len) {
     ksplit = std::min(std::min(8, sms / ntiles), nkb_all / 3);
-    const size_t need = (size_t)((a.rows + 127) / 128 * 128) * ((a.N + BN - 1) / BN * BN) * sizeof(float);
+    const size_t need = (size_t)((a.rows + 127) / 128 * 128) * ((a.N + bn - 1) / bn * bn) * sizeof(float);
     while (ksplit > 1 && need * ksplit > a.part_bytes) --ksplit;
     // every slice must own at least one k-block
     while (ksplit > 1 && (ksplit - 1) * ((nkb_all + ksplit - 1) / ksplit) >= nkb_all) --ksplit;
     if (ksplit < 1) ksplit = 1;
   }
-  dim3 grid(std::min(ntiles * ksplit, sms));
+  dim3 grid(std::min(ntiles * ksplit, sms / CG) * CG);
   // ring depth: no deeper than the K loop; L3_GEMM_MAXSTAGES caps it further so that two kernels' CTAs
   // fit one SM (programmatic dependent launch can then overlap a kernel's prologue with its predecessor)
-  static const int max_st = getenv("L3_GEMM_MAXSTAGES") ? atoi(getenv("L3_GEMM_MAXSTAGES")) : Cf::STAGES;
+  static const int env_st = getenv("L3_GEMM_MAXSTAGES") ? atoi(getenv("L3_GEMM_MAXSTAGES")) : 8;
   const int nkb = (nkb_all + ksplit - 1) / ksplit;
-  const int nst = std::max(2, std::min(std::min(Cf::STAGES, max_st), nkb));
-  const size_t smem = (size_t)nst * Cf::STAGE_BYTES + Cf::EPI_BYTES + 1024 + 512;
-  return launch_k(kern, grid, dim3(192), smem, s, *A0, *A1, *B0, *B1, a.rows, a.N, a.K, a_box, nst, ksplit, a.part, a.tile_cnt, a.e);
+  const int nst = std::max(2, std::min(std::min(Cf::stages(bn), env_st), nkb));
+  return launch_kc(kern, grid, dim3(TC_THREADS), (size_t)Cf::smem(bn, nst), s, CG, *A0, *A1, *B0, *B1, a.rows, a.N, a.K, bn, a_box, nst, ksplit, a.part, a.tile_cnt,
+                  a.err, g_tc_dbg_to.load(), a.e);
 }
 
-
-template <int KIND, int BN>
+template <int KIND, int BN, int CG>
 static cudaError_t launch_tc_e(const TcGemmArgs& a, cudaStream_t s) {
   switch (a.epi) {
-    case EPI_STORE: return launch_tc_t<KIND, BN, EPI_STORE>(a, s);
-    case EPI_RESID: return launch_tc_t<KIND, BN, EPI_RESID>(a, s);
-    case EPI_SWIGLU: return launch_tc_t<KIND, BN, EPI_SWIGLU>(a, s);
-    case EPI_ARGMAX: return launch_tc_t<KIND, BN, EPI_ARGMAX>(a, s);
-    default: return launch_tc_t<KIND, BN, EPI_ROPE_KV>(a, s);
+    case EPI_STORE: return launch_tc_t<KIND, BN, CG, EPI_STORE>(a, s);
+    case EPI_RESID: return launch_tc_t<KIND, BN, CG, EPI_RESID>(a, s);
+    case EPI_SWIGLU: return launch_tc_t<KIND, BN, CG, EPI_SWIGLU>(a, s);
+    case EPI_ARGMAX: return launch_tc_t<KIND, BN, CG, EPI_ARGMAX>(a, s);
+    default: return launch_tc_t<KIND, BN, CG, EPI_ROPE_KV>(a, s);
   }
 }
 
 cudaError_t launch_gemm_tc(const TcGemmArgs& args, cudaStream_t s) {
   TcGemmArgs a = args;
-  int bn = a.bn > 0 ? a.bn : tc_pick_bn(a.kind, a.rows, a.N);
-  if (a.kind == TC_BF16 && a.bn <= 0 && a.epi != EPI_ARGMAX) pick_bf16(a, sm_count(), &bn, &a.ksplit);
   if (a.kind == TC_BF16) {
-    switch (bn) {
-      case 256: return launch_tc_e<TC_BF16, 256>(a, s);
-      case 128: return launch_tc_e<TC_BF16, 128>(a, s);
-      case 64: return launch_tc_e<TC_BF16, 64>(a, s);
-      default: return launch_tc_e<TC_BF16, 32>(a, s);
-    }
+    int cg = 1;
+    pick_bf16(a, sm_count(), &cg, &a.bn, &a.ksplit);
+    return cg == 2 ? launch_tc_e<TC_BF16, 0, 2>(a, s) : launch_tc_e<TC_BF16, 0, 1>(a, s);
   }
+  const int bn = pick_tf32(a.kind, a.rows, a.N);
   if (a.kind == TC_TF32X3_2) {  // one main accumulator: only the LM-head epilogues are instantiated
     const bool argmax = a.epi == EPI_ARGMAX;
     switch (bn) {
-      case 256: return argmax ? launch_tc_t<TC_TF32X3_2, 256, EPI_ARGMAX>(a, s) : launch_tc_t<TC_TF32X3_2, 256, EPI_STORE>(a, s);
-      case 128: return argmax ? launch_tc_t<TC_TF32X3_2, 128, EPI_ARGMAX>(a, s) : launch_tc_t<TC_TF32X3_2, 128, EPI_STORE>(a, s);
-      default: return argmax ? launch_tc_t<TC_TF32X3_2, 64, EPI_ARGMAX>(a, s) : launch_tc_t<TC_TF32X3_2, 64, EPI_STORE>(a, s);
+      case 256: return argmax ? launch_tc_t<TC_TF32X3_2, 256, 1, EPI_ARGMAX>(a, s) : launch_tc_t<TC_TF32X3_2, 256, 1, EPI_STORE>(a, s);
+      case 128: return argmax ? launch_tc_t<TC_TF32X3_2, 128, 1, EPI_ARGMAX>(a, s) : launch_tc_t<TC_TF32X3_2, 128, 1, EPI_STORE>(a, s);
+      default: return argmax ? launch_tc_t<TC_TF32X3_2, 64, 1, EPI_ARGMAX>(a, s) : launch_tc_t<TC_TF32X3_2, 64, 1, EPI_STORE>(a, s);
     }
   }
   switch (bn) {
-    case 128: return launch_tc_e<TC_TF32X3, 128>(a, s);
-    case 64: return launch_tc_e<TC_TF32X3, 64>(a, s);
-    default: return launch_tc_e<TC_TF32X3, 32>(a, s);
+    case 128: return launch_tc_e<TC_TF32X3, 128, 1>(a, s);
+    case 64: return launch_tc_e<TC_TF32X3, 64, 1>(a, s);
+    default: return launch_tc_e<TC_TF32X3, 32, 1>(a, s);
   }
 }
 

@@ -13,8 +13,7 @@ struct TcGemmArgs {
   const void* A[2];     // activations [rows, K]: bf16, or fp32 (hi, lo) pair
   const void* W[2];     // weights [N, K], same element kind
   int rows, N, K;
-  int bn;               // 0 = choose (bf16: together with the K split)
-  int ksplit;           // set by the launcher
+  int bn, ksplit;       // set by the launcher
   int epi;
   EpiArgs e;
   // optional caller-owned scratch for the deterministic K-split of gemm_tc.cu (null: never split)
@@ -22,6 +21,7 @@ struct TcGemmArgs {
   size_t part_bytes;
   int* tile_cnt;     // zero-initialised arrival counters, one per output tile
   int tile_cnt_len;
+  int* err;             // gemm_tc.cu: set to 1 when a wait inside the kernel ran out (null: the launch fails)
 };
 
 cudaError_t launch_gemm_tc(const TcGemmArgs& a, cudaStream_t s);
@@ -30,7 +30,6 @@ bool gemm_swap_supported(int rows, int N);
 cudaError_t launch_gemm_swap(const TcGemmArgs& a, cudaStream_t s);
 cudaError_t launch_split_tf32(const float* src, float* hi, float* lo, int64_t n, cudaStream_t s);
 bool tc_gemm_supported(int K);
-int tc_pick_bn(int kind, int rows, int N);
 void tc_forget_maps();
 int tc_debug_timeline(int enable, unsigned long long* out64);
 // cached 2-D tensor map of a row-major [rows, cols] matrix: box = 128 bytes of columns x box_rows rows,

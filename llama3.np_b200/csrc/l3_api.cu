@@ -357,6 +357,8 @@ extern "C" int l3_finalize(L3Model* m) {
     CK(m, cudaMalloc((void**)&m->gemm_cnt, 1024 * sizeof(int)));
     CK(m, cudaMemsetAsync(m->gemm_cnt, 0, 1024 * sizeof(int), m->stream));
   }
+  if (m->tc_ok && m->bf16)
+    if (const int rc = make_err_word(m)) return rc;
   if (m->tc_ok && !m->bf16) {
     CK(m, cudaMalloc((void**)&m->xn_lo, ct * m->D * 4));
     CK(m, cudaMalloc((void**)&m->ctx_lo, ct * m->HN * m->HD * 4));
@@ -425,7 +427,8 @@ extern "C" int l3_finalize(L3Model* m) {
     if (m->cl_maxB) {
       CK(m, cudaMalloc((void**)&m->d_cl_done, sizeof(int)));
       CK(m, cudaMemset(m->d_cl_done, 0, sizeof(int)));
-      if (const int rc = make_err_word(m)) return rc;
+      if (!m->h_err)
+        if (const int rc = make_err_word(m)) return rc;
     }
     if (m->mega_ok) {
       CK(m, cudaMalloc((void**)&m->d_mega_bar, 64));
@@ -582,15 +585,15 @@ static int linear(L3Model* m, LinearArgs& a, Feed feed, const float* w_hi, const
     return L3_OK;
   }
   TcGemmArgs t{};
-  t.rows = a.rows; t.N = a.N; t.K = a.K; t.epi = a.epi; t.e = a.e; t.bn = 0;
-  t.part = m->gemm_part; t.part_bytes = (size_t)32 << 20; t.tile_cnt = m->gemm_cnt; t.tile_cnt_len = 1024;
+  t.rows = a.rows; t.N = a.N; t.K = a.K; t.epi = a.epi; t.e = a.e;
+  t.part = m->gemm_part; t.part_bytes = (size_t)32 << 20; t.tile_cnt = m->gemm_cnt; t.tile_cnt_len = 1024; t.err = m->h_err;
   if (m->bf16) {
     t.kind = TC_BF16;
     t.A[0] = feed == FEED_CTX ? m->ctx16 : feed == FEED_H ? m->h16 : n16;
     t.W[0] = a.W;
   } else {
     // LM head (rows >> tiles' K): one main accumulator is enough for K <= 512 and halves the TMEM columns
-    // (an MMA costs 128 cycles whatever its width, so the LM head wants 256-wide tiles; L3_LM_2ACC=0 restores the
+    // (256-wide tiles: the operands' way through shared memory is what a tile costs; L3_LM_2ACC=0 restores the
     // four-accumulator 64-wide tiles)
     static const bool lm2 = !(getenv("L3_LM_2ACC") && atoi(getenv("L3_LM_2ACC")) == 0);
     t.kind = (lm2 && feed == FEED_LAST_NORM && a.K <= 512 && (a.epi == EPI_ARGMAX || a.epi == EPI_STORE)) ? TC_TF32X3_2 : TC_TF32X3;
@@ -946,7 +949,7 @@ static int enqueue_decode_stack(L3Model* m, int B, int part = 0) {
   TcGemmArgs t{};
   t.kind = m->D <= 512 ? TC_TF32X3_2 : TC_TF32X3;
   t.A[0] = m->xlast; t.A[1] = m->xlast_lo; t.W[0] = m->lm_hi; t.W[1] = m->lm_lo;
-  t.rows = B; t.N = m->VS; t.K = m->D; t.bn = 0; t.epi = EPI_ARGMAX;
+  t.rows = B; t.N = m->VS; t.K = m->D; t.epi = EPI_ARGMAX;
   t.e.best = m->d_best; t.e.col_offset = 0; t.e.ld_out = m->VS;
   LAUNCH(m, launch_gemm_tc(t, m->stream));
   if (part == 2) return L3_OK;

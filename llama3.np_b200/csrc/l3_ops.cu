@@ -87,7 +87,7 @@ extern "C" int l3_op_linear(int device, const float* x, const float* w, int rows
   } else if (path == 3 || path == 4) {  // tcgen05: bf16 operands, or the 3xTF32 split of fp32 operands (4: swapped roles)
     if (!tc_gemm_supported(k)) return L3_EINVAL;
     TcGemmArgs t{};
-    t.rows = rows; t.N = n; t.K = k; t.epi = EPI_STORE; t.e = a.e; t.bn = 0;
+    t.rows = rows; t.N = n; t.K = k; t.epi = EPI_STORE; t.e = a.e;
     if (w_bf16) {
       bf16* dxb = sc.dev<bf16>((size_t)rows * k);
       if (!dxb) return L3_ENOMEM;

@@ -1503,8 +1503,8 @@ static int ll_linear(L3Model* m, const void* W, const float* x32, const void* x1
   if (mirror) {
     TcGemmArgs t{};
     t.kind = TC_BF16; t.A[0] = x16; t.W[0] = W;
-    t.rows = rows; t.N = N; t.K = K; t.epi = epi; t.e = e; t.bn = 0;
-    t.part = m->gemm_part; t.part_bytes = (size_t)32 << 20; t.tile_cnt = m->gemm_cnt; t.tile_cnt_len = 1024;
+    t.rows = rows; t.N = N; t.K = K; t.epi = epi; t.e = e;
+    t.part = m->gemm_part; t.part_bytes = (size_t)32 << 20; t.tile_cnt = m->gemm_cnt; t.tile_cnt_len = 1024; t.err = m->h_err;
     static const bool swap_on = !(getenv("L3_GEMM_SWAP") && atoi(getenv("L3_GEMM_SWAP")) == 0);
     if (swap_on && gemm_swap_supported(rows, N)) LAUNCH(m, launch_gemm_swap(t, m->stream));
     else LAUNCH(m, launch_gemm_tc(t, m->stream));
@@ -1698,7 +1698,7 @@ static int ll_latent_prompt(L3Model* m, LLLayer& Ly, LLState& St, int B, int L) 
       TcGemmArgs t{};
       t.kind = TC_BF16; t.A[0] = rows; t.W[0] = Ly.w_ukv; t.rows = T; t.N = n_exp; t.K = Dk; t.epi = EPI_STORE;
       t.e = store_to(nullptr, (bf16*)ll->lat_exp + (size_t)i * m->M * n_exp, n_exp);
-      t.part = m->gemm_part; t.part_bytes = (size_t)32 << 20; t.tile_cnt = m->gemm_cnt; t.tile_cnt_len = 1024;
+      t.part = m->gemm_part; t.part_bytes = (size_t)32 << 20; t.tile_cnt = m->gemm_cnt; t.tile_cnt_len = 1024; t.err = m->h_err;
       LAUNCH(m, launch_gemm_tc(t, m->stream));
     }
     at.b0 = b0;

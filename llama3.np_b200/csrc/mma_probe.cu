@@ -1,9 +1,10 @@
 // Micro-benchmark, not on any product path: what does one tcgen05.mma (M = 128, K = 32 bytes) cost as a function
 // of its kind (bf16 / tf32), its width N and the number of TMEM accumulators the issuing thread rotates over?
-// The GEMM designs (gemm_tc.cu, gemm_swap.cu) rest on this number (an M = 128 MMA costs about the same for
-// N = 32 as for N = 256, so narrow tiles buy parallelism, not time); scripts/mma_cost.py sweeps it.
+// The GEMM designs (gemm_tc.cu, gemm_swap.cu) rest on this number (N / 2 cycles from N = 128, 48 at 64, 40 below, bf16 and tf32
+// alike); scripts/mma_cost.py sweeps it.  It is the tensor pipe's only while the issuing code keeps up: with a division for the
+// accumulator's turn between the instructions this probe showed 133 cycles for every width.
 //
-// One warp allocates the whole TMEM, one thread issues `iters` groups of four MMAs on zero-filled, 128-byte
+// One warp allocates the whole TMEM, one of its lanes (elected, so that operands stay in uniform registers) issues `iters` groups of four MMAs on zero-filled, 128-byte
 // swizzled K-major operand tiles that stay in shared memory (no TMA, no epilogue: the tensor pipe alone) and
 // commits them to an mbarrier; clock64 around the issue loop and around issue + completion.
 #include <stdio.h>
@@ -37,23 +38,25 @@ __global__ void __launch_bounds__(128, 1) mma_probe_kernel(int n, int nacc, int 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<uint32_t*>(smem_raw + (slot - raw));
-  if (threadIdx.x == 0) {
+  const int warp = __shfl_sync(L3_FULL, threadIdx.x >> 5, 0);
+  if (warp == 0 && elect_one()) {
     constexpr uint32_t FMT = KIND == TC_BF16 ? 1u : 2u;
     const uint32_t idesc = (1u << 4) | (FMT << 7) | (FMT << 10) | ((uint32_t)(n >> 3) << 17) | ((128u >> 4) << 24);
     const uint64_t ad = umma_desc_sw128(a_addr), bd = umma_desc_sw128(b_addr);
-    auto group = [&](int i) {  // four 32-byte K slices of the swizzle atom, as in the GEMM main loops
+    int turn = 0;
+    auto group = [&]() {  // four 32-byte K slices of the swizzle atom, as in the GEMM main loops
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
-        const uint32_t acc = tmem_base + (uint32_t)(((i * 4 + kk) % nacc) * n);
-        tc_mma<KIND>(acc, ad + (uint64_t)(kk * 2), bd + (uint64_t)(kk * 2), idesc, 1u);
+        tc_mma<KIND>(tmem_base + (uint32_t)(turn * n), ad + (uint64_t)(kk * 2), bd + (uint64_t)(kk * 2), idesc, 1u);
+        if (++turn == nacc) turn = 0;
       }
     };
-    for (int i = 0; i < 4; ++i) group(i);  // warm-up
+    for (int i = 0; i < 4; ++i) group();  // warm-up
     tc_commit(bar);
     mbar_wait(bar, 0);
     tc_fence_after();
     const long long t0 = clock64();
-    for (int i = 0; i < iters; ++i) group(i);
+    for (int i = 0; i < iters; ++i) group();
     const long long t1 = clock64();
     tc_commit(bar);
     mbar_wait(bar, 1);
