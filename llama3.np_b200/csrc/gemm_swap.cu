@@ -1,6 +1,6 @@
 // Tensor-core projections for 9..128 activation rows (batched decode): y = x W^T with the roles
 // of the MMA operands SWAPPED - a tile's 128-row operand is a block of WEIGHT rows and the batch
-// is the N dimension (32 / 64 / 128 columns).  With the batch as the 128-row operand
+// is the N dimension (16 / 32 / 64 / 128 columns).  With the batch as the 128-row operand
 // (gemm_tc.cu) every CTA re-reads the whole activation tile to stream only 32 weight rows; here a
 // CTA streams 128 weight rows per 16-128 KB of activations, so shared-memory ingress is spent on
 // the bytes that matter (weights are read exactly once from HBM, the HBM-bound regime of
@@ -49,6 +49,12 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* tm,
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
       ::"r"(dst), "l"(tm), "r"(c0), "r"(c1), "r"(bar) : "memory");
 }
+// one lane of the (whole) warp, known as one to the compiler (see gemm_tc_dev.cuh)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
@@ -88,45 +94,54 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
+constexpr int SW_THREADS = 224;  // warp 0 = weight copies, warp 1 = TMEM + MMA, warps 2-5 = epilogue, warp 6 = activation copies
 // BNA = batch columns of the tile (activation rows padded up)
 template <int KIND, int BNA> struct SwCfg {
   static constexpr int PARTS = KIND == TC_TF32X3 ? 2 : 1;
-  static constexpr int BMW = 128;                       // weight rows per tile
+  static constexpr int BMW = 128;                       // weight rows of the MMA; a tile holds h <= BMW of them
   static constexpr int BK = KIND == TC_BF16 ? 64 : 32;  // elements per 128-byte row
-  static constexpr int W_BYTES = BMW * 128, X_BYTES = BNA * 128;
-  static constexpr int STAGE_BYTES = PARTS * (W_BYTES + X_BYTES);
+  static constexpr int X_BYTES = BNA * 128;
+  __host__ __device__ static constexpr int w_bytes(int h) { return (h + 7) / 8 * 1024; }
+  __host__ __device__ static constexpr int stage_bytes(int h) { return PARTS * (w_bytes(h) + X_BYTES); }
   // (bf16 with four round-robin accumulators was measured: no gain at 8B batch 32, so one accumulator)
   static constexpr int NACC = KIND == TC_TF32X3 ? 4 : 1;
-  static constexpr int ACC_COLS = NACC * BNA;
+  static constexpr int AW = BNA < 32 ? 32 : BNA;        // TMEM columns from one accumulator to the next (read 32 at a time)
+  static constexpr int CJ = BNA < 32 ? BNA : 32;        // rows of an epilogue chunk
+  static constexpr int ACC_COLS = NACC * AW;
   static constexpr int NBUF = 2 * ACC_COLS <= 512 ? 2 : 1;
   static constexpr int TMEM_COLS = NBUF * ACC_COLS <= 32 ? 32 : NBUF * ACC_COLS <= 64 ? 64 : NBUF * ACC_COLS <= 128 ? 128
                                    : NBUF * ACC_COLS <= 256 ? 256 : 512;
-  static constexpr int STAGES_RAW = (232448 - 1024 - 512) / STAGE_BYTES;
-  static constexpr int STAGES = STAGES_RAW > 10 ? 10 : STAGES_RAW;
-  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 512;
+  // The MMA reads BMW rows; behind a tile's h it reads whatever follows in shared memory (those accumulators are not looked at), so
+  // low tiles leave room for more stages - what keeps DRAM busy is the bytes in flight - and the last stage is followed by a tile's rest.
+  static constexpr int MAX_STAGES = 32, REST = BMW * 128, SMEM_MAX = 232448, BARS = 1024;
+  __host__ __device__ static constexpr int stages(int h) {
+    const int n = (SMEM_MAX - 1024 - BARS - REST) / stage_bytes(h);
+    return n > MAX_STAGES ? MAX_STAGES : n;
+  }
   static constexpr uint32_t FMT = KIND == TC_BF16 ? 1u : 2u;
   // D fp32, both operands K-major, N = BNA, M = 128
   static constexpr uint32_t IDESC = (1u << 4) | (FMT << 7) | (FMT << 10) | ((uint32_t)(BNA >> 3) << 17) | ((128u >> 4) << 24);
 };
 
 template <int KIND, int BNA, int EPI>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(SW_THREADS, 1)
 gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant__ CUtensorMap tmW1,
                  const __grid_constant__ CUtensorMap tmX0, const __grid_constant__ CUtensorMap tmX1,
-                 int rows, int N, int K, int ksplit, float* part, int* tile_cnt, EpiArgs e) {
+                 int rows, int N, int K, int h, int nst, int ksplit, float* part, int* tile_cnt, EpiArgs e) {
   using Cf = SwCfg<KIND, BNA>;
   using KVT = typename std::conditional<KIND == TC_BF16, bf16, float>::type;
-  constexpr int PARTS = Cf::PARTS, STAGES = Cf::STAGES, NBUF = Cf::NBUF;
+  constexpr int PARTS = Cf::PARTS, NBUF = Cf::NBUF, CJ = Cf::CJ;
+  const int W_BYTES = Cf::w_bytes(h), STAGE_BYTES = Cf::stage_bytes(h);
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t tiles = (raw + 1023u) & ~1023u;
-  const uint32_t bars = tiles + STAGES * Cf::STAGE_BYTES;
-  const uint32_t full0 = bars, empty0 = bars + 8 * STAGES, accfull0 = bars + 16 * STAGES, accempty0 = accfull0 + 16,
+  const uint32_t bars = tiles + nst * STAGE_BYTES + Cf::REST;
+  const uint32_t full0 = bars, empty0 = bars + 8 * nst, accfull0 = bars + 16 * nst, accempty0 = accfull0 + 16,
                  tmem_slot = accempty0 + 16;
   uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - raw));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_w = (N + Cf::BMW - 1) / Cf::BMW;
+  const int warp = __shfl_sync(L3_FULL, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int tiles_w = (N + h - 1) / h;
   const int ntiles = tiles_w * ksplit;
   const int nkb = (K + Cf::BK - 1) / Cf::BK;
   const int kb_per = (nkb + ksplit - 1) / ksplit;
@@ -139,7 +154,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
       asm volatile("prefetch.tensormap [%0];" ::"l"(&tmW1));
       asm volatile("prefetch.tensormap [%0];" ::"l"(&tmX1));
     }
-    for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
+    for (int s = 0; s < nst; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(accfull0 + 8 * b, 1); mbar_init(accempty0 + 8 * b, 4); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -147,70 +162,92 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "n"(Cf::TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot_ptr;
-
+  // the copies' warp, which made the barriers, goes ahead of the TMEM allocation
+  uint32_t tmem_base = 0;
   if (warp == 0) {
-    if (lane == 0) {  // ---------------- TMA producer
-      // weights do not depend on the previous kernel: their first stages are requested before the
-      // dependency wait; the activation boxes follow once the producer kernel's writes are visible
-      uint32_t it = 0;
-      bool waited = false;
-      for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const int n0 = (t % tiles_w) * Cf::BMW, ks = t / tiles_w;
-        const int kb0 = ks * kb_per, kb1 = min(nkb, kb0 + kb_per);
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % STAGES, ph = (it / STAGES) & 1;
-          mbar_wait(empty0 + 8 * s, ph ^ 1);
-          const uint32_t st = tiles + s * Cf::STAGE_BYTES;
-          mbar_expect_tx(full0 + 8 * s, PARTS * (Cf::W_BYTES + Cf::X_BYTES));
-          tma_load_2d(st, &tmW0, kb * Cf::BK, n0, full0 + 8 * s);
-          if (PARTS == 2) tma_load_2d(st + Cf::W_BYTES, &tmW1, kb * Cf::BK, n0, full0 + 8 * s);
-          if (!waited) { pdl_wait(); waited = true; }
-          tma_load_2d(st + PARTS * Cf::W_BYTES, &tmX0, kb * Cf::BK, 0, full0 + 8 * s);
-          if (PARTS == 2) tma_load_2d(st + PARTS * Cf::W_BYTES + Cf::X_BYTES, &tmX1, kb * Cf::BK, 0, full0 + 8 * s);
+    __syncwarp();
+    asm volatile("bar.arrive 1, %0;" ::"n"(SW_THREADS) : "memory");
+  } else {
+    tc_fence_before();
+    asm volatile("bar.sync 1, %0;" ::"n"(SW_THREADS) : "memory");
+    tc_fence_after();
+    tmem_base = *tmem_slot_ptr;
+  }
+
+  // The issuing warps run their loops whole, one elected lane issues, ring positions are counted: as one lane of a divergent warp with
+  // two divisions per k-block the issue code took ~600 cycles per 16 KB of weights - 5.2 TB/s over the chip.  With that and the gated
+  // epilogue's exponentials in front of its stores 32 x 28672 x 4096 went from 54.8 to 41.7 us (a plain read of the weights: 38.4).
+  if (warp == 0 || warp == 6) {  // ---------------- copies: weights, activations
+    // weights do not depend on the previous kernel: their first stages are requested before the
+    // dependency wait; the activation boxes follow once the producer kernel's writes are visible
+    if (warp == 6) pdl_wait();
+    int s = 0;
+    uint32_t ph = 1;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+      const int n0 = (t % tiles_w) * h, ks = t / tiles_w;
+      const int kb0 = ks * kb_per, kb1 = min(nkb, kb0 + kb_per);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        mbar_wait(empty0 + 8 * s, ph);
+        const uint32_t st = tiles + s * STAGE_BYTES, bar = full0 + 8 * s;
+        if (elect_one()) {
+          if (warp == 0) {
+            mbar_expect_tx(bar, PARTS * (h * 128 + Cf::X_BYTES));
+            tma_load_2d(st, &tmW0, kb * Cf::BK, n0, bar);
+            if (PARTS == 2) tma_load_2d(st + W_BYTES, &tmW1, kb * Cf::BK, n0, bar);
+          } else {
+            tma_load_2d(st + PARTS * W_BYTES, &tmX0, kb * Cf::BK, 0, bar);
+            if (PARTS == 2) tma_load_2d(st + PARTS * W_BYTES + Cf::X_BYTES, &tmX1, kb * Cf::BK, 0, bar);
+          }
         }
+        __syncwarp();
+        if (++s == nst) { s = 0; ph ^= 1; }
       }
     }
-  } else if (warp == 1) {
-    if (lane == 0) {  // ---------------- MMA issuer
-      uint32_t it = 0, ti = 0;
-      for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++ti) {
-        const int ks = t / tiles_w;
-        const int kb0 = ks * kb_per, kb1 = min(nkb, kb0 + kb_per);
-        const uint32_t buf = ti % NBUF, use = ti / NBUF;
-        if (use > 0) {
-          mbar_wait(accempty0 + 8 * buf, (use - 1) & 1);
-          tc_fence_after();
-        }
-        const uint32_t acc = tmem_base + buf * Cf::ACC_COLS;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % STAGES, ph = (it / STAGES) & 1;
-          mbar_wait(full0 + 8 * s, ph);
-          tc_fence_after();
-          const uint32_t st = tiles + s * Cf::STAGE_BYTES;
-          const uint64_t w_hi = umma_desc_sw128(st), x_hi = umma_desc_sw128(st + PARTS * Cf::W_BYTES);
+  } else if (warp == 1) {  // ---------------- MMA issuer
+    int s = 0;
+    uint32_t ph = 0, ti = 0;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++ti) {
+      const int ks = t / tiles_w;
+      const int kb0 = ks * kb_per, kb1 = min(nkb, kb0 + kb_per);
+      const uint32_t buf = ti % NBUF, use = ti / NBUF;
+      if (use > 0) {
+        mbar_wait(accempty0 + 8 * buf, (use - 1) & 1);
+        tc_fence_after();
+      }
+      const uint32_t acc = tmem_base + buf * Cf::ACC_COLS;
+      int third = 0;  // main accumulator of the next K slice (3xTF32)
+      for (int kb = kb0; kb < kb1; ++kb) {
+        mbar_wait(full0 + 8 * s, ph);
+        tc_fence_after();
+        const uint32_t st = tiles + s * STAGE_BYTES;
+        const uint64_t w_hi = umma_desc_sw128(st), x_hi = umma_desc_sw128(st + PARTS * W_BYTES);
+        if (elect_one()) {
+          const uint32_t more = kb > kb0;
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {
             const uint64_t adv = (uint64_t)(kk * 2);
-            const int slice = (kb - kb0) * 4 + kk;
             if (PARTS == 2) {
-              const uint64_t w_lo = umma_desc_sw128(st + Cf::W_BYTES);
-              const uint64_t x_lo = umma_desc_sw128(st + PARTS * Cf::W_BYTES + Cf::X_BYTES);
-              const uint32_t corr = acc + 3 * BNA, mainacc = acc + (slice % 3) * BNA;
-              tc_mma<KIND>(corr, w_lo + adv, x_hi + adv, Cf::IDESC, slice == 0 ? 0u : 1u);
+              const uint64_t w_lo = umma_desc_sw128(st + W_BYTES);
+              const uint64_t x_lo = umma_desc_sw128(st + PARTS * W_BYTES + Cf::X_BYTES);
+              int main = third + kk;
+              while (main >= 3) main -= 3;
+              const uint32_t corr = acc + 3 * Cf::AW, mainacc = acc + main * Cf::AW;
+              tc_mma<KIND>(corr, w_lo + adv, x_hi + adv, Cf::IDESC, kk ? 1u : more);
               tc_mma<KIND>(corr, w_hi + adv, x_lo + adv, Cf::IDESC, 1u);
-              tc_mma<KIND>(mainacc, w_hi + adv, x_hi + adv, Cf::IDESC, slice < 3 ? 0u : 1u);
+              tc_mma<KIND>(mainacc, w_hi + adv, x_hi + adv, Cf::IDESC, kk >= 3 ? 1u : more);
             } else {
-              tc_mma<KIND>(acc + (slice % Cf::NACC) * BNA, w_hi + adv, x_hi + adv, Cf::IDESC, slice < Cf::NACC ? 0u : 1u);
+              tc_mma<KIND>(acc, w_hi + adv, x_hi + adv, Cf::IDESC, kk ? 1u : more);
             }
           }
           tc_commit(empty0 + 8 * s);
+          if (kb == kb1 - 1) tc_commit(accfull0 + 8 * buf);
         }
-        tc_commit(accfull0 + 8 * buf);
+        __syncwarp();
+        if (PARTS == 2) { third += 4; while (third >= 3) third -= 3; }
+        if (++s == nst) { s = 0; ph ^= 1; }
       }
+      if (kb0 >= kb1 && elect_one()) tc_commit(accfull0 + 8 * buf);  // a slice without blocks
+      __syncwarp();
     }
   } else {  // ---------------- epilogue (warps 2-5): lane = output column, TMEM column = activation row
     pdl_wait();  // residual / position reads below depend on the previous kernel
@@ -218,29 +255,29 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
     const int start_pos = (EPI == EPI_ROPE_KV) ? *e.pos_ptr : 0;
     uint32_t ti = 0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++ti) {
-      const int n0 = (t % tiles_w) * Cf::BMW, ks = t / tiles_w;
+      const int n0 = (t % tiles_w) * h, ks = t / tiles_w;
       const int kb0 = ks * kb_per, kb1 = min(nkb, kb0 + kb_per);
       const uint32_t buf = ti % NBUF, use = ti / NBUF;
       mbar_wait(accfull0 + 8 * buf, use & 1);
       tc_fence_after();
       const uint32_t acc = tmem_base + buf * Cf::ACC_COLS + ((uint32_t)(quarter * 32) << 16);
       const int n = n0 + quarter * 32 + lane;       // this lane's output column
-      const bool n_ok = n < N && kb0 < kb1;
-      const bool live = n0 + quarter * 32 < N && kb0 < kb1;  // warp-uniform
+      const bool n_ok = quarter * 32 + lane < h && n < N && kb0 < kb1;
+      const bool live = quarter * 32 < h && n0 + quarter * 32 < N && kb0 < kb1;  // warp-uniform
       auto load_acc = [&](int c0, float (&v)[32]) {
         tmem_ld32(acc + (uint32_t)c0, v);
         if (Cf::NACC == 4) {
           float w[32];
 #pragma unroll
           for (int k2 = 1; k2 < 4; ++k2) {
-            tmem_ld32(acc + (uint32_t)c0 + k2 * BNA, w);
+            tmem_ld32(acc + (uint32_t)c0 + k2 * Cf::AW, w);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] += w[j];
+            for (int j = 0; j < CJ; ++j) v[j] += w[j];
           }
         }
       };
       const int Np = tiles_w * Cf::BMW;  // padded width of the K-split scratch [ksplit][BNA][Np]
-      const int tw = t % tiles_w;
+      const int tw = t % tiles_w, np = tw * Cf::BMW + quarter * 32 + lane;
       const bool det = ksplit > 1 && part != nullptr;  // else (residual epilogue only): fp32 atomics
       if (det) {
         // K-split: publish this slice's partial tile (for a fixed row the warp's 32 lanes store 32 consecutive
@@ -252,8 +289,8 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
           float v[32];
           load_acc(c0, v);
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (c0 + j < rows) __stcg(part + ((size_t)ks * BNA + c0 + j) * Np + n0 + quarter * 32 + lane, v[j]);
+          for (int j = 0; j < CJ; ++j)
+            if (c0 + j < rows) __stcg(part + ((size_t)ks * BNA + c0 + j) * Np + np, v[j]);
         }
         tc_fence_before();
         __syncwarp();
@@ -286,25 +323,25 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
           }
         } else {  // sum of the slices' partials, slice 0 first
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = 0.f;
+          for (int j = 0; j < CJ; ++j) v[j] = 0.f;
           // unconditional loads (the scratch holds BNA rows per slice): all 32 are in flight before the first add -
           // guarded ones are issued three at a time, ~10 dependent L2 round trips per slice
           for (int k2 = 0; k2 < ksplit; ++k2) {
-            const float* src = part + ((size_t)k2 * BNA + c0) * Np + n0 + quarter * 32 + lane;
+            const float* src = part + ((size_t)k2 * BNA + c0) * Np + np;
             float w[32];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) w[j] = __ldcg(src + (size_t)j * Np);
+            for (int j = 0; j < CJ; ++j) w[j] = __ldcg(src + (size_t)j * Np);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] += w[j];
+            for (int j = 0; j < CJ; ++j) v[j] += w[j];
           }
         }
         if constexpr (EPI == EPI_STORE) {
           if (e.unary) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = unary_act(e.unary, v[j]);
+            for (int j = 0; j < CJ; ++j) v[j] = unary_act(e.unary, v[j]);
           }
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
+          for (int j = 0; j < CJ; ++j) {
             const int m = c0 + j;
             if (m < rows && n_ok) {
               const size_t o = (size_t)m * e.ld_out + n;
@@ -320,29 +357,48 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
             const int nc = min(n, N - 1);
             float rr[32];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) rr[j] = e.resid[(size_t)min(c0 + j, rows - 1) * e.ld_out + nc];
+            for (int j = 0; j < CJ; ++j) rr[j] = e.resid[(size_t)min(c0 + j, rows - 1) * e.ld_out + nc];
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
+            for (int j = 0; j < CJ; ++j)
               if (c0 + j < rows && n_ok) e.out[(size_t)(c0 + j) * e.ld_out + n] = rr[j] + v[j];
           } else {  // bf16 mode: the slices add their partials into the residual stream in place (out == resid)
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
+            for (int j = 0; j < CJ; ++j)
               if (c0 + j < rows && n_ok) atomicAdd(e.out + (size_t)(c0 + j) * e.ld_out + n, v[j]);
           }
         } else if constexpr (EPI == EPI_SWIGLU) {
-          // rows interleaved gate_j, up_j: even lane holds the gate, its odd neighbour the up value
+          // weight rows interleave gate_j, up_j: an even lane holds the gate, its odd neighbour the up value.  The even lane takes the
+          // chunk's first half of the rows, the odd one the second; all values before the first store, the activation decided once.
+          constexpr int HF = CJ / 2;
+          const bool odd = lane & 1;
+          const int mb = c0 + (odd ? HF : 0);
+          float gt[HF], hv[HF];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float up = __shfl_xor_sync(L3_FULL, v[j], 1);
-            const int m = c0 + j;
-            if (m < rows && n_ok && !(lane & 1)) {
-              const float w = glu_in_weight(e, m, n >> 1);
-              const float h = glu_pair<KIND == TC_BF16>(e, v[j] * w, up * w);
-              const size_t o = (size_t)m * e.ld_out + (n >> 1);
-              if (e.out_lo) { float hh, hl; split_tf32(h, hh, hl); e.out[o] = hh; e.out_lo[o] = hl; }
-              else if (e.out) e.out[o] = h;
-              if (e.out_bf16) e.out_bf16[o] = __float2bfloat16_rn(h);
+          for (int j = 0; j < HF; ++j) {
+            const float got = __shfl_xor_sync(L3_FULL, odd ? v[j] : v[j + HF], 1);
+            gt[j] = odd ? got : v[j];
+            hv[j] = odd ? v[j + HF] : got;
+          }
+          if (KIND == TC_BF16 && e.act == GLU_SILU && !e.glu_w) {
+#pragma unroll
+            for (int j = 0; j < HF; ++j) hv[j] = gt[j] * __fdividef(1.0f, 1.0f + __expf(-gt[j])) * hv[j];
+          } else {
+#pragma unroll
+            for (int j = 0; j < HF; ++j) {
+              const float w = e.glu_w && mb + j < rows && n_ok ? glu_in_weight(e, mb + j, n >> 1) : 1.f;
+              hv[j] = glu_pair<KIND == TC_BF16>(e, gt[j] * w, hv[j] * w);
             }
+          }
+          if (n_ok) {
+            const size_t o = (size_t)mb * e.ld_out + (n >> 1);
+#pragma unroll
+            for (int j = 0; j < HF; ++j)
+              if (mb + j < rows) {
+                const size_t oj = o + (size_t)j * e.ld_out;
+                if (e.out_lo) split_tf32(hv[j], e.out[oj], e.out_lo[oj]);
+                else if (e.out) e.out[oj] = hv[j];
+                if (e.out_bf16) e.out_bf16[oj] = __float2bfloat16_rn(hv[j]);
+              }
           }
         } else if constexpr (EPI == EPI_ROPE_KV) {
           const int qcols = e.HN * e.HD, kcols = e.KVHN * e.HD;
@@ -354,19 +410,19 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
           int posv[32];
           float cs[32], sn[32];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
+          for (int j = 0; j < CJ; ++j) {
             const int m = min(c0 + j, rows - 1);  // clamped: values of rows past the end are not used
             const int b = m / e.L;
             posv[j] = (e.row_pos ? __ldg(e.row_pos + b) : start_pos) + (m - b * e.L);
           }
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
+          for (int j = 0; j < CJ; ++j) {
             const size_t ti = (size_t)posv[j] * (e.HD >> 1) + (d >> 1);
             cs[j] = (is_q || is_k) ? __ldg(e.cos_tab + ti) : 1.f;
             sn[j] = (is_q || is_k) ? __ldg(e.sin_tab + ti) : 0.f;
           }
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
+          for (int j = 0; j < CJ; ++j) {
             const float other = __shfl_xor_sync(L3_FULL, v[j], 1);  // the pair's partner (llama3.py:41-76)
             const int m = c0 + j;
             if (m >= rows || !n_ok) continue;
@@ -388,7 +444,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
           // two warp-wide integer reductions per row (redux.sync) on the order-preserving key halves:
           // the largest value first, then the smallest column among the lanes that hold it
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
+          for (int j = 0; j < CJ; ++j) {
             const int m = c0 + j;
             if (m >= rows) continue;  // warp-uniform
             uint32_t kv = 0u;  // ordered bits of the value; 0 = no candidate
@@ -417,60 +473,38 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
   }
 }
 
+int sm_count() {
+  static int n[16] = {0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!n[dev & 15]) cudaDeviceGetAttribute(&n[dev & 15], cudaDevAttrMultiProcessorCount, dev);
+  return n[dev & 15] > 0 ? n[dev & 15] : 148;
+}
+
 template <int KIND, int BNA, int EPI>
 cudaError_t launch_sw_t(const TcGemmArgs& a, cudaStream_t s) {
   using Cf = SwCfg<KIND, BNA>;
   auto kern = gemm_swap_kernel<KIND, BNA, EPI>;
   static bool attr_done[16] = {false};
-  static int n_sm[16] = {0};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_done[dev & 15]) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cf::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cf::SMEM_MAX);
     if (e != cudaSuccess) return e;
-    cudaDeviceGetAttribute(&n_sm[dev & 15], cudaDevAttrMultiProcessorCount, dev);
     attr_done[dev & 15] = true;
   }
   const bool b16 = KIND == TC_BF16;
-  const CUtensorMap* W0 = tc_get_map(a.W[0], b16, a.N, a.K, Cf::BMW);
+  const int h = a.bn;
+  const CUtensorMap* W0 = tc_get_map(a.W[0], b16, a.N, a.K, h);
   const CUtensorMap* X0 = tc_get_map(a.A[0], b16, a.rows, a.K, BNA);
-  const CUtensorMap* W1 = Cf::PARTS == 2 ? tc_get_map(a.W[1], b16, a.N, a.K, Cf::BMW) : W0;
+  const CUtensorMap* W1 = Cf::PARTS == 2 ? tc_get_map(a.W[1], b16, a.N, a.K, h) : W0;
   const CUtensorMap* X1 = Cf::PARTS == 2 ? tc_get_map(a.A[1], b16, a.rows, a.K, BNA) : X0;
   if (!W0 || !X0 || !W1 || !X1) return cudaErrorInvalidValue;
-  const int sms = n_sm[dev & 15] > 0 ? n_sm[dev & 15] : 148;
-  const int tiles_w = (a.N + Cf::BMW - 1) / Cf::BMW;
-  const int nkb = (a.K + Cf::BK - 1) / Cf::BK;
-  // K-split (deterministic, see the epilogue) when the weight row blocks cover less than half the machine
-  // (QKV: 48 blocks, Wo / Wdown: 32 blocks at the 8B shape): otherwise a few SMs stream the whole matrix at
-  // their per-SM ingress rate.  Needs caller-owned scratch (TcGemmArgs::part / tile_cnt).
-  int ksplit = 1;
-  float* part = a.part;
-  static const int resid_atomic = [] { const char* v = getenv("L3_SWAP_RESID_ATOMIC"); return v ? atoi(v) : 1; }();
-  static const int det_epi = [] { const char* v = getenv("L3_SWAP_KSPLIT_DET"); return v ? atoi(v) : 1; }();
-  if (EPI == EPI_RESID && b16 && a.e.out == a.e.resid && resid_atomic) {
-    // bf16 mode residual epilogue: partials can be added in place with fp32 atomics (reorders the sum, which
-    // the fp32 token-identical mode must not do) - no reduction tail at all
-    while (tiles_w * ksplit * 2 <= sms && nkb / (ksplit * 2) >= 8) ksplit *= 2;
-    part = nullptr;
-  } else if (a.part && a.tile_cnt && tiles_w * 2 <= sms && tiles_w <= a.tile_cnt_len && (det_epi || EPI == EPI_RESID)) {
-    static const int max_split = [] { const char* v = getenv("L3_SWAP_KSPLIT"); return v ? atoi(v) : 8; }();
-    ksplit = std::min(std::min(max_split, sms / tiles_w), nkb / 8);
-    const size_t need = (size_t)BNA * tiles_w * Cf::BMW * sizeof(float);
-    while (ksplit > 1 && need * ksplit > a.part_bytes) --ksplit;
-    while (ksplit > 1 && (ksplit - 1) * ((nkb + ksplit - 1) / ksplit) >= nkb) --ksplit;
-    if (ksplit < 1) ksplit = 1;
-  }
-  // Measured and rejected at the 8B shape, batch 32 (profiles/swap_gemm_experiments.txt): balanced K-ranges
-  // (every CTA an equal contiguous range of (row block, k-block) units: gate|up 55.9 vs 54.2 us - the kernel is not
-  // bound by the ragged second wave), a tile-contiguous copy of the weights read with one 16 KB bulk copy per stage
-  // (5.06 vs 5.08 ms per step: not DRAM page locality either), a whole ring of weight stages requested ahead of the first
-  // activation box (+2 us per GEMM: the first MMA then waits behind 160 KB of weights in the SM's TMA queue), and the
-  // slices of a row block sharing its reduction + epilogue by rows behind a cooperative launch (QKV 37 vs 29 us).
-  // (K-slices against wave quantisation when the row blocks exceed the SM count - gate|up at the 8B shape: 224 blocks
-  // on 148 SMs - were measured and removed: 6.25 vs 5.57 ms per 8B batch-32 decode step, the reduction tail costs
-  // more than the idle half wave.)
-  dim3 grid(std::min(tiles_w * ksplit, sms));
-  return launch_k(kern, grid, dim3(192), (size_t)Cf::SMEM, s, *W0, *W1, *X0, *X1, a.rows, a.N, a.K, ksplit, part, a.tile_cnt, a.e);
+  dim3 grid(std::min((a.N + h - 1) / h * a.ksplit, sm_count()));
+  // no more stages than a CTA has k-blocks
+  const int nkb = (a.K + Cf::BK - 1) / Cf::BK, items = ((a.N + h - 1) / h * a.ksplit + (int)grid.x - 1) / (int)grid.x;
+  const int nst = std::max(2, std::min(Cf::stages(h), (nkb + a.ksplit - 1) / a.ksplit * items));
+  return launch_k(kern, grid, dim3(SW_THREADS), (size_t)(nst * Cf::stage_bytes(h) + Cf::REST + 1024 + Cf::BARS), s, *W0, *W1, *X0, *X1, a.rows, a.N, a.K, h, nst, a.ksplit, a.part, a.tile_cnt, a.e);
 }
 
 template <int KIND, int BNA>
@@ -487,16 +521,60 @@ cudaError_t launch_sw_e(const TcGemmArgs& a, cudaStream_t s) {
 
 bool gemm_swap_supported(int rows, int N) { return rows >= 1 && rows <= 128 && N >= 128; }
 
-cudaError_t launch_gemm_swap(const TcGemmArgs& a, cudaStream_t s) {
-  const int bna = a.rows <= 32 ? 32 : (a.rows <= 64 ? 64 : 128);
+// bf16 mode's residual epilogue may add its slices in place, in any order (fp32 mode must not reorder a sum)
+static bool adds_in_place(const TcGemmArgs& a) {
+  static const int resid_atomic = [] { const char* v = getenv("L3_SWAP_RESID_ATOMIC"); return v ? atoi(v) : 1; }();
+  return a.epi == EPI_RESID && a.kind == TC_BF16 && a.e.out == a.e.resid && resid_atomic;
+}
+// Tile height and K split, by the cycles of the busiest CTA: a k-block takes the issue loops ~500 cycles, or its share of DRAM
+// (3560 bytes per cycle for all CTAs that stream); slices that are added in place cost little, published and summed ones ~2.5 us and more
+// with each slice and row.  More tiles than SMs: the height is what makes the last round full (28672 rows: 293 tiles of 98 instead of
+// 224 of 128).  us per launch in a row of such launches, before (a split that fills the SMs, tiles of 128) -> here: 8 x 2048 x 4096
+// 12.5 -> 9.0, 8 x 2048 x 8192 13.0 -> 11.7, 32 x 28672 x 4096 swiglu 41.7 -> 39.9; over 22 shapes it is at most 7 % behind the best.
+static void pick_swap(const TcGemmArgs& a, int bna, int sms, int* h_out, int* ks_out) {
+  static const int max_split = [] { const char* v = getenv("L3_SWAP_KSPLIT"); return v ? atoi(v) : 8; }();
+  static const int det_epi = [] { const char* v = getenv("L3_SWAP_KSPLIT_DET"); return v ? atoi(v) : 1; }();
+  const bool b16 = a.kind == TC_BF16, atomic = adds_in_place(a);
+  const int parts = b16 ? 1 : 2, nkb = (a.K + (b16 ? 63 : 31)) / (b16 ? 64 : 32);
+  const int rounds = ((a.N + 127) / 128 + sms - 1) / sms;
+  int h = 128;
+  if (rounds > 1) h = std::min(128, ((a.N + sms * rounds - 1) / (sms * rounds) + 1) & ~1);
+  const int tiles = (a.N + h - 1) / h;
+  double best = 0;
+  for (int ks = 1; ks <= std::max(1, atomic ? 8 : std::min(8, max_split)); ++ks) {
+    const int per = (nkb + ks - 1) / ks;
+    if (ks > 1 && (per < 4 || (ks - 1) * per >= nkb)) break;
+    if (ks > 1 && !atomic && (!a.part || !a.tile_cnt || tiles > a.tile_cnt_len || (size_t)bna * tiles * 128 * sizeof(float) * ks > a.part_bytes ||
+                              !(det_epi || a.epi == EPI_RESID))) break;
+    const double issue = b16 ? 500 : 700;
+    const int full = tiles * ks / sms, rest = tiles * ks % sms;
+    double c = full * per * std::max(issue, h * 128.0 * parts * sms / 3560);
+    if (rest) c += per * std::max(issue, h * 128.0 * parts * rest / 3560);
+    if (ks > 1) c += atomic ? 380 + 2.0 * ks * bna : 4400 + (160 + 22.0 * bna) * ks;
+    if (best == 0 || c < best) { best = c; *ks_out = ks; }
+  }
+  *h_out = h;
+}
+
+cudaError_t launch_gemm_swap(const TcGemmArgs& args, cudaStream_t s) {
+  TcGemmArgs a = args;
+  const int bna = a.rows <= 16 ? 16 : a.rows <= 32 ? 32 : (a.rows <= 64 ? 64 : 128);
+  pick_swap(a, bna, sm_count(), &a.bn, &a.ksplit);
+  if (adds_in_place(a)) a.part = nullptr;
+  // Measured and rejected at the 8B shape, batch 32 (profiles/swap_gemm_experiments.txt): a tile-contiguous copy of the weights read
+  // with one 16 KB bulk copy per stage (not DRAM page locality), and the slices of a row block sharing its reduction + epilogue by rows
+  // behind a cooperative launch (QKV 37 vs 29 us).  Later: tiles that start their turn over K one block apart (the activation boxes are
+  // no hot spot), low tiles in place of a K split (42 rows x 147 CTAs for QKV: 17 vs 14 us, the issue loops' cycles per block remain).
   if (a.kind == TC_BF16) {
     switch (bna) {
+      case 16: return launch_sw_e<TC_BF16, 16>(a, s);
       case 32: return launch_sw_e<TC_BF16, 32>(a, s);
       case 64: return launch_sw_e<TC_BF16, 64>(a, s);
       default: return launch_sw_e<TC_BF16, 128>(a, s);
     }
   }
   switch (bna) {
+    case 16: return launch_sw_e<TC_TF32X3, 16>(a, s);
     case 32: return launch_sw_e<TC_TF32X3, 32>(a, s);
     case 64: return launch_sw_e<TC_TF32X3, 64>(a, s);
     default: return launch_sw_e<TC_TF32X3, 128>(a, s);
