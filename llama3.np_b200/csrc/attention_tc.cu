@@ -10,8 +10,8 @@
 //             layout [key, head_dim] - no transposed copy.
 //             Issue order S_0, S_1, PV_0, S_2, PV_1, ...: the tensor core computes the next
 //             scores while the softmax warps work on the current block.
-//   warps 2-5 online softmax, thread = query row (tcgen05.ld 32x32b: no shuffles): the 128 scores of a
-//             row are read into registers with one wait, exp2 -> bf16 P is written to shared memory in
+//   warps 2-9 online softmax, two threads = a query row, 64 of a block's 128 keys each (tcgen05.ld 32x32b: no shuffles): a
+//             half row's scores are read into registers with one wait, exp2 -> bf16 P is written to shared memory in
 //             the K-major swizzled operand layout; the OUTPUT accumulates in TMEM across key blocks
 //             (PV_j with accumulate) and is rescaled lazily - only when a row maximum has grown by
 //             more than 2^8 (tcgen05.ld -> multiply -> tcgen05.st) - so a steady-state block costs the
@@ -60,6 +60,12 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
       "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum) : "memory");
+}
+// one lane of the (whole) warp, known as one to the compiler (see gemm_tc_dev.cuh)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+  return p != 0;
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
   uint32_t r[32];
@@ -133,14 +139,16 @@ template <int HD> struct FaCfg {
   static constexpr int P_BYTES = BQ * BKV * 2;
   static constexpr int STAGES = HD == 128 ? 2 : 4;
   static constexpr int TMEM_COLS = 512;                   // 2 x 128 score columns + 2 x HD output columns
-  static constexpr int SMEM = Q_BYTES + 2 * STAGES * KV_BYTES + P_BYTES + 1024 + 256;
+  static constexpr int XCH_BYTES = 2 * 2 * BQ * 4;        // row maxima of the two halves of a key block, two blocks' turns
+  static constexpr int SMEM = Q_BYTES + 2 * STAGES * KV_BYTES + P_BYTES + XCH_BYTES + 1024 + 256;
   // bf16 x bf16 -> fp32, M = 128; S: N = 128, both K-major;  PV: N = HD, B operand MN-major
   static constexpr uint32_t IDESC_S = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BKV >> 3) << 17) | ((128u >> 4) << 24);
   static constexpr uint32_t IDESC_PV = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((128u >> 4) << 24);
 };
 
+constexpr int FA_THREADS = 320;  // warp 0 = TMA, warp 1 = MMA, warps 2 - 9 = softmax: two warps share 32 query rows, half of a key block each
 template <int HD>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(FA_THREADS, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, AttnArgs a, int nrep) {
   using Cf = FaCfg<HD>;
@@ -149,18 +157,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sQ = (raw + 1023u) & ~1023u;
   const uint32_t sK = sQ + Cf::Q_BYTES, sV = sK + STAGES * Cf::KV_BYTES, sP = sV + STAGES * Cf::KV_BYTES;
-  const uint32_t bars = sP + Cf::P_BYTES;
+  const uint32_t bars = sP + Cf::P_BYTES + Cf::XCH_BYTES;
   // barrier map (8 bytes each)
   const uint32_t q_full = bars, k_full = bars + 8, k_empty = k_full + 8 * STAGES, v_full = k_empty + 8 * STAGES,
                  v_empty = v_full + 8 * STAGES, s_full = v_empty + 8 * STAGES, s_empty = s_full + 16,
-                 pv_full = s_empty + 16, pv_empty = pv_full + 16, p_full = pv_empty + 16, p_empty = p_full + 8,
+                 p_full = s_empty + 16, p_empty = p_full + 8,
                  tmem_slot = p_empty + 8;
   uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - raw));
   uint8_t* sP_ptr = smem_raw + (sP - raw);
+  float* xch = reinterpret_cast<float*>(sP_ptr + Cf::P_BYTES);  // [turn][half][row]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qt = gridDim.x - 1 - blockIdx.x;  // longest tiles (latest queries) first
-  const int head = blockIdx.y, b = blockIdx.z;
+  const int warp = __shfl_sync(L3_FULL, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int qt = gridDim.y - 1 - blockIdx.y;  // the longest tiles (latest queries) of every head and sequence first
+  const int head = blockIdx.x % a.HN, b = blockIdx.x / a.HN;
   const int kvh = head / nrep;
   const int q0 = qt * Cf::BQ;
   pdl_launch();
@@ -175,10 +184,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       mbar_init(v_full + 8 * s, 1); mbar_init(v_empty + 8 * s, 1);
     }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(s_full + 8 * i, 1); mbar_init(s_empty + 8 * i, 128);
-      mbar_init(pv_full + 8 * i, 1); mbar_init(pv_empty + 8 * i, 128);
+      mbar_init(s_full + 8 * i, 1); mbar_init(s_empty + 8 * i, 8);
     }
-    mbar_init(p_full, 128);
+    mbar_init(p_full, 8);
     mbar_init(p_empty, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -196,33 +204,40 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   const int nb = (start + last_q) / Cf::BKV + 1;            // key blocks holding a visible key
   const uint32_t tS = tmem_base, tO = tmem_base + 2 * Cf::BKV;  // two score buffers, then the output accumulator
 
-  if (warp == 0) {
-    if (lane == 0) {  // ---------------- TMA producer
+  if (warp == 0) {  // ---------------- TMA producer
+    if (elect_one()) {
       mbar_expect_tx(q_full, Cf::Q_BYTES);
       for (int s = 0; s < QS; ++s) tma_load_2d(sQ + s * Cf::BQ * 128, &tmQ, head * HD + s * 64, b * a.L + q0, q_full);
-      const int row0 = (b * a.KVHN + kvh) * a.M;
-      for (int j = 0; j < nb; ++j) {
-        const int st = j % STAGES, use = j / STAGES;
-        if (use > 0) mbar_wait(k_empty + 8 * st, (use - 1) & 1);
+    }
+    __syncwarp();
+    const int row0 = (b * a.KVHN + kvh) * a.M;
+    for (int j = 0; j < nb; ++j) {
+      const int st = j % STAGES, use = j / STAGES;
+      if (use > 0) mbar_wait(k_empty + 8 * st, (use - 1) & 1);
+      if (elect_one()) {
         mbar_expect_tx(k_full + 8 * st, Cf::KV_BYTES);
         for (int s = 0; s < QS; ++s)
           tma_load_2d(sK + st * Cf::KV_BYTES + s * Cf::BKV * 128, &tmK, s * 64, row0 + j * Cf::BKV, k_full + 8 * st);
-        if (use > 0) mbar_wait(v_empty + 8 * st, (use - 1) & 1);
+      }
+      __syncwarp();
+      if (use > 0) mbar_wait(v_empty + 8 * st, (use - 1) & 1);
+      if (elect_one()) {
         mbar_expect_tx(v_full + 8 * st, Cf::KV_BYTES);
         for (int s = 0; s < QS; ++s)
           tma_load_2d(sV + st * Cf::KV_BYTES + s * Cf::BKV * 128, &tmV, s * 64, row0 + j * Cf::BKV, v_full + 8 * st);
       }
+      __syncwarp();
     }
-  } else if (warp == 1) {
-    if (lane == 0) {  // ---------------- MMA issuer
-      mbar_wait(q_full, 0);
+  } else if (warp == 1) {  // ---------------- MMA issuer
+    mbar_wait(q_full, 0);
+    tc_fence_after();
+    auto issue_pv = [&](int j) {  // O += P_j V_j: the output accumulates in TMEM over all key blocks
+      const int st = j % STAGES;
+      mbar_wait(v_full + 8 * st, (j / STAGES) & 1);
+      mbar_wait(p_full, j & 1);     // P_j written, and O rescaled if the softmax warps decided to
       tc_fence_after();
-      auto issue_pv = [&](int j) {  // O += P_j V_j: the output accumulates in TMEM over all key blocks
-        const int st = j % STAGES;
-        mbar_wait(v_full + 8 * st, (j / STAGES) & 1);
-        mbar_wait(p_full, j & 1);     // P_j written, and O rescaled if the softmax warps decided to
-        tc_fence_after();
-        const uint32_t vb = sV + st * Cf::KV_BYTES;
+      const uint32_t vb = sV + st * Cf::KV_BYTES;
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < Cf::BKV / 16; ++kk) {  // 16 keys per MMA
           const uint64_t ad = desc_k_sw128(sP + (kk >> 2) * Cf::BQ * 128) + (uint64_t)((kk & 3) * 2);
@@ -231,13 +246,16 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         }
         tc_commit(v_empty + 8 * st);
         tc_commit(p_empty);           // P_j consumed and O holds blocks 0..j
-      };
-      for (int j = 0; j < nb; ++j) {
-        const int st = j % STAGES, buf = j & 1, use = j >> 1;
-        mbar_wait(k_full + 8 * st, (j / STAGES) & 1);
-        if (use > 0) mbar_wait(s_empty + 8 * buf, (use - 1) & 1);
-        tc_fence_after();
-        const uint32_t kb = sK + st * Cf::KV_BYTES;
+      }
+      __syncwarp();
+    };
+    for (int j = 0; j < nb; ++j) {
+      const int st = j % STAGES, buf = j & 1, use = j >> 1;
+      mbar_wait(k_full + 8 * st, (j / STAGES) & 1);
+      if (use > 0) mbar_wait(s_empty + 8 * buf, (use - 1) & 1);
+      tc_fence_after();
+      const uint32_t kb = sK + st * Cf::KV_BYTES;
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk) {
           const uint64_t adv = (uint64_t)((kk & 3) * 2);
@@ -247,52 +265,65 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         }
         tc_commit(k_empty + 8 * st);
         tc_commit(s_full + 8 * buf);
-        if (j > 0) issue_pv(j - 1);
       }
-      issue_pv(nb - 1);
+      __syncwarp();
+      if (j > 0) issue_pv(j - 1);
     }
-  } else {  // ---------------- softmax + output (warps 2-5): thread = query row
-    const int quarter = warp & 3;
+    issue_pv(nb - 1);
+  } else {  // ---------------- softmax + output (warps 2-9): a query row's key block is shared by two threads of two warps
+    // The softmax of a block is the longest part of its turn (16384 exponentials at 16 per cycle, and as much again around them): with
+    // a thread per row it took 3400 cycles per block against 1024 of products, half a row per thread 2100 on the busiest SM.  The halves meet once per
+    // block, over their row maxima; each rescales and writes out its half of the output columns.
+    constexpr int HK = Cf::BKV / 2, HO = HD / 2;
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
     const int r = quarter * 32 + lane;                 // row inside the tile = TMEM lane
     const int qpos = start + q0 + r;                   // keys [0, qpos] are visible (llama3.py:293-297)
     const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
     const float sc = 1.4426950408889634f / sqrtf((float)HD);  // log2(e) / sqrt(HD): p = 2^((s - m) * sc)
+    // the other half's value of this row
+    auto exchange = [&](int turn, float x) {
+      float* t = xch + (turn & 1) * 2 * Cf::BQ;
+      t[half * Cf::BQ + r] = x;
+      asm volatile("bar.sync %0, 64;" ::"r"(2 + quarter) : "memory");  // the two warps of this quarter
+      return t[(half ^ 1) * Cf::BQ + r];
+    };
     // m_used: the row maximum the exponentials are taken against.  It follows the true running maximum
     // lazily: only when the maximum has grown by more than 2^8 is the TMEM output rescaled (and then for the
     // whole warp, tcgen05.ld / .st being warp-wide); until then p may reach 2^8, harmless in bf16 / fp32, and
     // O / l is exact either way because numerator and denominator share m_used.
-    float m_used = -INFINITY, l_run = 0.f;
+    float m_used = -INFINITY, l_run = 0.f;             // l_run: this half's keys
     for (int j = 0; j < nb; ++j) {
       const int buf = j & 1, use = j >> 1;
       mbar_wait(s_full + 8 * buf, use & 1);
       tc_fence_after();
-      const uint32_t ts = tS + buf * Cf::BKV + lane_off;
-      const int key0 = j * Cf::BKV;
-      const bool need_mask = key0 + Cf::BKV - 1 > qpos;
-      // the whole score row in registers with ONE wait (the output no longer lives there)
-      float v[Cf::BKV];
+      const uint32_t ts = tS + buf * Cf::BKV + half * HK + lane_off;
+      const int key0 = j * Cf::BKV + half * HK;
+      const bool need_mask = key0 + HK - 1 > qpos;
+      // the half row of scores in registers with ONE wait (the output no longer lives there)
+      float v[HK];
       tmem_ld32_issue(ts, v + 0); tmem_ld32_issue(ts + 32, v + 32);
-      tmem_ld32_issue(ts + 64, v + 64); tmem_ld32_issue(ts + 96, v + 96);
       tmem_ld_wait();
       tc_fence_before();
-      mbar_arrive(s_empty + 8 * buf);                       // S_j is in registers: the tensor core may overwrite it
+      __syncwarp();
+      if (lane == 0) mbar_arrive(s_empty + 8 * buf);        // S_j is in registers: the tensor core may overwrite it
       if (need_mask) {
 #pragma unroll
-        for (int i = 0; i < Cf::BKV; ++i)
+        for (int i = 0; i < HK; ++i)
           if (key0 + i > qpos) v[i] = -INFINITY;
       }
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int i = 0; i < Cf::BKV; i += 4) {
+      for (int i = 0; i < HK; i += 4) {
         mx4[0] = fmaxf(mx4[0], v[i]); mx4[1] = fmaxf(mx4[1], v[i + 1]);
         mx4[2] = fmaxf(mx4[2], v[i + 2]); mx4[3] = fmaxf(mx4[3], v[i + 3]);
       }
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      mx = fmaxf(mx, exchange(j, mx));
       bool waited = false;
       if (j == 0) {
         m_used = mx;                                          // block 0 always holds a visible key (key 0)
       } else {
-        const bool grow = (mx - m_used) * sc > 8.0f;
+        const bool grow = (mx - m_used) * sc > 8.0f;          // the same in both halves
         if (__any_sync(L3_FULL, grow)) {
           mbar_wait(p_empty, (j - 1) & 1);                    // PV_{j-1} done: O is stable
           waited = true;
@@ -300,7 +331,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           const float alpha = grow ? fast_exp2((m_used - mx) * sc) : 1.0f;
           if (grow) { m_used = mx; l_run *= alpha; }
 #pragma unroll 1
-          for (int c = 0; c < HD; c += 32) {
+          for (int c = half * HO; c < half * HO + HO; c += 32) {
             float ov[32];
             tmem_ld32(tO + lane_off + c, ov);
 #pragma unroll
@@ -314,36 +345,32 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       // the shared-memory stores wait for it to release the P tile
       float rs4[4] = {0.f, 0.f, 0.f, 0.f};
       const float moff = m_used * sc;
-      uint32_t pk[Cf::BKV / 2];
+      uint32_t pk[HK / 2];
 #pragma unroll
-      for (int i = 0; i < Cf::BKV; i += 2) {
+      for (int i = 0; i < HK; i += 2) {
         const float p0 = fast_exp2(fmaf(v[i], sc, -moff)), p1 = fast_exp2(fmaf(v[i + 1], sc, -moff));  // 2^-inf = 0
         rs4[(i >> 1) & 3] += p0 + p1;
         __nv_bfloat162 t = __floats2bfloat162_rn(p0, p1);
         pk[i >> 1] = *reinterpret_cast<uint32_t*>(&t);
       }
       if (j > 0 && !waited) mbar_wait(p_empty, (j - 1) & 1);  // PV_{j-1} has consumed the previous P
+      // this half is one 64-key slice of the tile: 8 chunks of 16 bytes, swizzled inside the 128-byte row
+      uint8_t* prow = sP_ptr + half * (Cf::BQ * 128) + r * 128;
 #pragma unroll
-      for (int c = 0; c < Cf::BKV; c += 32) {
-        // columns c .. c+31 of row r: 4 chunks of 16 bytes, swizzled inside the 128-byte row
-        uint8_t* prow = sP_ptr + (c >> 6) * (Cf::BQ * 128) + r * 128;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int j8 = ((c & 63) >> 3) + q;
-          const int k4 = (c >> 1) + 4 * q;
-          *reinterpret_cast<uint4*>(prow + ((j8 ^ (r & 7)) << 4)) = make_uint4(pk[k4], pk[k4 + 1], pk[k4 + 2], pk[k4 + 3]);
-        }
-      }
+      for (int q = 0; q < 8; ++q) *reinterpret_cast<uint4*>(prow + ((q ^ (r & 7)) << 4)) = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
       l_run += (rs4[0] + rs4[1]) + (rs4[2] + rs4[3]);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // P (generic proxy) -> tensor core (async proxy)
-      mbar_arrive(p_full);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
     }
+    l_run += exchange(nb, l_run);
     mbar_wait(p_empty, (nb - 1) & 1);                        // the last PV has landed in O
     tc_fence_after();
     const float inv = 1.0f / l_run;
     bf16* dst = a.out_bf16 + ((size_t)(b * a.L + q0 + r) * a.HN + head) * HD;
 #pragma unroll 1
-    for (int c = 0; c < HD; c += 32) {
+    for (int c = half * HO; c < half * HO + HO; c += 32) {
       float ov[32];
       tmem_ld32(tO + lane_off + c, ov);
       if (q0 + r < a.L) {
@@ -384,8 +411,10 @@ cudaError_t launch_hd(const AttnArgs& a, const bf16* q16, cudaStream_t s) {
   const CUtensorMap* mk = tc_get_map(a.cache_k, true, cache_rows, HD, Cf::BKV);
   const CUtensorMap* mv = tc_get_map(a.cache_v, true, cache_rows, HD, Cf::BKV);
   if (!mq || !mk || !mv) return cudaErrorInvalidValue;
-  dim3 grid((a.L + Cf::BQ - 1) / Cf::BQ, a.HN, a.B);
-  return launch_k(kern, grid, dim3(192), (size_t)Cf::SMEM, s, *mq, *mk, *mv, a, a.HN / a.KVHN);
+  // one 4096-token prompt of 32 heads of 128, us: a thread per row 207, half a row 197, and with the longest tiles of all heads ahead of
+  // the shorter ones (head by head the SMs' shares differed by half) 176; 2 x 731 tokens of 32 heads of 64: 29 -> 24
+  dim3 grid(a.HN * a.B, (a.L + Cf::BQ - 1) / Cf::BQ);
+  return launch_k(kern, grid, dim3(FA_THREADS), (size_t)Cf::SMEM, s, *mq, *mk, *mv, a, a.HN / a.KVHN);
 }
 }  // namespace
 

@@ -75,6 +75,12 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* tm,
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
       ::"r"(dst), "l"(tm), "r"(c0), "r"(c1), "r"(bar) : "memory");
 }
+// one lane of the (whole) warp, known as one to the compiler (see gemm_tc_dev.cuh; 2048 tokens of 16 heads of 128: 58 -> 49 us)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
@@ -244,7 +250,7 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   volatile int* fail = reinterpret_cast<volatile int*>(tmem_slot_ptr + 1);
   float2* ml = reinterpret_cast<float2*>(smem_raw + (bars + 512 - raw));  // [group][row] (maximum, sum)
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(L3_FULL, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int qt = gridDim.y - 1 - blockIdx.y;  // longest tiles (latest queries) of every head first
   const int head = blockIdx.x, bl = blockIdx.z, b = a.b0 + bl;
   const int q0 = qt * BQ;
@@ -291,7 +297,7 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const int kcol0 = a.k_col + k_head * a.k_cols, vcol0 = a.v_col + v_head * a.v_cols;
 
   if (warp == 0) {
-    if (lane == 0) {  // ---------------- queries and keys
+    if (elect_one()) {  // ---------------- queries and keys
       const int nq = sh.qp * sh.nqs, DQ = nq * 64;
       mbar_expect_tx(q_full, sh.q_bytes());
       for (int s = 0; s < nq; ++s) tma_load_2d(sQ + s * SLICE_Q, &tmQ, head * DQ + s * 64, b * a.L + q0, q_full);
@@ -305,7 +311,7 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       }
     }
   } else if (warp == 10) {
-    if (lane == 0) {  // ---------------- values
+    if (elect_one()) {  // ---------------- values
       for (int j = 0; j < nb; ++j) {
         const int st = j % sh.vst, use = j / sh.vst;
         if (use > 0 && !mbar_wait(v_empty + 8 * st, (use - 1) & 1, fail)) break;
@@ -315,7 +321,7 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {  // ---------------- scores
+    if (elect_one()) {  // ---------------- scores
       uint32_t steps = 0;  // 16-entry steps of every slice, four bits each
       for (int s = 0; s < sh.nqs; ++s) {
         const int n = s < sh.nks ? a.dim - s * 64 : a.rot_dim - (s - sh.nks) * 64;
@@ -373,9 +379,9 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       int live = start + last_q + 1 - block_key(j);          // the blocks up to the next one with such rows: one thread alone
       int stop = j;
       while (stop < nb && (live = start + last_q + 1 - block_key(stop)) >= BKV) ++stop;
-      if (lane == 0)
+      if (elect_one())
         for (; j < stop && ok; ++j) ok = product(j);
-      ok = __shfl_sync(L3_FULL, ok, 0);
+      ok = __all_sync(L3_FULL, ok);
       j = stop;
       if (!ok || j == nb) break;
       const int st = j % sh.vst;
@@ -388,8 +394,8 @@ attn_latent_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
-      if (lane == 0) ok = product(j);
-      ok = __shfl_sync(L3_FULL, ok, 0);
+      if (elect_one()) ok = product(j);
+      ok = __all_sync(L3_FULL, ok);
       ++j;
     }
   } else {  // ---------------- softmax and output: thread = query row
