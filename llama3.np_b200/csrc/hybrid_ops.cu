@@ -13,6 +13,7 @@
 
 #include "common.cuh"
 #include "mixer.h"
+#include "rowvec.cuh"
 
 namespace {
 
@@ -55,6 +56,53 @@ __global__ void __launch_bounds__(256) ssd_prep_kernel(SsdPrepArgs a) {
       a.k_out[(size_t)r * gn + (c - inner)] = s;
     } else {
       a.q_out[(size_t)r * gn + (c - inner - gn)] = s;
+    }
+  }
+}
+
+// Prompts with 4 taps: a thread takes four channels of CONV_TOKENS tokens (delta_prep_vec_kernel's scheme).  2103 tokens, 32 heads of 64,
+// 2 groups of 128: 45.4 -> 21.1 us
+__global__ void __launch_bounds__(256) ssd_prep_vec_kernel(SsdPrepArgs a) {
+  extern __shared__ float sdt[];  // [CONV_TOKENS][H]
+  pdl_launch();
+  pdl_wait();
+  const int b = blockIdx.z, t0 = blockIdx.x * CONV_TOKENS, n = min(CONV_TOKENS, a.L - t0);
+  const int inner = a.H * a.DV, gn = a.G * a.N, C = inner + 2 * gn;
+  const size_t r0 = (size_t)b * a.L + t0;
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+  Conv4 cv;
+  float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (c < C) {
+    cv.load(a.proj + (size_t)b * a.L * a.ld + a.xbc_off + c, a.ld, a.conv_tail + ((size_t)b * C + c) * 3, a.conv_w + (size_t)c * 4, t0, a.L);
+    if (a.conv_b) bias = *reinterpret_cast<const float4*>(a.conv_b + c);
+  }
+  for (int j = threadIdx.x; j < n * a.H; j += blockDim.x) {
+    const size_t r = r0 + j / a.H;
+    const int h = j % a.H;
+    const float dt = softplus_f(a.proj[r * a.ld + a.dt_off + h] + a.dt_bias[h]);
+    sdt[j] = dt;
+    if (blockIdx.y == 0) {
+      const float ld = -expf(a.A_log[h]) * dt;
+      a.decay_out[r * a.H + h] = expf(ld);
+      if (a.logdecay_out) a.logdecay_out[r * a.H + h] = ld;
+    }
+  }
+  __syncthreads();
+  if (c >= C) return;
+#pragma unroll
+  for (int i = 0; i < CONV_TOKENS; ++i) {
+    if (i >= n) break;
+    float4 v = cv.at(i, bias);
+    v = make_float4(silu_ref(v.x), silu_ref(v.y), silu_ref(v.z), silu_ref(v.w));
+    const size_t r = r0 + i;
+    if (c < inner) {
+      const float dt = sdt[i * a.H + c / a.DV];  // DV is a multiple of 4
+      *reinterpret_cast<float4*>(a.x_out + r * inner + c) = v;
+      *reinterpret_cast<float4*>(a.v_out + r * inner + c) = make_float4(dt * v.x, dt * v.y, dt * v.z, dt * v.w);
+    } else if (c < inner + gn) {
+      *reinterpret_cast<float4*>(a.k_out + r * gn + (c - inner)) = v;
+    } else {
+      *reinterpret_cast<float4*>(a.q_out + r * gn + (c - inner - gn)) = v;
     }
   }
 }
@@ -121,58 +169,66 @@ __global__ void __launch_bounds__(256) mix_out_kernel(MixOutArgs a, int wpg) {
   }
 }
 
-// The same stage with every operand read once, as 16-byte vectors held in registers: a warp per group of 128 * NV values
-template <int NV>
+// The same stage with every operand read once, as 16-byte vectors held in registers: WPG warps per group of 128 * NV * WPG values.
+// 2103 rows in two groups of 1024 with skip term and gate: 46.3 -> 21.2 us
+template <int NV, int WPG>
 __global__ void __launch_bounds__(256) mix_out_vec_kernel(MixOutArgs a) {
+  __shared__ float red[8];
   pdl_launch();
   pdl_wait();
   const size_t r = blockIdx.x;
-  const int lane = threadIdx.x & 31, g = blockIdx.y * 8 + (threadIdx.x >> 5);
-  if (g * a.group >= a.n) return;
-  const int base = g * a.group;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = warp % WPG;
+  const int g = blockIdx.y * (int)(blockDim.x / (32 * WPG)) + warp / WPG;
+  const bool live = g * a.group < a.n;  // the same for all warps of a group
+  const int base = g * a.group + sub * NV * 128;
   auto act = [&](float z) { return a.gate_act ? z * sigmoid_f(z) : sigmoid_f(z); };
   float4 y[NV], z[NV];
-#pragma unroll
-  for (int u = 0; u < NV; ++u) {
-    const int c = base + u * 128 + lane * 4;
-    y[u] = *reinterpret_cast<const float4*>(a.o + r * a.n + c);
-    if (a.gate) z[u] = *reinterpret_cast<const float4*>(a.gate + r * a.ld_gate + c);
-  }
-  float dinv = 1.0f;
-  if (a.nq) {
-    const size_t rh = r * (a.n / a.DV) + base / a.DV;
-    dinv = 1.0f / (fmaxf(fabsf(a.nq[rh]), a.floor[rh]) + 1e-6f);
-  }
   float ss = 0.f;
+  if (live) {
 #pragma unroll
-  for (int u = 0; u < NV; ++u) {
-    const int c = base + u * 128 + lane * 4;
-    y[u].x *= dinv; y[u].y *= dinv; y[u].z *= dinv; y[u].w *= dinv;
-    if (a.skip_d) {
-      const float4 x = *reinterpret_cast<const float4*>(a.skip_x + r * a.n + c);
-      y[u].x = fmaf(a.skip_d[c / a.DV], x.x, y[u].x); y[u].y = fmaf(a.skip_d[(c + 1) / a.DV], x.y, y[u].y);
-      y[u].z = fmaf(a.skip_d[(c + 2) / a.DV], x.z, y[u].z); y[u].w = fmaf(a.skip_d[(c + 3) / a.DV], x.w, y[u].w);
+    for (int u = 0; u < NV; ++u) {
+      const int c = base + u * 128 + lane * 4;
+      y[u] = *reinterpret_cast<const float4*>(a.o + r * a.n + c);
+      if (a.gate) z[u] = *reinterpret_cast<const float4*>(a.gate + r * a.ld_gate + c);
     }
-    if (a.gate) {
-      z[u].x = act(z[u].x); z[u].y = act(z[u].y); z[u].z = act(z[u].z); z[u].w = act(z[u].w);
-      if (a.pre_gate) { y[u].x *= z[u].x; y[u].y *= z[u].y; y[u].z *= z[u].z; y[u].w *= z[u].w; }
+    float dinv = 1.0f;
+    if (a.nq) {
+      const size_t rh = r * (a.n / a.DV) + (g * a.group) / a.DV;
+      dinv = 1.0f / (fmaxf(fabsf(a.nq[rh]), a.floor[rh]) + 1e-6f);
     }
-    ss = fmaf(y[u].x, y[u].x, ss); ss = fmaf(y[u].y, y[u].y, ss); ss = fmaf(y[u].z, y[u].z, ss); ss = fmaf(y[u].w, y[u].w, ss);
+#pragma unroll
+    for (int u = 0; u < NV; ++u) {
+      const int c = base + u * 128 + lane * 4;
+      y[u].x *= dinv; y[u].y *= dinv; y[u].z *= dinv; y[u].w *= dinv;
+      if (a.skip_d) {
+        const float4 x = *reinterpret_cast<const float4*>(a.skip_x + r * a.n + c);
+        y[u].x = fmaf(a.skip_d[c / a.DV], x.x, y[u].x); y[u].y = fmaf(a.skip_d[(c + 1) / a.DV], x.y, y[u].y);
+        y[u].z = fmaf(a.skip_d[(c + 2) / a.DV], x.z, y[u].z); y[u].w = fmaf(a.skip_d[(c + 3) / a.DV], x.w, y[u].w);
+      }
+      if (a.gate) {
+        z[u].x = act(z[u].x); z[u].y = act(z[u].y); z[u].z = act(z[u].z); z[u].w = act(z[u].w);
+        if (a.pre_gate) { y[u].x *= z[u].x; y[u].y *= z[u].y; y[u].z *= z[u].z; y[u].w *= z[u].w; }
+      }
+      ss = fmaf(y[u].x, y[u].x, ss); ss = fmaf(y[u].y, y[u].y, ss); ss = fmaf(y[u].z, y[u].z, ss); ss = fmaf(y[u].w, y[u].w, ss);
+    }
   }
-  const float rinv = 1.0f / sqrtf(warp_sum(ss) / (float)a.group + a.eps) * a.out_scale;
+  ss = warp_sum(ss);
+  if (WPG > 1) {
+    if (lane == 0) red[warp] = ss;
+    __syncthreads();
+    ss = 0.f;
+#pragma unroll
+    for (int w = 0; w < WPG; ++w) ss += red[warp / WPG * WPG + w];
+  }
+  if (!live) return;
+  const float rinv = 1.0f / sqrtf(ss / (float)a.group + a.eps) * a.out_scale;
 #pragma unroll
   for (int u = 0; u < NV; ++u) {
     const int c = base + u * 128 + lane * 4;
     const float4 w = *reinterpret_cast<const float4*>(a.w + c % a.wlen);
     float4 v = make_float4(y[u].x * rinv * w.x, y[u].y * rinv * w.y, y[u].z * rinv * w.z, y[u].w * rinv * w.w);
     if (a.gate && !a.pre_gate) { v.x *= z[u].x; v.y *= z[u].y; v.z *= z[u].z; v.w *= z[u].w; }
-    if (a.out) *reinterpret_cast<float4*>(a.out + r * a.ld_out + c) = v;
-    if (a.out16) {
-      union { __nv_bfloat162 h[2]; uint2 q; } o;
-      o.h[0] = __floats2bfloat162_rn(v.x, v.y);
-      o.h[1] = __floats2bfloat162_rn(v.z, v.w);
-      *reinterpret_cast<uint2*>(a.out16 + r * a.ld_out + c) = o.q;
-    }
+    put4(a.out, a.out16, r * a.ld_out + c, v);
   }
 }
 
@@ -201,6 +257,13 @@ __global__ void concat_rows_kernel(const float* __restrict__ a, const float* __r
 cudaError_t launch_ssd_prep(const SsdPrepArgs& a, int rows, cudaStream_t s) {
   if (a.update_tail && a.L != 1) return cudaErrorInvalidValue;
   const int C = a.H * a.DV + 2 * a.G * a.N;
+  if (rows > 8 && a.L > 1 && a.taps == 4 && a.DV % 4 == 0 && (a.G * a.N) % 4 == 0 && a.ld % 4 == 0 && a.xbc_off % 4 == 0 && rows % a.L == 0 && rows / a.L <= 65535 &&
+      a.H <= 1024 && aligned16(a.proj) && aligned16(a.conv_w) && aligned16(a.conv_b) && aligned16(a.x_out) && aligned16(a.v_out) && aligned16(a.k_out) &&
+      aligned16(a.q_out)) {
+    const int threads = std::min(256, (C / 4 + 31) / 32 * 32);
+    return launch_k(ssd_prep_vec_kernel, dim3((a.L + CONV_TOKENS - 1) / CONV_TOKENS, (C / 4 + threads - 1) / threads, rows / a.L), dim3(threads),
+                    (size_t)CONV_TOKENS * a.H * sizeof(float), s, a);
+  }
   const int parts = rows <= 8 ? std::max(1, std::min(32, C / 256)) : 1;  // few rows: a row's channels spread over CTAs
   return launch_k(ssd_prep_kernel, dim3(rows, parts), dim3(256), (size_t)a.H * sizeof(float), s, a);
 }
@@ -212,19 +275,46 @@ cudaError_t launch_gla_prep(const float* q, int ld, float q_mul, const float* z,
                   (int64_t)rows, n, q_out, g_out, log_decay);
 }
 
+// NV * 128 values per warp, WPG warps per group: the first pair whose product is the group (0: none)
+static int mix_out_pair(int group, int* nv, int* wpg) {
+  for (int p = 1; p <= 8; p *= 2)
+    for (int n = 1; n <= 4; ++n)
+      if (n * p * 128 == group) { *nv = n; *wpg = p; return 1; }
+  return 0;
+}
+bool mix_out_vec_supported(const MixOutArgs& a) {
+  int nv, wpg;
+  const uintptr_t align = (uintptr_t)a.o | (uintptr_t)a.gate | (uintptr_t)a.skip_x | (uintptr_t)a.w | (uintptr_t)a.out | ((uintptr_t)a.out16 << 1);
+  return a.n % a.group == 0 && mix_out_pair(a.group, &nv, &wpg) && a.wlen % 4 == 0 && a.ld_gate % 4 == 0 && a.ld_out % 4 == 0 && a.n % 4 == 0 &&
+         align % 16 == 0;
+}
+template <int WPG>
+static cudaError_t launch_mix_vec_t(const MixOutArgs& a, int rows, int nv, cudaStream_t s) {
+  const int groups = a.n / a.group, gpc = std::min(8 / WPG, groups);
+  const dim3 grid(rows, (groups + gpc - 1) / gpc), block(32 * WPG * gpc);
+  switch (nv) {
+    case 1: return launch_k(mix_out_vec_kernel<1, WPG>, grid, block, 0, s, a);
+    case 2: return launch_k(mix_out_vec_kernel<2, WPG>, grid, block, 0, s, a);
+    case 3: return launch_k(mix_out_vec_kernel<3, WPG>, grid, block, 0, s, a);
+    default: return launch_k(mix_out_vec_kernel<4, WPG>, grid, block, 0, s, a);
+  }
+}
+
+cudaError_t launch_mix_out_vec(const MixOutArgs& a, int rows, cudaStream_t s) {
+  int nv = 0, p = 0;
+  if (!mix_out_pair(a.group, &nv, &p)) return cudaErrorInvalidValue;
+  switch (p) {
+    case 1: return launch_mix_vec_t<1>(a, rows, nv, s);
+    case 2: return launch_mix_vec_t<2>(a, rows, nv, s);
+    case 4: return launch_mix_vec_t<4>(a, rows, nv, s);
+    default: return launch_mix_vec_t<8>(a, rows, nv, s);
+  }
+}
+
 cudaError_t launch_mix_out(const MixOutArgs& a, int rows, cudaStream_t s) {
   if (a.group < 1 || a.n % a.group != 0 || (a.nq && a.DV % a.group != 0)) return cudaErrorInvalidValue;
   const int groups = a.n / a.group;
-  const uintptr_t align = (uintptr_t)a.o | (uintptr_t)a.gate | (uintptr_t)a.skip_x | (uintptr_t)a.w | (uintptr_t)a.out | ((uintptr_t)a.out16 << 1);
-  if (rows > 8 && a.group % 128 == 0 && a.group <= 512 && a.wlen % 4 == 0 && a.ld_gate % 4 == 0 && a.ld_out % 4 == 0 && align % 16 == 0) {
-    const dim3 grid(rows, (groups + 7) / 8), block(32 * std::min(8, groups));
-    switch (a.group / 128) {
-      case 1: return launch_k(mix_out_vec_kernel<1>, grid, block, 0, s, a);
-      case 2: return launch_k(mix_out_vec_kernel<2>, grid, block, 0, s, a);
-      case 3: return launch_k(mix_out_vec_kernel<3>, grid, block, 0, s, a);
-      default: return launch_k(mix_out_vec_kernel<4>, grid, block, 0, s, a);
-    }
-  }
+  if (rows > 8 && mix_out_vec_supported(a)) return launch_mix_out_vec(a, rows, s);
   const int wpg = a.group >= 1024 ? 8 : a.group >= 512 ? 4 : a.group >= 256 ? 2 : 1;  // warps per group
   const int gpc = 8 / wpg;
   return launch_k(mix_out_kernel, dim3(rows, (groups + gpc - 1) / gpc), dim3(256), 0, s, a, wpg);

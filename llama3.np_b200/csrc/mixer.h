@@ -54,6 +54,22 @@ cudaError_t launch_conv_tail(float* tail, const float* proj, int ld, int B, int 
 cudaError_t launch_rmsnorm_rows(const float* x, const float* w, float eps, int rows, int D, int src_mul, int src_add,
                                 const int32_t* src_rows, float* out, bf16* out16, cudaStream_t s, int groups = 1);
 cudaError_t launch_to_bf16(const float* in, int64_t n, bf16* out, cudaStream_t s);
+// norms of whole rows as vectors (prenorm_ops.cu): h = (x - mean) / sqrt(var + eps) * w with center, else x / rms * w, in `groups` equal
+// parts; row = src_rows[r] or r * src_mul + src_add.  shift: out = h + (h of the token before - h) * shift, with hprev [slots, D] as in
+// launch_prenorm_shift (L tokens per sequence).  Behind the launchers of the single forms wherever the row allows it.
+struct NormRowsArgs {
+  const float *x, *w;
+  float eps;
+  int center, D, groups, src_mul, src_add;
+  const int32_t* src_rows;
+  const float* shift;
+  float* hprev;
+  int L;
+  float* out;
+  bf16* out16;
+};
+bool norm_rows_supported(const NormRowsArgs& a);
+cudaError_t launch_norm_rows(const NormRowsArgs& a, int rows, cudaStream_t s);
 cudaError_t launch_add_one(float* p, int n, cudaStream_t s);
 
 // ---- recurrences over time (recurrent.cu): one fp32 state matrix [DK, DV] per (sequence slot, head)
@@ -431,6 +447,9 @@ struct MixOutArgs {
   const float *nq, *floor;
 };
 cudaError_t launch_mix_out(const MixOutArgs& a, int rows, cudaStream_t s);
+// the same with every operand read once, as vectors, where the shapes allow it
+bool mix_out_vec_supported(const MixOutArgs& a);
+cudaError_t launch_mix_out_vec(const MixOutArgs& a, int rows, cudaStream_t s);
 // x <- cap * tanh(x / cap), n values
 cudaError_t launch_softcap(float* x, int64_t n, float cap, cudaStream_t s);
 // out[r] = [a[r] | b[r]] (D values each; + bf16 mirror)
