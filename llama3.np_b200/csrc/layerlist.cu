@@ -1633,7 +1633,7 @@ static int ll_mix_unit(L3Model* m, LLLayer& Ly, LLState& St, const float* pin, i
     LAUNCH(m, launch_ssd_prep(pa, ntok, m->stream));
     if (s.conv_taps > 1 && L > 1) LAUNCH(m, launch_conv_tail(St.conv_tail, pin + Ly.off_q, ld, B, L, O + 2 * gn, s.conv_taps - 1, m->stream));
     ra.mode = 2; ra.q = m->q; ra.k = ll->rk; ra.v = ll->rv; ra.ld_q = ra.ld_k = gn; ra.ld_v = O; ra.g = ll->rg; ra.g_head = 1; ra.rep = H / G;
-    ra.log_g = pa.logdecay_out; ra.ws = ll->chunk_ws; ra.ws_floats = ll->chunk_ws_floats;  // prompts: chunk-parallel where the shape allows
+    ra.log_g = pa.logdecay_out; ra.ws = ll->chunk_ws; ra.ws_floats = ll->chunk_ws_floats; ra.bf16_ops = m->tc_ok;  // prompts: chunk-parallel where the shape allows
     LAUNCH(m, launch_recur(ra, m->stream));
     mo.skip_d = Ly.skip_d; mo.skip_x = ll->xs; mo.gate = pin + Ly.off_g; mo.ld_gate = ld; mo.gate_act = 1; mo.pre_gate = 1;
     mo.w = Ly.mix_norm; mo.wlen = O; mo.group = O / s.out_norm_groups;
@@ -2150,7 +2150,7 @@ int ll_enqueue_layers(L3Model* m, const int32_t* d_ids, int ids_ld, int ids_off,
       ra.mode = 0; ra.q = ll->pin + Ly.off_q; ra.k = ll->pin + Ly.off_k; ra.v = ll->pin + Ly.off_v;
       ra.ld_q = ra.ld_k = ra.ld_v = Ly.n_in; ra.act_in = m->bf16 ? 2 : 1; ra.head_decay = Ly.decay;
       ra.state = St.S; ra.out = ll->o; ra.B = B; ra.L = L; ra.H = H; ra.rep = 1; ra.DK = DK; ra.DV = DV;
-      ra.ws = ll->chunk_ws; ra.ws_floats = ll->chunk_ws_floats;
+      ra.ws = ll->chunk_ws; ra.ws_floats = ll->chunk_ws_floats; ra.bf16_ops = m->tc_ok;
       LAUNCH(m, launch_recur(ra, m->stream));
       LAUNCH(m, launch_gated_rmsnorm(ll->o, ll->pin + Ly.off_g, Ly.n_in, Ly.mix_norm, O, O, eps, ntok, O, m->ctx, (bf16*)m->ctx16, m->stream));
     } else {

@@ -96,8 +96,8 @@ struct RecurArgs {
   float q_mul;            // multiplies the queries (0: 1)
   float* n_state;         // [maxB, H, DK] a running sum of the keys with the state's own decay (the normaliser of an mLSTM) ...
   float* nq;              // ... and its product with the query, [B * L, H]
-  int bf16_ops;           // bf16 mode.  With n_state, chunk-parallel form: q, k and v may be rounded to bf16 (they are bf16 projections'
-                          // outputs).  With log_c: prompts run on tensor products of (hi, lo) pairs (recur_channel.cu)
+  int bf16_ops;           // bf16 mode: the chunk-parallel forms of prompts run on tensor products.  With n_state q, k and v may be rounded to
+                          // bf16 (they are bf16 projections' outputs), else all operands are (hi, lo) pairs (recur_chunk.cu, recur_channel.cu)
   float* ws;              // mode 0, may be null: room for one state matrix per (sequence, head, chunk of 64 tokens);
   size_t ws_floats;       // with it, prompts of the common shapes run in the chunk-parallel form (recur_chunk.cu)
 };

@@ -25,8 +25,14 @@
 // keys and values, which are outputs of bf16 projections, are operands as they are (bf16), while everything the recurrence
 // itself makes - decayed keys, decayed scores, the states - enters as a pair hi + lo of bf16 values (16 significant bits).
 // A chunk's products are 64 x 64 tiles with 64 .. 256 summed terms, and their operands are built in the kernel.
+// The other recurrences of bf16 mode run there as well, with queries, keys and values - which went through a silu or a convolution in
+// fp32 - as pairs too (the product of two low parts, 2^-18 of a term, is left out).  2048 tokens, 16 heads of 128 x 128, fixed decay, us,
+// FFMA tiles -> pairs: states 59 -> 25, outputs 109 -> 41; 2103 tokens, 32 heads of 128 x 64, a decay per token: 51 -> 24, 132 -> 47.
 // The sums run in another order than the token-by-token kernel, so the two agree to fp32 rounding, not bit for bit.
 #include <stdint.h>
+
+#include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "mixer.h"
@@ -353,6 +359,11 @@ struct Block {
       v[u] = j < n ? *reinterpret_cast<const float4*>(src + (size_t)j * ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
+  __device__ __forceinline__ void act(int act_in) {
+    if (!act_in) return;
+#pragma unroll
+    for (int u = 0; u < N; ++u) v[u] = make_float4(act_silu(act_in, v[u].x), act_silu(act_in, v[u].y), act_silu(act_in, v[u].z), act_silu(act_in, v[u].w));
+  }
   __device__ __forceinline__ void put(bf16* dst, int ld_dst, float mul) const {
 #pragma unroll
     for (int u = 0; u < N; ++u) {
@@ -374,16 +385,50 @@ struct Block {
   }
 };
 
+// Which recurrence: the mLSTM (normaliser, keys' scales, decays' sums in double precision), a decay per token, a fixed decay
+enum ChunkKind { CK_MLSTM, CK_TOKEN, CK_FIXED };
+// the decays inside a chunk: pw = running sums of the logarithms, or powers of the fixed decay
+template <int KIND>
+struct ChunkDecay {
+  const double* pd;
+  const float* pw;
+  __device__ __forceinline__ float between(int j, int i) const {  // tokens j + 1 .. i
+    if constexpr (KIND == CK_MLSTM) return expf((float)(pd[i] - pd[j]));
+    else if constexpr (KIND == CK_TOKEN) return expf(pw[i] - pw[j]);
+    else return pw[i - j];
+  }
+  __device__ __forceinline__ float upto(int i) const {  // tokens 0 .. i
+    if constexpr (KIND == CK_MLSTM) return expf((float)pd[i]);
+    else if constexpr (KIND == CK_TOKEN) return expf(pw[i]);
+    else return pw[i + 1];
+  }
+};
+template <int KIND>
+__device__ __forceinline__ ChunkDecay<KIND> chunk_decay(const RecurArgs& a, size_t row0, int h, int n, double* pd, float* pw) {
+  if constexpr (KIND == CK_MLSTM) fill_cumlog(pd, a.log_g + row0 * a.H + h, a.H, n);
+  else if constexpr (KIND == CK_TOKEN) fill_cumlog(pw, a.log_g + row0 * a.H + h, a.H, n);
+  else fill_powers(pw, a.head_decay[h]);
+  return {pd, pw};
+}
+constexpr size_t state_mma_smem(int DK, bool pair) { return ((size_t)2 * CH * (DK + 8) + (pair ? 2 : 1) * CH * LDE) * 2; }
+constexpr size_t out_mma_smem(int DK, bool pair) {
+  const size_t kp = std::max((size_t)CH * (DK + 8), (size_t)DK * LDE);  // pairs: the state's tiles take the keys' place
+  return pair ? ((size_t)2 * CH * (DK + 8) + 4 * CH * LDE + 2 * kp) * 2 : ((size_t)2 * CH * (DK + 8) + 3 * CH * LDE + 2 * (size_t)DK * LDE) * 2;
+}
+
 // grid (NC * NE, H, B): the chunk's D, value columns [e_lo, e_hi) of it.  8 warps on a 64 x 64 tile: 16 rows x 32 columns each
-template <int DK>
+template <int DK, int KIND>
 __global__ void __launch_bounds__(256) lin_chunk_state_mma_kernel(RecurArgs a, int NC, int NE) {
   extern __shared__ __align__(16) uint8_t smb[];
-  __shared__ double pd[CH];
+  __shared__ double pd[KIND == CK_MLSTM ? CH : 1];
+  __shared__ float pw[CH + 1];
   __shared__ float sc[CH];
   constexpr int LDK = DK + 8;
+  constexpr bool PAIR = KIND != CK_MLSTM;
   bf16* Kh = reinterpret_cast<bf16*>(smb);           // [CH][LDK] decayed keys, hi and lo
   bf16* Kl = Kh + (size_t)CH * LDK;
-  bf16* Vs = Kl + (size_t)CH * LDK;                  // [CH][LDE]
+  bf16* Vs = Kl + (size_t)CH * LDK;                  // [CH][LDE] (pairs: and what it leaves)
+  bf16* Vl = Vs + (size_t)CH * LDE;
   pdl_launch();
   pdl_wait();
   const int c = blockIdx.x / NE, ne = blockIdx.x - c * NE, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x;
@@ -396,19 +441,21 @@ __global__ void __launch_bounds__(256) lin_chunk_state_mma_kernel(RecurArgs a, i
   Block<CH, 64> vb;
   kb.fetch(a.k + row0 * a.ld_k + (size_t)(h / a.rep) * DK, a.ld_k, n);
   vb.fetch(vsrc + e_lo, a.ld_v, n);
-  fill_cumlog(pd, a.log_g + row0 * a.H + h, a.H, n);
+  const ChunkDecay<KIND> dec = chunk_decay<KIND>(a, row0, h, n, pd, pw);
+  if (PAIR) kb.act(a.act_in);
   __syncthreads();
-  for (int j = tid; j < CH; j += 256) sc[j] = j < n ? expf((float)(pd[n - 1] - pd[j])) * a.k_scale[(row0 + j) * a.H + h] : 0.f;
-  if (ne == 0 && tid == 0) chunk_decays(a, NC)[((size_t)b * a.H + h) * NC + c] = expf((float)pd[n - 1]);
+  for (int j = tid; j < CH; j += 256) sc[j] = j < n ? dec.between(j, n - 1) * (PAIR ? 1.f : a.k_scale[(row0 + j) * a.H + h]) : 0.f;
+  if (KIND != CK_FIXED && ne == 0 && tid == 0) chunk_decays(a, NC)[((size_t)b * a.H + h) * NC + c] = dec.upto(n - 1);
   __syncthreads();
   kb.put_split(Kh, Kl, LDK, sc);
   float* D = a.ws + (((size_t)b * a.H + h) * NC + c) * a.DK * a.DV;
   for (int e0 = e_lo; e0 < e_hi; e0 += 64) {
     if (e0 > e_lo) __syncthreads();  // the previous tile's values are no longer read
-    vb.put(Vs, LDE, 1.f);
+    if constexpr (PAIR) { vb.act(a.act_in); vb.put_split(Vs, Vl, LDE, nullptr); }
+    else vb.put(Vs, LDE, 1.f);
     __syncthreads();
     if (e0 + 64 < e_hi) vb.fetch(vsrc + e0 + 64, a.ld_v, n);  // in flight during the products
-    if (ne == 0 && e0 == 0)
+    if (!PAIR && ne == 0 && e0 == 0)
       for (int d = tid; d < DK; d += 256) {
         float t = 0.f;
 #pragma unroll 8
@@ -433,6 +480,12 @@ __global__ void __launch_bounds__(256) lin_chunk_state_mma_kernel(RecurArgs a, i
         mma16816(acc[2], ah, v1[0], v1[1]); mma16816(acc[3], ah, v1[2], v1[3]);
         mma16816(acc[0], al, v0[0], v0[1]); mma16816(acc[1], al, v0[2], v0[3]);
         mma16816(acc[2], al, v1[0], v1[1]); mma16816(acc[3], al, v1[2], v1[3]);
+        if constexpr (PAIR) {
+          ldsm4t(v0, smem_addr(vp + (Vl - Vs)));
+          ldsm4t(v1, smem_addr(vp + (Vl - Vs) + 16));
+          mma16816(acc[0], ah, v0[0], v0[1]); mma16816(acc[1], ah, v0[2], v0[3]);
+          mma16816(acc[2], ah, v1[0], v1[1]); mma16816(acc[3], ah, v1[2], v1[3]);
+        }
       }
       float* dp = D + (size_t)(d0 + wm * 16 + (lane >> 2)) * a.DV + e0 + wn * 32 + (lane & 3) * 2;
 #pragma unroll
@@ -445,18 +498,23 @@ __global__ void __launch_bounds__(256) lin_chunk_state_mma_kernel(RecurArgs a, i
 }
 
 // grid (NC * NE, H, B): the chunk's outputs, value columns as above
-template <int DK>
+template <int DK, int KIND>
 __global__ void __launch_bounds__(256) lin_chunk_out_mma_kernel(RecurArgs a, int NC, int NE) {
   extern __shared__ __align__(16) uint8_t smb[];
-  __shared__ double pd[CH];
+  __shared__ double pd[KIND == CK_MLSTM ? CH : 1];
+  __shared__ float pw[CH + 1];
   __shared__ float ks[CH], s_nq[2][CH];
   constexpr int LDK = DK + 8;
+  constexpr bool PAIR = KIND != CK_MLSTM;
   bf16* Qs = reinterpret_cast<bf16*>(smb);           // [CH][LDK]
-  bf16* Ks = Qs + (size_t)CH * LDK;                  // [CH][LDK]
-  bf16* Ah = Ks + (size_t)CH * LDK;                  // [CH][LDE] decayed scores, hi and lo
+  bf16* Ql = Qs + (PAIR ? (size_t)CH * LDK : 0);     // pairs: what Q, K and V leave
+  bf16* Ah = Ql + (size_t)CH * LDK;                  // [CH][LDE] decayed scores, hi and lo
   bf16* Al = Ah + (size_t)CH * LDE;
   bf16* Vs = Al + (size_t)CH * LDE;                  // [CH][LDE]
-  bf16* Ph = Vs + (size_t)CH * LDE;                  // [DK][LDE] the state ahead of the chunk, hi and lo
+  bf16* Vl = Vs + (PAIR ? (size_t)CH * LDE : 0);
+  bf16* Ks = Vl + (size_t)CH * LDE;                  // [CH][LDK]
+  bf16* Kl = Ks + (PAIR ? (size_t)CH * LDK : 0);
+  bf16* Ph = PAIR ? Ks : Ks + (size_t)CH * LDK;      // [DK][LDE] the state ahead of the chunk, hi and lo; pairs: where the keys were
   bf16* Pl = Ph + (size_t)DK * LDE;
   pdl_launch();
   pdl_wait();
@@ -464,14 +522,21 @@ __global__ void __launch_bounds__(256) lin_chunk_out_mma_kernel(RecurArgs a, int
   const int lane = tid & 31, warp = tid >> 5, wm = warp & 3, wn = warp >> 2;
   const int n = min(CH, a.L - c * CH);
   const size_t row0 = (size_t)b * a.L + (size_t)c * CH;
-  fill_cumlog(pd, a.log_g + row0 * a.H + h, a.H, n);
-  if (tid >= 32 && tid < 32 + CH) ks[tid - 32] = tid - 32 < n ? a.k_scale[(row0 + tid - 32) * a.H + h] : 0.f;
+  const ChunkDecay<KIND> dec = chunk_decay<KIND>(a, row0, h, n, pd, pw);
+  if (!PAIR && tid >= 32 && tid < 32 + CH) ks[tid - 32] = tid - 32 < n ? a.k_scale[(row0 + tid - 32) * a.H + h] : 0.f;
   {
     Block<CH, DK> qb, kb;
     qb.fetch(a.q + row0 * a.ld_q + (size_t)(h / a.rep) * DK, a.ld_q, n);
     kb.fetch(a.k + row0 * a.ld_k + (size_t)(h / a.rep) * DK, a.ld_k, n);
-    qb.put(Qs, LDK, a.q_mul);
-    kb.put(Ks, LDK, 1.f);
+    if constexpr (PAIR) {
+      qb.act(a.act_in);
+      kb.act(a.act_in);
+      qb.put_split(Qs, Ql, LDK, nullptr);
+      kb.put_split(Ks, Kl, LDK, nullptr);
+    } else {
+      qb.put(Qs, LDK, a.q_mul);
+      kb.put(Ks, LDK, 1.f);
+    }
   }
   const float* P = a.ws + (((size_t)b * a.H + h) * NC + c) * DK * a.DV;
   const float* vsrc = a.v + row0 * a.ld_v + (size_t)h * a.DV;
@@ -496,6 +561,16 @@ __global__ void __launch_bounds__(256) lin_chunk_out_mma_kernel(RecurArgs a, int
       ldsm4(k_1, smem_addr(kp + (size_t)16 * LDK + k0));
       mma16816(acc[0], q, k_0[0], k_0[1]); mma16816(acc[1], q, k_0[2], k_0[3]);
       mma16816(acc[2], q, k_1[0], k_1[1]); mma16816(acc[3], q, k_1[2], k_1[3]);
+      if constexpr (PAIR) {
+        uint32_t ql[4];
+        ldsm4(ql, smem_addr(Ql + qa + k0));
+        mma16816(acc[0], ql, k_0[0], k_0[1]); mma16816(acc[1], ql, k_0[2], k_0[3]);
+        mma16816(acc[2], ql, k_1[0], k_1[1]); mma16816(acc[3], ql, k_1[2], k_1[3]);
+        ldsm4(k_0, smem_addr(kp + (Kl - Ks) + k0));
+        ldsm4(k_1, smem_addr(kp + (Kl - Ks) + (size_t)16 * LDK + k0));
+        mma16816(acc[0], q, k_0[0], k_0[1]); mma16816(acc[1], q, k_0[2], k_0[3]);
+        mma16816(acc[2], q, k_1[0], k_1[1]); mma16816(acc[3], q, k_1[2], k_1[3]);
+      }
     }
     float sum[2] = {0.f, 0.f};
 #pragma unroll
@@ -503,22 +578,24 @@ __global__ void __launch_bounds__(256) lin_chunk_out_mma_kernel(RecurArgs a, int
 #pragma unroll
       for (int u = 0; u < 2; ++u) {                  // rows r0, r0 + 8
         const int i = r0 + u * 8, j = wn * 32 + t * 8 + (lane & 3) * 2;
-        const float x = j <= i ? acc[t][2 * u] * (expf((float)(pd[i] - pd[j])) * ks[j]) : 0.f;
-        const float y = j + 1 <= i ? acc[t][2 * u + 1] * (expf((float)(pd[i] - pd[j + 1])) * ks[j + 1]) : 0.f;
+        const float x = j <= i ? acc[t][2 * u] * (PAIR ? dec.between(j, i) : dec.between(j, i) * ks[j]) : 0.f;
+        const float y = j + 1 <= i ? acc[t][2 * u + 1] * (PAIR ? dec.between(j + 1, i) : dec.between(j + 1, i) * ks[j + 1]) : 0.f;
         sum[u] += x + y;
         const __nv_bfloat162 hi = __floats2bfloat162_rn(x, y);
         *reinterpret_cast<__nv_bfloat162*>(Ah + (size_t)i * LDE + j) = hi;
         *reinterpret_cast<__nv_bfloat162*>(Al + (size_t)i * LDE + j) = __floats2bfloat162_rn(x - __low2float(hi), y - __high2float(hi));
       }
+    if constexpr (!PAIR) {
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      sum[u] += __shfl_xor_sync(L3_FULL, sum[u], 1);
-      sum[u] += __shfl_xor_sync(L3_FULL, sum[u], 2);
-      if ((lane & 3) == 0) s_nq[wn][r0 + u * 8] = sum[u];
+      for (int u = 0; u < 2; ++u) {
+        sum[u] += __shfl_xor_sync(L3_FULL, sum[u], 1);
+        sum[u] += __shfl_xor_sync(L3_FULL, sum[u], 2);
+        if ((lane & 3) == 0) s_nq[wn][r0 + u * 8] = sum[u];
+      }
     }
   }
   __syncthreads();
-  if (ne == 0) {  // n . q of every token: four threads per row
+  if (!PAIR && ne == 0) {  // n . q of every token: four threads per row
     const float* Pn = chunk_norms(a, NC) + (((size_t)b * a.H + h) * NC + c) * DK;
     const int i = tid >> 2, part = tid & 3;
     float t = 0.f;
@@ -532,11 +609,12 @@ __global__ void __launch_bounds__(256) lin_chunk_out_mma_kernel(RecurArgs a, int
     t += __shfl_xor_sync(L3_FULL, t, 2);
     if (part == 0 && i < n) a.nq[(row0 + i) * a.H + h] = fmaf(t, expf((float)pd[i]), s_nq[0][i] + s_nq[1][i]);
   }
-  const float f0 = expf((float)pd[r0]), f1 = expf((float)pd[r0 + 8]);
+  const float f0 = dec.upto(r0), f1 = dec.upto(r0 + 8);
   const size_t va = (size_t)(lane & 15) * LDE + wn * 32 + (lane >> 4) * 8, aa = (size_t)(wm * 16 + (lane & 15)) * LDE + (lane >> 4) * 8;
   for (int e0 = e_lo; e0 < e_hi; e0 += 64) {
     if (e0 > e_lo) __syncthreads();  // the previous tile's Vs / P are no longer read
-    vb.put(Vs, LDE, 1.f);
+    if constexpr (PAIR) { vb.act(a.act_in); vb.put_split(Vs, Vl, LDE, nullptr); }
+    else vb.put(Vs, LDE, 1.f);
     pb.put_split(Ph, Pl, LDE, nullptr);
     __syncthreads();
     if (e0 + 64 < e_hi) { vb.fetch(vsrc + e0 + 64, a.ld_v, n); pb.fetch(P + e0 + 64, a.DV, DK); }
@@ -551,6 +629,12 @@ __global__ void __launch_bounds__(256) lin_chunk_out_mma_kernel(RecurArgs a, int
       ldsm4t(p1, smem_addr(Ph + o + 16));
       mma16816(acc[0], q, p0[0], p0[1]); mma16816(acc[1], q, p0[2], p0[3]);
       mma16816(acc[2], q, p1[0], p1[1]); mma16816(acc[3], q, p1[2], p1[3]);
+      if constexpr (PAIR) {
+        uint32_t ql[4];
+        ldsm4(ql, smem_addr(Ql + qa + k0));
+        mma16816(acc[0], ql, p0[0], p0[1]); mma16816(acc[1], ql, p0[2], p0[3]);
+        mma16816(acc[2], ql, p1[0], p1[1]); mma16816(acc[3], ql, p1[2], p1[3]);
+      }
       ldsm4t(p0, smem_addr(Pl + o));
       ldsm4t(p1, smem_addr(Pl + o + 16));
       mma16816(acc[0], q, p0[0], p0[1]); mma16816(acc[1], q, p0[2], p0[3]);
@@ -570,6 +654,12 @@ __global__ void __launch_bounds__(256) lin_chunk_out_mma_kernel(RecurArgs a, int
       mma16816(acc[2], ah, v1[0], v1[1]); mma16816(acc[3], ah, v1[2], v1[3]);
       mma16816(acc[0], al, v0[0], v0[1]); mma16816(acc[1], al, v0[2], v0[3]);
       mma16816(acc[2], al, v1[0], v1[1]); mma16816(acc[3], al, v1[2], v1[3]);
+      if constexpr (PAIR) {
+        ldsm4t(v0, smem_addr(Vl + o));
+        ldsm4t(v1, smem_addr(Vl + o + 16));
+        mma16816(acc[0], ah, v0[0], v0[1]); mma16816(acc[1], ah, v0[2], v0[3]);
+        mma16816(acc[2], ah, v1[0], v1[1]); mma16816(acc[3], ah, v1[2], v1[3]);
+      }
     }
     float* op = a.out + (row0 + r0) * O + (size_t)h * a.DV + e0 + wn * 32 + (lane & 3) * 2;
 #pragma unroll
@@ -623,23 +713,29 @@ cudaError_t launch_recur_chunk(const RecurArgs& a, cudaStream_t s) {
     if ((e = launch_k(k_scan, dim3((n4 + 255) / 256, a.H, a.B), dim3(256), 0, s, a, NC)) != cudaSuccess) return e;
     return launch_k(k_out, grid, dim3(256), sm3, s, a, NC);
   };
-  if (a.n_state && a.bf16_ops) {
-    const size_t sb1 = ((size_t)2 * CH * (a.DK + 8) + CH * LDE) * 2, sb3 = ((size_t)2 * CH * (a.DK + 8) + 3 * CH * LDE + 2 * (size_t)a.DK * LDE) * 2;
+  if (a.bf16_ops) {
     const int ctas = NC * a.H * a.B, tiles = a.DV / 64;
-    const int ne1 = value_splits(ctas, tiles, 100), ne3 = value_splits(ctas, tiles, 100);  // measured: only short prompts of few heads gain
-    auto go_mma = [&](auto k_state, auto k_out) {
+    const int ne = value_splits(ctas, tiles, 100);  // measured: only short prompts of few heads gain
+    auto go_mma = [&](auto k_state, auto k_scan, auto k_out) {
+      const size_t sb1 = state_mma_smem(a.DK, !a.n_state), sb3 = out_mma_smem(a.DK, !a.n_state);
       cudaError_t e;
       if ((e = cudaFuncSetAttribute(k_state, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb1)) != cudaSuccess) return e;
       if ((e = cudaFuncSetAttribute(k_out, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb3)) != cudaSuccess) return e;
-      if ((e = launch_k(k_state, dim3(NC * ne1, a.H, a.B), dim3(256), sb1, s, a, NC, ne1)) != cudaSuccess) return e;
-      if ((e = launch_k(lin_chunk_scan_kernel<true, true>, dim3((n4 + 255) / 256, a.H, a.B), dim3(256), 0, s, a, NC)) != cudaSuccess) return e;
-      return launch_k(k_out, dim3(NC * ne3, a.H, a.B), dim3(256), sb3, s, a, NC, ne3);
+      if ((e = launch_k(k_state, dim3(NC * ne, a.H, a.B), dim3(256), sb1, s, a, NC, ne)) != cudaSuccess) return e;
+      if ((e = launch_k(k_scan, dim3((n4 + 255) / 256, a.H, a.B), dim3(256), 0, s, a, NC)) != cudaSuccess) return e;
+      return launch_k(k_out, dim3(NC * ne, a.H, a.B), dim3(256), sb3, s, a, NC, ne);
+    };
+    auto go_kind = [&](auto dk) {
+      constexpr int DK = decltype(dk)::value;
+      if (a.n_state) return go_mma(lin_chunk_state_mma_kernel<DK, CK_MLSTM>, lin_chunk_scan_kernel<true, true>, lin_chunk_out_mma_kernel<DK, CK_MLSTM>);
+      if (a.mode == 2) return go_mma(lin_chunk_state_mma_kernel<DK, CK_TOKEN>, lin_chunk_scan_kernel<true, false>, lin_chunk_out_mma_kernel<DK, CK_TOKEN>);
+      return go_mma(lin_chunk_state_mma_kernel<DK, CK_FIXED>, lin_chunk_scan_kernel<false, false>, lin_chunk_out_mma_kernel<DK, CK_FIXED>);
     };
     switch (a.DK) {
-      case 64: return go_mma(lin_chunk_state_mma_kernel<64>, lin_chunk_out_mma_kernel<64>);
-      case 128: return go_mma(lin_chunk_state_mma_kernel<128>, lin_chunk_out_mma_kernel<128>);
-      case 192: return go_mma(lin_chunk_state_mma_kernel<192>, lin_chunk_out_mma_kernel<192>);
-      default: return go_mma(lin_chunk_state_mma_kernel<256>, lin_chunk_out_mma_kernel<256>);
+      case 64: return go_kind(std::integral_constant<int, 64>{});
+      case 128: return go_kind(std::integral_constant<int, 128>{});
+      case 192: return go_kind(std::integral_constant<int, 192>{});
+      default: return go_kind(std::integral_constant<int, 256>{});
     }
   }
   if (a.n_state) return go(lin_chunk_state_kernel<true, true>, lin_chunk_scan_kernel<true, true>, lin_chunk_out_kernel<true, true>);
