@@ -210,7 +210,10 @@ struct EpiArgs {
   int unary;             // STORE: UnaryAct applied to every output value
   // SWIGLU with a routing weight on the unit's INPUT: output j of row m is act(w g) * (w u) with
   // w = glu_w[m * glu_w_ld + j / glu_group] for j < glu_groups * glu_group and 1 beyond (a shared expert); w = 0 gives 0.
+  // (glu_w_out: on its OUTPUT, w act(g) u; the bf16 kernel of gemm_tc.cu only)
   const float* glu_w;    // null: no weight
+  int glu_w_out;
+  int glu_exact;         // silu with expf and a full division also where the kernel would take the fast forms
   int glu_w_ld, glu_group, glu_groups;
 };
 // a gated unit's output from its gate and up values (FAST: exp2-based exponential and approximate divide)

@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmB1,
                int rows, int N, int K, int bn, int a_box_rows, int nst, int ksplit, float* part, int* tile_cnt, int* err,
-               unsigned long long* dbg, EpiArgs e) {
+               unsigned long long* dbg, TcGroups grp, EpiArgs e) {
   extern __shared__ uint8_t smem_raw[];
   pdl_launch();  // the next kernel may start its own prologue now
   if (threadIdx.x == 0) {
@@ -64,7 +64,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
   tc_pipe_ready(p);
   pdl_wait();  // everything above overlapped the previous kernel; its outputs are visible from here
   if (threadIdx.x == 0) TC_STAMP(dbg, 1);
-  tc_gemm_run<KIND, BN, CG, EPI>(p, &tmA0, &tmA1, &tmB0, &tmB1, rows, N, K, a_box_rows, ksplit, part, tile_cnt, e, blockIdx.x / CG, gridDim.x / CG);
+  tc_gemm_run<KIND, BN, CG, EPI>(p, &tmA0, &tmA1, &tmB0, &tmB1, rows, N, K, a_box_rows, ksplit, part, tile_cnt, grp, e, blockIdx.x / CG, gridDim.x / CG);
   if (threadIdx.x == 64) TC_STAMP(dbg, 34);
   tc_pipe_teardown<KIND, BN, CG>(p, err);
   if (threadIdx.x == 0) TC_STAMP(dbg, 35);
@@ -174,12 +174,13 @@ static void pick_bf16(const TcGemmArgs& a, int sms, int* cg_out, int* bn_out, in
   const int nkb = (a.K + 63) / 64;
   const double per_col = a.epi == EPI_ROPE_KV ? 26 : a.epi == EPI_RESID ? 24 : a.epi == EPI_SWIGLU ? 14 : 20;
   double best = 0;
-  for (int cg = 1; cg <= (a.rows > 128 ? 2 : 1); ++cg) {
-    const int tm = (a.rows + 128 * cg - 1) / (128 * cg);
+  const int rows = a.groups ? a.group_rows : a.rows;
+  for (int cg = 1; cg <= (rows > 128 && !a.groups ? 2 : 1); ++cg) {
+    const int tm = (rows + 128 * cg - 1) / (128 * cg);
     for (int bn = 256; bn >= 32; bn -= 32) {
       const int tn = (a.N + bn - 1) / bn, tiles = tm * tn;
       const double block = std::max(2.0 * bn, cg == 1 ? 128 + 1.79 * bn : 160 + 0.93 * bn), epi = 1500 + per_col * bn;
-      for (int ks = 1; ks <= (a.epi == EPI_ARGMAX ? 1 : 8); ++ks) {
+      for (int ks = 1; ks <= (a.epi == EPI_ARGMAX || a.groups ? 1 : 8); ++ks) {
         const int per = (nkb + ks - 1) / ks;
         if (ks > 1 && (!a.part || !a.tile_cnt || tiles * cg > a.tile_cnt_len || per < 3 || (ks - 1) * per >= nkb ||
                        (size_t)tiles * cg * 128 * bn * sizeof(float) * ks > a.part_bytes)) continue;
@@ -208,7 +209,8 @@ static cudaError_t launch_tc_t(const TcGemmArgs& a, cudaStream_t s) {
   const int bn = BN ? BN : a.bn, TM = 128 * CG;
   const int a_box = a.rows >= 128 ? 128 : ((a.rows + 7) & ~7);
   const CUtensorMap* A0 = g_maps.get(a.A[0], b16, a.rows, a.K, a_box);
-  const CUtensorMap* B0 = g_maps.get(a.W[0], b16, a.N, a.K, bn / CG);
+  const int w_rows = a.groups ? a.w_rows : a.N, w_cols = a.groups ? a.w_cols : a.K;
+  const CUtensorMap* B0 = g_maps.get(a.W[0], b16, w_rows, w_cols, bn / CG, a.ldw ? a.ldw : w_cols);
   const CUtensorMap* A1 = Cf::PARTS == 2 ? g_maps.get(a.A[1], b16, a.rows, a.K, a_box) : A0;
   const CUtensorMap* B1 = Cf::PARTS == 2 ? g_maps.get(a.W[1], b16, a.N, a.K, bn / CG) : B0;
   if (!A0 || !B0 || !A1 || !B1) return cudaErrorInvalidValue;
@@ -234,7 +236,7 @@ static cudaError_t launch_tc_t(const TcGemmArgs& a, cudaStream_t s) {
   const int nkb = (nkb_all + ksplit - 1) / ksplit;
   const int nst = std::max(2, std::min(std::min(Cf::stages(bn), env_st), nkb));
   return launch_kc(kern, grid, dim3(TC_THREADS), (size_t)Cf::smem(bn, nst), s, CG, *A0, *A1, *B0, *B1, a.rows, a.N, a.K, bn, a_box, nst, ksplit, a.part, a.tile_cnt,
-                  a.err, g_tc_dbg_to.load(), a.e);
+                  a.err, g_tc_dbg_to.load(), TcGroups{a.groups, a.group_n, a.group_k}, a.e);
 }
 
 template <int KIND, int BN, int CG>

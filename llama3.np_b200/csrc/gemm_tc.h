@@ -16,6 +16,12 @@ struct TcGemmArgs {
   int bn, ksplit;       // set by the launcher
   int epi;
   EpiArgs e;
+  int ldw;              // row stride of W (0: K)
+  // bf16: rows in groups that take their own part of W.  groups (device): [0] the number of 128-row tiles, [1 + i] the group g of tile i;
+  // a tile's weight rows start at g * group_n, its K range at g * group_k.  W is [w_rows, w_cols]; `rows` is the room of A and of the
+  // outputs, group_rows what the caller expects to be used (the choice of the tile width).
+  const int* groups;
+  int group_n, group_k, w_rows, w_cols, group_rows;
   // optional caller-owned scratch for the deterministic K-split of gemm_tc.cu (null: never split)
   float* part;       // room for ksplit x (rows padded to 128) x (N padded to the tile) fp32 partial sums
   size_t part_bytes;

@@ -173,6 +173,9 @@ struct TcPipe {
   unsigned long long* dbg;
 };
 
+// rows in groups (TcGemmArgs::groups)
+struct TcGroups { const int* tiles; int n, k; };
+
 // TC_THREADS: warp 0 = TMA, warp 1 = TMEM + MMA, warps 2-9 = epilogue.  smem: nst stages | EPI_BYTES | barriers.
 // Only the barriers stand between a kernel's start and its first copy: TMEM is handed out meanwhile, and the warps that use it meet
 // in tc_pipe_ready.
@@ -255,7 +258,7 @@ __device__ __forceinline__ void tc_pipe_teardown(TcPipe& p, int* err) {
 template <int KIND, int BN, int CG, int EPI>
 __device__ __forceinline__ void tc_gemm_run(TcPipe& p, const CUtensorMap* tmA0, const CUtensorMap* tmA1, const CUtensorMap* tmB0,
                                             const CUtensorMap* tmB1, int rows, int N, int K, int a_box_rows, int ksplit, float* part,
-                                            int* tile_cnt, const EpiArgs& e, int first_tile, int tile_stride) {
+                                            int* tile_cnt, const TcGroups& grp, const EpiArgs& e, int first_tile, int tile_stride) {
   using Cf = TcCfg<KIND, BN, CG>;
   using KVT = typename std::conditional<KIND == TC_BF16, bf16, float>::type;
   constexpr int PARTS = Cf::PARTS, NBUF = Cf::NBUF;
@@ -265,7 +268,8 @@ __device__ __forceinline__ void tc_gemm_run(TcPipe& p, const CUtensorMap* tmA0, 
   const uint32_t tiles = p.tiles, full0 = p.full0, empty0 = p.empty0, accfull0 = p.accfull0, accempty0 = p.accempty0;
   const int warp = __shfl_sync(L3_FULL, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   constexpr int TM = CG * Cf::BM;  // rows of an output tile
-  const int tiles_m = (rows + TM - 1) / TM, tiles_n = (N + bn - 1) / bn;
+  const bool grouped = KIND == TC_BF16 && grp.tiles;
+  const int tiles_m = grouped ? grp.tiles[0] : (rows + TM - 1) / TM, tiles_n = (N + bn - 1) / bn;
   const int ntiles_mn = tiles_m * tiles_n;
   const int ntiles = ntiles_mn * ksplit;  // K-split: tile t = (k slice t / ntiles_mn, output tile t % ntiles_mn)
   const int nkb = (K + Cf::BK - 1) / Cf::BK;
@@ -279,7 +283,8 @@ __device__ __forceinline__ void tc_gemm_run(TcPipe& p, const CUtensorMap* tmA0, 
     uint32_t ph = 1;
     for (int t = first_tile; t < ntiles; t += tile_stride) {
       const int tmn = t % ntiles_mn, ks = t / ntiles_mn;
-      const int m0 = (tmn % tiles_m) * TM + rank * Cf::BM, n0 = (tmn / tiles_m) * bn + rank * (bn / CG);
+      const int g = grouped ? grp.tiles[1 + tmn % tiles_m] : 0, kg = g * grp.k;
+      const int m0 = (tmn % tiles_m) * TM + rank * Cf::BM, n0 = (tmn / tiles_m) * bn + rank * (bn / CG) + g * grp.n;
       const int kb0 = ks * kb_per, kb1 = min(nkb, kb0 + kb_per);
       for (int kb = kb0; kb < kb1; ++kb) {
         mbar_wait(empty0 + 8 * s, ph, fail);
@@ -289,13 +294,13 @@ __device__ __forceinline__ void tc_gemm_run(TcPipe& p, const CUtensorMap* tmA0, 
             const uint32_t bar = pair_addr(full0 + 8 * s, 0);
             if (rank == 0) mbar_expect_tx(full0 + 8 * s, CG * STAGE_BYTES);
             pair_load_2d(st, tmA0, kb * Cf::BK, m0, bar);
-            pair_load_2d(st + Cf::A_BYTES, tmB0, kb * Cf::BK, n0, bar);
+            pair_load_2d(st + Cf::A_BYTES, tmB0, kb * Cf::BK + kg, n0, bar);
           } else {
             // the A box holds only the rows that exist (decode batches of 9..127 rows): rows beyond it
             // keep stale shared memory, which only feeds accumulator rows the epilogue never reads
             mbar_expect_tx(full0 + 8 * s, PARTS * (a_box_rows * 128 + B_BYTES));
             tma_load_2d(st, tmA0, kb * Cf::BK, m0, full0 + 8 * s);
-            tma_load_2d(st + PARTS * Cf::A_BYTES, tmB0, kb * Cf::BK, n0, full0 + 8 * s);
+            tma_load_2d(st + PARTS * Cf::A_BYTES, tmB0, kb * Cf::BK + kg, n0, full0 + 8 * s);
             if (PARTS == 2) {
               tma_load_2d(st + Cf::A_BYTES, tmA1, kb * Cf::BK, m0, full0 + 8 * s);
               tma_load_2d(st + PARTS * Cf::A_BYTES + B_BYTES, tmB1, kb * Cf::BK, n0, full0 + 8 * s);
@@ -618,11 +623,18 @@ __device__ __forceinline__ void tc_gemm_run(TcPipe& p, const CUtensorMap* tmA0, 
                 else hv[i] = silu_ref(t.x) * t.y;
               }
             } else {
+              const int g = e.glu_w ? (col >> 1) / e.glu_group : 0;
+              const bool weighted = e.glu_w && g < e.glu_groups;
+              float wt[16];
+#pragma unroll
+              for (int i = 0; i < 16; ++i) wt[i] = weighted && mr + 2 * i < rows ? e.glu_w[(size_t)(mr + 2 * i) * e.glu_w_ld + g] : 1.f;
 #pragma unroll
               for (int i = 0; i < 16; ++i) {
                 float2 t = staged(i);
-                if (e.glu_w && mr + 2 * i < rows) { const float w = glu_in_weight(e, mr + 2 * i, col >> 1); t.x *= w; t.y *= w; }
-                hv[i] = e.act == GLU_SILU && KIND == TC_BF16 ? t.x * __fdividef(1.0f, 1.0f + __expf(-t.x)) * t.y : glu_pair<KIND == TC_BF16>(e, t.x, t.y);
+                const float wi = e.glu_w_out ? 1.f : wt[i];
+                t.x *= wi; t.y *= wi;
+                hv[i] = e.act == GLU_SILU && KIND == TC_BF16 && !e.glu_exact ? t.x * __fdividef(1.0f, 1.0f + __expf(-t.x)) * t.y : glu_pair<KIND == TC_BF16>(e, t.x, t.y);
+                if (e.glu_w_out) hv[i] *= wt[i];
               }
             }
             const size_t o = (size_t)mr * e.ld_out + (col >> 1);

@@ -1220,6 +1220,14 @@ int ll_finalize(L3Model* m) {
     CK(m, cudaMalloc((void**)&ll->moe_w, ct * max_top * 4));
     CK(m, cudaMalloc((void**)&ll->moe_dense, ct * max_exp * 4));
     CK(m, cudaMalloc((void**)&ll->moe_idw, ct * 4));
+    if (max_gu) {  // pairs in groups: places, tiles, weights (moe_group_tiles bounds the tiles)
+      const size_t tiles = moe_group_tiles((int)ct, max_top, max_exp);
+      CK(m, cudaMalloc((void**)&ll->moe_row_of, ct * max_top * 4));
+      CK(m, cudaMalloc((void**)&ll->moe_groups, (1 + tiles) * 4));
+      CK(m, cudaMalloc((void**)&ll->moe_wg, tiles * 128 * 4));
+      ll->moe_gu_bytes = ct * max_gu * 4;
+      ll->moe_h16_len = ct * std::max(1, ll->max_ff);
+    }
   }
   for (const LLLayer& L0 : ll->layers)
     for (const LLLayer* U = &L0; U; U = U->pair) {
@@ -1322,7 +1330,7 @@ void ll_destroy(L3Model* m) {
   fr(ll->diff_part_o); fr(ll->diff_part_ml);
   fr(ll->Xs); fr(ll->hn); fr(ll->hf); fr(ll->hf16); fr(ll->y1); fr(ll->y2); fr(ll->moe_gu);
   fr(ll->lat_q16); fr(ll->win_q16); fr(ll->diff_maps); fr(ll->lat_exp); fr(ll->lat_part_o); fr(ll->lat_part_ml);
-  fr(ll->loop_step); fr(ll->qlat); fr(ll->aux16); fr(ll->moe_sel); fr(ll->moe_w); fr(ll->moe_dense); fr(ll->moe_idw);
+  fr(ll->loop_step); fr(ll->qlat); fr(ll->aux16); fr(ll->moe_sel); fr(ll->moe_w); fr(ll->moe_dense); fr(ll->moe_idw); fr(ll->moe_row_of); fr(ll->moe_groups); fr(ll->moe_wg);
   fr(ll->pin); fr(ll->aux); fr(ll->rk); fr(ll->rv); fr(ll->rg); fr(ll->rbeta); fr(ll->o); fr(ll->sg); fr(ll->sg16); fr(ll->x2); fr(ll->chunk_ws);
   delete ll;
   m->ll = nullptr;
@@ -1548,6 +1556,56 @@ static EpiArgs resid_into(float* x, int ld) {
   EpiArgs e{};
   e.out = x; e.resid = x; e.ld_out = ld;
   return e;
+}
+
+// Gated experts of many rows: all of them as one product with zero weights, or in groups, every expert over the rows that chose it.
+// Groups cost a pass to order the pairs, a gather and a sum (8 + 7 + 10 us) and up to 127 rows of padding per expert; they run where the
+// products that they leave out take more than 20 us at 1.2 PFLOP/s (the masked pass over all hidden values goes as well).  2000
+// tokens of width 2048, the best 2 of 16 experts of 1024 and a shared one of 2048, us: masked 300 of products + 48 of hidden
+// values, groups 60 + 30 for the experts, 31 + 20 for the shared one, 25 for the order.
+static bool ll_moe_in_groups(const L3Model* m, const LLLayer& Ly, const void* x16, int ntok) {
+  const L3LayerSpec& s = Ly.spec;
+  const LayerList* ll = m->ll;
+  const int W = m->D, F = Ly.ff_total;
+  if (!x16 || !m->h16 || !ll->moe_row_of || ntok <= 128 || s.ff % 64 || W % 64 || s.shared_ff % 8 || s.experts > 1024 || !ll_takes_mirror(m, ntok, 2 * F, W)) return false;
+  const size_t rows = (size_t)moe_group_tiles(ntok, s.top, s.experts) * 128;
+  if (rows * W * 6 > ll->moe_gu_bytes || rows * s.ff > ll->moe_h16_len || (size_t)ntok * s.shared_ff > ll->moe_h16_len) return false;
+  const double mt = (ntok + 127) / 128, all = mt * F, grouped = (ntok * s.top / 128.0 + s.experts * 0.5) * s.ff + mt * s.shared_ff;  // row tiles x hidden columns
+  return (all - grouped) * 128 * W * 6 / 1.2e15 > 20e-6;
+}
+
+// dst (+)= the experts' outputs; the shared expert's go through `epi` first (sw: its weight per row, on the output).  Experts' weights scale
+// their outputs (w_out) or their inputs.
+static int ll_moe_groups(L3Model* m, const LLLayer& Ly, const void* x16, int ntok, bool w_out, const float* sw, int epi, const EpiArgs& e_shared, float* dst) {
+  const L3LayerSpec& s = Ly.spec;
+  LayerList* ll = m->ll;
+  const int W = m->D, F = Ly.ff_total, E = s.experts, ff = s.ff, sff = s.shared_ff;
+  const bf16 *w13 = (const bf16*)Ly.w13, *w2 = (const bf16*)Ly.w2;
+  TcGemmArgs t{};
+  t.kind = TC_BF16;
+  t.part = m->gemm_part; t.part_bytes = (size_t)32 << 20; t.tile_cnt = m->gemm_cnt; t.tile_cnt_len = 1024; t.err = m->h_err;
+  if (sff) {
+    t.A[0] = x16; t.W[0] = w13 + (size_t)2 * E * ff * W; t.rows = ntok; t.N = 2 * sff; t.K = W; t.epi = EPI_SWIGLU; t.e = store_to(nullptr, m->h16, sff);
+    t.e.act = GLU_SILU; t.e.glu_exact = 1;
+    if (sw) { t.e.glu_w = sw; t.e.glu_w_ld = 1; t.e.glu_group = sff; t.e.glu_groups = 1; t.e.glu_w_out = 1; }
+    LAUNCH(m, launch_gemm_tc(t, m->stream));
+    t.A[0] = m->h16; t.W[0] = w2 + (size_t)E * ff; t.N = W; t.K = sff; t.ldw = F; t.epi = epi; t.e = e_shared;
+    LAUNCH(m, launch_gemm_tc(t, m->stream));
+  }
+  const int rows = moe_group_tiles(ntok, s.top, E) * 128;
+  bf16* xg = (bf16*)ll->moe_gu;
+  float* yg = (float*)(xg + (size_t)rows * W);
+  LAUNCH(m, launch_moe_group(ll->moe_sel, ll->moe_w, ntok, s.top, E, W, (const bf16*)x16, ll->moe_row_of, ll->moe_groups, xg, ll->moe_wg, m->stream));
+  m->launch_acc += 1;
+  t.groups = ll->moe_groups; t.rows = rows; t.group_rows = ntok * s.top + E * 64; t.ldw = 0;
+  t.A[0] = xg; t.W[0] = w13; t.N = 2 * ff; t.K = W; t.group_n = 2 * ff; t.group_k = 0; t.w_rows = 2 * E * ff; t.w_cols = W;
+  t.epi = EPI_SWIGLU; t.e = store_to(nullptr, m->h16, ff);
+  t.e.act = GLU_SILU; t.e.glu_exact = 1; t.e.glu_w = ll->moe_wg; t.e.glu_w_ld = 1; t.e.glu_group = ff; t.e.glu_groups = 1; t.e.glu_w_out = w_out;
+  LAUNCH(m, launch_gemm_tc(t, m->stream));
+  t.A[0] = m->h16; t.W[0] = w2; t.N = W; t.K = ff; t.group_n = 0; t.group_k = ff; t.w_rows = W; t.w_cols = F; t.epi = EPI_STORE; t.e = store_to(yg, nullptr, W);
+  LAUNCH(m, launch_gemm_tc(t, m->stream));
+  LAUNCH(m, launch_moe_combine(yg, ll->moe_row_of, ntok, s.top, W, sff || epi == EPI_RESID, dst, m->stream));
+  return L3_OK;
 }
 
 // A recurrence with a decay per key channel (ra filled, decays in ll->rg): where its prompt runs on the tensor products, its
@@ -1921,6 +1979,8 @@ static int ll_enqueue_prenorm(L3Model* m, int B, int L, float* d_resid) {
       if (few) {
         LAUNCH(m, launch_moe_glu_rows(h2, Ly.w13, Ly.w2, m->bf16, ll->moe_sel, ll->moe_w, sw, true, ntok, W, E, ff, s.shared_ff, s.top, m->h, m->x, true, m->stream));
         m->launch_acc += 1;
+      } else if (ll_moe_in_groups(m, Ly, h2_16, ntok)) {
+        if ((rc = ll_moe_groups(m, Ly, h2_16, ntok, true, sw, EPI_RESID, resid_into(m->x, W), m->x)) != L3_OK) return rc;
       } else {
         if ((rc = ll_linear(m, Ly.w13, h2, h2_16, 0, ntok, 2 * F, W, EPI_STORE, store_to(ll->moe_gu, nullptr, 2 * F))) != L3_OK) return rc;
         LAUNCH(m, launch_moe_glu_act(ll->moe_gu, ll->moe_dense, sw, true, ntok, E, ff, s.shared_ff, m->h16 && ll_takes_mirror(m, ntok, W, F) ? nullptr : m->h,
@@ -2034,6 +2094,8 @@ static int ll_enqueue_parallel(L3Model* m, int B, int L, float* d_resid) {
       if (few) {
         LAUNCH(m, launch_moe_glu_rows(hf, Ly.w13, Ly.w2, m->bf16, ll->moe_sel, ll->moe_w, nullptr, false, ntok, W, E, ff, s.shared_ff, s.top, m->h, ll->y2, false, m->stream));
         m->launch_acc += 1;
+      } else if (ll_moe_in_groups(m, Ly, hf16, ntok)) {
+        if ((rc = ll_moe_groups(m, Ly, hf16, ntok, false, nullptr, EPI_STORE, store_to(ll->y2, nullptr, W), ll->y2)) != L3_OK) return rc;
       } else {
         // gate | up of every expert and of the shared one in ONE projection, then the routing weight (zero for experts the
         // row did not choose) and silu(g) * u in a streaming kernel.  L3_MOE_EPI=1 moves that step into the GEMM's epilogue:

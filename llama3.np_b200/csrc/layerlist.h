@@ -129,6 +129,10 @@ struct LayerList {
   int keys_end = 0;                        // position behind the last token of the chunk being enqueued
   float *lat_part_o = nullptr, *lat_part_ml = nullptr;  // split scratch of the latent attention
   float *moe_w = nullptr, *moe_dense = nullptr, *moe_idw = nullptr;  // [rows, top] | [rows, experts] | [rows]
+  // gated experts of many rows in groups (bf16 mode): pairs' places [rows, top], tiles and their experts, weights by place
+  int *moe_row_of = nullptr, *moe_groups = nullptr;
+  float* moe_wg = nullptr;
+  size_t moe_gu_bytes = 0, moe_h16_len = 0;  // room of moe_gu, entries of h16
   int32_t* moe_sel = nullptr;              // [rows, top]
   // parallel layers
   float* Xs = nullptr;                     // [n_layers + 1][cap_tok, width] embedding output and every layer's own result

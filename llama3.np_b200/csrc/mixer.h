@@ -331,6 +331,13 @@ struct MoeRouteArgs {
   float* idw;            // [rows] summed weight of the chosen identity slots (shared_gate: the shared expert's weight)
 };
 cudaError_t launch_moe_route(const MoeRouteArgs& a, int rows, cudaStream_t s);
+// pairs (row, chosen expert) ordered by expert in tiles of 128 rows: row_of [rows * top] a pair's place (-1: none), groups
+// [1 + moe_group_tiles] as TcGemmArgs::groups, xg / wg the pairs' inputs and weights at their places
+inline int moe_group_tiles(int rows, int top, int E) { return (rows * top + E * 127) / 128 + 1; }
+cudaError_t launch_moe_group(const int32_t* sel, const float* w, int rows, int top, int E, int D, const bf16* x16, int* row_of, int* groups, bf16* xg, float* wg,
+                             cudaStream_t s);
+// y[r] = (add: y[r] +) the sum of the row's pairs' results yg
+cudaError_t launch_moe_combine(const float* yg, const int* row_of, int rows, int top, int D, bool add, float* y, cudaStream_t s);
 // u[r, c] <- relu(u[r, c])^2 * dense[r, c / ff]  (+ bf16 mirror)
 cudaError_t launch_moe_act_mask(float* u, const float* dense, int rows, int E, int ff, bf16* out16, cudaStream_t s);
 // x[r, i] += idw[r] * h[r, i]

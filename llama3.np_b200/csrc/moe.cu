@@ -15,6 +15,9 @@
 //  down(silu(w g) * (w u)) and a shared expert:
 //  * moe_glu_act_kernel    masked-dense path: [rows, 2 F] interleaved (gate, up) of all experts and the shared one ->
 //                          [rows, F] hidden values, zero where the row did not choose the expert
+//  * moe_group_kernel, moe_gather_kernel, moe_combine_kernel   many rows of bf16 mode, where the masked-dense products would be mostly
+//                          zeros: (row, expert) pairs ordered by expert in tiles of 128, their inputs gathered, and after the two
+//                          grouped projections (gemm_tc.cu, TcGemmArgs::groups) every row adds up its pairs' results
 //  * moe_glu_up_rows / moe_glu_down_rows   few rows: only the chosen experts' and the shared expert's rows are read
 //  Router kind 2 (softmax scores, the largest win, weights = scores over the chosen scores' sum, applied to the expert's
 //  OUTPUT) runs the same gated experts; the shared expert's weight is the sigmoid of one more logit of the router launch.
@@ -271,6 +274,78 @@ __global__ void moe_glu_act_kernel(const float* __restrict__ gu, const float* __
   if (hid16) hid16[i] = __float2bfloat16_rn(o);
 }
 
+// One CTA: row_of[p] = place of pair p (= row * top + k) among tiles of 128 rows that each belong to one expert (-1: no weight, or no
+// such expert); groups = [number of tiles | expert of every tile].  The order of an expert's pairs changes no result.
+__global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t* __restrict__ sel, const float* __restrict__ w, int pairs, int E, int* __restrict__ row_of,
+                                                         int* __restrict__ groups) {
+  __shared__ int cnt[MOE_MAX_SLOTS], off[MOE_MAX_SLOTS];
+  pdl_launch();
+  pdl_wait();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
+  __syncthreads();
+  for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
+    const int e = sel[p];
+    if (e >= 0 && e < E && w[p] != 0.f) atomicAdd(&cnt[e], 1);
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {  // tiles ahead of every expert
+    int carry = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + threadIdx.x, n = e < E ? (cnt[e] + 127) >> 7 : 0;
+      int v = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(L3_FULL, v, o);
+        if ((int)threadIdx.x >= o) v += t;
+      }
+      if (e < E) {
+        off[e] = (carry + v - n) * 128;
+        for (int t = 0; t < n; ++t) groups[1 + carry + v - n + t] = e;
+      }
+      carry += __shfl_sync(L3_FULL, v, 31);
+    }
+    if (threadIdx.x == 0) groups[0] = carry;
+  }
+  __syncthreads();
+  for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
+    const int e = sel[p];
+    row_of[p] = e >= 0 && e < E && w[p] != 0.f ? atomicAdd(&off[e], 1) : -1;
+  }
+}
+
+// a warp per pair: its row's bf16 inputs and its weight to the pair's place
+__global__ void __launch_bounds__(256) moe_gather_kernel(const bf16* __restrict__ x16, const float* __restrict__ w, const int* __restrict__ row_of, int pairs, int top,
+                                                         int D, bf16* __restrict__ xg, float* __restrict__ wg) {
+  pdl_launch();
+  pdl_wait();
+  const int p = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (p >= pairs) return;
+  const int to = row_of[p];
+  if (to < 0) return;
+  const uint4* src = reinterpret_cast<const uint4*>(x16 + (size_t)(p / top) * D);
+  uint4* dst = reinterpret_cast<uint4*>(xg + (size_t)to * D);
+#pragma unroll 4
+  for (int i = lane; i < D / 8; i += 32) dst[i] = src[i];
+  if (lane == 0) wg[to] = w[p];
+}
+
+// y[r] (+)= sum over the row's pairs, in their order
+__global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restrict__ yg, const int* __restrict__ row_of, int top, int D, bool add, float* __restrict__ y) {
+  pdl_launch();
+  pdl_wait();
+  const size_t r = blockIdx.x;
+  for (int c = threadIdx.x * 4; c < D; c += blockDim.x * 4) {
+    float4 s = add ? *reinterpret_cast<const float4*>(y + r * D + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = 0; k < top; ++k) {
+      const int from = row_of[r * top + k];
+      if (from < 0) continue;
+      const float4 v = *reinterpret_cast<const float4*>(yg + (size_t)from * D + c);
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    *reinterpret_cast<float4*>(y + r * D + c) = s;
+  }
+}
+
 // grid (ceil(max(ff, sff) / 8), rows * (top + 1)): slot k < top of a row is its k-th chosen expert, slot top the shared expert
 template <typename WT>
 __global__ void __launch_bounds__(256) moe_glu_up_rows_kernel(const float* __restrict__ h, const WT* __restrict__ w_gu,
@@ -407,4 +482,17 @@ cudaError_t launch_moe_rows(const float* h, const void* w_up, const void* w_down
   if (e != cudaSuccess) return e;
   return launch_k(moe_down_rows_kernel<float>, gd, dim3(256), 0, s, h, (const float*)w_down, sel, w, idw, D, E, ff, top,
                   (const float*)hid, x);
+}
+
+cudaError_t launch_moe_group(const int32_t* sel, const float* w, int rows, int top, int E, int D, const bf16* x16, int* row_of, int* groups, bf16* xg, float* wg,
+                             cudaStream_t s) {
+  if (E > MOE_MAX_SLOTS || D % 8) return cudaErrorInvalidValue;
+  const int pairs = rows * top;
+  const cudaError_t e = launch_k(moe_group_kernel, dim3(1), dim3(1024), 0, s, sel, w, pairs, E, row_of, groups);
+  if (e != cudaSuccess) return e;
+  return launch_k(moe_gather_kernel, dim3((pairs + 7) / 8), dim3(256), 0, s, x16, w, (const int*)row_of, pairs, top, D, xg, wg);
+}
+
+cudaError_t launch_moe_combine(const float* yg, const int* row_of, int rows, int top, int D, bool add, float* y, cudaStream_t s) {
+  return launch_k(moe_combine_kernel, dim3(rows), dim3(D >= 1024 ? 256 : 128), 0, s, yg, row_of, top, D, add, y);
 }
