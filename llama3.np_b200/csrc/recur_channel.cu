@@ -69,16 +69,27 @@ template <int DK> struct Ws {
 };
 
 // ---------------------------------------------------------------------------------------------- 1. what a chunk needs by itself
+// One CTA per SM (104 KB of rows), bound by its own latencies: ~55000 cycles when every product took its exponentials anew from running
+// sums and values came one load at a time, of which 13500 went to the tiles between blocks, 7500 to the operands and up to 28000 to the
+// values' product.  Now what looks across a block's edge reads rows that are decayed once, in place - queries and keys from the block's
+// start, keys to its end -, and the blocks' totals enter as factors per channel.  2048 tokens, 16 heads of 128 x 128: 152 -> 86 us;
+// 3 x 701 tokens, 8 heads of 128 x 256 without the delta rule: 37 -> 26.
+template <int DK> constexpr int chunk_floats(bool delta) {
+  return 3 * CT * (DK + 8) + CT * (CT + 4) + 14 * DK + 2048 + (delta ? 2 * CT * (CT + 4) + 3 * 16 * 17 + CT : 0);
+}
+
 template <int DK, bool DELTA>
 __global__ void __launch_bounds__(512) channel_chunk_kernel(RecurArgs a, int c0) {
   extern __shared__ __align__(16) float sm[];
   constexpr int LD = DK + 8, LDA = CT + 4;
-  float* qf = sm;                       // [CT][LD]
-  float* kf = qf + CT * LD;
-  float* lf = kf + CT * LD;             // running log decay inside a block of 16 tokens, token included
+  float* qf = sm;                       // [CT][LD] queries; later decayed from the start of the block of 16 tokens
+  float* kf = qf + CT * LD;             // keys, likewise
+  float* lf = kf + CT * LD;             // running log decay inside a block, token included; later keys decayed to the end of the block
   float* Bm = lf + CT * LD;             // [CT][LDA]
   float* tot = Bm + CT * LDA;           // [4][DK] the blocks' totals
-  float* Am = tot + 4 * DK;             // [CT][LDA] diag(beta) A, strictly lower (delta rule, as what follows)
+  float* fac = tot + 4 * DK;            // [10][DK] decays over whole blocks: 0 | 0 1 | 0 1 2 | all | 1 2 3 | 2 3 | 3 | 1 | 1 2 | 2
+  float* part = fac + 10 * DK;          // [quarter of the channels][block][16][8]
+  float* Am = part + 2048;              // [CT][LDA] diag(beta) A, strictly lower (delta rule, as what follows)
   float* Tm = Am + CT * LDA;            // [CT][LDA]
   float* tmp = Tm + CT * LDA;           // [3][16][17]
   float* beta = tmp + 3 * 16 * 17;      // [CT]
@@ -88,26 +99,33 @@ __global__ void __launch_bounds__(512) channel_chunk_kernel(RecurArgs a, int c0)
   const int c = c0 + blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int n = min(CT, a.L - c * CT);
   const size_t row0 = (size_t)b * a.L + (size_t)c * CT;
+  constexpr int IT = CT * DK / 4 / 512;  // 16-byte pieces of a thread
   {
     const float* qs = a.q + row0 * a.ld_q + (size_t)(h / a.rep) * DK;
     const float* ks = a.k + row0 * a.ld_k + (size_t)(h / a.rep) * DK;
-    for (int i = tid; i < CT * DK / 4; i += 512) {
-      const int t = i / (DK / 4), d = (i % (DK / 4)) * 4;
-      float4 qv = make_float4(0.f, 0.f, 0.f, 0.f), kv = qv, lv = qv;
-      if (t < n) {
-        qv = *reinterpret_cast<const float4*>(qs + (size_t)t * a.ld_q + d);
-        kv = *reinterpret_cast<const float4*>(ks + (size_t)t * a.ld_k + d);
-        lv = *reinterpret_cast<const float4*>(a.log_c + (row0 + t) * a.H * DK + (size_t)h * DK + d);
-        // From -104 on a decay is zero in fp32.  Stronger ones are held at -110: the decays of the tokens behind them are differences
-        // of running sums, which are right to 2^-14 of a unit that way (a block's stay above -16 x 110), with one such token to 2^-18
-        lv.x = lv.x < -110.f ? -110.f : lv.x; lv.y = lv.y < -110.f ? -110.f : lv.y; lv.z = lv.z < -110.f ? -110.f : lv.z; lv.w = lv.w < -110.f ? -110.f : lv.w;
-      }
-      *reinterpret_cast<float4*>(qf + t * LD + d) = qv;
-      *reinterpret_cast<float4*>(kf + t * LD + d) = kv;
-      *reinterpret_cast<float4*>(lf + t * LD + d) = lv;
+    const float* ls = a.log_c + row0 * a.H * DK + (size_t)h * DK;
+    float4 qv[IT], kv[IT], lv[IT];
+#pragma unroll
+    for (int u = 0; u < IT; ++u) {       // all in flight; rows behind the last token read it again and count as zero
+      const int i = tid + u * 512, t = min(i / (DK / 4), n - 1), d = (i % (DK / 4)) * 4;
+      qv[u] = *reinterpret_cast<const float4*>(qs + (size_t)t * a.ld_q + d);
+      kv[u] = *reinterpret_cast<const float4*>(ks + (size_t)t * a.ld_k + d);
+      lv[u] = *reinterpret_cast<const float4*>(ls + (size_t)t * a.H * DK + d);
     }
     if (DELTA && tid < CT) beta[tid] = tid < n ? a.beta[(row0 + tid) * a.H + h] : 0.f;
     for (int i = tid; i < CT * LDA; i += 512) { Bm[i] = 0.f; if (DELTA) Am[i] = 0.f; }
+#pragma unroll
+    for (int u = 0; u < IT; ++u) {
+      const int i = tid + u * 512, t = i / (DK / 4), d = (i % (DK / 4)) * 4;
+      float4 l = lv[u];
+      // From -104 on a decay is zero in fp32.  Stronger ones are held at -110: the decays of the tokens behind them are differences
+      // of running sums, which are right to 2^-14 of a unit that way (a block's stay above -16 x 110), with one such token to 2^-18
+      l.x = l.x < -110.f ? -110.f : l.x; l.y = l.y < -110.f ? -110.f : l.y; l.z = l.z < -110.f ? -110.f : l.z; l.w = l.w < -110.f ? -110.f : l.w;
+      const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(qf + t * LD + d) = t < n ? qv[u] : z;
+      *reinterpret_cast<float4*>(kf + t * LD + d) = t < n ? kv[u] : z;
+      *reinterpret_cast<float4*>(lf + t * LD + d) = t < n ? l : z;
+    }
   }
   __syncthreads();
   for (int i = tid; i < 4 * DK; i += 512) {
@@ -118,62 +136,34 @@ __global__ void __launch_bounds__(512) channel_chunk_kernel(RecurArgs a, int c0)
     tot[i] = s;
   }
   __syncthreads();
-  // ---- A and B between blocks of 16, and between the halves of a block: one 16 x 16 (16 x 8) tile per warp
+  // ---- between the halves of a block: tokens 8 - 15 against keys 0 - 7, the reference ahead of the second half; A in the upper rows of
+  // the tile, B in the lower ones, a quarter of the channels per warp
   {
-    // warps 0 - 5: queries of block I against keys of block J < I; 6 - 11: keys likewise (delta); 12 - 15: second half of a block
-    const bool mid = warp >= 12;
-    const int pr = warp % 6;
-    const int I = mid ? warp - 12 : pr < 1 ? 1 : pr < 3 ? 2 : 3, J = mid ? I : pr < 1 ? 0 : pr < 3 ? pr - 1 : pr - 3;
-    if (mid || warp < 6 || DELTA) {
-      const float* xa = mid ? kf : warp < 6 ? qf : kf;   // rows 0 - 7 of the tile
-      const float* xb = mid ? qf : xa;                   // rows 8 - 15
-      const int ta = mid ? 16 * I + 8 + g : 16 * I + g, tb = mid ? ta : ta + 8;
-      const int j0 = 16 * J;
-      float acc[2][4] = {};
-#pragma unroll 2
-      for (int k0 = 0; k0 < DK; k0 += 16) {
-        uint32_t ah[4], al[4];
-        uint4 bb[2];
+    const int I = warp >> 2, kq = warp & 3, t = 16 * I + 8 + g, j = 16 * I + g;
+    float acc[4] = {};
 #pragma unroll
-        for (int s = 0; s < 2; ++s) {
-          const int d = k0 + q2 + 8 * s;
-          // the reference between rows and columns: the start of block I, or the token ahead of its second half
-          float2 ref = mid ? *reinterpret_cast<const float2*>(lf + (16 * I + 7) * LD + d) : make_float2(0.f, 0.f);
-          const float2 va = *reinterpret_cast<const float2*>(xa + ta * LD + d), la = *reinterpret_cast<const float2*>(lf + ta * LD + d);
-          const float2 vb = *reinterpret_cast<const float2*>(xb + tb * LD + d), lb = *reinterpret_cast<const float2*>(lf + tb * LD + d);
-          split2(va.x * __expf(la.x - ref.x), va.y * __expf(la.y - ref.y), ah[2 * s], al[2 * s]);
-          split2(vb.x * __expf(lb.x - ref.x), vb.y * __expf(lb.y - ref.y), ah[2 * s + 1], al[2 * s + 1]);
-          if (!mid) {  // decay from the end of token j to the start of block I
-            ref = make_float2(0.f, 0.f);
-            for (int m = J; m < I; ++m) { const float2 t = *reinterpret_cast<const float2*>(tot + m * DK + d); ref.x += t.x; ref.y += t.y; }
-          }
+    for (int k0 = kq * (DK / 4); k0 < (kq + 1) * (DK / 4); k0 += 16) {
+      uint32_t ah[4], al[4];
+      uint4 bb;
 #pragma unroll
-          for (int nt = 0; nt < 2; ++nt) {
-            if (mid && nt) continue;
-            const int j = j0 + nt * 8 + g;
-            const float2 kv = *reinterpret_cast<const float2*>(kf + j * LD + d), lj = *reinterpret_cast<const float2*>(lf + j * LD + d);
-            uint32_t hi, lo;
-            split2(kv.x * __expf(ref.x - lj.x), kv.y * __expf(ref.y - lj.y), hi, lo);
-            if (s) { bb[nt].y = hi; bb[nt].w = lo; } else { bb[nt].x = hi; bb[nt].z = lo; }
-          }
-        }
-        mma3(acc[0], ah, al, bb[0]);
-        if (!mid) mma3(acc[1], ah, al, bb[1]);
+      for (int s = 0; s < 2; ++s) {
+        const int d = k0 + q2 + 8 * s;
+        const float2 ref = *reinterpret_cast<const float2*>(lf + (16 * I + 7) * LD + d);
+        const float2 lt = *reinterpret_cast<const float2*>(lf + t * LD + d), lj = *reinterpret_cast<const float2*>(lf + j * LD + d);
+        const float2 kt = *reinterpret_cast<const float2*>(kf + t * LD + d), qt = *reinterpret_cast<const float2*>(qf + t * LD + d);
+        const float2 kj = *reinterpret_cast<const float2*>(kf + j * LD + d);
+        const float ex = __expf(lt.x - ref.x), ey = __expf(lt.y - ref.y);
+        split2(kt.x * ex, kt.y * ey, ah[2 * s], al[2 * s]);
+        split2(qt.x * ex, qt.y * ey, ah[2 * s + 1], al[2 * s + 1]);
+        uint32_t hi, lo;
+        split2(kj.x * __expf(ref.x - lj.x), kj.y * __expf(ref.y - lj.y), hi, lo);
+        if (s) { bb.y = hi; bb.w = lo; } else { bb.x = hi; bb.z = lo; }
       }
-      float* outa = mid || warp >= 6 ? Am : Bm;
-      float* outb = !mid && warp >= 6 ? Am : Bm;
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-        if (mid && nt) continue;
-        const int j = j0 + nt * 8 + q2;
-        if (outa == Bm || DELTA) {
-          const float f = outa == Bm ? 1.f : beta[ta];
-          *reinterpret_cast<float2*>(outa + ta * LDA + j) = make_float2(acc[nt][0] * f, acc[nt][1] * f);
-        }
-        const float f = outb == Bm ? 1.f : beta[tb];
-        *reinterpret_cast<float2*>(outb + tb * LDA + j) = make_float2(acc[nt][2] * f, acc[nt][3] * f);
-      }
+      mma3(acc, ah, al, bb);
     }
+    float* o = part + (kq * 4 + I) * 128 + g * 8 + q2;
+    *reinterpret_cast<float2*>(o) = make_float2(acc[0], acc[1]);
+    *reinterpret_cast<float2*>(o + 64) = make_float2(acc[2], acc[3]);
   }
   // ---- the 8 x 8 blocks on the diagonal, pair by pair: lane = (token, one of four keys)
   {
@@ -194,59 +184,122 @@ __global__ void __launch_bounds__(512) channel_chunk_kernel(RecurArgs a, int c0)
     if (DELTA && j < t) Am[t * LDA + j] = sa * beta[t];
   }
   __syncthreads();
-  // ---- operands of the chain kernel
+  // ---- the halves' products; rows decayed in place; decays over whole blocks
+  {
+    const int I = tid >> 7, r = (tid >> 3) & 15, j = 16 * I + (tid & 7), t = 16 * I + 8 + (r & 7);
+    float s = 0.f;
+#pragma unroll
+    for (int kq = 0; kq < 4; ++kq) s += part[(kq * 4 + I) * 128 + r * 8 + (tid & 7)];
+    if (r >= 8) Bm[t * LDA + j] = s;
+    else if (DELTA) Am[t * LDA + j] = s * beta[t];
+  }
+#pragma unroll
+  for (int u = 0; u < IT; ++u) {
+    const int i = tid + u * 512, t = i / (DK / 4), d = (i % (DK / 4)) * 4;
+    float4 q = *reinterpret_cast<float4*>(qf + t * LD + d), k = *reinterpret_cast<float4*>(kf + t * LD + d);
+    const float4 l = *reinterpret_cast<float4*>(lf + t * LD + d), e = *reinterpret_cast<float4*>(tot + (t >> 4) * DK + d);
+    *reinterpret_cast<float4*>(lf + t * LD + d) = make_float4(k.x * __expf(e.x - l.x), k.y * __expf(e.y - l.y), k.z * __expf(e.z - l.z), k.w * __expf(e.w - l.w));
+    const float ex = __expf(l.x), ey = __expf(l.y), ez = __expf(l.z), ew = __expf(l.w);
+    *reinterpret_cast<float4*>(qf + t * LD + d) = make_float4(q.x * ex, q.y * ey, q.z * ez, q.w * ew);
+    *reinterpret_cast<float4*>(kf + t * LD + d) = make_float4(k.x * ex, k.y * ey, k.z * ez, k.w * ew);
+  }
+  if (tid < DK) {
+    const float t0 = tot[tid], t1 = tot[DK + tid], t2 = tot[2 * DK + tid], t3 = tot[3 * DK + tid];
+    const float f[10] = {t0, t0 + t1, t0 + t1 + t2, t0 + t1 + t2 + t3, t1 + t2 + t3, t2 + t3, t3, t1, t1 + t2, t2};
+#pragma unroll
+    for (int m = 0; m < 10; ++m) fac[m * DK + tid] = __expf(f[m]);
+  }
+  __syncthreads();
+  // ---- A and B between blocks of 16: warps 0 - 5 queries of block I against keys of block J < I, 6 - 11 keys likewise (delta)
+  if (warp < (DELTA ? 12 : 6)) {
+    const int pr = warp % 6, I = pr < 1 ? 1 : pr < 3 ? 2 : 3, J = pr < 1 ? 0 : pr < 3 ? pr - 1 : pr - 3;
+    const float* x = warp < 6 ? qf : kf;
+    const float* f = I - J == 1 ? nullptr : fac + (J == 1 ? 9 : I == 2 ? 7 : 8) * DK;  // the blocks between them
+    const int ta = 16 * I + g;
+    float acc[2][4] = {};
+#pragma unroll 4
+    for (int k0 = 0; k0 < DK; k0 += 16) {
+      uint32_t ah[4], al[4];
+      uint4 bb[2];
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const int d = k0 + q2 + 8 * s;
+        const float2 va = *reinterpret_cast<const float2*>(x + ta * LD + d), vb = *reinterpret_cast<const float2*>(x + (ta + 8) * LD + d);
+        split2(va.x, va.y, ah[2 * s], al[2 * s]);
+        split2(vb.x, vb.y, ah[2 * s + 1], al[2 * s + 1]);
+        const float2 fd = f ? *reinterpret_cast<const float2*>(f + d) : make_float2(1.f, 1.f);
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          const float2 kv = *reinterpret_cast<const float2*>(lf + (16 * J + nt * 8 + g) * LD + d);
+          uint32_t hi, lo;
+          split2(kv.x * fd.x, kv.y * fd.y, hi, lo);
+          if (s) { bb[nt].y = hi; bb[nt].w = lo; } else { bb[nt].x = hi; bb[nt].z = lo; }
+        }
+      }
+      mma3(acc[0], ah, al, bb[0]);
+      mma3(acc[1], ah, al, bb[1]);
+    }
+    float* out = warp < 6 ? Bm : Am;
+    const float fa = warp < 6 ? 1.f : beta[ta], fb = warp < 6 ? 1.f : beta[ta + 8];
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) {
+      const int j = 16 * J + nt * 8 + q2;
+      *reinterpret_cast<float2*>(out + ta * LDA + j) = make_float2(acc[nt][0] * fa, acc[nt][1] * fa);
+      *reinterpret_cast<float2*>(out + (ta + 8) * LDA + j) = make_float2(acc[nt][2] * fb, acc[nt][3] * fb);
+    }
+  }
+  __syncthreads();
+  // ---- operands of the chain kernel; with the delta rule two warps invert the diagonal blocks of T = (I + Am)^-1 meanwhile, a column
+  // per thread
   using Wk = Ws<DK>;
   uint4* ws = reinterpret_cast<uint4*>(a.ws) + ((size_t)(b * a.H + h) * gridDim.x + blockIdx.x) * Wk::total(a.DV, DELTA);
-  auto before = [&](int blk, int d) { float s = 0.f; for (int m = 0; m < blk; ++m) s += tot[m * DK + d]; return s; };
-  for (int i = tid; i < Wk::Q; i += 512) {               // decayed queries: (token, channel pair)
-    const int l = i & 31, ks = (i >> 5) % (DK / 16), nt = (i >> 5) / (DK / 16), t = nt * 8 + (l >> 2), d = ks * 16 + (l & 3) * 2, blk = t >> 4;
-    uint4 o;
+  constexpr int T0 = DELTA ? CT : 0, TN = 512 - T0;
+  if (tid < T0) {
+    const int blk = tid >> 4, cc = tid & 15;
+    const float* Ld = Am + (blk * 16) * LDA + blk * 16;
+    float x[16];
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const int e = d + 8 * s;
-      const float x = qf[t * LD + e] * __expf(lf[t * LD + e] + before(blk, e));
-      const float y = qf[t * LD + e + 1] * __expf(lf[t * LD + e + 1] + before(blk, e + 1));
-      if (s) split2(x, y, o.y, o.w); else split2(x, y, o.x, o.z);
+    for (int r = 0; r < 16; ++r) {
+      float s = 0.f;
+#pragma unroll
+      for (int m = 0; m < r; ++m) s = fmaf(Ld[r * LDA + m], x[m], s);
+      x[r] = r == cc ? 1.f : r < cc ? 0.f : -s;
+      Tm[(blk * 16 + r) * LDA + blk * 16 + cc] = x[r];
     }
-    ws[Wk::oQ + i] = o;
-  }
-  for (int i = tid; i < Wk::K; i += 512) {               // decayed keys: (channel, token pair)
-    const int l = i & 31, ks = (i >> 5) & 3, nt = i >> 7, d = nt * 8 + (l >> 2), t = ks * 16 + (l & 3) * 2;
-    float rest = tot[ks * DK + d];                       // from the start of the block to the end of the chunk
-    for (int m = ks + 1; m < 4; ++m) rest += tot[m * DK + d];
-    uint4 o;
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const int u = t + 8 * s;
-      const float x = kf[u * LD + d] * __expf(rest - lf[u * LD + d]), y = kf[(u + 1) * LD + d] * __expf(rest - lf[(u + 1) * LD + d]);
-      if (s) split2(x, y, o.y, o.w); else split2(x, y, o.x, o.z);
-    }
-    ws[Wk::oK + i] = o;
-  }
-  for (int i = tid; i < Wk::B; i += 512) {
-    const int l = i & 31, ks = (i >> 5) & 3, nt = i >> 7;
-    const float* p = Bm + (nt * 8 + (l >> 2)) * LDA + ks * 16 + (l & 3) * 2;
-    uint4 o;
-    split2(p[0], p[1], o.x, o.z);
-    split2(p[8], p[9], o.y, o.w);
-    ws[Wk::oB + i] = o;
-  }
-  for (int d = tid; d < DK; d += 512) reinterpret_cast<float*>(ws + Wk::oE)[d] = __expf(before(4, d));
-  if constexpr (DELTA) {
-    // ---- T = (I + Am)^-1, blocks of 16: the diagonal ones column by column, then by distance from the diagonal
-    if (tid < CT) {
-      const int blk = tid >> 4, cc = tid & 15;
-      const float* Ld = Am + (blk * 16) * LDA + blk * 16;
-      float x[16];
-#pragma unroll
-      for (int r = 0; r < 16; ++r) {
-        float s = 0.f;
-#pragma unroll
-        for (int m = 0; m < r; ++m) s = fmaf(Ld[r * LDA + m], x[m], s);
-        x[r] = r == cc ? 1.f : r < cc ? 0.f : -s;
-        Tm[(blk * 16 + r) * LDA + blk * 16 + cc] = x[r];
+  } else {
+    for (int i = tid - T0; i < Wk::Q; i += TN) {         // decayed queries: (token, channel pair)
+      const int l = i & 31, ks = (i >> 5) % (DK / 16), nt = (i >> 5) / (DK / 16), t = nt * 8 + (l >> 2), d = ks * 16 + (l & 3) * 2, blk = t >> 4;
+      float2 x = *reinterpret_cast<const float2*>(qf + t * LD + d), y = *reinterpret_cast<const float2*>(qf + t * LD + d + 8);
+      if (blk) {
+        const float2 f = *reinterpret_cast<const float2*>(fac + (blk - 1) * DK + d), f8 = *reinterpret_cast<const float2*>(fac + (blk - 1) * DK + d + 8);
+        x.x *= f.x; x.y *= f.y; y.x *= f8.x; y.y *= f8.y;
       }
+      uint4 o;
+      split2(x.x, x.y, o.x, o.z);
+      split2(y.x, y.y, o.y, o.w);
+      ws[Wk::oQ + i] = o;
     }
+    for (int i = tid - T0; i < Wk::K; i += TN) {         // decayed keys: (channel, token pair)
+      const int l = i & 31, ks = (i >> 5) & 3, nt = i >> 7, d = nt * 8 + (l >> 2), t = ks * 16 + (l & 3) * 2;
+      const float f = ks < 3 ? fac[(4 + ks) * DK + d] : 1.f;  // from the end of the block to the end of the chunk
+      const float* p = lf + t * LD + d;
+      uint4 o;
+      split2(p[0] * f, p[LD] * f, o.x, o.z);
+      split2(p[8 * LD] * f, p[9 * LD] * f, o.y, o.w);
+      ws[Wk::oK + i] = o;
+    }
+    for (int i = tid - T0; i < Wk::B; i += TN) {
+      const int l = i & 31, ks = (i >> 5) & 3, nt = i >> 7;
+      const float* p = Bm + (nt * 8 + (l >> 2)) * LDA + ks * 16 + (l & 3) * 2;
+      uint4 o;
+      split2(p[0], p[1], o.x, o.z);
+      split2(p[8], p[9], o.y, o.w);
+      ws[Wk::oB + i] = o;
+    }
+    for (int d = tid - T0; d < DK; d += TN) reinterpret_cast<float*>(ws + Wk::oE)[d] = fac[3 * DK + d];
+  }
+  if constexpr (DELTA) {
+    // ---- T by distance from the diagonal
     __syncthreads();
 #pragma unroll 1
     for (int dist = 1; dist < 4; ++dist) {
@@ -254,7 +307,9 @@ __global__ void __launch_bounds__(512) channel_chunk_kernel(RecurArgs a, int c0)
       for (int i = tid; i < items; i += 512) {           // sum_m L_Im T_mJ
         const int J = i >> 8, I = J + dist, r = (i >> 4) & 15, cc = i & 15;
         float s = 0.f;
-        for (int m = J * 16; m < I * 16; ++m) s = fmaf(Am[(I * 16 + r) * LDA + m], Tm[m * LDA + J * 16 + cc], s);
+        for (int m0 = J * 16; m0 < I * 16; m0 += 16)
+#pragma unroll
+          for (int m = m0; m < m0 + 16; ++m) s = fmaf(Am[(I * 16 + r) * LDA + m], Tm[m * LDA + J * 16 + cc], s);
         tmp[J * 272 + r * 17 + cc] = s;
       }
       __syncthreads();
@@ -273,22 +328,32 @@ __global__ void __launch_bounds__(512) channel_chunk_kernel(RecurArgs a, int c0)
     for (int ct = warp; ct < n_all; ct += 16) {
       const bool is_w = ct < n_w;
       const int col0 = is_w ? ct * 16 : (ct - n_w) * 16;
+      float v[4][2][4];                                  // all loads in flight
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          const int col = col0 + nt * 8 + g;
+          const float f = is_w && ks ? fac[(ks - 1) * DK + col] : 1.f;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int t = ks * 16 + q2 + (u & 1) + (u >> 1) * 8;
+            v[ks][nt][u] = is_w ? kf[t * LD + col] * f : a.v[(row0 + min(t, n - 1)) * a.ld_v + (size_t)h * a.DV + col];
+          }
+        }
       float acc[4][2][4] = {};
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
         uint4 bb[2];
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
-          const int col = col0 + nt * 8 + g;
-          float v[4];
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             const int t = ks * 16 + q2 + (u & 1) + (u >> 1) * 8;
-            if (is_w) v[u] = beta[t] * kf[t * LD + col] * __expf(lf[t * LD + col] + before(ks, col));
-            else v[u] = t < n ? beta[t] * a.v[(row0 + t) * a.ld_v + (size_t)h * a.DV + col] : 0.f;
+            v[ks][nt][u] = t < n ? beta[t] * v[ks][nt][u] : 0.f;
           }
-          split2(v[0], v[1], bb[nt].x, bb[nt].z);
-          split2(v[2], v[3], bb[nt].y, bb[nt].w);
+          split2(v[ks][nt][0], v[ks][nt][1], bb[nt].x, bb[nt].z);
+          split2(v[ks][nt][2], v[ks][nt][3], bb[nt].y, bb[nt].w);
         }
 #pragma unroll
         for (int mt = ks; mt < 4; ++mt) {
@@ -463,7 +528,7 @@ template <int DK> size_t per_chunk(int DV, bool delta) { return Ws<DK>::total(DV
 template <int DK, bool DELTA>
 cudaError_t launch_channel_t(const RecurArgs& a, cudaStream_t s) {
   using Wk = Ws<DK>;
-  const size_t sm1 = (size_t)(3 * CT * (DK + 8) + CT * (CT + 4) + 4 * DK + (DELTA ? 2 * CT * (CT + 4) + 3 * 16 * 17 + CT : 0)) * sizeof(float);
+  const size_t sm1 = (size_t)chunk_floats<DK>(DELTA) * sizeof(float);
   const size_t sm2 = (size_t)((DELTA ? Wk::W : 0) + Wk::Q + Wk::K + Wk::B + (DELTA ? 2 : 1) * (DK / 16) * 256 + 256) * 16;
   cudaError_t e;
   if ((e = cudaFuncSetAttribute(channel_chunk_kernel<DK, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1)) != cudaSuccess) return e;
@@ -487,9 +552,10 @@ size_t recur_channel_ws_floats(int B, int L, int H, int DK, int DV) {
   return (size_t)B * H * ((L + CT - 1) / CT) * per;
 }
 
-// Portions from this length on.  A chunk's CTA takes ~20 us (gated linear attention: 264 of them in 37 us) to ~39 us (delta rule, with the
-// triangular system: 512 in 155 us, one per SM at a time) whatever it holds; the chain takes 0.2 - 0.3 us per token, and more where its
-// CTAs (a multiple of sequences x heads) fill the chip.  One layer, prompt through the public call, chain against chunks in us: delta rule, 1 x 16 heads, 48 tokens 240 : 256, 96
+// Portions from this length on.  A chunk's CTA takes ~13 us (gated linear attention: 264 of them in 26 us) to ~21 us (delta rule, with the
+// triangular system: 512 in 86 us, one per SM at a time) whatever it holds; the chain takes 0.2 - 0.3 us per token, and more where its
+// CTAs (a multiple of sequences x heads) fill the chip.  One layer, prompt through the public call, chain against chunks (when a CTA took
+// 20 and 39 us) in us: delta rule, 1 x 16 heads, 48 tokens 240 : 256, 96
 // 272 : 284, 128 306 : 308, 192 267 : 253, 400 347 : 284; 4 x 16 heads, 48 255 : 265, 64 278 : 269, 128 341 : 294.  Gated linear
 // attention, 1 x 2 heads, 48 tokens 152 : 158, 72 177 : 176, 96 188 : 180; 1 x 8 heads, 48 218 : 217, 64 228 : 220, 128 285 : 253.
 static int least_tokens(const RecurArgs& a) {

@@ -422,8 +422,8 @@ cudaError_t launch_recur(const RecurArgs& a, cudaStream_t s) {
   if ((a.n_state || a.k_scale) && (a.mode != 2 || !a.k_scale || !a.nq)) return cudaErrorInvalidValue;
   // Prompts in bf16 mode with decays per key channel: the chains below are bound by their latency - ~0.31 us per token for the delta
   // rule, 0.2 - 0.6 us for gated linear attention, however many CTAs run -, the chunk-parallel form does one step per 64 tokens.  16
-  // heads of 128 x 128, 2048 tokens, delta rule: 632 -> 154 + 84 us; 8 heads of 128 x 256, 3 x 701 tokens, gated linear attention:
-  // 425 -> 37 + 66 us.  From which length on: recur_channel.cu.
+  // heads of 128 x 128, 2048 tokens, delta rule: 632 -> 86 + 84 us; 8 heads of 128 x 256, 3 x 701 tokens, gated linear attention:
+  // 425 -> 26 + 66 us.  From which length on: recur_channel.cu.
   if (recur_channel_supported(a)) return launch_recur_channel(a, s);
   if (a.log_c) return cudaErrorInvalidValue;  // the other kernels read the decays themselves
   static const bool chunk_on = !(getenv("L3_RECUR_CHUNK") && atoi(getenv("L3_RECUR_CHUNK")) == 0);
