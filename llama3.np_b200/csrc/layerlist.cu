@@ -1233,7 +1233,7 @@ int ll_finalize(L3Model* m) {
     for (const LLLayer* U = &L0; U; U = U->pair) {
       const L3LayerSpec& s = U->spec;
       const bool chunked = s.mixer == L3_MIX_DECAY_LINEAR || (units && (s.mixer == L3_MIX_SSD || s.mixer == L3_MIX_MLSTM));
-      if (chunked && recur_chunk_shape(s.dim, s.vdim) && ct >= 128)
+      if (chunked && recur_chunk_shape(s.dim, s.vdim) && ct >= RECUR_CHUNK_MIN)
         ll->chunk_ws_floats = std::max(ll->chunk_ws_floats, (ct / 64 + m->maxB) * ((size_t)s.heads * s.dim * s.vdim + s.heads + (s.mixer == L3_MIX_MLSTM ? s.heads * s.dim : 0)) + 8);
     }
   if (ll->chunk_ws_floats) CK(m, cudaMalloc((void**)&ll->chunk_ws, ll->chunk_ws_floats * 4));

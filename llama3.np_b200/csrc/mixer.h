@@ -104,6 +104,7 @@ struct RecurArgs {
 bool recur_supported(int DK, int DV);
 cudaError_t launch_recur(const RecurArgs& a, cudaStream_t s);
 // chunk-parallel form of mode 0 (recur_chunk.cu): floats of workspace a call needs, whether a call can take it, the launch
+constexpr int RECUR_CHUNK_MIN = 48;  // tokens of the shortest portion that can run there (recur_chunk_supported: the rule)
 size_t recur_chunk_ws_floats(int B, int L, int H, int DK, int DV);
 bool recur_chunk_shape(int DK, int DV);
 bool recur_chunk_supported(const RecurArgs& a);

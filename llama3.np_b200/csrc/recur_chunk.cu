@@ -364,6 +364,10 @@ struct Block {
 #pragma unroll
     for (int u = 0; u < N; ++u) v[u] = make_float4(act_silu(act_in, v[u].x), act_silu(act_in, v[u].y), act_silu(act_in, v[u].z), act_silu(act_in, v[u].w));
   }
+  __device__ __forceinline__ void mul(float f) {
+#pragma unroll
+    for (int u = 0; u < N; ++u) v[u] = make_float4(v[u].x * f, v[u].y * f, v[u].z * f, v[u].w * f);
+  }
   __device__ __forceinline__ void put(bf16* dst, int ld_dst, float mul) const {
 #pragma unroll
     for (int u = 0; u < N; ++u) {
@@ -386,26 +390,27 @@ struct Block {
 };
 
 // Which recurrence: the mLSTM (normaliser, keys' scales, decays' sums in double precision), a decay per token, a fixed decay
-enum ChunkKind { CK_MLSTM, CK_TOKEN, CK_FIXED };
+enum ChunkKind { CK_MLSTM, CK_MLSTM_PAIR, CK_TOKEN, CK_FIXED };
+constexpr bool ck_norm(int kind) { return kind <= CK_MLSTM_PAIR; }  // with a normaliser, running sums in double precision
 // the decays inside a chunk: pw = running sums of the logarithms, or powers of the fixed decay
 template <int KIND>
 struct ChunkDecay {
   const double* pd;
   const float* pw;
   __device__ __forceinline__ float between(int j, int i) const {  // tokens j + 1 .. i
-    if constexpr (KIND == CK_MLSTM) return expf((float)(pd[i] - pd[j]));
+    if constexpr (ck_norm(KIND)) return expf((float)(pd[i] - pd[j]));
     else if constexpr (KIND == CK_TOKEN) return expf(pw[i] - pw[j]);
     else return pw[i - j];
   }
   __device__ __forceinline__ float upto(int i) const {  // tokens 0 .. i
-    if constexpr (KIND == CK_MLSTM) return expf((float)pd[i]);
+    if constexpr (ck_norm(KIND)) return expf((float)pd[i]);
     else if constexpr (KIND == CK_TOKEN) return expf(pw[i]);
     else return pw[i + 1];
   }
 };
 template <int KIND>
 __device__ __forceinline__ ChunkDecay<KIND> chunk_decay(const RecurArgs& a, size_t row0, int h, int n, double* pd, float* pw) {
-  if constexpr (KIND == CK_MLSTM) fill_cumlog(pd, a.log_g + row0 * a.H + h, a.H, n);
+  if constexpr (ck_norm(KIND)) fill_cumlog(pd, a.log_g + row0 * a.H + h, a.H, n);
   else if constexpr (KIND == CK_TOKEN) fill_cumlog(pw, a.log_g + row0 * a.H + h, a.H, n);
   else fill_powers(pw, a.head_decay[h]);
   return {pd, pw};
@@ -420,11 +425,11 @@ constexpr size_t out_mma_smem(int DK, bool pair) {
 template <int DK, int KIND>
 __global__ void __launch_bounds__(256) lin_chunk_state_mma_kernel(RecurArgs a, int NC, int NE) {
   extern __shared__ __align__(16) uint8_t smb[];
-  __shared__ double pd[KIND == CK_MLSTM ? CH : 1];
+  __shared__ double pd[ck_norm(KIND) ? CH : 1];
   __shared__ float pw[CH + 1];
   __shared__ float sc[CH];
   constexpr int LDK = DK + 8;
-  constexpr bool PAIR = KIND != CK_MLSTM;
+  constexpr bool PAIR = KIND != CK_MLSTM, NRM = ck_norm(KIND);
   bf16* Kh = reinterpret_cast<bf16*>(smb);           // [CH][LDK] decayed keys, hi and lo
   bf16* Kl = Kh + (size_t)CH * LDK;
   bf16* Vs = Kl + (size_t)CH * LDK;                  // [CH][LDE] (pairs: and what it leaves)
@@ -444,7 +449,7 @@ __global__ void __launch_bounds__(256) lin_chunk_state_mma_kernel(RecurArgs a, i
   const ChunkDecay<KIND> dec = chunk_decay<KIND>(a, row0, h, n, pd, pw);
   if (PAIR) kb.act(a.act_in);
   __syncthreads();
-  for (int j = tid; j < CH; j += 256) sc[j] = j < n ? dec.between(j, n - 1) * (PAIR ? 1.f : a.k_scale[(row0 + j) * a.H + h]) : 0.f;
+  for (int j = tid; j < CH; j += 256) sc[j] = j < n ? dec.between(j, n - 1) * (!NRM ? 1.f : a.k_scale[(row0 + j) * a.H + h]) : 0.f;
   if (KIND != CK_FIXED && ne == 0 && tid == 0) chunk_decays(a, NC)[((size_t)b * a.H + h) * NC + c] = dec.upto(n - 1);
   __syncthreads();
   kb.put_split(Kh, Kl, LDK, sc);
@@ -455,7 +460,7 @@ __global__ void __launch_bounds__(256) lin_chunk_state_mma_kernel(RecurArgs a, i
     else vb.put(Vs, LDE, 1.f);
     __syncthreads();
     if (e0 + 64 < e_hi) vb.fetch(vsrc + e0 + 64, a.ld_v, n);  // in flight during the products
-    if (!PAIR && ne == 0 && e0 == 0)
+    if (NRM && ne == 0 && e0 == 0)
       for (int d = tid; d < DK; d += 256) {
         float t = 0.f;
 #pragma unroll 8
@@ -501,11 +506,11 @@ __global__ void __launch_bounds__(256) lin_chunk_state_mma_kernel(RecurArgs a, i
 template <int DK, int KIND>
 __global__ void __launch_bounds__(256) lin_chunk_out_mma_kernel(RecurArgs a, int NC, int NE) {
   extern __shared__ __align__(16) uint8_t smb[];
-  __shared__ double pd[KIND == CK_MLSTM ? CH : 1];
+  __shared__ double pd[ck_norm(KIND) ? CH : 1];
   __shared__ float pw[CH + 1];
   __shared__ float ks[CH], s_nq[2][CH];
   constexpr int LDK = DK + 8;
-  constexpr bool PAIR = KIND != CK_MLSTM;
+  constexpr bool PAIR = KIND != CK_MLSTM, NRM = ck_norm(KIND);
   bf16* Qs = reinterpret_cast<bf16*>(smb);           // [CH][LDK]
   bf16* Ql = Qs + (PAIR ? (size_t)CH * LDK : 0);     // pairs: what Q, K and V leave
   bf16* Ah = Ql + (size_t)CH * LDK;                  // [CH][LDE] decayed scores, hi and lo
@@ -523,7 +528,7 @@ __global__ void __launch_bounds__(256) lin_chunk_out_mma_kernel(RecurArgs a, int
   const int n = min(CH, a.L - c * CH);
   const size_t row0 = (size_t)b * a.L + (size_t)c * CH;
   const ChunkDecay<KIND> dec = chunk_decay<KIND>(a, row0, h, n, pd, pw);
-  if (!PAIR && tid >= 32 && tid < 32 + CH) ks[tid - 32] = tid - 32 < n ? a.k_scale[(row0 + tid - 32) * a.H + h] : 0.f;
+  if (NRM && tid >= 32 && tid < 32 + CH) ks[tid - 32] = tid - 32 < n ? a.k_scale[(row0 + tid - 32) * a.H + h] : 0.f;
   {
     Block<CH, DK> qb, kb;
     qb.fetch(a.q + row0 * a.ld_q + (size_t)(h / a.rep) * DK, a.ld_q, n);
@@ -531,6 +536,7 @@ __global__ void __launch_bounds__(256) lin_chunk_out_mma_kernel(RecurArgs a, int
     if constexpr (PAIR) {
       qb.act(a.act_in);
       kb.act(a.act_in);
+      if (NRM) qb.mul(a.q_mul);
       qb.put_split(Qs, Ql, LDK, nullptr);
       kb.put_split(Ks, Kl, LDK, nullptr);
     } else {
@@ -578,14 +584,14 @@ __global__ void __launch_bounds__(256) lin_chunk_out_mma_kernel(RecurArgs a, int
 #pragma unroll
       for (int u = 0; u < 2; ++u) {                  // rows r0, r0 + 8
         const int i = r0 + u * 8, j = wn * 32 + t * 8 + (lane & 3) * 2;
-        const float x = j <= i ? acc[t][2 * u] * (PAIR ? dec.between(j, i) : dec.between(j, i) * ks[j]) : 0.f;
-        const float y = j + 1 <= i ? acc[t][2 * u + 1] * (PAIR ? dec.between(j + 1, i) : dec.between(j + 1, i) * ks[j + 1]) : 0.f;
+        const float x = j <= i ? acc[t][2 * u] * (!NRM ? dec.between(j, i) : dec.between(j, i) * ks[j]) : 0.f;
+        const float y = j + 1 <= i ? acc[t][2 * u + 1] * (!NRM ? dec.between(j + 1, i) : dec.between(j + 1, i) * ks[j + 1]) : 0.f;
         sum[u] += x + y;
         const __nv_bfloat162 hi = __floats2bfloat162_rn(x, y);
         *reinterpret_cast<__nv_bfloat162*>(Ah + (size_t)i * LDE + j) = hi;
         *reinterpret_cast<__nv_bfloat162*>(Al + (size_t)i * LDE + j) = __floats2bfloat162_rn(x - __low2float(hi), y - __high2float(hi));
       }
-    if constexpr (!PAIR) {
+    if constexpr (NRM) {
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         sum[u] += __shfl_xor_sync(L3_FULL, sum[u], 1);
@@ -595,13 +601,17 @@ __global__ void __launch_bounds__(256) lin_chunk_out_mma_kernel(RecurArgs a, int
     }
   }
   __syncthreads();
-  if (!PAIR && ne == 0) {  // n . q of every token: four threads per row
+  if (NRM && ne == 0) {  // n . q of every token: four threads per row
     const float* Pn = chunk_norms(a, NC) + (((size_t)b * a.H + h) * NC + c) * DK;
     const int i = tid >> 2, part = tid & 3;
     float t = 0.f;
 #pragma unroll 4
     for (int d = part * 2; d < DK; d += 8) {
-      const float2 q = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(Qs + (size_t)i * LDK + d));
+      float2 q = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(Qs + (size_t)i * LDK + d));
+      if (PAIR) {
+        const float2 ql = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(Ql + (size_t)i * LDK + d));
+        q.x += ql.x; q.y += ql.y;
+      }
       t = fmaf(q.x, Pn[d], t);
       t = fmaf(q.y, Pn[d + 1], t);
     }
@@ -689,9 +699,18 @@ size_t recur_chunk_ws_floats(int B, int L, int H, int DK, int DV) {
 
 bool recur_chunk_shape(int DK, int DV) { return DK % 64 == 0 && DK <= 256 && DV % 64 == 0 && DV >= 64 && DV <= 512; }
 
+// Portions from this length on: the chain of recurrent.cu takes 0.3 us per token and more where its CTAs fill the chip, the three launches
+// here take what they take from the first token on.  The mLSTM's chain is the longest (its columns carry the normaliser along) and
+// wins first; one layer of width 2048, prompt through the public call, chain : chunks in us: 1 sequence, 32 tokens 204 : 204, 48 219 : 217,
+// 64 231 : 219, 96 257 : 231; 8 sequences, 48 tokens 629 : 556, 96 702 : 595.  A state-space layer, 64 tokens 244 : 243, 96 265 : 253 (width
+// 1024, 8 sequences: 531 : 543), a fixed decay, 64 tokens 210 : 220, 96 228 : 235, 127 250 : 246: those keep the line of fp32 mode.  (With
+// queries, keys and values rounded to bf16, as from 128 tokens on; as pairs, which these portions take, 8 sequences of 96 tokens are 20 us
+// slower, and the logits of prompts of 50 - 90 tokens are as far from 64-bit ones as the chain's, where rounding made that 1.11 times.)
+static int least_tokens(const RecurArgs& a) { return a.bf16_ops && a.n_state ? RECUR_CHUNK_MIN : 2 * CH; }
+
 bool recur_chunk_supported(const RecurArgs& a) {
   const bool per_token = a.mode == 2 && a.g_head && a.log_g;  // one decay per head and token
-  if ((a.mode != 0 && !per_token) || !a.ws || a.L < 2 * CH) return false;
+  if ((a.mode != 0 && !per_token) || !a.ws || a.L < least_tokens(a)) return false;
   if (!recur_chunk_shape(a.DK, a.DV)) return false;
   if (a.ld_q % 4 || a.ld_k % 4 || a.ld_v % 4 || (a.H * a.DV) % 4) return false;
   if (!aligned16(a.q) || !aligned16(a.k) || !aligned16(a.v) || !aligned16(a.out) || !aligned16(a.ws) || !aligned16(a.state)) return false;
@@ -716,8 +735,9 @@ cudaError_t launch_recur_chunk(const RecurArgs& a, cudaStream_t s) {
   if (a.bf16_ops) {
     const int ctas = NC * a.H * a.B, tiles = a.DV / 64;
     const int ne = value_splits(ctas, tiles, 100);  // measured: only short prompts of few heads gain
+    const bool pair = !a.n_state || a.L < 2 * CH;  // shorter portions of an mLSTM: as exact as the fp32 chain that they leave
     auto go_mma = [&](auto k_state, auto k_scan, auto k_out) {
-      const size_t sb1 = state_mma_smem(a.DK, !a.n_state), sb3 = out_mma_smem(a.DK, !a.n_state);
+      const size_t sb1 = state_mma_smem(a.DK, pair), sb3 = out_mma_smem(a.DK, pair);
       cudaError_t e;
       if ((e = cudaFuncSetAttribute(k_state, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb1)) != cudaSuccess) return e;
       if ((e = cudaFuncSetAttribute(k_out, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb3)) != cudaSuccess) return e;
@@ -727,6 +747,7 @@ cudaError_t launch_recur_chunk(const RecurArgs& a, cudaStream_t s) {
     };
     auto go_kind = [&](auto dk) {
       constexpr int DK = decltype(dk)::value;
+      if (a.n_state && pair) return go_mma(lin_chunk_state_mma_kernel<DK, CK_MLSTM_PAIR>, lin_chunk_scan_kernel<true, true>, lin_chunk_out_mma_kernel<DK, CK_MLSTM_PAIR>);
       if (a.n_state) return go_mma(lin_chunk_state_mma_kernel<DK, CK_MLSTM>, lin_chunk_scan_kernel<true, true>, lin_chunk_out_mma_kernel<DK, CK_MLSTM>);
       if (a.mode == 2) return go_mma(lin_chunk_state_mma_kernel<DK, CK_TOKEN>, lin_chunk_scan_kernel<true, false>, lin_chunk_out_mma_kernel<DK, CK_TOKEN>);
       return go_mma(lin_chunk_state_mma_kernel<DK, CK_FIXED>, lin_chunk_scan_kernel<false, false>, lin_chunk_out_mma_kernel<DK, CK_FIXED>);
