@@ -12,9 +12,10 @@
 // One 128 x 128 tile per CTA and turn, persistent; 320 threads:
 //   warp 0: TMA   warp 1: TMEM + MMA issue   warps 2 - 9: conversion, running sums, epilogue
 // A step is 32 values of K.  The parts' tiles hold 64 (128-byte swizzled rows); their halves are two buffers of a ring, so that a
-// step is converted while the previous one is multiplied.  Bound by the MMAs: an M = 128 instruction takes ~132 cycles for N = 128 as
-// for N = 256 (mma_probe.cu), 12 of them per step against ~600 issue slots of conversion per scheduler (the tensor pipe then counts 22 - 28 % of the cycles at 600
-// rows, tiles' ends included); a 256-wide tile would halve that but its parts and raw tiles do not fit the shared memory together.
+// step is converted while the previous one is multiplied.  The products are not the bound: 12 of 64 cycles per
+// step (mma_probe.cu; the tensor pipe counts 22 - 28 % of the cycles at 600 rows, tiles' ends included), against ~600 issue slots of
+// conversion per scheduler and shared memory, whose bandwidth raw tiles, parts and the products' reads share; a 256-wide tile would
+// read less but its parts and raw tiles do not fit together.
 // An infinite operand leaves NaN behind (its parts are inf, NaN, NaN; inf times a zero part is NaN too): sums that end as NaN are
 // taken again as a plain chain of fp32 products, so that an infinity gives what it gives there.
 // Every wait is bounded: one that runs out sets a flag, all warps run on without waiting, and the host reports an error.
