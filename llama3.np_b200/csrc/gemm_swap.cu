@@ -516,10 +516,12 @@ cudaError_t launch_sw_e(const TcGemmArgs& a, cudaStream_t s) {
 
 bool gemm_swap_supported(int rows, int N) { return rows >= 1 && rows <= 128 && N >= 128; }
 
-// bf16 mode's residual epilogue may add its slices in place, in any order (fp32 mode must not reorder a sum)
-static bool adds_in_place(const TcGemmArgs& a) {
+// bf16 mode's residual epilogue may add its slices in place, in any order (fp32 mode must not reorder a sum).  Results then differ from
+// run to run in their last bits, so that is kept to products that are long (at least 16 k-blocks; shorter ones take less than 8000
+// cycles whole) and leave more than half of the SMs without a row block; the others are summed in slice order, or not cut.
+static bool adds_in_place(const TcGemmArgs& a, int sms) {
   static const int resid_atomic = [] { const char* v = getenv("L3_SWAP_RESID_ATOMIC"); return v ? atoi(v) : 1; }();
-  return a.epi == EPI_RESID && a.kind == TC_BF16 && a.e.out == a.e.resid && resid_atomic;
+  return a.epi == EPI_RESID && a.kind == TC_BF16 && a.e.out == a.e.resid && resid_atomic && (a.K + 63) / 64 >= 16 && (a.N + 127) / 128 * 2 <= sms;
 }
 // Tile height and K split, by the cycles of the busiest CTA: a k-block takes the issue loops ~500 cycles, or its share of DRAM
 // (3560 bytes per cycle for all CTAs that stream); slices that are added in place cost little, published and summed ones ~2.5 us and more
@@ -529,7 +531,7 @@ static bool adds_in_place(const TcGemmArgs& a) {
 static void pick_swap(const TcGemmArgs& a, int bna, int sms, int* h_out, int* ks_out) {
   static const int max_split = [] { const char* v = getenv("L3_SWAP_KSPLIT"); return v ? atoi(v) : 8; }();
   static const int det_epi = [] { const char* v = getenv("L3_SWAP_KSPLIT_DET"); return v ? atoi(v) : 1; }();
-  const bool b16 = a.kind == TC_BF16, atomic = adds_in_place(a);
+  const bool b16 = a.kind == TC_BF16, atomic = adds_in_place(a, sms);
   const int parts = b16 ? 1 : 2, nkb = (a.K + (b16 ? 63 : 31)) / (b16 ? 64 : 32);
   const int rounds = ((a.N + 127) / 128 + sms - 1) / sms;
   int h = 128;
@@ -551,11 +553,21 @@ static void pick_swap(const TcGemmArgs& a, int bna, int sms, int* h_out, int* ks
   *h_out = h;
 }
 
+static int batch_cols(int rows) { return rows <= 16 ? 16 : rows <= 32 ? 32 : rows <= 64 ? 64 : 128; }
+TcPlan gemm_swap_plan(const TcGemmArgs& a) {
+  const int sms = sm_count();
+  TcPlan p{1, 128, 1, 0};
+  pick_swap(a, batch_cols(a.rows), sms, &p.width, &p.slices);
+  p.any_order = p.slices > 1 && adds_in_place(a, sms);
+  return p;
+}
+
 cudaError_t launch_gemm_swap(const TcGemmArgs& args, cudaStream_t s) {
   TcGemmArgs a = args;
-  const int bna = a.rows <= 16 ? 16 : a.rows <= 32 ? 32 : (a.rows <= 64 ? 64 : 128);
-  pick_swap(a, bna, sm_count(), &a.bn, &a.ksplit);
-  if (adds_in_place(a)) a.part = nullptr;
+  const int bna = batch_cols(a.rows);
+  const TcPlan p = gemm_swap_plan(a);
+  a.bn = p.width; a.ksplit = p.slices;
+  if (p.any_order) a.part = nullptr;
   // Measured and rejected at the 8B shape, batch 32 (profiles/swap_gemm_experiments.txt): a tile-contiguous copy of the weights read
   // with one 16 KB bulk copy per stage (not DRAM page locality), and the slices of a row block sharing its reduction + epilogue by rows
   // behind a cooperative launch (QKV 37 vs 29 us).  Later: tiles that start their turn over K one block apart (the activation boxes are

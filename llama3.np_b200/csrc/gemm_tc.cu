@@ -250,12 +250,18 @@ static cudaError_t launch_tc_e(const TcGemmArgs& a, cudaStream_t s) {
   }
 }
 
+TcPlan gemm_tc_plan(const TcGemmArgs& a) {
+  TcPlan p{1, 32, 1, 0};
+  pick_bf16(a, sm_count(), &p.ctas, &p.width, &p.slices);
+  return p;
+}
+
 cudaError_t launch_gemm_tc(const TcGemmArgs& args, cudaStream_t s) {
   TcGemmArgs a = args;
   if (a.kind == TC_BF16) {
-    int cg = 1;
-    pick_bf16(a, sm_count(), &cg, &a.bn, &a.ksplit);
-    return cg == 2 ? launch_tc_e<TC_BF16, 0, 2>(a, s) : launch_tc_e<TC_BF16, 0, 1>(a, s);
+    const TcPlan p = gemm_tc_plan(a);
+    a.bn = p.width; a.ksplit = p.slices;
+    return p.ctas == 2 ? launch_tc_e<TC_BF16, 0, 2>(a, s) : launch_tc_e<TC_BF16, 0, 1>(a, s);
   }
   const int bn = pick_tf32(a.kind, a.rows, a.N);
   if (a.kind == TC_TF32X3_2) {  // one main accumulator: only the LM-head epilogues are instantiated

@@ -1,0 +1,48 @@
+"""How bf16 tensor-core projections are cut (l3_debug_gemm_plan; needs no GPU): where the slices of a residual projection may be added in
+the order they arrive, so that last bits differ from run to run, and where they may not."""
+import numpy as np
+import pytest
+
+from llama3_np_b200 import _cabi
+
+STORE, RESID, GATED = 0, 1, 2
+
+
+def plan(rows, n, k, epi=STORE):
+    p = np.zeros(5, np.int32)
+    _cabi.check(_cabi.lib().l3_debug_gemm_plan(rows, n, k, epi, _cabi.i32p(p)))
+    return dict(zip(("swapped", "ctas", "width", "slices", "any_order"), p.tolist()))
+
+
+@pytest.mark.parametrize("rows", [1, 9, 16, 17, 32, 36, 64, 100, 128])
+@pytest.mark.parametrize("n", [128, 256, 288, 512, 1024, 2048, 4096, 8192, 9472, 9473, 12288, 14336])
+def test_sums_that_always_came_in_order_still_do(rows, n):
+    for k in (72, 256, 384, 385, 392, 448, 512, 520, 704, 768, 896, 960, 1024, 2048, 4096, 14336):
+        if k % 8:
+            continue
+        p = plan(rows, n, k, RESID)
+        assert p["swapped"] == 1
+        if k <= 960 or n > 9472:   # fewer than 16 blocks of 64, or row blocks on more than half of 148 SMs
+            assert p["any_order"] == 0, (rows, n, k, p)
+        assert not p["any_order"] or p["slices"] > 1
+
+
+@pytest.mark.parametrize("epi", [STORE, GATED])
+def test_other_epilogues_sum_in_slice_order(epi):
+    for rows in (9, 36, 128, 129, 700, 4096):
+        for n in (96, 256, 2048, 28672):
+            for k in (72, 512, 2048, 14336):
+                assert plan(rows, n, k, epi)["any_order"] == 0
+
+
+def test_more_than_128_rows_add_to_the_residual_in_slice_order():
+    for rows in (129, 300, 2000):
+        for k in (448, 2048, 8192):
+            p = plan(rows, 1024, k, RESID)
+            assert p["swapped"] == 0 and p["any_order"] == 0
+
+
+def test_refused_arguments():
+    p = np.zeros(5, np.int32)
+    for bad in ((0, 256, 256, 0), (9, 0, 256, 0), (9, 256, 0, 0), (9, 256, 12, 0), (9, 256, 256, 3), (9, 256, 256, -1)):
+        assert _cabi.lib().l3_debug_gemm_plan(*bad, _cabi.i32p(p)) == _cabi.L3_EINVAL
