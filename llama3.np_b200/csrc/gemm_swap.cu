@@ -369,6 +369,8 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
         } else if constexpr (EPI == EPI_SWIGLU) {
           // weight rows interleave gate_j, up_j: an even lane holds the gate, its odd neighbour the up value.  The even lane takes the
           // chunk's first half of the rows, the odd one the second; all values before the first store, the activation decided once.
+          // silu with expf and a full reciprocal, in both modes: the fast forms take 2.3 us less per launch (32 x 28672 x 4096) but lose
+          // bits of every value and all of them from -87.4 down.
           constexpr int HF = CJ / 2;
           const bool odd = lane & 1;
           const int mb = c0 + (odd ? HF : 0);
@@ -379,9 +381,9 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
             gt[j] = odd ? got : v[j];
             hv[j] = odd ? v[j + HF] : got;
           }
-          if (KIND == TC_BF16 && e.act == GLU_SILU && !e.glu_w) {
+          if (e.act == GLU_SILU && !e.glu_w) {
 #pragma unroll
-            for (int j = 0; j < HF; ++j) hv[j] = gt[j] * __fdividef(1.0f, 1.0f + __expf(-gt[j])) * hv[j];
+            for (int j = 0; j < HF; ++j) hv[j] = silu_ref(gt[j]) * hv[j];
           } else {
 #pragma unroll
             for (int j = 0; j < HF; ++j) {
