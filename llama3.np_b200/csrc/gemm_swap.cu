@@ -369,8 +369,8 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
         } else if constexpr (EPI == EPI_SWIGLU) {
           // weight rows interleave gate_j, up_j: an even lane holds the gate, its odd neighbour the up value.  The even lane takes the
           // chunk's first half of the rows, the odd one the second; all values before the first store, the activation decided once.
-          // silu with expf and a full reciprocal, in both modes: the fast forms take 2.3 us less per launch (32 x 28672 x 4096) but lose
-          // bits of every value and all of them from -87.4 down.
+          // silu with expf and a full reciprocal, in both modes: the fast forms take 1 us less at 32 x 28672 x 4096 and 4 us at 100 rows
+          // but lose bits of every value, and all of them from -87.4 down.
           constexpr int HF = CJ / 2;
           const bool odd = lane & 1;
           const int mb = c0 + (odd ? HF : 0);

@@ -610,12 +610,12 @@ __device__ __forceinline__ void tc_gemm_run(TcPipe& p, const CUtensorMap* tmA0, 
           }
         } else if constexpr (EPI == EPI_SWIGLU) {
           // h = silu(gate) * up over interleaved (gate_j, up_j) columns (llama3.py:99-101).  bf16 mode
-          // uses the fast exponential / reciprocal (its bar is 3e-2); fp32 mode keeps the exact form.
+          // uses the fast exponential / reciprocal (its bar is 3e-2) unless glu_exact asks for the full ones; fp32 mode keeps the exact form.
           // All values before the first store, and the activation decided once per chunk: with a store between them the 16
           // exponentials and divisions follow one another (128 x 256 at K = 2048: the epilogue took longer than the products).
           if (col_ok) {
             float hv[16];
-            if (e.act == GLU_SILU && !e.glu_w) {
+            if (e.act == GLU_SILU && !e.glu_w && !e.glu_exact) {
 #pragma unroll
               for (int i = 0; i < 16; ++i) {
                 const float2 t = staged(i);
