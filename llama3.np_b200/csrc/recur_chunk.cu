@@ -671,6 +671,24 @@ __global__ void __launch_bounds__(256) lin_chunk_out_mma_kernel(RecurArgs a, int
         mma16816(acc[2], ah, v1[0], v1[1]); mma16816(acc[3], ah, v1[2], v1[3]);
       }
     }
+    // A token of these portions reads nothing of the ones behind it, as in the chain that they leave: zero scores times an infinity or a
+    // NaN among their values are NaN in the products, so what came out as NaN is taken again over the tokens up to its own
+    if constexpr (KIND == CK_MLSTM_PAIR) {
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = r0 + (u >> 1) * 8, e = e0 + wn * 32 + t * 8 + (lane & 3) * 2 + (u & 1);
+          if (acc[t][u] == acc[t][u] || i >= n) continue;
+          float s = 0.f;
+          for (int d = 0; d < DK; ++d)
+            s = fmaf(__bfloat162float(Qs[(size_t)i * LDK + d]) + __bfloat162float(Ql[(size_t)i * LDK + d]), P[(size_t)d * a.DV + e], s);
+          s *= dec.upto(i);
+          for (int j = 0; j <= i; ++j)
+            s = fmaf(__bfloat162float(Ah[(size_t)i * LDE + j]) + __bfloat162float(Al[(size_t)i * LDE + j]), vsrc[(size_t)j * a.ld_v + e], s);
+          acc[t][u] = s;
+        }
+    }
     float* op = a.out + (row0 + r0) * O + (size_t)h * a.DV + e0 + wn * 32 + (lane & 3) * 2;
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
