@@ -1024,6 +1024,27 @@ static void* optional_ws(size_t bytes) {
   return p;
 }
 
+static bool ll_takes_mirror(const L3Model* m, int rows, int N, int K);
+// Gated experts of many rows: all of them as one product with zero weights, or in groups, every expert over the rows that chose it.
+// Groups cost a pass to order the pairs, a gather and a sum (8 + 7 + 10 us) and up to 127 rows of padding per expert; they run where the
+// products that they leave out take more than 20 us at 1.2 PFLOP/s (the masked pass over all hidden values goes as well).  2000
+// tokens of width 2048, the best 2 of 16 experts of 1024 and a shared one of 2048, us: masked 300 of products + 48 of hidden
+// values, groups 60 + 30 for the experts, 31 + 20 for the shared one, 25 for the order.
+static bool ll_moe_groups_pay(const L3Model* m, const LLLayer& Ly, int ntok) {
+  const L3LayerSpec& s = Ly.spec;
+  const int W = m->D, F = Ly.ff_total;
+  if (!F || !m->h16 || ntok <= 128 || s.ff % 64 || W % 64 || s.shared_ff % 8 || s.experts > 1024 || !ll_takes_mirror(m, ntok, 2 * F, W)) return false;
+  const double mt = (ntok + 127) / 128, all = mt * F, grouped = (ntok * s.top / 128.0 + s.experts * 0.5) * s.ff + mt * s.shared_ff;  // row tiles x hidden columns
+  return (all - grouped) * 128 * W * 6 / 1.2e15 > 20e-6;
+}
+// per place of a pair: its result, its input, its hidden values
+static size_t ll_moe_groups_bytes(const L3Model* m, const LLLayer& Ly, int ntok) {
+  return (size_t)moe_group_tiles(ntok, Ly.spec.top, Ly.spec.experts) * 128 * (m->D * 6 + Ly.spec.ff * 2);
+}
+static bool ll_moe_in_groups(const L3Model* m, const LLLayer& Ly, const void* x16, int ntok) {
+  return x16 && ll_moe_groups_pay(m, Ly, ntok) && ll_moe_groups_bytes(m, Ly, ntok) <= m->ll->moe_ws_bytes;
+}
+
 // The workspaces of prompt paths that have another path beside them, behind everything a model cannot do without.
 static int ll_workspaces(L3Model* m, bool units, bool ksplit) {
   LayerList* ll = m->ll;
@@ -1044,6 +1065,12 @@ static int ll_workspaces(L3Model* m, bool units, bool ksplit) {
         chan = std::max(chan, recur_channel_ws_floats(1, (int)ct, s.heads, s.dim, s.vdim) + recur_channel_ws_floats(m->maxB, 1, s.heads, s.dim, s.vdim));
       if (ll_latent_expands_f32(m, s)) f_ld = std::max(f_ld, (size_t)s.heads * (s.dim + s.vdim));
     }
+  size_t moe = 0;  // pairs of gated experts in groups: which form a prompt takes does not hang on the room that the model was made with
+  for (auto& Ly : ll->layers)
+    for (int n = 129; n <= (int)ct; ++n)
+      if (ll_moe_groups_pay(m, Ly, n)) { moe = std::max(moe, ll_moe_groups_bytes(m, Ly, (int)ct)); break; }
+  if (moe > ll->moe_ws_bytes)
+    if (void* p = optional_ws(moe)) { ll->moe_ws = p; ll->moe_ws_bytes = moe; }
   if (ct > 8) {  // packed queries, maps of differential attention
     ll->win_q16 = optional_ws(ct * wq_ld * 2);
     ll->diff_maps = (float*)optional_ws(ct * maps_ld * 4);
@@ -1225,8 +1252,8 @@ int ll_finalize(L3Model* m) {
       CK(m, cudaMalloc((void**)&ll->moe_row_of, ct * max_top * 4));
       CK(m, cudaMalloc((void**)&ll->moe_groups, (1 + tiles) * 4));
       CK(m, cudaMalloc((void**)&ll->moe_wg, tiles * 128 * 4));
-      ll->moe_gu_bytes = ct * max_gu * 4;
-      ll->moe_h16_len = ct * std::max(1, ll->max_ff);
+      ll->moe_ws = ll->moe_gu;  // see ll_workspaces
+      ll->moe_ws_bytes = ct * max_gu * 4;
     }
   }
   for (const LLLayer& L0 : ll->layers)
@@ -1328,7 +1355,7 @@ void ll_destroy(L3Model* m) {
   }
   fr(ll->loop_in); fr(ll->embed_norm); fr(ll->final_b); fr(ll->final_alpha); fr(ll->x0); fr(ll->cat); fr(ll->cat16); fr(ll->win_part_o); fr(ll->win_part_ml); fr(ll->xs);
   fr(ll->diff_part_o); fr(ll->diff_part_ml);
-  fr(ll->Xs); fr(ll->hn); fr(ll->hf); fr(ll->hf16); fr(ll->y1); fr(ll->y2); fr(ll->moe_gu);
+  fr(ll->Xs); fr(ll->hn); fr(ll->hf); fr(ll->hf16); fr(ll->y1); fr(ll->y2); fr(ll->moe_ws == ll->moe_gu ? nullptr : ll->moe_ws); fr(ll->moe_gu);
   fr(ll->lat_q16); fr(ll->win_q16); fr(ll->diff_maps); fr(ll->lat_exp); fr(ll->lat_part_o); fr(ll->lat_part_ml);
   fr(ll->loop_step); fr(ll->qlat); fr(ll->aux16); fr(ll->moe_sel); fr(ll->moe_w); fr(ll->moe_dense); fr(ll->moe_idw); fr(ll->moe_row_of); fr(ll->moe_groups); fr(ll->moe_wg);
   fr(ll->pin); fr(ll->aux); fr(ll->rk); fr(ll->rv); fr(ll->rg); fr(ll->rbeta); fr(ll->o); fr(ll->sg); fr(ll->sg16); fr(ll->x2); fr(ll->chunk_ws);
@@ -1558,22 +1585,6 @@ static EpiArgs resid_into(float* x, int ld) {
   return e;
 }
 
-// Gated experts of many rows: all of them as one product with zero weights, or in groups, every expert over the rows that chose it.
-// Groups cost a pass to order the pairs, a gather and a sum (8 + 7 + 10 us) and up to 127 rows of padding per expert; they run where the
-// products that they leave out take more than 20 us at 1.2 PFLOP/s (the masked pass over all hidden values goes as well).  2000
-// tokens of width 2048, the best 2 of 16 experts of 1024 and a shared one of 2048, us: masked 300 of products + 48 of hidden
-// values, groups 60 + 30 for the experts, 31 + 20 for the shared one, 25 for the order.
-static bool ll_moe_in_groups(const L3Model* m, const LLLayer& Ly, const void* x16, int ntok) {
-  const L3LayerSpec& s = Ly.spec;
-  const LayerList* ll = m->ll;
-  const int W = m->D, F = Ly.ff_total;
-  if (!x16 || !m->h16 || !ll->moe_row_of || ntok <= 128 || s.ff % 64 || W % 64 || s.shared_ff % 8 || s.experts > 1024 || !ll_takes_mirror(m, ntok, 2 * F, W)) return false;
-  const size_t rows = (size_t)moe_group_tiles(ntok, s.top, s.experts) * 128;
-  if (rows * W * 6 > ll->moe_gu_bytes || rows * s.ff > ll->moe_h16_len || (size_t)ntok * s.shared_ff > ll->moe_h16_len) return false;
-  const double mt = (ntok + 127) / 128, all = mt * F, grouped = (ntok * s.top / 128.0 + s.experts * 0.5) * s.ff + mt * s.shared_ff;  // row tiles x hidden columns
-  return (all - grouped) * 128 * W * 6 / 1.2e15 > 20e-6;
-}
-
 // dst (+)= the experts' outputs; the shared expert's go through `epi` first (sw: its weight per row, on the output).  Experts' weights scale
 // their outputs (w_out) or their inputs.
 static int ll_moe_groups(L3Model* m, const LLLayer& Ly, const void* x16, int ntok, bool w_out, const float* sw, int epi, const EpiArgs& e_shared, float* dst) {
@@ -1593,16 +1604,16 @@ static int ll_moe_groups(L3Model* m, const LLLayer& Ly, const void* x16, int nto
     LAUNCH(m, launch_gemm_tc(t, m->stream));
   }
   const int rows = moe_group_tiles(ntok, s.top, E) * 128;
-  bf16* xg = (bf16*)ll->moe_gu;
-  float* yg = (float*)(xg + (size_t)rows * W);
+  float* yg = (float*)ll->moe_ws;
+  bf16 *xg = (bf16*)(yg + (size_t)rows * W), *hg = xg + (size_t)rows * W;
   LAUNCH(m, launch_moe_group(ll->moe_sel, ll->moe_w, ntok, s.top, E, W, (const bf16*)x16, ll->moe_row_of, ll->moe_groups, xg, ll->moe_wg, m->stream));
   m->launch_acc += 1;
   t.groups = ll->moe_groups; t.rows = rows; t.group_rows = ntok * s.top + E * 64; t.ldw = 0;
   t.A[0] = xg; t.W[0] = w13; t.N = 2 * ff; t.K = W; t.group_n = 2 * ff; t.group_k = 0; t.w_rows = 2 * E * ff; t.w_cols = W;
-  t.epi = EPI_SWIGLU; t.e = store_to(nullptr, m->h16, ff);
+  t.epi = EPI_SWIGLU; t.e = store_to(nullptr, hg, ff);
   t.e.act = GLU_SILU; t.e.glu_exact = 1; t.e.glu_w = ll->moe_wg; t.e.glu_w_ld = 1; t.e.glu_group = ff; t.e.glu_groups = 1; t.e.glu_w_out = w_out;
   LAUNCH(m, launch_gemm_tc(t, m->stream));
-  t.A[0] = m->h16; t.W[0] = w2; t.N = W; t.K = ff; t.group_n = 0; t.group_k = ff; t.w_rows = W; t.w_cols = F; t.epi = EPI_STORE; t.e = store_to(yg, nullptr, W);
+  t.A[0] = hg; t.W[0] = w2; t.N = W; t.K = ff; t.group_n = 0; t.group_k = ff; t.w_rows = W; t.w_cols = F; t.epi = EPI_STORE; t.e = store_to(yg, nullptr, W);
   LAUNCH(m, launch_gemm_tc(t, m->stream));
   LAUNCH(m, launch_moe_combine(yg, ll->moe_row_of, ntok, s.top, W, sff || epi == EPI_RESID, dst, m->stream));
   return L3_OK;

@@ -132,7 +132,8 @@ struct LayerList {
   // gated experts of many rows in groups (bf16 mode): pairs' places [rows, top], tiles and their experts, weights by place
   int *moe_row_of = nullptr, *moe_groups = nullptr;
   float* moe_wg = nullptr;
-  size_t moe_gu_bytes = 0, moe_h16_len = 0;  // room of moe_gu, entries of h16
+  void* moe_ws = nullptr;                  // pairs' inputs, hidden values and results: moe_gu where that is large enough for any call, or its own
+  size_t moe_ws_bytes = 0;
   int32_t* moe_sel = nullptr;              // [rows, top]
   // parallel layers
   float* Xs = nullptr;                     // [n_layers + 1][cap_tok, width] embedding output and every layer's own result

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 import test_mabedra_gpu as mab
+import test_vupitar_gpu as vup
 
 pytestmark = pytest.mark.gpu
 E, W, FF, V = 64, 1024, 256, 70
@@ -52,3 +53,68 @@ def test_silu_of_a_shared_expert_keeps_its_tail(n):
     m.close()
     assert more == 4
     assert mab.err(got[0], o.run(ids[0])) < mab.BF16_BAR
+
+
+def planted_rows(top, rng):
+    """64 directions at right angles; a token's embedding leans on its own and, less and less, on the next ones: its experts"""
+    a = np.linalg.qr(rng.standard_normal((W, E)))[0].T * np.sqrt(W)
+    return a, sum((1.0 - 0.2 * k) * a[(np.arange(V) + k) % E] for k in range(top))
+
+
+def planted_ids(n, rng):
+    """experts of 127, 128 and 129 first choices, one of one, the rest spread, some never chosen"""
+    ids = [0] * 127 + [4] * 128 + [8] * 129 + [12] if n > 400 else [0] * 127 + [12]
+    return rng.permutation(np.concatenate([ids, rng.integers(16, 50, n - len(ids))]))
+
+
+def sigmoid_model(top, shared):
+    cfg = mab.config([mab.attn(heads=2, kv_heads=1, dim=64, vdim=64, mlp=mab.moe(E, top, FF, shared))], width=W, vocab=V, taps=0)
+    t = mab.random_model(cfg, 11)
+    a, t["embed"] = planted_rows(top, np.random.default_rng(12))
+    t["l0.mlp.router"] = a * (2.0 / W)
+    t["l0.norm1"], t["l0.mix.o"] = np.ones(W), 0 * t["l0.mix.o"]
+    return cfg, bf16_values(t)
+
+
+@pytest.mark.parametrize("n,top,shared", [(257, 1, 0), (431, 3, 128), (600, 2, 264)])
+@pytest.mark.parametrize("room", ["tight", "wide", "none"])
+def test_the_form_does_not_hang_on_the_models_length(n, top, shared, room, monkeypatch):
+    """A model made for just the prompt, one made for much longer ones, and - the masked form, where it needs one - without a workspace."""
+    if room == "none":
+        monkeypatch.setenv("L3_SCRATCH_MB", "0")
+    cfg, t = sigmoid_model(top, shared)
+    m, o = mab.build(cfg, dtype="bfloat16", max_seq_len=2048 if room == "wide" else n + 2, tensors=t)
+    ids = planted_ids(n, np.random.default_rng(n))
+    got, more = run(m, ids[None])
+    m.close()
+    if room != "none":
+        assert more == (4 if shared else 2)
+    elif n == 257:
+        assert more == 0
+    assert mab.err(got[0], o.run(ids)) < mab.BF16_BAR
+
+
+@pytest.mark.parametrize("n,batch,top,shared", [(300, 1, 2, 256), (600, 1, 1, 64), (431, 1, 3, 128), (150, 2, 2, 0), (200, 3, 2, 264)])
+def test_weights_on_outputs_and_a_gated_shared_expert(n, batch, top, shared):
+    """Softmax scores over their sum on the experts' outputs, a sigmoid's on the shared one's, all added to the residual stream in
+    place; planted routing, so that every row is held to the bar."""
+    mlp = {"kind": "moe", "router": {"experts": E, "top": top}, "expert": {"ff": FF}}
+    if shared:
+        mlp["shared"] = {"ff": shared}
+    cfg = vup.config([vup.layer(l=vup.left(heads=2, kv_heads=1, dim=64, vdim=64, size=80), r=vup.right(heads=2, dim=64, vdim=64), mlp=mlp)],
+                     width=W, vocab=V, scale=1.0)
+    t = vup.random_model(cfg, 7)
+    rng = np.random.default_rng(13)
+    a, t["embed"] = planted_rows(top, rng)
+    t["l0.mlp.router"] = a * (4.0 / W)
+    for k in ("left.o", "left.o.b", "right.o"):
+        t["l0.mix." + k] = 0 * t["l0.mix." + k]
+    t["l0.norm2"], t["l0.norm2.b"], t["l0.norm2.alpha"] = np.ones(W), np.zeros(W), np.array(0.7)
+    t = bf16_values(t)
+    m, o = vup.build(cfg, dtype="bfloat16", max_seq_len=n + 2, max_batch_size=batch, tensors=t)
+    ids = np.stack([planted_ids(n, rng) for _ in range(batch)])
+    got, more = run(m, ids)
+    m.close()
+    assert more == (4 if shared else 2)
+    for b in range(batch):
+        assert vup.err(got[b], vup.fresh(o).run(ids[b])) < vup.BF16_BAR
