@@ -2097,6 +2097,7 @@ static int ll_enqueue_parallel(L3Model* m, int B, int L, float* d_resid) {
     if (Ly.ff_total) {
       const int E = s.experts, ff = s.ff, F = Ly.ff_total;
       const bool few = ntok <= 8;  // few rows read only their chosen experts' weights; many share one GEMM over all experts
+      static const bool fused = getenv("L3_MOE_EPI") && atoi(getenv("L3_MOE_EPI")) == 1;
       MoeRouteArgs ra{};
       ra.h = hf; ra.router = Ly.router; ra.correction = nullptr; ra.D = W; ra.E = E; ra.I = 0; ra.top = s.top;
       ra.groups = 1; ra.keep = 1; ra.kind = 1; ra.scale = 1.0f;
@@ -2105,14 +2106,13 @@ static int ll_enqueue_parallel(L3Model* m, int B, int L, float* d_resid) {
       if (few) {
         LAUNCH(m, launch_moe_glu_rows(hf, Ly.w13, Ly.w2, m->bf16, ll->moe_sel, ll->moe_w, nullptr, false, ntok, W, E, ff, s.shared_ff, s.top, m->h, ll->y2, false, m->stream));
         m->launch_acc += 1;
-      } else if (ll_moe_in_groups(m, Ly, hf16, ntok)) {
+      } else if (!fused && ll_moe_in_groups(m, Ly, hf16, ntok)) {
         if ((rc = ll_moe_groups(m, Ly, hf16, ntok, false, nullptr, EPI_STORE, store_to(ll->y2, nullptr, W), ll->y2)) != L3_OK) return rc;
       } else {
         // gate | up of every expert and of the shared one in ONE projection, then the routing weight (zero for experts the
-        // row did not choose) and silu(g) * u in a streaming kernel.  L3_MOE_EPI=1 moves that step into the GEMM's epilogue:
-        // measured slower (width 2048, 2048 tokens: 13.65 against 12.95 ms per prompt) - the epilogue then does a weight
-        // lookup and an exponential per output pair while the tensor pipe waits.
-        static const bool fused = getenv("L3_MOE_EPI") && atoi(getenv("L3_MOE_EPI")) == 1;
+        // row did not choose) and silu(g) * u in a streaming kernel.  L3_MOE_EPI=1 moves that step into the GEMM's epilogue, for any
+        // number of rows (no groups then).  Measured slower when all rows took this form (width 2048, 2048 tokens: 13.65 against 12.95
+        // ms per prompt) - the epilogue does a weight lookup and an exponential per output pair while the tensor pipe waits.
         if (fused) {
           EpiArgs e = store_to(m->h, m->h16, F);
           e.act = GLU_SILU; e.glu_w = ll->moe_dense; e.glu_w_ld = E; e.glu_group = ff; e.glu_groups = E;

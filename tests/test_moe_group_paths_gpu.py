@@ -1,6 +1,10 @@
 """Gated experts of many rows in groups (moe.cu, layerlist.cu: ll_moe_groups), with the path asserted by its number of launches: order,
 gather, two products and the sum - and two more products for a shared expert - where the masked form has two products and a pass over
 the hidden values."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -118,3 +122,18 @@ def test_weights_on_outputs_and_a_gated_shared_expert(n, batch, top, shared):
     assert more == (4 if shared else 2)
     for b in range(batch):
         assert vup.err(got[b], vup.fresh(o).run(ids[b])) < vup.BF16_BAR
+
+
+def test_the_fused_form_still_answers_to_its_switch():
+    """L3_MOE_EPI=1 (read once per process) takes prompts of any length to the one product with weights in its epilogue."""
+    code = ("import numpy as np, test_moe_group_paths_gpu as t\n"
+            "cfg, w = t.sigmoid_model(2, 264)\n"
+            "m, o = t.mab.build(cfg, dtype='bfloat16', max_seq_len=2048, tensors=w)\n"
+            "ids = t.planted_ids(300, np.random.default_rng(1))\n"
+            "got, more = t.run(m, ids[None])\n"
+            "assert more == 0 and t.mab.err(got[0], o.run(ids)) < t.mab.BF16_BAR")
+    here = os.path.dirname(os.path.abspath(__file__))
+    path = os.pathsep.join([here, os.path.dirname(here)] + [p for p in [os.environ.get("PYTHONPATH")] if p])
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, L3_MOE_EPI="1", PYTHONPATH=path), cwd=os.path.dirname(here),
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
