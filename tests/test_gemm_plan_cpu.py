@@ -46,3 +46,18 @@ def test_refused_arguments():
     p = np.zeros(5, np.int32)
     for bad in ((0, 256, 256, 0), (9, 0, 256, 0), (9, 256, 0, 0), (9, 256, 12, 0), (9, 256, 256, 3), (9, 256, 256, -1)):
         assert _cabi.lib().l3_debug_gemm_plan(*bad, _cabi.i32p(p)) == _cabi.L3_EINVAL
+
+
+def test_shapes_of_the_gpu_test_reach_every_cut():
+    from test_gemm_pairs_gpu import SHAPES
+    seen = set()
+    for rows, n, k in SHAPES:
+        p = plan(rows, n, k)
+        assert p["swapped"] == 0
+        tiles = -(-rows // (128 * p["ctas"])) * -(-n // p["width"]) * p["slices"]
+        rounds = -(-tiles // (148 // p["ctas"]))
+        seen |= {("width", p["ctas"], p["width"]), ("rounds", p["ctas"], rounds > 1), ("slices", p["ctas"], p["slices"] > 1, rounds > 1)}
+    assert {w for kind, c, w, *_ in seen if kind == "width" and c == 1} == set(range(32, 257, 32))
+    assert {w for kind, c, w, *_ in seen if kind == "width" and c == 2} >= set(range(96, 257, 32))
+    for c in (1, 2):
+        assert {("rounds", c, False), ("rounds", c, True), ("slices", c, True, False), ("slices", c, True, True), ("slices", c, False, True)} <= seen
