@@ -32,7 +32,7 @@
 #include "gemm_tc.h"
 
 __device__ unsigned long long g_tc_dbg[64];
-static std::atomic<unsigned long long*> g_tc_dbg_to{nullptr};  // where launches leave their timeline (null: nowhere)
+static std::atomic<unsigned long long*> g_tc_dbg_to[16];  // where a device's launches leave their timeline, in its own memory (null: nowhere)
 
 #include "gemm_tc_dev.cuh"
 
@@ -127,8 +127,10 @@ int tc_debug_timeline(int enable, unsigned long long* out64) {
   if (out64 && cudaMemcpyFromSymbol(out64, g_tc_dbg, sizeof(unsigned long long) * 64) != cudaSuccess) return -1;
   unsigned long long z[64] = {0};
   void* p = nullptr;
+  int dev = 0;
+  cudaGetDevice(&dev);
   if (cudaMemcpyToSymbol(g_tc_dbg, z, sizeof z) != cudaSuccess || cudaGetSymbolAddress(&p, g_tc_dbg) != cudaSuccess) return -1;
-  g_tc_dbg_to = enable ? (unsigned long long*)p : nullptr;
+  g_tc_dbg_to[dev & 15] = enable ? (unsigned long long*)p : nullptr;
   return 0;
 }
 
@@ -236,7 +238,7 @@ static cudaError_t launch_tc_t(const TcGemmArgs& a, cudaStream_t s) {
   const int nkb = (nkb_all + ksplit - 1) / ksplit;
   const int nst = std::max(2, std::min(std::min(Cf::stages(bn), env_st), nkb));
   return launch_kc(kern, grid, dim3(TC_THREADS), (size_t)Cf::smem(bn, nst), s, CG, *A0, *A1, *B0, *B1, a.rows, a.N, a.K, bn, a_box, nst, ksplit, a.part, a.tile_cnt,
-                  a.err, g_tc_dbg_to.load(), TcGroups{a.groups, a.group_n, a.group_k}, a.e);
+                  a.err, g_tc_dbg_to[dev & 15].load(), TcGroups{a.groups, a.group_n, a.group_k}, a.e);
 }
 
 template <int KIND, int BN, int CG>
