@@ -51,3 +51,23 @@ def test_timeline_is_left_where_it_was_asked_for():
         _linear(x, x)
         assert lib.l3_debug_tc_timeline(0, 0, buf) == 0
         assert any(buf) == bool(on)
+
+
+@pytest.mark.parametrize("batch", [130, 200])
+def test_pairs_inside_a_captured_decode_step(batch):
+    """More than 128 sequences decode through these products, replayed from a graph: the tokens of the same steps launched one by one."""
+    from llama3_np_b200 import Llama, ModelArgs, _cabi
+    from llama3_np_b200.synth import make_weights
+    args = ModelArgs(dim=512, n_layers=2, n_heads=8, n_kv_heads=4, vocab_size=1024, max_seq_len=32, max_batch_size=batch)
+    args.dtype = "bfloat16"
+    w = make_weights(args, 1536, seed=4)
+    ids = np.random.default_rng(5).integers(3, 1024, (batch, 6))
+    got = []
+    for flags in (0, _cabi.FLAG_NO_GRAPH):
+        m = Llama(w, args, flags=flags)
+        tokens = m.generate_all(ids, 24)
+        m.reset_cache()
+        got.append((tokens, m.forward_f32(ids, 0)))
+        m.close()
+    assert np.array_equal(got[0][0], got[1][0])
+    assert np.array_equal(got[0][1].view(np.uint32), got[1][1].view(np.uint32))

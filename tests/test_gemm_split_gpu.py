@@ -1,4 +1,4 @@
-"""bf16 tensor-core projections (gemm_tc.cu): tiles of one CTA and of pairs, and tiles cut along K: widths of 32 to 256 columns with remainders, two to eight
+"""bf16 tensor-core projections whose tiles are cut along K (gemm_tc.cu): widths of 32 to 256 columns with remainders, two to eight
 slices, more tiles than the machine holds at once.  Bound: the operands are bf16 numbers, products are exact, and the accumulator
 loses at most 2^-23 of its value per instruction of 16 terms, half of that on average: K / 16 * 2^-24 of the result, 3.1e-5 at
 K = 8192 - a slice that is missing, doubled or misplaced changes it by a share of order 1 / 8."""
@@ -31,7 +31,7 @@ def test_k_splits_add_up(rows, n, k):
 @pytest.mark.parametrize("rows,n,k", [(129, 7001, 3000), (385, 4096, 2056), (384, 14000, 600), (513, 8190, 520), (700, 1024, 4096), (1000, 3000, 1000),
                                       (1462, 2048, 2048), (2050, 1999, 2056), (130, 160, 520), (1000, 992, 72)])
 def test_widths_and_pairs(rows, n, k):
-    """Widths in steps of 32 up to 256, one CTA or two on a tile: a last pair whose second CTA has no row or one, columns and k-blocks
+    """Widths in steps of 32, one CTA or two on a tile (all of them: test_gemm_pairs_gpu.py): a last pair whose second CTA has no row or one, columns and k-blocks
     that end inside a tile, odd widths of the result (element stores)."""
     from llama3_np_b200 import _cabi
     rng = np.random.default_rng(rows + n + k)
