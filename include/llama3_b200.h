@@ -373,11 +373,12 @@ int l3_op_recurrence(int device, const float* q, const float* k, const float* v,
 /* logits[:, -1, :].argmax(-1) (llama3.py:320): first maximum wins. */
 int l3_op_argmax(int device, const float* logits, int rows, int n, int64_t* out);
 
-/* How the model path cuts a bf16 tensor-core projection of `rows` rows (epi 0: plain store, 1: added to the residual in place, 2: gated):
+/* How the model path cuts a tensor-core projection of `rows` rows in bf16 mode, or with fp32 != 0 one of up to 128 rows of the Llama
+ * path's fp32 mode (epi 0: plain store, 1: added to the residual in place, 2: gated):
  * plan[0] 1 = weights as the 128-row operand (gemm_swap.cu), 0 = activations (gemm_tc.cu); [1] CTAs that share a tile; [2] the tile's
  * width (gemm_swap.cu: height); [3] slices of K; [4] 1 = the slices are added in whatever order they arrive, so that the last bits
  * differ from run to run.  Without a GPU: for 148 SMs. */
-int l3_debug_gemm_plan(int rows, int n, int k, int epi, int32_t* plan);
+int l3_debug_gemm_plan(int rows, int n, int k, int epi, int fp32, int32_t* plan);
 
 /* Debug: switch the tcgen05 GEMM's clock64 milestone stamps on/off and read the last 64
  * stamps of CTA (0,0) (indices documented in gemm_tc.cu). */

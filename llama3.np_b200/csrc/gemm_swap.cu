@@ -525,8 +525,9 @@ static bool adds_in_place(const TcGemmArgs& a, int sms) {
   static const int resid_atomic = [] { const char* v = getenv("L3_SWAP_RESID_ATOMIC"); return v ? atoi(v) : 1; }();
   return a.epi == EPI_RESID && a.kind == TC_BF16 && a.e.out == a.e.resid && resid_atomic && (a.K + 63) / 64 >= 16 && (a.N + 127) / 128 * 2 <= sms;
 }
-// Tile height and K split, by the cycles of the busiest CTA: a k-block takes the issue loops ~500 cycles, or its share of DRAM
-// (3560 bytes per cycle for all CTAs that stream); slices that are added in place cost little, published and summed ones ~2.5 us and more
+// Tile height and K split, by the cycles of the busiest CTA: a k-block takes the issue loops ~500 cycles (fp32 mode, two parts and three
+// products: 750 - 980 with the columns; with 700 for all of them 74 x 288 x 768 took 26.7 us whole instead of 24.7 in slices, 74 x 8192 x
+// 1536 43.9 instead of 39.4), or its share of DRAM (3560 bytes per cycle for all CTAs that stream); slices that are added in place cost little, published and summed ones ~2.5 us and more
 // with each slice and row.  More tiles than SMs: the height is what makes the last round full (28672 rows: 293 tiles of 98 instead of
 // 224 of 128).  us per launch in a row of such launches, before (a split that fills the SMs, tiles of 128) -> here: 8 x 2048 x 4096
 // 12.5 -> 9.0, 8 x 2048 x 8192 13.0 -> 11.7, 32 x 28672 x 4096 swiglu 41.7 -> 39.9; over 22 shapes it is at most 7 % behind the best.
@@ -545,11 +546,11 @@ static void pick_swap(const TcGemmArgs& a, int bna, int sms, int* h_out, int* ks
     if (ks > 1 && (per < 4 || (ks - 1) * per >= nkb)) break;
     if (ks > 1 && !atomic && (!a.part || !a.tile_cnt || tiles > a.tile_cnt_len || (size_t)bna * tiles * 128 * sizeof(float) * ks > a.part_bytes ||
                               !(det_epi || a.epi == EPI_RESID))) break;
-    const double issue = b16 ? 500 : 700;
+    const double issue = b16 ? 500 : 720 + 2.0 * bna, slice = 160 + 22.0 * bna + (b16 ? 0 : 8.0 * a.rows);
     const int full = tiles * ks / sms, rest = tiles * ks % sms;
     double c = full * per * std::max(issue, h * 128.0 * parts * sms / 3560);
     if (rest) c += per * std::max(issue, h * 128.0 * parts * rest / 3560);
-    if (ks > 1) c += atomic ? 380 + 2.0 * ks * bna : 4400 + (160 + 22.0 * bna) * ks;
+    if (ks > 1) c += atomic ? 380 + 2.0 * ks * bna : 4400 + slice * ks;
     if (best == 0 || c < best) { best = c; *ks_out = ks; }
   }
   *h_out = h;

@@ -287,12 +287,12 @@ extern "C" int l3_op_recurrence(int device, const float* q, const float* k, cons
   return rc;
 }
 
-extern "C" int l3_debug_gemm_plan(int rows, int n, int k, int epi, int32_t* plan) {
-  if (rows < 1 || n < 1 || k < 1 || k % 8 || epi < EPI_STORE || epi > EPI_SWIGLU || !plan) return L3_EINVAL;
+extern "C" int l3_debug_gemm_plan(int rows, int n, int k, int epi, int fp32, int32_t* plan) {
+  if (rows < 1 || n < 1 || k < 1 || k % 8 || epi < EPI_STORE || epi > EPI_SWIGLU || !plan || (fp32 && !gemm_swap_supported(rows, n))) return L3_EINVAL;
   static float x;  // addresses stand for buffers: nothing reads or writes them
   static int cnt;
   TcGemmArgs t{};
-  t.kind = TC_BF16; t.rows = rows; t.N = n; t.K = k; t.epi = epi;
+  t.kind = fp32 ? TC_TF32X3 : TC_BF16; t.rows = rows; t.N = n; t.K = k; t.epi = epi;
   t.part = &x; t.part_bytes = (size_t)32 << 20; t.tile_cnt = &cnt; t.tile_cnt_len = 1024;
   t.e.out = &x;
   if (epi == EPI_RESID) t.e.resid = &x;

@@ -8,9 +8,9 @@ from llama3_np_b200 import _cabi
 STORE, RESID, GATED = 0, 1, 2
 
 
-def plan(rows, n, k, epi=STORE):
+def plan(rows, n, k, epi=STORE, fp32=0):
     p = np.zeros(5, np.int32)
-    _cabi.check(_cabi.lib().l3_debug_gemm_plan(rows, n, k, epi, _cabi.i32p(p)))
+    _cabi.check(_cabi.lib().l3_debug_gemm_plan(rows, n, k, epi, fp32, _cabi.i32p(p)))
     return dict(zip(("swapped", "ctas", "width", "slices", "any_order"), p.tolist()))
 
 
@@ -42,9 +42,17 @@ def test_more_than_128_rows_add_to_the_residual_in_slice_order():
             assert p["swapped"] == 0 and p["any_order"] == 0
 
 
+@pytest.mark.parametrize("rows,n,k,slices", [(74, 288, 768, 3), (100, 288, 768, 1), (128, 4096, 768, 1), (74, 1024, 768, 3), (12, 8192, 1536, 2), (48, 8192, 1536, 2),
+                                             (74, 8192, 1536, 2), (128, 8192, 1536, 2), (74, 8192, 768, 1), (128, 288, 288, 1), (9, 288, 288, 1)])
+def test_fp32_products_are_cut_where_that_was_measured_faster(rows, n, k, slices):
+    p = plan(rows, n, k, STORE, 1)
+    assert p["slices"] == slices and p["any_order"] == 0
+    assert plan(rows, n, k, RESID, 1)["any_order"] == 0   # fp32 sums always come in slice order
+
+
 def test_refused_arguments():
     p = np.zeros(5, np.int32)
-    for bad in ((0, 256, 256, 0), (9, 0, 256, 0), (9, 256, 0, 0), (9, 256, 12, 0), (9, 256, 256, 3), (9, 256, 256, -1)):
+    for bad in ((0, 256, 256, 0, 0), (9, 0, 256, 0, 0), (9, 256, 0, 0, 0), (9, 256, 12, 0, 0), (9, 256, 256, 3, 0), (9, 256, 256, -1, 0), (129, 256, 256, 0, 1)):
         assert _cabi.lib().l3_debug_gemm_plan(*bad, _cabi.i32p(p)) == _cabi.L3_EINVAL
 
 
