@@ -23,16 +23,17 @@
 // the activation rows are staged - weights do not depend on the previous kernel - so the HBM
 // stream starts while RMSNorm staging (and, under PDL, the predecessor's tail) is still running.
 // From 2 rows on the staged activations' way out of shared memory is the bound, not HBM.  A lane's eight values behind a 16-byte bf16
-// vector are two 16-byte reads: in x's own order lanes would be 32 bytes apart and every read take twice its wavefronts, so blocks of
-// 256 values are staged as the lanes' first halves, then their second halves.
-// One and two rows are bound by the weights, and their plain order is 2 - 8 % faster.  28672 x 4096, us: 4 rows 85 -> 75, 8 rows 142 -> 115.
-constexpr bool rows_by_halves(int vec, int rows) { return vec == 8 && rows > 2; }
+// vector are two 16-byte reads: in x's own order lanes would be 32 bytes apart and every read take twice its wavefronts, so for 3 - 8 rows
+// blocks of 256 values are staged as the lanes' first halves, then their second halves (HALVES).  28672 x 4096, us: 4 rows 85 -> 75, 8
+// rows 142 -> 115; 4096 x 2048, 5 rows 22.6 -> 20.5.  The staging itself costs more that way, which shows where a CTA has few weight rows
+// or short ones to read: 1024 x 4096, 5 rows 58 : 69, 1536 x 4104, 8 rows 32.8 : 34.7, 16384 x 288, 4 rows 16.4 : 17.8.  From 2048 rows of
+// 768 values on it loses nowhere.  One and two rows are bound by the weights, and their plain order is 2 - 8 % faster.
+static bool rows_by_halves(int npairs, int K) { return npairs >= 1024 && K >= 768; }
 __host__ __device__ constexpr int rows_stage_len(int K, bool halves) { return halves ? (K + 255) / 256 * 256 : K; }
-template <typename WT, int MB, int EPI, typename KVT, int PF>
+template <typename WT, int MB, int EPI, typename KVT, int PF, bool HALVES>
 __global__ void __launch_bounds__(512) linear_rows_kernel(LinearArgs a) {
   extern __shared__ __align__(16) float xs[];  // [MB][KS]
   constexpr int VEC = Vec16<WT>::N;            // PF = weight vectors per row in flight per lane
-  constexpr bool HALVES = rows_by_halves(VEC, MB);
   const int K = a.K, KS = rows_stage_len(K, HALVES);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   auto at = [](int k) { return HALVES ? (k & ~255) + (k & 4) * 32 + ((k >> 3) & 31) * 4 : k; };  // of values k .. k + 3
@@ -203,14 +204,17 @@ static cudaError_t launch_rows_t(const LinearArgs& a_in, cudaStream_t s) {
   a.l2_prefetch_pairs = l2pf;
   // prefetch depth: 8 vectors per row per lane for the single-row kernel (tunable: L3_GEMV_PF)
   static const int pf = gemv_env("L3_GEMV_PF", 4);
-  auto kern = (MB == 1 && pf == 8) ? linear_rows_kernel<WT, MB, EPI, KVT, (MB == 1 ? 8 : 4)>
-                                   : linear_rows_kernel<WT, MB, EPI, KVT, 4>;
-  const size_t smem = (size_t)MB * rows_stage_len(a.K, rows_by_halves(Vec16<WT>::N, MB)) * sizeof(float);
+  constexpr bool CAN = Vec16<WT>::N == 8 && MB > 2;
+  const int npairs = (a.N + 1) / 2;
+  const bool halves = CAN && rows_by_halves(npairs, a.K);
+  auto kern = (MB == 1 && pf == 8) ? linear_rows_kernel<WT, MB, EPI, KVT, (MB == 1 ? 8 : 4), false>
+              : halves             ? linear_rows_kernel<WT, MB, EPI, KVT, 4, CAN>
+                                   : linear_rows_kernel<WT, MB, EPI, KVT, 4, false>;
+  const size_t smem = (size_t)MB * rows_stage_len(a.K, halves) * sizeof(float);
   if (smem + 2048 > 48 * 1024) {  // the 48 KB default limit covers static + dynamic shared memory: opt in near it, too
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  const int npairs = (a.N + 1) / 2;
   // choose warps per SM so that npairs / (148 * warps) sits just below an integer (balanced SMs)
   static const int max_wps = gemv_env("L3_GEMV_WPS", MB <= 2 ? 32 : 16);
   int best_w = 4;
