@@ -615,12 +615,13 @@ __device__ __forceinline__ void tc_gemm_run(TcPipe& p, const CUtensorMap* tmA0, 
           // exponentials and divisions follow one another (128 x 256 at K = 2048: the epilogue took longer than the products).
           if (col_ok) {
             float hv[16];
-            if (e.act == GLU_SILU && !e.glu_w && !e.glu_exact) {
+            if (e.act == GLU_SILU && !e.glu_w) {
+              if (KIND == TC_BF16 && !e.glu_exact) {
 #pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                const float2 t = staged(i);
-                if constexpr (KIND == TC_BF16) hv[i] = t.x * __fdividef(1.0f, 1.0f + __expf(-t.x)) * t.y;
-                else hv[i] = silu_ref(t.x) * t.y;
+                for (int i = 0; i < 16; ++i) { const float2 t = staged(i); hv[i] = t.x * __fdividef(1.0f, 1.0f + __expf(-t.x)) * t.y; }
+              } else {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) { const float2 t = staged(i); hv[i] = silu_ref(t.x) * t.y; }
               }
             } else {
               const int g = e.glu_w ? (col >> 1) / e.glu_group : 0;

@@ -1026,10 +1026,10 @@ static void* optional_ws(size_t bytes) {
 
 static bool ll_takes_mirror(const L3Model* m, int rows, int N, int K);
 // Gated experts of many rows: all of them as one product with zero weights, or in groups, every expert over the rows that chose it.
-// Groups cost a pass to order the pairs, a gather and a sum (8 + 7 + 10 us) and up to 127 rows of padding per expert; they run where the
+// Groups cost a pass to order the pairs, a gather and a sum (9 + 8 + 10 us) and up to 127 rows of padding per expert; they run where the
 // products that they leave out take more than 20 us at 1.2 PFLOP/s (the masked pass over all hidden values goes as well).  2000
 // tokens of width 2048, the best 2 of 16 experts of 1024 and a shared one of 2048, us: masked 300 of products + 48 of hidden
-// values, groups 60 + 30 for the experts, 31 + 20 for the shared one, 25 for the order.
+// values, groups 61 + 28 for the experts, 39 + 20 for the shared one, 27 for the order.
 static bool ll_moe_groups_pay(const L3Model* m, const LLLayer& Ly, int ntok) {
   const L3LayerSpec& s = Ly.spec;
   const int W = m->D, F = Ly.ff_total;
