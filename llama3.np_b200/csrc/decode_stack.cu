@@ -21,9 +21,10 @@
 // Math: plain fp32 FFMA.  Thread tile = 4 output features x ALL S sequences (48 accumulators) over a k-group (1/4 or
 // 1/8 of each slab's k rows): per k row one float4 of weights from the k-major slab (quarter warps read 128
 // contiguous bytes) and S / 4 broadcast float4s of activations from a k-major [K][S + 8] buffer (80-byte rows keep
-// the k-groups' reads in different banks) feed 48 FFMAs; k-groups are the high lane bits and are summed with shuffles.  (tcgen05 is the wrong tool
-// for S = 12 rows: an M = 128 MMA costs 40 cycles below N = 64 - profiles/mma_cost.jsonl -, three of them less than FFMAs do, and the legacy
-// mma.sync path at 3xTF32 is only 1.4x the FFMA peak.)
+// the k-groups' reads in different banks) feed 48 FFMAs; k-groups are the high lane bits and are summed with shuffles.  (tcgen05 gives
+// nothing at S = 12 rows: an M = 128 MMA takes 45 cycles below N = 64 - profiles/mma_cost.jsonl -, so the three of a 3xTF32 product do
+// 128 x 12 x 8 terms in 135 cycles, 91 per cycle, where the FFMA phases reach 80 - 92, and the slabs would hold both parts, twice the
+// bytes.  At 24 rows it would be 180 per cycle: not built.  The legacy mma.sync path at 3xTF32 is 1.4x the FFMA peak.)
 #include <stdio.h>
 
 #include "common.cuh"

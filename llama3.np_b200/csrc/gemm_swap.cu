@@ -175,8 +175,9 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
   }
 
   // The issuing warps run their loops whole, one elected lane issues, ring positions are counted: as one lane of a divergent warp with
-  // two divisions per k-block the issue code took ~600 cycles per 16 KB of weights - 5.2 TB/s over the chip.  With that and the gated
-  // epilogue's exponentials in front of its stores 32 x 28672 x 4096 went from 54.8 to 41.7 us (a plain read of the weights: 38.4).
+  // two divisions per k-block the issue code took ~600 cycles per 16 KB of weights - 5.2 TB/s over the chip.  With that, with the gated
+  // epilogue's values taken in front of its stores 32 x 28672 x 4096 went from 59.1 to 45.8 us, launched in a
+  // row over weights that no cache holds (a plain read of them: 38.4).
   if (warp == 0 || warp == 6) {  // ---------------- copies: weights, activations
     // weights do not depend on the previous kernel: their first stages are requested before the
     // dependency wait; the activation boxes follow once the producer kernel's writes are visible
@@ -369,7 +370,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
         } else if constexpr (EPI == EPI_SWIGLU) {
           // weight rows interleave gate_j, up_j: an even lane holds the gate, its odd neighbour the up value.  The even lane takes the
           // chunk's first half of the rows, the odd one the second; all values before the first store, the activation decided once.
-          // silu with expf and a full reciprocal, in both modes: the fast forms take 1 us less at 32 x 28672 x 4096 and 4 us at 100 rows
+          // silu with expf and a full reciprocal, in both modes: the fast forms take 0.7 us less at 32 x 28672 x 4096 and 3.5 us at 100 rows
           // but lose bits of every value, and all of them from -87.4 down.
           constexpr int HF = CJ / 2;
           const bool odd = lane & 1;
@@ -528,9 +529,10 @@ static bool adds_in_place(const TcGemmArgs& a, int sms) {
 // Tile height and K split, by the cycles of the busiest CTA: a k-block takes the issue loops ~500 cycles (fp32 mode, two parts and three
 // products: 750 - 980 with the columns; with 700 for all of them 74 x 288 x 768 took 26.7 us whole instead of 24.7 in slices, 74 x 8192 x
 // 1536 43.9 instead of 39.4), or its share of DRAM (3560 bytes per cycle for all CTAs that stream); slices that are added in place cost little, published and summed ones ~2.5 us and more
-// with each slice and row.  More tiles than SMs: the height is what makes the last round full (28672 rows: 293 tiles of 98 instead of
-// 224 of 128).  us per launch in a row of such launches, before (a split that fills the SMs, tiles of 128) -> here: 8 x 2048 x 4096
-// 12.5 -> 9.0, 8 x 2048 x 8192 13.0 -> 11.7, 32 x 28672 x 4096 swiglu 41.7 -> 39.9; over 22 shapes it is at most 7 % behind the best.
+// with each slice and row: 9 x 2048 x 4096 added in place, 1, 2, 4, 8 slices 18.0, 12.4, 10.1, 8.6 us, 9 x 2048 x 8192 28.8, 18.2, 12.4,
+// 11.5.  More tiles than SMs: the height that makes the last round full (28672 rows: 293 tiles of 98 instead of 224 of 128 - 100 rows
+// 57.5 -> 56.2 us, 32 rows 46.0 : 46.1, 9 rows 43.6 : 44.5).  Over 22 shapes (profiles/gemm_cuts.jsonl) it is 0.8 % behind the best in the
+// mean, at most 7 %.
 static void pick_swap(const TcGemmArgs& a, int bna, int sms, int* h_out, int* ks_out) {
   static const int max_split = [] { const char* v = getenv("L3_SWAP_KSPLIT"); return v ? atoi(v) : 8; }();
   static const int det_epi = [] { const char* v = getenv("L3_SWAP_KSPLIT_DET"); return v ? atoi(v) : 1; }();

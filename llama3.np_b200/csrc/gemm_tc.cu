@@ -168,8 +168,8 @@ static int sm_count() {
 // bandwidth, which the arriving tiles and the products' reads share: measured 583 cycles at 256 columns and 354 at 128 for a CTA alone,
 // 500, 390 and 275 at 256, 192 and 128 in a pair, whose CTAs hold half of the weight tile each.  The last tile's epilogue is not
 // overlapped, a split adds the partial tiles' way through L2, a pair its barrier at the start.  Any width in steps of 32 is taken, so
-// that the tiles of a shape fill the machine's last round.  Over 36 shapes of 130 - 4096 rows the choice is 0.8 % behind the best of
-// all (at most 7 %); what it gave against single CTAs and widths of 2^n, us (fp32 results; swiglu: bf16): 1462 x 2048 x 8192 66 -> 45,
+// that the tiles of a shape fill the machine's last round.  Over 40 shapes of 130 - 4096 rows (profiles/gemm_cuts.jsonl) the choice is
+// 0.8 % behind the best of all cuts in the mean, at most 5 % but for 4096 x 1024 x 1024 (16.5 : 14.5 us); what it gave against single CTAs and widths of 2^n, us (fp32 results; swiglu: bf16): 1462 x 2048 x 8192 66 -> 45,
 // 1462 x 16384 x 2048 swiglu 122 -> 73, 4096 x 28672 x 4096 swiglu 700 -> 593 (1.62 PFLOP/s), 4096 x 6144 x 4096 165 -> 138,
 // 2048 x 2048 x 8192 59 -> 51, 200 x 6144 x 4096 27 -> 20, 300 x 1024 x 1024 12.5 -> 8.5.
 static void pick_bf16(const TcGemmArgs& a, int sms, int* cg_out, int* bn_out, int* ks_out) {

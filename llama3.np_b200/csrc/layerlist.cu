@@ -1030,6 +1030,7 @@ static bool ll_takes_mirror(const L3Model* m, int rows, int N, int K);
 // products that they leave out take more than 20 us at 1.2 PFLOP/s (the masked pass over all hidden values goes as well).  2000
 // tokens of width 2048, the best 2 of 16 experts of 1024 and a shared one of 2048, us: masked 300 of products + 48 of hidden
 // values, groups 61 + 28 for the experts, 39 + 20 for the shared one, 27 for the order.
+// (Where they cannot have a workspace, prompts too long for the masked form's buffer keep that form: ll_workspaces.)
 static bool ll_moe_groups_pay(const L3Model* m, const LLLayer& Ly, int ntok) {
   const L3LayerSpec& s = Ly.spec;
   const int W = m->D, F = Ly.ff_total;

@@ -554,10 +554,11 @@ size_t recur_channel_ws_floats(int B, int L, int H, int DK, int DV) {
 
 // Portions from this length on.  A chunk's CTA takes ~13 us (gated linear attention: 264 of them in 26 us) to ~21 us (delta rule, with the
 // triangular system: 512 in 86 us, one per SM at a time) whatever it holds; the chain takes 0.2 - 0.3 us per token, and more where its
-// CTAs (a multiple of sequences x heads) fill the chip.  One layer, prompt through the public call, chain against chunks (when a CTA took
-// 20 and 39 us) in us: delta rule, 1 x 16 heads, 48 tokens 240 : 256, 96
-// 272 : 284, 128 306 : 308, 192 267 : 253, 400 347 : 284; 4 x 16 heads, 48 255 : 265, 64 278 : 269, 128 341 : 294.  Gated linear
-// attention, 1 x 2 heads, 48 tokens 152 : 158, 72 177 : 176, 96 188 : 180; 1 x 8 heads, 48 218 : 217, 64 228 : 220, 128 285 : 253.
+// CTAs (a multiple of sequences x heads) fill the chip.  One layer, prompt through the public call, chain : chunks in us: delta rule, 1 x
+// 16 heads, 48 tokens 248 : 258, 64 258 : 262, 96 283 : 281, 128 306 : 293, 192 278 : 254, 400 360 : 278; 1 x 4 heads, 64 219 : 223, 96
+// 239 : 238, 128 261 : 249; 4 x 16 heads, 32 401 : 438, 48 359 : 359, 64 376 : 367, 128 445 : 395.  Gated linear attention, 1 x 2 heads,
+// 32 152 : 154, 48 166 : 165, 64 174 : 166, 72 186 : 176, 128 215 : 189 (it would not lose from 48 on; the line is from when a chunk took
+// longer); 1 x 8 heads, 48 212 : 203, 64 218 : 203, 128 254 : 221; 4 x 8 heads, 32 341 : 348, 48 349 : 335.
 static int least_tokens(const RecurArgs& a) {
   if (a.mode == 1) return a.B * a.H >= 64 ? 64 : 128;
   return a.B * a.H >= 8 ? RECUR_CHANNEL_MIN : 72;

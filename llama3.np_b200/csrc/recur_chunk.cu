@@ -21,13 +21,16 @@
 // the column sums of its scaled keys, and n . q is q . P_n plus the row sums of A.  Keys carry a factor per token
 // (k_scale), and the decays' running sums are kept in double precision: a log decay can be as large as -30, and the
 // difference of two sums of 64 of them is what enters the exponential.
-// In bf16 mode (RecurArgs::bf16_ops, mLSTM) steps 1 and 3 run on warp-level tensor products with fp32 accumulation: queries,
-// keys and values, which are outputs of bf16 projections, are operands as they are (bf16), while everything the recurrence
-// itself makes - decayed keys, decayed scores, the states - enters as a pair hi + lo of bf16 values (16 significant bits).
+// In bf16 mode (RecurArgs::bf16_ops, mLSTM) steps 1 and 3 run on warp-level tensor products with fp32 accumulation: from 128 tokens on
+// queries, keys and values, which are outputs of bf16 projections, are rounded to bf16, while everything the recurrence
+// itself makes - decayed keys, decayed scores, the states - enters as a pair hi + lo of bf16 values (16 significant bits).  In portions of
+// 48 - 127 tokens queries, keys and values are pairs as well.
 // A chunk's products are 64 x 64 tiles with 64 .. 256 summed terms, and their operands are built in the kernel.
 // The other recurrences of bf16 mode run there as well, with queries, keys and values - which went through a silu or a convolution in
 // fp32 - as pairs too (the product of two low parts, 2^-18 of a term, is left out).  2048 tokens, 16 heads of 128 x 128, fixed decay, us,
 // FFMA tiles -> pairs: states 59 -> 25, outputs 109 -> 41; 2103 tokens, 32 heads of 128 x 64, a decay per token: 51 -> 24, 132 -> 47.
+// Error of one-layer models' logits against 64 bits, pairs over FFMA tiles, 20 - 40 seeds each at widths 512 - 2048: fixed decay 0.9998
+// +- 0.0003, 1.0001 +- 0.0001, 1.0001 +- 0.0001; a decay per token 1.0002 +- 0.0004, 1.0002 +- 0.0006; mLSTM portions 0.9995 +- 0.0002.
 // The sums run in another order than the token-by-token kernel, so the two agree to fp32 rounding, not bit for bit.
 #include <stdint.h>
 
