@@ -18,10 +18,12 @@
 // ~220 GB/s per SM: scripts/ubench, profiles/ubench.jsonl); nine compute warps consume.  Weights and cached
 // K / V do not depend on this step's activations, so the producers run ahead across phase changes.
 //
-// Math: plain fp32 FFMA.  Thread tile = 4 output features x ALL S sequences (48 accumulators) over a k-group (1/4 or
+// Math: fp32 FFMA in pairs of sequences (fma2).  Thread tile = 4 output features x ALL S sequences (48 accumulators) over a k-group (1/4 or
 // 1/8 of each slab's k rows): per k row one float4 of weights from the k-major slab (quarter warps read 128
 // contiguous bytes) and S / 4 broadcast float4s of activations from a k-major [K][S + 8] buffer (80-byte rows keep
-// the k-groups' reads in different banks) feed 48 FFMAs; k-groups are the high lane bits and are summed with shuffles.  (tcgen05 gives
+// the k-groups' reads in different banks) feed 24 pairs; k-groups are the high lane bits and are summed with shuffles, each lane ending
+// with its share of the tile.  256 sequences at position 133: 267.5 us a launch with single FFMAs and all sums in all lanes, 252.5 with
+// pairs, 236.4 with shares, the same bits.  (tcgen05 gives
 // nothing at S = 12 rows: an M = 128 MMA takes 45 cycles below N = 64 - profiles/mma_cost.jsonl -, so the three of a 3xTF32 product do
 // 128 x 12 x 8 terms in 135 cycles, 91 per cycle, where the FFMA phases reach 80 - 92, and the slabs would hold both parts, twice the
 // bytes.  At 24 rows it would be 180 per cycle: not built.  The legacy mma.sync path at 3xTF32 is 1.4x the FFMA peak.)
@@ -283,19 +285,53 @@ template <int F, int G> struct Tile {
   }
 };
 
-// One projection phase of this CTA: acc[4][S] (features 4 fg .. 4 fg + 3, every sequence) = sum over k.  The
+// Sums a tile's values over its G lanes (k-groups) and leaves each lane its 4 S / G of them: at every step a lane hands half of what it
+// holds to its partner, lowest bit of the k-group first.  42 shuffles at G = 8 and 36 at G = 4 where all sums in every lane took 144 and 96.
+//   by pairs:    lane kg ends with features 2 (kg & 1) + p of the sequences s = (G / 2) j + (kg >> 1), in own[p * 2 S / G + j]
+//   by features: lane kg of four ends with feature kg of every sequence, in own[s]
+template <bool BY_FEATURE, int S, int G, int FPW>
+__device__ __forceinline__ void sum_groups(const float2 (&sum)[4][S / 2], int kg, float (&own)[4 * S / G]) {
+  auto meet = [](bool up, float lo, float hi, int off) { return (up ? hi : lo) + __shfl_xor_sync(L3_FULL, up ? lo : hi, off); };
+  auto at = [&](int f, int s) { return s & 1 ? sum[f][s / 2].y : sum[f][s / 2].x; };
+  const bool b0 = kg & 1, b1 = kg & 2, b2 = kg & 4;
+  float r[2][S];
+#pragma unroll
+  for (int p = 0; p < 2; ++p)
+#pragma unroll
+    for (int s = 0; s < S; ++s) r[p][s] = BY_FEATURE ? meet(b0, at(2 * p, s), at(2 * p + 1, s), FPW) : meet(b0, at(p, s), at(2 + p, s), FPW);
+  if constexpr (BY_FEATURE) {
+    static_assert(G == 4, "a feature per lane");
+#pragma unroll
+    for (int s = 0; s < S; ++s) own[s] = meet(b1, r[0][s], r[1][s], 2 * FPW);
+  } else {
+    static_assert(G == 4 || G == 8, "pairs of features, every second or fourth sequence");
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      float h[S / 2];
+#pragma unroll
+      for (int j = 0; j < S / 2; ++j) h[j] = meet(b1, r[p][2 * j], r[p][2 * j + 1], 2 * FPW);
+#pragma unroll
+      for (int j = 0; j < 2 * S / G; ++j)
+        if constexpr (G == 8) own[p * (S / 4) + j] = meet(b2, h[2 * j], h[2 * j + 1], 4 * FPW);
+        else own[p * (S / 2) + j] = h[j];
+    }
+  }
+}
+
+// One projection phase of this CTA: features 4 fg .. 4 fg + 3 of every sequence = sum over k.  The
 // weights arrive as K / (ITER G) slabs of [ITER G k rows][F] floats in consecutive ring units; xt is the k-major
-// activation buffer [K][XLD].  Returns with the k-groups summed: every lane of a tile holds the full sums.
-template <class Cf, int F, int K, int G>
+// activation buffer [K][XLD].  Returns with the k-groups summed: each lane of a tile holds its share of the sums (sum_groups).
+template <class Cf, int F, int K, int G, bool BY_FEATURE>
 __device__ __forceinline__ void gemm_phase(const Ring<Cf>& rg, const uint8_t* ring, const float* xt, uint32_t& n,
-                                           float (&acc)[4][Cf::S], long long* wait_cycles = nullptr) {
+                                           float (&own)[4 * Cf::S / G], long long* wait_cycles = nullptr) {
   constexpr int S = Cf::S, QS = Cf::QS, ITER = Cf::ITER, KSLAB = ITER * G, NSLAB = K / KSLAB;
   const Tile<F, G> tl;
   const int lane = threadIdx.x & 31;
+  float2 sum[4][S / 2];  // pairs of sequences
 #pragma unroll
   for (int f = 0; f < 4; ++f)
 #pragma unroll
-    for (int s = 0; s < S; ++s) acc[f][s] = 0.f;
+    for (int s = 0; s < S / 2; ++s) sum[f][s] = make_float2(0.f, 0.f);
   const float* w0 = reinterpret_cast<const float*>(ring) + tl.kg * F + 4 * tl.fg;
   auto math = [&](int slab, uint32_t slot) {
     const float* w = w0 + (size_t)slot * (Cf::STAGE / 4);
@@ -303,16 +339,14 @@ __device__ __forceinline__ void gemm_phase(const Ring<Cf>& rg, const uint8_t* ri
 #pragma unroll
     for (int i = 0; i < ITER; ++i) {
       const float4 w4 = *reinterpret_cast<const float4*>(w + i * G * F);
+      const float2 wp[4] = {make_float2(w4.x, w4.x), make_float2(w4.y, w4.y), make_float2(w4.z, w4.z), make_float2(w4.w, w4.w)};
 #pragma unroll
       for (int q = 0; q < QS; ++q) {
         const float4 x4 = *reinterpret_cast<const float4*>(x + i * G * Cf::XLD + 4 * q);
-        const float xv[4] = {x4.x, x4.y, x4.z, x4.w};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          acc[0][4 * q + e] = fmaf(w4.x, xv[e], acc[0][4 * q + e]);
-          acc[1][4 * q + e] = fmaf(w4.y, xv[e], acc[1][4 * q + e]);
-          acc[2][4 * q + e] = fmaf(w4.z, xv[e], acc[2][4 * q + e]);
-          acc[3][4 * q + e] = fmaf(w4.w, xv[e], acc[3][4 * q + e]);
+        for (int f = 0; f < 4; ++f) {
+          sum[f][2 * q] = fma2(wp[f], make_float2(x4.x, x4.y), sum[f][2 * q]);
+          sum[f][2 * q + 1] = fma2(wp[f], make_float2(x4.z, x4.w), sum[f][2 * q + 1]);
         }
       }
     }
@@ -337,8 +371,7 @@ __device__ __forceinline__ void gemm_phase(const Ring<Cf>& rg, const uint8_t* ri
       int dep = 0;
 #pragma unroll
       for (int f = 0; f < 4; ++f)
-        asm volatile("" : "+r"(dep) : "f"(acc[f][0]), "f"(acc[f][1]), "f"(acc[f][2]), "f"(acc[f][3]), "f"(acc[f][4]), "f"(acc[f][5]),
-                     "f"(acc[f][6]), "f"(acc[f][7]), "f"(acc[f][8]), "f"(acc[f][9]), "f"(acc[f][10]), "f"(acc[f][11]));
+        asm volatile("" : "+r"(dep) : "f"(sum[f][0].x), "f"(sum[f][1].x), "f"(sum[f][2].x), "f"(sum[f][3].x), "f"(sum[f][4].x), "f"(sum[f][5].x));
       wait_cycles[4] += clock64() - tc0 + dep;
     }
     // The stages were read through the generic proxy (LDS) and will be overwritten through the async proxy
@@ -350,12 +383,7 @@ __device__ __forceinline__ void gemm_phase(const Ring<Cf>& rg, const uint8_t* ri
     if (lane < cnt) mbar_arrive_n(rg.empty((n + lane) % Cf::ST), 1);  // this warp is done with the stages
     n += (uint32_t)cnt;
   }
-#pragma unroll
-  for (int off = Tile<F, G>::FPW; off < 32; off <<= 1)
-#pragma unroll
-    for (int f = 0; f < 4; ++f)
-#pragma unroll
-      for (int s = 0; s < S; ++s) acc[f][s] += __shfl_xor_sync(L3_FULL, acc[f][s], off);
+  sum_groups<BY_FEATURE, S, G, Tile<F, G>::FPW>(sum, tl.kg, own);
 }
 
 // RMSNorm (llama3.py:111-114) of the S residual rows, in place on the k-major buffer xt[D][XLD].
@@ -407,19 +435,16 @@ __device__ __forceinline__ void rms_inplace(float* xt, const float* __restrict__
 
 // Partial sums of a row-parallel projection (Wo / Wdown restricted to this CTA's columns) go straight from the
 // registers into slot [this rank] of the receive buffer of the CTA that owns the output columns.  The (feature,
-// quad of sequences) items of a thread tile are dealt to its G lanes (every lane holds the full sums).
+// quad of sequences) items of a thread tile lie with its G lanes: feature kg with lane kg.
 template <class Cf, int F, int G>
-__device__ __forceinline__ void push_partials(const float (&acc)[4][Cf::S], uint32_t recv_local, uint32_t pbar_local, int rank) {
+__device__ __forceinline__ void push_partials(const float (&own)[Cf::S], uint32_t recv_local, uint32_t pbar_local, int rank) {
   const Tile<F, G> tl;
   static_assert(Tile<F, G>::NFG == Cf::NCW * Tile<F, G>::FPW && G == Cf::GB && F == Cf::D, "every lane of every compute warp holds a tile");
   const int f0 = 4 * tl.fg, owner = f0 / Cf::DS, fl = f0 % Cf::DS;  // DS % 4 == 0: the four features share an owner
   const uint32_t dst = mapa(recv_local, (uint32_t)owner) + (uint32_t)(((rank * Cf::DS + fl) * Cf::RLD) * 4);
 #pragma unroll
-  for (int f = 0; f < 4; ++f)
-#pragma unroll
-    for (int q = 0; q < Cf::QS; ++q)
-      if (((f + 4 * q) % G) == tl.kg)
-        st_cluster_f4(dst + (uint32_t)((f * Cf::RLD + 4 * q) * 4), acc[f][4 * q], acc[f][4 * q + 1], acc[f][4 * q + 2], acc[f][4 * q + 3]);
+  for (int q = 0; q < Cf::QS; ++q)
+    st_cluster_f4(dst + (uint32_t)((tl.kg * Cf::RLD + 4 * q) * 4), own[4 * q], own[4 * q + 1], own[4 * q + 2], own[4 * q + 3]);
   __syncwarp();
   // this warp's tiles belong to one owner or to two adjacent ones: lane 0 reports to the first, lane 1 to the second
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -639,7 +664,6 @@ __global__ void __launch_bounds__(Cf::NTHREADS, 1) decode_stack_kernel(const __g
     comp_sync<Cf>();
     SK_STAMP(a, 0);
 
-    float acc[4][S];
     for (int l = 0; l < a.NL; ++l) {
       const StackLayer ly = a.layers[l];
       long long wc[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};  // debug: thread 0's cycles waiting for ring data [0..3] / in the math [4..7], per projection
@@ -647,7 +671,8 @@ __global__ void __launch_bounds__(Cf::NTHREADS, 1) decode_stack_kernel(const __g
       // ---- q, k, v = rope(norm(x) Wqkv^T) of head `rank`; k, v -> cache          llama3.py:248, 166-187
       rms_inplace<Cf>(xt, ly.norm_in, a.eps, red, rinv);
       SK_STAMP2(a, l, 0);
-      gemm_phase<Cf, Cf::FA, Cf::KA, Cf::GA>(rg, ring, xt, n, acc, wcp);
+      float qkv[4 * S / Cf::GA];
+      gemm_phase<Cf, Cf::FA, Cf::KA, Cf::GA, false>(rg, ring, xt, n, qkv, wcp);
       SK_STAMP2(a, l, 1);
       {
         // the tile's (feature pair, sequence) items are dealt to its G lanes: lane kg rotates pair kg & 1 of the
@@ -663,9 +688,9 @@ __global__ void __launch_bounds__(Cf::NTHREADS, 1) decode_stack_kernel(const __g
           float* dst_s = region == 0 ? q_s : (region == 1 ? kn_s : vn_s);
           float* cache = region == 1 ? ly.ck : ly.cv;
 #pragma unroll
-          for (int s = 0; s < S; ++s) {
-            if ((s % (G / 2)) != sm) continue;
-            const float v0 = pr ? acc[2][s] : acc[0][s], v1 = pr ? acc[3][s] : acc[1][s];
+          for (int j = 0; j < 2 * S / G; ++j) {
+            const int s = G / 2 * j + sm;
+            const float v0 = qkv[j], v1 = qkv[2 * S / G + j];
             const float2 o = make_float2(v0 * c0 - v1 * s0, v0 * s0 + v1 * c0);
             *reinterpret_cast<float2*>(dst_s + s * HD + d) = o;
             if (region > 0 && s < s_act)  // cache append at this position (llama3.py:184-185)
@@ -826,9 +851,10 @@ __global__ void __launch_bounds__(Cf::NTHREADS, 1) decode_stack_kernel(const __g
       if (a.dbg_x) dump_kmajor<Cf>(a, l, 1, b0, s_act, rank * HD, HD, XLD, ctx_t);
       if (l < 6) SK_STAMP(a, 2 + l * 10);
       // ---- x += ctx Wo^T                                                        llama3.py:210-211, 253
-      gemm_phase<Cf, Cf::FB, Cf::KB, Cf::GB>(rg, ring, ctx_t, n, acc, wcp ? wcp + 1 : nullptr);
+      float part_sums[S];
+      gemm_phase<Cf, Cf::FB, Cf::KB, Cf::GB, true>(rg, ring, ctx_t, n, part_sums, wcp ? wcp + 1 : nullptr);
       SK_STAMP2(a, l, 7);
-      push_partials<Cf, Cf::FB, Cf::GB>(acc, smem_u32(recv), xb.pbar0 + 8 * (xb.np & 1), rank);
+      push_partials<Cf, Cf::FB, Cf::GB>(part_sums, smem_u32(recv), xb.pbar0 + 8 * (xb.np & 1), rank);
       if (l < 6) SK_STAMP(a, 3 + l * 10);
       xb.wait_p();  // all partial sums for my columns are here
       reduce_and_gather<Cf>(recv, xres, smem_u32(xt), xb.gbar0 + 8 * (xb.ng & 1), rank);
@@ -838,7 +864,8 @@ __global__ void __launch_bounds__(Cf::NTHREADS, 1) decode_stack_kernel(const __g
       // ---- h = silu(norm(x) Wgate^T) * (norm(x) Wup^T) of FFN slice `rank`          llama3.py:256, 99-101
       rms_inplace<Cf>(xt, ly.norm_post, a.eps, red, rinv);
       SK_STAMP2(a, l, 2);
-      gemm_phase<Cf, Cf::FC, Cf::KC, Cf::GC>(rg, ring, xt, n, acc, wcp ? wcp + 2 : nullptr);
+      float gu[4 * S / Cf::GC];
+      gemm_phase<Cf, Cf::FC, Cf::KC, Cf::GC, false>(rg, ring, xt, n, gu, wcp ? wcp + 2 : nullptr);
       SK_STAMP2(a, l, 3);
       {
         // features 4 fg .. 4 fg + 3 = (gate, up) of h columns 2 fg and 2 fg + 1 of this slice; lane kg takes column
@@ -849,19 +876,15 @@ __global__ void __launch_bounds__(Cf::NTHREADS, 1) decode_stack_kernel(const __g
         if (tl.active) {
           const int pr = tl.kg & 1, sm = tl.kg >> 1;
 #pragma unroll
-          for (int s = 0; s < S; ++s) {
-            if ((s % (G / 2)) != sm) continue;
-            const float gt = pr ? acc[2][s] : acc[0][s], up = pr ? acc[3][s] : acc[1][s];
-            h_t[(2 * tl.fg + pr) * XLD + s] = silu_ref(gt) * up;
-          }
+          for (int j = 0; j < 2 * S / G; ++j) h_t[(2 * tl.fg + pr) * XLD + G / 2 * j + sm] = silu_ref(gu[j]) * gu[2 * S / G + j];
         }
       }
       comp_sync<Cf>();
       if (l < 6) SK_STAMP(a, 5 + l * 10);
       // ---- x += h Wdown^T                                                        llama3.py:102, 259
-      gemm_phase<Cf, Cf::FE, Cf::KE, Cf::GE>(rg, ring, h_t, n, acc, wcp ? wcp + 3 : nullptr);
+      gemm_phase<Cf, Cf::FE, Cf::KE, Cf::GE, true>(rg, ring, h_t, n, part_sums, wcp ? wcp + 3 : nullptr);
       SK_STAMP2(a, l, 4);
-      push_partials<Cf, Cf::FE, Cf::GE>(acc, smem_u32(recv), xb.pbar0 + 8 * (xb.np & 1), rank);
+      push_partials<Cf, Cf::FE, Cf::GE>(part_sums, smem_u32(recv), xb.pbar0 + 8 * (xb.np & 1), rank);
       if (l < 6) SK_STAMP(a, 6 + l * 10);
       xb.wait_p();
       SK_STAMP2(a, l, 5);
