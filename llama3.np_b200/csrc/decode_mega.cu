@@ -41,7 +41,8 @@ constexpr int MG_THREADS = MG_CONS + 32;        // + TMA producer warp
 constexpr int MG_STAGE = 16 * 1024;
 constexpr int MG_STAGES = 10;
 constexpr int MG_XS_BYTES = MG_MAX_K * 4;
-constexpr int MG_SMEM = MG_STAGES * MG_STAGE + MG_XS_BYTES + 2 * MG_STAGES * 8 + 256 + 128;
+constexpr int MG_PLANS = 5;                     // wqkv, wo, w13, w2, LM head
+constexpr int MG_SMEM = MG_STAGES * MG_STAGE + MG_XS_BYTES + 2 * MG_STAGES * 8 + 256 + 128 + MG_PLANS * 32;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -144,8 +145,11 @@ __device__ __forceinline__ MgPlan mg_plan(int N, int K, int es) {
   return pl;
 }
 
+// The plans lie in shared memory: computed where they are used, their divisions are hoisted out of the loop over the layers and held in
+// registers that the attention phase needs (255 of them, with spills).
 struct Ring {
   uint32_t stages, full0, empty0;
+  const MgPlan* plans;
 };
 
 // ---------------------------------------------------------------------------------- producer
@@ -153,8 +157,8 @@ struct Ring {
 // src1, bytes1, off1)`: one contiguous range (several whole row pairs) or two (a chunk of each
 // row of a pair; the second lands off1 bytes into the stage).
 template <typename Issue>
-__device__ __forceinline__ void walk_matrix(const void* W, int N, int K, int es, uint32_t& n, Issue&& issue) {
-  const MgPlan pl = mg_plan(N, K, es);
+__device__ __forceinline__ void walk_matrix(const MgPlan& plan, const void* W, int K, int es, uint32_t& n, Issue&& issue) {
+  const MgPlan pl = plan;
   const char* Wb = (const char*)W;
   if (pl.C == 1) {
     for (int u = 0; u < pl.nunits; ++u, ++n) {
@@ -178,21 +182,20 @@ __device__ __forceinline__ void walk_matrix(const void* W, int N, int K, int es,
 }
 
 template <typename Issue>
-__device__ __forceinline__ void walk_step(const MegaArgs& a, int es, bool stamp, Issue&& issue) {
-  const int qkv_rows = (a.HN + 2 * a.KVHN) * a.HD;
+__device__ __forceinline__ void walk_step(const MegaArgs& a, const MgPlan* plans, int es, bool stamp, Issue&& issue) {
   uint32_t n = 0;
   for (int l = 0; l < a.NL; ++l) {
     const MegaLayer& ly = a.layers[l];
-    walk_matrix(ly.wqkv, qkv_rows, a.D, es, n, issue);
+    walk_matrix(plans[0], ly.wqkv, a.D, es, n, issue);
     if (stamp && l < 32) MG_STAMP(a, 384 + l * 4 + 0);
-    walk_matrix(ly.wo, a.D, a.HN * a.HD, es, n, issue);
+    walk_matrix(plans[1], ly.wo, a.HN * a.HD, es, n, issue);
     if (stamp && l < 32) MG_STAMP(a, 384 + l * 4 + 1);
-    walk_matrix(ly.w13, 2 * a.FD, a.D, es, n, issue);
+    walk_matrix(plans[2], ly.w13, a.D, es, n, issue);
     if (stamp && l < 32) MG_STAMP(a, 384 + l * 4 + 2);
-    walk_matrix(ly.w2, a.D, a.FD, es, n, issue);
+    walk_matrix(plans[3], ly.w2, a.FD, es, n, issue);
     if (stamp && l < 32) MG_STAMP(a, 384 + l * 4 + 3);
   }
-  walk_matrix(a.lm_head, a.VS, a.D, es, n, issue);
+  walk_matrix(plans[4], a.lm_head, a.D, es, n, issue);
 }
 
 // A consumer warp waits for ring unit n.  Stages of one slot are consumed by DIFFERENT warps, so a
@@ -285,9 +288,9 @@ __device__ __forceinline__ void mg_epilogue(const MegaArgs& a, const MegaLayer& 
 // One projection phase for the consumer warps: y = W xs with the fused epilogue.
 template <typename WT, typename KVT, int EPI>
 __device__ __forceinline__ void consume_matrix(const MegaArgs& a, const MegaLayer& ly, const Ring& rg, const uint8_t* ring,
-                                               const float* xs, int N, int K, int pos, uint32_t& nbase, Best& best,
+                                               const float* xs, int which, int K, int pos, uint32_t& nbase, Best& best,
                                                unsigned tp_next = 0) {
-  const MgPlan pl = mg_plan(N, K, (int)sizeof(WT));
+  const MgPlan pl = rg.plans[which];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (pl.C == 1) {
     for (int u = warp; u < pl.nunits; u += MG_NW) {
@@ -594,13 +597,19 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
     for (int s = 0; s < MG_STAGES; ++s) { mbar_init(rg.full0 + 8 * s, 1); mbar_init(rg.empty0 + 8 * s, 1); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  MgPlan* plans = reinterpret_cast<MgPlan*>(red + 64);
+  static_assert(sizeof(MgPlan) <= 32, "room for the plans");
+  if (threadIdx.x < MG_PLANS) {
+    const int w = threadIdx.x;
+    plans[w] = mg_plan(w == 0 ? (a.HN + 2 * a.KVHN) * a.HD : w == 2 ? 2 * a.FD : w == 4 ? a.VS : a.D, w == 1 ? a.HN * a.HD : w == 3 ? a.FD : a.D, ES);
+  }
+  rg.plans = plans;
   __syncthreads();
 
-  const int qkv_rows = (a.HN + 2 * a.KVHN) * a.HD;
   if (threadIdx.x >= MG_CONS) {
     if (threadIdx.x == MG_CONS) {
       // ================================================================ TMA producer (warp 7)
-      walk_step(a, ES, true, [&](uint32_t n, const char* s0, uint32_t b0, const char* s1, uint32_t b1, uint32_t off1) {
+      walk_step(a, plans, ES, true, [&](uint32_t n, const char* s0, uint32_t b0, const char* s1, uint32_t b1, uint32_t off1) {
         const uint32_t slot = n % MG_STAGES, use = n / MG_STAGES;
         if (use > 0) mbar_wait(rg.empty0 + 8 * slot, (use - 1) & 1);
         mbar_expect_tx(rg.full0 + 8 * slot, b0 + b1);
@@ -634,7 +643,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
     else
       stage_sum(a, tp_epoch, xs, red, a.D, ly.norm_in, a.eps);
     if (tid == 0 && l < 24) MG_STAMP(a, l * 16 + 0);   // activations staged
-    consume_matrix<WT, KVT, EPI_ROPE_KV>(a, ly, rg, ring, xs, qkv_rows, a.D, pos, nbase, best);
+    consume_matrix<WT, KVT, EPI_ROPE_KV>(a, ly, rg, ring, xs, 0, a.D, pos, nbase, best);
     grid_sync(a, gb, l < 24 ? l * 16 + 1 : 512);
     // ---- ctx = softmax(q k^T / sqrt(HD)) v over keys [0, pos]              llama3.py:190-207
     {
@@ -658,24 +667,24 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
     // ---- x += ctx Wo^T                                                    llama3.py:210-211, 253
     stage_tagged(a.ll_ctx, tp_epoch + 1, xs, a.HN * a.HD);
     if (tid == 0 && l < 24) MG_STAMP(a, l * 16 + 5);
-    consume_matrix<WT, KVT, EPI_RESID>(a, ly, rg, ring, xs, a.D, a.HN * a.HD, pos, nbase, best, tp_epoch + 1);
+    consume_matrix<WT, KVT, EPI_RESID>(a, ly, rg, ring, xs, 1, a.HN * a.HD, pos, nbase, best, tp_epoch + 1);
     // ---- h = silu(norm(x) Wgate^T) * (norm(x) Wup^T)                      llama3.py:256, 99-101
     // no grid barrier: the staging waits for the tagged values themselves
     if (tid == 0 && l < 24) { MG_STAMP(a, l * 16 + 6); MG_STAMP(a, l * 16 + 7); }
     stage_sum(a, ++tp_epoch, xs, red, a.D, ly.norm_post, a.eps);
     if (tid == 0 && l < 24) MG_STAMP(a, l * 16 + 8);
-    consume_matrix<WT, KVT, EPI_SWIGLU>(a, ly, rg, ring, xs, 2 * a.FD, a.D, pos, nbase, best);
+    consume_matrix<WT, KVT, EPI_SWIGLU>(a, ly, rg, ring, xs, 2, a.D, pos, nbase, best);
     grid_sync(a, gb, l < 24 ? l * 16 + 9 : 512);
     // ---- x += h Wdown^T                                                   llama3.py:102, 259
     stage_x(xs, red, xst, a.h, a.FD, nullptr, 0.f);
     if (tid == 0 && l < 24) MG_STAMP(a, l * 16 + 11);
-    consume_matrix<WT, KVT, EPI_RESID>(a, ly, rg, ring, xs, a.D, a.FD, pos, nbase, best, tp_epoch + 1);
+    consume_matrix<WT, KVT, EPI_RESID>(a, ly, rg, ring, xs, 3, a.FD, pos, nbase, best, tp_epoch + 1);
     if (tid == 0 && l < 24) { MG_STAMP(a, l * 16 + 12); MG_STAMP(a, l * 16 + 13); }
     ++tp_epoch;  // summed by the next staging (layer l + 1 or the head)
   }
   // ---- next = argmax(norm(x) lm_head^T)                                   llama3.py:304-307, 320
   stage_sum(a, tp_epoch, xs, red, a.D, a.norm_final, a.eps);
-  consume_matrix<WT, KVT, EPI_ARGMAX>(a, a.layers[0], rg, ring, xs, a.VS, a.D, pos, nbase, best);
+  consume_matrix<WT, KVT, EPI_ARGMAX>(a, a.layers[0], rg, ring, xs, 4, a.D, pos, nbase, best);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float ov = __shfl_xor_sync(L3_FULL, best.v, o);
