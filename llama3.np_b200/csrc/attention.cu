@@ -20,6 +20,8 @@
 #include "attn_decode.cuh"
 #include "common.cuh"
 #include "gemm_tc.h"
+#include "mixer.h"
+#include "../../include/llama3_b200.h"
 
 bool attn_decode_mma_eligible(int HD, int nrep, bool kv_bf16) {
   static const bool mma_on = !(getenv("L3_ATTN_MMA") && atoi(getenv("L3_ATTN_MMA")) == 0);
@@ -767,7 +769,7 @@ __global__ void __launch_bounds__(256) attn_prefill64_kernel(AttnArgs a, int nre
 template <int HD, typename KVT>
 static cudaError_t launch_prefill_hd(const AttnArgs& a, cudaStream_t s) {
   static const int big_min = [] { const char* v = getenv("L3_ATTN_PF64_MIN"); return v ? atoi(v) : 48; }();
-  if (big_min > 0 && a.L >= big_min) {  // long prompts: the 64 x 64 tiling
+  if constexpr (sizeof(KVT) == 2) if (big_min > 0 && a.L >= big_min) {  // long prompts: the 64 x 64 tiling
     auto kern = attn_prefill64_kernel<HD, KVT>;
     const size_t smem = (size_t)(PF2_ROWS * HD + PF2_TK * (HD + 4) + PF2_TK * HD + PF2_ROWS * PF2_LDS) * sizeof(float);
     if (smem > 48 * 1024) {
@@ -801,5 +803,16 @@ static cudaError_t launch_prefill_t(const AttnArgs& a, cudaStream_t s) {
 }
 
 cudaError_t launch_attn_prefill(const AttnArgs& a, bool kv_bf16, cudaStream_t s) {
+  // fp32 caches: the 32-row tiles of attn_f32.cu from two tiles a head or four waves of CTAs on.  Six heads of 48, whole prompts, us with the
+  // 16- and 64-row tiles here : there: one sequence, 16 tokens 328 : 351, 32 370 : 396, 48 551 : 536, 64 556 : 541, 100 760 : 714; eight, 32
+  // 528 : 539, 48 556 : 542, 64 587 : 568; 256, 5 tokens 2594 : 2446, 32 3494 : 3327, 64 5115 : 4907.
+  if (!kv_bf16 && (a.L > 32 || (long)a.B * a.KVHN >= 4 * 148)) {
+    WinAttnArgs w{};
+    w.q = a.q; w.cache_k = a.cache_k; w.cache_v = a.cache_v; w.out = a.out; w.out_lo = a.out_lo; w.out16 = a.out_bf16; w.ld_out = a.HN * a.HD;
+    w.out_scale = 1.f; w.gate = a.head_gate; w.ld_gate = a.ld_gate; w.pos_ptr = a.pos_ptr; w.kind = L3_ATTN_SOFTMAX;
+    w.scale = a.scale != 0.f ? a.scale : 1.0f / sqrtf((float)a.HD);
+    w.B = a.B; w.L = a.L; w.H = a.HN; w.G = a.KVHN; w.DK = w.DV = a.HD; w.M = a.M; w.nsplit = 1;
+    return launch_attn_f32(w, s);
+  }
   return kv_bf16 ? launch_prefill_t<bf16>(a, s) : launch_prefill_t<float>(a, s);
 }

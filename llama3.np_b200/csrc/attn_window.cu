@@ -14,7 +14,8 @@
 //                        4 floats), in the output phase a lane owns value columns read as 16-byte pieces while the weights
 //                        arrive as 16-byte broadcasts.  Softmax rows run the online form,
 //                        started at (max = sink, sum = 1) so that the sink needs no key; sigmoid rows just accumulate.
-//                        Calls of few tokens split the key tiles over CTAs (win_attn_combine_kernel merges).
+//                        Calls of few tokens split the key tiles over CTAs (win_attn_combine_kernel merges).  Prompts over fp32
+//                        caches run attn_f32.cu.
 //  * win_decode_kernel   one token per sequence, groups of 1, 2, 4 or 8 query heads: a CTA per (key split, key head, sequence).
 //                        Four threads per key score it for all heads of the group, a warp per head turns the scores into
 //                        weights, and the values - requested together with the keys - are summed by (16-byte column piece,
@@ -648,6 +649,9 @@ cudaError_t launch_win_attn(const WinAttnArgs& a, bool kv_bf16, cudaStream_t s) 
   // 16-byte pieces of every row
   if (a.k_ld && ((((uintptr_t)a.cache_k | (uintptr_t)a.cache_v | (uintptr_t)a.k2) & 15) || a.k_ld % 8 || a.k2_ld % 8 || a.DK % 8 || a.dk2 % 8 || a.DV % 8))
     return cudaErrorInvalidValue;
+  // Prompts over fp32 caches; win_attn_kernel keeps rows that are not whole 16-byte pieces and the key splits of calls of few tokens.  Never
+  // slower over 9 - 400 tokens, widths 512 and 1024: debuzen 64 tokens 506 : 511, 130 644 : 625, 400 1007 : 954; vupitar 400 681 : 609.
+  if (!kv_bf16 && attn_f32_supported(a)) return launch_attn_f32(a, s);
   const int rep = a.H / a.G;
   const dim3 grid((a.L * rep + WA_ROWS - 1) / WA_ROWS, a.G, a.B * a.nsplit);
   cudaError_t e = kv_bf16 ? launch_win_t<bf16>(a, grid, s) : launch_win_t<float>(a, grid, s);

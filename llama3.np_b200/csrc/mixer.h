@@ -407,8 +407,12 @@ struct WinAttnArgs {
   int gate_wide;         // 1: the gate has an entry per value, gate[r * ld_gate + h * DV + d] (win_attn_kernel without splits)
   int nsplit;            // > 1: the key tiles of a query spread over that many CTAs; partials in part_o / part_ml
   float *part_o, *part_ml;
+  float* out_lo;         // attn_f32.cu: if set, out receives the TF32 hi part and out_lo the rest
 };
 bool win_attn_supported(int DK, int DV);
+// prompts over fp32 caches whose rows are whole 16-byte pieces (attn_f32.cu)
+bool attn_f32_supported(const WinAttnArgs& a);
+cudaError_t launch_attn_f32(const WinAttnArgs& a, cudaStream_t s);
 int win_attn_splits(int B, int L, int H, int G, int window, int keep_first, int max_keys, int max_split);
 size_t win_attn_part_floats(int max_rows, int H, int DV, int max_split);
 cudaError_t launch_win_attn(const WinAttnArgs& a, bool kv_bf16, cudaStream_t s);
