@@ -30,6 +30,8 @@ struct ClusterHeadArgs {             // next = argmax(norm(x) W^T), then the ste
   int32_t* d_next;
   int64_t* d_tokens;                 // [B, M]
   int* scal;
+  float* logits;                     // [B, VS]: the logits in place of argmax and bookkeeping (null: these)
+  int* err;                          // as ClusterArgs::err
 };
 // most sequences a step can take, 0: the shape or the device is not one for it
 int decode_cluster_max_batch(int NL, int D, int HN, int KVHN, int HD, int FD, int M);

@@ -440,16 +440,35 @@ __global__ void __launch_bounds__(TH, 1) decode_cluster_kernel(const __grid_cons
   if (!ok) __nanosleep(1000000);  // what this CTA did not wait for lands before its shared memory is given up
 }
 
-// LM head and argmax: four rows of W per warp and turn, eight lanes per row; the CTA that finishes last settles the step.  Bound by the
-// stream of W (stories15M: 37 MB, from L2 where it stayed).
-template <int NB>
-__global__ void __launch_bounds__(256) cluster_head_kernel(ClusterHeadArgs a) {
-  extern __shared__ __align__(16) float xs[];  // [NB][D]
-  __shared__ unsigned long long s_best[8][NB];
+// LM head: its argmax and the step's bookkeeping, or (LOGITS) the logits.  The layers ahead of it run on 16 SMs; on the others this kernel is
+// resident meanwhile, one CTA each, and draws its rows of W into shared memory (stories15M: 190 of 243 rows, 26 of 37 MB; the rest is asked
+// into L2).  Behind the wait there is the norm of x, a pass over shared memory and the merge of the maxima.  Four rows per warp and turn,
+// eight lanes per row.  stories15M, one sequence: from the layers' end to the step's 10.9 -> 8.3 us (a wait, three passes of few microseconds,
+// two rounds of atomics), a forward step with its logits 125.5 -> 113.5 us.
+constexpr int HT = 512, HW = HT / 32;
+template <int NB, bool LOGITS>
+__global__ void __launch_bounds__(HT, 1) cluster_head_kernel(ClusterHeadArgs a, int keep) {
+  extern __shared__ __align__(16) float sh[];  // [keep][D] rows of W | [NB][D] normed x
+  __shared__ unsigned long long s_best[HW][NB];
+  __shared__ __align__(8) unsigned long long s_bar;
   __shared__ int s_last;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = lane & 7;
+  float* xs = sh + (size_t)keep * a.D;
+  const int r_lo = (int)((long long)a.VS * blockIdx.x / gridDim.x), r_hi = (int)((long long)a.VS * (blockIdx.x + 1) / gridDim.x);
+  const int n_s = min(keep, r_hi - r_lo);
+  const float* W = a.w + (size_t)r_lo * a.D;
+  const uint32_t bar = s32(&s_bar);
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    bar_arm(bar, (uint32_t)(n_s * a.D * 4));
+    const int piece = max(1, 4096 / a.D);  // rows per copy
+    for (int r = 0; r < n_s; r += piece) bulk_load(sh + (size_t)r * a.D, W + (size_t)r * a.D, min(piece, n_s - r) * a.D, bar);
+    for (int r = n_s; r < r_hi - r_lo; r += piece) l2_prefetch_bulk(W + (size_t)r * a.D, (uint32_t)(min(piece, r_hi - r_lo - r) * a.D * 4));
+  }
+  __syncthreads();
   pdl_launch();
-  pdl_wait();
+  pdl_wait();  // W is constant; x comes from the kernel before
 #pragma unroll
   for (int b = 0; b < NB; ++b) {
     const float* x = a.x + (size_t)min(b, a.B - 1) * a.D;
@@ -459,21 +478,22 @@ __global__ void __launch_bounds__(256) cluster_head_kernel(ClusterHeadArgs a) {
       ss = fmaf(v.x, v.x, ss); ss = fmaf(v.y, v.y, ss); ss = fmaf(v.z, v.z, ss); ss = fmaf(v.w, v.w, ss);
     }
     const float rinv = 1.0f / sqrtf(warp_sum(ss) / (float)a.D + a.eps);
-    for (int i = tid; i < a.D; i += 256) xs[b * a.D + i] = x[i] * rinv * a.norm[i];
+    for (int i = tid; i < a.D; i += HT) xs[b * a.D + i] = x[i] * rinv * a.norm[i];
   }
+  const bool ok = bar_wait(bar, 0, true);
   __syncthreads();
   unsigned long long best[NB];
 #pragma unroll
   for (int b = 0; b < NB; ++b) best[b] = 0ull;
-  for (int r0 = (blockIdx.x * 8 + warp) * 4; r0 < a.VS; r0 += gridDim.x * 32) {
-    const int row = r0 + (lane >> 3);
-    const float* w = a.w + (size_t)min(row, a.VS - 1) * a.D;
+  auto four_rows = [&](const float* rows, int r0, int end, auto load) {  // rows r0 .. r0 + 3 of this CTA's, those below `end`
+    const int r = r0 + (lane >> 3);
+    const float* w = rows + (size_t)min(r, end - 1) * a.D;
     float acc[NB];
 #pragma unroll
     for (int b = 0; b < NB; ++b) acc[b] = 0.f;
 #pragma unroll 9
     for (int k = sub * 4; k < a.D; k += 32) {
-      const float4 wv = __ldg(reinterpret_cast<const float4*>(w + k));
+      const float4 wv = load(w + k);
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
         const float4 xv = *reinterpret_cast<const float4*>(xs + b * a.D + k);
@@ -486,43 +506,55 @@ __global__ void __launch_bounds__(256) cluster_head_kernel(ClusterHeadArgs a) {
       float t = acc[b];
 #pragma unroll
       for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(L3_FULL, t, o);
-      const unsigned long long key = row < a.VS && t == t ? argmax_key(t, row) : 0ull;
-      best[b] = key > best[b] ? key : best[b];
+      if (LOGITS) {
+        if (sub == 0 && r < end && b < a.B) a.logits[(size_t)b * a.VS + r_lo + r] = t;
+      } else {
+        const unsigned long long key = r < end && t == t ? argmax_key(t, r_lo + r) : 0ull;
+        best[b] = key > best[b] ? key : best[b];
+      }
     }
+  };
+  for (int r0 = n_s + warp * 4; r0 < r_hi - r_lo; r0 += HW * 4) four_rows(W, r0, r_hi - r_lo, [](const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); });
+  for (int r0 = warp * 4; r0 < n_s; r0 += HW * 4) four_rows(sh, r0, n_s, [](const float* p) { return *reinterpret_cast<const float4*>(p); });
+  if (!ok) {  // gave up: the host finds the error word; what is in flight lands before the shared memory is given up
+    *a.err = 1;
+    __nanosleep(1000000);
   }
+  if constexpr (!LOGITS) {
 #pragma unroll
-  for (int b = 0; b < NB; ++b) {
+    for (int b = 0; b < NB; ++b) {
 #pragma unroll
-    for (int o = 16; o >= 8; o >>= 1) {
-      const unsigned long long k = __shfl_xor_sync(L3_FULL, best[b], o);
-      best[b] = k > best[b] ? k : best[b];
+      for (int o = 16; o >= 8; o >>= 1) {
+        const unsigned long long k = __shfl_xor_sync(L3_FULL, best[b], o);
+        best[b] = k > best[b] ? k : best[b];
+      }
+      if (lane == 0) s_best[warp][b] = best[b];
     }
-    if (lane == 0) s_best[warp][b] = best[b];
+    __syncthreads();
+    if (tid < NB && tid < a.B) {
+      unsigned long long k = 0ull;
+      for (int w = 0; w < HW; ++w) k = s_best[w][tid] > k ? s_best[w][tid] : k;
+      if (k) atomicMax(a.best + tid, k);
+      __threadfence();
+    }
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();
+      s_last = atomicAdd(a.done, 1) == (int)gridDim.x - 1;
+      __threadfence();
+    }
+    __syncthreads();
+    if (!s_last) return;
+    const int step = a.scal[1] + 1, pos = a.scal[2] + step;
+    __syncthreads();
+    if (tid < a.B) {
+      const unsigned long long k = atomicExch(a.best + tid, 0ull);
+      const int idx = k ? (int)(0xffffffffu - (uint32_t)(k & 0xffffffffull)) : 0;
+      a.d_next[tid] = idx;
+      a.d_tokens[(size_t)tid * a.M + step] = (int64_t)idx;
+    }
+    if (tid == 0) { a.scal[1] = step; a.scal[0] = pos; *a.done = 0; }
   }
-  __syncthreads();
-  if (tid < NB && tid < a.B) {
-    unsigned long long k = 0ull;
-    for (int w = 0; w < 8; ++w) k = s_best[w][tid] > k ? s_best[w][tid] : k;
-    if (k) atomicMax(a.best + tid, k);
-    __threadfence();
-  }
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    s_last = atomicAdd(a.done, 1) == (int)gridDim.x - 1;
-    __threadfence();
-  }
-  __syncthreads();
-  if (!s_last) return;
-  const int step = a.scal[1] + 1, pos = a.scal[2] + step;
-  __syncthreads();
-  if (tid < a.B) {
-    const unsigned long long k = atomicExch(a.best + tid, 0ull);
-    const int idx = k ? (int)(0xffffffffu - (uint32_t)(k & 0xffffffffull)) : 0;
-    a.d_next[tid] = idx;
-    a.d_tokens[(size_t)tid * a.M + step] = (int64_t)idx;
-  }
-  if (tid == 0) { a.scal[1] = step; a.scal[0] = pos; *a.done = 0; }
 }
 
 int batch_slots(int B) { return B <= 1 ? 1 : B <= 2 ? 2 : B <= 4 ? 4 : 8; }
@@ -592,14 +624,28 @@ cudaError_t launch_decode_cluster(const ClusterArgs& a, cudaStream_t s) {
   }
 }
 
+template <int NB, bool LOGITS>
+static cudaError_t launch_head_t(const ClusterHeadArgs& a, int n_sm, cudaStream_t s) {
+  constexpr int ROOM = 220 * 1024;  // beside 16 x NB + 16 bytes of static shared memory
+  static bool done[16] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!done[dev & 15]) {
+    const cudaError_t e = cudaFuncSetAttribute(cluster_head_kernel<NB, LOGITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROOM);
+    if (e != cudaSuccess) return e;
+    done[dev & 15] = true;
+  }
+  const int row = a.D * 4, grid = std::max(1, std::min(n_sm > 2 * CL ? n_sm - CL : n_sm, (a.VS + 3) / 4)), most = (a.VS + grid - 1) / grid;
+  const int keep = std::min((most + 3) / 4 * 4, (ROOM - NB * row) / row / 4 * 4);
+  return launch_k(cluster_head_kernel<NB, LOGITS>, dim3(grid), dim3(HT), (size_t)(keep + NB) * row, s, a, keep);
+}
+
 cudaError_t launch_cluster_head(const ClusterHeadArgs& a, int n_sm, cudaStream_t s) {
-  const int nb = batch_slots(a.B);
-  const dim3 grid(std::max(1, std::min(4 * n_sm, (a.VS + 31) / 32)));
-  const size_t smem = (size_t)nb * a.D * 4;
-  switch (nb) {
-    case 1: return launch_k(cluster_head_kernel<1>, grid, dim3(256), smem, s, a);
-    case 2: return launch_k(cluster_head_kernel<2>, grid, dim3(256), smem, s, a);
-    case 4: return launch_k(cluster_head_kernel<4>, grid, dim3(256), smem, s, a);
-    default: return launch_k(cluster_head_kernel<8>, grid, dim3(256), smem, s, a);
+  const bool lg = a.logits != nullptr;
+  switch (batch_slots(a.B)) {
+    case 1: return lg ? launch_head_t<1, true>(a, n_sm, s) : launch_head_t<1, false>(a, n_sm, s);
+    case 2: return lg ? launch_head_t<2, true>(a, n_sm, s) : launch_head_t<2, false>(a, n_sm, s);
+    case 4: return lg ? launch_head_t<4, true>(a, n_sm, s) : launch_head_t<4, false>(a, n_sm, s);
+    default: return lg ? launch_head_t<8, true>(a, n_sm, s) : launch_head_t<8, false>(a, n_sm, s);
   }
 }

@@ -751,6 +751,15 @@ static int enqueue_chunk(L3Model* m, const int32_t* d_ids, int ids_ld, int ids_o
   }
   if (want_logits || want_argmax) {
     // logits = norm(x)[:, -1] @ lm_head^T                         llama3.py:304-307
+    if (in_cluster) {
+      ClusterHeadArgs h{};
+      h.x = m->x; h.w = (const float*)m->lm_head; h.norm = m->norm_final; h.eps = m->cfg.norm_eps; h.B = B; h.D = D; h.VS = m->VS; h.M = m->M;
+      h.logits = m->logits; h.err = m->h_err;
+      g_l3_pdl_next = !(m->cfg.flags & L3_FLAG_NO_PDL);
+      LAUNCH(m, launch_cluster_head(h, m->n_sm, m->stream));
+      if (want_argmax) LAUNCH(m, launch_argmax(m->logits, B, m->VS, os.next, os.out64, os.stride, os.step_ptr, m->stream));
+      return L3_OK;
+    }
     LinearArgs a{};
     a.W = m->lm_head; a.x = m->x; a.rows = B; a.N = m->VS; a.K = D;
     a.norm_w = m->norm_final; a.eps = m->cfg.norm_eps; a.src_mul = L; a.src_add = L - 1;
@@ -978,7 +987,7 @@ static int enqueue_decode_nodes(L3Model* m, int B, int ragged, int eos) {
     if (rc != L3_OK) return rc;
     ClusterHeadArgs h{};
     h.x = m->x; h.w = (const float*)m->lm_head; h.norm = m->norm_final; h.eps = m->cfg.norm_eps; h.B = B; h.D = m->D; h.VS = m->VS; h.M = m->M;
-    h.best = m->d_best; h.done = m->d_cl_done; h.d_next = m->d_next; h.d_tokens = m->d_tokens; h.scal = m->d_scal;
+    h.best = m->d_best; h.done = m->d_cl_done; h.d_next = m->d_next; h.d_tokens = m->d_tokens; h.scal = m->d_scal; h.err = m->h_err;
     g_l3_pdl_next = !(m->cfg.flags & L3_FLAG_NO_PDL);
     LAUNCH(m, launch_cluster_head(h, m->n_sm, m->stream));
     return L3_OK;

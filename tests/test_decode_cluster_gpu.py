@@ -112,3 +112,22 @@ def test_a_wait_that_ran_out_is_reported():
     m = Llama(w, args, flags=_cabi.FLAG_NO_MEGA)   # no kernel of this handle has such a wait
     assert _cabi.lib().l3_debug_fail_wait(m._h) == -1
     m.close()
+
+
+@pytest.mark.parametrize("B", [1, 3, 8])
+@pytest.mark.parametrize("vocab", [5, 531, 26003])
+def test_head_of_every_vocabulary_size(vocab, B):
+    """The LM head behind the layers: fewer rows than CTAs, a few rows each, and more rows than shared memory holds (26003 x 288 x 4 bytes
+    over 132 CTAs: 220 KB); logits of a forward step and greedy tokens.  Bound as above."""
+    args = ModelArgs(dim=288, n_layers=1, n_heads=6, n_kv_heads=6, vocab_size=vocab, max_seq_len=40, max_batch_size=B)
+    w = make_weights(args, 768, seed=7)
+    ids = np.random.default_rng(vocab).integers(0, vocab, (B, 9))
+    m, o = Llama(w, args), orc.OracleLlama(w, args)
+    for p, q in ((0, 8), (8, 9)):
+        want = np.asarray(o(ids[:, p:q], p))
+        np.testing.assert_allclose(np.asarray(m(ids[:, p:q], p)), want, rtol=0, atol=5e-5 * np.abs(want).max())
+    m.reset_cache()
+    got = np.concatenate(list(m.generate(ids, 30)), axis=1)
+    want = np.concatenate(list(orc.OracleLlama(w, args).generate(ids, 30)), axis=1)
+    m.close()
+    assert np.array_equal(got, want)
