@@ -164,6 +164,17 @@ __global__ void __launch_bounds__(256) win_prep_kernel(WinPrepArgs a) {
   }
 }
 
+__device__ __forceinline__ float ld_cluster(const float* p, int rank) {  // the same place in another CTA of the cluster
+  uint32_t a;
+  float v;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.0f / (1.0f + expf(-z)); }
 
 // One row of a key / value tile from the cache into shared memory as floats: `n` values (dst padded with zeros up to np).
@@ -376,7 +387,10 @@ __global__ void __launch_bounds__(256) win_attn_kernel(WinAttnArgs a) {
 
 constexpr int WD_KEYS = 64, WD_KV = 8, WD_VV = 8;  // keys per tile; 16-byte pieces of a key / keys of a value part per thread
 
-template <typename KVT, int REP>
+// CL: the key splits of a (key head, sequence) are a cluster and merge their sums through its shared memory, in the order and with the
+// roundings of win_attn_combine_kernel, whose launch they save: 6.5 us a layer (8 sequences, 4 key heads, 4 splits), where the merge adds 1.5.
+// 32 greedy tokens of 8 sequences of the two-layer vupitar stack, with the router's early loads (moe.cu): 6006 -> 5675 us.
+template <typename KVT, int REP, bool CL>
 __global__ void __launch_bounds__(256) win_decode_kernel(WinAttnArgs a) {
   constexpr int VEC = Vec16<KVT>::N;
   extern __shared__ __align__(16) float sm[];
@@ -501,11 +515,13 @@ __global__ void __launch_bounds__(256) win_decode_kernel(WinAttnArgs a) {
     for (int x = 0; x < VEC; x += 4)
       *reinterpret_cast<float4*>(sR + ((size_t)vp * REP + r) * a.DV + vc * VEC + x) = make_float4(acc[r][x], acc[r][x + 1], acc[r][x + 2], acc[r][x + 3]);
   __syncthreads();
+  float* sT = sR + (size_t)parts * REP * a.DV;  // CL: [REP][DV] this split's sums | [REP][8] the splits' weights | [REP] their sum
   for (int i = tid; i < REP * a.DV; i += 256) {
     const int r = i / a.DV, d = i - r * a.DV, h = g * REP + r;
     float t = 0.f;
 #pragma unroll 8
     for (int q = 0; q < parts; ++q) t += sR[((size_t)q * REP + r) * a.DV + d];
+    if (CL) { sT[i] = t; continue; }
     const size_t rh = (size_t)b * a.H + h;
     if (a.nsplit > 1) {
       const size_t pi = rh * a.nsplit + split;
@@ -518,6 +534,35 @@ __global__ void __launch_bounds__(256) win_decode_kernel(WinAttnArgs a) {
     const size_t oi = (size_t)b * a.ld_out + (size_t)h * a.DV + d;
     if (a.out) a.out[oi] = t * mul;
     if (a.out16) a.out16[oi] = __float2bfloat16_rn(t * mul);
+  }
+  if constexpr (CL) {
+    float *sF = sT + REP * a.DV, *sD = sF + REP * 8;
+    cluster_sync_all();
+    if (warp < REP) {  // a lane per split
+      const bool on = lane < a.nsplit;
+      const float m = on ? ld_cluster(sM + warp, lane) : -INFINITY, l = on ? ld_cluster(sM + REP + warp, lane) : 0.f;
+      float f = 1.f, den = 1.f;
+      if (a.kind != L3_ATTN_SIGMOID) {
+        const float M = warp_max(m);
+        f = m == -INFINITY ? 0.f : expf(m - M);
+        den = warp_sum(f * l);
+      }
+      if (on) sF[warp * 8 + lane] = f;
+      if (lane == 0) sD[warp] = den;
+    }
+    __syncthreads();
+    const int per = (REP * a.DV + a.nsplit - 1) / a.nsplit, end = min(REP * a.DV, (split + 1) * per);
+    for (int i = split * per + tid; i < end; i += 256) {
+      const int r = i / a.DV, d = i - r * a.DV, h = g * REP + r;
+      float mul = a.out_scale * (sD[r] > 0.f ? 1.0f / sD[r] : 0.f);
+      if (a.gate) mul *= sigmoid_f(a.gate[(size_t)b * a.ld_gate + h]);
+      float acc = 0.f;
+      for (int s = 0; s < a.nsplit; ++s) acc = fmaf(ld_cluster(sT + i, s), sF[r * 8 + s], acc);
+      const size_t oi = (size_t)b * a.ld_out + (size_t)h * a.DV + d;
+      if (a.out) a.out[oi] = acc * mul;
+      if (a.out16) a.out16[oi] = __float2bfloat16_rn(acc * mul);
+    }
+    cluster_sync_all();  // nobody leaves while a peer reads its sums
   }
 }
 
@@ -573,6 +618,10 @@ cudaError_t launch_win_nj(const WinAttnArgs& a, dim3 grid, cudaStream_t s) {
   return launch_k(win_attn_kernel<KVT, NJ>, grid, dim3(256), smem, s, a);
 }
 
+bool win_decode_on() {
+  static const bool on = !(getenv("L3_WINDOW_DECODE") && atoi(getenv("L3_WINDOW_DECODE")) == 0);
+  return on;
+}
 // decode sizes: whole 16-byte pieces, a tile's keys and values in registers
 template <typename KVT>
 bool win_decode_supported(const WinAttnArgs& a) {
@@ -582,21 +631,29 @@ bool win_decode_supported(const WinAttnArgs& a) {
          256 % nvv == 0 && WD_KEYS * nvv <= 256 * WD_VV;
 }
 
+// up to 8 splits, the portable cluster
+template <typename KVT>
+bool win_decode_in_cluster(const WinAttnArgs& a) {
+  static const bool on = !(getenv("L3_WINDOW_CLUSTER") && atoi(getenv("L3_WINDOW_CLUSTER")) == 0);
+  return on && win_decode_on() && win_decode_supported<KVT>(a) && a.nsplit > 1 && a.nsplit <= 8;
+}
+
 template <typename KVT, int REP>
 cudaError_t launch_win_decode(const WinAttnArgs& a, cudaStream_t s) {
   const int parts = 256 / (a.DV / Vec16<KVT>::N);
-  const size_t smem = ((size_t)REP * a.DK + REP * WD_KEYS + 3 * REP + 4 + (size_t)parts * REP * a.DV) * sizeof(float);
+  const bool cl = win_decode_in_cluster<KVT>(a);
+  const size_t smem = ((size_t)REP * a.DK + REP * WD_KEYS + 3 * REP + 4 + (size_t)parts * REP * a.DV + (cl ? (size_t)REP * (a.DV + 9) : 0)) * sizeof(float);
+  auto kern = cl ? win_decode_kernel<KVT, REP, true> : win_decode_kernel<KVT, REP, false>;
   if (smem > 40 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(win_decode_kernel<KVT, REP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  return launch_k(win_decode_kernel<KVT, REP>, dim3(a.nsplit, a.G, a.B), dim3(256), smem, s, a);
+  return launch_kc(kern, dim3(a.nsplit, a.G, a.B), dim3(256), smem, s, cl ? a.nsplit : 1, a);
 }
 
 template <typename KVT>
 cudaError_t launch_win_t(const WinAttnArgs& a, dim3 grid, cudaStream_t s) {
-  static const bool decode_on = !(getenv("L3_WINDOW_DECODE") && atoi(getenv("L3_WINDOW_DECODE")) == 0);
-  if (decode_on && win_decode_supported<KVT>(a)) {
+  if (win_decode_on() && win_decode_supported<KVT>(a)) {
     switch (a.H / a.G) {
       case 1: return launch_win_decode<KVT, 1>(a, s);
       case 2: return launch_win_decode<KVT, 2>(a, s);
@@ -642,6 +699,10 @@ cudaError_t launch_win_prep(const WinPrepArgs& a, int rows, bool kv_bf16, cudaSt
   return launch_k(win_prep_kernel<float>, grid, dim3(32 * warps), smem, s, a);
 }
 
+int win_attn_launches(const WinAttnArgs& a, bool kv_bf16) {
+  return a.nsplit == 1 || (kv_bf16 ? win_decode_in_cluster<bf16>(a) : win_decode_in_cluster<float>(a)) ? 1 : 2;
+}
+
 cudaError_t launch_win_attn(const WinAttnArgs& a, bool kv_bf16, cudaStream_t s) {
   if (!win_attn_supported(a.DK, a.DV) || a.H % a.G != 0 || a.nsplit < 1 || a.nsplit > WA_SPLIT_MAX) return cudaErrorInvalidValue;
   if (a.nsplit > 1 && (!a.part_o || !a.part_ml)) return cudaErrorInvalidValue;
@@ -655,6 +716,6 @@ cudaError_t launch_win_attn(const WinAttnArgs& a, bool kv_bf16, cudaStream_t s) 
   const int rep = a.H / a.G;
   const dim3 grid((a.L * rep + WA_ROWS - 1) / WA_ROWS, a.G, a.B * a.nsplit);
   cudaError_t e = kv_bf16 ? launch_win_t<bf16>(a, grid, s) : launch_win_t<float>(a, grid, s);
-  if (e != cudaSuccess || a.nsplit == 1) return e;
+  if (e != cudaSuccess || win_attn_launches(a, kv_bf16) == 1) return e;
   return launch_k(win_attn_combine_kernel, dim3((unsigned)(a.B * a.L * a.H)), dim3(128), 0, s, a);
 }

@@ -1664,7 +1664,7 @@ static int ll_mix_unit(L3Model* m, LLLayer& Ly, LLState& St, const float* pin, i
     at.nsplit = win_attn_splits(B, L, H, G, s.window, s.keep_first, m->M, 32);
     at.part_o = ll->win_part_o; at.part_ml = ll->win_part_ml;
     LAUNCH(m, launch_win_attn(at, m->bf16, m->stream));
-    if (at.nsplit > 1) m->launch_acc += 1;
+    m->launch_acc += win_attn_launches(at, m->bf16) - 1;
     return L3_OK;
   }
   MixOutArgs mo{};

@@ -415,6 +415,7 @@ bool attn_f32_supported(const WinAttnArgs& a);
 cudaError_t launch_attn_f32(const WinAttnArgs& a, cudaStream_t s);
 int win_attn_splits(int B, int L, int H, int G, int window, int keep_first, int max_keys, int max_split);
 size_t win_attn_part_floats(int max_rows, int H, int DV, int max_split);
+int win_attn_launches(const WinAttnArgs& a, bool kv_bf16);  // kernels that launch_win_attn starts
 cudaError_t launch_win_attn(const WinAttnArgs& a, bool kv_bf16, cudaStream_t s);
 // the same attention for prompts in bf16 mode on the tensor cores (attn_latent_tc.cu).  q16 [n_seq * L, H, q_parts,
 // latent_tc_q_ld(DK, 0)] takes the place of WinAttnArgs::q; cache_seqs = sequences the caches hold; err as LatentTcArgs::err.

@@ -58,7 +58,6 @@ template <int R>
 __global__ void __launch_bounds__(256) moe_route_kernel(MoeRouteArgs a, int rows) {
   extern __shared__ float sm[];
   pdl_launch();
-  pdl_wait();
   const int r0 = blockIdx.x * R, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int n = a.E + a.I, nl = n + a.shared_gate, D = a.D;  // slots; logits (a shared expert's gate behind the slots)
   const int live = min(R, rows - r0);
@@ -73,6 +72,22 @@ __global__ void __launch_bounds__(256) moe_route_kernel(MoeRouteArgs a, int rows
   const int per_w = ((D + nw - 1) / nw + 3) & ~3;
   const int k_lo = min(D, warp * per_w), k_hi = min(D, k_lo + per_w);
   const bool vec4 = (D % 4 == 0) && (((uintptr_t)h0 & 15) == 0) && (((uintptr_t)a.router & 15) == 0);
+  // One row per CTA is a decode step, where the router's rows come from DRAM: they are constants, so a thread asks for its first values of
+  // the first eight slots, and L2 for those of the others, ahead of the wait (figures: win_decode_kernel).
+  constexpr int PRE = R == 1 ? 2 : 0;
+  float4 pre[PRE ? PRE : 1][8];
+  if (PRE && vec4) {
+#pragma unroll
+    for (int i = 0; i < PRE; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int k = k_lo + lane * 4 + i * 128;
+        pre[i][j] = k < k_hi && j < nl ? *reinterpret_cast<const float4*>(a.router + (size_t)j * D + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    for (int e = 8; e < nl; ++e)
+      for (int k = k_lo + lane * 32; k < k_hi; k += 1024) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.router + (size_t)e * D + k));
+  }
+  pdl_wait();
   for (int e0 = 0; e0 < nl; e0 += 8) {
     float acc[R][8];
 #pragma unroll
@@ -87,7 +102,10 @@ __global__ void __launch_bounds__(256) moe_route_kernel(MoeRouteArgs a, int rows
 #pragma unroll
         for (int j = 0; j < 8; ++j)
           if (e0 + j < nl) {
-            const float4 wv = *reinterpret_cast<const float4*>(a.router + (size_t)(e0 + j) * D + k);
+            float4 wv;
+            if (PRE && e0 == 0 && k < k_lo + 128) wv = pre[0][j];
+            else if (PRE && e0 == 0 && k < k_lo + 256) wv = pre[PRE ? PRE - 1 : 0][j];
+            else wv = *reinterpret_cast<const float4*>(a.router + (size_t)(e0 + j) * D + k);
 #pragma unroll
             for (int i = 0; i < R; ++i) {
               acc[i][j] = fmaf(wv.x, hv[i].x, acc[i][j]); acc[i][j] = fmaf(wv.y, hv[i].y, acc[i][j]);
