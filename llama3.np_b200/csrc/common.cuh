@@ -104,6 +104,35 @@ __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(L3_FULL, v, o);
   return v;
 }
+// Sums V values over the lanes of a warp: while the count is even a step hands half of them to the other half of the lanes (V = 32: 31
+// shuffles, where 32 sums of their own take 160).  A lane is left with the V >> h values from slot_base<V>(lane) on, h = steps_of(V); each is added up as warp_sum adds it.
+template <int V, int O>
+__device__ __forceinline__ void warp_sums(float* v, int lane) {
+  if constexpr (O > 0) {
+    if constexpr (V % 2 == 0) {
+      const bool up = lane & O;
+#pragma unroll
+      for (int i = 0; i < V / 2; ++i) {
+        const float keep = up ? v[i + V / 2] : v[i], give = up ? v[i] : v[i + V / 2];
+        v[i] = keep + __shfl_xor_sync(L3_FULL, give, O);
+      }
+      warp_sums<V / 2, O / 2>(v, lane);
+    } else {
+#pragma unroll
+      for (int i = 0; i < V; ++i) v[i] += __shfl_xor_sync(L3_FULL, v[i], O);
+      warp_sums<V, O / 2>(v, lane);
+    }
+  }
+}
+__host__ __device__ constexpr int halvings(int v) { return v % 2 || v == 0 ? 0 : 1 + halvings(v / 2); }
+__host__ __device__ constexpr int steps_of(int v) { return halvings(v) < 5 ? halvings(v) : 5; }
+template <int V>
+__device__ __forceinline__ int slot_base(int lane) {
+  int base = 0;
+#pragma unroll
+  for (int h = 0; h < steps_of(V); ++h) base += lane & (16 >> h) ? V >> (h + 1) : 0;
+  return base;
+}
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(L3_FULL, v, o));

@@ -85,29 +85,6 @@ __device__ __forceinline__ void send4(uint32_t dst, float4 v, uint32_t bar) {
                ::"r"(dst), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar) : "memory");
 }
 
-// Sums V values over the lanes of a warp: while the count is even a step hands half of them to the other half of the lanes (V = 32: 31
-// shuffles, where 32 sums of their own take 160).  A lane is left with the V >> h values from slot_base() on.
-template <int V, int O>
-__device__ __forceinline__ void warp_sums(float* v, int lane) {
-  if constexpr (O > 0) {
-    if constexpr (V % 2 == 0) {
-      const bool up = lane & O;
-#pragma unroll
-      for (int i = 0; i < V / 2; ++i) {
-        const float keep = up ? v[i + V / 2] : v[i], give = up ? v[i] : v[i + V / 2];
-        v[i] = keep + __shfl_xor_sync(L3_FULL, give, O);
-      }
-      warp_sums<V / 2, O / 2>(v, lane);
-    } else {
-#pragma unroll
-      for (int i = 0; i < V; ++i) v[i] += __shfl_xor_sync(L3_FULL, v[i], O);
-      warp_sums<V, O / 2>(v, lane);
-    }
-  }
-}
-__host__ __device__ constexpr int halvings(int v) { return v % 2 || v == 0 ? 0 : 1 + halvings(v / 2); }
-__host__ __device__ constexpr int steps_of(int v) { return halvings(v) < 5 ? halvings(v) : 5; }
-
 // The share of a warp: row groups g0, g0 + step, ... over values k0 .. k1 of K, to piece `piece` of the output
 struct Part { int g0, step, k0, k1, piece; };
 __device__ __forceinline__ Part part_of(int K, int ks) {
@@ -161,9 +138,7 @@ __device__ __forceinline__ void gemv(const float* w, int rows, int K, const Part
       rinv = 1.0f / sqrtf(ss[0] / (float)K + eps);
     }
     constexpr int H = steps_of(R * NB), C = (R * NB) >> H, REST = 32 >> H;
-    int base = 0;
-#pragma unroll
-    for (int h = 0; h < H; ++h) base += lane & (16 >> h) ? (R * NB) >> (h + 1) : 0;
+    const int base = slot_base<R * NB>(lane);
 #pragma unroll
     for (int i = 0; i < C; ++i) {
       const int b = (base + i) / R, row = g * R + (base + i) % R;

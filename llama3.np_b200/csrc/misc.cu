@@ -116,11 +116,50 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ 
   }
 }
 
+// Rows of up to 512 values, a warp each: the CTA of such a row has lanes to spare and two barriers for ~9 values per lane.  A lane's four
+// values of each 128 are what a thread of rmsnorm_kernel holds, and the sums meet in its order: the same bits.  8192 x 288 with (hi, lo) outputs: 256 x 64 tokens
+// of stories15M in front of 64 decode steps, 25 norms, 19457 -> 19229 us (18.6 us each before).
+__global__ void __launch_bounds__(256) rmsnorm_warp_kernel(const float* __restrict__ x, const float* __restrict__ w, float eps, int rows, int D,
+                                                           int src_mul, int src_add, float* __restrict__ out, bf16* __restrict__ out_bf16,
+                                                           float* __restrict__ out_lo, const int32_t* __restrict__ src_rows) {
+  const int lane = threadIdx.x & 31, r = blockIdx.x * 8 + (threadIdx.x >> 5);
+  float4 gv[4], xv[4];
+  pdl_launch();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int k = (lane + i * 32) * 4;
+    gv[i] = k < D ? __ldg(reinterpret_cast<const float4*>(w + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  pdl_wait();
+  if (r >= rows) return;
+  const float* src = x + (src_rows ? (size_t)src_rows[r] : (size_t)r * src_mul + src_add) * D;
+  float ss[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int k = (lane + i * 32) * 4;
+    xv[i] = k < D ? *reinterpret_cast<const float4*>(src + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) ss[i] = xv[i].x * xv[i].x + xv[i].y * xv[i].y + xv[i].z * xv[i].z + xv[i].w * xv[i].w;
+  warp_sums<4, 16>(ss, lane);  // lanes 8 i .. 8 i + 7 hold the sum of the i-th 128 values
+  float tot = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) tot += __shfl_sync(L3_FULL, ss[0], 8 * i);
+  const float rinv = 1.0f / sqrtf(tot / (float)D + eps);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int k = (lane + i * 32) * 4;
+    if (k < D) rmsnorm_emit(xv[i], gv[i], rinv, (size_t)r * D + k, out, out_bf16, out_lo);
+  }
+}
+
 cudaError_t launch_rmsnorm(const float* x, const float* w, float eps, int rows, int D, int src_mul, int src_add,
                            float* out, bf16* out_bf16, float* out_lo, cudaStream_t s, const int32_t* src_rows) {
   // 128 threads as before wherever that was the whole story (the sum of squares keeps its order of additions: the
   // fp32 path is token-identical to the oracle); 256 threads for rows that would not fit 128 threads' registers
   const int threads = D > 128 * 32 ? 256 : 128;
+  if (D <= 512 && rows > 8)  // one row and up: no difference below a wave of CTAs, so few rows keep a CTA each
+    return launch_k(rmsnorm_warp_kernel, dim3((rows + 7) / 8), dim3(256), 0, s, x, w, eps, rows, D, src_mul, src_add, out, out_bf16, out_lo, src_rows);
   return launch_k(rmsnorm_kernel, dim3(rows), dim3(threads), 0, s, x, w, eps, rows, D, src_mul, src_add, out, out_bf16,
                   out_lo, src_rows);
 }
