@@ -18,6 +18,10 @@
 // read less but its parts and raw tiles do not fit together.
 // An infinite operand leaves NaN behind (its parts are inf, NaN, NaN; inf times a zero part is NaN too): sums that end as NaN are
 // taken again as a plain chain of fp32 products, so that an infinity gives what it gives there.
+// Where both operands were cut beforehand (OP_PLANES: matrices once at load time, inputs by cut_rows_kernel; ll_cut_operands has the rule)
+// TMA brings the parts themselves, three planes a copy, and nothing is converted: 24 products per 64 values of K, bound by shared memory,
+// whose bandwidth the arriving 96 KB and the products' reads share (~2600 cycles, of which the products take 1536).  600 x 4096 x 1024:
+// 64.7 -> 43.4 us, 600 x 1024 x 4096 52.3 -> 37.6, 600 x 1024 x 1024 23 -> 18.8; the same bits.
 // Every wait is bounded: one that runs out sets a flag, all warps run on without waiting, and the host reports an error.
 #include <cuda.h>
 
@@ -56,6 +60,17 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* tm,
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
       ::"r"(dst), "l"(tm), "r"(c0), "r"(c1), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* tm, int c0, int c1, int c2, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+      ::"r"(dst), "l"(tm), "r"(c0), "r"(c1), "r"(c2), "r"(bar) : "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+  return p;
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -111,16 +126,22 @@ __device__ float plain_dot(const float* a, const WT* w, int K) {
   return s;
 }
 
-template <bool WB16> constexpr int raw_bytes() { return WB16 ? HALF : 2 * HALF; }
-template <bool WB16> constexpr int smem_bytes() { return 1024 + 3 * HALF + (WB16 ? WST : 3) * HALF + RAW * raw_bytes<WB16>() + 512; }
+// how the operands come: both fp32, W in bf16, or both cut beforehand (three planes each, GemmF32Args::planes)
+enum Operands : int { OP_F32 = 0, OP_W16 = 1, OP_PLANES = 2 };
+template <int OP> constexpr int raw_bytes() { return OP == OP_W16 ? HALF : 2 * HALF; }
+constexpr int BLOCK = 6 * HALF, PST = 2;  // planes: a block of 64 values of K, three parts of both operands; blocks in flight
+template <int OP> constexpr int smem_bytes() {
+  return OP == OP_PLANES ? 1024 + PST * BLOCK + 512 : 1024 + 3 * HALF + (OP == OP_W16 ? WST : 3) * HALF + RAW * raw_bytes<OP>() + 512;
+}
 
-template <bool WB16, int EPI>
+template <int OP, int EPI>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, int rows, int N, int K, int ksplit, float* part,
                 int* tile_cnt, int* err, const float* A, int lda, const void* W, EpiArgs e) {
+  constexpr bool WB16 = OP == OP_W16, PLANES = OP == OP_PLANES;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
-  const uint32_t sA = (raw + 1023u) & ~1023u, sW = sA + 3 * HALF, sR = sW + (WB16 ? WST : 3) * HALF, bars = sR + RAW * raw_bytes<WB16>();
+  const uint32_t sA = (raw + 1023u) & ~1023u, sW = sA + 3 * HALF, sR = sW + (WB16 ? WST : 3) * HALF, bars = PLANES ? sA + PST * BLOCK : sR + RAW * raw_bytes<OP>();
   uint8_t* base = smem_raw + (sA - raw);
   const uint32_t r_full = bars, r_empty = r_full + 8 * RAW, h_full = r_empty + 8 * RAW, h_empty = h_full + 16, w_full = h_empty + 16,
                  w_empty = w_full + 8 * WST, a_full = w_empty + 8 * WST, a_empty = a_full + 16, slot = a_empty + 16;
@@ -133,7 +154,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmA));
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmW));
     *fail = 0;
-    for (int s = 0; s < RAW; ++s) { mbar_init(r_full + 8 * s, 1); mbar_init(r_empty + 8 * s, 8); }
+    for (int s = 0; s < RAW; ++s) { mbar_init(r_full + 8 * s, 1); mbar_init(r_empty + 8 * s, PLANES ? 1 : 8); }
     for (int s = 0; s < WST; ++s) { mbar_init(w_full + 8 * s, 1); mbar_init(w_empty + 8 * s, 1); }
     for (int s = 0; s < 2; ++s) {
       mbar_init(h_full + 8 * s, 8); mbar_init(h_empty + 8 * s, 1);
@@ -159,7 +180,59 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     n = 2 * (b1 - b0);
   };
 
-  if (warp == 0) {
+  if (PLANES && warp == 0) {  // ---------------- TMA; the issuing warps run their loops whole, one elected lane issues
+    uint32_t st = 0, ph = 1;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+      const int tmn = t % ntiles_mn, m0 = (tmn % tiles_m) * TILE, n0 = (tmn / tiles_m) * TILE;
+      int k0, n;
+      slice(t, k0, n);
+      for (int b = 0; b < n / 2; ++b) {
+        mbar_wait(r_empty + 8 * st, ph, fail);
+        if (elect_one()) {
+          const uint32_t dst = sA + st * BLOCK, bar = r_full + 8 * st;
+          mbar_expect_tx(bar, BLOCK);
+          tma_load_3d(dst, &tmA, k0 + b * 64, m0, 0, bar);
+          tma_load_3d(dst + 3 * HALF, &tmW, k0 + b * 64, n0, 0, bar);
+        }
+        __syncwarp();
+        if (++st == PST) { st = 0; ph ^= 1; }
+      }
+    }
+  } else if (PLANES && warp == 1) {  // ---------------- products
+    constexpr uint64_t PART = HALF >> 4;
+    uint32_t st = 0, ph = 0, ci = 0;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+      int k0, n;
+      slice(t, k0, n);
+      n /= 2;
+      for (int b = 0; b < n; ++b) {
+        const uint32_t buf = ci & 1, turn = b & 1;  // an accumulator takes two blocks, 128 terms of each kind
+        if (!turn && ci >= 2) mbar_wait(a_empty + 8 * buf, (ci / 2 - 1) & 1, fail);
+        mbar_wait(r_full + 8 * st, ph, fail);
+        tc_fence_after();
+        if (elect_one()) {
+          const uint32_t lead = tmem + buf * 256, corr = lead + TILE;
+          const uint64_t da = desc_sw128(sA + st * BLOCK), dw = da + 3 * PART;
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) {
+            const uint64_t a = da + kk * 2, w = dw + kk * 2;
+            const uint32_t go = turn | kk ? 1u : 0u;
+            mma(lead, a, w, go);
+            mma(corr, a, w + PART, go);
+            mma(corr, a + PART, w, 1u);
+            mma(corr, a + PART, w + PART, 1u);
+            mma(corr, a, w + 2 * PART, 1u);
+            mma(corr, a + 2 * PART, w, 1u);
+          }
+          tc_commit(r_empty + 8 * st);
+          if (turn || b == n - 1) tc_commit(a_full + 8 * buf);
+        }
+        __syncwarp();
+        if (turn || b == n - 1) ++ci;
+        if (++st == PST) { st = 0; ph ^= 1; }
+      }
+    }
+  } else if (warp == 0) {
     if (lane == 0) {  // ---------------- TMA
       uint32_t it = 0, wt = 0;
       for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -176,9 +249,9 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           }
           const uint32_t st = it % RAW;
           if (it >= RAW) mbar_wait(r_empty + 8 * st, (it / RAW - 1) & 1, fail);
-          mbar_expect_tx(r_full + 8 * st, raw_bytes<WB16>());
-          tma_load_2d(sR + st * raw_bytes<WB16>(), &tmA, k0 + s * STEP, m0, r_full + 8 * st);
-          if (!WB16) tma_load_2d(sR + st * raw_bytes<WB16>() + HALF, &tmW, k0 + s * STEP, n0, r_full + 8 * st);
+          mbar_expect_tx(r_full + 8 * st, raw_bytes<OP>());
+          tma_load_2d(sR + st * raw_bytes<OP>(), &tmA, k0 + s * STEP, m0, r_full + 8 * st);
+          if (!WB16) tma_load_2d(sR + st * raw_bytes<OP>() + HALF, &tmW, k0 + s * STEP, n0, r_full + 8 * st);
         }
       }
     }
@@ -251,13 +324,13 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         ++pi;
       };
 #pragma unroll 1
-      for (int s = 0; s < n; ++s, ++it) {
+      for (int s = 0; s < (PLANES ? 0 : n); ++s, ++it) {
         const uint32_t st = it % RAW, h = it & 1;
         mbar_wait(r_full + 8 * st, (it / RAW) & 1, fail);
         if (it >= 2) mbar_wait(h_empty + 8 * h, ((it >> 1) - 1) & 1, fail);
         // a thread: a row of 32 values (W bf16: half a row of A); 16-byte pieces swizzled inside the 128-byte rows on both sides
         const int r = WB16 ? ct >> 1 : ct & 127, op = WB16 ? 0 : ct >> 7, q0 = WB16 ? (ct & 1) * 4 : 0;
-        const uint8_t* src = base + (sR - sA) + st * raw_bytes<WB16>() + op * HALF + r * 128;
+        const uint8_t* src = base + (sR - sA) + st * raw_bytes<OP>() + op * HALF + r * 128;
         uint8_t* dst = base + op * 3 * HALF + r * 128;
 #pragma unroll
         for (int q = 0; q < (WB16 ? 4 : 8); q += 2) {
@@ -275,7 +348,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         if (lane == 0) { mbar_arrive(r_empty + 8 * st); mbar_arrive(h_full + 8 * h); }
         if (s % CHUNK == CHUNK - 1 && s >= CHUNK) promote();  // the turn before this one: its products are long issued
       }
-      for (int left = (n + CHUNK - 1) / CHUNK - max(0, n / CHUNK - 1); left > 0; --left) promote();
+      for (int left = (n + CHUNK - 1) / CHUNK - (PLANES ? 0 : max(0, n / CHUNK - 1)); left > 0; --left) promote();
       const int m = m0 + quarter * 32 + lane, nc = n0 + c0;
       if (ksplit > 1) {
         // publish this slice's sums; the slice that arrives last adds all of them in slice order (the result does not depend on timing)
@@ -355,19 +428,20 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
 }
 
-template <bool WB16, int EPI>
+template <int OP, int EPI>
 cudaError_t launch_t(const GemmF32Args& a, cudaStream_t s) {
-  auto kern = gemm_f32_kernel<WB16, EPI>;
+  auto kern = gemm_f32_kernel<OP, EPI>;
   static bool done[16] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!done[dev & 15]) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<WB16>());
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<OP>());
     if (e != cudaSuccess) return e;
     done[dev & 15] = true;
   }
-  const CUtensorMap* ma = tc_get_map(a.A, false, a.rows, a.K, TILE, a.lda);
-  const CUtensorMap* mw = tc_get_map(a.W, WB16, a.N, a.K, TILE);
+  const bool pl = OP == OP_PLANES;
+  const CUtensorMap* ma = pl ? tc_get_planes_map(a.A_planes, a.rows, a.K, TILE, a.a_plane) : tc_get_map(a.A, false, a.rows, a.K, TILE, a.lda);
+  const CUtensorMap* mw = pl ? tc_get_planes_map(a.W_planes, a.N, a.K, TILE, a.w_plane) : tc_get_map(a.W, OP == OP_W16, a.N, a.K, TILE);
   if (!ma || !mw) return cudaErrorInvalidValue;
   static int n_sm[16] = {0};
   if (!n_sm[dev & 15]) cudaDeviceGetAttribute(&n_sm[dev & 15], cudaDevAttrMultiProcessorCount, dev);
@@ -384,16 +458,16 @@ cudaError_t launch_t(const GemmF32Args& a, cudaStream_t s) {
       if (!best || cost < best) { best = cost; ksplit = ks; }
     }
   }
-  return launch_k(kern, dim3(std::min(tiles * ksplit, sms)), dim3(THREADS), (size_t)smem_bytes<WB16>(), s, *ma, *mw, a.rows, a.N, a.K, ksplit, a.part,
+  return launch_k(kern, dim3(std::min(tiles * ksplit, sms)), dim3(THREADS), (size_t)smem_bytes<OP>(), s, *ma, *mw, a.rows, a.N, a.K, ksplit, a.part,
                   a.tile_cnt, a.err, a.A, a.lda ? a.lda : a.K, a.W, a.e);
 }
 
-template <bool WB16>
+template <int OP>
 cudaError_t launch_e(const GemmF32Args& a, cudaStream_t s) {
   switch (a.epi) {
-    case EPI_STORE: return launch_t<WB16, EPI_STORE>(a, s);
-    case EPI_RESID: return launch_t<WB16, EPI_RESID>(a, s);
-    case EPI_SWIGLU: return launch_t<WB16, EPI_SWIGLU>(a, s);
+    case EPI_STORE: return launch_t<OP, EPI_STORE>(a, s);
+    case EPI_RESID: return launch_t<OP, EPI_RESID>(a, s);
+    case EPI_SWIGLU: return launch_t<OP, EPI_SWIGLU>(a, s);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -410,5 +484,35 @@ bool gemm_f32_supported(const GemmF32Args& a) {
 
 cudaError_t launch_gemm_f32(const GemmF32Args& a, cudaStream_t s) {
   if (!gemm_f32_supported(a)) return cudaErrorInvalidValue;
-  return a.w_bf16 ? launch_e<true>(a, s) : launch_e<false>(a, s);
+  if (!a.w_bf16 && a.A_planes && a.W_planes) {
+    if (a.K % 8 || a.a_plane % 8 || a.w_plane % 8 || (((uintptr_t)a.A_planes | (uintptr_t)a.W_planes) & 15)) return cudaErrorInvalidValue;
+    return launch_e<OP_PLANES>(a, s);
+  }
+  return a.w_bf16 ? launch_e<OP_W16>(a, s) : launch_e<OP_F32>(a, s);
+}
+
+bool gemm_f32_planes_supported(const void* W_planes, int64_t w_plane, int K) { return W_planes && K % 8 == 0 && w_plane % 8 == 0 && ((uintptr_t)W_planes & 15) == 0; }
+
+// rows of fp32 values -> three planes [rows][K] of bf16 parts, K a multiple of 8
+__global__ void __launch_bounds__(256) cut_rows_kernel(const float* __restrict__ src, int lda, int rows, int K, bf16* __restrict__ dst, int64_t plane) {
+  pdl_launch();
+  pdl_wait();
+  const int per = K / 8;
+  const int64_t n = (int64_t)rows * per;
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
+    const int64_t r = i / per;
+    const int k = (int)(i - r * per) * 8;
+    const float4* s = reinterpret_cast<const float4*>(src + r * lda + k);
+    uint4 p1, p2, p3;
+    cut8(s[0], s[1], p1, p2, p3);
+    uint4* d = reinterpret_cast<uint4*>(dst + r * K + k);
+    *d = p1;
+    *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(d) + plane) = p2;
+    *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(d) + 2 * plane) = p3;
+  }
+}
+cudaError_t launch_cut_rows(const float* src, int lda, int rows, int K, void* dst, int64_t plane, cudaStream_t s) {
+  if (K % 8 || lda % 4 || plane % 8 || (((uintptr_t)src | (uintptr_t)dst) & 15)) return cudaErrorInvalidValue;
+  const int64_t n = (int64_t)rows * (K / 8);
+  return launch_k(cut_rows_kernel, dim3((unsigned)std::min<int64_t>((n + 255) / 256, 148 * 8)), dim3(256), 0, s, src, lda, rows, K, (bf16*)dst, plane);
 }

@@ -103,8 +103,30 @@ static bool make_map(CUtensorMap* tm, const void* ptr, bool is_bf16, int rows, i
   return r == CUDA_SUCCESS;
 }
 
+// three planes of a row-major [rows, K] bf16 matrix, box = 64 values of K x box_rows rows x 3
+static bool make_planes_map(CUtensorMap* tm, const void* ptr, int rows, int K, int box_rows, int64_t plane) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, 3};
+  cuuint64_t strides[2] = {(cuuint64_t)K * 2, (cuuint64_t)plane * 2};
+  cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 3};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return fn(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 struct MapCache {
   std::map<std::tuple<const void*, int, int, int, int, int>, CUtensorMap> m;
+  std::map<std::tuple<const void*, int, int, int, int64_t>, CUtensorMap> planes;
+  const CUtensorMap* get_planes(const void* ptr, int rows, int K, int box_rows, int64_t plane) {
+    std::lock_guard<std::mutex> g(mu);
+    auto key = std::make_tuple(ptr, rows, K, box_rows, plane);
+    auto it = planes.find(key);
+    if (it != planes.end()) return &it->second;
+    CUtensorMap tm;
+    if (!make_planes_map(&tm, ptr, rows, K, box_rows, plane)) return nullptr;
+    return &planes.emplace(key, tm).first->second;
+  }
   std::mutex mu;
   const CUtensorMap* get(const void* ptr, bool is_bf16, int rows, int K, int box_rows, int ld = 0) {
     std::lock_guard<std::mutex> g(mu);
@@ -123,6 +145,8 @@ const CUtensorMap* tc_get_map(const void* ptr, bool is_bf16, int rows, int cols,
   return g_maps.get(ptr, is_bf16, rows, cols, box_rows, ld);
 }
 
+const CUtensorMap* tc_get_planes_map(const void* ptr, int rows, int cols, int box_rows, int64_t plane) { return g_maps.get_planes(ptr, rows, cols, box_rows, plane); }
+
 int tc_debug_timeline(int enable, unsigned long long* out64) {
   if (out64 && cudaMemcpyFromSymbol(out64, g_tc_dbg, sizeof(unsigned long long) * 64) != cudaSuccess) return -1;
   unsigned long long z[64] = {0};
@@ -137,6 +161,7 @@ int tc_debug_timeline(int enable, unsigned long long* out64) {
 void tc_forget_maps() {
   std::lock_guard<std::mutex> g(g_maps.mu);
   g_maps.m.clear();
+  g_maps.planes.clear();
 }
 
 bool tc_gemm_supported(int K) { return K % 8 == 0 && encode_fn() != nullptr; }

@@ -61,6 +61,12 @@ struct GemmF32Args {
   int* tile_cnt;
   int tile_cnt_len;
   int* err;             // set to 1 when a wait inside the kernel ran out
+  // both operands cut beforehand (launch_cut_rows): planes of [rows, K] and [N, K] bf16 parts, x_plane values apart; A and W as well
+  const void *A_planes, *W_planes;
+  int64_t a_plane, w_plane;
 };
+bool gemm_f32_planes_supported(const void* W_planes, int64_t w_plane, int K);
+cudaError_t launch_cut_rows(const float* src, int lda, int rows, int K, void* dst, int64_t plane, cudaStream_t s);
+const CUtensorMap* tc_get_planes_map(const void* ptr, int rows, int cols, int box_rows, int64_t plane);  // box: 64 columns, three planes
 bool gemm_f32_supported(const GemmF32Args& a);
 cudaError_t launch_gemm_f32(const GemmF32Args& a, cudaStream_t s);

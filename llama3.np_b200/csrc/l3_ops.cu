@@ -113,7 +113,7 @@ extern "C" int l3_op_linear(int device, const float* x, const float* w, int rows
     tc_forget_maps();  // the scratch buffers are about to be freed
     if (rc == L3_OK) cudaMemcpy(out, dout, (size_t)rows * n * 4, cudaMemcpyDeviceToHost);
     return rc;
-  } else if (path == 5) {  // fp32 operands (or fp32 rows and a bf16 matrix) cut into bf16 parts, fp32 precision
+  } else if (path == 5 || path == 6) {  // fp32 operands (or fp32 rows and a bf16 matrix) cut into bf16 parts, fp32 precision; 6: cut beforehand
     GemmF32Args t{};
     t.A = dx; t.W = dw; t.w_bf16 = w_bf16 != 0; t.rows = rows; t.N = n; t.K = k; t.epi = EPI_STORE; t.e = a.e;
     t.part_bytes = (size_t)32 << 20;
@@ -123,6 +123,13 @@ extern "C" int l3_op_linear(int device, const float* x, const float* w, int rows
     if (!t.part || !t.tile_cnt || !t.err) return L3_ENOMEM;
     if (cudaMemsetAsync(t.tile_cnt, 0, 1024 * sizeof(int), sc.s) != cudaSuccess || cudaMemsetAsync(t.err, 0, sizeof(int), sc.s) != cudaSuccess) return L3_ECUDA;
     if (!gemm_f32_supported(t)) return L3_EINVAL;
+    if (path == 6) {
+      bf16 *pa = sc.dev<bf16>((size_t)3 * rows * k), *pw = sc.dev<bf16>((size_t)3 * n * k);
+      t.A_planes = pa; t.W_planes = pw; t.a_plane = (int64_t)rows * k; t.w_plane = (int64_t)n * k;
+      if (!pa || !pw) return L3_ENOMEM;
+      if (w_bf16 || !gemm_f32_planes_supported(pw, t.w_plane, k)) return L3_EINVAL;
+      if (launch_cut_rows(dx, k, rows, k, pa, t.a_plane, sc.s) != cudaSuccess || launch_cut_rows((const float*)dw, k, n, k, pw, t.w_plane, sc.s) != cudaSuccess) return L3_ECUDA;
+    }
     int rc = finish(sc, launch_gemm_f32(t, sc.s)), err = 0;
     tc_forget_maps();
     if (rc == L3_OK) cudaMemcpy(&err, t.err, sizeof err, cudaMemcpyDeviceToHost);

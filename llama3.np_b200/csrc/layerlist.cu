@@ -284,9 +284,13 @@ extern "C" int l3_create_stack(const L3StackConfig* c, const L3LayerSpec* specs,
     l3_destroy(m);                                                                            \
     return L3_ENOMEM;                                                                         \
   }
+#define AW(p, count)                 /* a matrix that projections of many rows read */  \
+  AL(p, (size_t)(count) * w);                                                           \
+  ll->weights.push_back({p, (size_t)(count)})
   AL(m->embed, (size_t)c->vocab * W * w);
   if (c->tied_head) m->lm_head = m->embed;
   else AL(m->lm_head, (size_t)c->vocab * W * w);
+  ll->weights.push_back({m->lm_head, (size_t)c->vocab * W});
   AL(m->norm_final, (size_t)W * 4);
   if (c->norm_tanh) { AL(ll->final_b, (size_t)W * 4); AL(ll->final_alpha, 4); }
   if (sd) AL(ll->side_embed, (size_t)c->vocab * c->n_layers * sd * w);
@@ -322,9 +326,9 @@ extern "C" int l3_create_stack(const L3StackConfig* c, const L3LayerSpec* specs,
       AL(L.q_norm, (size_t)s.q_rank * 4);
       if (!s.kv_source) AL(L.k_norm, (size_t)s.kv_rank * 4);
       if (s.sink) AL(L.head_vec, (size_t)H * 4);
-      AL(L.w_uq, (size_t)H * (DK + s.rot_dim) * s.q_rank * w);
+      AW(L.w_uq, (size_t)H * (DK + s.rot_dim) * s.q_rank);
       const size_t ukv = (size_t)H * (DK + DV) * (s.kv_rank + s.rot_dim) * w;
-      AL(L.w_ukv, ukv);
+      AW(L.w_ukv, ukv / w);
       cudaMemset(L.w_ukv, 0, ukv);
       AL(L.inv_freq, (size_t)std::max(1, s.rot_dims / 2) * 4);
       std::vector<float> f(std::max(1, s.rot_dims / 2), 0.f);
@@ -391,9 +395,9 @@ extern "C" int l3_create_stack(const L3StackConfig* c, const L3LayerSpec* specs,
     if (c->dual_norm && unit_mixer(s.mixer) && s.ff > 0 && s.experts == 0) { L.h_base = pad8(n_ctx); L.ctx_ld = pad8(L.h_base + s.ff); }
     if (L.pair) { L.pair->in_base = L.n_in; L.pair->ctx_base = L.n_ctx; L.pair->ctx_ld = L.ctx_ld; L.n_in += L.pair->n_in; L.pair->in_ld = L.n_in; }
     L.in_ld = L.n_in;  // n_in: the rows of the whole fused projection
-    AL(L.w_in, (size_t)L.n_in * W * w);
+    AW(L.w_in, (size_t)L.n_in * W);
     cudaMemset(L.w_in, 0, (size_t)L.n_in * W * w);  // padding rows project to zero
-    AL(L.w_o, (size_t)W * L.ctx_ld * w);
+    AW(L.w_o, (size_t)W * L.ctx_ld);
     cudaMemset(L.w_o, 0, (size_t)W * L.ctx_ld * w);  // padding columns take nothing
     if (L.h_base) L.w2 = (char*)L.w_o + (size_t)L.h_base * w;
     if (L.pair) { L.pair->w_in = (char*)L.w_in + (size_t)L.pair->in_base * W * w; L.pair->w_o = (char*)L.w_o + (size_t)L.pair->ctx_base * w; }
@@ -414,22 +418,22 @@ extern "C" int l3_create_stack(const L3StackConfig* c, const L3LayerSpec* specs,
     if (gated_experts(s)) {
       L.ff_total = s.experts * s.ff + s.shared_ff;
       if (!c->parallel) AL(L.norm2, (size_t)W * 4);
-      AL(L.w13, (size_t)2 * L.ff_total * W * w);
-      AL(L.w2, (size_t)W * L.ff_total * w);
+      AW(L.w13, (size_t)2 * L.ff_total * W);
+      AW(L.w2, (size_t)W * L.ff_total);
       AL(L.router, (size_t)(s.experts + s.shared_gate) * W * 4);  // a shared expert's gate is one more row
     } else if (s.ff > 0 && s.ff_kind == L3_FF_POLYNORM) {
-      AL(L.w13, (size_t)s.ff * W * w);
+      AW(L.w13, (size_t)s.ff * W);
       AL(L.w2, (size_t)W * s.ff * w);
       AL(L.poly, 4 * 4);
     } else if (s.experts > 0) {
-      AL(L.w13, (size_t)s.experts * s.ff * W * w);
-      AL(L.w2, (size_t)W * s.experts * s.ff * w);
+      AW(L.w13, (size_t)s.experts * s.ff * W);
+      AW(L.w2, (size_t)W * s.experts * s.ff);
       AL(L.norm2, (size_t)W * 4);
       AL(L.router, (size_t)(s.experts + s.identity) * W * 4);
       AL(L.correction, (size_t)(s.experts + s.identity) * 4);
     } else if (s.ff > 0) {
-      AL(L.w13, (size_t)(s.ff_kind == L3_FF_RELU2 ? 1 : 2) * s.ff * W * w);
-      if (!L.h_base) AL(L.w2, (size_t)W * s.ff * w);
+      AW(L.w13, (size_t)(s.ff_kind == L3_FF_RELU2 ? 1 : 2) * s.ff * W);
+      if (!L.h_base) { AW(L.w2, (size_t)W * s.ff); }
       if (!c->parallel) AL(L.norm2, (size_t)W * 4);
     }
     if (sd) {
@@ -446,7 +450,7 @@ extern "C" int l3_create_stack(const L3StackConfig* c, const L3LayerSpec* specs,
     ll->max_ff = std::max(ll->max_ff, s.experts > 0 ? s.experts * s.ff : s.ff);
   }
   if (c->loop_times > 0 && !c->loop_in) AL(ll->loop_step, (size_t)c->loop_times * W * 4);
-  if (c->loop_in) AL(ll->loop_in, (size_t)W * 2 * W * w);
+  if (c->loop_in) { AW(ll->loop_in, (size_t)W * 2 * W); }
   if (c->embed_norm) AL(ll->embed_norm, (size_t)W * 4);
 #undef AL
   // execution order: the layers ahead of the loop, the looped block loop_times times, the rest
@@ -1083,6 +1087,26 @@ static int ll_workspaces(L3Model* m, bool units, bool ksplit) {
       ll->chunk_ws = p;
       ll->chunk_ws_floats = chan;
     }
+  if (!m->bf16 && ll->f32_tc && ct > 8) {  // the matrices of fp32 projections, cut into bf16 parts once, and room for their inputs' parts
+    size_t n = 0, k = std::max<size_t>(m->D, std::max(ll->max_ctx, ll->max_ff));
+    for (auto& L : ll->layers) k = std::max<size_t>(k, std::max(L.spec.ff, std::max(L.ff_total, L.ctx_ld)));
+    for (auto& w : ll->weights) n += w.n % 8 ? 0 : w.n;
+    if (void* p = optional_ws(ct * k * 6)) {
+      ll->x_cut = (bf16*)p;
+      if ((p = optional_ws(n * 6))) {
+        ll->cut = (bf16*)p;
+        ll->x_cut_n = ct * k;
+        bf16* to = ll->cut;
+        for (auto& w : ll->weights) {
+          if (w.n % 8) continue;  // rows that are no whole 16-byte pieces
+          w.plane = (int64_t)w.n;
+          CK(m, launch_cut_rows((const float*)w.p, 8, (int)(w.n / 8), 8, to, w.plane, m->stream));
+          w.cut = to;
+          to += 3 * w.plane;
+        }
+      }
+    }
+  }
   const size_t per = (size_t)m->M * f_ld * 4;
   if (f_ld && ct >= LATENT_F32_MIN && per <= ((size_t)1 << 30)) {  // expanded latent rows in fp32 mode; longer contexts keep the folded form
     const int seqs = (int)std::max<size_t>(1, std::min<size_t>(m->maxB, ((size_t)1 << 28) / per));
@@ -1332,7 +1356,7 @@ void ll_destroy(L3Model* m) {
   LayerList* ll = m->ll;
   if (!ll) return;
   auto fr = [](void* p) { if (p) cudaFree(p); };
-  fr(ll->side_embed); fr(ll->one); fr(ll->X);
+  fr(ll->side_embed); fr(ll->one); fr(ll->X); fr(ll->cut); fr(ll->x_cut);
   if (m->lm_head == m->embed) m->lm_head = nullptr;  // a tied output projection has no storage of its own
   for (auto& L : ll->layers) {
     fr(L.w_in); fr(L.w_o); fr(L.w_a2); fr(L.w_g2); fr(L.w13); fr(L.h_base ? nullptr : L.w2); fr(L.side_gate); fr(L.side_proj);
@@ -1504,6 +1528,24 @@ static bool ll_takes_mirror(const L3Model* m, int rows, int N, int K) {
   return m->tc_ok && !ll_gemv(m, rows, N, K) && K % 8 == 0 && K >= 64 && N >= 64;
 }
 
+// The parts of an fp32 product's operands, where its matrix was cut at load time: the input's are made here, a launch of ~3 us.  That pays
+// from two row tiles and ~400 million products on (prompt through the public call, in the kernel : beforehand, us): gifudra width 1024, 400
+// tokens 525 : 489, 2 x 400 790 : 703, 2 x 64 463 : 476; debuzen width 1024, 130 tokens 826 : 762, 2 x 400 1719 : 1418; width 512, 400
+// tokens 938 : 914, mabedra 581 : 569, risalix 666 : 667, with all products cut 666 : 680.
+static int ll_cut_operands(L3Model* m, GemmF32Args& t) {
+  LayerList* ll = m->ll;
+  if (!ll->x_cut || t.rows <= 128 || (int64_t)t.rows * t.N * t.K < 400000000 || t.K % 8 || (size_t)t.rows * t.K > ll->x_cut_n) return L3_OK;
+  for (const auto& w : ll->weights) {
+    const int64_t off = (const float*)t.W - (const float*)w.p;
+    if (!w.cut || off < 0 || off + (int64_t)t.N * t.K > (int64_t)w.n || off % 8) continue;
+    t.W_planes = w.cut + off; t.w_plane = w.plane;
+    t.A_planes = ll->x_cut; t.a_plane = (int64_t)t.rows * t.K;
+    LAUNCH(m, launch_cut_rows(t.A, t.lda ? t.lda : t.K, t.rows, t.K, ll->x_cut, t.a_plane, m->stream));
+    break;
+  }
+  return L3_OK;
+}
+
 // y = x W^T (+ epilogue).  x32: fp32 rows with stride lda (0 = K); x16: bf16 mirror with stride K, or null.
 // pd: non-null when x32 is the residual stream (ll->xcur) - a deferred step is applied on the way.
 // norm_w: the row-streaming GEMV norms the rows while staging them (only where ll_gemv says it runs).
@@ -1560,6 +1602,7 @@ static int ll_linear(L3Model* m, const void* W, const float* x32, const void* x1
     t.A = a.x; t.lda = ld; t.W = W; t.w_bf16 = m->bf16; t.rows = rows; t.N = N; t.K = K; t.epi = epi; t.e = e;
     t.part = m->gemm_part; t.part_bytes = (size_t)32 << 20; t.tile_cnt = m->gemm_cnt; t.tile_cnt_len = 1024; t.err = m->h_err;
     if (gemm_f32_supported(t)) {
+      if (const int rc = ll_cut_operands(m, t)) return rc;
       LAUNCH(m, launch_gemm_f32(t, m->stream));
       return L3_OK;
     }
@@ -1797,6 +1840,7 @@ static int ll_latent_prompt_f32(L3Model* m, LLLayer& Ly, LLState& St, int B, int
       t.A = (const float*)St.lat + (size_t)(b0 + i) * m->M * Dk; t.W = Ly.w_ukv; t.rows = T; t.N = n_exp; t.K = Dk; t.epi = EPI_STORE;
       t.e = store_to(exp + (size_t)i * m->M * n_exp, nullptr, n_exp);
       t.part = m->gemm_part; t.part_bytes = (size_t)32 << 20; t.tile_cnt = m->gemm_cnt; t.tile_cnt_len = 1024; t.err = m->h_err;
+      if (const int rc = ll_cut_operands(m, t)) return rc;
       LAUNCH(m, launch_gemm_f32(t, m->stream));
     }
     WinAttnArgs at{};

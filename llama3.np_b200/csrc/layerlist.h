@@ -2,6 +2,7 @@
 // with its own token mixer, an optional gated feed-forward and an optional per-layer token input, sharing the
 // handle, the entry points, the generate loop, the graphs and the projection kernels of the Llama path.
 #pragma once
+#include <cuda_bf16.h>
 #include <set>
 #include <string>
 #include <vector>
@@ -142,6 +143,12 @@ struct LayerList {
   float *y1 = nullptr, *y2 = nullptr;      // the two sublayers' results [cap_tok, width] (with streams: y1 alone)
   float* moe_gu = nullptr;                 // [cap_tok, 2 ff_total] gate | up of every expert
   float *diff_part_o = nullptr, *diff_part_ml = nullptr;  // split scratch of the differential decode attention
+  // fp32 mode: the matrices that projections read, with their bf16 parts (three planes, `plane` values apart; null: not cut), and room for
+  // the parts of an input of up to x_cut_n values
+  struct Weight { void* p; size_t n; __nv_bfloat16* cut = nullptr; int64_t plane = 0; };
+  std::vector<Weight> weights;
+  __nv_bfloat16 *cut = nullptr, *x_cut = nullptr;
+  size_t x_cut_n = 0;
   bool f32_tc = false;  // fp32 rows of many tokens run the fp32-precision tensor-core GEMM (gemm_f32.cu)
   int max_in = 0, max_o = 0, max_ctx = 0, max_ff = 0;  // max_ctx: columns of an output projection's input
   int head_rows = 0;  // rows the LM head's buffers hold
