@@ -18,6 +18,7 @@
 
 #include <stdlib.h>
 #include <algorithm>
+#include <mutex>
 
 #include "common.cuh"
 #include "gemm_tc.h"
@@ -94,6 +95,17 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
+__device__ __forceinline__ float ld_cluster(const float* p, int rank) {  // the same place in another CTA of the cluster
+  uint32_t a;
+  float v;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 constexpr int SW_THREADS = 224;  // warp 0 = weight copies, warp 1 = TMEM + MMA, warps 2-5 = epilogue, warp 6 = activation copies
 // BNA = batch columns of the tile (activation rows padded up)
 template <int KIND, int BNA> struct SwCfg {
@@ -127,7 +139,7 @@ template <int KIND, int BNA, int EPI>
 __global__ void __launch_bounds__(SW_THREADS, 1)
 gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant__ CUtensorMap tmW1,
                  const __grid_constant__ CUtensorMap tmX0, const __grid_constant__ CUtensorMap tmX1,
-                 int rows, int N, int K, int h, int nst, int ksplit, float* part, int* tile_cnt, EpiArgs e) {
+                 int rows, int N, int K, int h, int nst, int ksplit, int cl, float* part, int* tile_cnt, EpiArgs e) {
   using Cf = SwCfg<KIND, BNA>;
   using KVT = typename std::conditional<KIND == TC_BF16, bf16, float>::type;
   constexpr int PARTS = Cf::PARTS, NBUF = Cf::NBUF, CJ = Cf::CJ;
@@ -145,6 +157,9 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
   const int ntiles = tiles_w * ksplit;
   const int nkb = (K + Cf::BK - 1) / Cf::BK;
   const int kb_per = (nkb + ksplit - 1) / ksplit;
+  // cl: the slices of a tile are a cluster, one item per CTA
+  auto tile_of = [&](int t) { return cl ? t / ksplit : t % tiles_w; };
+  auto slice_of = [&](int t) { return cl ? t % ksplit : t / tiles_w; };
   pdl_launch();
 
   if (warp == 0 && lane == 0) {
@@ -185,7 +200,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
     int s = 0;
     uint32_t ph = 1;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-      const int n0 = (t % tiles_w) * h, ks = t / tiles_w;
+      const int n0 = tile_of(t) * h, ks = slice_of(t);
       const int kb0 = ks * kb_per, kb1 = min(nkb, kb0 + kb_per);
       for (int kb = kb0; kb < kb1; ++kb) {
         mbar_wait(empty0 + 8 * s, ph);
@@ -208,7 +223,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
     int s = 0;
     uint32_t ph = 0, ti = 0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++ti) {
-      const int ks = t / tiles_w;
+      const int ks = slice_of(t);
       const int kb0 = ks * kb_per, kb1 = min(nkb, kb0 + kb_per);
       const uint32_t buf = ti % NBUF, use = ti / NBUF;
       if (use > 0) {
@@ -256,7 +271,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
     const int start_pos = (EPI == EPI_ROPE_KV) ? *e.pos_ptr : 0;
     uint32_t ti = 0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++ti) {
-      const int n0 = (t % tiles_w) * h, ks = t / tiles_w;
+      const int n0 = tile_of(t) * h, ks = slice_of(t);
       const int kb0 = ks * kb_per, kb1 = min(nkb, kb0 + kb_per);
       const uint32_t buf = ti % NBUF, use = ti / NBUF;
       mbar_wait(accfull0 + 8 * buf, use & 1);
@@ -278,9 +293,28 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
         }
       };
       const int Np = tiles_w * Cf::BMW;  // padded width of the K-split scratch [ksplit][BNA][Np]
-      const int tw = t % tiles_w, np = tw * Cf::BMW + quarter * 32 + lane;
-      const bool det = ksplit > 1 && part != nullptr;  // else (residual epilogue only): fp32 atomics
-      if (det) {
+      const int tw = tile_of(t), np = tw * Cf::BMW + quarter * 32 + lane;
+      const bool det = ksplit > 1 && (cl || part != nullptr);  // else (residual epilogue only): fp32 atomics
+      int m_lo = 0, m_hi = rows;  // rows that this CTA finishes
+      float* mine = reinterpret_cast<float*>(smem_raw + (tiles - raw)) + quarter * 32 + lane;  // cl: [row][128 columns]
+      if (cl) {
+        // The slices' sums stay in shared memory - the ring, which nothing reads any more - and every CTA of the cluster adds up and
+        // finishes its share of the rows, slices in order: the sums of the published form below without its trip through L2 and
+        // without a last arriver that works alone.  40 greedy tokens of 32 sequences at the 8B shape 11120 -> 10960 us.
+#pragma unroll 1
+        for (int c0 = 0; c0 < BNA; c0 += 32) {
+          if (c0 >= rows || !live) break;
+          float v[32];
+          load_acc(c0, v);
+#pragma unroll
+          for (int j = 0; j < CJ; ++j)
+            if (c0 + j < rows) mine[(c0 + j) * Cf::BMW] = v[j];
+        }
+        __syncwarp();
+        cluster_sync_all();
+        m_lo = rows * ks / ksplit;
+        m_hi = rows * (ks + 1) / ksplit;
+      } else if (det) {
         // K-split: publish this slice's partial tile (for a fixed row the warp's 32 lanes store 32 consecutive
         // columns); the LAST slice of an output tile to arrive sums all slices in slice order - a fixed order,
         // so the result does not depend on timing - and runs the fused epilogue on the sum.
@@ -313,9 +347,21 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
       }
 #pragma unroll 1
       for (int c0 = 0; c0 < BNA; c0 += 32) {
-        if (c0 >= rows || !live) break;  // warp-uniform
+        if (c0 >= m_hi || !live) break;  // warp-uniform
+        if (c0 + 32 <= m_lo) continue;
+        auto mine_too = [&](int m) { return m >= m_lo && m < m_hi; };
         float v[32];
-        if (!det) {
+        if (cl) {
+#pragma unroll
+          for (int j = 0; j < CJ; ++j) v[j] = 0.f;
+          for (int k2 = 0; k2 < ksplit; ++k2) {
+            float w[32];
+#pragma unroll
+            for (int j = 0; j < CJ; ++j) w[j] = mine_too(c0 + j) ? ld_cluster(mine + (c0 + j) * Cf::BMW, k2) : 0.f;
+#pragma unroll
+            for (int j = 0; j < CJ; ++j) v[j] += w[j];
+          }
+        } else if (!det) {
           load_acc(c0, v);
           if (c0 + 32 >= BNA || c0 + 32 >= rows) {  // last TMEM read of this tile: hand the buffer back early
             tc_fence_before();
@@ -344,7 +390,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
 #pragma unroll
           for (int j = 0; j < CJ; ++j) {
             const int m = c0 + j;
-            if (m < rows && n_ok) {
+            if (mine_too(m) && n_ok) {
               const size_t o = (size_t)m * e.ld_out + n;
               if (e.out_lo) { float hi, lo; split_tf32(v[j], hi, lo); e.out[o] = hi; e.out_lo[o] = lo; }
               else if (e.out) e.out[o] = v[j];
@@ -361,7 +407,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
             for (int j = 0; j < CJ; ++j) rr[j] = e.resid[(size_t)min(c0 + j, rows - 1) * e.ld_out + nc];
 #pragma unroll
             for (int j = 0; j < CJ; ++j)
-              if (c0 + j < rows && n_ok) e.out[(size_t)(c0 + j) * e.ld_out + n] = rr[j] + v[j];
+              if (mine_too(c0 + j) && n_ok) e.out[(size_t)(c0 + j) * e.ld_out + n] = rr[j] + v[j];
           } else {  // bf16 mode: the slices add their partials into the residual stream in place (out == resid)
 #pragma unroll
             for (int j = 0; j < CJ; ++j)
@@ -396,7 +442,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
             const size_t o = (size_t)mb * e.ld_out + (n >> 1);
 #pragma unroll
             for (int j = 0; j < HF; ++j)
-              if (mb + j < rows) {
+              if (mine_too(mb + j)) {
                 const size_t oj = o + (size_t)j * e.ld_out;
                 if (e.out_lo) split_tf32(hv[j], e.out[oj], e.out_lo[oj]);
                 else if (e.out) e.out[oj] = hv[j];
@@ -425,7 +471,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
           for (int j = 0; j < CJ; ++j) {
             const float other = __shfl_xor_sync(L3_FULL, v[j], 1);  // the pair's partner (llama3.py:41-76)
             const int m = c0 + j, row = __shfl_sync(L3_FULL, lrow, j);
-            if (m >= rows || !n_ok) continue;
+            if (!mine_too(m) || !n_ok) continue;
             float r = v[j];
             // even: x0 c - x1 s, odd: x0 s + x1 c
             if (is_q || is_k) r = (lane & 1) ? other * sn[j] + v[j] * cs[j] : v[j] * cs[j] - other * sn[j];
@@ -444,7 +490,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
 #pragma unroll
           for (int j = 0; j < CJ; ++j) {
             const int m = c0 + j;
-            if (m >= rows) continue;  // warp-uniform
+            if (!mine_too(m)) continue;  // warp-uniform
             uint32_t kv = 0u;  // ordered bits of the value; 0 = no candidate
             if (n_ok) {
               const uint32_t b = __float_as_uint(v[j]);
@@ -464,6 +510,10 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
       }
     }
   }
+  if (cl) {
+    if (warp < 2 || warp == 6) cluster_sync_all();  // the others have met where the slices' sums were complete
+    cluster_sync_all();                             // nobody leaves while its sums are read
+  }
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -480,7 +530,7 @@ int sm_count() {
 }
 
 template <int KIND, int BNA, int EPI>
-cudaError_t launch_sw_t(const TcGemmArgs& a, cudaStream_t s) {
+cudaError_t launch_sw_t(const TcGemmArgs& a, bool cluster, cudaStream_t s) {
   using Cf = SwCfg<KIND, BNA>;
   auto kern = gemm_swap_kernel<KIND, BNA, EPI>;
   static bool attr_done[16] = {false};
@@ -502,17 +552,20 @@ cudaError_t launch_sw_t(const TcGemmArgs& a, cudaStream_t s) {
   // no more stages than a CTA has k-blocks
   const int nkb = (a.K + Cf::BK - 1) / Cf::BK, items = ((a.N + h - 1) / h * a.ksplit + (int)grid.x - 1) / (int)grid.x;
   const int nst = std::max(2, std::min(Cf::stages(h), (nkb + a.ksplit - 1) / a.ksplit * items));
-  return launch_k(kern, grid, dim3(SW_THREADS), (size_t)(nst * Cf::stage_bytes(h) + Cf::REST + 1024 + Cf::BARS), s, *W0, *W1, *X0, *X1, a.rows, a.N, a.K, h, nst, a.ksplit, a.part, a.tile_cnt, a.e);
+  const int cl = cluster ? 1 : 0;
+  if (cl && a.rows * Cf::BMW * 4 > nst * Cf::stage_bytes(h)) return cudaErrorInvalidValue;  // the sums lie in the ring: four blocks and more
+  if (cl) grid.x = (a.N + h - 1) / h * a.ksplit;
+  return launch_kc(kern, grid, dim3(SW_THREADS), (size_t)(nst * Cf::stage_bytes(h) + Cf::REST + 1024 + Cf::BARS), s, cl ? a.ksplit : 1, *W0, *W1, *X0, *X1, a.rows, a.N, a.K, h, nst, a.ksplit, cl, a.part, a.tile_cnt, a.e);
 }
 
 template <int KIND, int BNA>
-cudaError_t launch_sw_e(const TcGemmArgs& a, cudaStream_t s) {
+cudaError_t launch_sw_e(const TcGemmArgs& a, bool cl, cudaStream_t s) {
   switch (a.epi) {
-    case EPI_STORE: return launch_sw_t<KIND, BNA, EPI_STORE>(a, s);
-    case EPI_RESID: return launch_sw_t<KIND, BNA, EPI_RESID>(a, s);
-    case EPI_SWIGLU: return launch_sw_t<KIND, BNA, EPI_SWIGLU>(a, s);
-    case EPI_ARGMAX: return launch_sw_t<KIND, BNA, EPI_ARGMAX>(a, s);
-    default: return launch_sw_t<KIND, BNA, EPI_ROPE_KV>(a, s);
+    case EPI_STORE: return launch_sw_t<KIND, BNA, EPI_STORE>(a, cl, s);
+    case EPI_RESID: return launch_sw_t<KIND, BNA, EPI_RESID>(a, cl, s);
+    case EPI_SWIGLU: return launch_sw_t<KIND, BNA, EPI_SWIGLU>(a, cl, s);
+    case EPI_ARGMAX: return launch_sw_t<KIND, BNA, EPI_ARGMAX>(a, cl, s);
+    default: return launch_sw_t<KIND, BNA, EPI_ROPE_KV>(a, cl, s);
   }
 }
 }  // namespace
@@ -528,12 +581,33 @@ static bool adds_in_place(const TcGemmArgs& a, int sms) {
 }
 // Tile height and K split, by the cycles of the busiest CTA: a k-block takes the issue loops ~500 cycles (fp32 mode, two parts and three
 // products: 750 - 980 with the columns; with 700 for all of them 74 x 288 x 768 took 26.7 us whole instead of 24.7 in slices, 74 x 8192 x
-// 1536 43.9 instead of 39.4), or its share of DRAM (3560 bytes per cycle for all CTAs that stream); slices that are added in place cost little, published and summed ones ~2.5 us and more
-// with each slice and row: 9 x 2048 x 4096 added in place, 1, 2, 4, 8 slices 18.0, 12.4, 10.1, 8.6 us, 9 x 2048 x 8192 28.8, 18.2, 12.4,
+// 1536 43.9 instead of 39.4), or its share of DRAM (3560 bytes per cycle for all CTAs that stream); slices that are added in place cost little, a cluster's ~1 us (taken where all
+// tiles' clusters are resident at once; 1000 - 3000 cycles choose alike), published and summed ones ~2.5 us and more with each slice and row: 9 x 2048 x 4096 added in place, 1, 2, 4, 8 slices 18.0, 12.4, 10.1, 8.6 us, 9 x 2048 x 8192 28.8, 18.2, 12.4,
 // 11.5.  More tiles than SMs: the height that makes the last round full (28672 rows: 293 tiles of 98 instead of 224 of 128 - 100 rows
 // 57.5 -> 56.2 us, 32 rows 46.0 : 46.1, 9 rows 43.6 : 44.5).  Over 22 shapes (profiles/gemm_cuts.jsonl) it is 0.8 % behind the best in the
 // mean, at most 7 %.
-static void pick_swap(const TcGemmArgs& a, int bna, int sms, int* h_out, int* ks_out) {
+// clusters of n CTAs with all of an SM's shared memory each that the device holds at once (GPCs have 16 - 20 SMs)
+static int clusters_of(int n) {
+  static std::mutex mu;
+  static int most[16][9] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> g(mu);
+  int& v = most[dev & 15][n];
+  if (v) return v;
+  auto kern = gemm_swap_kernel<TC_BF16, 32, EPI_STORE>;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at[1];
+  cfg.gridDim = dim3(n); cfg.blockDim = dim3(SW_THREADS); cfg.dynamicSmemBytes = SwCfg<TC_BF16, 32>::SMEM_MAX;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = n; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  v = 1;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&v, kern, &cfg) != cudaSuccess || v < 1) { cudaGetLastError(); v = 1; }
+  return v;
+}
+static void pick_swap(const TcGemmArgs& a, int bna, int sms, int* h_out, int* ks_out, bool* cl_out) {
   static const int max_split = [] { const char* v = getenv("L3_SWAP_KSPLIT"); return v ? atoi(v) : 8; }();
   static const int det_epi = [] { const char* v = getenv("L3_SWAP_KSPLIT_DET"); return v ? atoi(v) : 1; }();
   const bool b16 = a.kind == TC_BF16, atomic = adds_in_place(a, sms);
@@ -543,17 +617,19 @@ static void pick_swap(const TcGemmArgs& a, int bna, int sms, int* h_out, int* ks
   if (rounds > 1) h = std::min(128, ((a.N + sms * rounds - 1) / (sms * rounds) + 1) & ~1);
   const int tiles = (a.N + h - 1) / h;
   double best = 0;
+  *cl_out = false;
   for (int ks = 1; ks <= std::max(1, atomic ? 8 : std::min(8, max_split)); ++ks) {
     const int per = (nkb + ks - 1) / ks;
     if (ks > 1 && (per < 4 || (ks - 1) * per >= nkb)) break;
-    if (ks > 1 && !atomic && (!a.part || !a.tile_cnt || tiles > a.tile_cnt_len || (size_t)bna * tiles * 128 * sizeof(float) * ks > a.part_bytes ||
+    const bool cl = ks > 1 && !atomic && det_epi && clusters_of(ks) >= tiles;
+    if (ks > 1 && !atomic && !cl && (!a.part || !a.tile_cnt || tiles > a.tile_cnt_len || (size_t)bna * tiles * 128 * sizeof(float) * ks > a.part_bytes ||
                               !(det_epi || a.epi == EPI_RESID))) break;
     const double issue = b16 ? 500 : 720 + 2.0 * bna, slice = 160 + 22.0 * bna + (b16 ? 0 : 8.0 * a.rows);
     const int full = tiles * ks / sms, rest = tiles * ks % sms;
     double c = full * per * std::max(issue, h * 128.0 * parts * sms / 3560);
     if (rest) c += per * std::max(issue, h * 128.0 * parts * rest / 3560);
-    if (ks > 1) c += atomic ? 380 + 2.0 * ks * bna : 4400 + slice * ks;
-    if (best == 0 || c < best) { best = c; *ks_out = ks; }
+    if (ks > 1) c += atomic ? 380 + 2.0 * ks * bna : cl ? 1800 : 4400 + slice * ks;
+    if (best == 0 || c < best) { best = c; *ks_out = ks; *cl_out = cl; }
   }
   *h_out = h;
 }
@@ -562,7 +638,7 @@ static int batch_cols(int rows) { return rows <= 16 ? 16 : rows <= 32 ? 32 : row
 TcPlan gemm_swap_plan(const TcGemmArgs& a) {
   const int sms = sm_count();
   TcPlan p{1, 128, 1, 0};
-  pick_swap(a, batch_cols(a.rows), sms, &p.width, &p.slices);
+  pick_swap(a, batch_cols(a.rows), sms, &p.width, &p.slices, &p.cluster);
   p.any_order = p.slices > 1 && adds_in_place(a, sms);
   return p;
 }
@@ -579,16 +655,16 @@ cudaError_t launch_gemm_swap(const TcGemmArgs& args, cudaStream_t s) {
   // no hot spot), low tiles in place of a K split (42 rows x 147 CTAs for QKV: 17 vs 14 us, the issue loops' cycles per block remain).
   if (a.kind == TC_BF16) {
     switch (bna) {
-      case 16: return launch_sw_e<TC_BF16, 16>(a, s);
-      case 32: return launch_sw_e<TC_BF16, 32>(a, s);
-      case 64: return launch_sw_e<TC_BF16, 64>(a, s);
-      default: return launch_sw_e<TC_BF16, 128>(a, s);
+      case 16: return launch_sw_e<TC_BF16, 16>(a, p.cluster, s);
+      case 32: return launch_sw_e<TC_BF16, 32>(a, p.cluster, s);
+      case 64: return launch_sw_e<TC_BF16, 64>(a, p.cluster, s);
+      default: return launch_sw_e<TC_BF16, 128>(a, p.cluster, s);
     }
   }
   switch (bna) {
-    case 16: return launch_sw_e<TC_TF32X3, 16>(a, s);
-    case 32: return launch_sw_e<TC_TF32X3, 32>(a, s);
-    case 64: return launch_sw_e<TC_TF32X3, 64>(a, s);
-    default: return launch_sw_e<TC_TF32X3, 128>(a, s);
+    case 16: return launch_sw_e<TC_TF32X3, 16>(a, p.cluster, s);
+    case 32: return launch_sw_e<TC_TF32X3, 32>(a, p.cluster, s);
+    case 64: return launch_sw_e<TC_TF32X3, 64>(a, p.cluster, s);
+    default: return launch_sw_e<TC_TF32X3, 128>(a, p.cluster, s);
   }
 }

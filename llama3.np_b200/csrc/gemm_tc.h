@@ -33,7 +33,7 @@ struct TcGemmArgs {
 cudaError_t launch_gemm_tc(const TcGemmArgs& a, cudaStream_t s);
 // how a launch cuts its work: CTAs that share a tile, the tile's width (gemm_swap.cu: height), slices of K, and whether slices are added
 // in whatever order they arrive
-struct TcPlan { int ctas, width, slices, any_order; };
+struct TcPlan { int ctas, width, slices, any_order; bool cluster = false; };  // cluster: the slices of a tile are one
 TcPlan gemm_tc_plan(const TcGemmArgs& a);    // bf16
 TcPlan gemm_swap_plan(const TcGemmArgs& a);
 // swapped operand roles for 9..128 activation rows (gemm_swap.cu): same arguments
