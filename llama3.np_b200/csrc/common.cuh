@@ -91,10 +91,11 @@ __device__ __forceinline__ void split_tf32(float v, float& hi, float& lo) {
 // silu exactly as the reference writes it: x * (1 / (1 + exp(-x)))   (llama3.py:27-28)
 __device__ __forceinline__ float silu_ref(float x) { return x * (1.0f / (1.0f + expf(-x))); }
 
-// tanh form of GELU: 0.5 z (1 + tanh(sqrt(2 / pi) (z + 0.044715 z^3)))
-__device__ __forceinline__ float gelu_tanh_ref(float z) {
-  return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
-}
+// tanh form of GELU, 0.5 z (1 + tanh(y)) with y = sqrt(2 / pi) (z + 0.044715 z^3), as z / (1 + exp(-2 y)): the same function, without the
+// difference of nearly equal numbers for z < 0, and one exponential in place of tanhf.  2048 x 16384 x 2048 with
+// it in the epilogue, as a loop of its own like silu's: 148.8 -> 110.2 us (the formula alone, inside the loop that asks for the activation
+// at every value: no change)
+__device__ __forceinline__ float gelu_tanh_ref(float z) { return z / (1.0f + expf(-1.5957691216057308f * (z + 0.044715f * z * z * z))); }
 // activation of a gated linear unit's gate column (EpiArgs::act)
 enum GluAct : int { GLU_SILU = 0, GLU_GELU_TANH = 1, GLU_CLAMP = 2 };
 __device__ __forceinline__ float glu_act(int act, float z) { return act == GLU_GELU_TANH ? gelu_tanh_ref(z) : silu_ref(z); }
@@ -257,14 +258,15 @@ struct EpiArgs {
 };
 // a gated unit's output from its gate and up values (FAST: exp2-based exponential and approximate divide)
 template <bool FAST>
+__device__ __forceinline__ float glu_clamp(float limit, float slope, float g, float u) {
+  g = fminf(g, limit);
+  u = fminf(fmaxf(u, -limit), limit);
+  const float z = -slope * g;
+  return (FAST ? __fdividef(g, 1.0f + __expf(z)) : g / (1.0f + expf(z))) * (u + 1.0f);
+}
+template <bool FAST>
 __device__ __forceinline__ float glu_pair(const EpiArgs& e, float g, float u) {
-  if (e.act == GLU_CLAMP) {
-    g = fminf(g, e.act_limit);
-    u = fminf(fmaxf(u, -e.act_limit), e.act_limit);
-    const float z = -e.act_slope * g;
-    return (FAST ? __fdividef(g, 1.0f + __expf(z)) : g / (1.0f + expf(z))) * (u + 1.0f);
-  }
-  return glu_act(e.act, g) * u;
+  return e.act == GLU_CLAMP ? glu_clamp<FAST>(e.act_limit, e.act_slope, g, u) : glu_act(e.act, g) * u;
 }
 // routing weight of output j (= column pair index) of row m
 __device__ __forceinline__ float glu_in_weight(const EpiArgs& e, int m, int j) {

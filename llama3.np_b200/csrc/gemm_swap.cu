@@ -431,6 +431,13 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
           if (e.act == GLU_SILU && !e.glu_w) {
 #pragma unroll
             for (int j = 0; j < HF; ++j) hv[j] = silu_ref(gt[j]) * hv[j];
+          } else if (e.act == GLU_GELU_TANH && !e.glu_w) {
+#pragma unroll
+            for (int j = 0; j < HF; ++j) hv[j] = gelu_tanh_ref(gt[j]) * hv[j];
+          } else if (e.act == GLU_CLAMP && !e.glu_w) {
+            const float limit = e.act_limit, slope = e.act_slope;
+#pragma unroll
+            for (int j = 0; j < HF; ++j) hv[j] = glu_clamp<KIND == TC_BF16>(limit, slope, gt[j], hv[j]);
           } else {
 #pragma unroll
             for (int j = 0; j < HF; ++j) {

@@ -623,6 +623,13 @@ __device__ __forceinline__ void tc_gemm_run(TcPipe& p, const CUtensorMap* tmA0, 
 #pragma unroll
                 for (int i = 0; i < 16; ++i) { const float2 t = staged(i); hv[i] = silu_ref(t.x) * t.y; }
               }
+            } else if (!e.glu_w && e.act == GLU_GELU_TANH) {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) { const float2 t = staged(i); hv[i] = gelu_tanh_ref(t.x) * t.y; }
+            } else if (!e.glu_w && e.act == GLU_CLAMP) {
+              const float limit = e.act_limit, slope = e.act_slope;
+#pragma unroll
+              for (int i = 0; i < 16; ++i) { const float2 t = staged(i); hv[i] = glu_clamp<KIND == TC_BF16>(limit, slope, t.x, t.y); }
             } else {
               const int g = e.glu_w ? (col >> 1) / e.glu_group : 0;
               const bool weighted = e.glu_w && g < e.glu_groups;
