@@ -50,7 +50,7 @@ typedef struct L3Config {
 
 #define L3_FLAG_NO_GRAPH 1      /* never capture CUDA graphs (debug)                      */
 #define L3_FLAG_NO_TENSORCORE 2 /* keep SIMT GEMMs (A/B against the tcgen05 kernels)         */
-#define L3_FLAG_NO_PDL 4        /* process-wide: no programmatic dependent launch           */
+#define L3_FLAG_NO_PDL 4        /* no programmatic dependent launches by this handle        */
 #define L3_FLAG_NO_MEGA 8       /* batch-1 decode as one kernel per projection (A/B against
                                    the persistent single-kernel step)                       */
 

@@ -20,8 +20,9 @@ typedef __nv_bfloat16 bf16;
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-extern bool g_l3_pdl;  // l3_api.cu; false = plain stream-ordered launches
-extern bool g_l3_pdl_next;  // l3_api.cu; set right before ONE launch that should overlap its predecessor's tail (consumed by launch_k)
+// l3_api.cu; of the calling thread: launches of a scope (PdlScope, internal.h), and set right before ONE launch that should overlap its
+// predecessor's tail (consumed by launch_k)
+extern thread_local bool g_l3_pdl, g_l3_pdl_next;
 // Pins a kernel to the max-shared-memory carveout (once per function and device).  The tcgen05
 // GEMM needs ~200 KB of shared memory; if its neighbours in the stream ran with the default
 // carveout every GEMM launch would pay an SM drain + L1/shared reconfiguration.

@@ -7,6 +7,12 @@
 void set_err(L3Model* m, const char* fmt, ...);  // l3_api.cu
 int make_err_word(L3Model* m);                   // L3Model::h_err
 int check_waits(L3Model* m);                     // behind a synchronisation: did a kernel of the calls before it give up waiting?
+// The calling thread's launches are programmatic dependents of their predecessors for as long as this lives (where it pays; see pdl_pays)
+struct PdlScope {
+  const bool before;
+  PdlScope(const L3Model* m, bool pays);
+  ~PdlScope();
+};
 extern const bool g_l3_debug_sync;               // L3_DEBUG_SYNC=1: synchronise after every launch
 
 #define CK(m, call)                                                                         \

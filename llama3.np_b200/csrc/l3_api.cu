@@ -22,9 +22,14 @@
 
 static thread_local char g_err[512] = "";
 const bool g_l3_debug_sync = getenv("L3_DEBUG_SYNC") && atoi(getenv("L3_DEBUG_SYNC")) != 0;
-bool g_l3_pdl_next = false;  // one-shot: the next launch is a programmatic dependent of its predecessor (linear())
-bool g_l3_pdl = false;  // programmatic dependent launch for step kernels (common.cuh); measured slower
-                        // than plain graph edges on this workload, so opt-in (L3_PDL=1)
+thread_local bool g_l3_pdl_next = false;  // one-shot: the next launch is a programmatic dependent of its predecessor (linear())
+thread_local bool g_l3_pdl = false;       // programmatic dependent launches (PdlScope)
+// L3_PDL: 0 nowhere, 1 in every scope whatever it holds
+static const int g_l3_pdl_env = getenv("L3_PDL") ? (atoi(getenv("L3_PDL")) != 0 ? 1 : 0) : -1;
+PdlScope::PdlScope(const L3Model* m, bool pays) : before(g_l3_pdl) {
+  g_l3_pdl = !(m->cfg.flags & L3_FLAG_NO_PDL) && (g_l3_pdl_env < 0 ? pays : g_l3_pdl_env == 1);
+}
+PdlScope::~PdlScope() { g_l3_pdl = before; }
 
 #include <mutex>
 #include <set>
@@ -77,8 +82,6 @@ extern "C" int l3_create(const L3Config* c, L3Model** out) {
   REQUIRE(nullptr, c->tp_world <= L3_MAX_TP, "tensor parallel world %d exceeds %d", c->tp_world, L3_MAX_TP);
   REQUIRE(nullptr, c->max_batch_size >= 1 && c->max_seq_len >= 1 && c->vocab_size >= 1, "bad sizes");
 
-  if (getenv("L3_PDL")) g_l3_pdl = atoi(getenv("L3_PDL")) != 0;
-  if (c->flags & L3_FLAG_NO_PDL) g_l3_pdl = false;
   L3Model* m = new L3Model();
   m->cfg = *c;
   m->bf16 = c->dtype == L3_DTYPE_BF16;
@@ -606,8 +609,8 @@ static int linear(L3Model* m, LinearArgs& a, Feed feed, const float* w_hi, const
   // Decode-sized batches: every swapped-role GEMM is launched as a programmatic dependent of whatever precedes it
   // (RMSNorm, attention, the previous GEMM), so that its prologue - TMEM allocation, barriers, tensor-map prefetch, the
   // first weight stage - runs under the predecessor's tail.  Measured at the 8B shape, ms per decode step at 32 rows:
-  // off 4.34, behind RMSNorm only 4.27, every GEMM 4.17; at 128 rows (a 128-token prefill) it costs 6 %, and on every
-  // kernel of the step (L3_PDL=1) it loses, so: these launches only.  L3_PDL_GEMM: 0 off, 1 behind RMSNorm, 2 all.
+  // off 4.34, behind RMSNorm only 4.27, every GEMM 4.17; every kernel of the step
+  // (L3_PDL=1) is no better at 32 rows, see pdl_pays.  L3_PDL_GEMM: 0 off, 1 behind RMSNorm, 2 all.
   static const int pdl_gemm = [] { const char* v = getenv("L3_PDL_GEMM"); return v ? atoi(v) : 2; }();
   if (swap_on && gemm_swap_supported(a.rows, a.N)) {  // 9..128 rows: weights as the 128-row operand
     g_l3_pdl_next = ((norm && pdl_gemm == 1) || pdl_gemm == 2) && a.rows <= 32 && !(m->cfg.flags & L3_FLAG_NO_PDL);
@@ -668,6 +671,23 @@ static int enqueue_cluster_layers(L3Model* m, const int32_t* d_ids, int ids_ld, 
   return L3_OK;
 }
 
+// Programmatic dependent launches: the kernels of a chunk are a chain, each of which waits for its predecessor (pdl_wait) ahead of its first
+// dependent access, so a kernel's prologue and its share of the launch latency run under the predecessor's tail.  Off : on, us.  Prompts:
+// 1B layers 33 tokens 224 : 198, 128 259 : 235, 2 x 731 494 : 464; 8B layers 33 337 : 319, 200 398 : 365, 800 773 : 749; stories15M 2
+// tokens 273 : 224, 100 666 : 593, 32 x 100 1096 : 1004.  Not 9 - 32 rows of layers that L2 does not hold, where every product waits for
+// DRAM and the swapped products are dependents already (8B, 9 tokens 269 : 263, 20 284 : 294, 32 287 : 296; 1B, 32 197 : 177).  Steps of 9 -
+// 16 sequences: 1B 9 sequences 1923 : 1759 a call, 16 1960 : 1805, 32 2222 : 2227, 8B 9 3393 : 3298, 16 3470 : 3444, 32 3806 : 3833, fp32
+// stories15M 9 5570 : 5403, 16 5597 : 5639, 30 6828 : 7182.  Layer lists: latent attention of width 2048 0.69 : 0.62 ms a step, 3.20 : 3.02
+// ms a prompt of 2048 tokens; prompts of 2048 tokens: linear mixers of width 2048 1042 : 982 us, parallel
+// layers 888 : 839, states and experts 1729 : 1688; eight sequences through chunk attention and matrix memories 6340 : 5612 us for 32 tokens.  NCCL's kernels between them take no part (tensor parallelism).
+static bool pdl_pays(const L3Model* m, int ntok, int L) {
+  if (m->ll) return true;
+  if (m->G > 1) return false;
+  if (L == 1) return ntok > 8 && ntok <= 16;
+  const size_t layer = ((size_t)(m->qkv_rows + m->HN * m->HD) * m->D + (size_t)3 * m->FD * m->D) * (m->bf16 ? 2 : 4);
+  return ntok <= 8 || ntok > 32 || layer <= (size_t)126 << 20;
+}
+
 // Enqueue one chunk: tokens ids[b * ids_ld + ids_off + t], t < L, at start_pos = *d_pos.
 // Layer-list handles: d_rows / n_rows choose the rows whose logits are wanted (null: the last token of every sequence),
 // d_resid (may be null) receives the residual stream after every layer.
@@ -675,6 +695,7 @@ static int enqueue_chunk(L3Model* m, const int32_t* d_ids, int ids_ld, int ids_o
                          bool want_argmax, OutSpec os, const Ragged* rg = nullptr, const int32_t* d_rows = nullptr,
                          int n_rows = 0, float* d_resid = nullptr) {
   const int ntok = B * L, D = m->D, HD = m->HD;
+  PdlScope pdl(m, pdl_pays(m, ntok, L));
   if (m->ll) {
     LAUNCH(m, launch_embed(m->embed, m->bf16, d_ids, ids_ld, ids_off, L, ntok, D, m->cfg.vocab_size, m->x, m->stream));
     int rc = ll_enqueue_layers(m, d_ids, ids_ld, ids_off, B, L, d_resid);

@@ -2191,18 +2191,6 @@ static int ll_enqueue_parallel(L3Model* m, int B, int L, float* d_resid) {
 }
 
 // ------------------------------------------------------------------------------ the layers of one chunk
-// Pre-norm layers are long chains of short kernels, every one of which waits for its predecessor (pdl_wait) ahead of its first
-// dependent access: launched as programmatic dependents, a kernel's prologue and its share of the launch latency run under the
-// predecessor's tail.  Measured on a latent-attention stack of width 2048: 0.69 -> 0.62 ms per decode step, 3.20 -> 3.02 ms
-// per 2048-token prompt; at width 1024 no difference.  L3_PDL=0 turns it off.
-namespace {
-struct PdlScope {
-  const bool before = g_l3_pdl;
-  explicit PdlScope(bool on) { if (on) g_l3_pdl = true; }
-  ~PdlScope() { g_l3_pdl = before; }
-};
-}  // namespace
-
 int ll_enqueue_layers(L3Model* m, const int32_t* d_ids, int ids_ld, int ids_off, int B, int L, float* d_resid) {
   LayerList* ll = m->ll;
   const int ntok = B * L, W = m->D, sd = ll->cfg.side_dim;
@@ -2216,11 +2204,7 @@ int ll_enqueue_layers(L3Model* m, const int32_t* d_ids, int ids_ld, int ids_off,
   ll->xalt = ll->x2;
   LLPending pd;
   if (ll->cfg.parallel) return ll_enqueue_parallel(m, B, L, d_resid);
-  if (ll->cfg.norm_input) {
-    static const bool off = getenv("L3_PDL") && atoi(getenv("L3_PDL")) == 0;
-    PdlScope pdl(!off && !(m->cfg.flags & L3_FLAG_NO_PDL));
-    return ll_enqueue_prenorm(m, B, L, d_resid);
-  }
+  if (ll->cfg.norm_input) return ll_enqueue_prenorm(m, B, L, d_resid);
   // rows <= 8 never reach a tensor-core projection of the residual stream: no mirror needed
   if (x16 && !linear_rows_supported(ntok, W)) LAUNCH(m, launch_to_bf16(m->x, (int64_t)ntok * W, x16, m->stream));
   for (int ri = 0; ri < (int)ll->runs.size(); ++ri) {
