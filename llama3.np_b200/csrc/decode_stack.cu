@@ -533,10 +533,9 @@ __global__ void __launch_bounds__(Cf::NTHREADS, 1) decode_stack_kernel(const __g
   const int rank = (int)cluster_ctarank();
   const int b0 = (int)(blockIdx.x / C) * S;           // first sequence of this cluster
   const int s_act = min(S, a.B - b0);                  // sequences that exist
-  const int step = a.scal[1] + 1;                      // llama3.py:316-318: decode step i runs at pos = L + i
-  const int pos = a.scal[2] + step;
-  const int nch = (pos + TCH - 1) / TCH;               // attention units per sequence: cache rows [0, pos)
+  auto position = [&]() { return a.scal[2] + a.scal[1] + 1; };  // llama3.py:316-318: decode step i runs at pos = L + i; behind pdl_wait
 
+  pdl_launch();
   SK_STAMP(a, 63);
   if (t == 0) {
     for (int s = 0; s < Cf::ST; ++s) { mbar_init(rg.full(s), 1); mbar_init(rg.empty(s), Cf::NCW); }
@@ -562,8 +561,9 @@ __global__ void __launch_bounds__(Cf::NTHREADS, 1) decode_stack_kernel(const __g
       // the projection phases between them leave HBM idle: as soon as layer l - 1's attention has drained the
       // ring, one thread asks L2 for the first pf_rows cache rows of layer l's K / V of this CTA's head
       // (cp.async.bulk.prefetch.L2: no destination, no completion), so the ring's copies find them in L2.
+      pdl_wait();
       if (lane == 0 && a.pf_rows > 0) {
-        const uint32_t bytes = (uint32_t)min(pos, a.pf_rows) * HD * 4;
+        const uint32_t bytes = (uint32_t)min(position(), a.pf_rows) * HD * 4;
         for (int l = 1; l < a.NL; ++l) {
           uint32_t spins = 0;
           while (*prog < l) {
@@ -604,6 +604,7 @@ __global__ void __launch_bounds__(Cf::NTHREADS, 1) decode_stack_kernel(const __g
         for (int sl = 0; sl < K / ks; ++sl, ++n)
           if ((int)(n % Cf::NISS) == pw) issue(w + (size_t)sl * ks * F, (uint32_t)(ks * F * 4), nullptr, 0u, 0u);
       };
+      int pos = 0, nch = 0;  // nch: attention units per sequence: cache rows [0, pos)
       auto kv_units = [&](const StackLayer& ly) {
         uint32_t u = n;
         kv_hint = a.kv_evict_first != 0;
@@ -627,6 +628,11 @@ __global__ void __launch_bounds__(Cf::NTHREADS, 1) decode_stack_kernel(const __g
         const float* w = ly.wpack + (size_t)rank * Cf::CTA_FLOATS;
         slabs(w, Cf::FA, Cf::KA, Cf::GA);
         w += Cf::KA * Cf::FA;
+        if (l == 0) {  // the first weights were constants; positions and caches come from the step before
+          pdl_wait();
+          pos = position();
+          nch = (pos + TCH - 1) / TCH;
+        }
         kv_units(ly);
         slabs(w, Cf::FB, Cf::KB, Cf::GB);
         w += Cf::KB * Cf::FB;
@@ -641,6 +647,8 @@ __global__ void __launch_bounds__(Cf::NTHREADS, 1) decode_stack_kernel(const __g
     // ================================================================== compute warps
     uint32_t n = 0;
     const float scale = 1.0f / sqrtf((float)HD);
+    pdl_wait();
+    const int pos = position(), nch = (pos + TCH - 1) / TCH;
     // x = tok_embedding[token] (llama3.py:287), k-major; rows of sequences beyond the batch stay zero
     if (t < S) tok[t] = t < s_act ? a.d_next[b0 + t] : -1;
     if (t < HD / 2) {
@@ -948,8 +956,10 @@ __global__ void stack_pack_kernel(const float* __restrict__ wqkv, const float* _
   }
 }
 
-__global__ void stack_finalize_kernel(unsigned long long* __restrict__ best, int B, int32_t* __restrict__ next_ids,
+__global__ void __launch_bounds__(256) stack_finalize_kernel(unsigned long long* __restrict__ best, int B, int32_t* __restrict__ next_ids,
                                       int64_t* __restrict__ tokens, int stride, int* __restrict__ scal) {
+  pdl_launch();
+  pdl_wait();
   const int step = scal[1] + 1;
   for (int r = threadIdx.x; r < B; r += blockDim.x) {
     const unsigned long long k = best[r];
@@ -988,8 +998,10 @@ template <class Cf> void fill_cfg(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* 
   at[0].val.clusterDim.x = Cf::C;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // its first weights are drawn in the predecessor's tail
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = g_l3_pdl ? 2 : 1;
 }
 
 }  // namespace
@@ -1013,7 +1025,7 @@ int decode_stack_max_clusters() {
   using Cf = Stories15M;
   if (prepare<Cf>() != cudaSuccess) { cudaGetLastError(); return 0; }
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   fill_cfg<Cf>(cfg, at, 1, nullptr);
   int n = 0;
   if (cudaOccupancyMaxActiveClusters(&n, decode_stack_kernel<Cf>, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
@@ -1025,13 +1037,12 @@ cudaError_t launch_decode_stack(const StackArgs& a, int, int, int, int, cudaStre
   cudaError_t e = prepare<Cf>();
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   fill_cfg<Cf>(cfg, at, (a.B + Cf::S - 1) / Cf::S, s);
   return cudaLaunchKernelEx(&cfg, decode_stack_kernel<Cf>, a);
 }
 
 cudaError_t launch_stack_finalize(unsigned long long* best, int B, int32_t* next_ids, int64_t* tokens, int stride, int* scal,
                                   cudaStream_t s) {
-  stack_finalize_kernel<<<1, 256, 0, s>>>(best, B, next_ids, tokens, stride, scal);
-  return cudaGetLastError();
+  return launch_k(stack_finalize_kernel, dim3(1), dim3(256), 0, s, best, B, next_ids, tokens, stride, scal);
 }

@@ -974,6 +974,7 @@ static int enqueue_decode_stack(L3Model* m, int B, int part = 0) {
   static const int pf_rows = [] { const char* v = getenv("L3_STACK_PF"); return v ? atoi(v) : 64; }();
   static const int kv_ef = [] { const char* v = getenv("L3_STACK_KV_EVICT_FIRST"); return v ? atoi(v) : 1; }();
   a.pf_rows = pf_rows; a.kv_evict_first = kv_ef;
+  PdlScope pdl(m, m->G == 1);  // 64 tokens of 256 sequences 19030 : 18860 us
   if (part != 2) LAUNCH(m, launch_decode_stack(a, m->D, m->HN, m->HD, m->FD, m->stream));
   if (part == 1) return L3_OK;
   TcGemmArgs t{};
@@ -996,7 +997,6 @@ static int enqueue_decode_nodes(L3Model* m, int B, int ragged, int eos) {
     if (eos >= 0) LAUNCH(m, launch_ragged_eos(m->d_next, m->d_done, eos, B, m->d_tokens, m->M, m->d_scal + 1, m->stream));
     return L3_OK;
   }
-  if (m->stack_ok && B >= m->stack_min_B) return enqueue_decode_stack(m, B);
   // Small fp32 models: layers in one cluster, then the LM head with its argmax.  stories15M, us per call before (batch 1: decode_mega,
   // 2 - 8: a kernel per product) -> here.  5 + 45 tokens: batch 1 5466 -> 3463, 2 9461 -> 4355, 4 12295 -> 5951, 8 19050 -> 9791; 400 + 111
   // tokens: batch 1 14821 -> 10985, 2 23670 -> 12857, 4 30876 -> 20772, 5 38503 -> 29316, 8 47911 -> 36211.  One forward step at position
@@ -1023,6 +1023,9 @@ static int enqueue_decode_nodes(L3Model* m, int B, int ragged, int eos) {
 static int decode_step(L3Model* m, int B, int ragged = 0, int eos = -1) {
   if (m->ll)
     for (int b = 0; b < B; ++b) m->ll->slot_pos[b] += 1;
+  // three launches a step, which the host makes long before the step ends: out of a graph the first is a dependent of the step before
+  // (64 tokens of 256 sequences 18860 -> 18700 us; the two launches of a step in one cluster gain nothing)
+  if (!ragged && m->stack_ok && B >= m->stack_min_B) return enqueue_decode_stack(m, B);
   L3Graph* g = nullptr;
   const int key = ragged ? ragged + 4 * (eos + 1) : 0;  // the EOS id is baked into the captured node
   for (auto& it : m->graphs)
