@@ -15,7 +15,7 @@
 //  2. channel_chain_kernel  a CTA per (16 value columns, head, sequence) walks the chunks: S^T (16 x DK) stays in fp32 accumulator
 //                           registers - a warp owns 16 key channels -, which are the left operand of the next product without a
 //                           move.  Per chunk two products against S (W and the decayed queries), a sum over the warps through shared
-//                           memory, then the state's and the outputs' products with U; operand blocks are fetched a phase ahead.
+//                           memory, then the state's and the outputs' products with U; operand blocks are fetched a chunk ahead.
 // Every exponential has an argument <= 0: c is kept relative to blocks of 16 tokens, products between blocks take a reference
 // between them (e^(c_t - ref) e^(ref - c_j)), 8 x 8 blocks on the diagonal are formed pair by pair.  All operands of the tensor
 // products - keys, queries, scores, T, U and the state - are pairs hi + lo of bf16 values (right to 2^-18), a product is
@@ -54,11 +54,6 @@ __device__ __forceinline__ void mma3(float (&c)[4], const uint32_t (&ah)[4], con
   mma16816(c, al, b.x, b.y);
   mma16816(c, ah, b.z, b.w);
 }
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // One (chunk, head, sequence) of the workspace, in 16-byte units: operand blocks W and decayed queries [token tile 8][k step DK / 16]
 // [lane], decayed keys [channel tile DK / 8][k step 4][lane], B [token tile 8][k step 4][lane], then e^(c_C) and U' as floats
@@ -388,16 +383,17 @@ __global__ void __launch_bounds__(512) channel_chunk_kernel(RecurArgs a, int c0)
 
 // ---------------------------------------------------------------------------------------------- 2. the chain over the chunks
 // grid (DV / 16, H, B); DK / 16 warps, warp w owns key channels 16 w .. 16 w + 15 of S^T and the token tiles w, w + DK / 16, ..
+// Bound by shared memory's and L1's throughput (65 % with the waits around its two barriers) and by latencies.  The operand blocks, of
+// which every one is read once, come straight into registers, asked for where the block of the chunk before was used last; through shared
+// memory (written and read: half of its traffic) it took two more barriers a chunk: 2048 tokens, 16 heads of 128 x 128 89.6 -> 78 us, 3 x 701 tokens,
+// 8 heads of 128 x 256 without the delta rule 67.6 -> 56.  The state shared as an operand in place of the partial products' exchange:
+// 76 -> 71 us alone, nothing for a prompt, and 56 -> 60.
 template <int DK, bool DELTA>
 __global__ void __launch_bounds__(DK * 2, 1) channel_chain_kernel(RecurArgs a, int c0, int NC) {
   extern __shared__ __align__(16) uint4 sm4[];
   using Wk = Ws<DK>;
   constexpr int NW = DK / 16, TH = DK * 2, TPW = 8 / NW;
-  uint4* sW = sm4;                                       // W (delta) and decayed queries
-  uint4* sQ = sW + (DELTA ? Wk::W : 0);
-  uint4* sK = sQ + Wk::Q;                                // decayed keys
-  uint4* sB = sK + Wk::K;
-  float4* exU = reinterpret_cast<float4*>(sB + Wk::B);   // [warp][token tile][lane] partial products with S
+  float4* exU = reinterpret_cast<float4*>(sm4);          // [warp][token tile][lane] partial products with S
   float4* exO = exU + (DELTA ? NW * 256 : 0);
   uint4* sU = reinterpret_cast<uint4*>(exO + NW * 256);  // U^T as left operand: [k step 4][hi, lo][lane]
   pdl_launch();
@@ -413,43 +409,49 @@ __global__ void __launch_bounds__(DK * 2, 1) channel_chain_kernel(RecurArgs a, i
   for (int t = 0; t < 2; ++t)
 #pragma unroll
     for (int u = 0; u < 4; ++u) sacc[t][u] = st[(size_t)(warp * 16 + t * 8 + q2 + (u & 1)) * a.DV + g + (u >> 1) * 8];
-  auto fetch_wq = [&](int c) {
-    if (c < NC) {
-      const uint4* src = ws + (size_t)c * per + (DELTA ? 0 : Wk::oQ);
-      for (int i = tid; i < (DELTA ? Wk::W : 0) + Wk::Q; i += TH) cp_async16(sW + i, src + i);
-    }
-    cp_commit();
+  // Operands of the chunk at hand; each is asked for anew for the next chunk where it was used last
+  uint4 rW[DELTA ? 8 : 1], rQ[8], rK[2][4], rB[TPW][4];
+  float uv[TPW][4], ec[2][2];  // U' or V at value columns g, g + 8 and tokens q2, q2 + 1 of this lane's tiles; the chunk's decays
+  auto get_q = [&](int c, int nt) {
+    const uint4* w = ws + (size_t)c * per + (nt * NW + warp) * 32 + lane;
+    if (DELTA) rW[nt] = __ldcg(w);
+    rQ[nt] = __ldcg(w + Wk::oQ);
   };
-  auto fetch_kb = [&](int c) {
-    if (c < NC) {
-      const uint4* src = ws + (size_t)c * per + Wk::oK;
-      for (int i = tid; i < Wk::K + Wk::B; i += TH) cp_async16(sK + i, src + i);
-    }
-    cp_commit();
+  auto get_k = [&](int c, int ks) {
+    const uint4* w = ws + (size_t)c * per + ks * 32 + lane;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) rK[t][ks] = __ldcg(w + Wk::oK + (warp * 2 + t) * 128);
+#pragma unroll
+    for (int p = 0; p < TPW; ++p)
+      if (ks <= (warp + p * NW) >> 1) rB[p][ks] = __ldcg(w + Wk::oB + (warp + p * NW) * 128);  // keys up to the query
   };
-  fetch_wq(0);
-  fetch_kb(0);
+  auto get_u = [&](int c, int p) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int t = (warp + p * NW) * 8 + q2 + (u & 1), e = e0 + g + (u >> 1) * 8;
+      if (DELTA) uv[p][u] = __ldcg(reinterpret_cast<const float*>(ws + (size_t)c * per + Wk::oU) + (size_t)t * a.DV + e);
+      else uv[p][u] = (c0 + c) * CT + t < a.L ? a.v[((size_t)b * a.L + (size_t)(c0 + c) * CT + t) * a.ld_v + (size_t)h * a.DV + e] : 0.f;
+    }
+  };
+  auto get_e = [&](int c) {
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const float2 v = __ldcg(reinterpret_cast<const float2*>(reinterpret_cast<const float*>(ws + (size_t)c * per + Wk::oE) + warp * 16 + t * 8 + q2));
+      ec[t][0] = v.x; ec[t][1] = v.y;
+    }
+  };
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt) get_q(0, nt);
+#pragma unroll
+  for (int p = 0; p < TPW; ++p) get_u(0, p);
+  get_e(0);
+#pragma unroll
+  for (int ks = 0; ks < 4; ++ks) get_k(0, ks);
 #pragma unroll 1
   for (int c = 0; c < NC; ++c) {
     const int n = min(CT, a.L - (c0 + c) * CT);
     const size_t row0 = (size_t)b * a.L + (size_t)(c0 + c) * CT;
-    // what this lane needs of U' or V (value columns g, g + 8; tokens q2, q2 + 1 of its tiles) and the chunk's decays
-    float uv[TPW][4], ec[2][2];
-#pragma unroll
-    for (int p = 0; p < TPW; ++p)
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int t = (warp + p * NW) * 8 + q2 + (u & 1), e = e0 + g + (u >> 1) * 8;
-        if (DELTA) uv[p][u] = reinterpret_cast<const float*>(ws + (size_t)c * per + Wk::oU)[(size_t)t * a.DV + e];
-        else uv[p][u] = t < n ? a.v[(row0 + t) * a.ld_v + (size_t)h * a.DV + e] : 0.f;
-      }
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-      const float2 v = *reinterpret_cast<const float2*>(reinterpret_cast<const float*>(ws + (size_t)c * per + Wk::oE) + warp * 16 + t * 8 + q2);
-      ec[t][0] = v.x; ec[t][1] = v.y;
-    }
-    cp_wait<1>();
-    __syncthreads();
+    const bool more = c + 1 < NC;
     {
       uint32_t ah[4], al[4];
       split2(sacc[0][0], sacc[0][1], ah[0], al[0]); split2(sacc[0][2], sacc[0][3], ah[1], al[1]);
@@ -458,16 +460,16 @@ __global__ void __launch_bounds__(DK * 2, 1) channel_chain_kernel(RecurArgs a, i
       for (int nt = 0; nt < 8; ++nt) {
         if (DELTA) {
           float p[4] = {};
-          mma3(p, ah, al, sW[(nt * NW + warp) * 32 + lane]);
+          mma3(p, ah, al, rW[nt]);
           exU[(warp * 8 + nt) * 32 + lane] = make_float4(p[0], p[1], p[2], p[3]);
         }
         float p[4] = {};
-        mma3(p, ah, al, sQ[(nt * NW + warp) * 32 + lane]);
+        mma3(p, ah, al, rQ[nt]);
         exO[(warp * 8 + nt) * 32 + lane] = make_float4(p[0], p[1], p[2], p[3]);
+        if (more) get_q(c + 1, nt);
       }
     }
     __syncthreads();
-    fetch_wq(c + 1);
     float o[TPW][4];
 #pragma unroll
     for (int p = 0; p < TPW; ++p) {
@@ -485,6 +487,7 @@ __global__ void __launch_bounds__(DK * 2, 1) channel_chain_kernel(RecurArgs a, i
       o[p][0] = so.x; o[p][1] = so.y; o[p][2] = so.z; o[p][3] = so.w;
       float u0 = uv[p][0], u1 = uv[p][1], u2 = uv[p][2], u3 = uv[p][3];
       if (DELTA) { u0 -= su.x; u1 -= su.y; u2 -= su.z; u3 -= su.w; }
+      if (more) get_u(c + 1, p);
       uint2 hi, lo;                                      // half of an operand's four registers: tokens (nt & 1) * 8 + q2 of step nt / 2
       split2(u0, u1, hi.x, lo.x);
       split2(u2, u3, hi.y, lo.y);
@@ -492,19 +495,20 @@ __global__ void __launch_bounds__(DK * 2, 1) channel_chain_kernel(RecurArgs a, i
       dst[0] = hi;
       dst[64] = lo;                                      // 32 lanes of 16 bytes further
     }
-    cp_wait<1>();
     __syncthreads();
 #pragma unroll
     for (int t = 0; t < 2; ++t) { sacc[t][0] *= ec[t][0]; sacc[t][1] *= ec[t][1]; sacc[t][2] *= ec[t][0]; sacc[t][3] *= ec[t][1]; }
+    if (more) get_e(c + 1);
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
       const uint4 uh = sU[(ks * 2) * 32 + lane], ul = sU[(ks * 2 + 1) * 32 + lane];
       const uint32_t ah[4] = {uh.x, uh.y, uh.z, uh.w}, al[4] = {ul.x, ul.y, ul.z, ul.w};
 #pragma unroll
-      for (int t = 0; t < 2; ++t) mma3(sacc[t], ah, al, sK[((warp * 2 + t) * 4 + ks) * 32 + lane]);
+      for (int t = 0; t < 2; ++t) mma3(sacc[t], ah, al, rK[t][ks]);
 #pragma unroll
       for (int p = 0; p < TPW; ++p)
-        if (ks <= (warp + p * NW) >> 1) mma3(o[p], ah, al, sB[((warp + p * NW) * 4 + ks) * 32 + lane]);  // keys up to the query
+        if (ks <= (warp + p * NW) >> 1) mma3(o[p], ah, al, rB[p][ks]);
+      if (more) get_k(c + 1, ks);
     }
 #pragma unroll
     for (int p = 0; p < TPW; ++p)
@@ -513,10 +517,7 @@ __global__ void __launch_bounds__(DK * 2, 1) channel_chain_kernel(RecurArgs a, i
         const int t = (warp + p * NW) * 8 + q2 + (u & 1);
         if (t < n) a.out[(row0 + t) * O + (size_t)h * a.DV + e0 + g + (u >> 1) * 8] = o[p][u];
       }
-    __syncthreads();
-    fetch_kb(c + 1);
   }
-  cp_wait<0>();
 #pragma unroll
   for (int t = 0; t < 2; ++t)
 #pragma unroll
@@ -529,7 +530,7 @@ template <int DK, bool DELTA>
 cudaError_t launch_channel_t(const RecurArgs& a, cudaStream_t s) {
   using Wk = Ws<DK>;
   const size_t sm1 = (size_t)chunk_floats<DK>(DELTA) * sizeof(float);
-  const size_t sm2 = (size_t)((DELTA ? Wk::W : 0) + Wk::Q + Wk::K + Wk::B + (DELTA ? 2 : 1) * (DK / 16) * 256 + 256) * 16;
+  const size_t sm2 = (size_t)((DELTA ? 2 : 1) * (DK / 16) * 256 + 256) * 16;
   cudaError_t e;
   if ((e = cudaFuncSetAttribute(channel_chunk_kernel<DK, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1)) != cudaSuccess) return e;
   if ((e = cudaFuncSetAttribute(channel_chain_kernel<DK, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2)) != cudaSuccess) return e;
