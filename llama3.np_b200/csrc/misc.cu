@@ -251,6 +251,8 @@ cudaError_t launch_argmax_keys(const float* logits, int rows, int n, int col_off
 
 // [G, rows, n] rank-major all-gathered slices -> [rows, G * n]
 __global__ void gather_permute_kernel(const float* __restrict__ in, int G, int rows, int n, float* __restrict__ out) {
+  pdl_launch();
+  pdl_wait();
   const int64_t total = (int64_t)G * rows * n;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int c = (int)(i % n);
