@@ -832,11 +832,11 @@ cudaError_t launch_diff_attn(const DiffAttnArgs& a, bool kv_bf16, float* part_o,
   const dim3 grid((unsigned)((size_t)a.B * a.L * a.H));
   if (kv_bf16) {
     auto kern = attn_diff_cta_kernel<bf16>;
-    if (smem > 48 * 1024) { cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); if (e != cudaSuccess) return e; }
+    if (const cudaError_t e = allow_smem(kern, smem)) return e;
     return launch_k(kern, grid, dim3(DIFF_CTA_WARPS * 32), smem, s, a);
   }
   auto kern = attn_diff_cta_kernel<float>;
-  if (smem > 48 * 1024) { cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); if (e != cudaSuccess) return e; }
+  if (const cudaError_t e = allow_smem(kern, smem)) return e;
   return launch_k(kern, grid, dim3(DIFF_CTA_WARPS * 32), smem, s, a);
 }
 

@@ -297,10 +297,7 @@ __global__ void __launch_bounds__(32 * FW * GR, GR == 1 && NC <= 2 ? 2 : 1) attn
 
 template <int NC, int GR> cudaError_t launch_gr(const WinAttnArgs& a, dim3 grid, cudaStream_t s) {
   const size_t smem = smem_bytes(a.DK, a.DV, GR);
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(attn_f32_kernel<NC, GR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  if (const cudaError_t e = allow_smem(attn_f32_kernel<NC, GR>, smem)) return e;
   return launch_k(attn_f32_kernel<NC, GR>, grid, dim3(32 * FW * GR), smem, s, a);
 }
 template <int NC> cudaError_t launch_nc(const WinAttnArgs& a, cudaStream_t s) {

@@ -611,10 +611,7 @@ int win_nj(int DV) { return DV <= 32 ? 1 : DV <= 64 ? 2 : DV <= 128 ? 4 : DV <= 
 template <typename KVT, int NJ>
 cudaError_t launch_win_nj(const WinAttnArgs& a, dim3 grid, cudaStream_t s) {
   const size_t smem = win_attn_smem(a.DK, NJ);
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(win_attn_kernel<KVT, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  if (const cudaError_t e = allow_smem(win_attn_kernel<KVT, NJ>, smem)) return e;
   return launch_k(win_attn_kernel<KVT, NJ>, grid, dim3(256), smem, s, a);
 }
 
@@ -644,10 +641,7 @@ cudaError_t launch_win_decode(const WinAttnArgs& a, cudaStream_t s) {
   const bool cl = win_decode_in_cluster<KVT>(a);
   const size_t smem = ((size_t)REP * a.DK + REP * WD_KEYS + 3 * REP + 4 + (size_t)parts * REP * a.DV + (cl ? (size_t)REP * (a.DV + 9) : 0)) * sizeof(float);
   auto kern = cl ? win_decode_kernel<KVT, REP, true> : win_decode_kernel<KVT, REP, false>;
-  if (smem > 40 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  if (const cudaError_t e = allow_smem(kern, smem)) return e;
   return launch_kc(kern, dim3(a.nsplit, a.G, a.B), dim3(256), smem, s, cl ? a.nsplit : 1, a);
 }
 

@@ -27,6 +27,13 @@ extern thread_local bool g_l3_pdl, g_l3_pdl_next;
 // GEMM needs ~200 KB of shared memory; if its neighbours in the stream ran with the default
 // carveout every GEMM launch would pay an SM drain + L1/shared reconfiguration.
 bool l3_carveout_seen(const void* fn);
+// Lets a kernel be launched with `smem` bytes of dynamic shared memory: its limit goes to all that an SM has beside its static part, once per
+// function and device.  The limit belongs to the function and not to a launch, so where head sizes share a kernel a limit of one call's size
+// could be lowered by another thread's call between this call's setting and its launch.
+cudaError_t l3_raise_smem(const void* fn);
+template <typename... KArgs> static inline cudaError_t allow_smem(void (*kern)(KArgs...), size_t smem) {
+  return smem > 32 * 1024 ? l3_raise_smem((const void*)kern) : cudaSuccess;
+}
 // cluster: blocks per thread-block cluster
 template <typename... KArgs, typename... Args>
 static inline cudaError_t launch_kc(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, int cluster, Args... args) {

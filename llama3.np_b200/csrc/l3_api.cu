@@ -43,6 +43,22 @@ bool l3_carveout_seen(const void* fn) {
   return !seen.insert({dev, fn}).second;
 }
 
+cudaError_t l3_raise_smem(const void* fn) {
+  static std::mutex mu;
+  static std::set<std::pair<int, const void*>> raised;
+  int dev = 0, most = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> g(mu);
+  if (raised.count({dev, fn})) return cudaSuccess;
+  cudaFuncAttributes at{};
+  if ((e = cudaFuncGetAttributes(&at, fn)) != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)at.sharedSizeBytes)) != cudaSuccess) return e;
+  raised.insert({dev, fn});
+  return cudaSuccess;
+}
+
 void set_err(L3Model* m, const char* fmt, ...) {  // also used by packed_io.cu
   char buf[512];
   va_list ap;

@@ -211,10 +211,7 @@ static cudaError_t launch_rows_t(const LinearArgs& a_in, cudaStream_t s) {
               : halves             ? linear_rows_kernel<WT, MB, EPI, KVT, 4, CAN>
                                    : linear_rows_kernel<WT, MB, EPI, KVT, 4, false>;
   const size_t smem = (size_t)MB * rows_stage_len(a.K, halves) * sizeof(float);
-  if (smem + 2048 > 48 * 1024) {  // the 48 KB default limit covers static + dynamic shared memory: opt in near it, too
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  if (const cudaError_t e = allow_smem(kern, smem)) return e;
   // choose warps per SM so that npairs / (148 * warps) sits just below an integer (balanced SMs)
   static const int max_wps = gemv_env("L3_GEMV_WPS", MB <= 2 ? 32 : 16);
   int best_w = 4;

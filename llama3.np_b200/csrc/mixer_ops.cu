@@ -463,10 +463,7 @@ cudaError_t launch_delta_prep(const DeltaPrepArgs& a, int rows, cudaStream_t s) 
     return launch_k(delta_prep_vec_kernel, dim3((a.L + CONV_TOKENS - 1) / CONV_TOKENS, (items + 7) / 8, rows / a.L), dim3(256), 0, s, a);
   }
   const size_t smem = (size_t)8 * a.DK * sizeof(float);
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(delta_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  if (const cudaError_t e = allow_smem(delta_prep_kernel, smem)) return e;
   const int items = 2 * a.G + 2 * a.H + 1;
   const int parts = rows <= 8 ? std::max(1, std::min(32, (items + 7) / 8)) : 1;  // few rows: a row's items spread over CTAs
   return launch_k(delta_prep_kernel, dim3(rows, parts), dim3(256), smem, s, a);

@@ -198,10 +198,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256) mlstm_step_ker
 template <int V, int CL>
 cudaError_t launch_step(const MlstmStepArgs& a, int B, cudaStream_t s) {
   const size_t smem = ((size_t)2 * a.DK + ((a.DV / CL + 3) & ~3) + 256 * V) * sizeof(float);
-  if (smem > 40 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(mlstm_step_kernel<V, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  if (const cudaError_t e = allow_smem(mlstm_step_kernel<V, CL>, smem)) return e;
   return launch_k(mlstm_step_kernel<V, CL>, dim3(CL, a.H, B), dim3(256), smem, s, a);
 }
 

@@ -747,8 +747,8 @@ cudaError_t launch_recur_chunk(const RecurArgs& a, cudaStream_t s) {
   const int n4 = (a.DK * a.DV + (a.n_state ? a.DK : 0)) / 4;
   auto go = [&](auto k_state, auto k_scan, auto k_out) {
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(k_state, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_out, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm3)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_state, sm1)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_out, sm3)) != cudaSuccess) return e;
     if ((e = launch_k(k_state, grid, dim3(256), sm1, s, a, NC)) != cudaSuccess) return e;
     if ((e = launch_k(k_scan, dim3((n4 + 255) / 256, a.H, a.B), dim3(256), 0, s, a, NC)) != cudaSuccess) return e;
     return launch_k(k_out, grid, dim3(256), sm3, s, a, NC);
@@ -760,8 +760,8 @@ cudaError_t launch_recur_chunk(const RecurArgs& a, cudaStream_t s) {
     auto go_mma = [&](auto k_state, auto k_scan, auto k_out) {
       const size_t sb1 = state_mma_smem(a.DK, pair), sb3 = out_mma_smem(a.DK, pair);
       cudaError_t e;
-      if ((e = cudaFuncSetAttribute(k_state, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb1)) != cudaSuccess) return e;
-      if ((e = cudaFuncSetAttribute(k_out, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb3)) != cudaSuccess) return e;
+      if ((e = allow_smem(k_state, sb1)) != cudaSuccess) return e;
+      if ((e = allow_smem(k_out, sb3)) != cudaSuccess) return e;
       if ((e = launch_k(k_state, dim3(NC * ne, a.H, a.B), dim3(256), sb1, s, a, NC, ne)) != cudaSuccess) return e;
       if ((e = launch_k(k_scan, dim3((n4 + 255) / 256, a.H, a.B), dim3(256), 0, s, a, NC)) != cudaSuccess) return e;
       return launch_k(k_out, dim3(NC * ne, a.H, a.B), dim3(256), sb3, s, a, NC, ne);

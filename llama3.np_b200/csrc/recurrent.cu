@@ -382,10 +382,7 @@ cudaError_t launch_recur_pipe(const RecurArgs& a, cudaStream_t s) {
   const size_t smem = (size_t)(2 * (RP_TCH * (NA * DKP + CPB) + RP_TCH) + RP_TCH * CPB) * sizeof(float);
   const dim3 grid(a.H * ((a.DV + (a.n_state ? 1 : 0) + CPB - 1) / CPB), a.B);
   auto go = [&](auto kern) {
-    if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-    }
+    if (const cudaError_t e = allow_smem(kern, smem)) return e;
     return launch_k(kern, grid, dim3(256), smem, s, a);
   };
   return a.mode == 0 ? go(recur_pipe_kernel<TPC, 0>) : a.mode == 1 ? go(recur_pipe_kernel<TPC, 1>) : go(recur_pipe_kernel<TPC, 2>);

@@ -174,10 +174,7 @@ cudaError_t launch_stream_t(const StreamArgs& a, int rows, cudaStream_t s) {
   }
   auto kern = stream_rows_kernel<NS, EXACT, VEC>;
   const size_t smem = a.in_w ? (size_t)a.D * sizeof(float) : 0;
-  if (smem > 40 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  if (const cudaError_t e = allow_smem(kern, smem)) return e;
   const int threads = a.D >= 1024 ? 256 : a.D >= 256 ? 128 : 64;
   return launch_k(kern, dim3(rows), dim3(threads), smem, s, a);
 }
