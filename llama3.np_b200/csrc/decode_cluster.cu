@@ -416,9 +416,10 @@ __global__ void __launch_bounds__(TH, 1) decode_cluster_kernel(const __grid_cons
 }
 
 // LM head: its argmax and the step's bookkeeping, or (LOGITS) the logits.  The layers ahead of it run on 16 SMs; on the others this kernel is
-// resident meanwhile, one CTA each, and draws its rows of W into shared memory (stories15M: 190 of 243 rows, 26 of 37 MB; the rest is asked
+// resident meanwhile, one CTA each, and draws its rows of W into shared memory (stories15M: 192 of 243 rows, 29 of 37 MB; the rest is asked
 // into L2).  Behind the wait there is the norm of x, a pass over shared memory and the merge of the maxima.  Four rows per warp and turn,
-// eight lanes per row.  stories15M, one sequence: from the layers' end to the step's 10.9 -> 8.3 us (a wait, three passes of few microseconds,
+// eight lanes per row, four chains of sums per lane: of stories15M's 288 terms a chain has nine, as in the row-streaming GEMV (one chain of 36
+// is 1.4 times as far from 64 bits).  stories15M, one sequence: from the layers' end to the step's 10.9 -> 8.3 us (a wait, three passes of few microseconds,
 // two rounds of atomics), a forward step with its logits 125.5 -> 113.5 us.
 constexpr int HT = 512, HW = HT / 32;
 template <int NB, bool LOGITS>
@@ -463,22 +464,24 @@ __global__ void __launch_bounds__(HT, 1) cluster_head_kernel(ClusterHeadArgs a, 
   auto four_rows = [&](const float* rows, int r0, int end, auto load) {  // rows r0 .. r0 + 3 of this CTA's, those below `end`
     const int r = r0 + (lane >> 3);
     const float* w = rows + (size_t)min(r, end - 1) * a.D;
-    float acc[NB];
+    float2 lo[NB], hi[NB];
 #pragma unroll
-    for (int b = 0; b < NB; ++b) acc[b] = 0.f;
-#pragma unroll 9
+    for (int b = 0; b < NB; ++b) lo[b] = hi[b] = make_float2(0.f, 0.f);
+    constexpr int AHEAD = NB <= 4 ? 9 : 3;  // of eight sequences nine do not fit the registers
+#pragma unroll AHEAD
     for (int k = sub * 4; k < a.D; k += 32) {
       const float4 wv = load(w + k);
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
         const float4 xv = *reinterpret_cast<const float4*>(xs + b * a.D + k);
-        acc[b] = fmaf(wv.x, xv.x, acc[b]); acc[b] = fmaf(wv.y, xv.y, acc[b]); acc[b] = fmaf(wv.z, xv.z, acc[b]); acc[b] = fmaf(wv.w, xv.w, acc[b]);
+        lo[b] = fma2(make_float2(wv.x, wv.y), make_float2(xv.x, xv.y), lo[b]);
+        hi[b] = fma2(make_float2(wv.z, wv.w), make_float2(xv.z, xv.w), hi[b]);
       }
     }
     __syncwarp();
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
-      float t = acc[b];
+      float t = (lo[b].x + lo[b].y) + (hi[b].x + hi[b].y);
 #pragma unroll
       for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(L3_FULL, t, o);
       if (LOGITS) {

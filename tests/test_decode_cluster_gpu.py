@@ -131,3 +131,24 @@ def test_head_of_every_vocabulary_size(vocab, B):
     want = np.concatenate(list(orc.OracleLlama(w, args).generate(ids, 30)), axis=1)
     m.close()
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("B", [1, 8])
+def test_logits_are_as_exact_as_short_chains_of_sums(B):
+    """Layers that add nothing: the logits are norm(embedding) W^T.  An fp32 rounding is 2.5e-8 of its value in the mean square, so 288
+    products as 32 chains of nine that meet in five steps (1440 + 5 x 288 partial sums of unit variance, and two roundings of the normed
+    row) are sqrt(12) of them or 8.8e-8 away from 64 bits; chains of 36 sqrt(23.5) or 1.23e-7.  The one factor of the norm is left out."""
+    args = ModelArgs(dim=288, n_layers=1, n_heads=6, n_kv_heads=6, vocab_size=32000, max_seq_len=8, max_batch_size=B)
+    w = make_weights(args, 768, seed=3)
+    w["model.layers.0.self_attn.o_proj.weight"][:] = 0
+    w["model.layers.0.mlp.down_proj.weight"][:] = 0
+    ids = np.arange(7, 7 + B)[:, None]
+    m = Llama(w, args)
+    got = np.asarray(m(ids, 0), np.float64).reshape(B, -1)
+    m.close()
+    x = w["model.embed_tokens.weight"][ids[:, 0]].astype(np.float64)
+    x = x / np.sqrt((x * x).mean(-1, keepdims=True) + args.norm_eps) * w["model.norm.weight"]
+    want = x @ w["lm_head.weight"].astype(np.float64).T
+    want *= (got * want).sum(-1, keepdims=True) / (want * want).sum(-1, keepdims=True)
+    err = np.linalg.norm(got - want, axis=-1) / np.linalg.norm(want, axis=-1)
+    assert err.max() < 1.05e-7, err
