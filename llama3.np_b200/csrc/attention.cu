@@ -10,8 +10,9 @@
 //    merged through shared memory; with nsplit > 1 CTAs emit (m, l, o) partials that
 //    attn_combine_kernel merges (flash-decoding).
 //  * attn_prefill_kernel (L > 1): shared-memory tiled flash attention in fp32 FFMA,
-//    16 queries x 64 keys per tile, online softmax.  (The bf16 tensor-core prefill is
-//    attention_tc.cu.)
+//    16 queries x 64 keys per tile, online softmax: short prompts.  Longer ones over fp32 caches
+//    run attn_f32.cu (launch_attn_prefill has the line), over bf16 caches attention_tc.cu on the
+//    tensor cores or, where that does not take them, attn_prefill64_kernel.
 #include <stdlib.h>
 
 #include <algorithm>
@@ -769,7 +770,7 @@ __global__ void __launch_bounds__(256) attn_prefill64_kernel(AttnArgs a, int nre
 template <int HD, typename KVT>
 static cudaError_t launch_prefill_hd(const AttnArgs& a, cudaStream_t s) {
   static const int big_min = [] { const char* v = getenv("L3_ATTN_PF64_MIN"); return v ? atoi(v) : 48; }();
-  if constexpr (sizeof(KVT) == 2) if (big_min > 0 && a.L >= big_min) {  // long prompts: the 64 x 64 tiling
+  if constexpr (sizeof(KVT) == 2) if (big_min > 0 && a.L >= big_min) {  // long prompts: the 64 x 64 tiling (fp32: attn_f32.cu)
     auto kern = attn_prefill64_kernel<HD, KVT>;
     const size_t smem = (size_t)(PF2_ROWS * HD + PF2_TK * (HD + 4) + PF2_TK * HD + PF2_ROWS * PF2_LDS) * sizeof(float);
     if (smem > 48 * 1024) {
@@ -803,10 +804,15 @@ static cudaError_t launch_prefill_t(const AttnArgs& a, cudaStream_t s) {
 }
 
 cudaError_t launch_attn_prefill(const AttnArgs& a, bool kv_bf16, cudaStream_t s) {
-  // fp32 caches: the 32-row tiles of attn_f32.cu from two tiles a head or four waves of CTAs on.  Six heads of 48, whole prompts, us with the
-  // 16- and 64-row tiles here : there: one sequence, 16 tokens 328 : 351, 32 370 : 396, 48 551 : 536, 64 556 : 541, 100 760 : 714; eight, 32
-  // 528 : 539, 48 556 : 542, 64 587 : 568; 256, 5 tokens 2594 : 2446, 32 3494 : 3327, 64 5115 : 4907.
-  if (!kv_bf16 && (a.L > 32 || (long)a.B * a.KVHN >= 4 * 148)) {
+  // fp32 caches: the 32-row tiles of attn_f32.cu from 48 tokens on, and of shorter prompts where the 16-row tiles are several waves of CTAs that
+  // the wider ones halve or whose heads are wide.  Head sizes 32 - 128, 4 - 32 heads in groups of 1 - 8, two layers, time here over the
+  // 16-row kernel's (from 48 on the 64-row kernel's that was here before): one sequence, 9 - 32 tokens 1.00 - 1.18, 33 - 47 1.01 - 1.11, 48
+  // 0.94 - 1.02, 64 0.94 - 1.02, 100 0.84 - 0.95; 16 sequences of 17 or 33, heads from 96 on 0.93 - 0.99 (four heads of 128 and 33 tokens 1.03),
+  // of 32 1.07; 64 of 17 0.86 - 0.99; 64 of 3 or 9, groups of four 0.83 - 0.96, no groups and heads of 48 - 64 1.01 - 1.08, from 96 on 0.95 -
+  // 0.99; 250 of 5, heads of 32 1.17, of 48 1.10, groups of three of them 0.85.
+  const int rep = a.HN / a.KVHN;
+  const long narrow = (long)a.B * a.HN * ((a.L + PF_ROWS - 1) / PF_ROWS), wide = (long)a.B * a.KVHN * (((long)a.L * rep + 31) / 32);
+  if (!kv_bf16 && (a.L >= 48 || (a.L > 1 && a.HD >= 48 && narrow >= 384 && (a.HD >= 96 || 2 * narrow >= 3 * wide)))) {
     WinAttnArgs w{};
     w.q = a.q; w.cache_k = a.cache_k; w.cache_v = a.cache_v; w.out = a.out; w.out_lo = a.out_lo; w.out16 = a.out_bf16; w.ld_out = a.HN * a.HD;
     w.out_scale = 1.f; w.gate = a.head_gate; w.ld_gate = a.ld_gate; w.pos_ptr = a.pos_ptr; w.kind = L3_ATTN_SOFTMAX;

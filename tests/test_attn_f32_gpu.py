@@ -37,6 +37,14 @@ def test_softmax(B, L, H, G, HD, start):
     assert orc.scaled_max_err(got, want) < 3e-6   # the bar of the other fp32 attention kernels
 
 
+# short prompts of many sequences, which run the same kernel by the count of their tiles; beside them the ones that keep the 16-row tiles
+@pytest.mark.parametrize("B,L,H,G,HD,start", [
+    (64, 33, 6, 6, 48, 0), (250, 7, 6, 2, 48, 60), (129, 17, 8, 8, 64, 3), (48, 2, 16, 4, 128, 40), (64, 15, 8, 8, 96, 0),
+    (1, 47, 16, 16, 128, 0), (250, 5, 4, 4, 48, 9), (64, 33, 8, 8, 32, 0)])
+def test_softmax_of_many_short_prompts(B, L, H, G, HD, start):
+    test_softmax(B, L, H, G, HD, start)
+
+
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
 def test_a_later_token_does_not_reach_rows_ahead_of_its_eight(bad):
     q, k, v = _inputs(1, 100, 2, 2, 64, 0, 5)
