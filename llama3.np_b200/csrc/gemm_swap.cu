@@ -95,11 +95,15 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
-__device__ __forceinline__ float ld_cluster(const float* p, int rank) {  // the same place in another CTA of the cluster
+__device__ __forceinline__ uint32_t at_rank(const float* p, int rank) {  // the same place in another CTA of the cluster
   uint32_t a;
-  float v;
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return a;
+}
+// 0 where not `on`: a predicate and no branch, so that a row of such loads is in flight together
+__device__ __forceinline__ float ld_cluster_if(bool on, uint32_t a) {
+  float v;
+  asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %2, 0;\nmov.f32 %0, 0f00000000;\n@p ld.shared::cluster.f32 %0, [%1];\n}" : "=f"(v) : "r"(a), "r"((int)on) : "memory");
   return v;
 }
 __device__ __forceinline__ void cluster_sync_all() {
@@ -135,11 +139,15 @@ template <int KIND, int BNA> struct SwCfg {
   static constexpr uint32_t IDESC = (1u << 4) | (FMT << 7) | (FMT << 10) | ((uint32_t)(BNA >> 3) << 17) | ((128u >> 4) << 24);
 };
 
-template <int KIND, int BNA, int EPI>
+// CL: the slices of a tile are a cluster, one item per CTA.  EPI_GATED: EPI_SWIGLU with any activation, with routing weights or without; the
+// plain silu is EPI_SWIGLU.  Both are kernels of their own: as arguments their row bounds, branches and loops cost every other launch 0.1 -
+// 0.5 us (9 rows, 2048 x 2048 added in place 3.89 : 4.16, 16384 x 2048 gated 13.3 : 13.8).
+constexpr int EPI_GATED = 8;
+template <int KIND, int BNA, int EPI, bool CL>
 __global__ void __launch_bounds__(SW_THREADS, 1)
 gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant__ CUtensorMap tmW1,
                  const __grid_constant__ CUtensorMap tmX0, const __grid_constant__ CUtensorMap tmX1,
-                 int rows, int N, int K, int h, int nst, int ksplit, int cl, float* part, int* tile_cnt, EpiArgs e) {
+                 int rows, int N, int K, int h, int nst, int ksplit, float* part, int* tile_cnt, EpiArgs e) {
   using Cf = SwCfg<KIND, BNA>;
   using KVT = typename std::conditional<KIND == TC_BF16, bf16, float>::type;
   constexpr int PARTS = Cf::PARTS, NBUF = Cf::NBUF, CJ = Cf::CJ;
@@ -157,9 +165,8 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
   const int ntiles = tiles_w * ksplit;
   const int nkb = (K + Cf::BK - 1) / Cf::BK;
   const int kb_per = (nkb + ksplit - 1) / ksplit;
-  // cl: the slices of a tile are a cluster, one item per CTA
-  auto tile_of = [&](int t) { return cl ? t / ksplit : t % tiles_w; };
-  auto slice_of = [&](int t) { return cl ? t % ksplit : t / tiles_w; };
+  auto tile_of = [&](int t) { return CL ? t / ksplit : t % tiles_w; };
+  auto slice_of = [&](int t) { return CL ? t % ksplit : t / tiles_w; };
   pdl_launch();
 
   if (warp == 0 && lane == 0) {
@@ -294,10 +301,10 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
       };
       const int Np = tiles_w * Cf::BMW;  // padded width of the K-split scratch [ksplit][BNA][Np]
       const int tw = tile_of(t), np = tw * Cf::BMW + quarter * 32 + lane;
-      const bool det = ksplit > 1 && (cl || part != nullptr);  // else (residual epilogue only): fp32 atomics
+      const bool det = CL || (ksplit > 1 && part != nullptr);  // else (residual epilogue only): fp32 atomics
       int m_lo = 0, m_hi = rows;  // rows that this CTA finishes
-      float* mine = reinterpret_cast<float*>(smem_raw + (tiles - raw)) + quarter * 32 + lane;  // cl: [row][128 columns]
-      if (cl) {
+      float* mine = reinterpret_cast<float*>(smem_raw + (tiles - raw)) + quarter * 32 + lane;  // CL: [row][128 columns]
+      if constexpr (CL) {
         // The slices' sums stay in shared memory - the ring, which nothing reads any more - and every CTA of the cluster adds up and
         // finishes its share of the rows, slices in order: the sums of the published form below without its trip through L2 and
         // without a last arriver that works alone.  40 greedy tokens of 32 sequences at the 8B shape 11120 -> 10960 us.
@@ -346,18 +353,17 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
         if (!is_last) continue;
       }
 #pragma unroll 1
-      for (int c0 = 0; c0 < BNA; c0 += 32) {
+      for (int c0 = m_lo; c0 < BNA; c0 += CJ) {
         if (c0 >= m_hi || !live) break;  // warp-uniform
-        if (c0 + 32 <= m_lo) continue;
-        auto mine_too = [&](int m) { return m >= m_lo && m < m_hi; };
         float v[32];
-        if (cl) {
+        if (CL) {
 #pragma unroll
           for (int j = 0; j < CJ; ++j) v[j] = 0.f;
           for (int k2 = 0; k2 < ksplit; ++k2) {
+            const uint32_t src = at_rank(mine + c0 * Cf::BMW, k2);
             float w[32];
 #pragma unroll
-            for (int j = 0; j < CJ; ++j) w[j] = mine_too(c0 + j) ? ld_cluster(mine + (c0 + j) * Cf::BMW, k2) : 0.f;
+            for (int j = 0; j < CJ; ++j) w[j] = ld_cluster_if(c0 + j < m_hi, src + j * Cf::BMW * 4);
 #pragma unroll
             for (int j = 0; j < CJ; ++j) v[j] += w[j];
           }
@@ -390,7 +396,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
 #pragma unroll
           for (int j = 0; j < CJ; ++j) {
             const int m = c0 + j;
-            if (mine_too(m) && n_ok) {
+            if (m < m_hi && n_ok) {
               const size_t o = (size_t)m * e.ld_out + n;
               if (e.out_lo) { float hi, lo; split_tf32(v[j], hi, lo); e.out[o] = hi; e.out_lo[o] = lo; }
               else if (e.out) e.out[o] = v[j];
@@ -407,13 +413,13 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
             for (int j = 0; j < CJ; ++j) rr[j] = e.resid[(size_t)min(c0 + j, rows - 1) * e.ld_out + nc];
 #pragma unroll
             for (int j = 0; j < CJ; ++j)
-              if (mine_too(c0 + j) && n_ok) e.out[(size_t)(c0 + j) * e.ld_out + n] = rr[j] + v[j];
+              if (c0 + j < m_hi && n_ok) e.out[(size_t)(c0 + j) * e.ld_out + n] = rr[j] + v[j];
           } else {  // bf16 mode: the slices add their partials into the residual stream in place (out == resid)
 #pragma unroll
             for (int j = 0; j < CJ; ++j)
               if (c0 + j < rows && n_ok) atomicAdd(e.out + (size_t)(c0 + j) * e.ld_out + n, v[j]);
           }
-        } else if constexpr (EPI == EPI_SWIGLU) {
+        } else if constexpr (EPI == EPI_SWIGLU || EPI == EPI_GATED) {
           // weight rows interleave gate_j, up_j: an even lane holds the gate, its odd neighbour the up value.  The even lane takes the
           // chunk's first half of the rows, the odd one the second; all values before the first store, the activation decided once.
           // silu with expf and a full reciprocal, in both modes: the fast forms take 0.7 us less at 32 x 28672 x 4096 and 3.5 us at 100 rows
@@ -428,7 +434,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
             gt[j] = odd ? got : v[j];
             hv[j] = odd ? v[j + HF] : got;
           }
-          if (e.act == GLU_SILU && !e.glu_w) {
+          if (EPI == EPI_SWIGLU || (e.act == GLU_SILU && !e.glu_w)) {
 #pragma unroll
             for (int j = 0; j < HF; ++j) hv[j] = silu_ref(gt[j]) * hv[j];
           } else if (e.act == GLU_GELU_TANH && !e.glu_w) {
@@ -449,7 +455,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
             const size_t o = (size_t)mb * e.ld_out + (n >> 1);
 #pragma unroll
             for (int j = 0; j < HF; ++j)
-              if (mine_too(mb + j)) {
+              if (mb + j < m_hi) {
                 const size_t oj = o + (size_t)j * e.ld_out;
                 if (e.out_lo) split_tf32(hv[j], e.out[oj], e.out_lo[oj]);
                 else if (e.out) e.out[oj] = hv[j];
@@ -478,7 +484,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
           for (int j = 0; j < CJ; ++j) {
             const float other = __shfl_xor_sync(L3_FULL, v[j], 1);  // the pair's partner (llama3.py:41-76)
             const int m = c0 + j, row = __shfl_sync(L3_FULL, lrow, j);
-            if (!mine_too(m) || !n_ok) continue;
+            if (m >= m_hi || !n_ok) continue;
             float r = v[j];
             // even: x0 c - x1 s, odd: x0 s + x1 c
             if (is_q || is_k) r = (lane & 1) ? other * sn[j] + v[j] * cs[j] : v[j] * cs[j] - other * sn[j];
@@ -497,7 +503,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
 #pragma unroll
           for (int j = 0; j < CJ; ++j) {
             const int m = c0 + j;
-            if (!mine_too(m)) continue;  // warp-uniform
+            if (m >= m_hi) continue;  // warp-uniform
             uint32_t kv = 0u;  // ordered bits of the value; 0 = no candidate
             if (n_ok) {
               const uint32_t b = __float_as_uint(v[j]);
@@ -517,7 +523,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
       }
     }
   }
-  if (cl) {
+  if constexpr (CL) {
     if (warp < 2 || warp == 6) cluster_sync_all();  // the others have met where the slices' sums were complete
     cluster_sync_all();                             // nobody leaves while its sums are read
   }
@@ -536,10 +542,10 @@ int sm_count() {
   return n[dev & 15] > 0 ? n[dev & 15] : 148;
 }
 
-template <int KIND, int BNA, int EPI>
-cudaError_t launch_sw_t(const TcGemmArgs& a, bool cluster, cudaStream_t s) {
+template <int KIND, int BNA, int EPI, bool CL>
+cudaError_t launch_sw_t(const TcGemmArgs& a, cudaStream_t s) {
   using Cf = SwCfg<KIND, BNA>;
-  auto kern = gemm_swap_kernel<KIND, BNA, EPI>;
+  auto kern = gemm_swap_kernel<KIND, BNA, EPI, CL>;
   static bool attr_done[16] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -559,21 +565,25 @@ cudaError_t launch_sw_t(const TcGemmArgs& a, bool cluster, cudaStream_t s) {
   // no more stages than a CTA has k-blocks
   const int nkb = (a.K + Cf::BK - 1) / Cf::BK, items = ((a.N + h - 1) / h * a.ksplit + (int)grid.x - 1) / (int)grid.x;
   const int nst = std::max(2, std::min(Cf::stages(h), (nkb + a.ksplit - 1) / a.ksplit * items));
-  const int cl = cluster ? 1 : 0;
-  if (cl && a.rows * Cf::BMW * 4 > nst * Cf::stage_bytes(h)) return cudaErrorInvalidValue;  // the sums lie in the ring: four blocks and more
-  if (cl) grid.x = (a.N + h - 1) / h * a.ksplit;
-  return launch_kc(kern, grid, dim3(SW_THREADS), (size_t)(nst * Cf::stage_bytes(h) + Cf::REST + 1024 + Cf::BARS), s, cl ? a.ksplit : 1, *W0, *W1, *X0, *X1, a.rows, a.N, a.K, h, nst, a.ksplit, cl, a.part, a.tile_cnt, a.e);
+  if (CL && a.rows * Cf::BMW * 4 > nst * Cf::stage_bytes(h)) return cudaErrorInvalidValue;  // the sums lie in the ring: four blocks and more
+  if (CL) grid.x = (a.N + h - 1) / h * a.ksplit;
+  return launch_kc(kern, grid, dim3(SW_THREADS), (size_t)(nst * Cf::stage_bytes(h) + Cf::REST + 1024 + Cf::BARS), s, CL ? a.ksplit : 1, *W0, *W1, *X0, *X1, a.rows, a.N, a.K, h, nst, a.ksplit, a.part, a.tile_cnt, a.e);
 }
 
-template <int KIND, int BNA>
-cudaError_t launch_sw_e(const TcGemmArgs& a, bool cl, cudaStream_t s) {
+template <int KIND, int BNA, bool CL>
+cudaError_t launch_sw_e(const TcGemmArgs& a, cudaStream_t s) {
   switch (a.epi) {
-    case EPI_STORE: return launch_sw_t<KIND, BNA, EPI_STORE>(a, cl, s);
-    case EPI_RESID: return launch_sw_t<KIND, BNA, EPI_RESID>(a, cl, s);
-    case EPI_SWIGLU: return launch_sw_t<KIND, BNA, EPI_SWIGLU>(a, cl, s);
-    case EPI_ARGMAX: return launch_sw_t<KIND, BNA, EPI_ARGMAX>(a, cl, s);
-    default: return launch_sw_t<KIND, BNA, EPI_ROPE_KV>(a, cl, s);
+    case EPI_STORE: return launch_sw_t<KIND, BNA, EPI_STORE, CL>(a, s);
+    case EPI_RESID: return launch_sw_t<KIND, BNA, EPI_RESID, CL>(a, s);
+    case EPI_SWIGLU:
+      return a.e.act == GLU_SILU && !a.e.glu_w ? launch_sw_t<KIND, BNA, EPI_SWIGLU, CL>(a, s) : launch_sw_t<KIND, BNA, EPI_GATED, CL>(a, s);
+    case EPI_ARGMAX: return launch_sw_t<KIND, BNA, EPI_ARGMAX, CL>(a, s);
+    default: return launch_sw_t<KIND, BNA, EPI_ROPE_KV, CL>(a, s);
   }
+}
+template <int KIND, int BNA>
+cudaError_t launch_sw_c(const TcGemmArgs& a, bool cluster, cudaStream_t s) {
+  return cluster ? launch_sw_e<KIND, BNA, true>(a, s) : launch_sw_e<KIND, BNA, false>(a, s);
 }
 }  // namespace
 
@@ -602,7 +612,7 @@ static int clusters_of(int n) {
   std::lock_guard<std::mutex> g(mu);
   int& v = most[dev & 15][n];
   if (v) return v;
-  auto kern = gemm_swap_kernel<TC_BF16, 32, EPI_STORE>;
+  auto kern = gemm_swap_kernel<TC_BF16, 32, EPI_STORE, true>;
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute at[1];
   cfg.gridDim = dim3(n); cfg.blockDim = dim3(SW_THREADS); cfg.dynamicSmemBytes = SwCfg<TC_BF16, 32>::SMEM_MAX;
@@ -662,16 +672,16 @@ cudaError_t launch_gemm_swap(const TcGemmArgs& args, cudaStream_t s) {
   // no hot spot), low tiles in place of a K split (42 rows x 147 CTAs for QKV: 17 vs 14 us, the issue loops' cycles per block remain).
   if (a.kind == TC_BF16) {
     switch (bna) {
-      case 16: return launch_sw_e<TC_BF16, 16>(a, p.cluster, s);
-      case 32: return launch_sw_e<TC_BF16, 32>(a, p.cluster, s);
-      case 64: return launch_sw_e<TC_BF16, 64>(a, p.cluster, s);
-      default: return launch_sw_e<TC_BF16, 128>(a, p.cluster, s);
+      case 16: return launch_sw_c<TC_BF16, 16>(a, p.cluster, s);
+      case 32: return launch_sw_c<TC_BF16, 32>(a, p.cluster, s);
+      case 64: return launch_sw_c<TC_BF16, 64>(a, p.cluster, s);
+      default: return launch_sw_c<TC_BF16, 128>(a, p.cluster, s);
     }
   }
   switch (bna) {
-    case 16: return launch_sw_e<TC_TF32X3, 16>(a, p.cluster, s);
-    case 32: return launch_sw_e<TC_TF32X3, 32>(a, p.cluster, s);
-    case 64: return launch_sw_e<TC_TF32X3, 64>(a, p.cluster, s);
-    default: return launch_sw_e<TC_TF32X3, 128>(a, p.cluster, s);
+    case 16: return launch_sw_c<TC_TF32X3, 16>(a, p.cluster, s);
+    case 32: return launch_sw_c<TC_TF32X3, 32>(a, p.cluster, s);
+    case 64: return launch_sw_c<TC_TF32X3, 64>(a, p.cluster, s);
+    default: return launch_sw_c<TC_TF32X3, 128>(a, p.cluster, s);
   }
 }
