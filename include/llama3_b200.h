@@ -343,7 +343,8 @@ int l3_read_cache(L3Model* m, int layer, float* k_out, float* v_out);
 int l3_op_rmsnorm(int device, const float* x, const float* w, float eps, int rows, int dim, float* out);
 /* y = x @ W.T with W [n, k] (the `x @ self.*_weight` lines, llama3.py:99-102,166-168,211,307).
  * path: 0 auto, 1 row-streaming GEMV, 2 SIMT tiled GEMM, 3 tcgen05 (bf16 or 3xTF32 operands),
- * 4 tcgen05 with swapped operand roles (rows <= 128, n >= 128), 5 tcgen05 at fp32 precision (fp32 x; W fp32 or bf16).
+ * 4 tcgen05 with swapped operand roles (rows <= 128, n >= 128), 5 tcgen05 at fp32 precision (fp32 x; W fp32 or bf16), 6 the same with both
+ * operands cut into bf16 parts beforehand (fp32 W, k a multiple of 8), 7 as 4 with K slices that meet in device memory in place of a cluster.
  * w_bf16 != 0 rounds W (and for path 3 x) to bf16 first. */
 int l3_op_linear(int device, const float* x, const float* w, int rows, int n, int k,
                  int path, int w_bf16, float* out);
@@ -375,7 +376,8 @@ int l3_op_argmax(int device, const float* logits, int rows, int n, int64_t* out)
 
 /* How the model path cuts a tensor-core projection of `rows` rows in bf16 mode, or with fp32 != 0 one of up to 128 rows of the Llama
  * path's fp32 mode (epi 0: plain store, 1: added to the residual in place, 2: gated):
- * plan[0] 1 = weights as the 128-row operand (gemm_swap.cu), 0 = activations (gemm_tc.cu); [1] CTAs that share a tile; [2] the tile's
+ * plan[0] 1 = weights as the 128-row operand (gemm_swap.cu), 0 = activations (gemm_tc.cu); [1] CTAs that share a tile as a pair or, where
+ * the slices of K are a thread-block cluster, as those; [2] the tile's
  * width (gemm_swap.cu: height); [3] slices of K; [4] 1 = the slices are added in whatever order they arrive, so that the last bits
  * differ from run to run.  Without a GPU: for 148 SMs. */
 int l3_debug_gemm_plan(int rows, int n, int k, int epi, int fp32, int32_t* plan);

@@ -18,7 +18,6 @@
 
 #include <stdlib.h>
 #include <algorithm>
-#include <mutex>
 
 #include "common.cuh"
 #include "gemm_tc.h"
@@ -596,34 +595,19 @@ static bool adds_in_place(const TcGemmArgs& a, int sms) {
   static const int resid_atomic = [] { const char* v = getenv("L3_SWAP_RESID_ATOMIC"); return v ? atoi(v) : 1; }();
   return a.epi == EPI_RESID && a.kind == TC_BF16 && a.e.out == a.e.resid && resid_atomic && (a.K + 63) / 64 >= 16 && (a.N + 127) / 128 * 2 <= sms;
 }
+// Clusters of n CTAs with all of an SM's shared memory each that the device holds at once, whatever its GPCs' populations: eight of them with even
+// numbers of SMs, of which each leaves up to n - 1 (n - 2 for even n) without a cluster.  148 SMs, n = 2 .. 8: 74, 44, 33, 24, 20, 15, 13
+// (cudaOccupancyMaxActiveClusters there: 74, 45, 33, 26, 22, 15, 15).  By the SM count alone, so that one product is cut, and its sums come,
+// alike on every device of that count.
+static int clusters_of(int n, int sms) { return std::max(0, (sms - 8 * (n - 1 & ~1) + n - 1) / n); }
 // Tile height and K split, by the cycles of the busiest CTA: a k-block takes the issue loops ~500 cycles (fp32 mode, two parts and three
-// products: 750 - 980 with the columns; with 700 for all of them 74 x 288 x 768 took 26.7 us whole instead of 24.7 in slices, 74 x 8192 x
-// 1536 43.9 instead of 39.4), or its share of DRAM (3560 bytes per cycle for all CTAs that stream); slices that are added in place cost little, a cluster's ~1 us (taken where all
-// tiles' clusters are resident at once; 1000 - 3000 cycles choose alike), published and summed ones ~2.5 us and more with each slice and row: 9 x 2048 x 4096 added in place, 1, 2, 4, 8 slices 18.0, 12.4, 10.1, 8.6 us, 9 x 2048 x 8192 28.8, 18.2, 12.4,
-// 11.5.  More tiles than SMs: the height that makes the last round full (28672 rows: 293 tiles of 98 instead of 224 of 128 - 100 rows
-// 57.5 -> 56.2 us, 32 rows 46.0 : 46.1, 9 rows 43.6 : 44.5).  Over 22 shapes (profiles/gemm_cuts.jsonl) it is 0.8 % behind the best in the
-// mean, at most 7 %.
-// clusters of n CTAs with all of an SM's shared memory each that the device holds at once (GPCs have 16 - 20 SMs)
-static int clusters_of(int n) {
-  static std::mutex mu;
-  static int most[16][9] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> g(mu);
-  int& v = most[dev & 15][n];
-  if (v) return v;
-  auto kern = gemm_swap_kernel<TC_BF16, 32, EPI_STORE, true>;
-  cudaLaunchConfig_t cfg{};
-  cudaLaunchAttribute at[1];
-  cfg.gridDim = dim3(n); cfg.blockDim = dim3(SW_THREADS); cfg.dynamicSmemBytes = SwCfg<TC_BF16, 32>::SMEM_MAX;
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = n; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at; cfg.numAttrs = 1;
-  v = 1;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&v, kern, &cfg) != cudaSuccess || v < 1) { cudaGetLastError(); v = 1; }
-  return v;
-}
+// products: 750 - 980 with the columns), or its share of DRAM (3560 bytes per cycle for all CTAs that stream).  Slices that are added in place
+// cost little (9 x 2048 x 4096, 1, 2, 4, 8 slices 18.0, 12.4, 10.1, 8.6 us); a cluster's, taken where all tiles' clusters are resident at once,
+// 3000 cycles whatever their number (with 1800, as one would count from the kernel alone, short products are cut that run faster whole under
+// their neighbours' tails: 28 x 7680 x 760 6.7 : 7.8 us); published and summed ones 2800 and more with each slice and row (9 x 6144 x 4096 two
+// slices as clusters 13.0 us, three published 11.6).  More tiles than SMs: the height that makes the last round full (28672 rows: 293 tiles of
+// 98 instead of 224 of 128 - 100 rows 57.5 -> 56.2 us).  Over 547 shapes in both modes (profiles/gemm_swap_cuts.jsonl) the choice is 1 % behind
+// the best of all cuts in the mean and takes 0.83 of the time of the plan and kernel without clusters.
 static void pick_swap(const TcGemmArgs& a, int bna, int sms, int* h_out, int* ks_out, bool* cl_out) {
   static const int max_split = [] { const char* v = getenv("L3_SWAP_KSPLIT"); return v ? atoi(v) : 8; }();
   static const int det_epi = [] { const char* v = getenv("L3_SWAP_KSPLIT_DET"); return v ? atoi(v) : 1; }();
@@ -638,14 +622,14 @@ static void pick_swap(const TcGemmArgs& a, int bna, int sms, int* h_out, int* ks
   for (int ks = 1; ks <= std::max(1, atomic ? 8 : std::min(8, max_split)); ++ks) {
     const int per = (nkb + ks - 1) / ks;
     if (ks > 1 && (per < 4 || (ks - 1) * per >= nkb)) break;
-    const bool cl = ks > 1 && !atomic && det_epi && clusters_of(ks) >= tiles;
+    const bool cl = ks > 1 && !atomic && det_epi && clusters_of(ks, sms) >= tiles;
     if (ks > 1 && !atomic && !cl && (!a.part || !a.tile_cnt || tiles > a.tile_cnt_len || (size_t)bna * tiles * 128 * sizeof(float) * ks > a.part_bytes ||
                               !(det_epi || a.epi == EPI_RESID))) break;
-    const double issue = b16 ? 500 : 720 + 2.0 * bna, slice = 160 + 22.0 * bna + (b16 ? 0 : 8.0 * a.rows);
+    const double issue = b16 ? 500 : 720 + 2.0 * bna, slice = 22.0 * bna + (b16 ? 0 : 8.0 * a.rows);
     const int full = tiles * ks / sms, rest = tiles * ks % sms;
     double c = full * per * std::max(issue, h * 128.0 * parts * sms / 3560);
     if (rest) c += per * std::max(issue, h * 128.0 * parts * rest / 3560);
-    if (ks > 1) c += atomic ? 380 + 2.0 * ks * bna : cl ? 1800 : 4400 + slice * ks;
+    if (ks > 1) c += atomic ? 380 + 2.0 * ks * bna : cl ? 3000 : 2800 + slice * ks;
     if (best == 0 || c < best) { best = c; *ks_out = ks; *cl_out = cl; }
   }
   *h_out = h;
@@ -663,7 +647,11 @@ TcPlan gemm_swap_plan(const TcGemmArgs& a) {
 cudaError_t launch_gemm_swap(const TcGemmArgs& args, cudaStream_t s) {
   TcGemmArgs a = args;
   const int bna = batch_cols(a.rows);
-  const TcPlan p = gemm_swap_plan(a);
+  TcPlan p = gemm_swap_plan(a);
+  if (a.no_cluster) {
+    if (!a.part || !a.tile_cnt) return cudaErrorInvalidValue;
+    p.cluster = false;
+  }
   a.bn = p.width; a.ksplit = p.slices;
   if (p.any_order) a.part = nullptr;
   // Measured and rejected at the 8B shape, batch 32 (profiles/swap_gemm_experiments.txt): a tile-contiguous copy of the weights read

@@ -28,12 +28,13 @@ struct TcGemmArgs {
   int* tile_cnt;     // zero-initialised arrival counters, one per output tile
   int tile_cnt_len;
   int* err;             // gemm_tc.cu: set to 1 when a wait inside the kernel ran out (null: the launch fails)
+  bool no_cluster;      // gemm_swap.cu: slices that would be a cluster are published in the scratch instead, for comparisons
 };
 
 cudaError_t launch_gemm_tc(const TcGemmArgs& a, cudaStream_t s);
 // how a launch cuts its work: CTAs that share a tile, the tile's width (gemm_swap.cu: height), slices of K, and whether slices are added
 // in whatever order they arrive
-struct TcPlan { int ctas, width, slices, any_order; bool cluster = false; };  // cluster: the slices of a tile are one
+struct TcPlan { int ctas, width, slices, any_order; bool cluster = false; };  // cluster: the slices of a tile are one (gemm_swap.cu)
 TcPlan gemm_tc_plan(const TcGemmArgs& a);    // bf16
 TcPlan gemm_swap_plan(const TcGemmArgs& a);
 // swapped operand roles for 9..128 activation rows (gemm_swap.cu): same arguments

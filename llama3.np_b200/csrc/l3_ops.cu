@@ -84,7 +84,7 @@ extern "C" int l3_op_linear(int device, const float* x, const float* w, int rows
     e = launch_linear_rows(a, w_bf16 != 0, false, sc.s);
   } else if (path == 2) {
     e = launch_linear_simt(a, w_bf16 != 0, false, sc.s);
-  } else if (path == 3 || path == 4) {  // tcgen05: bf16 operands, or the 3xTF32 split of fp32 operands (4: swapped roles)
+  } else if (path == 3 || path == 4 || path == 7) {  // tcgen05: bf16 operands, or the 3xTF32 split of fp32 operands (4, 7: swapped roles)
     if (!tc_gemm_supported(k)) return L3_EINVAL;
     TcGemmArgs t{};
     t.rows = rows; t.N = n; t.K = k; t.epi = EPI_STORE; t.e = a.e;
@@ -101,14 +101,15 @@ extern "C" int l3_op_linear(int device, const float* x, const float* w, int rows
       if (launch_split_tf32(dw32, wh, wl, (int64_t)n * k, sc.s) != cudaSuccess) return L3_ECUDA;
       t.kind = TC_TF32X3; t.A[0] = xh; t.A[1] = xl; t.W[0] = wh; t.W[1] = wl;
     }
-    if (path == 4 && !gemm_swap_supported(rows, n)) return L3_EINVAL;
+    if (path != 3 && !gemm_swap_supported(rows, n)) return L3_EINVAL;
+    t.no_cluster = path == 7;
     // K-split scratch, as the model path owns it (l3_api.cu linear()): short-and-wide shapes split along K
     const size_t part_bytes = (size_t)32 << 20;
     t.part = sc.dev<float>(part_bytes / 4); t.part_bytes = part_bytes;
     t.tile_cnt = sc.dev<int>(1024); t.tile_cnt_len = 1024;
     if (!t.part || !t.tile_cnt) return L3_ENOMEM;
     if (cudaMemsetAsync(t.tile_cnt, 0, 1024 * sizeof(int), sc.s) != cudaSuccess) return L3_ECUDA;
-    e = path == 4 ? launch_gemm_swap(t, sc.s) : launch_gemm_tc(t, sc.s);
+    e = path != 3 ? launch_gemm_swap(t, sc.s) : launch_gemm_tc(t, sc.s);
     int rc = finish(sc, e);
     tc_forget_maps();  // the scratch buffers are about to be freed
     if (rc == L3_OK) cudaMemcpy(out, dout, (size_t)rows * n * 4, cudaMemcpyDeviceToHost);
@@ -305,7 +306,7 @@ extern "C" int l3_debug_gemm_plan(int rows, int n, int k, int epi, int fp32, int
   if (epi == EPI_RESID) t.e.resid = &x;
   const bool swapped = gemm_swap_supported(rows, n);
   const TcPlan p = swapped ? gemm_swap_plan(t) : gemm_tc_plan(t);
-  plan[0] = swapped; plan[1] = p.ctas; plan[2] = p.width; plan[3] = p.slices; plan[4] = p.any_order;
+  plan[0] = swapped; plan[1] = p.cluster ? p.slices : p.ctas; plan[2] = p.width; plan[3] = p.slices; plan[4] = p.any_order;
   return L3_OK;
 }
 

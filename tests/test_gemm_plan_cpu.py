@@ -42,12 +42,24 @@ def test_more_than_128_rows_add_to_the_residual_in_slice_order():
             assert p["swapped"] == 0 and p["any_order"] == 0
 
 
-@pytest.mark.parametrize("rows,n,k,slices", [(74, 288, 768, 3), (100, 288, 768, 1), (128, 4096, 768, 1), (74, 1024, 768, 3), (12, 8192, 1536, 2), (48, 8192, 1536, 2),
-                                             (74, 8192, 1536, 2), (128, 8192, 1536, 2), (74, 8192, 768, 1), (128, 288, 288, 1), (9, 288, 288, 1)])
+# us whole, in the best number of published slices and as these clusters: 74 x 288 x 768 26.8, 24.7, 14.5; 100 x 288 x 768 28.8, 28.8, 14.6;
+# 128 x 4096 x 768 31.0, 32.9, 18.3; 12 x 8192 x 1536 25.0, 21.8, 20.8; 128 x 8192 x 1536 50.6, 46.8, 34.6; 9 x 288 x 288 7.3, 7.2, 6.7
+@pytest.mark.parametrize("rows,n,k,slices", [(74, 288, 768, 6), (100, 288, 768, 6), (128, 4096, 768, 4), (74, 1024, 768, 6), (12, 8192, 1536, 2), (48, 8192, 1536, 2),
+                                             (74, 8192, 1536, 2), (128, 8192, 1536, 2), (74, 8192, 768, 2), (128, 288, 288, 2), (9, 288, 288, 2)])
 def test_fp32_products_are_cut_where_that_was_measured_faster(rows, n, k, slices):
     p = plan(rows, n, k, STORE, 1)
-    assert p["slices"] == slices and p["any_order"] == 0
+    assert p["slices"] == slices and p["ctas"] == slices and p["any_order"] == 0
     assert plan(rows, n, k, RESID, 1)["any_order"] == 0   # fp32 sums always come in slice order
+
+
+@pytest.mark.parametrize("rows,n,k,epi,fp32,slices,ctas", [
+    (9, 6144, 4096, STORE, 0, 3, 1), (16, 6144, 4096, STORE, 0, 3, 1),   # 48 clusters of three are more than fit at once
+    (32, 6144, 4096, STORE, 0, 2, 2), (20, 3072, 2048, STORE, 0, 5, 5),
+    (28, 7680, 760, STORE, 0, 1, 1), (32, 28672, 4096, GATED, 0, 1, 1),
+    (32, 4096, 4096, RESID, 0, 4, 1)])                                   # added in place, in any order
+def test_slices_are_a_cluster_where_all_of_them_are_resident(rows, n, k, epi, fp32, slices, ctas):
+    p = plan(rows, n, k, epi, fp32)
+    assert (p["slices"], p["ctas"]) == (slices, ctas)
 
 
 def test_refused_arguments():
