@@ -695,9 +695,12 @@ static int enqueue_cluster_layers(L3Model* m, const int32_t* d_ids, int ids_ld, 
 // 16 sequences: 1B 9 sequences 1923 : 1759 a call, 16 1960 : 1805, 32 2222 : 2227, 8B 9 3393 : 3298, 16 3470 : 3444, 32 3806 : 3833, fp32
 // stories15M 9 5570 : 5403, 16 5597 : 5639, 30 6828 : 7182.  Layer lists: latent attention of width 2048 0.69 : 0.62 ms a step, 3.20 : 3.02
 // ms a prompt of 2048 tokens; prompts of 2048 tokens: linear mixers of width 2048 1042 : 982 us, parallel
-// layers 888 : 839, states and experts 1729 : 1688; eight sequences through chunk attention and matrix memories 6340 : 5612 us for 32 tokens.  NCCL's kernels between them take no part (tensor parallelism).
+// layers 888 : 839, states and experts 1729 : 1688; eight sequences through chunk attention and matrix memories 6340 : 5612 us for 32 tokens.  Not
+// parallel layers of 5 - 8 rows, whose row-streaming products lose more to waiting successors in their shared memory than the launches
+// take (12 tokens of six sequences, width 512 2001 : 1955, 1024 2763 : 2972, 1536 2826 : 2901, 2048 3326 : 3271; four sequences 2138 : 2072 at
+// 1024).  NCCL's kernels between them take no part (tensor parallelism).
 static bool pdl_pays(const L3Model* m, int ntok, int L) {
-  if (m->ll) return true;
+  if (m->ll) return !(m->ll->cfg.parallel && ntok > 4 && ntok <= 8);
   if (m->G > 1) return false;
   if (L == 1) return ntok > 8 && ntok <= 16;
   const size_t layer = ((size_t)(m->qkv_rows + m->HN * m->HD) * m->D + (size_t)3 * m->FD * m->D) * (m->bf16 ? 2 : 4);
