@@ -290,7 +290,6 @@ extern "C" int l3_create_stack(const L3StackConfig* c, const L3LayerSpec* specs,
   AL(m->embed, (size_t)c->vocab * W * w);
   if (c->tied_head) m->lm_head = m->embed;
   else AL(m->lm_head, (size_t)c->vocab * W * w);
-  ll->weights.push_back({m->lm_head, (size_t)c->vocab * W});
   AL(m->norm_final, (size_t)W * 4);
   if (c->norm_tanh) { AL(ll->final_b, (size_t)W * 4); AL(ll->final_alpha, 4); }
   if (sd) AL(ll->side_embed, (size_t)c->vocab * c->n_layers * sd * w);
@@ -1050,6 +1049,9 @@ static bool ll_moe_in_groups(const L3Model* m, const LLLayer& Ly, const void* x1
   return x16 && ll_moe_groups_pay(m, Ly, ntok) && ll_moe_groups_bytes(m, Ly, ntok) <= m->ll->moe_ws_bytes;
 }
 
+// Products of fp32 rows whose operands are worth cutting into bf16 parts beforehand (figures: ll_cut_operands)
+static bool ll_cut_pays(int64_t rows, int64_t matrix) { return rows > 128 && rows * matrix >= 400000000; }
+
 // The workspaces of prompt paths that have another path beside them, behind everything a model cannot do without.
 static int ll_workspaces(L3Model* m, bool units, bool ksplit) {
   LayerList* ll = m->ll;
@@ -1087,31 +1089,30 @@ static int ll_workspaces(L3Model* m, bool units, bool ksplit) {
       ll->chunk_ws = p;
       ll->chunk_ws_floats = chan;
     }
-  if (!m->bf16 && ll->f32_tc && ct > 8) {  // the matrices of fp32 projections, cut into bf16 parts once, and room for their inputs' parts
-    size_t n = 0, k = std::max<size_t>(m->D, std::max(ll->max_ctx, ll->max_ff));
-    for (auto& L : ll->layers) k = std::max<size_t>(k, std::max(L.spec.ff, std::max(L.ff_total, L.ctx_ld)));
-    for (auto& w : ll->weights) n += w.n % 8 ? 0 : w.n;
-    if (void* p = optional_ws(ct * k * 6)) {
-      ll->x_cut = (bf16*)p;
-      if ((p = optional_ws(n * 6))) {
-        ll->cut = (bf16*)p;
-        ll->x_cut_n = ct * k;
-        bf16* to = ll->cut;
-        for (auto& w : ll->weights) {
-          if (w.n % 8) continue;  // rows that are no whole 16-byte pieces
-          w.plane = (int64_t)w.n;
-          CK(m, launch_cut_rows((const float*)w.p, 8, (int)(w.n / 8), 8, to, w.plane, m->stream));
-          w.cut = to;
-          to += 3 * w.plane;
-        }
-      }
-    }
-  }
   const size_t per = (size_t)m->M * f_ld * 4;
   if (f_ld && ct >= LATENT_F32_MIN && per <= ((size_t)1 << 30)) {  // expanded latent rows in fp32 mode; longer contexts keep the folded form
     const int seqs = (int)std::max<size_t>(1, std::min<size_t>(m->maxB, ((size_t)1 << 28) / per));
     ll->lat_exp = optional_ws(seqs * per);
     ll->exp_seqs = ll->lat_exp ? seqs : 0;
+  }
+  if (!m->bf16 && ll->f32_tc) {  // behind all others, as the largest: matrices of fp32 projections cut into bf16 parts, and room for an input's parts
+    size_t n = 0, k = std::max<size_t>(m->D, std::max(ll->max_ctx, ll->max_ff));
+    for (auto& L : ll->layers) k = std::max<size_t>(k, std::max(L.spec.ff, std::max(L.ff_total, L.ctx_ld)));
+    auto cuts = [&](const LayerList::Weight& w) { return w.n % 8 == 0 && ll_cut_pays(m->cap_tok, (int64_t)w.n); };  // whole 16-byte pieces; a chunk can be long enough
+    for (auto& w : ll->weights) n += cuts(w) ? w.n : 0;
+    ll->cut = (bf16*)optional_ws(n * 6);
+    if (ll->cut && !(ll->x_cut = (bf16*)optional_ws(ct * k * 6))) { CK(m, cudaFree(ll->cut)); ll->cut = nullptr; }
+    if (ll->cut) {
+      ll->x_cut_n = ct * k;
+      bf16* to = ll->cut;
+      for (auto& w : ll->weights) {
+        if (!cuts(w)) continue;
+        w.plane = (int64_t)w.n;
+        CK(m, launch_cut_rows((const float*)w.p, 8, (int)(w.n / 8), 8, to, w.plane, m->stream));
+        w.cut = to;
+        to += 3 * w.plane;
+      }
+    }
   }
   return L3_OK;
 }
@@ -1528,13 +1529,14 @@ static bool ll_takes_mirror(const L3Model* m, int rows, int N, int K) {
   return m->tc_ok && !ll_gemv(m, rows, N, K) && K % 8 == 0 && K >= 64 && N >= 64;
 }
 
-// The parts of an fp32 product's operands, where its matrix was cut at load time: the input's are made here, a launch of ~3 us.  That pays
+// The parts of an fp32 product's operands, where its matrix was cut at load time (not the output projection, which few calls ask for more
+// than 128 rows of): the input's are made here, a launch of ~3 us.  That pays
 // from two row tiles and ~400 million products on (prompt through the public call, in the kernel : beforehand, us): gifudra width 1024, 400
 // tokens 525 : 489, 2 x 400 790 : 703, 2 x 64 463 : 476; debuzen width 1024, 130 tokens 826 : 762, 2 x 400 1719 : 1418; width 512, 400
 // tokens 938 : 914, mabedra 581 : 569, risalix 666 : 667, with all products cut 666 : 680.
 static int ll_cut_operands(L3Model* m, GemmF32Args& t) {
   LayerList* ll = m->ll;
-  if (!ll->x_cut || t.rows <= 128 || (int64_t)t.rows * t.N * t.K < 400000000 || t.K % 8 || (size_t)t.rows * t.K > ll->x_cut_n) return L3_OK;
+  if (!ll->x_cut || !ll_cut_pays(t.rows, (int64_t)t.N * t.K) || t.K % 8 || (size_t)t.rows * t.K > ll->x_cut_n) return L3_OK;
   for (const auto& w : ll->weights) {
     const int64_t off = (const float*)t.W - (const float*)w.p;
     if (!w.cut || off < 0 || off + (int64_t)t.N * t.K > (int64_t)w.n || off % 8) continue;
