@@ -414,6 +414,10 @@ int l3_debug_mega_timeline(L3Model* m, uint64_t* out, int64_t capacity);
  * which 1: float [n_layers][max_batch_size][dim], the residual stream after every layer. */
 int l3_debug_stack(L3Model* m, int which, void* out, int64_t capacity_bytes);
 
+/* Debug: 1 if the launches of a chunk of L tokens of each of B sequences are programmatic dependents of one another, else 0 (L3_PDL as it was
+ * set when the handle was made, L3_FLAG_NO_PDL, and otherwise a rule by rows and layer size). */
+int l3_debug_pdl(L3Model* m, int B, int L);
+
 /* Debug: sets the word that a kernel sets when one of its bounded waits runs out, so that the next call that waits for the
  * GPU reports it (for tests of the host side).  L3_EINVAL for a handle none of whose kernels reports its waits. */
 int l3_debug_fail_wait(L3Model* m);

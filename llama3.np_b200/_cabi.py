@@ -127,6 +127,7 @@ SIGNATURES = {
     "l3_debug_mega_timeline": (_I, [_P, C.POINTER(C.c_uint64), C.c_int64]),
     "l3_debug_stack": (_I, [_P, _I, _P, C.c_int64]),
     "l3_debug_fail_wait": (_I, [_P]),
+    "l3_debug_pdl": (_I, [_P, _I, _I]),
     "l3_debug_gemm_plan": (_I, [_I, _I, _I, _I, _I, _I32P]),
     "l3_bench_gemv": (_I, [_I, _I, _I, _I, _I, _I, _F32P]),
     "l3_probe_mma": (_I, [_I, _I, _I, _I, _I, _I, _F64P]),

@@ -25,10 +25,12 @@ const bool g_l3_debug_sync = getenv("L3_DEBUG_SYNC") && atoi(getenv("L3_DEBUG_SY
 thread_local bool g_l3_pdl_next = false;  // one-shot: the next launch is a programmatic dependent of its predecessor (linear())
 thread_local bool g_l3_pdl = false;       // programmatic dependent launches (PdlScope)
 // L3_PDL: 0 nowhere, 1 in every scope whatever it holds
-static const int g_l3_pdl_env = getenv("L3_PDL") ? (atoi(getenv("L3_PDL")) != 0 ? 1 : 0) : -1;
-PdlScope::PdlScope(const L3Model* m, bool pays) : before(g_l3_pdl) {
-  g_l3_pdl = !(m->cfg.flags & L3_FLAG_NO_PDL) && (g_l3_pdl_env < 0 ? pays : g_l3_pdl_env == 1);
+int l3_pdl_env() {
+  const char* v = getenv("L3_PDL");
+  return v ? atoi(v) != 0 : -1;
 }
+static bool pdl_on(const L3Model* m, bool pays) { return !(m->cfg.flags & L3_FLAG_NO_PDL) && (m->pdl_env < 0 ? pays : m->pdl_env == 1); }
+PdlScope::PdlScope(const L3Model* m, bool pays) : before(g_l3_pdl) { g_l3_pdl = pdl_on(m, pays); }
 PdlScope::~PdlScope() { g_l3_pdl = before; }
 
 #include <mutex>
@@ -705,6 +707,11 @@ static bool pdl_pays(const L3Model* m, int ntok, int L) {
   if (L == 1) return ntok > 8 && ntok <= 16;
   const size_t layer = ((size_t)(m->qkv_rows + m->HN * m->HD) * m->D + (size_t)3 * m->FD * m->D) * (m->bf16 ? 2 : 4);
   return ntok <= 8 || ntok > 32 || layer <= (size_t)126 << 20;
+}
+
+extern "C" int l3_debug_pdl(L3Model* m, int B, int L) {
+  if (!m || B < 1 || L < 1) return L3_EINVAL;
+  return pdl_on(m, pdl_pays(m, B * L, L));
 }
 
 // Enqueue one chunk: tokens ids[b * ids_ld + ids_off + t], t < L, at start_pos = *d_pos.

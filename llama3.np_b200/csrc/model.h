@@ -34,10 +34,12 @@ struct L3Graph {
 
 struct LayerList;  // layerlist.h: the layers, state and workspace of a layer-list decoder
 
+int l3_pdl_env();  // l3_api.cu
 struct L3Model {
   L3Config cfg{};
   LayerList* ll = nullptr;  // non-null: made by l3_create_stack; cfg holds the shared fields (dim = width, ...)
   bool bf16 = false;
+  const int pdl_env = l3_pdl_env();  // L3_PDL when the handle was made: 0, 1, or -1 unset
   // local (per tensor-parallel rank) dimensions
   int D = 0, HD = 0, G = 1, HN = 0, KVHN = 0, FD = 0, VS = 0, M = 0, maxB = 0, qkv_rows = 0;
   cudaStream_t stream = nullptr;
