@@ -627,8 +627,8 @@ static int linear(L3Model* m, LinearArgs& a, Feed feed, const float* w_hi, const
   // Decode-sized batches: every swapped-role GEMM is launched as a programmatic dependent of whatever precedes it
   // (RMSNorm, attention, the previous GEMM), so that its prologue - TMEM allocation, barriers, tensor-map prefetch, the
   // first weight stage - runs under the predecessor's tail.  Measured at the 8B shape, ms per decode step at 32 rows:
-  // off 4.34, behind RMSNorm only 4.27, every GEMM 4.17; every kernel of the step
-  // (L3_PDL=1) is no better at 32 rows, see pdl_pays.  L3_PDL_GEMM: 0 off, 1 behind RMSNorm, 2 all.
+  // off 4.34, behind RMSNorm only 4.27, every GEMM 4.17 (all kernels of a step:
+  // pdl_pays).  L3_PDL_GEMM: 0 off, 1 behind RMSNorm, 2 all.
   static const int pdl_gemm = [] { const char* v = getenv("L3_PDL_GEMM"); return v ? atoi(v) : 2; }();
   if (swap_on && gemm_swap_supported(a.rows, a.N)) {  // 9..128 rows: weights as the 128-row operand
     g_l3_pdl_next = ((norm && pdl_gemm == 1) || pdl_gemm == 2) && a.rows <= 32 && !(m->cfg.flags & L3_FLAG_NO_PDL);
@@ -690,23 +690,25 @@ static int enqueue_cluster_layers(L3Model* m, const int32_t* d_ids, int ids_ld, 
 }
 
 // Programmatic dependent launches: the kernels of a chunk are a chain, each of which waits for its predecessor (pdl_wait) ahead of its first
-// dependent access, so a kernel's prologue and its share of the launch latency run under the predecessor's tail.  Off : on, us.  Prompts:
-// 1B layers 33 tokens 224 : 198, 128 259 : 235, 2 x 731 494 : 464; 8B layers 33 337 : 319, 200 398 : 365, 800 773 : 749; stories15M 2
-// tokens 273 : 224, 100 666 : 593, 32 x 100 1096 : 1004.  Not 9 - 32 rows of layers that L2 does not hold, where every product waits for
-// DRAM and the swapped products are dependents already (8B, 9 tokens 269 : 263, 20 284 : 294, 32 287 : 296; 1B, 32 197 : 177).  Steps of 9 -
-// 16 sequences: 1B 9 sequences 1923 : 1759 a call, 16 1960 : 1805, 32 2222 : 2227, 8B 9 3393 : 3298, 16 3470 : 3444, 32 3806 : 3833, fp32
-// stories15M 9 5570 : 5403, 16 5597 : 5639, 30 6828 : 7182.  Layer lists: latent attention of width 2048 0.69 : 0.62 ms a step, 3.20 : 3.02
-// ms a prompt of 2048 tokens; prompts of 2048 tokens: linear mixers of width 2048 1042 : 982 us, parallel
-// layers 888 : 839, states and experts 1729 : 1688; eight sequences through chunk attention and matrix memories 6340 : 5612 us for 32 tokens.  Not
-// parallel layers of 5 - 8 rows, whose row-streaming products lose more to waiting successors in their shared memory than the launches
-// take (12 tokens of six sequences, width 512 2001 : 1955, 1024 2763 : 2972, 1536 2826 : 2901, 2048 3326 : 3271; four sequences 2138 : 2072 at
-// 1024).  NCCL's kernels between them take no part (tensor parallelism).
+// dependent access, so a kernel's prologue and its share of the launch latency run under the predecessor's tail.  Off : on, us.
+// Prompts: 1B layers 2 tokens 209 : 198, 8 285 : 283, 9 166 : 146, 20 172 : 164, 33 199 : 172, 2 x 731 494 : 464; 8B layers 2 331 : 313, 4 411 :
+// 413, 8 567 : 572, 9 275 : 266, 20 271 : 270, 28 277 : 277, 32 282 : 275, 33 311 : 290, 800 773 : 749; fp32 of width 4096 2 432 : 416, 9 636 :
+// 618, 32 663 : 658; stories15M 2 269 : 228, 9 296 : 274, 40 428 : 344.
+// Greedy runs of 12 steps by sequences.  Up to 8, row-streaming products, the sides differ by size: 1B 2 2147 : 2194, 8 3494 : 3466; fp32 of width
+// 1024 2 1576 : 1723; bf16 of width 1024 8 2984 : 3151.  9 - 16: 1B 9 1794 : 1582, 16 1855 : 1649; 8B 9 3262 : 3134, 16 3275 : 3208; fp32 of width
+// 1024 16 1893 : 1774; stories15M 9 3361 : 3183, 16 3558 : 3420.  17 - 32, whose products are dependents already, differ by size again: 1B 17 1877 :
+// 1751, 8B 17 3346 : 3357, 31 3520 : 3428; bf16 of width 1024 17 1324 : 1378, stories15M 17 3863 : 4093.  More than 32: 1B 33 2269 : 1981, 128 3074 :
+// 2863; 8B 40 3918 : 3615, 100 4827 : 4894, 160 5330 : 5203; fp32 of width 2048 40 3927 : 3751; bf16 of width 512 40 1515 : 1427.
+// Layer lists: latent attention of width 2048 0.69 : 0.62 ms a step, 3.20 : 3.02 ms a prompt of 2048 tokens; prompts of 2048 tokens: linear
+// mixers of width 2048 1042 : 982 us, parallel layers 888 : 839, states and experts 1729 : 1688; eight sequences through chunk attention and
+// matrix memories 6340 : 5612 us for 32 tokens.  Not parallel layers of 5 - 8 rows, whose row-streaming products lose more to waiting
+// successors in their shared memory than the launches take (12 tokens of six sequences, width 512 2001 : 1955, 1024 2763 : 2972, 1536 2826 :
+// 2901, 2048 3326 : 3271; four sequences 2138 : 2072 at 1024).
+// NCCL's kernels between them take no part (tensor parallelism).
 static bool pdl_pays(const L3Model* m, int ntok, int L) {
   if (m->ll) return !(m->ll->cfg.parallel && ntok > 4 && ntok <= 8);
   if (m->G > 1) return false;
-  if (L == 1) return ntok > 8 && ntok <= 16;
-  const size_t layer = ((size_t)(m->qkv_rows + m->HN * m->HD) * m->D + (size_t)3 * m->FD * m->D) * (m->bf16 ? 2 : 4);
-  return ntok <= 8 || ntok > 32 || layer <= (size_t)126 << 20;
+  return L > 1 || (ntok > 8 && ntok <= 16) || ntok > 32;
 }
 
 extern "C" int l3_debug_pdl(L3Model* m, int B, int L) {

@@ -58,11 +58,11 @@ def _outputs(m, vocab, B, llama):
     return out, n
 
 
-@pytest.mark.parametrize("B", [1, 6, 12, 40])
+@pytest.mark.parametrize("B", [1, 6, 12, 20, 40])
 @pytest.mark.parametrize("name,dtype", [("llama", "float32"), ("llama", "bfloat16")] + [(f, d) for f in sorted(FAMILIES) for d in ("float32", "bfloat16")])
 def test_every_switch_gives_the_same_bits(name, dtype, B, monkeypatch):
-    if name != "llama" and B == 40:
-        B = 3
+    if name != "llama" and B > 12:
+        B = B // 20 + 2
     make = (lambda flags: _llama(dtype, B, flags)) if name == "llama" else (lambda flags: _family(name, dtype, B, flags))
     want, n = _outputs(*make(0), B, name == "llama")
     for env, flags in (("0", 0), ("1", 0), (None, _cabi.FLAG_NO_PDL)):
@@ -95,11 +95,8 @@ def test_the_switches_belong_to_a_handle(monkeypatch):
 
 def test_the_rule():
     m, _ = _llama("float32", 64, 0)
-    assert [_dependent(m, b, 1) for b in (1, 8, 9, 16, 17, 64)] == [0, 0, 1, 1, 0, 0]    # steps: 9 - 16 sequences
-    assert [_dependent(m, 1, n) for n in (2, 8, 9, 32, 33, 90)] == [1] * 6               # prompts of layers that L2 holds
-    m.close()
-    m, _ = _llama("bfloat16", 1, 0, dim=4096, heads=32, ff=11008, layers=1)              # 405 MB a layer
-    assert [_dependent(m, 1, n) for n in (2, 8, 9, 32, 33, 90)] == [1, 1, 0, 0, 1, 1]
+    assert [_dependent(m, b, 1) for b in (1, 8, 9, 16, 17, 32, 33, 64)] == [0, 0, 1, 1, 0, 0, 1, 1]    # steps by sequences
+    assert all(_dependent(m, 1, n) for n in (2, 8, 9, 32, 33, 90))                                      # prompts
     m.close()
     for name in FAMILIES:
         m, _ = _family(name, "float32", 12, 0)
