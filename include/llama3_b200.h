@@ -354,6 +354,8 @@ int l3_op_rope(int device, const float* x, const double* cos_tab, const double* 
                int B, int L, int heads, int head_dim, int start_pos, float* out);
 /* silu(gate) * up (llama3.py:27-28, 99-101) elementwise over n values */
 int l3_op_swiglu(int device, const float* gate, const float* up, int64_t n, float* out);
+/* gelu(gate) * up elementwise, GELU in its tanh form (a feed-forward of the Risalix family) */
+int l3_op_geglu(int device, const float* gate, const float* up, int64_t n, float* out);
 /* Attention core (llama3.py:190-207): q [B, L, HN, HD]; k, v caches in the reference layout
  * [B, T, KVHN, HD] holding T = start_pos + L valid positions; out [B, L, HN*HD]. */
 int l3_op_attention(int device, const float* q, const float* k, const float* v,

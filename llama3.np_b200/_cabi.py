@@ -109,6 +109,7 @@ SIGNATURES = {
     "l3_op_linear": (_I, [_I, _F32P, _F32P, _I, _I, _I, _I, _I, _F32P]),
     "l3_op_rope": (_I, [_I, _F32P, _F64P, _F64P, _I, _I, _I, _I, _I, _F32P]),
     "l3_op_swiglu": (_I, [_I, _F32P, _F32P, C.c_int64, _F32P]),
+    "l3_op_geglu": (_I, [_I, _F32P, _F32P, C.c_int64, _F32P]),
     "l3_op_attention": (_I, [_I, _F32P, _F32P, _F32P, _I, _I, _I, _I, _I, _I, _I, _I, _F32P]),
     "l3_op_prompt_attention": (_I, [_I, _F32P, _F32P] + [_I] * 12 + [C.c_float, _F32P]),
     "l3_op_recurrence": (_I, [_I] + [_F32P] * 6 + [_I] * 6 + [_F32P]),

@@ -99,11 +99,16 @@ __device__ __forceinline__ void split_tf32(float v, float& hi, float& lo) {
 // silu exactly as the reference writes it: x * (1 / (1 + exp(-x)))   (llama3.py:27-28)
 __device__ __forceinline__ float silu_ref(float x) { return x * (1.0f / (1.0f + expf(-x))); }
 
-// tanh form of GELU, 0.5 z (1 + tanh(y)) with y = sqrt(2 / pi) (z + 0.044715 z^3), as z / (1 + exp(-2 y)): the same function, without the
-// difference of nearly equal numbers for z < 0, and one exponential in place of tanhf.  2048 x 16384 x 2048 with
-// it in the epilogue, as a loop of its own like silu's: 148.8 -> 110.2 us (the formula alone, inside the loop that asks for the activation
-// at every value: no change)
-__device__ __forceinline__ float gelu_tanh_ref(float z) { return z / (1.0f + expf(-1.5957691216057308f * (z + 0.044715f * z * z * z))); }
+// tanh form of GELU, 0.5 z (1 + tanh(y)) with y = sqrt(2 / pi) (z + 0.044715 z^3), as max(z, 0) - |z| q, q = 1 / (1 + exp(2 |y|)): the same
+// function with one exponential in place of tanhf and without the difference of nearly equal numbers for z < 0.  Error against 64 bits, 2-norm
+// over 4 million normal z: sigma 0.1 4.1e-8 (tanhf's form 3.9e-8), 0.3 3.9e-8 (4.5e-8), 1 2.9e-8 (3.8e-8), 4 1.6e-8 (2.2e-8); z / (1 + exp(-2 y)),
+// as fast, has 4.3e-8 at 1.  2048 x 16384 x 2048 with it in the epilogue, as a loop of its own like silu's: 148.8 -> 110.2 us (the formula
+// alone, inside the loop that asks for the activation at every value: no change)
+__device__ __forceinline__ float gelu_tanh_ref(float z) {
+  const float e = expf(-fabsf(z) * fmaf(0.07135481282f, z * z, 1.5957691216057308f)), q = e / (1.0f + e);
+  const float r = fmaf(-fabsf(z), q, fmaxf(z, 0.f));
+  return z > 1e30f ? z : r;  // an infinity stays one
+}
 // activation of a gated linear unit's gate column (EpiArgs::act)
 enum GluAct : int { GLU_SILU = 0, GLU_GELU_TANH = 1, GLU_CLAMP = 2 };
 __device__ __forceinline__ float glu_act(int act, float z) { return act == GLU_GELU_TANH ? gelu_tanh_ref(z) : silu_ref(z); }
@@ -405,7 +410,7 @@ cudaError_t launch_set_int(int* p, int v, cudaStream_t s);
 cudaError_t launch_add_int(int* p, int v, cudaStream_t s);
 cudaError_t launch_rope_only(const float* x, const float* cos_tab, const float* sin_tab, int B, int L, int heads,
                              int HD, const int* pos_ptr, float* out, cudaStream_t s);
-cudaError_t launch_swiglu(const float* gate, const float* up, int64_t n, float* out, cudaStream_t s);
+cudaError_t launch_glu(int act, const float* gate, const float* up, int64_t n, float* out, cudaStream_t s);  // GLU_SILU, GLU_GELU_TANH
 cudaError_t launch_pack_rows(const float* src, int rows, int cols, void* dst, bool dst_bf16, int dst_row0,
                              int dst_row_stride, int dst_ld, cudaStream_t s);
 cudaError_t launch_ragged_setup(const int* len, int B, int Lmax, int32_t* lastrow, int* done, cudaStream_t s);

@@ -162,17 +162,19 @@ extern "C" int l3_op_rope(int device, const float* x, const double* cos_tab, con
   return rc;
 }
 
-extern "C" int l3_op_swiglu(int device, const float* gate, const float* up, int64_t n, float* out) {
+static int op_glu(int act, int device, const float* gate, const float* up, int64_t n, float* out) {
   Scratch sc;
   if (begin(sc, device)) return L3_ECUDA;
   float* dg = sc.up(gate, (size_t)n);
   float* du = sc.up(up, (size_t)n);
   float* dout = sc.dev<float>((size_t)n);
   if (!dg || !du || !dout) return L3_ENOMEM;
-  int rc = finish(sc, launch_swiglu(dg, du, n, dout, sc.s));
+  int rc = finish(sc, launch_glu(act, dg, du, n, dout, sc.s));
   if (rc == L3_OK) cudaMemcpy(out, dout, (size_t)n * 4, cudaMemcpyDeviceToHost);
   return rc;
 }
+extern "C" int l3_op_swiglu(int device, const float* gate, const float* up, int64_t n, float* out) { return op_glu(GLU_SILU, device, gate, up, n, out); }
+extern "C" int l3_op_geglu(int device, const float* gate, const float* up, int64_t n, float* out) { return op_glu(GLU_GELU_TANH, device, gate, up, n, out); }
 
 extern "C" int l3_op_attention(int device, const float* q, const float* k, const float* v, int B, int L, int n_heads,
                                int n_kv_heads, int head_dim, int start_pos, int kv_bf16, int nsplit, float* out) {

@@ -315,13 +315,15 @@ cudaError_t launch_rope_only(const float* x, const float* cos_tab, const float* 
   return cudaGetLastError();
 }
 
-__global__ void swiglu_kernel(const float* __restrict__ gate, const float* __restrict__ up, int64_t n,
-                              float* __restrict__ out) {
+template <int ACT>
+__global__ void glu_kernel(const float* __restrict__ gate, const float* __restrict__ up, int64_t n,
+                           float* __restrict__ out) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = silu_ref(gate[i]) * up[i];
+  if (i < n) out[i] = glu_act(ACT, gate[i]) * up[i];
 }
-cudaError_t launch_swiglu(const float* gate, const float* up, int64_t n, float* out, cudaStream_t s) {
-  swiglu_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(gate, up, n, out);
+cudaError_t launch_glu(int act, const float* gate, const float* up, int64_t n, float* out, cudaStream_t s) {
+  if (act == GLU_GELU_TANH) glu_kernel<GLU_GELU_TANH><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(gate, up, n, out);
+  else glu_kernel<GLU_SILU><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(gate, up, n, out);
   return cudaGetLastError();
 }
 
