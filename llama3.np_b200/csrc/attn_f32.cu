@@ -12,8 +12,8 @@
 // What bounds it: the FFMA pipe (a tile of 32 x 64 with heads of 192 | 128 is 655 k products, 128 a cycle), then the latency of a tile.  The
 // kernels it took over from read 12 wavefronts per 8 cycles of products and loaded each tile in between (attn_window.cu), or had a barrier
 // between scores, softmax and output (attention.cu).  600 tokens, 8 heads of 192 | 128: 123.5 -> 79 us a layer.
-// A warp's output loop runs over the keys that one of its rows sees: values of other keys - a NaN or an infinity in a later token - do
-// not reach it.
+// A warp's output loop runs over the keys that one of its eight rows sees: values of other keys - a NaN or an infinity in a later token -
+// do not reach it.
 #include <stdlib.h>
 
 #include <algorithm>

@@ -165,14 +165,9 @@ __global__ void __launch_bounds__(256) win_prep_kernel(WinPrepArgs a) {
 }
 
 __device__ __forceinline__ float ld_cluster(const float* p, int rank) {  // the same place in another CTA of the cluster
-  uint32_t a;
   float v;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_at((uint32_t)__cvta_generic_to_shared(p), (uint32_t)rank)) : "memory");
   return v;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.0f / (1.0f + expf(-z)); }

@@ -20,6 +20,22 @@ typedef __nv_bfloat16 bf16;
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// one lane of the (whole) warp; the compiler knows it is one, and that what the warp agrees on is uniform inside the branch
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+  return p != 0;
+}
+// this CTA's shared address `addr` in the CTA of that rank of its cluster; a barrier for every thread of every CTA of the cluster
+__device__ __forceinline__ uint32_t cluster_at(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // l3_api.cu; of the calling thread: launches of a scope (PdlScope, internal.h), and set right before ONE launch that should overlap its
 // predecessor's tail (consumed by launch_k)
 extern thread_local bool g_l3_pdl, g_l3_pdl_next;

@@ -74,11 +74,6 @@ __device__ __forceinline__ void bulk_load(float* dst, const float* src, int n, u
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(s32(dst)), "l"(src), "r"(n * 4), "r"(bar) : "memory");
 }
-__device__ __forceinline__ uint32_t in_cta(uint32_t addr, int r) {
-  uint32_t d;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(addr), "r"(r));
-  return d;
-}
 // Four values into another CTA's shared memory; its barrier counts the bytes as they land
 __device__ __forceinline__ void send4(uint32_t dst, float4 v, uint32_t bar) {
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
@@ -232,7 +227,7 @@ __global__ void __launch_bounds__(TH, 1) decode_cluster_kernel(const __grid_cons
     }
   };
   auto send_rows = [&](const float* o, int n, uint32_t to, int ld, int p) {  // o[b][n] -> to + b * ld, warp w to CTA w
-    const uint32_t dst = in_cta(to, warp), bar = in_cta(bar0 + 8 * (p - 1), warp);
+    const uint32_t dst = cluster_at(to, warp), bar = cluster_at(bar0 + 8 * (p - 1), warp);
     const int sh = n <= 32 ? 3 : n <= 64 ? 4 : 5;  // lanes for a sequence's fours: 8, 16 or 32
     for (int b = lane >> sh; b < B; b += 32 >> sh)
       for (int i = 4 * (lane & ((1 << sh) - 1)); i < n; i += 4 << sh) send4(dst + (b * ld + i) * 4, *reinterpret_cast<const float4*>(o + b * n + i), bar);
@@ -277,7 +272,7 @@ __global__ void __launch_bounds__(TH, 1) decode_cluster_kernel(const __grid_cons
     wait(1);
     // ---- 2: keys of the cache from registers, this step's from the exchange.  Every warp keeps the running maximum of its own keys.
     {
-      const uint32_t dst = in_cta(s32(att), warp), bar = in_cta(bar0 + 8, warp);
+      const uint32_t dst = cluster_at(s32(att), warp), bar = cluster_at(bar0 + 8, warp);
       int copy = 0, b = it_b, h = it_h;
       while (b < B) {
         const int g = rep == 1 ? h : h / rep;

@@ -15,7 +15,7 @@
 // Data movement: every CTA streams ITS slice of the layer's weights (pre-packed k-major slabs, 648 KB per layer
 // at the stories15M shape) and the K / V rows of its head from L2 / HBM with cp.async.bulk into a ring of 8 x 18 KB
 // stages.  Four producer warps issue the copies (one thread sustains only ~49 GB/s of bulk copies, four reach
-// ~220 GB/s per SM: scripts/ubench, profiles/ubench.jsonl); nine compute warps consume.  Weights and cached
+// ~220 GB/s per SM: profiles/ubench.jsonl); nine compute warps consume.  Weights and cached
 // K / V do not depend on this step's activations, so the producers run ahead across phase changes.
 //
 // Math: fp32 FFMA in pairs of sequences (fma2).  Thread tile = 4 output features x ALL S sequences (48 accumulators) over a k-group (1/4 or
@@ -119,16 +119,8 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
 __device__ __forceinline__ void st_cluster_f4(uint32_t addr, float a, float b, float c, float d) {
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-__device__ __forceinline__ void cluster_sync_all() {  // every thread of every CTA of the cluster
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ unsigned long long gtime() {
   unsigned long long t;
@@ -441,7 +433,7 @@ __device__ __forceinline__ void push_partials(const float (&own)[Cf::S], uint32_
   const Tile<F, G> tl;
   static_assert(Tile<F, G>::NFG == Cf::NCW * Tile<F, G>::FPW && G == Cf::GB && F == Cf::D, "every lane of every compute warp holds a tile");
   const int f0 = 4 * tl.fg, owner = f0 / Cf::DS, fl = f0 % Cf::DS;  // DS % 4 == 0: the four features share an owner
-  const uint32_t dst = mapa(recv_local, (uint32_t)owner) + (uint32_t)(((rank * Cf::DS + fl) * Cf::RLD) * 4);
+  const uint32_t dst = cluster_at(recv_local, (uint32_t)owner) + (uint32_t)(((rank * Cf::DS + fl) * Cf::RLD) * 4);
 #pragma unroll
   for (int q = 0; q < Cf::QS; ++q)
     st_cluster_f4(dst + (uint32_t)((tl.kg * Cf::RLD + 4 * q) * 4), own[4 * q], own[4 * q + 1], own[4 * q + 2], own[4 * q + 3]);
@@ -450,8 +442,8 @@ __device__ __forceinline__ void push_partials(const float (&own)[Cf::S], uint32_
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int o_lo = (warp * Tile<F, G>::FPW * 4) / Cf::DS, o_hi = ((warp + 1) * Tile<F, G>::FPW * 4 - 1) / Cf::DS;
   static_assert(Tile<F, G>::FPW * 4 <= Cf::DS, "a warp's tiles span at most two owners");
-  if (lane == 0) mbar_arrive_remote(mapa(pbar_local, (uint32_t)o_lo));
-  if (lane == 1 && o_hi != o_lo) mbar_arrive_remote(mapa(pbar_local, (uint32_t)o_hi));
+  if (lane == 0) mbar_arrive_remote(cluster_at(pbar_local, (uint32_t)o_lo));
+  if (lane == 1 && o_hi != o_lo) mbar_arrive_remote(cluster_at(pbar_local, (uint32_t)o_hi));
 }
 
 // The owner of residual columns [rank DS, rank DS + DS): x_new = x + sum over ranks (in rank order) of the
@@ -473,10 +465,10 @@ __device__ __forceinline__ void reduce_and_gather(const float* recv, float* xres
     *xr = r;
     const uint32_t off = (uint32_t)(((rank * DS + fl) * Cf::XLD + 4 * q) * 4);
 #pragma unroll
-    for (int p = 0; p < Cf::C; ++p) st_cluster_f4(mapa(xt_local, (uint32_t)p) + off, r.x, r.y, r.z, r.w);
+    for (int p = 0; p < Cf::C; ++p) st_cluster_f4(cluster_at(xt_local, (uint32_t)p) + off, r.x, r.y, r.z, r.w);
   }
   __syncwarp();
-  if (lane < Cf::C) mbar_arrive_remote(mapa(gbar_local, (uint32_t)lane));
+  if (lane < Cf::C) mbar_arrive_remote(cluster_at(gbar_local, (uint32_t)lane));
 }
 
 // debug dumps, [NL][4][B][D]: kind 0 = q, 1 = attention output, 2 / 3 = the residual stream after the first / second

@@ -50,11 +50,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* tm,
       ::"r"(dst), "l"(tm), "r"(c0), "r"(c1), "r"(bar) : "memory");
 }
 // one lane of the (whole) warp, known as one to the compiler (see gemm_tc_dev.cuh)
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(p));
-  return p != 0;
-}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
@@ -94,19 +89,11 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
-__device__ __forceinline__ uint32_t at_rank(const float* p, int rank) {  // the same place in another CTA of the cluster
-  uint32_t a;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
-  return a;
-}
 // 0 where not `on`: a predicate and no branch, so that a row of such loads is in flight together
 __device__ __forceinline__ float ld_cluster_if(bool on, uint32_t a) {
   float v;
   asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %2, 0;\nmov.f32 %0, 0f00000000;\n@p ld.shared::cluster.f32 %0, [%1];\n}" : "=f"(v) : "r"(a), "r"((int)on) : "memory");
   return v;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 constexpr int SW_THREADS = 224;  // warp 0 = weight copies, warp 1 = TMEM + MMA, warps 2-5 = epilogue, warp 6 = activation copies
@@ -359,7 +346,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant
 #pragma unroll
           for (int j = 0; j < CJ; ++j) v[j] = 0.f;
           for (int k2 = 0; k2 < ksplit; ++k2) {
-            const uint32_t src = at_rank(mine + c0 * Cf::BMW, k2);
+            const uint32_t src = cluster_at(smem_u32(mine + c0 * Cf::BMW), (uint32_t)k2);
             float w[32];
 #pragma unroll
             for (int j = 0; j < CJ; ++j) w[j] = ld_cluster_if(c0 + j < m_hi, src + j * Cf::BMW * 4);

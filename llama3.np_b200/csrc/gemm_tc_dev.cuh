@@ -54,24 +54,12 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* tm,
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
       ::"r"(dst), "l"(tm), "r"(c0), "r"(c1), "r"(bar) : "memory");
 }
-// one lane of the (whole) warp; the compiler knows it is one, and that what the warp agrees on is uniform inside the branch
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(p));
-  return p != 0;
-}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-// the same between the two CTAs of a pair: shared::cluster address of this CTA's `addr` in the CTA of rank r; an arrival and a tile
-// load that complete there; products over both CTAs' operand tiles and the commit that reports them to both
-__device__ __forceinline__ uint32_t pair_addr(uint32_t addr, uint32_t r) {
-  uint32_t d;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(addr), "r"(r));
-  return d;
-}
+// between the two CTAs of a pair: an arrival and a tile load that complete at a shared::cluster address (cluster_at); products over both CTAs' operand tiles and the commit that reports them to both
 __device__ __forceinline__ void pair_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -88,9 +76,6 @@ __device__ __forceinline__ void pair_mma(uint32_t tmem_d, uint64_t adesc, uint64
       "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
       "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}"
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum) : "memory");
-}
-__device__ __forceinline__ void pair_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 template <int KIND>
 __device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
@@ -218,7 +203,7 @@ __device__ __forceinline__ void tc_pipe_setup(TcPipe& p, uint8_t* smem_raw, int 
   }
   if (CG == 2) {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // the other CTA's barriers stand before anything arrives there
-    if (p.rank && warp == 1 && lane == 0) pair_arrive(pair_addr(p.peer, 0));  // this CTA's TMEM is there: the first one's products may write to it
+    if (p.rank && warp == 1 && lane == 0) pair_arrive(cluster_at(p.peer, 0));  // this CTA's TMEM is there: the first one's products may write to it
   }
   __syncwarp();
 }
@@ -245,7 +230,7 @@ __device__ __forceinline__ void tc_pipe_teardown(TcPipe& p, int* err) {
     *err = 1;
   }
   __syncthreads();
-  if (CG == 2) pair_sync();  // nothing of the other CTA is under way to this one any more
+  if (CG == 2) cluster_sync_all();  // nothing of the other CTA is under way to this one any more
   if ((threadIdx.x >> 5) == 1) {
     if constexpr (CG == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(p.tmem_base), "r"(Cf::tmem_cols(p.bn)));
     else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(p.tmem_base), "r"(Cf::tmem_cols(p.bn)));
@@ -291,7 +276,7 @@ __device__ __forceinline__ void tc_gemm_run(TcPipe& p, const CUtensorMap* tmA0, 
         const uint32_t st = tiles + s * STAGE_BYTES;
         if (elect_one()) {
           if constexpr (CG == 2) {  // both CTAs' tiles are counted by the first one's barrier, where the products wait for them
-            const uint32_t bar = pair_addr(full0 + 8 * s, 0);
+            const uint32_t bar = cluster_at(full0 + 8 * s, 0);
             if (rank == 0) mbar_expect_tx(full0 + 8 * s, CG * STAGE_BYTES);
             pair_load_2d(st, tmA0, kb * Cf::BK, m0, bar);
             pair_load_2d(st + Cf::A_BYTES, tmB0, kb * Cf::BK + kg, n0, bar);
@@ -388,7 +373,7 @@ __device__ __forceinline__ void tc_gemm_run(TcPipe& p, const CUtensorMap* tmA0, 
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
-        if constexpr (CG == 2) pair_arrive(pair_addr(accempty0 + 8 * buf, 0));
+        if constexpr (CG == 2) pair_arrive(cluster_at(accempty0 + 8 * buf, 0));
         else mbar_arrive(accempty0 + 8 * buf);
       }
     };

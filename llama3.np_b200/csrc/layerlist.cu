@@ -967,7 +967,7 @@ static bool ll_latent_on_tc(const L3Model* m, const L3LayerSpec& s) {
 // key, head) instead of the folded form's 2 (2 kv_rank + rot_dim), for an expansion of 2 (dim + vdim) kv_rank per (key, head), which
 // runs on the tensor cores while the attention is FFMA in both forms.  8 heads of 128 + 64, values 128, rank 512, per layer: 600 tokens
 // 338 + 90 us (attention, products of the folded form) -> 123 + 45 us; the two-layer prompt 1624 -> 1097 us, at 64 tokens 436 -> 329 us.
-// A portion expands its whole prefix again, and the window kernel walks a tile's keys in one CTA where the folded kernel splits them, so
+// A portion expands its whole prefix again, and the attention kernel walks a tile's keys in one CTA where the folded kernel splits them, so
 // behind a prefix it takes enough query rows to fill the chip: from 128 tokens and 2048 rows (sequences x heads x tokens) on it gains for
 // every prefix (two layers of width 1024, 256 tokens behind 6144: 1.07, 400 behind 6000: 1.98; 16 heads, 128 behind 2048: 1.08), below
 // that up to a prefix of twice the portion where sequences x heads are at most 32 (64 behind 128: 1.15, 64 behind 2048: 0.52, 64 behind
