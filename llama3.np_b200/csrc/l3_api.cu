@@ -703,10 +703,14 @@ static int enqueue_cluster_layers(L3Model* m, const int32_t* d_ids, int ids_ld, 
 // mixers of width 2048 1042 : 982 us, parallel layers 888 : 839, states and experts 1729 : 1688; eight sequences through chunk attention and
 // matrix memories 6340 : 5612 us for 32 tokens.  Not parallel layers of 5 - 8 rows, whose row-streaming products lose more to waiting
 // successors in their shared memory than the launches take (12 tokens of six sequences, width 512 2001 : 1955, 1024 2763 : 2972, 1536 2826 :
-// 2901, 2048 3326 : 3271; four sequences 2138 : 2072 at 1024).
+// 2901, 2048 3326 : 3271; four sequences 2138 : 2072 at 1024).  Nor fp32 steps of 9 - 32 sequences without parallel layers, by size again (12
+// tokens, 9 sequences, width 512 linear mixers 3674 : 3786, states 4492 : 4731, latent attention 3914 : 3929, matrix memories 2670 : 2760; 32
+// sequences of width 1024 5698 : 5700, 7456 : 7363, 4888 : 5501, 4313 : 4264; parallel layers 16 of width 1024 3849 : 3679); in bf16 linear mixers
+// 9 of width 2048 3963 : 3524.
 // NCCL's kernels between them take no part (tensor parallelism).
 static bool pdl_pays(const L3Model* m, int ntok, int L) {
-  if (m->ll) return !(m->ll->cfg.parallel && ntok > 4 && ntok <= 8);
+  if (m->ll && m->ll->cfg.parallel) return ntok <= 4 || ntok > 8;
+  if (m->ll) return m->bf16 || L > 1 || ntok <= 8 || ntok > 32;
   if (m->G > 1) return false;
   return L > 1 || (ntok > 8 && ntok <= 16) || ntok > 32;
 }

@@ -99,6 +99,10 @@ def test_the_rule():
     assert all(_dependent(m, 1, n) for n in (2, 8, 9, 32, 33, 90))                                      # prompts
     m.close()
     for name in FAMILIES:
-        m, _ = _family(name, "float32", 12, 0)
-        assert [_dependent(m, b, 1) for b in (1, 4, 5, 8, 9, 12)] == ([1, 1, 0, 0, 1, 1] if name == "mabedra" else [1] * 6)
-        m.close()
+        for dtype in ("float32", "bfloat16"):
+            m, _ = _family(name, dtype, 36, 0)
+            rows = (1, 4, 5, 8, 9, 32, 33)
+            want = [1, 1, 0, 0, 1, 1, 1] if name == "mabedra" else [1, 1, 1, 1, 0, 0, 1] if dtype == "float32" else [1] * 7
+            assert [_dependent(m, b, 1) for b in rows] == want, (name, dtype)
+            assert [_dependent(m, 1, n) for n in rows[1:]] == ([1, 0, 0, 1, 1, 1] if name == "mabedra" else [1] * 6), (name, dtype)
+            m.close()
