@@ -29,7 +29,7 @@ __device__ __forceinline__ bool elect_one() {
 // this CTA's shared address `addr` in the CTA of that rank of its cluster; a barrier for every thread of every CTA of the cluster
 __device__ __forceinline__ uint32_t cluster_at(uint32_t addr, uint32_t rank) {
   uint32_t r;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
 __device__ __forceinline__ void cluster_sync_all() {
