@@ -288,7 +288,7 @@ def shape_record(name, shape, dtype, B, L, n_decode, device=0, ids=None, iters=2
         tokens = np.empty((B, n_decode), np.int64)
         _cabi.check(lib.l3_memcpy_d2h(h, tokens.ctypes.data_as(C.c_void_p), d_out, tokens.nbytes), h)
         ms_dec = (ms_gen - ms_pf) / (n_decode - 1)            # per decode step (the first token comes from the prefill)
-        params = param_count(args, hidden) - VS * D + D        # weights read per decoded token (SURVEY 8d)
+        params = param_count(args, hidden) - VS * D + D        # weights read per decoded token
         pos_mid = L + n_decode // 2
         bytes_step = params * wb + B * NL * nkv * pos_mid * hd * 2 * wb
         rec.update(value=B / (ms_dec / 1e3), unit="tokens/s", ms_per_step=ms_dec, gpu_launches_per_generate=launches,
@@ -370,7 +370,7 @@ def cpu_shape_baseline(shape, B, L, n_decode_sample):
 def run_extras(a, local):
     from llama3_np_b200.tokenizer import Tokenizer  # noqa: F401  (host tokenizer stays on the host; ids are fed directly)
     recs = []
-    dream = np.array([[1, 76, 505, 263, 12561]])  # "I have a dream" through the reference tokenizer (SURVEY 8d C1)
+    dream = np.array([[1, 76, 505, 263, 12561]])  # "I have a dream" through the reference tokenizer
 
     def guarded(fn, name):
         try:

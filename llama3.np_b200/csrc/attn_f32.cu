@@ -304,7 +304,8 @@ template <int NC> cudaError_t launch_nc(const WinAttnArgs& a, cudaStream_t s) {
   const dim3 grid((a.L * (a.H / a.G) + FR - 1) / FR, a.G, a.B);
   const long ctas = (long)grid.x * grid.y * grid.z;
   // One CTA per SM: two groups, us with one : two.  Grids of up to one CTA per SM, vupitar width 512, 800 tokens 784 : 712; up to two, debuzen
-  // width 1024, 800 tokens 2230 : 2146; above, and with one tile of keys to walk, within 1 %.
+  // width 1024, 800 tokens 2230 : 2146; above, and with one tile of keys to walk, within 1 %.  (296: twice the SMs.  The instance of 256 value
+  // columns and two groups spills 136 bytes; over value sizes of 160 - 256, 40 - 800 tokens, it takes 0.88 - 1.01 of the tiled kernel's time.)
   const bool fits = smem_bytes(a.DK, a.DV, 2) <= 220 * 1024, pair = smem_bytes(a.DK, a.DV, 1) <= 113 * 1024;
   return fits && (!pair || (a.L > FK && ctas <= 296)) ? launch_gr<NC, 2>(a, grid, s) : launch_gr<NC, 1>(a, grid, s);
 }

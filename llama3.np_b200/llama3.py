@@ -27,7 +27,7 @@ from .utils import checkpoint_digest, load_parameters, packed_cache_path
 def compute_cos_sin_cache(head_dim: int, max_seq_len: int, base: int = 10000):
     """float64 RoPE tables `[max_seq_len, head_dim // 2]` (reference llama3.py:31-38).
     Computed on the host in float64 and uploaded: fp32 `sincosf` of `t * inv_freq` on the
-    device would drift by ~1e-5 at t <= 256 and ~2e-3 rad at t = 32k (SURVEY 7.2-4)."""
+    device would drift by ~1e-5 at t <= 256 and ~2e-3 rad at t = 32k."""
     inv_freq = 1.0 / (base ** (np.arange(0, head_dim, 2)[: head_dim // 2] / head_dim))
     freqs = np.outer(np.arange(max_seq_len), inv_freq)
     return np.cos(freqs), np.sin(freqs)

@@ -186,7 +186,7 @@ class OracleLlama:
 
 
 def scaled_max_err(got: np.ndarray, want: np.ndarray) -> float:
-    """max|got - want| / max|want| - the 'relative error' of the parity bar (SURVEY 8(c))."""
+    """max|got - want| / max|want| - the 'relative error' of the parity bar."""
     want = np.asarray(want, dtype=np.float64)
     got = np.asarray(got, dtype=np.float64)
     return float(np.max(np.abs(got - want)) / max(np.max(np.abs(want)), 1e-30))

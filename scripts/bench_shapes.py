@@ -88,7 +88,7 @@ def run(name, shape, dtype, B, L, n_decode, n_layers=None, flags=0, iters=2):
         ms_gen = timed(m, gen, iters)
         launches = m.launch_count(reset=True) // iters
         ms_dec = (ms_gen - ms_pf) / (n_decode - 1)          # per decode step (first token comes from the prefill)
-        params = param_count(args, hidden) - VS * D + D      # weights read per decoded token (SURVEY 8d)
+        params = param_count(args, hidden) - VS * D + D      # weights read per decoded token
         pos_mid = L + n_decode // 2
         bytes_step = params * wb + B * NL * nkv * pos_mid * hd * 2 * wb
         out.update(decode_ms_per_step=ms_dec, decode_tok_s=B / (ms_dec / 1e3), launches_per_generate=launches,

@@ -48,7 +48,7 @@ def test_synth_layout_and_param_counts():
     assert shapes["model.layers.0.mlp.up_proj.weight"] == (768, 288)
     assert shapes["lm_head.weight"] == (32000, 288)
     assert len(shapes) == 3 + 9 * 6
-    # SURVEY 8(d): params read per decoded token = everything but the embedding table + one row
+    # params read per decoded token = everything but the embedding table + one row
     assert param_count(args, hidden) - 32000 * 288 + 288 == 15_192_000
     a8, h8 = named_config("llama3-8b")
     assert param_count(a8, h8) == 8_030_261_248

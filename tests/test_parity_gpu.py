@@ -3,7 +3,7 @@ the oracle on the same seeded inputs and against the golden fixtures recorded fr
 unmodified reference.
 
 Bars: fp32 mode - identical greedy tokens, logits within 1e-4 of
-max|logit| ("relative" as defined in SURVEY 8(c)); bf16 mode - scaled error <= 3e-2 and
+max|logit| (relative to the largest logit); bf16 mode - scaled error <= 3e-2 and
 top-1 agreement on the tested steps where the oracle's top-1/top-2 gap exceeds the error.
 """
 import numpy as np
